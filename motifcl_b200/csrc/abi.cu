@@ -231,32 +231,41 @@ bool tc_wanted(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
     return (double)M * (double)N * (double)K >= (double)(1u << 22);
 }
 
-// term lists: product of plane pa of A with plane pb of B, smallest contributions first
-void act_term_list(int act_terms, int* pa, int* pb, int* n) {
-    *n = act_terms;
-    for (int t = 0; t < act_terms; ++t) { pa[t] = act_terms - 1 - t; pb[t] = 0; }
-}
-void grad_term_list(int grad_terms, int* pa, int* pb, int* n, int* planes) {
-    if (grad_terms >= 6) {
-        const int a[6] = {2, 0, 1, 1, 0, 0}, b[6] = {0, 2, 1, 0, 1, 0};
-        for (int t = 0; t < 6; ++t) { pa[t] = a[t]; pb[t] = b[t]; }
-        *n = 6; *planes = 3;
-    } else {
-        const int a[3] = {1, 0, 0}, b[3] = {0, 1, 0};
-        for (int t = 0; t < 3; ++t) { pa[t] = a[t]; pb[t] = b[t]; }
-        *n = 3; *planes = 2;
-    }
-}
-
 #define MCL_CU(ctx, what, call) do { cudaError_t _e = (call); if (_e != cudaSuccess) return fail_cuda(ctx, what, _e); } while (0)
 
-// One tensor-core product on prepared planes (adds the split-K workspace to the carve).
-int tc_product(mcl_cuda_ctx* ctx, const void* a, int a_planes, int lda, size_t a_stride, const void* b,
-               int b_planes, int ldb, size_t b_stride, float* c, int ldc, int M, int N, int K, const int* pa,
-               const int* pb, int nterms, const float* col_scale, float* splitk_ws, int splits) {
+// Tensor-core products on fp16 terms (tc_gemm.cu).  A call carves the terms of its tensors from the workspace, clears one
+// pair of magnitude words per tensor, fills the terms, and runs its products.
+struct TermBuf { size_t planes, scaled, words; size_t rows; int cols, ld; };
+size_t term_bytes(size_t rows, int ld) { return 2 * rows * (size_t)ld * 2; }
+TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled, size_t words) {
+    TermBuf t = {0, 0, words, rows, (int)cols, up8(cols)};
+    if (plain) t.planes = cv->reserve(term_bytes(rows, t.ld));
+    if (scaled) t.scaled = cv->reserve(term_bytes(rows, t.ld));
+    return t;
+}
+int fill_terms(mcl_cuda_ctx* ctx, const char* op, char* w, const TermBuf& t, const float* src, const float* col_scale, bool plain) {
+    cudaError_t e = mcl::launch_split_terms(src, (int)t.rows, t.cols, t.ld, col_scale, plain ? w + t.planes : nullptr,
+                                            col_scale ? w + t.scaled : nullptr, reinterpret_cast<uint32_t*>(w + t.words),
+                                            ctx->sm_count, ctx->stream);
+    if (e != cudaSuccess) return fail_cuda(ctx, op, e);
+    ctx->launches += 2;
+    return MCL_CUDA_OK;
+}
+mcl::TcOperand terms_of(char* w, const TermBuf& t, bool scaled, bool mn_major) {
+    mcl::TcOperand o = {w + (scaled ? t.scaled : t.planes), (int)t.rows, t.cols, t.ld, 2, mn_major ? 1 : 0,
+                        reinterpret_cast<const uint32_t*>(w + t.words) + (scaled ? 1 : 0)};
+    return o;
+}
+mcl::TcOperand digits_of(const char* T, size_t O, size_t I, bool mn_major) {
+    mcl::TcOperand o = {T, (int)O, (int)I, up8(I), 1, mn_major ? 1 : 0, nullptr};
+    return o;
+}
+constexpr size_t kWordBytes = 64;      // magnitude words of a call: one pair per tensor, 8 bytes each
+
+int tc_product(mcl_cuda_ctx* ctx, const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K,
+               const float* col_scale, float* splitk_ws, int splits) {
     int launches = 0;
-    cudaError_t e = mcl::launch_tc_gemm(a, a_planes, lda, a_stride, b, b_planes, ldb, b_stride, c, ldc, M, N, K,
-                                        pa, pb, nterms, col_scale, splitk_ws, splits, ctx->err_word,
+    cudaError_t e = mcl::launch_tc_gemm(a, b, c, (int)N, (int)M, (int)N, (int)K, col_scale, splitk_ws, splits, ctx->err_word,
                                         ctx->max_smem, ctx->sm_count, ctx->stream, &launches);
     ctx->launches += launches;
     if (e != cudaSuccess) return fail_cuda(ctx, "tensor-core contraction", e);
@@ -512,25 +521,22 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
         fused_wanted(ctx, x, nullptr, state, scale, y, nullptr, nullptr, in_features, out_features, batch))
         return fused_products(ctx, op, x, nullptr, state, nullptr, scale, y, nullptr, nullptr, C, in_features, out_features, batch);
     if (tc_wanted(ctx, batch, out_features, in_features)) {
-        const int ta = ctx->act_terms, ldi = up8(in_features);
         int splits = 1;
         const size_t sk = mcl::tc_splitk_workspace_bytes((int)batch, (int)out_features, (int)in_features,
                                                          ctx->sm_count, 0, &splits);
         Carver cv;
-        const size_t o_x = cv.reserve((size_t)ta * batch * ldi * 2), o_t = cv.reserve(out_features * (size_t)ldi * 2),
-                     o_k = cv.reserve(sk);
+        const size_t o_w = cv.reserve(kWordBytes);
+        const TermBuf xb = carve_terms(&cv, batch, in_features, true, false, o_w);
+        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2), o_k = cv.reserve(sk);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
-        MCL_LAUNCH(ctx, op, mcl::launch_split_planes(x, (int)batch, (int)in_features, nullptr, w + o_x, ldi, ta,
-                                                     nullptr, 0, 0, ctx->stream));
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, (int)C, (int)out_features, (int)in_features,
-                                                       w + o_t, ldi, nullptr, 0, ctx->stream));
-        int pa[6], pb[6], nt;
-        act_term_list(ta, pa, pb, &nt);
-        return tc_product(ctx, w + o_x, ta, ldi, batch * (size_t)ldi, w + o_t, 1, ldi, out_features * (size_t)ldi, y,
-                          (int)out_features, (int)batch, (int)out_features, (int)in_features, pa, pb, nt, scale,
-                          reinterpret_cast<float*>(w + o_k), splits);
+        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
+        MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
+        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
+                                                       up8(in_features), ctx->sm_count, ctx->stream));
+        return tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, out_features, in_features, false), y, batch,
+                          out_features, in_features, scale, reinterpret_cast<float*>(w + o_k), splits);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_forward(x, state, scale, y, (int)batch, (int)in_features,
                                                          (int)out_features, (int)C, ctx->stream));
@@ -553,25 +559,22 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
         fused_wanted(ctx, nullptr, grad_out, state, scale, nullptr, grad_x, nullptr, in_features, out_features, batch))
         return fused_products(ctx, op, nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, C, in_features, out_features, batch);
     if (tc_wanted(ctx, batch, in_features, out_features)) {
-        const int ta = ctx->act_terms, ldo = up8(out_features);
         int splits = 1;
         const size_t sk = mcl::tc_splitk_workspace_bytes((int)batch, (int)in_features, (int)out_features,
                                                          ctx->sm_count, 0, &splits);
         Carver cv;
-        const size_t o_g = cv.reserve((size_t)ta * batch * ldo * 2), o_t = cv.reserve(in_features * (size_t)ldo * 2),
-                     o_k = cv.reserve(sk);
+        const size_t o_w = cv.reserve(kWordBytes);
+        const TermBuf gb = carve_terms(&cv, batch, out_features, false, true, o_w);
+        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2), o_k = cv.reserve(sk);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
-        MCL_LAUNCH(ctx, op, mcl::launch_split_planes(grad_out, (int)batch, (int)out_features, scale, w + o_g, ldo, ta,
-                                                     nullptr, 0, 0, ctx->stream));
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, (int)C, (int)out_features, (int)in_features,
-                                                       nullptr, 0, w + o_t, ldo, ctx->stream));
-        int pa[6], pb[6], nt;
-        act_term_list(ta, pa, pb, &nt);
-        return tc_product(ctx, w + o_g, ta, ldo, batch * (size_t)ldo, w + o_t, 1, ldo, in_features * (size_t)ldo,
-                          grad_x, (int)in_features, (int)batch, (int)in_features, (int)out_features, pa, pb, nt,
-                          nullptr, reinterpret_cast<float*>(w + o_k), splits);
+        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
+        MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, scale, false));
+        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
+                                                       up8(in_features), ctx->sm_count, ctx->stream));
+        return tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, out_features, in_features, true), grad_x, batch,
+                          in_features, out_features, nullptr, reinterpret_cast<float*>(w + o_k), splits);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_backward_input(state, scale, grad_out, grad_x, (int)batch,
                                                                 (int)in_features, (int)out_features,
@@ -642,17 +645,18 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     DeviceGuard guard(ctx->device);
     const size_t state_row = in_features / 4 * 3;
     const bool tc = tc_wanted(ctx, tile_rows, in_features, batch) && tile_rows >= 64;
-    int pa[6], pb[6], nt = 0, planes = 0, splits = 1;
-    const int ldn = up8(batch);
+    if (tc) tile_rows &= ~size_t(7);      // a tile starts at a 16-byte aligned column of the terms of grad_out
+    int splits = 1;
     Carver cv;
     const size_t o_gw = cv.reserve(tile_rows * row_b);
-    size_t o_a = 0, o_b = 0, o_k = 0;
+    size_t o_k = 0, o_w = 0;
+    TermBuf gb, xb;
     if (tc) {
-        grad_term_list(ctx->grad_terms, pa, pb, &nt, &planes);
         const size_t sk = mcl::tc_splitk_workspace_bytes((int)tile_rows, (int)in_features, (int)batch,
                                                          ctx->sm_count, mcl::kGradDepthLimit, &splits);
-        o_a = cv.reserve((size_t)planes * out_features * ldn * 2);   // dY^T term planes (activation-sized)
-        o_b = cv.reserve((size_t)planes * in_features * ldn * 2);    // X^T term planes
+        o_w = cv.reserve(kWordBytes);
+        gb = carve_terms(&cv, batch, out_features, true, false, o_w);      // activation-sized, not weight-sized
+        xb = carve_terms(&cv, batch, in_features, true, false, o_w + 8);
         o_k = cv.reserve(sk);
     }
     void* wsp = nullptr;
@@ -660,19 +664,18 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     char* w = static_cast<char*>(wsp);
     float* gw = reinterpret_cast<float*>(w + o_gw);
     if (tc) {
-        MCL_LAUNCH(ctx, op, mcl::launch_split_planes(grad_out, (int)batch, (int)out_features, nullptr, nullptr, 0, 0,
-                                                     w + o_a, ldn, planes, ctx->stream));
-        MCL_LAUNCH(ctx, op, mcl::launch_split_planes(x, (int)batch, (int)in_features, nullptr, nullptr, 0, 0,
-                                                     w + o_b, ldn, planes, ctx->stream));
+        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
+        MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, nullptr, true));
+        MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
     }
     for (size_t r0 = 0; r0 < out_features; r0 += tile_rows) {
         const size_t nr = (out_features - r0 < tile_rows) ? out_features - r0 : tile_rows;
         if (tc) {
-            int sp = splits;
-            MCL_TRY(tc_product(ctx, w + o_a + r0 * (size_t)ldn * 2, planes, ldn, out_features * (size_t)ldn,
-                               w + o_b, planes, ldn, in_features * (size_t)ldn, gw, (int)in_features, (int)nr,
-                               (int)in_features, (int)batch, pa, pb, nt, nullptr,
-                               reinterpret_cast<float*>(w + o_k), sp));
+            mcl::TcOperand a = terms_of(w, gb, false, true);
+            a.ptr = static_cast<const char*>(a.ptr) + r0 * 2;
+            a.cols = (int)nr;
+            MCL_TRY(tc_product(ctx, a, terms_of(w, xb, false, true), gw, nr, in_features, batch, nullptr,
+                               reinterpret_cast<float*>(w + o_k), splits));
         } else {
             MCL_LAUNCH(ctx, "counter update (grad_w tile)",
                        mcl::launch_simt_grad_w(grad_out, x, gw, (int)batch, (int)in_features,
@@ -782,10 +785,6 @@ static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, co
     }
     if (fused_wanted(ctx, x, grad_out, state ? static_cast<const void*>(state) : packed2, scale, y, grad_x, grad_w, I, O, Nt))
         return fused_products(ctx, op, x, grad_out, state, packed2, scale, y, grad_x, grad_w, C, I, O, Nt);
-    const int ta = ctx->act_terms;
-    int pa[6], pb[6], nt, gp;
-    grad_term_list(ctx->grad_terms, pa, pb, &nt, &gp);
-    const int ldi = up8(I), ldo = up8(O), ldn = up8(Nt);
     int s_y = 1, s_x = 1, s_w = 1;
     const size_t k_y = mcl::tc_splitk_workspace_bytes((int)Nt, (int)O, (int)I, ctx->sm_count, 0, &s_y);
     const size_t k_x = mcl::tc_splitk_workspace_bytes((int)Nt, (int)I, (int)O, ctx->sm_count, 0, &s_x);
@@ -793,36 +792,23 @@ static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, co
     size_t k_max = k_y > k_x ? k_y : k_x;
     if (k_w > k_max) k_max = k_w;
     Carver cv;
-    const size_t o_xp = cv.reserve((size_t)ta * Nt * ldi * 2);    // X terms        [ta][N][I]
-    const size_t o_xt = cv.reserve((size_t)gp * I * ldn * 2);     // X^T terms      [gp][I][N]
-    const size_t o_gp = cv.reserve((size_t)ta * Nt * ldo * 2);    // (dY.s) terms   [ta][N][O]
-    const size_t o_gt = cv.reserve((size_t)gp * O * ldn * 2);     // dY^T terms     [gp][O][N]
-    const size_t o_t = cv.reserve(O * (size_t)ldi * 2);           // T   [O][I]
-    const size_t o_tt = cv.reserve(I * (size_t)ldo * 2);          // T^T [I][O]
+    const size_t o_w = cv.reserve(kWordBytes);
+    const TermBuf xb = carve_terms(&cv, Nt, I, y || grad_w, false, o_w);
+    const TermBuf gb = carve_terms(&cv, Nt, O, grad_w != nullptr, grad_x != nullptr, o_w + 8);
+    const size_t o_t = cv.reserve(O * (size_t)up8(I) * 2);
     const size_t o_k = cv.reserve(k_max);
     void* wsp = nullptr;
     MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
     char* w = static_cast<char*>(wsp);
     float* kws = reinterpret_cast<float*>(w + o_k);
-    // each fp32 tensor is read once and written as terms in the orientations its products need
-    MCL_LAUNCH(ctx, op, mcl::launch_split_planes(x, (int)Nt, (int)I, nullptr, y ? w + o_xp : nullptr, ldi, ta,
-                                                 grad_w ? w + o_xt : nullptr, ldn, gp, ctx->stream));
-    if (state)
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, (int)C, (int)O, (int)I, y ? w + o_t : nullptr, ldi,
-                                                       grad_x ? w + o_tt : nullptr, ldo, ctx->stream));
-    else
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary_p2(packed2, (int)O, (int)I, y ? w + o_t : nullptr, ldi,
-                                                          grad_x ? w + o_tt : nullptr, ldo, ctx->stream));
-    MCL_LAUNCH(ctx, op, mcl::launch_split_planes(grad_out, (int)Nt, (int)O, scale, grad_x ? w + o_gp : nullptr, ldo, ta,
-                                                 grad_w ? w + o_gt : nullptr, ldn, gp, ctx->stream));
-    int qa[6], qb[6], qn;
-    act_term_list(ta, qa, qb, &qn);
-    if (y) MCL_TRY(tc_product(ctx, w + o_xp, ta, ldi, Nt * (size_t)ldi, w + o_t, 1, ldi, O * (size_t)ldi, y, (int)O,
-                              (int)Nt, (int)O, (int)I, qa, qb, qn, scale, kws, s_y));
-    if (grad_x) MCL_TRY(tc_product(ctx, w + o_gp, ta, ldo, Nt * (size_t)ldo, w + o_tt, 1, ldo, I * (size_t)ldo, grad_x,
-                                   (int)I, (int)Nt, (int)I, (int)O, qa, qb, qn, nullptr, kws, s_x));
-    if (grad_w) MCL_TRY(tc_product(ctx, w + o_gt, gp, ldn, O * (size_t)ldn, w + o_xt, gp, ldn, I * (size_t)ldn, grad_w,
-                                   (int)I, (int)O, (int)I, (int)Nt, pa, pb, nt, nullptr, kws, s_w));
+    MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
+    if (y || grad_w) MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
+    if (grad_x || grad_w) MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, grad_x ? scale : nullptr, grad_w != nullptr));
+    if (y || grad_x)
+        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, packed2, (int)C, (int)O, (int)I, w + o_t, up8(I), ctx->sm_count, ctx->stream));
+    if (y) MCL_TRY(tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, O, I, false), y, Nt, O, I, scale, kws, s_y));
+    if (grad_x) MCL_TRY(tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, O, I, true), grad_x, Nt, I, O, nullptr, kws, s_x));
+    if (grad_w) MCL_TRY(tc_product(ctx, terms_of(w, gb, false, true), terms_of(w, xb, false, true), grad_w, O, I, Nt, nullptr, kws, s_w));
     return MCL_CUDA_OK;
 }
 
@@ -1149,25 +1135,22 @@ int mcl_cuda_matmul_f32(mcl_cuda_ctx* ctx, const float* a, const float* b, float
     MCL_TRY(check_ptr(ctx, op, "c", c, 4));
     DeviceGuard guard(ctx->device);
     if (tc_wanted(ctx, M, N, K)) {
-        int pa[6], pb[6], nt, planes;
-        grad_term_list(ctx->grad_terms, pa, pb, &nt, &planes);
-        const int ldk = up8(K);
         int splits = 1;
         const size_t sk = mcl::tc_splitk_workspace_bytes((int)M, (int)N, (int)K, ctx->sm_count, mcl::kGradDepthLimit, &splits);
         Carver cv;
-        const size_t o_a = cv.reserve((size_t)planes * M * ldk * 2), o_b = cv.reserve((size_t)planes * N * ldk * 2),
-                     o_k = cv.reserve(sk);
+        const size_t o_w = cv.reserve(kWordBytes);
+        // a stored [M,K] or (trans_a) [K,M], b stored [K,N] or (trans_b) [N,K]: split as stored, read in the needed orientation
+        const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false, o_w);
+        const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false, o_w + 8);
+        const size_t o_k = cv.reserve(sk);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
-        // A logical [M,K]: stored [M,K] -> planes as is; stored [K,M] (trans_a) -> transposed planes
-        if (!trans_a) MCL_LAUNCH(ctx, op, mcl::launch_split_planes(a, (int)M, (int)K, nullptr, w + o_a, ldk, planes, nullptr, 0, 0, ctx->stream));
-        else MCL_LAUNCH(ctx, op, mcl::launch_split_planes(a, (int)K, (int)M, nullptr, nullptr, 0, 0, w + o_a, ldk, planes, ctx->stream));
-        // B logical [K,N], needed as [N,K]: stored [N,K] (trans_b) -> as is; stored [K,N] -> transposed planes
-        if (trans_b) MCL_LAUNCH(ctx, op, mcl::launch_split_planes(b, (int)N, (int)K, nullptr, w + o_b, ldk, planes, nullptr, 0, 0, ctx->stream));
-        else MCL_LAUNCH(ctx, op, mcl::launch_split_planes(b, (int)K, (int)N, nullptr, nullptr, 0, 0, w + o_b, ldk, planes, ctx->stream));
-        return tc_product(ctx, w + o_a, planes, ldk, M * (size_t)ldk, w + o_b, planes, ldk, N * (size_t)ldk, c, (int)N,
-                          (int)M, (int)N, (int)K, pa, pb, nt, nullptr, reinterpret_cast<float*>(w + o_k), splits);
+        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
+        MCL_TRY(fill_terms(ctx, op, w, ab, a, nullptr, true));
+        MCL_TRY(fill_terms(ctx, op, w, bb, b, nullptr, true));
+        return tc_product(ctx, terms_of(w, ab, false, trans_a != 0), terms_of(w, bb, false, trans_b == 0), c, M, N, K, nullptr,
+                          reinterpret_cast<float*>(w + o_k), splits);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_matmul_f32(a, b, c, (int)M, (int)K, (int)N, trans_a, trans_b, ctx->stream));
     return MCL_CUDA_OK;

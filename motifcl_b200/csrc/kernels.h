@@ -52,26 +52,30 @@ cudaError_t launch_simt_grad_w(const float* grad_out, const float* x, float* gra
                                int in_features, int out_features, int row0, int rows,
                                cudaStream_t stream);
 
-// tc_gemm.cu -- tcgen05 / TMEM / TMA contractions on bf16 term planes (see the file header)
+// tc_gemm.cu -- tcgen05 / TMEM / TMA contractions on fp16 term planes (see the file header)
 int tc_pick_bn(int N);
 size_t tc_splitk_workspace_bytes(int M, int N, int K, int sm_count, int depth_limit, int* splits_out);
-constexpr int kGradDepthLimit = 32;   // k-tiles per accumulator for fp32 x fp32 products (K = 2048)
-// C[M,N] (+= over terms) A_pa[M,K] . B_pb[N,K]^T ; planes are bf16 [P][rows][ld], plane stride in elements
-cudaError_t launch_tc_gemm(const void* a_planes, int a_nplanes, int lda, size_t a_plane_stride,
-                           const void* b_planes, int b_nplanes, int ldb, size_t b_plane_stride, float* c,
-                           int ldc, int M, int N, int K, const int* pa, const int* pb, int nterms,
-                           const float* col_scale, float* splitk_ws, int splits, int* err_word,
-                           size_t max_smem, int sm_count, cudaStream_t stream, int* launches);
-// fp32 [R,Cc] -> bf16 term planes [t][R][ld_n] of (src * col_scale) and/or transposed planes
-// [t][Cc][ld_t] of src
-cudaError_t launch_split_planes(const float* src, int R, int Cc, const float* col_scale, void* planes, int ld_n,
-                                int nterms, void* planes_t, int ld_t, int nterms_t, cudaStream_t stream);
-// packed 6-bit state -> bf16 ternary digits T [O][ld_i] and/or T^T [I][ld_o]
-cudaError_t launch_expand_ternary(const uint8_t* state, int C, int O, int I, void* T, int ld_i, void* Tt, int ld_o,
-                                  cudaStream_t stream);
-
-cudaError_t launch_expand_ternary_p2(const uint32_t* packed2, int O, int I, void* T, int ld_i, void* Tt, int ld_o,
-                                     cudaStream_t stream);
+// k-tiles of 64 per accumulator for fp32 x fp32 products: 3 x 4 instructions per k-tile add into it, each with a truncation
+// error of about 2.7e-9 relative (K = 4096: 2e-6)
+constexpr int kGradDepthLimit = 64;
+struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major tensor with `cols` columns
+    const void* ptr;
+    int rows, cols, ld;
+    int planes;                // 2: hi and lo terms of an fp32 tensor; 1: ternary digits
+    int mn_major;              // the contraction runs over the rows (0: over the columns)
+    const uint32_t* amax;      // bits of the split tensor's largest magnitude (null for digits)
+};
+// C[M,N] = sum over k of A B (b.planes == 1: two products, b.planes == 2: three)
+cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int ldc, int M, int N, int K,
+                           const float* col_scale, float* splitk_ws, int splits, int* err_word, size_t max_smem,
+                           int sm_count, cudaStream_t stream, int* launches);
+// fp32 [R,Cc] -> fp16 terms [2][R][ld] of src (planes) and / or of src . col_scale (planes_s); amax: two zeroed words that
+// receive the largest magnitudes of the two.  Two launches.
+cudaError_t launch_split_terms(const float* src, int R, int Cc, int ld, const float* col_scale, void* planes, void* planes_s,
+                               uint32_t* amax, int sm_count, cudaStream_t stream);
+// ternary digits as fp16 [O][ld], from the 6-bit state (state != null) or the 2-bit words (I % 16 == 0, ld == I)
+cudaError_t launch_expand_ternary(const uint8_t* state, const uint32_t* packed2, int C, int O, int I, void* T, int ld,
+                                  int sm_count, cudaStream_t stream);
 
 // tc_fused.cu -- grouped tcgen05 (tf32, two terms) contractions straight from fp32 tensors
 // kFusedYB / kFusedDXB are Y and dX with the activation split into two bf16 terms and the ternary digits given

@@ -3,32 +3,24 @@
 //
 // One kernel serves the three products of a training step (MotifCL
 // src/nn/compact_counter.cpp:233-300 and kernels/matmul.cl:413-563 compute them with fp32
-// scalar FMAs):
-//     Y  [tokens,out] = X  . T^T          A = planes of X  [tokens,in],   B = T   [out,in]
-//     dX [tokens,in ] = (dY.s) . T        A = planes of dY.s [tokens,out], B = T^T [in,out]
-//     dW [out,in]     = dY^T . X          A = planes of dY^T [out,tokens], B = planes of X^T [in,tokens]
-// Every operand is K-major bf16 ("NT" form), produced by the pre-pass kernels below:
-//   * an fp32 tensor is split into bf16 terms a = a1 + a2 (+ a3), a1 = bf16(a),
-//     a2 = bf16(a - a1), a3 = bf16(a - a1 - a2); products of terms are accumulated in fp32
-//     in TMEM, so fp32 activations keep (nearly) fp32 accuracy on bf16 tensor cores;
-//   * ternary weights {-1,0,1,(2)} are exact in bf16 and are expanded from the packed 6-bit
-//     state, in both orientations.
-// The kernel computes  C[M,N] = sum over a list of (plane of A, plane of B) pairs of
-// A_p[M,K] . B_q[N,K]^T, optionally scaled per column, or writes split-K partial sums that a
-// fixed-order reduction kernel adds up (deterministic).
+// scalar FMAs) and the dense fp32 matmul:
+//     Y  [tokens,out] = X  . T^T          A = terms of X    [tokens,in]     B = T [out,in]
+//     dX [tokens,in ] = (dY.s) . T        A = terms of dY.s [tokens,out]    B = T [out,in], read MN-major
+//     dW [out,in]     = dY^T . X          A = terms of dY, B = terms of X   both [tokens, .], read MN-major
+// so every tensor is split once, in its own layout, and T is expanded once: a transposed operand is the
+// same shared-memory tile with the MN-major bit of the instruction descriptor.
 //
-// Structure of the persistent CTA (192 threads; work items = 128 x BN output tile x split-K slice, dealt
-// round-robin; BN a multiple of 32 up to 256):
-//   warp 0 lane 0   TMA producer: cp.async.bulk.tensor (3-D tile {64 k, rows, plane}, 128-byte
-//                   swizzle) into a ring of `stages` shared-memory slots, mbarrier complete_tx
-//   warp 1 lane 0   MMA issuer: four tcgen05.mma (K = 16 each) per slot, tcgen05.commit to
-//                   release the slot, final commit to signal the accumulator; warp 1 owns TMEM
-//   warps 2..5      epilogue: tcgen05.ld 32 lanes x 32 columns, scale, 128-bit stores
-// Two accumulators in TMEM let the epilogue of one item overlap the main loop of the next.
-// Every mbarrier wait is bounded: on time-out the kernel records an error word, skips the
-// rest of its work, frees its TMEM and returns.
+// How an fp32 tensor becomes two fp16 terms (split_terms_kernel): with m = the largest magnitude of the tensor and
+// f = 2^(14 - floor(log2 m)), hi = fp16(a f) and lo = fp16((a f - hi) 2^12).  hi keeps 11 bits, the residual is at most
+// half a unit of hi and keeps 11 more below its sign: |a f - hi - lo 2^-12| <= 2^-23 |a f|, the last bit of fp32 (the first
+// bf16 form of this file needed three 8-bit terms for the same bits).  lo is stored 2^12 up so that it stays a normal
+// number wherever hi is: elements down to 2^-28 of the largest keep all their bits, smaller ones are off by less
+// than 2^-50 of it.  The lo products go into the accumulator first; the first hi product scales it down by 2^-12
+// (tcgen05.mma scale-input-d), and the epilogue undoes f.  Ternary digits are exact in fp16.  Cost per product of a
+// step in bf16-rate passes: Y, dX 2 (3 before), dW 3 (hi.hi + hi.lo + lo.hi; 6 before).
+// The kernel is bound by the tensor pipe; its time at a stated size stands at tc_gemm_kernel.
 #include <cuda.h>
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "counter_codec.cuh"
 #include "kernels.h"
@@ -38,25 +30,68 @@ namespace mcl {
 namespace {
 
 constexpr int BM = 128;          // UMMA M
-constexpr int BK = 64;           // 64 bf16 = 128 bytes = one swizzle row
+constexpr int BK = 64;           // 64 fp16 = 128 bytes = one swizzle row
 constexpr int kMaxStages = 8;
 constexpr int kATileBytes = BM * BK * 2;   // 16 KiB
+constexpr int kLoShift = 12;               // lo terms are stored 2^12 up
 
 struct TcParams {
     float* C;                 // output [M, ldc] (or split-K partials [splits][M][ldc])
     const float* col_scale;   // optional, applied when splits == 1
+    const uint32_t* a_amax;   // bits of the largest magnitude of the split tensor (null: operand is unscaled)
+    const uint32_t* b_amax;
     int M, N, K, ldc;
-    int BN, stages;
-    int nterms;
-    int pa[6], pb[6];
+    int BN, stages, b_bytes;
+    int a_mn, b_mn;           // operand is stored with M / N contiguous
+    int nterms;               // 2: A lo, A hi against one B plane; 3: lo.hi, hi.lo, hi.hi
     int ktiles_per_split, splits;
+    int group_m;
     int* err;
 };
 
-// Instruction descriptor, kind::f16: D = f32 (bits 4-5 = 1), A = B = bf16 (bits 7-9, 10-12 = 1),
-// both K-major (bits 15, 16 = 0), N >> 3 at bit 17, M >> 4 at bit 24.
-__device__ __forceinline__ uint32_t idesc_bf16(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// exponent of f (see the file header): the largest magnitude lands in [2^14, 2^15)
+__device__ __forceinline__ int term_exp(uint32_t amax_bits) {
+    const int e = (int)(amax_bits >> 23);
+    const int s = 141 - (e < 1 ? 1 : e);
+    return s > 126 ? 126 : s;
+}
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// Instruction descriptor, kind::f16: D = f32 (bits 4-5 = 1), A = B = f16 (bits 7-9, 10-12 = 0), A / B MN-major at bits
+// 15 / 16, N >> 3 at bit 17, M >> 4 at bit 24.
+__device__ __forceinline__ uint32_t idesc_f16(int m, int n, int a_mn, int b_mn) {
+    return (1u << 4) | ((uint32_t)a_mn << 15) | ((uint32_t)b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+// MN-major 16-bit tile in the 128-byte swizzle: chunks of 64 MN elements x 64 k rows of 128 bytes; leading byte offset =
+// 8192 (next chunk), stride byte offset = 1024 (next 8 k rows).
+__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// D = A.B + D 2^-12
+__device__ __forceinline__ void umma_f16_down12(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, 1, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 12;\n\t}"
+        ::"r"(tmem_c), "l"(da), "l"(db), "r"(idesc) : "memory");
+}
+
+// item -> output tile and K slice.  Groups of group_m row tiles run through all column tiles before the next group, so
+// that the CTAs in flight share both operands' tiles in L2.
+struct TcItem { int mt, nt, split; };
+__device__ __forceinline__ TcItem tc_item(int item, int tiles_m, int tiles_n, int group_m) {
+    TcItem t;
+    const int per_split = tiles_m * tiles_n;
+    t.split = item / per_split;
+    int r = item - t.split * per_split;
+    const int per_group = group_m * tiles_n;
+    const int g = r / per_group;
+    r -= g * per_group;
+    const int gm = min(group_m, tiles_m - g * group_m);
+    t.nt = r / gm;
+    t.mt = g * group_m + (r - t.nt * gm);
+    return t;
 }
 
 // Persistent CTA of 192 threads; work items (output tile x split-K slice) are dealt round-robin.
@@ -78,7 +113,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int BN = p.BN, S = p.stages;
     const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t stage_bytes = kATileBytes + (uint32_t)BN * BK * 2;
+    const uint32_t stage_bytes = kATileBytes + (uint32_t)p.b_bytes;
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
@@ -91,7 +126,6 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + BM - 1) / BM;
     const int ktiles = (p.K + BK - 1) / BK;
     const int n_items = tiles_m * tiles_n * p.splits;
-    // item -> (m tile fastest, then n tile, then split): CTAs running together share a B tile
 
     if (threadIdx.x == 0) {
         abort_flag = (*reinterpret_cast<volatile int*>(p.err) != 0);   // an earlier CTA gave up: do not wait at all
@@ -114,20 +148,32 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             // ---- TMA producer --------------------------------------------------------------
             uint32_t it = 0;       // slot counter across all items of this CTA
             for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x) {
-                const int mt = item % tiles_m, rest = item / tiles_m;
-                const int nt = rest % tiles_n, split = rest / tiles_n;
-                const int kt0 = split * p.ktiles_per_split;
+                const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
+                const int kt0 = t.split * p.ktiles_per_split;
                 const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
                 for (int term = 0; term < p.nterms; ++term) {
-                    const int pa = p.pa[term], pb = p.pb[term];
+                    // planes: 0 = hi, 1 = lo; products with a lo term first
+                    const int pa = p.nterms == 3 ? (term == 0) : (term + 1 < p.nterms);
+                    const int pb = p.nterms == 3 && term == 1;
                     for (int kk = 0; kk < my_kt; ++kk, ++it) {
                         const int s = (int)(it % (uint32_t)S);
                         const uint32_t ph = (it / (uint32_t)S) & 1u;
                         if (!mbar_wait(empty_bar(s), ph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 1); break; }
                         const uint32_t a_dst = tiles + (uint32_t)s * stage_bytes;
                         mbar_expect_tx(full_bar(s), stage_bytes);
-                        tma_load_3d(a_dst, &tmA, full_bar(s), (kt0 + kk) * BK, mt * BM, pa);
-                        tma_load_3d(a_dst + kATileBytes, &tmB, full_bar(s), (kt0 + kk) * BK, nt * BN, pb);
+                        const int k0 = (kt0 + kk) * BK;
+                        if (p.a_mn) {
+                            tma_load_3d(a_dst, &tmA, full_bar(s), t.mt * BM, k0, pa);
+                            tma_load_3d(a_dst + 8192, &tmA, full_bar(s), t.mt * BM + 64, k0, pa);
+                        } else {
+                            tma_load_3d(a_dst, &tmA, full_bar(s), k0, t.mt * BM, pa);
+                        }
+                        if (p.b_mn) {
+                            for (int c = 0; c < BN; c += 64)
+                                tma_load_3d(a_dst + kATileBytes + (uint32_t)c * 128u, &tmB, full_bar(s), t.nt * BN + c, k0, pb);
+                        } else {
+                            tma_load_3d(a_dst + kATileBytes, &tmB, full_bar(s), k0, t.nt * BN, pb);
+                        }
                     }
                     if (abort_flag) break;
                 }
@@ -136,13 +182,13 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     } else if (warp == 1) {
         if (lane == 0) {
             // ---- MMA issuer ----------------------------------------------------------------
-            const uint32_t idesc = idesc_bf16(BM, BN);
+            const uint32_t idesc = idesc_f16(BM, BN, p.a_mn, p.b_mn);
+            const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;   // 16 k further, in 16-byte units
             uint32_t it = 0, n_local = 0;
             for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x, ++n_local) {
-                const int split = item / (tiles_m * tiles_n);
-                const int kt0 = split * p.ktiles_per_split;
+                const int kt0 = (item / (tiles_m * tiles_n)) * p.ktiles_per_split;
                 const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
-                const int total = p.nterms * my_kt;
+                const int total = p.nterms * my_kt, first_hi = total - my_kt;
                 const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
                 if (!mbar_wait(acc_empty(acc), aph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 4); break; }
                 tc_fence_after();
@@ -153,10 +199,16 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                     if (!mbar_wait(full_bar(s), ph, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 2); break; }
                     tc_fence_after();
                     const uint32_t a_addr = tiles + (uint32_t)s * stage_bytes;
-                    const uint64_t da = smem_desc_k_sw128(a_addr), db = smem_desc_k_sw128(a_addr + kATileBytes);
+                    const uint32_t b_addr = a_addr + kATileBytes;
+                    const uint64_t da = p.a_mn ? smem_desc_mn_sw128(a_addr) : smem_desc_k_sw128(a_addr);
+                    const uint64_t db = p.b_mn ? smem_desc_mn_sw128(b_addr) : smem_desc_k_sw128(b_addr);
 #pragma unroll
-                    for (int kk = 0; kk < BK / 16; ++kk)   // 16 bf16 = 32 bytes = +2 in the address field
-                        umma_bf16(d_tmem, da + 2u * kk, db + 2u * kk, idesc, (j | kk) != 0 ? 1u : 0u);
+                    for (int kk = 0; kk < BK / 16; ++kk) {
+                        if (kk == 0 && j == first_hi && p.nterms > 1)
+                            umma_f16_down12(d_tmem, da, db, idesc);
+                        else
+                            umma_bf16(d_tmem, da + (uint64_t)(a_step * kk), db + (uint64_t)(b_step * kk), idesc, (j | kk) != 0 ? 1u : 0u);
+                    }
                     umma_commit(empty_bar(s));
                 }
                 if (abort_flag) break;
@@ -167,10 +219,12 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         // ---- epilogue warps: TMEM -> registers -> global ---------------------------------------
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const bool scale = (p.col_scale != nullptr) && p.splits == 1;
+        const float fa = p.a_amax ? pow2(-term_exp(__ldg(p.a_amax))) : 1.0f;      // undo the powers of two of the split
+        const float fb = p.b_amax ? pow2(-term_exp(__ldg(p.b_amax))) : 1.0f;
         uint32_t n_local = 0;
         for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n_local) {
-            const int mt = item % tiles_m, rest = item / tiles_m;
-            const int nt = rest % tiles_n, split = rest / tiles_n;
+            const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
+            const int mt = t.mt, nt = t.nt, split = t.split;
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
             bool ok = !abort_flag;
             if (ok && !mbar_wait(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 3); ok = false; }
@@ -192,6 +246,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                         if (col >= p.N) break;
                         float4 o = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
                                                __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+                        o.x = o.x * fa * fb; o.y = o.y * fa * fb; o.z = o.z * fa * fb; o.w = o.w * fa * fb;
                         if (scale) {
                             const float4 sc = __ldg(reinterpret_cast<const float4*>(p.col_scale + col));
                             o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
@@ -236,173 +291,153 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, float* _
     }
 }
 
-// ---- pre-pass: fp32 -> bf16 term planes (optionally column-scaled, optionally transposed) ----
-// src [R, Cc] fp32.  Writes, for t < nterms:
-//   planes   [t][R ][ld_n]  = term t of (src * col_scale), t < nterms    (when planes   != null)
-//   planes_t [t][Cc][ld_t]  = term t of  src (unscaled), transposed, t < nterms_t (when planes_t != null)
-// 64 x 64 tiles through shared memory so that both outputs are written with coalesced rows.
-__device__ __forceinline__ void split3(float v, __nv_bfloat16 (&h)[3]) {
-    h[0] = __float2bfloat16_rn(v);
-    const float r1 = v - __bfloat162float(h[0]);
-    h[1] = __float2bfloat16_rn(r1);
-    const float r2 = r1 - __bfloat162float(h[1]);
-    h[2] = __float2bfloat16_rn(r2);
-}
-
-__global__ void __launch_bounds__(256) split_planes_kernel(const float* __restrict__ src, int R, int Cc,
-                                                           const float* __restrict__ col_scale,
-                                                           __nv_bfloat16* __restrict__ planes, int ld_n,
-                                                           __nv_bfloat16* __restrict__ planes_t, int ld_t,
-                                                           int nterms, int nterms_t) {
-    __shared__ float tile[64][65];
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;    // 64 x 4
-    for (int rr = ty; rr < 64; rr += 4) {
-        const int r = r0 + rr, c = c0 + tx;
-        float v = 0.0f;
-        if (r < R && c < Cc) v = __ldg(src + (size_t)r * Cc + c);
-        tile[rr][tx] = v;
-        if (planes != nullptr && r < R && c < Cc) {
-            const float sv = col_scale ? __fmul_rn(v, __ldg(col_scale + c)) : v;
-            __nv_bfloat16 h[3];
-            split3(sv, h);
-            for (int t = 0; t < nterms; ++t) planes[((size_t)t * R + r) * ld_n + c] = h[t];
-        }
-    }
-    if (planes_t == nullptr) return;
-    __syncthreads();
-    for (int cc = ty; cc < 64; cc += 4) {
-        const int c = c0 + cc, r = r0 + tx;
-        if (c < Cc && r < R) {
-            __nv_bfloat16 h[3];
-            split3(tile[tx][cc], h);
-            for (int t = 0; t < nterms_t; ++t) planes_t[((size_t)t * Cc + c) * ld_t + r] = h[t];
-        }
-    }
-}
-
-// Vectorised form of the same pre-pass for Cc % 4 == 0, R % 4 == 0 and 16-byte aligned src:
-// 128-bit loads, 64-bit stores of four bf16 in both orientations.
-__device__ __forceinline__ uint2 pack4(const __nv_bfloat16 a, const __nv_bfloat16 b, const __nv_bfloat16 c,
-                                       const __nv_bfloat16 d) {
-    uint2 o;
-    o.x = (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
-    o.y = (uint32_t)__bfloat16_as_ushort(c) | ((uint32_t)__bfloat16_as_ushort(d) << 16);
-    return o;
-}
-
-__global__ void __launch_bounds__(256) split_planes_vec_kernel(const float* __restrict__ src, int R, int Cc,
-                                                               const float* __restrict__ col_scale,
-                                                               __nv_bfloat16* __restrict__ planes, int ld_n,
-                                                               __nv_bfloat16* __restrict__ planes_t, int ld_t,
-                                                               int nterms, int nterms_t) {
-    __shared__ float tile[64][65];
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;    // 16 column quads x 16 rows
-    const int c = c0 + tx * 4;
-    float4 sc4 = make_float4(1.f, 1.f, 1.f, 1.f);
-    if (col_scale != nullptr && c < Cc) sc4 = __ldg(reinterpret_cast<const float4*>(col_scale + c));
-#pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-        const int rr = pass * 16 + ty, r = r0 + rr;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < R && c < Cc) v = __ldg(reinterpret_cast<const float4*>(src + (size_t)r * Cc + c));
-        tile[rr][tx * 4 + 0] = v.x; tile[rr][tx * 4 + 1] = v.y; tile[rr][tx * 4 + 2] = v.z; tile[rr][tx * 4 + 3] = v.w;
-        if (planes != nullptr && r < R && c < Cc) {
-            if (col_scale != nullptr) {
-                v.x = __fmul_rn(v.x, sc4.x); v.y = __fmul_rn(v.y, sc4.y);
-                v.z = __fmul_rn(v.z, sc4.z); v.w = __fmul_rn(v.w, sc4.w);
+// ---- pre-pass 1: largest magnitude of a tensor, and of the tensor times a per-column factor ----------------
+// amax[0] = max |src|, amax[1] = max |src . col_scale| (when col_scale != null), as float bits, by atomicMax into zeroed
+// words.  HBM-bound: one read.
+template <bool VEC>
+__global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ src, size_t R, int Cc,
+                                                   const float* __restrict__ col_scale, uint32_t* __restrict__ amax) {
+    constexpr int W = VEC ? 4 : 1;
+    const int n = Cc / W;                                   // VEC needs Cc % 4 == 0
+    const size_t total = R * (size_t)n, stride = (size_t)gridDim.x * 256;
+    const size_t i0 = (size_t)blockIdx.x * 256 + threadIdx.x;
+    int c = (int)(i0 % (size_t)n);
+    const int step = (int)(stride % (size_t)n);
+    float m0 = 0.0f, m1 = 0.0f;
+#pragma unroll 4
+    for (size_t i = i0; i < total; i += stride) {
+        if (VEC) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(src) + i);
+            m0 = fmaxf(fmaxf(m0, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+            if (col_scale) {
+                const float4 s = __ldg(reinterpret_cast<const float4*>(col_scale) + c);
+                m1 = fmaxf(fmaxf(m1, fmaxf(fabsf(v.x * s.x), fabsf(v.y * s.y))), fmaxf(fabsf(v.z * s.z), fabsf(v.w * s.w)));
             }
-            __nv_bfloat16 h0[3], h1[3], h2[3], h3[3];
-            split3(v.x, h0); split3(v.y, h1); split3(v.z, h2); split3(v.w, h3);
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-                if (t < nterms)
-                    *reinterpret_cast<uint2*>(planes + ((size_t)t * R + r) * ld_n + c) = pack4(h0[t], h1[t], h2[t], h3[t]);
+        } else {
+            const float v = __ldg(src + i);
+            m0 = fmaxf(m0, fabsf(v));
+            if (col_scale) m1 = fmaxf(m1, fabsf(v * __ldg(col_scale + c)));
         }
+        c += step;
+        if (c >= n) c -= n;
     }
-    if (planes_t == nullptr) return;
+    uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
+    __shared__ uint32_t w0[8], w1[8];
+    if ((threadIdx.x & 31) == 0) { w0[threadIdx.x >> 5] = b0; w1[threadIdx.x >> 5] = b1; }
     __syncthreads();
-    // transposed: thread owns 4 consecutive source rows (= 4 consecutive output columns) of one source column
-    const int rq = threadIdx.x & 15, cl = threadIdx.x >> 4;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) { b0 = max(b0, w0[w]); b1 = max(b1, w1[w]); }
+        if (b0) atomicMax(amax, b0);
+        if (col_scale && b1) atomicMax(amax + 1, b1);
+    }
+}
+
+// ---- pre-pass 2: fp32 [R, Cc] -> fp16 terms [2][R][ld] of src (planes) and of src . col_scale (planes_s) ----------
+// Thread = 8 consecutive columns: two 128-bit loads, one 128-bit store per term.  HBM-bound: 4 bytes read, 4 written per
+// element and output.
+__device__ __forceinline__ void split_terms8(const float (&v)[8], float f, uint4* hi, uint4* lo) {
+    uint32_t h[4], l[4];
 #pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-        const int cc = pass * 16 + cl, cg = c0 + cc, r = r0 + rq * 4;
-        if (cg < Cc && r < R) {
-            __nv_bfloat16 h0[3], h1[3], h2[3], h3[3];
-            split3(tile[rq * 4 + 0][cc], h0); split3(tile[rq * 4 + 1][cc], h1);
-            split3(tile[rq * 4 + 2][cc], h2); split3(tile[rq * 4 + 3][cc], h3);
+    for (int k = 0; k < 4; ++k) {
+        const float a = v[2 * k] * f, b = v[2 * k + 1] * f;
+        const __half2 hh = __floats2half2_rn(a, b);
+        const float2 back = __half22float2(hh);
+        const __half2 ll = __floats2half2_rn((a - back.x) * (float)(1 << kLoShift), (b - back.y) * (float)(1 << kLoShift));
+        h[k] = *reinterpret_cast<const uint32_t*>(&hh);
+        l[k] = *reinterpret_cast<const uint32_t*>(&ll);
+    }
+    *hi = make_uint4(h[0], h[1], h[2], h[3]);
+    *lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+template <bool VEC>
+__global__ void __launch_bounds__(256) split_terms_kernel(const float* __restrict__ src, int R, int Cc, int ld,
+                                                          const float* __restrict__ col_scale, __half* __restrict__ planes,
+                                                          __half* __restrict__ planes_s, const uint32_t* __restrict__ amax) {
+    const int n8 = (Cc + 7) >> 3;
+    const float f0 = planes ? pow2(term_exp(__ldg(amax))) : 0.0f, f1 = planes_s ? pow2(term_exp(__ldg(amax + 1))) : 0.0f;
+    const size_t total = (size_t)R * n8, stride = (size_t)gridDim.x * 256, ps = (size_t)R * ld;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += stride) {
+        const size_t r = i / (size_t)n8;
+        const int c = (int)(i - r * n8) * 8;
+        const float* s = src + r * Cc + c;
+        float v[8];
+        if (VEC && c + 8 <= Cc) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(s)), b = __ldg(reinterpret_cast<const float4*>(s) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
 #pragma unroll
-            for (int t = 0; t < 3; ++t)
-                if (t < nterms_t)
-                    *reinterpret_cast<uint2*>(planes_t + ((size_t)t * Cc + cg) * ld_t + r) = pack4(h0[t], h1[t], h2[t], h3[t]);
+            for (int k = 0; k < 8; ++k) v[k] = c + k < Cc ? __ldg(s + k) : 0.0f;
+        }
+        uint4 hi, lo;
+        const size_t at = r * ld + c;                       // ld % 8 == 0
+        if (planes) {
+            split_terms8(v, f0, &hi, &lo);
+            *reinterpret_cast<uint4*>(planes + at) = hi;
+            *reinterpret_cast<uint4*>(planes + ps + at) = lo;
+        }
+        if (planes_s) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], c + k < Cc ? __ldg(col_scale + c + k) : 0.0f);
+            split_terms8(v, f1, &hi, &lo);
+            *reinterpret_cast<uint4*>(planes_s + at) = hi;
+            *reinterpret_cast<uint4*>(planes_s + ps + at) = lo;
         }
     }
 }
 
-// ---- pre-pass: packed 6-bit state -> bf16 ternary digits, both orientations ------------------
-//   T  [O][ld_i] (when T  != null),  Tt [I][ld_o] (when Tt != null)
-__global__ void __launch_bounds__(256) expand_ternary_kernel(const uint8_t* __restrict__ state, int C,
-                                                             int O, int I, __nv_bfloat16* __restrict__ T,
-                                                             int ld_i, __nv_bfloat16* __restrict__ Tt, int ld_o) {
-    __shared__ DecodeLut lut;
-    __shared__ __nv_bfloat16 tile[64][66];
-    build_decode_lut(&lut, C, threadIdx.x, blockDim.x);
+// ---- pre-pass 3: packed 6-bit state -> fp16 ternary digits T [O][ld] --------------------------------------------
+// VEC (in_features % 16 == 0, 4-byte aligned rows): thread = 16 weights = three words in, 32 bytes out, two codes per
+// look-up in a 4096-entry table.  16 KB per table and CTA; a 14336 x 4096 layer took 101 us with the transposing
+// byte-wise form, HBM needs 25.
+__device__ __forceinline__ uint32_t digit_pair(uint32_t two_codes, int lv) {
+    const __half2 h = __floats2half2_rn((float)((int)(two_codes & 63u) / lv - 1), (float)((int)(two_codes >> 6) / lv - 1));
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+template <bool VEC>
+__global__ void __launch_bounds__(256) expand_ternary_kernel(const uint8_t* __restrict__ state, int C, int O, int I,
+                                                             __half* __restrict__ T, int ld) {
+    __shared__ uint32_t lut[4096];
+    for (int e = threadIdx.x; e < 4096; e += 256) lut[e] = digit_pair((uint32_t)e, 2 * C - 1);
     __syncthreads();
-    const int o0 = blockIdx.y * 64, i0 = blockIdx.x * 64;
-    const int gpr = I >> 2;
-    // 64 rows x 16 groups per tile; thread handles one group (4 weights) at a time
-    for (int e = threadIdx.x; e < 64 * 16; e += 256) {
-        const int oo = e >> 4, g = (i0 >> 2) + (e & 15);
-        const int o = o0 + oo;
-        if (o < O && g < gpr) {
-            const uint8_t* s = state + ((size_t)o * gpr + g) * 3;
-            const uint32_t w = (uint32_t)__ldg(s) | ((uint32_t)__ldg(s + 1) << 8) | ((uint32_t)__ldg(s + 2) << 16);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat16 t = __float2bfloat16_rn(lut.e[(w >> (6 * k)) & 63u].x);
-                tile[oo][(e & 15) * 4 + k] = t;
-                if (T != nullptr) T[(size_t)o * ld_i + g * 4 + k] = t;
-            }
+    if (VEC) {
+        const size_t total = (size_t)O * (I >> 4);
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(state);
+        for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {   // ld == I here
+            const uint32_t a = __ldg(w + 3 * i), b = __ldg(w + 3 * i + 1), c = __ldg(w + 3 * i + 2);
+            const uint32_t g0 = a & 0xFFFFFFu, g1 = (a >> 24) | (b << 8), g2 = (b >> 16) | (c << 16), g3 = c >> 8;
+            uint4* o = reinterpret_cast<uint4*>(T + 16 * i);
+            o[0] = make_uint4(lut[g0 & 4095u], lut[g0 >> 12], lut[g1 & 4095u], lut[(g1 >> 12) & 4095u]);
+            o[1] = make_uint4(lut[g2 & 4095u], lut[(g2 >> 12) & 4095u], lut[g3 & 4095u], lut[g3 >> 12]);
         }
-    }
-    if (Tt == nullptr) return;
-    __syncthreads();
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-    for (int ii = ty; ii < 64; ii += 4) {
-        const int i = i0 + ii, o = o0 + tx;
-        if (i < I && o < O) Tt[(size_t)i * ld_o + o] = tile[tx][ii];
+    } else {
+        const int gpr = I >> 2;
+        const size_t total = (size_t)O * gpr;
+        for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
+            const uint8_t* s = state + i * 3;
+            const uint32_t g = (uint32_t)__ldg(s) | ((uint32_t)__ldg(s + 1) << 8) | ((uint32_t)__ldg(s + 2) << 16);
+            const size_t o = i / (size_t)gpr;
+            *reinterpret_cast<uint2*>(T + o * ld + (i - o * gpr) * 4) = make_uint2(lut[g & 4095u], lut[g >> 12]);
+        }
     }
 }
 
 // Same expansion from the 2-bit packed weights (field = t + 1, 16 per word): what ranks that do
 // not own a layer's counter state use after the all-gather of packed weights.
-__global__ void __launch_bounds__(256) expand_ternary_p2_kernel(const uint32_t* __restrict__ packed2, int O, int I,
-                                                                __nv_bfloat16* __restrict__ T, int ld_i,
-                                                                __nv_bfloat16* __restrict__ Tt, int ld_o) {
-    __shared__ __nv_bfloat16 tile[64][66];
-    const int o0 = blockIdx.y * 64, i0 = blockIdx.x * 64;
-    const int wpr = I >> 4;
-    // 64 rows x 4 words per tile; thread handles one word (16 weights)
-    {
-        const int oo = threadIdx.x >> 2, wq = threadIdx.x & 3;
-        const int o = o0 + oo, wi = (i0 >> 4) + wq;
-        if (o < O && wi < wpr) {
-            const uint32_t word = __ldg(packed2 + (size_t)o * wpr + wi);
+__global__ void __launch_bounds__(256) expand_ternary_p2_kernel(const uint32_t* __restrict__ packed2, size_t words,
+                                                                __half* __restrict__ T) {
+    const __half2 off = __floats2half2_rn(1025.0f, 1025.0f);
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) {
+        const uint32_t w = __ldg(packed2 + i);
+        uint32_t h[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const __nv_bfloat16 t = __float2bfloat16_rn((float)((int)((word >> (2 * k)) & 3u) - 1));
-                tile[oo][wq * 16 + k] = t;
-                if (T != nullptr) T[(size_t)o * ld_i + wi * 16 + k] = t;
-            }
+        for (int j = 0; j < 8; ++j) {      // fp16 1024 + field in both halves, minus 1025
+            const uint32_t two = 0x64006400u | ((w >> (4 * j)) & 3u) | (((w >> (4 * j + 2)) & 3u) << 16);
+            const __half2 t = __hsub2(*reinterpret_cast<const __half2*>(&two), off);
+            h[j] = *reinterpret_cast<const uint32_t*>(&t);
         }
-    }
-    if (Tt == nullptr) return;
-    __syncthreads();
-    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
-    for (int ii = ty; ii < 64; ii += 4) {
-        const int i = i0 + ii, o = o0 + tx;
-        if (i < I && o < O) Tt[(size_t)i * ld_o + o] = tile[tx][ii];
+        uint4* o = reinterpret_cast<uint4*>(T + 16 * i);       // in_features % 16 == 0, so rows follow one another
+        o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+        o[1] = make_uint4(h[4], h[5], h[6], h[7]);
     }
 }
 
@@ -423,17 +458,17 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// 3-D map over bf16 planes [P][rows][ld]: dims {K, rows, P}, box {64, box_rows, 1}, 128-byte swizzle.
-// Reads beyond K or rows return zeros, so ragged edges need no padding in memory.
-bool make_map(CUtensorMap* map, const void* base, int K, int rows, int planes, int ld, size_t plane_stride,
-              int box_rows) {
+// 3-D map over fp16 planes [P][rows][ld] with `cols` used columns: dims {cols, rows, P}, 128-byte swizzle; box
+// {64, box_rows, 1} for a K-major operand, {64, 64, 1} for an MN-major one (one chunk of 64 columns, 64 k rows).
+// Reads beyond cols or rows return zeros, so ragged edges need no padding in memory.
+bool make_map(CUtensorMap* map, const TcOperand& o, int box_rows) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
-    cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)planes};
-    cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)plane_stride * 2};
+    cuuint64_t dims[3] = {(cuuint64_t)o.cols, (cuuint64_t)o.rows, (cuuint64_t)o.planes};
+    cuuint64_t strides[2] = {(cuuint64_t)o.ld * 2, (cuuint64_t)o.rows * o.ld * 2};
     cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(o.ptr), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -474,21 +509,23 @@ size_t tc_splitk_workspace_bytes(int M, int N, int K, int sm_count, int depth_li
     return splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
 }
 
-cudaError_t launch_tc_gemm(const void* a_planes, int a_nplanes, int lda, size_t a_plane_stride,
-                           const void* b_planes, int b_nplanes, int ldb, size_t b_plane_stride, float* c,
-                           int ldc, int M, int N, int K, const int* pa, const int* pb,
-                           int nterms, const float* col_scale, float* splitk_ws, int splits, int* err_word,
-                           size_t max_smem, int sm_count, cudaStream_t stream, int* launches) {
-    if (nterms < 1 || nterms > 6 || (N & 3) || (ldc & 3) || (lda & 7) || (ldb & 7)) return cudaErrorInvalidValue;
-    const int bn = tc_pick_bn(N);
+cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int ldc, int M, int N, int K,
+                           const float* col_scale, float* splitk_ws, int splits, int* err_word, size_t max_smem,
+                           int sm_count, cudaStream_t stream, int* launches) {
+    if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (N & 3) || (ldc & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
+    const int bn = tc_pick_bn(N), nterms = b.planes == 2 ? 3 : 2;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, a_planes, K, M, a_nplanes, lda, a_plane_stride, BM)) return cudaErrorInvalidValue;
-    if (!make_map(&mb, b_planes, K, N, b_nplanes, ldb, b_plane_stride, bn)) return cudaErrorInvalidValue;
+    if (!make_map(&ma, a, a.mn_major ? BK : BM)) return cudaErrorInvalidValue;
+    if (!make_map(&mb, b, b.mn_major ? BK : bn)) return cudaErrorInvalidValue;
     TcParams p;
     p.col_scale = col_scale;
     p.M = M; p.N = N; p.K = K;
     p.BN = bn;
-    const size_t stage_bytes = (size_t)kATileBytes + (size_t)bn * BK * 2;
+    p.a_mn = a.mn_major; p.b_mn = b.mn_major;
+    p.a_amax = a.amax; p.b_amax = b.amax;
+    p.b_bytes = (b.mn_major ? (bn + 63) / 64 * 64 : bn) * BK * 2;
+    p.group_m = 12;               // 12 row tiles x 12 column tiles in flight on 148 SMs
+    const size_t stage_bytes = (size_t)kATileBytes + (size_t)p.b_bytes;
     const int ktiles = (K + BK - 1) / BK;
     int stages = (int)((max_smem - 2048) / stage_bytes);
     if (stages > kMaxStages) stages = kMaxStages;
@@ -507,7 +544,6 @@ cudaError_t launch_tc_gemm(const void* a_planes, int a_nplanes, int lda, size_t 
     if (stages < 2) return cudaErrorInvalidConfiguration;
     p.stages = stages;
     p.nterms = nterms;
-    for (int t = 0; t < 6; ++t) { p.pa[t] = t < nterms ? pa[t] : 0; p.pb[t] = t < nterms ? pb[t] : 0; }
     p.splits = splits;
     p.ktiles_per_split = (ktiles + splits - 1) / splits;
     // drop empty trailing splits
@@ -585,34 +621,39 @@ cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* co
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_planes(const float* src, int R, int Cc, const float* col_scale, void* planes, int ld_n,
-                                int nterms, void* planes_t, int ld_t, int nterms_t, cudaStream_t stream) {
-    dim3 grid((Cc + 63) / 64, (R + 63) / 64);
-    if ((Cc & 3) == 0 && (R & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
-        (col_scale == nullptr || (reinterpret_cast<uintptr_t>(col_scale) & 15) == 0)) {
-        split_planes_vec_kernel<<<grid, 256, 0, stream>>>(src, R, Cc, col_scale, static_cast<__nv_bfloat16*>(planes),
-                                                          ld_n, static_cast<__nv_bfloat16*>(planes_t), ld_t, nterms,
-                                                          nterms_t);
-        return cudaGetLastError();
-    }
-    split_planes_kernel<<<grid, 256, 0, stream>>>(src, R, Cc, col_scale, static_cast<__nv_bfloat16*>(planes), ld_n,
-                                                  static_cast<__nv_bfloat16*>(planes_t), ld_t, nterms, nterms_t);
+cudaError_t launch_split_terms(const float* src, int R, int Cc, int ld, const float* col_scale, void* planes, void* planes_s,
+                               uint32_t* amax, int sm_count, cudaStream_t stream) {
+    const bool vec = (Cc & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
+                     (col_scale == nullptr || (reinterpret_cast<uintptr_t>(col_scale) & 15) == 0);
+    __half* p0 = static_cast<__half*>(planes);
+    __half* p1 = static_cast<__half*>(planes_s);
+    const float* cs = p1 ? col_scale : nullptr;
+    auto blocks = [&](size_t work, int per_sm) {
+        const size_t b = (work + 255) / 256;
+        return (int)(b < (size_t)sm_count * per_sm ? (b ? b : 1) : (size_t)sm_count * per_sm);
+    };
+    const size_t n = (size_t)R * Cc;
+    if (vec) amax_kernel<true><<<blocks(n / 4, 8), 256, 0, stream>>>(src, R, Cc, cs, amax);
+    else amax_kernel<false><<<blocks(n, 8), 256, 0, stream>>>(src, R, Cc, cs, amax);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const int nb = blocks((size_t)R * ((Cc + 7) / 8), 8);
+    if (vec) split_terms_kernel<true><<<nb, 256, 0, stream>>>(src, R, Cc, ld, cs, p0, p1, amax);
+    else split_terms_kernel<false><<<nb, 256, 0, stream>>>(src, R, Cc, ld, cs, p0, p1, amax);
     return cudaGetLastError();
 }
 
-cudaError_t launch_expand_ternary(const uint8_t* state, int C, int O, int I, void* T, int ld_i, void* Tt, int ld_o,
-                                  cudaStream_t stream) {
-    dim3 grid((I + 63) / 64, (O + 63) / 64);
-    expand_ternary_kernel<<<grid, 256, 0, stream>>>(state, C, O, I, static_cast<__nv_bfloat16*>(T), ld_i,
-                                                    static_cast<__nv_bfloat16*>(Tt), ld_o);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_expand_ternary_p2(const uint32_t* packed2, int O, int I, void* T, int ld_i, void* Tt, int ld_o,
-                                     cudaStream_t stream) {
-    dim3 grid((I + 63) / 64, (O + 63) / 64);
-    expand_ternary_p2_kernel<<<grid, 256, 0, stream>>>(packed2, O, I, static_cast<__nv_bfloat16*>(T), ld_i,
-                                                       static_cast<__nv_bfloat16*>(Tt), ld_o);
+cudaError_t launch_expand_ternary(const uint8_t* state, const uint32_t* packed2, int C, int O, int I, void* T, int ld,
+                                  int sm_count, cudaStream_t stream) {
+    __half* t = static_cast<__half*>(T);
+    const size_t units = (size_t)O * ((I + 15) / 16);
+    int blocks = (int)((units + 255) / 256 < (size_t)sm_count * 8 ? (units + 255) / 256 : (size_t)sm_count * 8);
+    if (!state)
+        expand_ternary_p2_kernel<<<blocks, 256, 0, stream>>>(packed2, (size_t)O * (I / 16), t);
+    else if (I % 16 == 0 && ld == I && (reinterpret_cast<uintptr_t>(state) & 3) == 0)
+        expand_ternary_kernel<true><<<blocks, 256, 0, stream>>>(state, C, O, I, t, ld);
+    else
+        expand_ternary_kernel<false><<<blocks, 256, 0, stream>>>(state, C, O, I, t, ld);
     return cudaGetLastError();
 }
 
