@@ -223,9 +223,11 @@ struct Carver {
 
 inline int up8(size_t x) { return (int)((x + 7) & ~size_t(7)); }
 
-bool tc_wanted(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
+// out, col_scale: where the output goes and what its columns are scaled by (null: not checked)
+bool tc_wanted(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K, const void* out = nullptr, const void* col_scale = nullptr) {
     if (ctx->gemm_mode == MCL_CUDA_GEMM_EXACT) return false;
-    if (N % 4 != 0) return false;                       // 128-bit stores of the output tile
+    if (N % 4 != 0) return false;                       // rows of the output are written in 16-byte units
+    if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(col_scale)) & 15) return false;
     if (M > 0x7fffffffull / 2 || N > 0x7fffffffull / 2 || K > 0x7fffffffull / 2) return false;
     if (ctx->gemm_mode == MCL_CUDA_GEMM_TENSOR) return true;
     return (double)M * (double)N * (double)K >= (double)(1u << 22);
@@ -236,7 +238,7 @@ bool tc_wanted(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
 // Tensor-core products on fp16 terms (tc_gemm.cu).  A call carves the terms of its tensors from the workspace, clears one
 // pair of magnitude words per tensor, fills the terms, and runs its products.
 struct TermBuf { size_t planes, scaled, words; size_t rows; int cols, ld; };
-size_t term_bytes(size_t rows, int ld) { return 2 * rows * (size_t)ld * 2; }
+size_t term_bytes(size_t rows, int ld) { return 2 * rows * (size_t)ld * 2 + mcl::kTermPad; }
 TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled, size_t words) {
     TermBuf t = {0, 0, words, rows, (int)cols, up8(cols)};
     if (plain) t.planes = cv->reserve(term_bytes(rows, t.ld));
@@ -262,10 +264,15 @@ mcl::TcOperand digits_of(const char* T, size_t O, size_t I, bool mn_major) {
 }
 constexpr size_t kWordBytes = 64;      // magnitude words of a call: one pair per tensor, 8 bytes each
 
+// plan of a product with ternary digits (depth unbounded: exact digits) or of two split tensors
+mcl::TcPlan digit_plan(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) { return mcl::tc_plan((int)M, (int)N, (int)K, 2, ctx->sm_count, 0); }
+mcl::TcPlan dense_plan(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
+    return mcl::tc_plan((int)M, (int)N, (int)K, 3, ctx->sm_count, mcl::kGradDepthLimit);
+}
 int tc_product(mcl_cuda_ctx* ctx, const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K,
-               const float* col_scale, float* splitk_ws, int splits) {
+               const float* col_scale, float* splitk_ws, const mcl::TcPlan& plan) {
     int launches = 0;
-    cudaError_t e = mcl::launch_tc_gemm(a, b, c, (int)N, (int)M, (int)N, (int)K, col_scale, splitk_ws, splits, ctx->err_word,
+    cudaError_t e = mcl::launch_tc_gemm(a, b, c, (int)M, (int)N, (int)K, plan, col_scale, splitk_ws, ctx->err_word,
                                         ctx->max_smem, ctx->sm_count, ctx->stream, &launches);
     ctx->launches += launches;
     if (e != cudaSuccess) return fail_cuda(ctx, "tensor-core contraction", e);
@@ -517,17 +524,15 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
     MCL_TRY(check_ptr(ctx, op, "y", y, 4));
     DeviceGuard guard(ctx->device);
     // narrow layers: the tf32 hi/lo kernel reads x in place (no operand-splitting pass)
-    if (tc_wanted(ctx, batch, out_features, in_features) &&
+    if (tc_wanted(ctx, batch, out_features, in_features, y, scale) &&
         fused_wanted(ctx, x, nullptr, state, scale, y, nullptr, nullptr, in_features, out_features, batch))
         return fused_products(ctx, op, x, nullptr, state, nullptr, scale, y, nullptr, nullptr, C, in_features, out_features, batch);
-    if (tc_wanted(ctx, batch, out_features, in_features)) {
-        int splits = 1;
-        const size_t sk = mcl::tc_splitk_workspace_bytes((int)batch, (int)out_features, (int)in_features,
-                                                         ctx->sm_count, 0, &splits);
+    if (tc_wanted(ctx, batch, out_features, in_features, y, scale)) {
+        const mcl::TcPlan plan = digit_plan(ctx, batch, out_features, in_features);
         Carver cv;
         const size_t o_w = cv.reserve(kWordBytes);
         const TermBuf xb = carve_terms(&cv, batch, in_features, true, false, o_w);
-        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2), o_k = cv.reserve(sk);
+        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2 + mcl::kTermPad), o_k = cv.reserve(plan.workspace_bytes);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
@@ -536,7 +541,7 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
         MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
                                                        up8(in_features), ctx->sm_count, ctx->stream));
         return tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, out_features, in_features, false), y, batch,
-                          out_features, in_features, scale, reinterpret_cast<float*>(w + o_k), splits);
+                          out_features, in_features, scale, reinterpret_cast<float*>(w + o_k), plan);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_forward(x, state, scale, y, (int)batch, (int)in_features,
                                                          (int)out_features, (int)C, ctx->stream));
@@ -555,17 +560,15 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
     MCL_TRY(check_ptr(ctx, op, "grad_out", grad_out, 4));
     MCL_TRY(check_ptr(ctx, op, "grad_x", grad_x, 4));
     DeviceGuard guard(ctx->device);
-    if (tc_wanted(ctx, batch, in_features, out_features) &&
+    if (tc_wanted(ctx, batch, in_features, out_features, grad_x) &&
         fused_wanted(ctx, nullptr, grad_out, state, scale, nullptr, grad_x, nullptr, in_features, out_features, batch))
         return fused_products(ctx, op, nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, C, in_features, out_features, batch);
-    if (tc_wanted(ctx, batch, in_features, out_features)) {
-        int splits = 1;
-        const size_t sk = mcl::tc_splitk_workspace_bytes((int)batch, (int)in_features, (int)out_features,
-                                                         ctx->sm_count, 0, &splits);
+    if (tc_wanted(ctx, batch, in_features, out_features, grad_x)) {
+        const mcl::TcPlan plan = digit_plan(ctx, batch, in_features, out_features);
         Carver cv;
         const size_t o_w = cv.reserve(kWordBytes);
         const TermBuf gb = carve_terms(&cv, batch, out_features, false, true, o_w);
-        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2), o_k = cv.reserve(sk);
+        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2 + mcl::kTermPad), o_k = cv.reserve(plan.workspace_bytes);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
@@ -574,7 +577,7 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
         MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
                                                        up8(in_features), ctx->sm_count, ctx->stream));
         return tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, out_features, in_features, true), grad_x, batch,
-                          in_features, out_features, nullptr, reinterpret_cast<float*>(w + o_k), splits);
+                          in_features, out_features, nullptr, reinterpret_cast<float*>(w + o_k), plan);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_backward_input(state, scale, grad_out, grad_x, (int)batch,
                                                                 (int)in_features, (int)out_features,
@@ -646,18 +649,17 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     const size_t state_row = in_features / 4 * 3;
     const bool tc = tc_wanted(ctx, tile_rows, in_features, batch) && tile_rows >= 64;
     if (tc) tile_rows &= ~size_t(7);      // a tile starts at a 16-byte aligned column of the terms of grad_out
-    int splits = 1;
+    mcl::TcPlan plan = {};
     Carver cv;
     const size_t o_gw = cv.reserve(tile_rows * row_b);
     size_t o_k = 0, o_w = 0;
     TermBuf gb, xb;
     if (tc) {
-        const size_t sk = mcl::tc_splitk_workspace_bytes((int)tile_rows, (int)in_features, (int)batch,
-                                                         ctx->sm_count, mcl::kGradDepthLimit, &splits);
+        plan = dense_plan(ctx, tile_rows, in_features, batch);
         o_w = cv.reserve(kWordBytes);
         gb = carve_terms(&cv, batch, out_features, true, false, o_w);      // activation-sized, not weight-sized
         xb = carve_terms(&cv, batch, in_features, true, false, o_w + 8);
-        o_k = cv.reserve(sk);
+        o_k = cv.reserve(plan.workspace_bytes);
     }
     void* wsp = nullptr;
     MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
@@ -675,7 +677,7 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
             a.ptr = static_cast<const char*>(a.ptr) + r0 * 2;
             a.cols = (int)nr;
             MCL_TRY(tc_product(ctx, a, terms_of(w, xb, false, true), gw, nr, in_features, batch, nullptr,
-                               reinterpret_cast<float*>(w + o_k), splits));
+                               reinterpret_cast<float*>(w + o_k), plan));
         } else {
             MCL_LAUNCH(ctx, "counter update (grad_w tile)",
                        mcl::launch_simt_grad_w(grad_out, x, gw, (int)batch, (int)in_features,
@@ -770,7 +772,7 @@ static int fused_products(mcl_cuda_ctx* ctx, const char* op, const float* x, con
 static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, const float* grad_out,
                            const uint8_t* state, const uint32_t* packed2, const float* scale, float* y,
                            float* grad_x, float* grad_w, size_t C, size_t I, size_t O, size_t Nt) {
-    const bool tc = tc_wanted(ctx, Nt, O, I) && tc_wanted(ctx, Nt, I, O) && tc_wanted(ctx, O, I, Nt);
+    const bool tc = tc_wanted(ctx, Nt, O, I, y, scale) && tc_wanted(ctx, Nt, I, O, grad_x) && tc_wanted(ctx, O, I, Nt, grad_w);
     if (!tc) {
         if (state) {
             if (y) MCL_TRY(mcl_cuda_counter_forward(ctx, x, state, scale, y, Nt, I, O, C));
@@ -785,17 +787,16 @@ static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, co
     }
     if (fused_wanted(ctx, x, grad_out, state ? static_cast<const void*>(state) : packed2, scale, y, grad_x, grad_w, I, O, Nt))
         return fused_products(ctx, op, x, grad_out, state, packed2, scale, y, grad_x, grad_w, C, I, O, Nt);
-    int s_y = 1, s_x = 1, s_w = 1;
-    const size_t k_y = mcl::tc_splitk_workspace_bytes((int)Nt, (int)O, (int)I, ctx->sm_count, 0, &s_y);
-    const size_t k_x = mcl::tc_splitk_workspace_bytes((int)Nt, (int)I, (int)O, ctx->sm_count, 0, &s_x);
-    const size_t k_w = mcl::tc_splitk_workspace_bytes((int)O, (int)I, (int)Nt, ctx->sm_count, mcl::kGradDepthLimit, &s_w);
-    size_t k_max = k_y > k_x ? k_y : k_x;
-    if (k_w > k_max) k_max = k_w;
+    const mcl::TcPlan p_y = digit_plan(ctx, Nt, O, I), p_x = digit_plan(ctx, Nt, I, O), p_w = dense_plan(ctx, O, I, Nt);
+    size_t k_max = 0;
+    if (y) k_max = p_y.workspace_bytes;
+    if (grad_x && p_x.workspace_bytes > k_max) k_max = p_x.workspace_bytes;
+    if (grad_w && p_w.workspace_bytes > k_max) k_max = p_w.workspace_bytes;
     Carver cv;
     const size_t o_w = cv.reserve(kWordBytes);
     const TermBuf xb = carve_terms(&cv, Nt, I, y || grad_w, false, o_w);
     const TermBuf gb = carve_terms(&cv, Nt, O, grad_w != nullptr, grad_x != nullptr, o_w + 8);
-    const size_t o_t = cv.reserve(O * (size_t)up8(I) * 2);
+    const size_t o_t = cv.reserve(O * (size_t)up8(I) * 2 + mcl::kTermPad);
     const size_t o_k = cv.reserve(k_max);
     void* wsp = nullptr;
     MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
@@ -806,9 +807,9 @@ static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, co
     if (grad_x || grad_w) MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, grad_x ? scale : nullptr, grad_w != nullptr));
     if (y || grad_x)
         MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, packed2, (int)C, (int)O, (int)I, w + o_t, up8(I), ctx->sm_count, ctx->stream));
-    if (y) MCL_TRY(tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, O, I, false), y, Nt, O, I, scale, kws, s_y));
-    if (grad_x) MCL_TRY(tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, O, I, true), grad_x, Nt, I, O, nullptr, kws, s_x));
-    if (grad_w) MCL_TRY(tc_product(ctx, terms_of(w, gb, false, true), terms_of(w, xb, false, true), grad_w, O, I, Nt, nullptr, kws, s_w));
+    if (y) MCL_TRY(tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, O, I, false), y, Nt, O, I, scale, kws, p_y));
+    if (grad_x) MCL_TRY(tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, O, I, true), grad_x, Nt, I, O, nullptr, kws, p_x));
+    if (grad_w) MCL_TRY(tc_product(ctx, terms_of(w, gb, false, true), terms_of(w, xb, false, true), grad_w, O, I, Nt, nullptr, kws, p_w));
     return MCL_CUDA_OK;
 }
 
@@ -1134,15 +1135,14 @@ int mcl_cuda_matmul_f32(mcl_cuda_ctx* ctx, const float* a, const float* b, float
     MCL_TRY(check_ptr(ctx, op, "b", b, 4));
     MCL_TRY(check_ptr(ctx, op, "c", c, 4));
     DeviceGuard guard(ctx->device);
-    if (tc_wanted(ctx, M, N, K)) {
-        int splits = 1;
-        const size_t sk = mcl::tc_splitk_workspace_bytes((int)M, (int)N, (int)K, ctx->sm_count, mcl::kGradDepthLimit, &splits);
+    if (tc_wanted(ctx, M, N, K, c)) {
+        const mcl::TcPlan plan = dense_plan(ctx, M, N, K);
         Carver cv;
         const size_t o_w = cv.reserve(kWordBytes);
         // a stored [M,K] or (trans_a) [K,M], b stored [K,N] or (trans_b) [N,K]: split as stored, read in the needed orientation
         const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false, o_w);
         const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false, o_w + 8);
-        const size_t o_k = cv.reserve(sk);
+        const size_t o_k = cv.reserve(plan.workspace_bytes);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
@@ -1150,7 +1150,7 @@ int mcl_cuda_matmul_f32(mcl_cuda_ctx* ctx, const float* a, const float* b, float
         MCL_TRY(fill_terms(ctx, op, w, ab, a, nullptr, true));
         MCL_TRY(fill_terms(ctx, op, w, bb, b, nullptr, true));
         return tc_product(ctx, terms_of(w, ab, false, trans_a != 0), terms_of(w, bb, false, trans_b == 0), c, M, N, K, nullptr,
-                          reinterpret_cast<float*>(w + o_k), splits);
+                          reinterpret_cast<float*>(w + o_k), plan);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_matmul_f32(a, b, c, (int)M, (int)K, (int)N, trans_a, trans_b, ctx->stream));
     return MCL_CUDA_OK;

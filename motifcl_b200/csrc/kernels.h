@@ -53,11 +53,12 @@ cudaError_t launch_simt_grad_w(const float* grad_out, const float* x, float* gra
                                cudaStream_t stream);
 
 // tc_gemm.cu -- tcgen05 / TMEM / TMA contractions on fp16 term planes (see the file header)
-int tc_pick_bn(int N);
-size_t tc_splitk_workspace_bytes(int M, int N, int K, int sm_count, int depth_limit, int* splits_out);
+struct TcPlan { int pair, bn, splits, ktiles_per_split; size_t workspace_bytes; };
+TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit);
 // k-tiles of 64 per accumulator for fp32 x fp32 products: 3 x 4 instructions per k-tile add into it, each with a truncation
 // error of about 2.7e-9 relative (K = 4096: 2e-6)
 constexpr int kGradDepthLimit = 64;
+constexpr size_t kTermPad = 1024;  // readable bytes after the last plane of a TcOperand
 struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major tensor with `cols` columns
     const void* ptr;
     int rows, cols, ld;
@@ -66,9 +67,9 @@ struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major 
     const uint32_t* amax;      // bits of the split tensor's largest magnitude (null for digits)
 };
 // C[M,N] = sum over k of A B (b.planes == 1: two products, b.planes == 2: three)
-cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int ldc, int M, int N, int K,
-                           const float* col_scale, float* splitk_ws, int splits, int* err_word, size_t max_smem,
-                           int sm_count, cudaStream_t stream, int* launches);
+cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int M, int N, int K, const TcPlan& plan,
+                           const float* col_scale, float* splitk_ws, int* err_word, size_t max_smem, int sm_count,
+                           cudaStream_t stream, int* launches);
 // fp32 [R,Cc] -> fp16 terms [2][R][ld] of src (planes) and / or of src . col_scale (planes_s); amax: two zeroed words that
 // receive the largest magnitudes of the two.  Two launches.
 cudaError_t launch_split_terms(const float* src, int R, int Cc, int ld, const float* col_scale, void* planes, void* planes_s,

@@ -36,12 +36,11 @@ constexpr int kATileBytes = BM * BK * 2;   // 16 KiB
 constexpr int kLoShift = 12;               // lo terms are stored 2^12 up
 
 struct TcParams {
-    float* C;                 // output [M, ldc] (or split-K partials [splits][M][ldc])
     const float* col_scale;   // optional, applied when splits == 1
     const uint32_t* a_amax;   // bits of the largest magnitude of the split tensor (null: operand is unscaled)
     const uint32_t* b_amax;
-    int M, N, K, ldc;
-    int BN, stages, b_bytes;
+    int M, N, K;
+    int BN, stages, b_bytes;   // b_bytes: one CTA's share of a B tile
     int a_mn, b_mn;           // operand is stored with M / N contiguous
     int nterms;               // 2: A lo, A hi against one B plane; 3: lo.hi, hi.lo, hi.hi
     int ktiles_per_split, splits;
@@ -68,13 +67,70 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// D = A.B + D 2^-12
-__device__ __forceinline__ void umma_f16_down12(uint32_t tmem_c, uint64_t da, uint64_t db, uint32_t idesc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, 1, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, 12;\n\t}"
-        ::"r"(tmem_c), "l"(da), "l"(db), "r"(idesc) : "memory");
+// One lane of a converged warp.  The lanes that issue copies and MMAs run their loops with the whole warp and branch here
+// only around the instructions themselves: addresses and descriptors are then warp-uniform for the compiler.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+// D = A.B + (accum ? D : 0), and D = A.B + D 2^-12; descriptors as low and high words; CG = 2: issued by the pair's leader for
+// both CTAs
+template <int CG>
+__device__ __forceinline__ void umma_f16(uint32_t tmem_c, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                         uint32_t accum) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
+                     ::"r"(tmem_c), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, p;\n\t}"
+                     ::"r"(tmem_c), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void umma_f16_down12(uint32_t tmem_c, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc) {
+    if (CG == 1)
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, 1, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p, 12;\n\t}"
+                     ::"r"(tmem_c), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, 1, 0;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, p, 12;\n\t}"
+                     ::"r"(tmem_c), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc) : "memory");
+}
+// arrive on the barrier at this shared-memory offset, in both CTAs of a pair, when the MMAs issued so far are done
+template <int CG>
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    if (CG == 1) umma_commit(bar);
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// tile load whose bytes are counted by `bar`; CG = 2: the barrier may be the other CTA's (a shared::cluster address)
+template <int CG>
+__device__ __forceinline__ void tc_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    if (CG == 1) tma_load_3d(dst, map, bar, c0, c1, c2);
+    else
+        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+                     ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void tc_load4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+    if (CG == 1)
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // item -> output tile and K slice.  Groups of group_m row tiles run through all column tiles before the next group, so
@@ -94,16 +150,29 @@ __device__ __forceinline__ TcItem tc_item(int item, int tiles_m, int tiles_n, in
     return t;
 }
 
-// Persistent CTA of 192 threads; work items (output tile x split-K slice) are dealt round-robin.
-//   warp 0        TMA producer (one elected lane)
-//   warp 1        MMA issuer (one elected lane); also allocates / frees TMEM
-//   warps 2..5    epilogue: TMEM lanes 32*(warp%4) .. +31
+// Persistent CTAs of 192 threads; work items (output tile x split-K slice) are dealt round-robin.
+//   warp 0        TMA producer (one elected lane): tiles of A and B into a ring of `stages` shared-memory slots
+//   warp 1        MMA issuer (one elected lane): four tcgen05.mma (K = 16 each) per slot; also allocates / frees TMEM
+//   warps 2..5    epilogue: tcgen05.ld of 32 lanes x 64 columns, scale, a swizzled 32 x 32 tile in shared memory, TMA store
 // Two accumulators live in TMEM (columns [0,BN) and [ACC,ACC+BN)), so the epilogue of one item
 // overlaps the main loop of the next.
+//
+// CG = 2: a cluster of two CTAs shares a 256 x BN tile (tcgen05 cta_group::2).  Each CTA loads its own 128 rows of A and
+// its own half of the BN rows of B, the leader's lane issues the MMAs for both tensor cores, and every CTA holds the
+// accumulator rows of its own A.  That halves the B bytes a CTA has to write to and read from shared memory: with
+// CG = 1 and BN = 256 a k-tile of 64 moves 96 KB through a 128 B/clk pipe (768 cycles) for 512 cycles of MMA; with CG = 2
+// 64 KB (512).  All loads count on the leader's barrier.
+//
+// Every mbarrier wait is bounded: on time-out the kernel records an error word, skips the rest of its work, frees
+// its TMEM and returns.
 constexpr int kTcThreads = 192;
+constexpr int kSmemSlotTcPair = 16;       // ensure_dynamic_smem: see there
+constexpr int kStageBytes = 8 * 4096;      // epilogue staging: two 32 x 32 float tiles per warp
 
+template <int CG>
 __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                                                              const __grid_constant__ CUtensorMap tmB,
+                                                             const __grid_constant__ CUtensorMap tmC,
                                                              const TcParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4];
@@ -112,7 +181,10 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int BN = p.BN, S = p.stages;
-    const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t rank = CG == 2 ? (blockIdx.x & 1u) : 0u;      // cluster of two consecutive CTAs
+    const int unit = (int)blockIdx.x / CG, n_units = (int)gridDim.x / CG;
+    const uint32_t staging = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t tiles = staging + kStageBytes;
     const uint32_t stage_bytes = kATileBytes + (uint32_t)p.b_bytes;
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
@@ -123,141 +195,168 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     while ((int)acc_cols < BN) acc_cols <<= 1;
     const uint32_t tmem_cols = 2 * acc_cols;      // <= 512
 
-    const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + BM - 1) / BM;
+    const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + CG * BM - 1) / (CG * BM);
     const int ktiles = (p.K + BK - 1) / BK;
     const int n_items = tiles_m * tiles_n * p.splits;
 
     if (threadIdx.x == 0) {
         abort_flag = (*reinterpret_cast<volatile int*>(p.err) != 0);   // an earlier CTA gave up: do not wait at all
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 128); }
+        for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 4 * CG); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                         ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    if (CG == 2) cluster_sync();
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- TMA producer --------------------------------------------------------------
-            uint32_t it = 0;       // slot counter across all items of this CTA
-            for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x) {
-                const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
-                const int kt0 = t.split * p.ktiles_per_split;
-                const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
-                for (int term = 0; term < p.nterms; ++term) {
-                    // planes: 0 = hi, 1 = lo; products with a lo term first
-                    const int pa = p.nterms == 3 ? (term == 0) : (term + 1 < p.nterms);
-                    const int pb = p.nterms == 3 && term == 1;
-                    for (int kk = 0; kk < my_kt; ++kk, ++it) {
-                        const int s = (int)(it % (uint32_t)S);
-                        const uint32_t ph = (it / (uint32_t)S) & 1u;
-                        if (!mbar_wait(empty_bar(s), ph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 1); break; }
-                        const uint32_t a_dst = tiles + (uint32_t)s * stage_bytes;
-                        mbar_expect_tx(full_bar(s), stage_bytes);
-                        const int k0 = (kt0 + kk) * BK;
-                        if (p.a_mn) {
-                            tma_load_3d(a_dst, &tmA, full_bar(s), t.mt * BM, k0, pa);
-                            tma_load_3d(a_dst + 8192, &tmA, full_bar(s), t.mt * BM + 64, k0, pa);
-                        } else {
-                            tma_load_3d(a_dst, &tmA, full_bar(s), k0, t.mt * BM, pa);
-                        }
-                        if (p.b_mn) {
-                            for (int c = 0; c < BN; c += 64)
-                                tma_load_3d(a_dst + kATileBytes + (uint32_t)c * 128u, &tmB, full_bar(s), t.nt * BN + c, k0, pb);
-                        } else {
-                            tma_load_3d(a_dst + kATileBytes, &tmB, full_bar(s), k0, t.nt * BN, pb);
-                        }
+        // ---- TMA producer ------------------------------------------------------------------
+        int s = 0;                 // ring slot and its phase, across all items of this CTA
+        uint32_t ph = 1;
+        bool ok = true;
+        for (int item = unit; item < n_items && ok; item += n_units) {
+            const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
+            const int kt0 = t.split * p.ktiles_per_split;
+            const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
+            const int m0 = (t.mt * CG + (int)rank) * BM, n0 = t.nt * BN + (int)rank * (BN / CG);
+            for (int term = 0; term < p.nterms && ok; ++term) {
+                // planes: 0 = hi, 1 = lo; products with a lo term first
+                const int pa = p.nterms == 3 ? (term == 0) : (term + 1 < p.nterms);
+                const int pb = p.nterms == 3 && term == 1;
+                for (int kk = 0; kk < my_kt; ++kk) {
+                    ok = mbar_wait_all(empty_bar(s), ph, &abort_flag);
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 1); break; }
+                    const uint32_t a_dst = tiles + (uint32_t)s * stage_bytes;
+                    const uint32_t bar = CG == 2 ? cluster_addr(full_bar(s), 0) : full_bar(s);
+                    const int k0 = (kt0 + kk) * BK;
+                    if (elect_one()) {
+                        if (rank == 0) mbar_expect_tx(full_bar(s), CG * stage_bytes);
+                        if (p.a_mn) tc_load4<CG>(a_dst, &tmA, bar, m0, k0, 0, pa);
+                        else tc_load<CG>(a_dst, &tmA, bar, k0, m0, pa);
+                        if (p.b_mn) tc_load4<CG>(a_dst + kATileBytes, &tmB, bar, n0, k0, 0, pb);
+                        else tc_load<CG>(a_dst + kATileBytes, &tmB, bar, k0, n0, pb);
                     }
-                    if (abort_flag) break;
+                    __syncwarp();
+                    if (++s == S) { s = 0; ph ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (rank == 0) {
             // ---- MMA issuer ----------------------------------------------------------------
-            const uint32_t idesc = idesc_f16(BM, BN, p.a_mn, p.b_mn);
+            const uint32_t idesc = idesc_f16(CG * BM, BN, p.a_mn, p.b_mn);
             const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;   // 16 k further, in 16-byte units
-            uint32_t it = 0, n_local = 0;
-            for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x, ++n_local) {
+            const uint64_t da0 = p.a_mn ? smem_desc_mn_sw128(tiles) : smem_desc_k_sw128(tiles);
+            const uint64_t db0 = p.b_mn ? smem_desc_mn_sw128(tiles + kATileBytes) : smem_desc_k_sw128(tiles + kATileBytes);
+            const uint32_t a_hi = (uint32_t)(da0 >> 32), b_hi = (uint32_t)(db0 >> 32), a0 = (uint32_t)da0, b0 = (uint32_t)db0;
+            uint32_t n_local = 0, ph = 0;
+            int s = 0;
+            bool ok = true;
+            for (int item = unit; item < n_items && ok; item += n_units, ++n_local) {
                 const int kt0 = (item / (tiles_m * tiles_n)) * p.ktiles_per_split;
                 const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
                 const int total = p.nterms * my_kt, first_hi = total - my_kt;
                 const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
-                if (!mbar_wait(acc_empty(acc), aph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 4); break; }
+                ok = mbar_wait_all(acc_empty(acc), aph ^ 1u, &abort_flag);
+                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 4); break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * acc_cols;
-                for (int j = 0; j < total; ++j, ++it) {
-                    const int s = (int)(it % (uint32_t)S);
-                    const uint32_t ph = (it / (uint32_t)S) & 1u;
-                    if (!mbar_wait(full_bar(s), ph, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 2); break; }
+                for (int j = 0; j < total; ++j) {
+                    ok = mbar_wait_all(full_bar(s), ph, &abort_flag);
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 2); break; }
                     tc_fence_after();
-                    const uint32_t a_addr = tiles + (uint32_t)s * stage_bytes;
-                    const uint32_t b_addr = a_addr + kATileBytes;
-                    const uint64_t da = p.a_mn ? smem_desc_mn_sw128(a_addr) : smem_desc_k_sw128(a_addr);
-                    const uint64_t db = p.b_mn ? smem_desc_mn_sw128(b_addr) : smem_desc_k_sw128(b_addr);
+                    const uint32_t off = ((uint32_t)s * stage_bytes) >> 4;
+                    const uint32_t a_lo = a0 + off, b_lo = b0 + off;
+                    if (elect_one()) {
+                        if (j == first_hi) umma_f16_down12<CG>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc);
+                        else umma_f16<CG>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, j != 0 ? 1u : 0u);
 #pragma unroll
-                    for (int kk = 0; kk < BK / 16; ++kk) {
-                        if (kk == 0 && j == first_hi && p.nterms > 1)
-                            umma_f16_down12(d_tmem, da, db, idesc);
-                        else
-                            umma_bf16(d_tmem, da + (uint64_t)(a_step * kk), db + (uint64_t)(b_step * kk), idesc, (j | kk) != 0 ? 1u : 0u);
+                        for (int kk = 1; kk < BK / 16; ++kk)
+                            umma_f16<CG>(d_tmem, a_lo + a_step * kk, a_hi, b_lo + b_step * kk, b_hi, idesc, 1u);
+                        tc_commit<CG>(empty_bar(s));
+                        if (j == total - 1) tc_commit<CG>(acc_full(acc));
                     }
-                    umma_commit(empty_bar(s));
+                    __syncwarp();
+                    if (++s == S) { s = 0; ph ^= 1u; }
                 }
-                if (abort_flag) break;
-                umma_commit(acc_full(acc));
             }
         }
     } else {
-        // ---- epilogue warps: TMEM -> registers -> global ---------------------------------------
+        // ---- epilogue warps: TMEM -> registers -> shared memory -> global ---------------------------
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const bool scale = (p.col_scale != nullptr) && p.splits == 1;
         const float fa = p.a_amax ? pow2(-term_exp(__ldg(p.a_amax))) : 1.0f;      // undo the powers of two of the split
         const float fb = p.b_amax ? pow2(-term_exp(__ldg(p.b_amax))) : 1.0f;
-        uint32_t n_local = 0;
-        for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n_local) {
+        const uint32_t my_stage = staging + (uint32_t)q * 8192u;
+        uint32_t n_local = 0, n_store = 0;
+        for (int item = unit; item < n_items; item += n_units, ++n_local) {
             const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
-            const int mt = t.mt, nt = t.nt, split = t.split;
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
-            bool ok = !abort_flag;
-            if (ok && !mbar_wait(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 3); ok = false; }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            const bool was = !abort_flag;
+            if (!__all_sync(0xffffffffu, was)) break;
+            if (!mbar_wait_warp(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 3); break; }
             tc_fence_after();
-            const int n0 = nt * BN;
-            const int row = mt * BM + q * 32 + lane;
-            float* crow = p.C + ((size_t)split * p.M + row) * p.ldc;
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                if (n0 + c0 >= p.N) break;
-                uint32_t r[32];
-                tmem_ld32(tmem_base + acc * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+            const int n0 = t.nt * BN, row0 = (t.mt * CG + (int)rank) * BM + q * 32;
+            const int ncols = min(BN, p.N - n0);
+            for (int c0 = 0; c0 < ncols; c0 += 64) {
+                uint32_t r[2][32];
+                const uint32_t t_addr = tmem_base + acc * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+                tmem_ld32(t_addr, r[0]);
+                if (c0 + 32 < ncols) tmem_ld32(t_addr + 32, r[1]);
                 tmem_ld_wait();
-                if (row < p.M) {
+                if (c0 + 64 >= ncols) {                // the accumulator is in registers: release it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CG == 1) mbar_arrive(acc_empty(acc));
+                        else asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(acc_empty(acc), 0)) : "memory");
+                    }
+                }
+                if (row0 >= p.M) continue;             // rows of the padding: nothing to store
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        const int col = n0 + c0 + j;
-                        if (col >= p.N) break;
-                        float4 o = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                               __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+                for (int h = 0; h < 2; ++h) {
+                    const int cc = c0 + 32 * h;
+                    if (cc >= ncols) break;
+                    const uint32_t buf = my_stage + (n_store & 1u) * 4096u;
+                    ++n_store;
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");     // the store before last has read this buffer
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float4 o = make_float4(__uint_as_float(r[h][4 * j]), __uint_as_float(r[h][4 * j + 1]),
+                                               __uint_as_float(r[h][4 * j + 2]), __uint_as_float(r[h][4 * j + 3]));
                         o.x = o.x * fa * fb; o.y = o.y * fa * fb; o.z = o.z * fa * fb; o.w = o.w * fa * fb;
-                        if (scale) {
-                            const float4 sc = __ldg(reinterpret_cast<const float4*>(p.col_scale + col));
+                        if (scale && cc + 4 * j < ncols) {            // N % 4 == 0
+                            const float4 sc = __ldg(reinterpret_cast<const float4*>(p.col_scale + n0 + cc + 4 * j));
                             o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
                         }
-                        *reinterpret_cast<float4*>(crow + col) = o;    // N % 4 == 0, ldc % 4 == 0
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(buf + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) << 4)), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                     ::"l"(reinterpret_cast<uint64_t>(&tmC)), "r"(buf), "r"(n0 + cc), "r"(row0), "r"(t.split) : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
             }
-            tc_fence_before();
-            mbar_arrive(acc_empty(acc));               // 128 arrivals free the accumulator
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     __syncwarp();
     if (abort_flag) {
@@ -266,9 +365,11 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         while (clock64() - t0 < 2000000ull) {}
     }
     tc_fence_before();
-    __syncthreads();
+    if (CG == 2) cluster_sync();
+    else __syncthreads();
     if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
 
@@ -458,115 +559,143 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// 3-D map over fp16 planes [P][rows][ld] with `cols` used columns: dims {cols, rows, P}, 128-byte swizzle; box
-// {64, box_rows, 1} for a K-major operand, {64, 64, 1} for an MN-major one (one chunk of 64 columns, 64 k rows).
-// Reads beyond cols or rows return zeros, so ragged edges need no padding in memory.
-bool make_map(CUtensorMap* map, const TcOperand& o, int box_rows) {
+// Map over fp16 planes [P][rows][ld] with `cols` used columns, 128-byte swizzle.  K-major: dims {cols, rows, P}, box
+// {64, tile_rows, 1}.  MN-major: a tile of more than 64 columns is several 128-byte wide chunks in shared memory, so a third
+// dimension of stride 64 columns walks over the chunks: dims {cols, rows, chunks, P}, box {64, 64 k rows, chunks, 1}, one
+// copy per tile (the lane that issues copies was the limit with one copy per chunk: 613 cycles per k-tile against 565).
+// Reads beyond cols or rows return zeros; chunks after the first may run past the end of a row into the next (those
+// columns of the output are clipped), or past the last row: buffers are padded by kTermPad bytes.
+bool make_map(CUtensorMap* map, const TcOperand& o, int tile_rows) {
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return false;
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    const cuuint64_t plane = (cuuint64_t)o.rows * o.ld * 2;
+    if (o.mn_major) {
+        const int chunks = (tile_rows + 63) / 64;
+        cuuint64_t dims[4] = {(cuuint64_t)o.cols, (cuuint64_t)o.rows, (cuuint64_t)chunks, (cuuint64_t)o.planes};
+        cuuint64_t strides[3] = {(cuuint64_t)o.ld * 2, 128, plane};
+        cuuint32_t box[4] = {64, (cuuint32_t)BK, (cuuint32_t)chunks, 1};
+        return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(o.ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
     cuuint64_t dims[3] = {(cuuint64_t)o.cols, (cuuint64_t)o.rows, (cuuint64_t)o.planes};
-    cuuint64_t strides[2] = {(cuuint64_t)o.ld * 2, (cuuint64_t)o.rows * o.ld * 2};
-    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
+    cuuint64_t strides[2] = {(cuuint64_t)o.ld * 2, plane};
+    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)tile_rows, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(o.ptr), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Output [splits][M][N] fp32, written in boxes of 32 rows x 32 columns (128-byte swizzle); boxes are clipped at M and N.
+bool make_out_map(CUtensorMap* map, float* c, int M, int N, int splits) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits};
+    cuuint64_t strides[2] = {(cuuint64_t)N * 4, (cuuint64_t)M * N * 4};
+    cuuint32_t box[3] = {32, 32, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, c, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace
 
-int tc_pick_bn(int N) {
-    // widest tile that wastes least: N = 288 -> 96 x 3, 768 -> 256 x 3, 1024.. -> 256
-    int best = 256, best_waste = 1 << 30;
-    for (int bn = 256; bn >= 64; bn -= 32) {
-        const int tiles = (N + bn - 1) / bn;
-        const int waste = tiles * bn - N;
-        if (waste < best_waste) { best_waste = waste; best = bn; }
+// How a product is cut.  Time of a work item in cycles: per k-tile of 64 and term, the larger of 2 BN (MMA) and the shared-
+// memory traffic ((128 + B rows of the CTA) x 128 bytes, written once and read once, at 128 B/clk), plus a fixed part; the
+// launch takes that times the number of waves.  Split-K adds the traffic of its partial sums.  The rule takes the cheapest of
+// one CTA or a pair per tile, tile widths of 64 to 256 and the K splits.
+// Accuracy: tensor-core accumulation into TMEM truncates, and the error of a product of two fp32-split operands grows
+// linearly with the accumulation depth.  `depth_limit` (k-tiles of 64) bounds what one accumulator absorbs; deeper
+// contractions are cut into slices that the reduction kernel adds in fp32 with round-to-nearest.
+TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit) {
+    TcPlan best = {};
+    double best_cost = 1e300;
+    const int ktiles = (K + BK - 1) / BK;
+    const int min_splits = depth_limit > 0 ? (ktiles + depth_limit - 1) / depth_limit : 1;
+    for (int cg = 1; cg <= 2; ++cg) {
+        if (cg == 2 && M <= BM) break;
+        const int tm = (M + cg * BM - 1) / (cg * BM), units = sm_count / cg;
+        for (int bn = 64; bn <= 256; bn += 32) {
+            const int tiles = tm * ((N + bn - 1) / bn);
+            const double cyc = (double)nterms * (2 * bn > 2 * (128 + bn / cg) ? 2 * bn : 2 * (128 + bn / cg));
+            for (int s = min_splits; s <= 64; s = s < 4 ? s + 1 : s * 5 / 4) {
+                if (s > min_splits && (ktiles < 4 * s || tiles * (s - 1) >= 2 * units)) break;
+                const int per = (ktiles + s - 1) / s, real = (ktiles + per - 1) / per;
+                const int waves = (tiles * real + units - 1) / units;
+                double cost = waves * (per * cyc + 500.0) + 12.0 * bn;
+                if (real > 1) cost += ((double)(real + 1) * M * N * 4.0) / 3000.0 + 4000.0;
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per;
+                }
+            }
+        }
     }
+    best.workspace_bytes = best.splits > 1 ? (size_t)best.splits * M * N * sizeof(float) : 0;
     return best;
 }
 
-
-size_t tc_splitk_workspace_bytes(int M, int N, int K, int sm_count, int depth_limit, int* splits_out) {
-    const int bn = tc_pick_bn(N);
-    const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
-    const int ktiles = (K + BK - 1) / BK;
-    int splits = 1;
-    if (tiles < sm_count && ktiles >= 8) {
-        splits = (2 * sm_count + tiles - 1) / tiles;
-        if (splits > ktiles / 4) splits = ktiles / 4;
-        if (splits > 32) splits = 32;
-        if (splits < 1) splits = 1;
-    }
-    // Accuracy: tensor-core accumulation into TMEM truncates, and the error of a product of two
-    // fp32-split operands was measured to grow linearly with the accumulation depth (3e-7 relative
-    // at K = 1024, 6e-6 at K = 16384).  `depth_limit` (k-tiles of 64) bounds what one accumulator
-    // absorbs; deeper contractions are cut into slices that the reduction kernel adds in fp32 with
-    // round-to-nearest.
-    const int lim = depth_limit;
-    if (lim > 0 && (ktiles + splits - 1) / splits > lim) splits = (ktiles + lim - 1) / lim;
-    *splits_out = splits;
-    return splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
-}
-
-cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int ldc, int M, int N, int K,
-                           const float* col_scale, float* splitk_ws, int splits, int* err_word, size_t max_smem,
-                           int sm_count, cudaStream_t stream, int* launches) {
-    if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (N & 3) || (ldc & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
-    const int bn = tc_pick_bn(N), nterms = b.planes == 2 ? 3 : 2;
-    CUtensorMap ma, mb;
-    if (!make_map(&ma, a, a.mn_major ? BK : BM)) return cudaErrorInvalidValue;
-    if (!make_map(&mb, b, b.mn_major ? BK : bn)) return cudaErrorInvalidValue;
+cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int M, int N, int K, const TcPlan& plan,
+                           const float* col_scale, float* splitk_ws, int* err_word, size_t max_smem, int sm_count,
+                           cudaStream_t stream, int* launches) {
+    if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
+    const int bn = plan.bn, cg = plan.pair ? 2 : 1, splits = plan.splits, b_rows = bn / cg;
+    float* out = splits > 1 ? splitk_ws : c;
+    CUtensorMap ma, mb, mc;
+    if (!make_map(&ma, a, BM)) return cudaErrorInvalidValue;
+    if (!make_map(&mb, b, b_rows)) return cudaErrorInvalidValue;
+    if (!make_out_map(&mc, out, M, N, splits)) return cudaErrorInvalidValue;
     TcParams p;
     p.col_scale = col_scale;
     p.M = M; p.N = N; p.K = K;
     p.BN = bn;
     p.a_mn = a.mn_major; p.b_mn = b.mn_major;
     p.a_amax = a.amax; p.b_amax = b.amax;
-    p.b_bytes = (b.mn_major ? (bn + 63) / 64 * 64 : bn) * BK * 2;
-    p.group_m = 12;               // 12 row tiles x 12 column tiles in flight on 148 SMs
+    p.b_bytes = (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
+    p.group_m = 12 / cg;          // 12 row tiles x 12 column tiles in flight on 148 SMs
+    p.nterms = b.planes == 2 ? 3 : 2;
+    p.splits = splits;
+    p.ktiles_per_split = plan.ktiles_per_split;
+    p.err = err_word;
     const size_t stage_bytes = (size_t)kATileBytes + (size_t)p.b_bytes;
-    const int ktiles = (K + BK - 1) / BK;
-    int stages = (int)((max_smem - 2048) / stage_bytes);
+    int stages = (int)((max_smem - 2048 - kStageBytes) / stage_bytes);
     if (stages > kMaxStages) stages = kMaxStages;
-    const int want = nterms * ((ktiles + splits - 1) / splits);   // slots one work item fills
+    const int want = p.nterms * p.ktiles_per_split;   // slots one work item fills
+    const int n_items = ((N + bn - 1) / bn) * ((M + cg * BM - 1) / (cg * BM)) * splits;
     // Two accumulators of one CTA take 2 * pow2(BN) TMEM columns of the SM's 512.  Narrow tiles
     // (BN <= 128) with short main loops leave room for a second resident CTA, which doubles the
     // loads in flight where the loop is latency-bound; then each CTA gets half the shared memory.
     bool two_ctas = false;
-    if (bn <= 128 && want <= 32) {
-        const int half = (int)((((max_smem - 4096) / 2) - 1024) / stage_bytes);
+    if (cg == 1 && bn <= 128 && want <= 32 && n_items > sm_count) {
+        const int half = (int)((((max_smem - 4096) / 2) - 1024 - kStageBytes) / stage_bytes);
         if (half >= 3) { two_ctas = true; if (half < stages) stages = half; }
     }
     if (stages > want) stages = want;
     if (stages < 2) stages = 2;
-    if ((size_t)stages * stage_bytes + 1024 > max_smem) return cudaErrorInvalidConfiguration;
-    if (stages < 2) return cudaErrorInvalidConfiguration;
+    const size_t smem = (size_t)stages * stage_bytes + 1024 + kStageBytes;
+    if (smem > max_smem) return cudaErrorInvalidConfiguration;
     p.stages = stages;
-    p.nterms = nterms;
-    p.splits = splits;
-    p.ktiles_per_split = (ktiles + splits - 1) / splits;
-    // drop empty trailing splits
-    p.splits = splits = (ktiles + p.ktiles_per_split - 1) / p.ktiles_per_split;
-    p.err = err_word;
-    p.C = splits > 1 ? splitk_ws : c;
-    p.ldc = splits > 1 ? N : ldc;
-    const size_t smem = (size_t)stages * stage_bytes + 1024;
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(tc_gemm_kernel), 4, max_smem);
+    const void* kern = cg == 2 ? reinterpret_cast<const void*>(tc_gemm_kernel<2>) : reinterpret_cast<const void*>(tc_gemm_kernel<1>);
+    cudaError_t e = ensure_dynamic_smem(kern, cg == 2 ? kSmemSlotTcPair : 4, max_smem);
     if (e != cudaSuccess) return e;
-    const int n_items = ((N + bn - 1) / bn) * ((M + BM - 1) / BM) * splits;
-    int ctas = sm_count * (two_ctas ? 2 : 1);
-    if (ctas > n_items) ctas = n_items;
-    tc_gemm_kernel<<<ctas, kTcThreads, smem, stream>>>(ma, mb, p);
-    e = cudaGetLastError();
+    int units = (sm_count / cg) * (two_ctas ? 2 : 1);
+    if (units > n_items) units = n_items;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(units * cg));
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cg == 2 ? 1 : 0;
+    e = cg == 2 ? cudaLaunchKernelEx(&cfg, tc_gemm_kernel<2>, ma, mb, mc, p) : cudaLaunchKernelEx(&cfg, tc_gemm_kernel<1>, ma, mb, mc, p);
     if (e != cudaSuccess) return e;
     ++*launches;
     if (splits > 1) {
-        const size_t n4 = (size_t)M * (N / 4);
-        int blocks = (int)((n4 + 255) / 256);
-        if (blocks > 148 * 8) blocks = 148 * 8;
-        splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(splitk_ws, c, col_scale, M, N, ldc, splits);
-        e = cudaGetLastError();
+        e = launch_splitk_reduce(splitk_ws, c, col_scale, M, N, N, splits, stream);
         if (e != cudaSuccess) return e;
         ++*launches;
     }

@@ -63,6 +63,20 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     if (ok) ok = mbar_try_wait(bar, parity);      // completed phase: returns true without waiting
     return __all_sync(0xffffffffu, ok);
 }
+// The same wait with every lane polling (the hardware suspends the warp inside try_wait), for the warps that issue copies and
+// MMAs: no shuffle between the phase change and the issue.
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const unsigned long long t0 = clock64();
+    unsigned spins = 0;
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        if ((++spins & 0x3FFu) == 0) {
+            const bool stop = *abort_flag || clock64() - t0 > kWaitCycles;
+            if (__any_sync(0xffffffffu, stop)) return false;
+        }
+    }
+    return true;
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0,
                                             int c1, int c2) {
     asm volatile(
