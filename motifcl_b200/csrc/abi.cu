@@ -206,6 +206,7 @@ int check_device_error(mcl_cuda_ctx* ctx) {
             case 14: who = "MMA lane (accumulator never drained)"; break;
             case 16: case 17: who = "work-item queue (scheduler lane and its readers lost step)"; break;
             case 21: who = "wide-row counter update (a row slot was never marked ready or released)"; break;
+            case 41: who = "single-layer kernel (a k-tile's MMAs never completed)"; break;
             case 31: who = "peer all-reduce (a rank never announced its partial result)"; break;
             default: who = "epilogue (accumulator never completed)"; break;
         }
@@ -231,6 +232,12 @@ bool tc_wanted(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K, const void
     if (M > 0x7fffffffull / 2 || N > 0x7fffffffull / 2 || K > 0x7fffffffull / 2) return false;
     if (ctx->gemm_mode == MCL_CUDA_GEMM_TENSOR) return true;
     return (double)M * (double)N * (double)K >= (double)(1u << 22);
+}
+
+// one-launch kernels of narrow layers (layer_kernels.cu)
+bool layer_wanted(const mcl_cuda_ctx* ctx, size_t tokens, size_t I, size_t O) {
+    if (ctx->gemm_mode == MCL_CUDA_GEMM_EXACT || !mcl::layer_kernels_fit(tokens, I, O)) return false;
+    return ctx->gemm_mode == MCL_CUDA_GEMM_TENSOR || (double)tokens * (double)I * (double)O >= (double)(1u << 22);
 }
 
 #define MCL_CU(ctx, what, call) do { cudaError_t _e = (call); if (_e != cudaSuccess) return fail_cuda(ctx, what, _e); } while (0)
@@ -503,14 +510,6 @@ int mcl_cuda_counter_pack2(mcl_cuda_ctx* ctx, const uint8_t* state, uint32_t* pa
     return MCL_CUDA_OK;
 }
 
-// defined below, with the grouped step
-static bool fused_wanted(const mcl_cuda_ctx* ctx, const float* x, const float* grad_out, const void* ternary,
-                         const float* scale, const float* y, const float* grad_x, const float* grad_w, size_t I,
-                         size_t O, size_t Nt);
-static int fused_products(mcl_cuda_ctx* ctx, const char* op, const float* x, const float* grad_out,
-                          const uint8_t* state, const uint32_t* packed2, const float* scale, float* y,
-                          float* grad_x, float* grad_w, size_t C, size_t I, size_t O, size_t Nt);
-
 int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* state,
                              const float* scale, float* y, size_t batch, size_t in_features,
                              size_t out_features, size_t C) {
@@ -523,10 +522,11 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
     MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
     MCL_TRY(check_ptr(ctx, op, "y", y, 4));
     DeviceGuard guard(ctx->device);
-    // narrow layers: the tf32 hi/lo kernel reads x in place (no operand-splitting pass)
-    if (tc_wanted(ctx, batch, out_features, in_features, y, scale) &&
-        fused_wanted(ctx, x, nullptr, state, scale, y, nullptr, nullptr, in_features, out_features, batch))
-        return fused_products(ctx, op, x, nullptr, state, nullptr, scale, y, nullptr, nullptr, C, in_features, out_features, batch);
+    if (layer_wanted(ctx, batch, in_features, out_features)) {
+        MCL_LAUNCH(ctx, op, mcl::launch_layer_rows(0, x, state, scale, y, (int)batch, (int)in_features, (int)out_features, (int)C,
+                                                   ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream));
+        return MCL_CUDA_OK;
+    }
     if (tc_wanted(ctx, batch, out_features, in_features, y, scale)) {
         const mcl::TcPlan plan = digit_plan(ctx, batch, out_features, in_features);
         Carver cv;
@@ -560,9 +560,11 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
     MCL_TRY(check_ptr(ctx, op, "grad_out", grad_out, 4));
     MCL_TRY(check_ptr(ctx, op, "grad_x", grad_x, 4));
     DeviceGuard guard(ctx->device);
-    if (tc_wanted(ctx, batch, in_features, out_features, grad_x) &&
-        fused_wanted(ctx, nullptr, grad_out, state, scale, nullptr, grad_x, nullptr, in_features, out_features, batch))
-        return fused_products(ctx, op, nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, C, in_features, out_features, batch);
+    if (layer_wanted(ctx, batch, in_features, out_features)) {
+        MCL_LAUNCH(ctx, op, mcl::launch_layer_rows(1, grad_out, state, scale, grad_x, (int)batch, (int)in_features, (int)out_features, (int)C,
+                                                   ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream));
+        return MCL_CUDA_OK;
+    }
     if (tc_wanted(ctx, batch, in_features, out_features, grad_x)) {
         const mcl::TcPlan plan = digit_plan(ctx, batch, in_features, out_features);
         Carver cv;
@@ -631,6 +633,18 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     MCL_TRY(check_ptr(ctx, op, "state", state, 1));
     if (packed2_out && in_features % 16 != 0)
         return fail(ctx, MCL_CUDA_EINVAL, "counter update: packed2 output requires in_features % 16 == 0");
+    if (layer_wanted(ctx, batch, in_features, out_features) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
+        MCL_TRY(check_ptr(ctx, op, "v", v, 4));
+        if (packed2_out) MCL_TRY(check_ptr(ctx, op, "packed2_out", packed2_out, 4));
+        DeviceGuard guard(ctx->device);
+        mcl::UpdateDesc d;
+        d.state = state; d.scale = scale; d.v = v; d.grad_w = nullptr; d.packed2 = packed2_out;
+        d.in_features = (int)in_features; d.rows = (int)out_features; d.row_offset = 0;
+        MCL_LAUNCH(ctx, op, mcl::launch_layer_update(d, grad_out, x, (int)batch, (int)C, lr, lr_scale, rms_beta, rms_eps, seed, ctx->seed_offset,
+                                                     ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
+        return MCL_CUDA_OK;
+    }
     // Row tile of grad_w: 1/8 of the dense [out,in] gradient, raised to 4 MiB where that is still under 1/5 of the
     // dense gradient (fewer launches for mid-sized layers) and capped at 32 MiB; at least one row; rounded to a multiple
     // of 128 rows when that fits.  The dense gradient is never materialised: the reference's memory-truth gate

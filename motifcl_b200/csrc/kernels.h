@@ -32,6 +32,16 @@ cudaError_t launch_decode_weight(const uint8_t* state, const float* scale, float
 cudaError_t launch_pack2(const uint8_t* state, uint32_t* packed2, int C, int in_features,
                          int out_features, int sm_count, cudaStream_t stream);
 
+// layer_kernels.cu -- one launch per product of a narrow layer, operands converted inside the kernel
+bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features);
+// dx = 0: c[tokens, O] = a (scale T)^T;  dx = 1: c[tokens, I] = (a . scale) T
+cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, const float* scale, float* c, int tokens, int I, int O,
+                              int C, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream);
+// the counter update of a whole layer from its activations (d.grad_w unused, d.row_offset == 0; x 16-byte aligned)
+cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
+                                float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int sm_count,
+                                size_t max_smem, cudaStream_t stream);
+
 // simt_gemm.cu -- fp32 CUDA-core contractions (any shape; exact fp32 FMA accumulation)
 cudaError_t launch_simt_matmul_f32(const float* a, const float* b, float* c, int M, int K, int N,
                                    int transA, int transB, cudaStream_t stream);

@@ -1,0 +1,591 @@
+// Single-layer kernels of narrow counter linears: one launch each for Y, for dX and for the memory-native update.
+//
+// MotifCL's autograd asks for one product of one layer at a time (src/nn/compact_counter.cpp:40-50,158-300), and a layer of a
+// few hundred features is a few microseconds of arithmetic: what a call costs is its launches, its passes over scratch memory
+// and the latency of each.  So the operands are made where they are used: threads load fp32 activations and packed
+// 6-bit codes, split and expand them in registers, and store bf16 tiles straight into the swizzled shared-memory layouts that
+// tcgen05.mma reads.  An fp32 value is three bf16 terms (24 bits: exact up to the smallest exponents); a ternary digit is one.
+//   Y, dX   three products per k (term x digit)
+//   dW      six products per k (terms x terms, those above 2^-24)
+// Tensor-core accumulation truncates in proportion to what the accumulator holds, so the products of leading terms have an
+// accumulator of their own and all smaller ones share a second; the epilogue adds the two in fp32 (one accumulator for
+// all: 1.1e-6 relative error at K = 512).
+// Loads of the next k-tile are in flight while the current one is converted; two shared-memory stages let the tensor core work on
+// one while the threads fill the other.  These kernels are latency-bound (tens of CTAs, a handful of k-tiles each).
+//
+// Every wait on an mbarrier is bounded; on time-out the error word is set and the results are invalid.
+#include <cuda_bf16.h>
+
+#include "counter_codec.cuh"
+#include "counter_update_body.cuh"
+#include "kernels.h"
+#include "tc_ptx.cuh"
+
+namespace mcl {
+namespace {
+
+constexpr int kLThreads = 256;
+constexpr int kErrLayer = 41;
+
+// two fp32 values -> their three bf16 terms, packed two per word
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&t)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        t[i] = *reinterpret_cast<const uint32_t*>(&h);
+        if (i < 2) { a -= __uint_as_float(t[i] << 16); b -= __uint_as_float(t[i] & 0xFFFF0000u); }
+    }
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+__device__ __forceinline__ void sts128u(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// MN-major bf16 tile in the 128-byte swizzle: chunks of 64 MN elements, `chunk` bytes apart, each k rows of 128 bytes
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr, uint32_t chunk) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(chunk >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// kind::f16, D = f32, A = B = bf16, major bits 15 / 16 as given
+__device__ __forceinline__ uint32_t idesc_bf16(int m, int n, uint32_t a_mn, uint32_t b_mn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn << 15) | (b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_peer(uint32_t addr, uint32_t rank) {      // 16 bytes of a cluster peer's shared memory
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+// four consecutive floats of a row of n, zero beyond its end
+__device__ __forceinline__ float4 load4(const float* __restrict__ row, int c, int n, bool vec) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+        if (c < n) v = __ldg(reinterpret_cast<const float4*>(row + c));
+    } else {
+        if (c < n) v.x = __ldg(row + c);
+        if (c + 1 < n) v.y = __ldg(row + c + 1);
+        if (c + 2 < n) v.z = __ldg(row + c + 2);
+        if (c + 3 < n) v.w = __ldg(row + c + 3);
+    }
+    return v;
+}
+__device__ __forceinline__ void tmem_alloc(uint32_t slot_addr, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_addr), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+
+// ---- Y = X (s T)^T and dX = (dY s) T ----------------------------------------------------------------------------
+// CTA = 128 rows x BN columns, k-tiles of 64.  Shared memory per stage: A terms 3 x [128 rows][64 k] (K-major), digits
+// [BN rows][64 k] for Y (K-major) or [64 k][BN] in chunks of 64 columns for dX (MN-major): both are the state's own order.
+struct RowParams {
+    const float* a;           // [M, K]
+    const uint8_t* state;     // [out, in] packed
+    const float* scale;       // [out]
+    float* c;                 // [M, N]
+    int M, N, K, in_features, C;
+    int BN, stage_bytes;
+    int vec;                  // rows of a start on 16-byte boundaries
+    int* err;
+};
+constexpr int kRowATerm = 128 * 128;          // bytes of one A term per stage
+
+template <bool DX>
+__global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ uint32_t tmem_slot, digit[64], lut[4096];
+    __shared__ int abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t stage0 = (smem_u32(smem) + 1023u) & ~1023u;
+    const uint32_t bar0 = smem_u32(bars);
+    const int BN = p.BN, I = p.in_features;
+    const int m0 = blockIdx.x * 128, n0 = blockIdx.y * BN;
+    const bool words = (I & 15) == 0 && (reinterpret_cast<uintptr_t>(p.state) & 3) == 0;     // 16 weights = 3 aligned words
+    uint32_t cols = 32;
+    while ((int)cols < BN) cols <<= 1;
+    if (tid == 0) {
+        mbar_init(bar0, 1); mbar_init(bar0 + 8, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 2 * cols);       // leading terms, smaller terms
+    if (tid < 64) {
+        const __nv_bfloat16 h = __float2bfloat16_rn((float)(tid / (2 * p.C - 1) - 1));
+        digit[tid] = __bfloat16_as_ushort(h);
+    }
+    // A: 8 float4 of a k-tile per thread (row = idx / 16, 4 k each); digits: units of 16 weights, up to BN / 64 per thread
+    float4 a[8];
+    uint32_t w[4][3];
+    const int nkt = (p.K + 63) / 64, nu = 4 * BN;         // units per k-tile: BN rows x 4 (Y) or 64 rows x BN / 16 (dX)
+    auto unit_at = [&](int u, int kt, int& row, int& col) -> bool {      // unit -> state row / first column; false: outside
+        if (DX) { const int per = BN >> 4; row = kt * 64 + u / per; col = n0 + (u % per) * 16; return row < p.K && col < p.N; }
+        row = n0 + (u >> 2); col = kt * 64 + (u & 3) * 16;
+        return row < p.N && col < p.K;
+    };
+    auto load = [&](int kt) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int idx = tid + kLThreads * j, row = m0 + (idx >> 4), k = kt * 64 + (idx & 15) * 4;
+            a[j] = row < p.M ? load4(p.a + (size_t)row * p.K, k, p.K, p.vec != 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int u = tid + kLThreads * j;
+            int row, col;
+            w[j][0] = w[j][1] = w[j][2] = 0;
+            if (u < nu && unit_at(u, kt, row, col)) {
+                const size_t at = ((size_t)row * I + col) / 4 * 3;
+                if (words) {
+                    const uint32_t* s = reinterpret_cast<const uint32_t*>(p.state + at);
+                    w[j][0] = __ldg(s); w[j][1] = __ldg(s + 1); w[j][2] = __ldg(s + 2);
+                } else {
+                    const int nb = min(12, (I - col) / 4 * 3);
+                    for (int b = 0; b < nb; ++b) w[j][b >> 2] |= (uint32_t)__ldg(p.state + at + b) << (8 * (b & 3));
+                }
+            }
+        }
+    };
+    load(0);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    for (int e = tid; e < 4096; e += kLThreads) lut[e] = digit[e & 63] | (digit[e >> 6] << 16);
+    __syncthreads();
+    const uint32_t tmem = tmem_slot;
+    const uint32_t idesc = idesc_bf16(128, BN, 0, DX ? 1u : 0u);
+    bool ok = true;
+    for (int kt = 0; kt < nkt; ++kt) {
+        const int s = kt & 1;
+        const uint32_t st = stage0 + (uint32_t)s * (uint32_t)p.stage_bytes, sb = st + 3u * kRowATerm;
+        if (kt >= 2 && ok) ok = mbar_wait(bar0 + 8u * s, ((uint32_t)(kt >> 1) - 1u) & 1u, &abort_flag);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int idx = tid + kLThreads * j, row = idx >> 4, c4 = idx & 15;
+            float4 v = a[j];
+            if (DX) {                                      // grad_out times the scale of its column, rounded to fp32
+                const int k = kt * 64 + c4 * 4;
+                if (k < p.K) v.x = __fmul_rn(v.x, __ldg(p.scale + k));
+                if (k + 1 < p.K) v.y = __fmul_rn(v.y, __ldg(p.scale + k + 1));
+                if (k + 2 < p.K) v.z = __fmul_rn(v.z, __ldg(p.scale + k + 2));
+                if (k + 3 < p.K) v.w = __fmul_rn(v.w, __ldg(p.scale + k + 3));
+            }
+            uint32_t t0[3], t1[3];
+            split3(v.x, v.y, t0); split3(v.z, v.w, t1);
+            const uint32_t at = st + (uint32_t)row * 128u + (uint32_t)(((c4 >> 1) ^ (row & 7)) << 4) + (uint32_t)((c4 & 1) << 3);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * kRowATerm, t0[t], t1[t]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int u = tid + kLThreads * j;
+            if (u < nu) {
+                int row, col;
+                const bool in = unit_at(u, kt, row, col);
+                uint32_t h[8];
+                const uint32_t g[4] = {w[j][0] & 0xFFFFFFu, (w[j][0] >> 24) | ((w[j][1] & 0xFFFFu) << 8),
+                                       (w[j][1] >> 16) | ((w[j][2] & 0xFFu) << 16), w[j][2] >> 8};
+                const int left = in ? (I - col) >> 2 : 0;   // groups of 4 that exist
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    h[2 * q] = q < left ? lut[g[q] & 4095u] : 0u;
+                    h[2 * q + 1] = q < left ? lut[g[q] >> 12] : 0u;
+                }
+                uint32_t at, x;
+                int c16;
+                if (DX) {
+                    const int per = BN >> 4, kr = u / per, cu = u % per;
+                    at = sb + (uint32_t)(cu >> 2) * 8192u + (uint32_t)kr * 128u; x = (uint32_t)(kr & 7); c16 = 2 * (cu & 3);
+                } else {
+                    at = sb + (uint32_t)(u >> 2) * 128u; x = (uint32_t)((u >> 2) & 7); c16 = 2 * (u & 3);
+                }
+                sts128u(at + (((uint32_t)c16 ^ x) << 4), h[0], h[1], h[2], h[3]);
+                sts128u(at + (((uint32_t)(c16 + 1) ^ x) << 4), h[4], h[5], h[6], h[7]);
+            }
+        }
+        if (kt + 1 < nkt) load(kt + 1);
+        fence_proxy_async();
+        __syncthreads();
+        if (warp == 0) {
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int t = 2; t >= 0; --t) {              // smallest term first
+                    const uint64_t da = smem_desc_k_sw128(st + (uint32_t)t * kRowATerm);
+                    const uint64_t db = DX ? desc_mn(sb, 8192) : smem_desc_k_sw128(sb);
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_bf16(t == 0 ? tmem : tmem + cols, da + 2u * kk, db + (DX ? 128u : 2u) * kk, idesc,
+                                  (kt | kk) != 0 || t == 1 ? 1u : 0u);
+                }
+                umma_commit(bar0 + 8u * s);
+            }
+            __syncwarp();
+        }
+    }
+    if (ok) ok = mbar_wait(bar0 + 8u * ((nkt - 1) & 1), (uint32_t)((nkt - 1) >> 1) & 1u, &abort_flag);
+    if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
+    tc_fence_after();
+    // epilogue: warp = 32 rows x half of the columns; a 32 x 33 tile in shared memory turns lane = row into lane = column
+    {
+        const int q = warp & 3, half = warp >> 2;
+        float* tile = reinterpret_cast<float*>(smem) + warp * 32 * 33;
+        for (int c0 = half * 32; c0 < BN && n0 + c0 < p.N; c0 += 64) {
+            uint32_t r[32], r1[32];
+            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)c0, r1);
+            tmem_ld_wait();
+            const int col = n0 + c0 + lane;
+            const float sc = !DX && col < p.N ? __ldg(p.scale + col) : 1.0f;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = __uint_as_float(r[j]) + __uint_as_float(r1[j]);
+            __syncwarp();
+            const int rows = min(32, p.M - m0 - q * 32);
+            if (col < p.N) {
+                float* out = p.c + (size_t)(m0 + q * 32) * p.N + col;
+#pragma unroll 8
+                for (int i = 0; i < rows; ++i) out[(size_t)i * p.N] = DX ? tile[i * 33 + lane] : tile[i * 33 + lane] * sc;
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * cols) : "memory");
+}
+
+// ---- memory-native update: dW = dY^T X of 128 rows in tensor memory, then the counter update, in one launch ----------------
+// A cluster of CTAs owns 128 rows of the layer; each CTA contracts a slice of the tokens into its own tensor memory (all
+// columns of the rows, in passes of up to 256).  The slices are added through distributed shared memory, 128 columns at a
+// time: every CTA publishes its partial tile, then sums its share of the rows over all CTAs in rank order (deterministic) into its
+// own shared memory, where the update runs on whole rows.  grad_w never exists outside the chip.
+struct LayerUpdParams {
+    const float* dy;          // [tokens, O]
+    const float* x;           // [tokens, I]
+    int tokens, O, slice;     // slice: tokens per CTA, a multiple of 16
+    int np, pw;               // passes over the columns and their width (a multiple of 64, at most 256)
+    int off_stage, stage_bytes;
+    int vec_dy;
+    uint32_t magic;
+    int* err;
+    UpdParams u;              // of the whole layer; rows_per_batch = rows of a CTA
+};
+constexpr int kDwK = 16;                      // tokens per k-tile: one MMA step
+constexpr int kDwChunk = kDwK * 128;          // bytes of 64 columns x 16 tokens
+constexpr int kDwATerm = 2 * kDwChunk;
+
+// the update for in_features % 16 != 0: groups of four weights read and written as bytes
+template <bool WITH_Q>
+__device__ __forceinline__ void update_rows_by_group(const UpdParams& p, const int nrows, unsigned char* smem, const U16Layout& L) {
+    DecodeLut* lut = reinterpret_cast<DecodeLut*>(smem);
+    RowK* rowc = reinterpret_cast<RowK*>(smem + L.off_rowc);
+    float* part = reinterpret_cast<float*>(smem + L.off_part);
+    const float4* gw_s = reinterpret_cast<const float4*>(smem + L.off_gw);
+    const int tid = threadIdx.x, lane = tid & 31, pair = tid >> 6, vlane = tid & 63;
+    const int I = p.in_features, gpr = I >> 2, lv = 2 * p.C - 1;
+    const uint32_t seed = p.seed + (p.seed_offset ? __ldg(p.seed_offset) : 0u);
+    auto group = [&](int r, int g) -> uint32_t {
+        const uint8_t* s = p.state + ((size_t)r * gpr + g) * 3;
+        return (uint32_t)s[0] | ((uint32_t)s[1] << 8) | ((uint32_t)s[2] << 16);
+    };
+    build_decode_lut(lut, p.C, tid, kLThreads);
+    __syncthreads();
+    for (int r = pair; r < nrows; r += kPairs) {
+        float a = 0.0f, b = 0.0f;
+        for (int g = vlane; g < gpr; g += 64) {
+            const float4 gw = gw_s[r * gpr + g];
+            a = __fadd_rn(a, __fmul_rn(gw.x, gw.x)); a = __fadd_rn(a, __fmul_rn(gw.y, gw.y));
+            a = __fadd_rn(a, __fmul_rn(gw.z, gw.z)); a = __fadd_rn(a, __fmul_rn(gw.w, gw.w));
+            if (WITH_Q) {
+                const uint32_t w = group(r, g);
+                b = __fadd_rn(b, __fmul_rn(gw.x, lut->e[w & 63u].x)); b = __fadd_rn(b, __fmul_rn(gw.y, lut->e[(w >> 6) & 63u].x));
+                b = __fadd_rn(b, __fmul_rn(gw.z, lut->e[(w >> 12) & 63u].x)); b = __fadd_rn(b, __fmul_rn(gw.w, lut->e[(w >> 18) & 63u].x));
+            }
+        }
+        if (vlane >= 32) { part[pair * 64 + lane] = a; part[pair * 64 + 32 + lane] = b; }
+        asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
+        if (vlane < 32) {
+            a = __fadd_rn(a, part[pair * 64 + lane]); b = __fadd_rn(b, part[pair * 64 + 32 + lane]);
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) {
+                a = __fadd_rn(a, __shfl_down_sync(0xffffffffu, a, s)); b = __fadd_rn(b, __shfl_down_sync(0xffffffffu, b, s));
+            }
+            if (lane == 0) rowc[r] = finish_row_stats<WITH_Q>(p, r, a, b, (float)p.C, p.scale[r], p.v[r]);
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
+    }
+    __syncthreads();
+    for (int i = tid; i < nrows * gpr; i += kLThreads) {
+        const int r = i / gpr, g = i - r * gpr;
+        const RowK rc = rowc[r];
+        const float4 gw = gw_s[i];
+        const float gv[4] = {gw.x, gw.y, gw.z, gw.w};
+        const uint32_t w = group(r, g), e0 = (uint32_t)(p.row_offset + r) * (uint32_t)I + 4u * (uint32_t)g;
+        uint32_t nw = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 tc = lut->e[(w >> (6 * k)) & 63u];
+            uint32_t fld;
+            nw |= (counter_tick(gv[k], tc.x, tc.y, e0 + (uint32_t)k, seed, -p.lr, rc.dn, rc.k_tick, rc.k_reb, (float)p.C, p.C, lv, &fld) & 0x3Fu) << (6 * k);
+        }
+        uint8_t* s = p.state + (size_t)i * 3;
+        s[0] = (uint8_t)nw; s[1] = (uint8_t)(nw >> 8); s[2] = (uint8_t)(nw >> 16);
+    }
+}
+
+template <bool WITH_Q, bool U16>
+__global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid_constant__ LayerUpdParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    uint32_t cs;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cs));
+    const int rank = (int)cluster_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int I = p.u.in_features, gpr = I >> 2, R = p.u.rows_per_batch;
+    const U16Layout L = u16_layout(I, R, WITH_Q);
+    const int m0 = ((int)blockIdx.x / (int)cs) * 128;
+    const int valid = min(128, p.O - m0), rpc = (valid + (int)cs - 1) / (int)cs;
+    const int my_row0 = rank * rpc, my_rows = max(0, min(rpc, valid - my_row0));
+    const int t0 = rank * p.slice, t1 = min(p.tokens, t0 + p.slice);
+    const int nkt = t1 > t0 ? (t1 - t0 + kDwK - 1) / kDwK : 0;
+    const uint32_t stage0 = ((smem_u32(smem) + 1023u) & ~1023u) + (uint32_t)p.off_stage;
+    const uint32_t bar0 = smem_u32(bars);
+    float4* gw_s = reinterpret_cast<float4*>(smem + L.off_gw);
+    uint32_t cols = 32;
+    while ((int)cols < p.pw) cols <<= 1;
+    if (tid == 0) {
+        mbar_init(bar0, 1); mbar_init(bar0 + 8, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 2 * cols);       // leading products, smaller products
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    bool ok = true;
+    int it = 0;                                   // k-tiles so far: stage = it & 1
+    for (int pass = 0; pass < p.np; ++pass) {
+        const int n0 = pass * p.pw, nw = min(p.pw, I - n0), nwp = (nw + 15) & ~15, per = nwp >> 2;
+        const uint32_t bterm = (uint32_t)((nwp + 63) / 64) * kDwChunk;
+        // this thread's float4s of a k-tile: 2 of dY (128 columns), up to 4 of x
+        float4 a[2], b[4];
+        int brow[4], bcol[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int idx = tid + kLThreads * j;
+            brow[j] = idx < kDwK * per ? idx / per : -1;
+            bcol[j] = 4 * (idx % per);
+        }
+        auto load = [&](int kt) {
+            const int tb = t0 + kt * kDwK;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int idx = tid + kLThreads * j, t = tb + (idx >> 5);
+                a[j] = t < t1 ? load4(p.dy + (size_t)t * p.O, m0 + (idx & 31) * 4, p.O, p.vec_dy != 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = tb + brow[j];
+                b[j] = brow[j] >= 0 && t < t1 ? load4(p.x + (size_t)t * I, n0 + bcol[j], I, true) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        if (nkt > 0) load(0);
+        for (int kt = 0; kt < nkt; ++kt, ++it) {
+            const uint32_t st = stage0 + (uint32_t)(it & 1) * (uint32_t)p.stage_bytes, sb = st + 3u * kDwATerm;
+            if (it >= 2 && ok) ok = mbar_wait(bar0 + 8u * (it & 1), ((uint32_t)(it >> 1) - 1u) & 1u, &abort_flag);
+            auto put = [&](uint32_t base, uint32_t term, int row, int col, float4 v) {     // four columns of one token, three terms
+                uint32_t u0[3], u1[3];
+                split3(v.x, v.y, u0); split3(v.z, v.w, u1);
+                const uint32_t at = base + (uint32_t)(col >> 6) * kDwChunk + (uint32_t)row * 128u +
+                                    (uint32_t)((((col & 63) >> 3) ^ (row & 7)) << 4) + (uint32_t)((col & 4) << 1);
+#pragma unroll
+                for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * term, u0[t], u1[t]);
+            };
+#pragma unroll
+            for (int j = 0; j < 2; ++j) { const int idx = tid + kLThreads * j; put(st, kDwATerm, idx >> 5, (idx & 31) * 4, a[j]); }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (brow[j] >= 0) put(sb, bterm, brow[j], bcol[j], b[j]);
+            if (kt + 1 < nkt) load(kt + 1);
+            fence_proxy_async();
+            __syncthreads();
+            if (warp == 0) {
+                tc_fence_after();
+                if (elect_one()) {
+                    // terms: 0 = hi .. 2 = lo, smallest products first
+                    const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+                    for (int q = 0; q < 6; ++q) {
+                        umma_bf16(q == 5 ? tmem : tmem + cols, desc_mn(st + (uint32_t)pa[q] * kDwATerm, kDwChunk),
+                                  desc_mn(sb + (uint32_t)pb[q] * bterm, kDwChunk), idesc_bf16(128, nwp, 1, 1), kt != 0 || (q > 0 && q < 5) ? 1u : 0u);
+                    }
+                    umma_commit(bar0 + 8u * (it & 1));
+                }
+                __syncwarp();
+            }
+        }
+        if (it > 0 && ok) ok = mbar_wait(bar0 + 8u * ((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, &abort_flag);
+        tc_fence_after();
+        // sum over the cluster, 128 columns at a time; the exchange tile lies over the (finished) stages
+        for (int c0 = 0; c0 < nw; c0 += 128) {
+            const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int cc = half * 64 + h * 32;
+                if (c0 + cc < nw) {
+                    uint32_t r[32], r1[32];
+                    if (nkt > 0) {
+                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + cc), r);
+                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)(c0 + cc), r1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = 0;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        sts128u(stage0 + (uint32_t)row * 512u + (uint32_t)(((cc >> 2) + j) ^ (row & 7)) * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                }
+            }
+            tc_fence_before();
+            cluster_sync_all();
+            for (int i = tid; i < my_rows * 32; i += kLThreads) {
+                const int r = i >> 5, c = i & 31, g = ((n0 + c0) >> 2) + c;
+                if (c0 + 4 * c < nw) {
+                    const int mr = my_row0 + r;
+                    const uint32_t at = stage0 + (uint32_t)mr * 512u + (uint32_t)(c ^ (mr & 7)) * 16u;
+                    float4 sum = ld_peer(at, 0);
+                    for (uint32_t k = 1; k < cs; ++k) {
+                        const float4 v = ld_peer(at, k);
+                        sum.x = __fadd_rn(sum.x, v.x); sum.y = __fadd_rn(sum.y, v.y);
+                        sum.z = __fadd_rn(sum.z, v.z); sum.w = __fadd_rn(sum.w, v.w);
+                    }
+                    gw_s[r * gpr + (U16 ? swz4(g) : g)] = sum;
+                }
+            }
+            cluster_sync_all();
+            tc_fence_after();
+        }
+    }
+    if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * cols) : "memory");
+    if (my_rows == 0) return;
+    UpdParams u = p.u;
+    const int row = m0 + my_row0;
+    u.state += (size_t)row * gpr * 3;
+    u.scale += row; u.v += row;
+    if (u.packed2) u.packed2 += (size_t)row * (I >> 4);
+    u.rows = my_rows; u.row_offset = row;
+    if (U16) update_u16_body<WITH_Q, true>(u, p.magic, 1u << 16, 1u << 17, 0, 1, true);
+    else update_rows_by_group<WITH_Q>(u, my_rows, smem, L);
+}
+
+}  // namespace
+
+bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features) {
+    // A row kernel converts its activations once per column tile and the update converts x once per 128 output rows: beyond
+    // these widths the terms split once by tc_gemm.cu are cheaper.
+    return in_features % 4 == 0 && in_features <= 1024 && out_features <= 2048 && tokens <= (1u << 20);
+}
+
+cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, const float* scale, float* c, int tokens, int I, int O,
+                              int C, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream) {
+    RowParams p;
+    p.a = a; p.state = state; p.scale = scale; p.c = c;
+    p.M = tokens; p.N = dx ? I : O; p.K = dx ? O : I; p.in_features = I; p.C = C;
+    p.vec = (p.K & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
+    p.err = err_word;
+    // column tile: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per column)
+    const int tm = (tokens + 127) / 128;
+    double best = 1e30;
+    for (int bn = 32; bn <= 256; bn += 32) {
+        const int tiles = tm * ((p.N + bn - 1) / bn), nkt = (p.K + 63) / 64;
+        const double cost = (double)((tiles + sm_count - 1) / sm_count) * (nkt * (900.0 + 5.0 * bn) + 4000.0 + 6.0 * bn);
+        if (cost < best) { best = cost; p.BN = bn; }
+    }
+    p.stage_bytes = 3 * kRowATerm + (dx ? (p.BN + 63) / 64 * 8192 : p.BN * 128);
+    const size_t smem = 2 * (size_t)p.stage_bytes + 1024;
+    const void* kern = dx ? reinterpret_cast<const void*>(layer_rows_kernel<true>) : reinterpret_cast<const void*>(layer_rows_kernel<false>);
+    cudaError_t e = ensure_dynamic_smem(kern, dx ? 18 : 17, max_smem);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned)tm, (unsigned)((p.N + p.BN - 1) / p.BN));
+    if (dx) layer_rows_kernel<true><<<grid, kLThreads, smem, stream>>>(p);
+    else layer_rows_kernel<false><<<grid, kLThreads, smem, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
+                                float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int sm_count,
+                                size_t max_smem, cudaStream_t stream) {
+    const int I = d.in_features, O = d.rows, tiles = (O + 127) / 128;
+    const bool with_q = lr_scale != 0.0f;
+    const bool u16 = I % 16 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 3) == 0;
+    auto kern = u16 ? (with_q ? layer_update_kernel<true, true> : layer_update_kernel<false, true>)
+                    : (with_q ? layer_update_kernel<true, false> : layer_update_kernel<false, false>);
+    const int slot = 20 + (u16 ? 2 : 0) + (with_q ? 1 : 0);
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), slot, max_smem);
+    if (e != cudaSuccess) return e;
+    // CTAs per 128 rows: 8 (portable), or 16 while all of them fit the device at once
+    for (int cs = tiles * 16 <= sm_count * 3 / 4 ? 16 : 8;; cs = 8) {
+        LayerUpdParams p;
+        const int R = 128 / cs;
+        const size_t base = (u16_layout(I, R, with_q).total + 1023) & ~size_t(1023);
+        size_t smem = 0;
+        for (p.np = 1; p.np <= 16; ++p.np) {
+            p.pw = ((I + p.np - 1) / p.np + 63) / 64 * 64;
+            p.stage_bytes = 3 * kDwATerm + 3 * (p.pw / 64) * kDwChunk;
+            const size_t area = 2 * (size_t)p.stage_bytes > 65536 ? 2 * (size_t)p.stage_bytes : 65536;
+            smem = base + area + 1024;
+            if (p.pw <= 256 && smem + 1024 <= max_smem) break;
+        }
+        if (p.np > 16) return cudaErrorInvalidConfiguration;
+        p.off_stage = (int)base;
+        p.dy = dy; p.x = x; p.tokens = tokens; p.O = O;
+        p.slice = ((tokens + cs - 1) / cs + kDwK - 1) / kDwK * kDwK;
+        p.vec_dy = (O & 3) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
+        const uint32_t upr = (uint32_t)(I / 16);
+        p.magic = upr <= 1 ? 0u : (uint32_t)((0x100000000ull + upr - 1) / upr);
+        p.err = err_word;
+        UpdParams& u = p.u;
+        u.state = d.state; u.scale = d.scale; u.v = d.v; u.grad_w = nullptr; u.packed2 = d.packed2;
+        u.C = C; u.in_features = I; u.rows = O; u.row_offset = 0; u.rows_per_batch = R;
+        u.state_align = (I % 64 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 15) == 0 && (reinterpret_cast<uintptr_t>(d.packed2) & 15) == 0) ? 16 : 4;
+        u.lr = lr; u.lr_scale = lr_scale; u.rms_beta = rms_beta; u.rms_eps = rms_eps; u.seed = seed; u.seed_offset = seed_offset;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(tiles * cs));
+        cfg.blockDim = dim3(kLThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cs == 16) {
+            // asked once per kernel and device: a part whose GPCs cannot hold 16 such CTAs keeps clusters of 8
+            static int fits[64][4] = {};                  // 0 unknown, 1 yes, 2 no
+            int dev = 0;
+            cudaGetDevice(&dev);
+            int& f = fits[dev & 63][slot - 20];
+            if (f == 0) {
+                int n = 0;
+                cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                f = cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kern), &cfg) == cudaSuccess && n >= 4 ? 1 : 2;
+                cudaGetLastError();
+            }
+            if (f == 2) continue;
+        }
+        return cudaLaunchKernelEx(&cfg, kern, p);
+    }
+}
+
+}  // namespace mcl

@@ -93,20 +93,20 @@ __device__ __forceinline__ uint32_t idesc_tf32(int m, int n, bool a_mn, bool b_m
 // 32-bit data from): 4 k-rows per 512 bytes (stride byte offset), the next 32 m one box = 4096 bytes
 // further (leading byte offset).
 // tf32 MMA with the A operand in tensor memory: row m of the tile = TMEM lane m, one tf32 per 32-bit column
-__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
+__device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_c, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accum) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_c), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accum) : "memory");
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_c), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
 }
 // kind::f16 (bf16 operands, two per 32-bit TMEM column for A), A in tensor memory
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_c, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accum) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_c), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accum) : "memory");
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n\t}"
+        ::"r"(tmem_c), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
 }
 // Instruction descriptor, kind::f16: D = f32, A = B = bf16 (1 at bits 7 and 10), both K-major
 __device__ __forceinline__ uint32_t idesc_bf16_k(int m, int n) {
@@ -311,128 +311,75 @@ __global__ void __launch_bounds__(kFThreads, 1) tc_fused_kernel(const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer ------------------------------------------------------------------------
-            uint32_t it = 0, n_local = 0, rs = 0;
-            int pi = 0;
-            for (;;) {
-                int item = n_items;
-                {   // single-lane form of next_from_queue
-                    const int s = (int)(q_seq % kQueue);
-                    if (mbar_wait(q_full(s), (q_seq / kQueue) & 1u, &abort_flag)) {
-                        item = *reinterpret_cast<volatile int*>(&queue_item[s]);
-                        mbar_arrive(q_empty(s));
-                    } else { abort_flag = 1; atomicExch(err, 16); }
-                    ++q_seq;
-                }
-                if (item >= n_items || abort_flag) break;
-                const Item I = decode_item(sp, n_problems, item, pi);
-                const FusedProblem& P = sp[I.pi];
-                const bool bf = is_bf16_mode(P.mode);
-                const bool b_mn = P.mode != kFusedY;
-                const uint32_t idesc = bf ? idesc_bf16_k(128, P.BN) : idesc_tf32(128, P.BN, false, b_mn);
-                // B descriptor words: low = address / 16 | leading byte offset / 16 << 16, high = stride byte offset / 16 |
-                // version bit | layout type << 29 (1 = 128-byte swizzle with 32-byte atoms, 2 = 128-byte swizzle)
-                const uint32_t b_step = b_mn ? 64u : 2u;                                    // 16-byte units per 8 k
-                const uint32_t b_lo = b_mn ? ((uint32_t)(kBox >> 4) << 16) : (1u << 16);
-                const uint32_t b_hi = b_mn ? ((512u >> 4) | (1u << 14) | (1u << 29)) : ((1024u >> 4) | (1u << 14) | (2u << 29));
-                const uint32_t nprod = (uint32_t)P.nprod, prod0 = P.prod;
-                if (P.flush <= 0) {
-                // ---- the whole item in one accumulator ----
+        // ---- MMA issuer: the warp runs converged, one elected lane issues --------------------------------
+        uint32_t n_local = 0;
+        int rs = 0, sl = 0, pi = 0;
+        uint32_t lph = 0;
+        for (;;) {
+            const int item = next_from_queue();
+            if (item >= n_items || abort_flag) break;
+            const Item I = decode_item(sp, n_problems, item, pi);
+            const FusedProblem& P = sp[I.pi];
+            const int mode = P.mode;
+            const bool bf = is_bf16_mode(mode);
+            const bool b_mn = mode != kFusedY;
+            const uint32_t idesc = bf ? idesc_bf16_k(128, P.BN) : idesc_tf32(128, P.BN, false, b_mn);
+            // B descriptor words: low = address / 16 | leading byte offset / 16 << 16, high = stride byte offset / 16 |
+            // version bit | layout type << 29 (1 = 128-byte swizzle with 32-byte atoms, 2 = 128-byte swizzle)
+            const uint32_t b_step = b_mn && !bf ? 64u : 2u;                             // 16-byte units per instruction
+            const uint32_t b_lo = b_mn && !bf ? ((uint32_t)(kBox >> 4) << 16) : (1u << 16);
+            const uint32_t b_hi = b_mn && !bf ? ((512u >> 4) | (1u << 14) | (1u << 29)) : ((1024u >> 4) | (1u << 14) | (2u << 29));
+            const uint32_t nprod = (uint32_t)P.nprod, prod0 = P.prod;
+            const uint32_t b_at = (bf ? 2u : 1u) * (uint32_t)kABytes;
+            // An accumulator takes at most P.flush k-tiles (0: the whole item): tensor-core accumulation truncates, and the
+            // error grows with the number of instructions that add into one accumulator.  A long item hands its accumulator to
+            // the epilogue every P.flush k-tiles and goes on in the other one; the epilogue adds the pieces in fp32.
+            const int flush = P.flush > 0 ? P.flush : I.nkt, nkt = I.nkt;
+            bool ok = true;
+            for (int j0 = 0; j0 < nkt && ok; j0 += flush, ++n_local) {
+                const int j1 = min(nkt, j0 + flush);
                 const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
-                if (!mbar_wait(acc_empty(acc), aph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(err, 14); break; }
+                ok = mbar_wait_all(acc_empty(acc), aph ^ 1u, &abort_flag);
+                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(err, 14); break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * kAccStride;
-                uint32_t accum = 0;
-                for (int j = 0; j < I.nkt; ++j, ++it) {
-                    const int s = (int)rs, sl = (int)(it % kLoSlots);
-                    if (++rs == (uint32_t)n_raw) rs = 0;
-                    const uint32_t hi16 = (raw0 + (uint32_t)s * raw_slot + (bf ? 2u : 1u) * (uint32_t)kABytes) >> 4;     // B as TMA delivered it
+                for (int j = j0; j < j1; ++j) {
+                    const uint32_t hi16 = (raw0 + (uint32_t)rs * raw_slot + b_at) >> 4;                 // B as TMA delivered it
                     const uint32_t lo16 = (lo0 + (uint32_t)sl * lo_slot) >> 4;                          // B lo
                     const uint32_t a_tm = tmem_base + a_col(sl);                                        // A hi, A lo at +32
                     // the converters arrive after they have seen the raw tile, so this wait covers the copies as well
-                    if (!mbar_wait(lo_full(sl), (it / kLoSlots) & 1u, &abort_flag)) { abort_flag = 1; atomicExch(err, 12); break; }
+                    ok = mbar_wait_all(lo_full(sl), lph, &abort_flag);
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(err, 12); break; }
                     tc_fence_after();
-                    uint32_t prod = prod0;
-                    if (bf) {
-                        // the ternary tile is K-major bf16 in the 128-byte swizzle (rows of 64 k); A terms: hi, lo
-                        const uint64_t db0 = smem_desc_k_sw128(hi16 << 4);
+                    const uint32_t first = j != j0 ? 1u : 0u;
+                    if (elect_one()) {
+                        if (bf) {
+                            // the ternary tile is K-major bf16 in the 128-byte swizzle (rows of 64 k); A terms: hi, lo
 #pragma unroll
-                        for (uint32_t t = 0; t < 2; ++t)
+                            for (uint32_t t = 0; t < 2; ++t)
 #pragma unroll
-                            for (uint32_t kk = 0; kk < 4; ++kk) {
-                                umma_bf16_ts(d_tmem, a_tm + 32u * t + kk * 8u, db0 + 2u * kk, idesc, accum);
-                                accum = 1u;
+                                for (uint32_t kk = 0; kk < 4; ++kk)
+                                    umma_bf16_ts(d_tmem, a_tm + 32u * t + kk * 8u, (b_lo | hi16) + 2u * kk, b_hi, idesc, (t | kk) ? 1u : first);
+                        } else {
+                            uint32_t prod = prod0;
+                            for (uint32_t q = 0; q < nprod; ++q, prod >>= 4) {
+                                const uint32_t a_t = a_tm + ((prod & 3u) ? 32u : 0u);
+                                const uint32_t b16 = b_lo | (((prod >> 2) & 3u) ? lo16 : hi16);
+#pragma unroll
+                                for (uint32_t kk = 0; kk < 4; ++kk)
+                                    umma_tf32_ts(d_tmem, a_t + kk * 8u, b16 + kk * b_step, b_hi, idesc, (q | kk) ? 1u : first);
                             }
-                    } else
-                    for (uint32_t q = 0; q < nprod; ++q, prod >>= 4) {
-                        const uint32_t a_t = a_tm + ((prod & 3u) ? 32u : 0u);
-                        const uint32_t b16 = b_lo | (((prod >> 2) & 3u) ? lo16 : hi16);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) {
-                            const uint64_t db = ((uint64_t)b_hi << 32) | (uint64_t)(b16 + kk * b_step);
-                            umma_tf32_ts(d_tmem, a_t + kk * 8u, db, idesc, accum);
-                            accum = 1u;
                         }
+                        umma_commit(raw_empty(rs));
+                        umma_commit(lo_empty(sl));
+                        if (j == j1 - 1) umma_commit(acc_full(acc));
                     }
-                    umma_commit(raw_empty(s));
-                    umma_commit(lo_empty(sl));
+                    __syncwarp();
+                    if (++rs == n_raw) rs = 0;
+                    if (++sl == kLoSlots) { sl = 0; lph ^= 1u; }
                 }
-                if (abort_flag) break;
-                umma_commit(acc_full(acc));
-                ++n_local;
-                } else {
-                // An accumulator takes at most P.flush k-tiles (tensor-core accumulation truncates, and the error grows
-                // with the number of instructions that add into one accumulator): a long item hands its accumulator to
-                // the epilogue every P.flush k-tiles and goes on in the other one; the epilogue adds the pieces in fp32.
-                const int flush = P.flush > 0 ? P.flush : I.nkt;
-                for (int j0 = 0; j0 < I.nkt && !abort_flag; j0 += flush, ++n_local) {
-                const int j1 = min(I.nkt, j0 + flush);
-                const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
-                if (!mbar_wait(acc_empty(acc), aph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(err, 14); break; }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * kAccStride;
-                uint32_t accum = 0;
-                for (int j = j0; j < j1; ++j, ++it) {
-                    const int s = (int)rs, sl = (int)(it % kLoSlots);
-                    if (++rs == (uint32_t)n_raw) rs = 0;
-                    const uint32_t hi16 = (raw0 + (uint32_t)s * raw_slot + (bf ? 2u : 1u) * (uint32_t)kABytes) >> 4;     // B as TMA delivered it
-                    const uint32_t lo16 = (lo0 + (uint32_t)sl * lo_slot) >> 4;                          // B lo
-                    const uint32_t a_tm = tmem_base + a_col(sl);                                        // A hi, A lo at +32
-                    // the converters arrive after they have seen the raw tile, so this wait covers the copies as well
-                    if (!mbar_wait(lo_full(sl), (it / kLoSlots) & 1u, &abort_flag)) { abort_flag = 1; atomicExch(err, 12); break; }
-                    tc_fence_after();
-                    uint32_t prod = prod0;
-                    if (bf) {
-                        // the ternary tile is K-major bf16 in the 128-byte swizzle (rows of 64 k); A terms: hi, lo
-                        const uint64_t db0 = smem_desc_k_sw128(hi16 << 4);
-#pragma unroll
-                        for (uint32_t t = 0; t < 2; ++t)
-#pragma unroll
-                            for (uint32_t kk = 0; kk < 4; ++kk) {
-                                umma_bf16_ts(d_tmem, a_tm + 32u * t + kk * 8u, db0 + 2u * kk, idesc, accum);
-                                accum = 1u;
-                            }
-                    } else
-                    for (uint32_t q = 0; q < nprod; ++q, prod >>= 4) {
-                        const uint32_t a_t = a_tm + ((prod & 3u) ? 32u : 0u);
-                        const uint32_t b16 = b_lo | (((prod >> 2) & 3u) ? lo16 : hi16);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) {
-                            const uint64_t db = ((uint64_t)b_hi << 32) | (uint64_t)(b16 + kk * b_step);
-                            umma_tf32_ts(d_tmem, a_t + kk * 8u, db, idesc, accum);
-                            accum = 1u;
-                        }
-                    }
-                    umma_commit(raw_empty(s));
-                    umma_commit(lo_empty(sl));
-                }
-                if (abort_flag) break;
-                umma_commit(acc_full(acc));
-                }
-                }
-                if (abort_flag) break;
             }
+            if (abort_flag) break;
         }
     } else if (warp == 2) {
         if (lane == 0) {

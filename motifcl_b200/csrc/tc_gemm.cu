@@ -67,13 +67,6 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// One lane of a converged warp.  The lanes that issue copies and MMAs run their loops with the whole warp and branch here
-// only around the instructions themselves: addresses and descriptors are then warp-uniform for the compiler.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t e;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-    return e != 0;
-}
 // D = A.B + (accum ? D : 0), and D = A.B + D 2^-12; descriptors as low and high words; CG = 2: issued by the pair's leader for
 // both CTAs
 template <int CG>

@@ -77,6 +77,13 @@ __device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, vol
     }
     return true;
 }
+// One lane of a converged warp.  The lanes that issue copies and MMAs run their loops with the whole warp and branch here
+// only around the instructions themselves: addresses and descriptors are then warp-uniform for the compiler.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0,
                                             int c1, int c2) {
     asm volatile(

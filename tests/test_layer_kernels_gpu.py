@@ -1,0 +1,66 @@
+"""Single-layer kernels of narrow layers (motifcl_b200/csrc/layer_kernels.cu) at the edges of their tiles: rows around 128,
+columns around the tile widths, in_features that are no multiple of 16 or 64, token counts below one slice per CTA."""
+import numpy as np
+import pytest
+import torch
+
+from motifcl_b200 import synth
+
+pytestmark = pytest.mark.gpu
+SHAPES = [(16, 64, 32), (33, 68, 37), (127, 288, 288), (257, 108, 130), (300, 512, 96), (129, 1024, 200), (1000, 1020, 129), (2050, 80, 1536)]
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from motifcl_b200 import Context
+    c = Context.on_torch_stream(0)
+    c.set_gemm_mode("tensor")
+    yield c
+    c.close()
+
+
+def _layer(N, I, O, seed):
+    rng = np.random.default_rng(seed)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    return (dev(synth.counters(77, seed, O, I).reshape(-1)), dev(rng.uniform(0.02, 0.2, O).astype(np.float32)),
+            dev(rng.uniform(1e-4, 1e-2, O).astype(np.float32)), dev(rng.standard_normal((N, I)).astype(np.float32)),
+            dev((rng.standard_normal((N, O)) * 0.02).astype(np.float32)))
+
+
+@pytest.mark.parametrize("N,I,O", SHAPES)
+def test_row_products_against_float64(ctx, N, I, O):
+    st, sc, _, x, dy = _layer(N, I, O, N + I + O)
+    w = torch.empty(O, I, device="cuda")
+    ctx.counter_decode_weight(st, torch.ones_like(sc), w, I, O, 11)
+    y, dx = torch.full((N, O), 7.0, device="cuda"), torch.full((N, I), 7.0, device="cuda")
+    ctx.counter_forward(x, st, sc, y, N, I, O, 11)
+    ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+    ctx.finish()
+    ry = (x.double() @ w.double().T) * sc.double()
+    rdx = (dy * sc).double() @ w.double()
+    assert float((y - ry).norm() / ry.norm()) < 1e-6
+    assert float((dx - rdx).norm() / rdx.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("lr_scale", [0.0, 1e-3])
+@pytest.mark.parametrize("N,I,O", SHAPES)
+def test_update_against_the_exact_path(ctx, N, I, O, lr_scale):
+    res = []
+    for mode in ("tensor", "exact"):
+        st, sc, v, x, dy = _layer(N, I, O, N + I + O)
+        p2 = torch.zeros(O, I // 16, dtype=torch.int32, device="cuda") if I % 16 == 0 else None
+        ctx.set_gemm_mode(mode)
+        try:
+            ctx.counter_update_fused(st, sc, v, dy, x, p2, 11, I, O, N, 3e-3, lr_scale, 0.9, 1e-3, 99)
+            ctx.finish()
+        finally:
+            ctx.set_gemm_mode("tensor")
+        if p2 is not None:
+            want = torch.empty_like(p2)
+            ctx.counter_pack2(st, want, I, O, 11)
+            ctx.finish()
+            assert torch.equal(p2, want)
+        res.append((st, sc, v))
+    (st, sc, v), (est, esc, ev) = res
+    assert float((st != est).double().mean()) <= 2e-4          # a rounding that falls the other way for a last-bit gradient difference
+    assert float((sc - esc).norm() / esc.norm()) < 1e-6 and float((v - ev).norm() / ev.norm()) < 1e-5
