@@ -249,7 +249,7 @@ struct U16Layout {
     int sb, off_tick, off_rowc, off_part, off_rowtab, off_gw, off_st, off_so, off_p2;
     size_t total;
 };
-__host__ __device__ inline U16Layout u16_layout(int I, int R, bool with_q) {
+__host__ __device__ inline U16Layout u16_layout(int I, int R, bool with_q, int pairs = kPairs) {
     (void)with_q;
     U16Layout L;
     const int row_bytes = (I >> 2) * 3;
@@ -257,7 +257,7 @@ __host__ __device__ inline U16Layout u16_layout(int I, int R, bool with_q) {
     size_t o = sizeof(DecodeLut);
     L.off_tick = (int)o; o += kTickBytes;
     L.off_rowc = (int)o; o += sizeof(RowK) * R;
-    L.off_part = (int)o; o += sizeof(float) * 64 * kPairs;
+    L.off_part = (int)o; o += sizeof(float) * 64 * pairs;
     L.off_rowtab = (int)o; o += sizeof(RowEntry) * 64 * (size_t)R;
     L.off_gw = (int)o; o += sizeof(float) * (size_t)R * I;
     L.off_st = (int)o; o += (size_t)R * L.sb + 16;
@@ -267,11 +267,32 @@ __host__ __device__ inline U16Layout u16_layout(int I, int R, bool with_q) {
     return L;
 }
 
+// state rows row0 .. row0 + nrows - 1 into shared memory
+template <int NT>
+__device__ __forceinline__ void u16_load_state(const UpdParams& p, const U16Layout& L, unsigned char* smem, const int row0, const int nrows) {
+    const int row_bytes = (p.in_features >> 2) * 3, tid = threadIdx.x;
+    unsigned char* st_s = smem + L.off_st;
+    const uint8_t* src = p.state + (size_t)row0 * row_bytes;
+    if (p.state_align >= 16) {        // row_bytes % 16 == 0: one flat copy, smem row stride == row_bytes
+        const uint4* s4 = reinterpret_cast<const uint4*>(src);
+        uint4* d4 = reinterpret_cast<uint4*>(st_s);
+        for (int i = tid; i < nrows * (row_bytes >> 4); i += NT) d4[i] = __ldg(s4 + i);
+    } else {                          // rows are 4-byte aligned; smem rows padded to L.sb
+        const uint32_t* s1 = reinterpret_cast<const uint32_t*>(src);
+        const int wpr = row_bytes >> 2;
+        for (int i = tid; i < nrows * wpr; i += NT) {
+            const int r = i / wpr, w = i - r * wpr;
+            reinterpret_cast<uint32_t*>(st_s + (size_t)r * L.sb)[w] = __ldg(s1 + i);
+        }
+    }
+}
+
 // Body shared by the single-layer and the grouped kernel: batches batch0, batch0 + batch_step, ... of the
 // layer `p`.  The decode and tick tables depend on C alone; `build_tables` is false when an earlier call
 // of the same CTA already built them for this C.
-// GW_READY: the gradient rows of the one batch already lie in shared memory, swizzled as the load phase leaves them.
-template <bool WITH_Q, bool GW_READY = false>
+// GW_READY: state and gradient rows of the one batch already lie in shared memory as the load phase leaves them.
+// NT: threads of the CTA.
+template <bool WITH_Q, bool GW_READY = false, int NT = kUpdThreads>
 __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32_t unit_magic, const uint32_t pow16,
                                                 const uint32_t pow17, const int batch0, const int batch_step,
                                                 const bool build_tables) {
@@ -281,7 +302,7 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
     const int upr = I >> 4;               // 16-weight units per row
     const int row_bytes = gpr * 3;
     const int R = p.rows_per_batch;
-    const U16Layout L = u16_layout(I, R, WITH_Q);
+    const U16Layout L = u16_layout(I, R, WITH_Q, NT / 64);
 
     DecodeLut* lut = reinterpret_cast<DecodeLut*>(smem);
     uint32_t* tick_tab = reinterpret_cast<uint32_t*>(smem + L.off_tick);
@@ -308,8 +329,8 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
 
     if (build_tables) {
         __syncthreads();                  // an earlier layer's batches may still read the old tables
-        build_decode_lut(lut, p.C, tid, kUpdThreads);
-        build_tick_table(tick_tab, p.C, tid, kUpdThreads);
+        build_decode_lut(lut, p.C, tid, NT);
+        build_tick_table(tick_tab, p.C, tid, NT);
     }
     __syncthreads();
 
@@ -320,33 +341,21 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
 
         // ---- load: the batch's rows are contiguous in global memory ------------------------
         {
-            const uint8_t* src = p.state + (size_t)row0 * row_bytes;
-            if (aligned16) {        // row_bytes % 16 == 0: one flat copy, smem row stride == row_bytes
-                const uint4* s4 = reinterpret_cast<const uint4*>(src);
-                uint4* d4 = reinterpret_cast<uint4*>(st_s);
-                for (int i = tid; i < nrows * (row_bytes >> 4); i += kUpdThreads) d4[i] = __ldg(s4 + i);
-            } else {                // rows are 4-byte aligned; smem rows padded to L.sb
-                const uint32_t* s1 = reinterpret_cast<const uint32_t*>(src);
-                const int wpr = row_bytes >> 2;
-                for (int i = tid; i < nrows * wpr; i += kUpdThreads) {
-                    const int r = i / wpr, w = i - r * wpr;
-                    reinterpret_cast<uint32_t*>(st_s + (size_t)r * L.sb)[w] = __ldg(s1 + i);
-                }
-            }
+            if (!GW_READY) u16_load_state<NT>(p, L, smem, row0, nrows);
             if (!GW_READY) {
             const float4* gsrc = reinterpret_cast<const float4*>(p.grad_w + (size_t)row0 * I);
             const int n4 = nrows * gpr;
             if ((gpr & 31) == 0) {  // rows start on a period of the swizzle: the flat float4 index can be swizzled as it is
                 int i = tid;
-                for (; i + 3 * kUpdThreads < n4; i += 4 * kUpdThreads) {       // four loads in flight per thread
-                    const float4 v0 = __ldg(gsrc + i), v1 = __ldg(gsrc + i + kUpdThreads), v2 = __ldg(gsrc + i + 2 * kUpdThreads),
-                                 v3 = __ldg(gsrc + i + 3 * kUpdThreads);
-                    gw_s[swz4(i)] = v0; gw_s[swz4(i + kUpdThreads)] = v1;
-                    gw_s[swz4(i + 2 * kUpdThreads)] = v2; gw_s[swz4(i + 3 * kUpdThreads)] = v3;
+                for (; i + 3 * NT < n4; i += 4 * NT) {       // four loads in flight per thread
+                    const float4 v0 = __ldg(gsrc + i), v1 = __ldg(gsrc + i + NT), v2 = __ldg(gsrc + i + 2 * NT),
+                                 v3 = __ldg(gsrc + i + 3 * NT);
+                    gw_s[swz4(i)] = v0; gw_s[swz4(i + NT)] = v1;
+                    gw_s[swz4(i + 2 * NT)] = v2; gw_s[swz4(i + 3 * NT)] = v3;
                 }
-                for (; i < n4; i += kUpdThreads) gw_s[swz4(i)] = __ldg(gsrc + i);
+                for (; i < n4; i += NT) gw_s[swz4(i)] = __ldg(gsrc + i);
             } else {                // flat over the batch; row = i / gpr by multiply-high (gpr = 4 * units per row)
-                for (int i = tid; i < n4; i += kUpdThreads) {
+                for (int i = tid; i < n4; i += NT) {
                     const int r = unit_magic ? (int)__umulhi((uint32_t)i >> 2, unit_magic) : (i >> 2);
                     const int g = i - r * gpr;
                     gw_s[r * gpr + swz4(g)] = __ldg(gsrc + i);
@@ -356,8 +365,8 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
         }
         __syncthreads();
 
-        // ---- stats: warp pair `pair` walks rows pair, pair + kPairs, ... ---------------------
-        for (int r = pair; r < nrows; r += kPairs) {
+        // ---- stats: warp pair `pair` walks rows pair, pair + (NT / 64), ... ---------------------
+        for (int r = pair; r < nrows; r += (NT / 64)) {
             float a = 0.0f, b = 0.0f;
             const float4* g4 = gw_s + r * gpr;
             const uint32_t* raw = reinterpret_cast<const uint32_t*>(st_s + (size_t)r * L.sb);
@@ -399,7 +408,7 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
         // Shared memory is addressed with 32-bit shared-space addresses (ld.shared / st.shared), which
         // keeps the address arithmetic of the data-dependent table look-ups to one add each.
         const int nunits = nrows * upr;
-        for (int u = tid; u < nunits; u += kUpdThreads) {
+        for (int u = tid; u < nunits; u += NT) {
             const int r = unit_magic ? (int)__umulhi((uint32_t)u, unit_magic) : u;       // u / upr (magic 0: upr == 1)
             const int j = u - r * upr;
             const uint32_t g4 = sa_gw + ((uint32_t)(r * gpr + 4 * j) << 4);
@@ -422,11 +431,11 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
             if (aligned16) {
                 const uint4* s4 = reinterpret_cast<const uint4*>(so_s);
                 uint4* d4 = reinterpret_cast<uint4*>(dst);
-                for (int i = tid; i < nrows * (row_bytes >> 4); i += kUpdThreads) d4[i] = s4[i];
+                for (int i = tid; i < nrows * (row_bytes >> 4); i += NT) d4[i] = s4[i];
             } else {
                 uint32_t* d1 = reinterpret_cast<uint32_t*>(dst);
                 const int wpr = row_bytes >> 2;
-                for (int i = tid; i < nrows * wpr; i += kUpdThreads) {
+                for (int i = tid; i < nrows * wpr; i += NT) {
                     const int r = i / wpr, w = i - r * wpr;
                     d1[i] = reinterpret_cast<const uint32_t*>(so_s + (size_t)r * L.sb)[w];
                 }
@@ -436,9 +445,9 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
                 if (aligned16) {
                     const uint4* s4 = reinterpret_cast<const uint4*>(p2_s);
                     uint4* d4 = reinterpret_cast<uint4*>(d);
-                    for (int i = tid; i < (nrows * upr) >> 2; i += kUpdThreads) d4[i] = s4[i];
+                    for (int i = tid; i < (nrows * upr) >> 2; i += NT) d4[i] = s4[i];
                 } else {
-                    for (int i = tid; i < nrows * upr; i += kUpdThreads) d[i] = p2_s[i];
+                    for (int i = tid; i < nrows * upr; i += NT) d[i] = p2_s[i];
                 }
             }
         }

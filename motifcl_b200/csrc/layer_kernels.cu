@@ -10,8 +10,9 @@
 // Tensor-core accumulation truncates in proportion to what the accumulator holds, so the products of leading terms have an
 // accumulator of their own and all smaller ones share a second; the epilogue adds the two in fp32 (one accumulator for
 // all: 1.1e-6 relative error at K = 512).
-// Loads of the next k-tile are in flight while the current one is converted; two shared-memory stages let the tensor core work on
-// one while the threads fill the other.  These kernels are latency-bound (tens of CTAs, a handful of k-tiles each).
+// Loads run two k-tiles ahead in registers (one tile ahead left 1000 of 1550 cycles per k-tile waiting for them); two shared-memory
+// stages let the tensor core work on one while the threads fill the other.  These kernels are latency-bound (tens of CTAs, a
+// handful of k-tiles each).
 //
 // Every wait on an mbarrier is bounded; on time-out the error word is set and the results are invalid.
 #include <cuda_bf16.h>
@@ -24,7 +25,7 @@
 namespace mcl {
 namespace {
 
-constexpr int kLThreads = 256;
+constexpr int kLThreads = 512;
 constexpr int kErrLayer = 41;
 
 // two fp32 values -> their three bf16 terms, packed two per word
@@ -119,39 +120,71 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
         const __nv_bfloat16 h = __float2bfloat16_rn((float)(tid / (2 * p.C - 1) - 1));
         digit[tid] = __bfloat16_as_ushort(h);
     }
-    // A: 8 float4 of a k-tile per thread (row = idx / 16, 4 k each); digits: units of 16 weights, up to BN / 64 per thread
-    float4 a[8];
-    uint32_t w[4][3];
+    // A: 4 float4 of a k-tile per thread: rows tid / 16 + 32 j, the same 4 k in each.  Digits: units of 16 weights, up to 2 per
+    // thread.  All addresses are formed once and advance by a constant per k-tile.
+    struct Regs { float4 a[4], sc4; uint32_t w[2][3]; };
     const int nkt = (p.K + 63) / 64, nu = 4 * BN;         // units per k-tile: BN rows x 4 (Y) or 64 rows x BN / 16 (dX)
-    auto unit_at = [&](int u, int kt, int& row, int& col) -> bool {      // unit -> state row / first column; false: outside
-        if (DX) { const int per = BN >> 4; row = kt * 64 + u / per; col = n0 + (u % per) * 16; return row < p.K && col < p.N; }
-        row = n0 + (u >> 2); col = kt * 64 + (u & 3) * 16;
-        return row < p.N && col < p.K;
-    };
-    auto load = [&](int kt) {
+    const int rb = I / 4 * 3, ka = (tid & 15) * 4, arow = tid >> 4;
+    const float* ap = p.a + (size_t)(m0 + arow) * p.K + ka;
+    const size_t astep = (size_t)32 * p.K;
+    uint32_t arows = 0;                                    // bit j: row m0 + arow + 32 j exists
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int idx = tid + kLThreads * j, row = m0 + (idx >> 4), k = kt * 64 + (idx & 15) * 4;
-            a[j] = row < p.M ? load4(p.a + (size_t)row * p.K, k, p.K, p.vec != 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < 4; ++j) arows |= (m0 + arow + 32 * j < p.M ? 1u : 0u) << j;
+    const uint32_t a_at = (uint32_t)arow * 128u + (uint32_t)(((ka >> 3) ^ (arow & 7)) << 4) + (uint32_t)((ka & 4) << 1);
+    uint32_t u_off[2], u_at[2];                            // byte offset of the unit's codes, shared-memory address of its first 8 digits
+    int u_row[2], u_left[2];                               // row (Y: constant, dX: k within the tile) and groups of 4 up to the row's end
+    const uint8_t* sp = DX ? p.state + (size_t)(n0 / 4) * 3 : p.state + (size_t)n0 * rb;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int u = tid + kLThreads * j;
+        if (DX) {
+            const int per = BN >> 4, kr = u / per, cu = u - kr * per;
+            u_row[j] = u < nu ? kr : 1 << 30;
+            u_left[j] = (I - n0) / 4 - 4 * cu;
+            u_off[j] = (uint32_t)(kr * rb + 12 * cu);
+            u_at[j] = (uint32_t)(cu >> 2) * 8192u + (uint32_t)kr * 128u + ((uint32_t)((2 * (cu & 3)) ^ (kr & 7)) << 4);
+        } else {
+            const int r = u >> 2, ku = u & 3;
+            u_row[j] = u < nu && n0 + r < p.N ? 0 : 1 << 30;
+            u_left[j] = I / 4 - 4 * ku;
+            u_off[j] = (uint32_t)(r * rb + 12 * ku);
+            u_at[j] = (uint32_t)r * 128u + ((uint32_t)((2 * ku) ^ (r & 7)) << 4);
         }
+    }
+    const size_t ustep = DX ? (size_t)64 * rb : 48;
+    auto load = [&](int kt, Regs& r) {
+        const int k = kt * 64 + ka;
+        const float* q = ap + kt * 64;
+        if (p.vec) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int u = tid + kLThreads * j;
-            int row, col;
-            w[j][0] = w[j][1] = w[j][2] = 0;
-            if (u < nu && unit_at(u, kt, row, col)) {
-                const size_t at = ((size_t)row * I + col) / 4 * 3;
+            for (int j = 0; j < 4; ++j)
+                r.a[j] = ((arows >> j) & 1u) && k < p.K ? __ldg(reinterpret_cast<const float4*>(q + j * astep)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r.a[j] = load4(q + j * astep - k, k, (arows >> j) & 1u ? p.K : 0, false);
+        }
+        if (DX) r.sc4 = load4(p.scale, k, p.K, false);
+        const uint8_t* g = sp + kt * ustep;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            r.w[j][0] = r.w[j][1] = r.w[j][2] = 0;
+            const bool in = DX ? u_row[j] + kt * 64 < p.K && u_left[j] > 0 : u_row[j] == 0 && u_left[j] > 16 * kt;
+            if (in) {
                 if (words) {
-                    const uint32_t* s = reinterpret_cast<const uint32_t*>(p.state + at);
-                    w[j][0] = __ldg(s); w[j][1] = __ldg(s + 1); w[j][2] = __ldg(s + 2);
+                    const uint32_t* s = reinterpret_cast<const uint32_t*>(g + u_off[j]);
+                    r.w[j][0] = __ldg(s); r.w[j][1] = __ldg(s + 1); r.w[j][2] = __ldg(s + 2);
                 } else {
-                    const int nb = min(12, (I - col) / 4 * 3);
-                    for (int b = 0; b < nb; ++b) w[j][b >> 2] |= (uint32_t)__ldg(p.state + at + b) << (8 * (b & 3));
+                    const int nb = 3 * min(4, u_left[j] - (DX ? 0 : 16 * kt));
+#pragma unroll
+                    for (int b = 0; b < 12; ++b)
+                        if (b < nb) r.w[j][b >> 2] |= (uint32_t)__ldg(g + u_off[j] + b) << (8 * (b & 3));
                 }
             }
         }
     };
-    load(0);
+    Regs r0, r1;
+    load(0, r0);
+    if (nkt > 1) load(1, r1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -160,55 +193,40 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16(128, BN, 0, DX ? 1u : 0u);
     bool ok = true;
-    for (int kt = 0; kt < nkt; ++kt) {
+    auto step = [&](int kt, Regs& r) {
         const int s = kt & 1;
         const uint32_t st = stage0 + (uint32_t)s * (uint32_t)p.stage_bytes, sb = st + 3u * kRowATerm;
         if (kt >= 2 && ok) ok = mbar_wait(bar0 + 8u * s, ((uint32_t)(kt >> 1) - 1u) & 1u, &abort_flag);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int idx = tid + kLThreads * j, row = idx >> 4, c4 = idx & 15;
-            float4 v = a[j];
+        for (int j = 0; j < 4; ++j) {
+            float4 v = r.a[j];
             if (DX) {                                      // grad_out times the scale of its column, rounded to fp32
-                const int k = kt * 64 + c4 * 4;
-                if (k < p.K) v.x = __fmul_rn(v.x, __ldg(p.scale + k));
-                if (k + 1 < p.K) v.y = __fmul_rn(v.y, __ldg(p.scale + k + 1));
-                if (k + 2 < p.K) v.z = __fmul_rn(v.z, __ldg(p.scale + k + 2));
-                if (k + 3 < p.K) v.w = __fmul_rn(v.w, __ldg(p.scale + k + 3));
+                v.x = __fmul_rn(v.x, r.sc4.x); v.y = __fmul_rn(v.y, r.sc4.y);
+                v.z = __fmul_rn(v.z, r.sc4.z); v.w = __fmul_rn(v.w, r.sc4.w);
             }
             uint32_t t0[3], t1[3];
             split3(v.x, v.y, t0); split3(v.z, v.w, t1);
-            const uint32_t at = st + (uint32_t)row * 128u + (uint32_t)(((c4 >> 1) ^ (row & 7)) << 4) + (uint32_t)((c4 & 1) << 3);
 #pragma unroll
-            for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * kRowATerm, t0[t], t1[t]);
+            for (int t = 0; t < 3; ++t) sts64(st + a_at + (uint32_t)(4096 * j + kRowATerm * t), t0[t], t1[t]);
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int u = tid + kLThreads * j;
-            if (u < nu) {
-                int row, col;
-                const bool in = unit_at(u, kt, row, col);
+        for (int j = 0; j < 2; ++j) {
+            if (tid + kLThreads * j < nu) {
+                // groups of 4 that exist (the others, and rows outside, were loaded as zero codes and must become zero digits)
+                const int left = DX ? (u_row[j] + kt * 64 < p.K ? u_left[j] : 0) : (u_row[j] == 0 ? u_left[j] - 16 * kt : 0);
                 uint32_t h[8];
-                const uint32_t g[4] = {w[j][0] & 0xFFFFFFu, (w[j][0] >> 24) | ((w[j][1] & 0xFFFFu) << 8),
-                                       (w[j][1] >> 16) | ((w[j][2] & 0xFFu) << 16), w[j][2] >> 8};
-                const int left = in ? (I - col) >> 2 : 0;   // groups of 4 that exist
+                const uint32_t g[4] = {r.w[j][0] & 0xFFFFFFu, (r.w[j][0] >> 24) | ((r.w[j][1] & 0xFFFFu) << 8),
+                                       (r.w[j][1] >> 16) | ((r.w[j][2] & 0xFFu) << 16), r.w[j][2] >> 8};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     h[2 * q] = q < left ? lut[g[q] & 4095u] : 0u;
                     h[2 * q + 1] = q < left ? lut[g[q] >> 12] : 0u;
                 }
-                uint32_t at, x;
-                int c16;
-                if (DX) {
-                    const int per = BN >> 4, kr = u / per, cu = u % per;
-                    at = sb + (uint32_t)(cu >> 2) * 8192u + (uint32_t)kr * 128u; x = (uint32_t)(kr & 7); c16 = 2 * (cu & 3);
-                } else {
-                    at = sb + (uint32_t)(u >> 2) * 128u; x = (uint32_t)((u >> 2) & 7); c16 = 2 * (u & 3);
-                }
-                sts128u(at + (((uint32_t)c16 ^ x) << 4), h[0], h[1], h[2], h[3]);
-                sts128u(at + (((uint32_t)(c16 + 1) ^ x) << 4), h[4], h[5], h[6], h[7]);
+                sts128u(sb + u_at[j], h[0], h[1], h[2], h[3]);
+                sts128u(sb + (u_at[j] ^ 16u), h[4], h[5], h[6], h[7]);
             }
         }
-        if (kt + 1 < nkt) load(kt + 1);
+        if (kt + 2 < nkt) load(kt + 2, r);
         fence_proxy_async();
         __syncthreads();
         if (warp == 0) {
@@ -227,15 +245,19 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
             }
             __syncwarp();
         }
+    };
+    for (int kt = 0; kt < nkt; kt += 2) {
+        step(kt, r0);
+        if (kt + 1 < nkt) step(kt + 1, r1);
     }
     if (ok) ok = mbar_wait(bar0 + 8u * ((nkt - 1) & 1), (uint32_t)((nkt - 1) >> 1) & 1u, &abort_flag);
     if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
     tc_fence_after();
-    // epilogue: warp = 32 rows x half of the columns; a 32 x 33 tile in shared memory turns lane = row into lane = column
+    // epilogue: warp = 32 rows x a quarter of the columns; a 32 x 33 tile in shared memory turns lane = row into lane = column
     {
-        const int q = warp & 3, half = warp >> 2;
+        const int q = warp & 3, part = warp >> 2;
         float* tile = reinterpret_cast<float*>(smem) + warp * 32 * 33;
-        for (int c0 = half * 32; c0 < BN && n0 + c0 < p.N; c0 += 64) {
+        for (int c0 = part * 32; c0 < BN && n0 + c0 < p.N; c0 += 128) {
             uint32_t r[32], r1[32];
             tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
             tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)c0, r1);
@@ -267,7 +289,8 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
 struct LayerUpdParams {
     const float* dy;          // [tokens, O]
     const float* x;           // [tokens, I]
-    int tokens, O, slice;     // slice: tokens per CTA, a multiple of 16
+    int tokens, O, slice;     // slice: tokens per CTA, a multiple of 32
+    int mr;                   // rows of the layer that a cluster owns (at most 128)
     int np, pw;               // passes over the columns and their width (a multiple of 64, at most 256)
     int off_stage, stage_bytes;
     int vec_dy;
@@ -275,8 +298,8 @@ struct LayerUpdParams {
     int* err;
     UpdParams u;              // of the whole layer; rows_per_batch = rows of a CTA
 };
-constexpr int kDwK = 16;                      // tokens per k-tile: one MMA step
-constexpr int kDwChunk = kDwK * 128;          // bytes of 64 columns x 16 tokens
+constexpr int kDwK = 32;                      // tokens per k-tile: two MMA steps
+constexpr int kDwChunk = kDwK * 128;          // bytes of 64 columns x 32 tokens
 constexpr int kDwATerm = 2 * kDwChunk;
 
 // the update for in_features % 16 != 0: groups of four weights read and written as bytes
@@ -295,7 +318,7 @@ __device__ __forceinline__ void update_rows_by_group(const UpdParams& p, const i
     };
     build_decode_lut(lut, p.C, tid, kLThreads);
     __syncthreads();
-    for (int r = pair; r < nrows; r += kPairs) {
+    for (int r = pair; r < nrows; r += kLThreads / 64) {
         float a = 0.0f, b = 0.0f;
         for (int g = vlane; g < gpr; g += 64) {
             const float4 gw = gw_s[r * gpr + g];
@@ -348,9 +371,9 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
     asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cs));
     const int rank = (int)cluster_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int I = p.u.in_features, gpr = I >> 2, R = p.u.rows_per_batch;
-    const U16Layout L = u16_layout(I, R, WITH_Q);
-    const int m0 = ((int)blockIdx.x / (int)cs) * 128;
-    const int valid = min(128, p.O - m0), rpc = (valid + (int)cs - 1) / (int)cs;
+    const U16Layout L = u16_layout(I, R, WITH_Q, kLThreads / 64);
+    const int m0 = ((int)blockIdx.x / (int)cs) * p.mr;
+    const int valid = min(p.mr, p.O - m0), rpc = (valid + (int)cs - 1) / (int)cs;
     const int my_row0 = rank * rpc, my_rows = max(0, min(rpc, valid - my_row0));
     const int t0 = rank * p.slice, t1 = min(p.tokens, t0 + p.slice);
     const int nkt = t1 > t0 ? (t1 - t0 + kDwK - 1) / kDwK : 0;
@@ -365,6 +388,23 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), 2 * cols);       // leading products, smaller products
+    UpdParams u = p.u;                            // of this CTA's rows
+    {
+        const int row = m0 + my_row0;
+        u.state += (size_t)row * gpr * 3;
+        u.scale += row; u.v += row;
+        if (u.packed2) u.packed2 += (size_t)row * (I >> 4);
+        u.rows = my_rows; u.row_offset = row;
+    }
+    if (U16 && my_rows > 0) {                     // what the update needs beside the gradient is in place before it
+        build_decode_lut(reinterpret_cast<DecodeLut*>(smem), u.C, tid, kLThreads);
+        build_tick_table(reinterpret_cast<uint32_t*>(smem + L.off_tick), u.C, tid, kLThreads);
+        u16_load_state<kLThreads>(u, L, smem, 0, my_rows);
+        if (tid < my_rows) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(u.scale + tid));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(u.v + tid));
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -374,46 +414,60 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
     for (int pass = 0; pass < p.np; ++pass) {
         const int n0 = pass * p.pw, nw = min(p.pw, I - n0), nwp = (nw + 15) & ~15, per = nwp >> 2;
         const uint32_t bterm = (uint32_t)((nwp + 63) / 64) * kDwChunk;
-        // this thread's float4s of a k-tile: 2 of dY (128 columns), up to 4 of x
-        float4 a[2], b[4];
-        int brow[4], bcol[4];
+        // this thread's float4s of a k-tile: 2 of dY (tokens tid / 32 + 16 j, the same 4 columns), up to 4 of x; addresses are
+        // formed once and advance by a constant per k-tile
+        struct Regs { float4 a[2], b[4]; };
+        int b_off[4], b_tok[4];
+        uint32_t b_at[4];
+        const int ac = m0 + lane * 4;
+        const bool a_in = lane * 4 < valid;
+        const float* ap = p.dy + (size_t)(t0 + warp) * p.O + ac;
+        const float* bp = p.x + (size_t)t0 * I + n0;
+        auto place = [](int row, int col) -> uint32_t {        // shared-memory offset of four columns of one token
+            return (uint32_t)(col >> 6) * kDwChunk + (uint32_t)row * 128u + (uint32_t)((((col & 63) >> 3) ^ (row & 7)) << 4) + (uint32_t)((col & 4) << 1);
+        };
+        const uint32_t a_at = place(warp, lane * 4);           // rows 16 further: + 2048, the swizzle repeats
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int idx = tid + kLThreads * j;
-            brow[j] = idx < kDwK * per ? idx / per : -1;
-            bcol[j] = 4 * (idx % per);
+            const int idx = tid + kLThreads * j, row = idx / per, col = 4 * (idx - row * per);
+            b_tok[j] = row < kDwK ? row : 1 << 30;
+            b_off[j] = n0 + col < I ? row * I + col : -1;
+            b_at[j] = place(row, col);
         }
-        auto load = [&](int kt) {
-            const int tb = t0 + kt * kDwK;
+        auto load = [&](int kt, Regs& r) {
+            const int left = t1 - t0 - kt * kDwK;              // tokens from this k-tile on
+            const float* q = ap + (size_t)kt * kDwK * p.O;
+            if (p.vec_dy) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int idx = tid + kLThreads * j, t = tb + (idx >> 5);
-                a[j] = t < t1 ? load4(p.dy + (size_t)t * p.O, m0 + (idx & 31) * 4, p.O, p.vec_dy != 0) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+                for (int j = 0; j < 2; ++j)
+                    r.a[j] = warp + 16 * j < left && a_in ? __ldg(reinterpret_cast<const float4*>(q + (size_t)(16 * j) * p.O)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int t = tb + brow[j];
-                b[j] = brow[j] >= 0 && t < t1 ? load4(p.x + (size_t)t * I, n0 + bcol[j], I, true) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int j = 0; j < 2; ++j) r.a[j] = load4(q + (size_t)(16 * j) * p.O - ac, ac, warp + 16 * j < left && a_in ? p.O : 0, false);
             }
+            const float* g = bp + (size_t)kt * kDwK * I;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                r.b[j] = b_tok[j] < left && b_off[j] >= 0 ? __ldg(reinterpret_cast<const float4*>(g + b_off[j])) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
-        if (nkt > 0) load(0);
-        for (int kt = 0; kt < nkt; ++kt, ++it) {
+        Regs r0, r1;
+        if (nkt > 0) load(0, r0);
+        if (nkt > 1) load(1, r1);
+        auto step = [&](int kt, Regs& r) {
             const uint32_t st = stage0 + (uint32_t)(it & 1) * (uint32_t)p.stage_bytes, sb = st + 3u * kDwATerm;
             if (it >= 2 && ok) ok = mbar_wait(bar0 + 8u * (it & 1), ((uint32_t)(it >> 1) - 1u) & 1u, &abort_flag);
-            auto put = [&](uint32_t base, uint32_t term, int row, int col, float4 v) {     // four columns of one token, three terms
+            auto put = [&](uint32_t at, uint32_t term, float4 v) {     // four columns of one token, three terms
                 uint32_t u0[3], u1[3];
                 split3(v.x, v.y, u0); split3(v.z, v.w, u1);
-                const uint32_t at = base + (uint32_t)(col >> 6) * kDwChunk + (uint32_t)row * 128u +
-                                    (uint32_t)((((col & 63) >> 3) ^ (row & 7)) << 4) + (uint32_t)((col & 4) << 1);
 #pragma unroll
                 for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * term, u0[t], u1[t]);
             };
 #pragma unroll
-            for (int j = 0; j < 2; ++j) { const int idx = tid + kLThreads * j; put(st, kDwATerm, idx >> 5, (idx & 31) * 4, a[j]); }
+            for (int j = 0; j < 2; ++j) put(st + a_at + 2048u * j, kDwATerm, r.a[j]);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (brow[j] >= 0) put(sb, bterm, brow[j], bcol[j], b[j]);
-            if (kt + 1 < nkt) load(kt + 1);
+                if (b_tok[j] < kDwK) put(sb + b_at[j], bterm, r.b[j]);
+            if (kt + 2 < nkt) load(kt + 2, r);
             fence_proxy_async();
             __syncthreads();
             if (warp == 0) {
@@ -423,38 +477,42 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
                     const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
                     for (int q = 0; q < 6; ++q) {
-                        umma_bf16(q == 5 ? tmem : tmem + cols, desc_mn(st + (uint32_t)pa[q] * kDwATerm, kDwChunk),
-                                  desc_mn(sb + (uint32_t)pb[q] * bterm, kDwChunk), idesc_bf16(128, nwp, 1, 1), kt != 0 || (q > 0 && q < 5) ? 1u : 0u);
+                        const uint64_t da = desc_mn(st + (uint32_t)pa[q] * kDwATerm, kDwChunk), db = desc_mn(sb + (uint32_t)pb[q] * bterm, kDwChunk);
+#pragma unroll
+                        for (int kk = 0; kk < kDwK / 16; ++kk)         // 16 tokens = 2048 bytes further
+                            umma_bf16(q == 5 ? tmem : tmem + cols, da + 128u * kk, db + 128u * kk, idesc_bf16(128, nwp, 1, 1),
+                                      (kt | kk) != 0 || (q > 0 && q < 5) ? 1u : 0u);
                     }
                     umma_commit(bar0 + 8u * (it & 1));
                 }
                 __syncwarp();
             }
+            ++it;
+        };
+        for (int kt = 0; kt < nkt; kt += 2) {
+            step(kt, r0);
+            if (kt + 1 < nkt) step(kt + 1, r1);
         }
         if (it > 0 && ok) ok = mbar_wait(bar0 + 8u * ((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, &abort_flag);
         tc_fence_after();
         // sum over the cluster, 128 columns at a time; the exchange tile lies over the (finished) stages
         for (int c0 = 0; c0 < nw; c0 += 128) {
-            const int q = warp & 3, half = warp >> 2, row = q * 32 + lane;
+            const int q = warp & 3, cc = (warp >> 2) * 32, row = q * 32 + lane;
+            if (c0 + cc < nw && q * 32 < valid) {
+                uint32_t r[32], r1[32];
+                if (nkt > 0) {
+                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + cc), r);
+                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)(c0 + cc), r1);
+                    tmem_ld_wait();
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int cc = half * 64 + h * 32;
-                if (c0 + cc < nw) {
-                    uint32_t r[32], r1[32];
-                    if (nkt > 0) {
-                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + cc), r);
-                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)(c0 + cc), r1);
-                        tmem_ld_wait();
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
+                } else {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) r[j] = 0;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        sts128u(stage0 + (uint32_t)row * 512u + (uint32_t)(((cc >> 2) + j) ^ (row & 7)) * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                    for (int j = 0; j < 32; ++j) r[j] = 0;
                 }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    sts128u(stage0 + (uint32_t)row * 512u + (uint32_t)(((cc >> 2) + j) ^ (row & 7)) * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
             }
             tc_fence_before();
             cluster_sync_all();
@@ -463,11 +521,16 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
                 if (c0 + 4 * c < nw) {
                     const int mr = my_row0 + r;
                     const uint32_t at = stage0 + (uint32_t)mr * 512u + (uint32_t)(c ^ (mr & 7)) * 16u;
-                    float4 sum = ld_peer(at, 0);
-                    for (uint32_t k = 1; k < cs; ++k) {
-                        const float4 v = ld_peer(at, k);
-                        sum.x = __fadd_rn(sum.x, v.x); sum.y = __fadd_rn(sum.y, v.y);
-                        sum.z = __fadd_rn(sum.z, v.z); sum.w = __fadd_rn(sum.w, v.w);
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (uint32_t k = 0; k < cs; k += 4) {             // four remote loads in flight
+                        float4 v[4];
+#pragma unroll
+                        for (uint32_t i4 = 0; i4 < 4; ++i4) v[i4] = ld_peer(at, k + i4);
+#pragma unroll
+                        for (uint32_t i4 = 0; i4 < 4; ++i4) {
+                            sum.x = __fadd_rn(sum.x, v[i4].x); sum.y = __fadd_rn(sum.y, v[i4].y);
+                            sum.z = __fadd_rn(sum.z, v[i4].z); sum.w = __fadd_rn(sum.w, v[i4].w);
+                        }
                     }
                     gw_s[r * gpr + (U16 ? swz4(g) : g)] = sum;
                 }
@@ -479,13 +542,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
     if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * cols) : "memory");
     if (my_rows == 0) return;
-    UpdParams u = p.u;
-    const int row = m0 + my_row0;
-    u.state += (size_t)row * gpr * 3;
-    u.scale += row; u.v += row;
-    if (u.packed2) u.packed2 += (size_t)row * (I >> 4);
-    u.rows = my_rows; u.row_offset = row;
-    if (U16) update_u16_body<WITH_Q, true>(u, p.magic, 1u << 16, 1u << 17, 0, 1, true);
+    if (U16) update_u16_body<WITH_Q, true, kLThreads>(u, p.magic, 1u << 16, 1u << 17, 0, 1, false);
     else update_rows_by_group<WITH_Q>(u, my_rows, smem, L);
 }
 
@@ -526,7 +583,7 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
 cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
                                 float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int sm_count,
                                 size_t max_smem, cudaStream_t stream) {
-    const int I = d.in_features, O = d.rows, tiles = (O + 127) / 128;
+    const int I = d.in_features, O = d.rows;
     const bool with_q = lr_scale != 0.0f;
     const bool u16 = I % 16 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 3) == 0;
     auto kern = u16 ? (with_q ? layer_update_kernel<true, true> : layer_update_kernel<false, true>)
@@ -534,18 +591,32 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
     const int slot = 20 + (u16 ? 2 : 0) + (with_q ? 1 : 0);
     cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), slot, max_smem);
     if (e != cudaSuccess) return e;
-    // CTAs per 128 rows: 8 (portable), or 16 while all of them fit the device at once
-    for (int cs = tiles * 16 <= sm_count * 3 / 4 ? 16 : 8;; cs = 8) {
+    // Rows per cluster and CTAs per cluster: a CTA contracts its slice of the tokens (all columns, whatever the rows), then
+    // moves its rows x columns through the exchange once.  More CTAs shorten the slices, fewer rows per cluster shorten the
+    // exchange; all CTAs should be resident at once.  Times in cycles from the stamps of both phases.
+    const int np = (I + 255) / 256, pw = ((I + np - 1) / np + 63) / 64 * 64;
+    int mr = 128, cs = 8;
+    double best = 1e30;
+    for (int c = 4; c <= 8; c *= 2)            // clusters of 16 need two waves where eights need one: 288 x 288 at 256 rows 55 us, not 40
+        for (int m = 128; m >= 32; m /= 2) {
+            const int ctas = (O + m - 1) / m * c, kt = ((tokens + c - 1) / c + kDwK - 1) / kDwK;
+            const double cost = (double)((ctas + sm_count - 1) / sm_count) *
+                                ((double)np * kt * (400.0 + 5.0 * (m + pw)) + (double)m * I * 4 / 16.0 + np * ((pw + 127) / 128) * 1500.0 + 4000.0 + (double)(m / c) * I * 0.6);
+            if (cost < best) { best = cost; mr = m; cs = c; }
+        }
+    {
+        const int tiles = (O + mr - 1) / mr;
         LayerUpdParams p;
-        const int R = 128 / cs;
-        const size_t base = (u16_layout(I, R, with_q).total + 1023) & ~size_t(1023);
+        p.mr = mr;
+        const int R = mr / cs;
+        const size_t base = (u16_layout(I, R, with_q, kLThreads / 64).total + 1023) & ~size_t(1023);
         size_t smem = 0;
-        for (p.np = 1; p.np <= 16; ++p.np) {
+        for (p.np = np; p.np <= 16; ++p.np) {
             p.pw = ((I + p.np - 1) / p.np + 63) / 64 * 64;
             p.stage_bytes = 3 * kDwATerm + 3 * (p.pw / 64) * kDwChunk;
             const size_t area = 2 * (size_t)p.stage_bytes > 65536 ? 2 * (size_t)p.stage_bytes : 65536;
             smem = base + area + 1024;
-            if (p.pw <= 256 && smem + 1024 <= max_smem) break;
+            if (smem + 1024 <= max_smem) break;
         }
         if (p.np > 16) return cudaErrorInvalidConfiguration;
         p.off_stage = (int)base;
@@ -570,20 +641,6 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
         attr[0].val.clusterDim.x = (unsigned)cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (cs == 16) {
-            // asked once per kernel and device: a part whose GPCs cannot hold 16 such CTAs keeps clusters of 8
-            static int fits[64][4] = {};                  // 0 unknown, 1 yes, 2 no
-            int dev = 0;
-            cudaGetDevice(&dev);
-            int& f = fits[dev & 63][slot - 20];
-            if (f == 0) {
-                int n = 0;
-                cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-                f = cudaOccupancyMaxActiveClusters(&n, reinterpret_cast<const void*>(kern), &cfg) == cudaSuccess && n >= 4 ? 1 : 2;
-                cudaGetLastError();
-            }
-            if (f == 2) continue;
-        }
         return cudaLaunchKernelEx(&cfg, kern, p);
     }
 }
