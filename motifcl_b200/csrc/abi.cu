@@ -1229,7 +1229,7 @@ int mcl_cuda_rmsnorm_backward_weight(mcl_cuda_ctx* ctx, const float* x, const fl
     MCL_TRY(check_ptr(ctx, op, "grad_weight", grad_weight, 4));
     DeviceGuard guard(ctx->device);
     MCL_LAUNCH(ctx, op, mcl::launch_rmsnorm_backward_weight(x, grad_out, row_inv_scratch, grad_weight, rows, (int)cols, eps, ctx->sm_count, ctx->stream));
-    ctx->launches += 1;     // the row pass and the column pass
+    if (cols > 1024) ctx->launches += 1;     // a row pass and a column pass
     return MCL_CUDA_OK;
 }
 int mcl_cuda_mse_loss_partial(mcl_cuda_ctx* ctx, const float* pred, const float* target, float* partial, size_t n) {
@@ -1346,12 +1346,14 @@ int mcl_cuda_gqa_forward(mcl_cuda_ctx* ctx, const float* q, const float* k, cons
     DeviceGuard guard(ctx->device);
     // scores of every (batch, head, query) row live in the workspace between the two products; the batch is
     // served in slices that keep it under 4 GiB (one batch element at least)
-    const size_t per_batch = n_head * query_tokens * key_tokens * sizeof(float);
-    size_t slice = ((size_t)4 << 30) / per_batch;
+    // (the tiled kernels need none)
+    const size_t per_batch = mcl::gqa_forward_scratch_floats((int)batch, (int)query_tokens, (int)key_tokens, (int)n_head, (int)head_dim,
+                                                             (int)v_head_dim) / batch * sizeof(float);
+    size_t slice = per_batch ? ((size_t)4 << 30) / per_batch : batch;
     if (slice < 1) slice = 1;
     if (slice > batch) slice = batch;
     void* ws = nullptr;
-    MCL_TRY(ws_reserve(ctx, slice * per_batch, &ws));
+    if (per_batch) MCL_TRY(ws_reserve(ctx, slice * per_batch, &ws));
     int launches = 0;
     cudaError_t e = cudaSuccess;
     for (size_t b0 = 0; b0 < batch && e == cudaSuccess; b0 += slice) {

@@ -215,6 +215,7 @@ cudaError_t launch_rope(const float* x, float* out, size_t rows, int tokens, int
                         cudaStream_t stream);
 cudaError_t launch_adam(float* param, const float* grad, float* m, float* v, size_t n, float lr, float beta1, float beta2,
                         float eps, float weight_decay, float c1, float c2, int sm_count, cudaStream_t stream);
+size_t gqa_forward_scratch_floats(int batch, int tq, int tk, int n_head, int hd, int vhd);
 cudaError_t launch_gqa_forward(const float* q, const float* k, const float* v, float* out, int batch, int tq, int tk,
                                int key_stride, int n_head, int n_kv, int hd, int vhd, int causal, int q_off, int window,
                                float scale, float* scores_ws, cudaStream_t stream, int* launches);

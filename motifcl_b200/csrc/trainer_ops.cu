@@ -46,44 +46,139 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 }
 
 // ---- rmsnorm -------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
+// One warp per row; a lane holds the columns 4 (lane + 32 j) .. + 3 of the row in registers (rows of up to kNormHold * 128
+// columns; longer ones are read again), so HBM sees each row once.  4096 x 288: 7 us with a block and three barriers per row.
+constexpr int kNormHold = 8;          // H of the kernels: 3 for rows of up to 384 columns, else kNormHold
+struct Vec4 {                     // 128-bit accesses where rows start on 16-byte boundaries, else scalar ones
+    bool vec;
+    int cols;
+    __device__ __forceinline__ float4 get(const float* __restrict__ r, int c) const {
+        if (vec) return c < cols ? __ldg(reinterpret_cast<const float4*>(r + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return make_float4(c < cols ? __ldg(r + c) : 0.f, c + 1 < cols ? __ldg(r + c + 1) : 0.f, c + 2 < cols ? __ldg(r + c + 2) : 0.f,
+                           c + 3 < cols ? __ldg(r + c + 3) : 0.f);
+    }
+    __device__ __forceinline__ void put(float* r, int c, float4 v) const {
+        if (vec) { if (c < cols) *reinterpret_cast<float4*>(r + c) = v; return; }
+        if (c < cols) r[c] = v.x;
+        if (c + 1 < cols) r[c + 1] = v.y;
+        if (c + 2 < cols) r[c + 2] = v.z;
+        if (c + 3 < cols) r[c + 3] = v.w;
+    }
+};
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+
+template <int H>
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                       float* __restrict__ out, float* __restrict__ row_inv,
-                                                      size_t rows, int cols, float eps) {
-    __shared__ float red[32];
-    for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
+                                                      size_t rows, Vec4 a, float eps) {
+    const int lane = threadIdx.x & 31, cols = a.cols;
+    for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (size_t)gridDim.x * 8) {
         const float* xr = x + row * (size_t)cols;
+        float4 h[H], wh[H];         // the row and the weights, requested together
         float ss = 0.0f;
-        for (int c = threadIdx.x; c < cols; c += blockDim.x) ss += xr[c] * xr[c];
-        ss = block_sum(ss, red);
-        const float inv = rsqrtf(ss / (float)cols + eps);
-        if (row_inv != nullptr) {
-            if (threadIdx.x == 0) row_inv[row] = inv;
-        } else {
-            float* o = out + row * (size_t)cols;
-            for (int c = threadIdx.x; c < cols; c += blockDim.x) o[c] = xr[c] * inv * w[c];
+#pragma unroll
+        for (int j = 0; j < H; ++j) h[j] = a.get(xr, 4 * (lane + 32 * j));
+        if (w != nullptr) {
+#pragma unroll
+            for (int j = 0; j < H; ++j) wh[j] = a.get(w, 4 * (lane + 32 * j));
         }
+#pragma unroll
+        for (int j = 0; j < H; ++j) ss += dot4(h[j], h[j]);
+        for (int c = 4 * (lane + 32 * H); c < cols; c += 128) { const float4 v = a.get(xr, c); ss += dot4(v, v); }
+        const float inv = rsqrtf(warp_sum(ss) / (float)cols + eps);
+        if (row_inv != nullptr) {
+            if (lane == 0) row_inv[row] = inv;
+            continue;
+        }
+        float* o = out + row * (size_t)cols;
+        auto put = [&](int c, float4 v, float4 wv) {
+            a.put(o, c, make_float4(v.x * inv * wv.x, v.y * inv * wv.y, v.z * inv * wv.z, v.w * inv * wv.w));
+        };
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (4 * (lane + 32 * j) < cols) put(4 * (lane + 32 * j), h[j], wh[j]);
+        for (int c = 4 * (lane + 32 * H); c < cols; c += 128) put(c, a.get(xr, c), a.get(w, c));
     }
 }
 
-__global__ void __launch_bounds__(128) rmsnorm_bwd_x_kernel(const float* __restrict__ x, const float* __restrict__ w,
+template <int H>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                             const float* __restrict__ dy, float* __restrict__ dx,
-                                                            size_t rows, int cols, float eps) {
-    __shared__ float red[32];
-    for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
+                                                            size_t rows, Vec4 a, float eps) {
+    const int lane = threadIdx.x & 31, cols = a.cols;
+    for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (size_t)gridDim.x * 8) {
         const float* xr = x + row * (size_t)cols;
         const float* gr = dy + row * (size_t)cols;
+        float4 h[H], g[H], wh[H];   // x, dy (then dy * w) and w, requested together
         float ss = 0.0f, dot = 0.0f;
-        for (int c = threadIdx.x; c < cols; c += blockDim.x) {
-            const float xv = xr[c];
-            ss += xv * xv;
-            dot += gr[c] * w[c] * xv;
+        auto gw = [&](int c) {
+            const float4 gv = a.get(gr, c), wv = a.get(w, c);
+            return make_float4(gv.x * wv.x, gv.y * wv.y, gv.z * wv.z, gv.w * wv.w);
+        };
+#pragma unroll
+        for (int j = 0; j < H; ++j) { h[j] = a.get(xr, 4 * (lane + 32 * j)); g[j] = a.get(gr, 4 * (lane + 32 * j)); wh[j] = a.get(w, 4 * (lane + 32 * j)); }
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            g[j] = make_float4(g[j].x * wh[j].x, g[j].y * wh[j].y, g[j].z * wh[j].z, g[j].w * wh[j].w);
+            ss += dot4(h[j], h[j]);
+            dot += dot4(g[j], h[j]);
         }
-        ss = block_sum(ss, red);
-        dot = block_sum(dot, red);
-        const float inv = rsqrtf(ss / (float)cols + eps);
-        const float k = inv * inv * inv * dot / (float)cols;
+        for (int c = 4 * (lane + 32 * H); c < cols; c += 128) { const float4 v = a.get(xr, c); ss += dot4(v, v); dot += dot4(gw(c), v); }
+        const float inv = rsqrtf(warp_sum(ss) / (float)cols + eps);
+        const float k = inv * inv * inv * warp_sum(dot) / (float)cols;
         float* o = dx + row * (size_t)cols;
-        for (int c = threadIdx.x; c < cols; c += blockDim.x) o[c] = gr[c] * w[c] * inv - xr[c] * k;
+        auto put = [&](int c, float4 v, float4 q) {
+            a.put(o, c, make_float4(q.x * inv - v.x * k, q.y * inv - v.y * k, q.z * inv - v.z * k, q.w * inv - v.w * k));
+        };
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (4 * (lane + 32 * j) < cols) put(4 * (lane + 32 * j), h[j], g[j]);
+        for (int c = 4 * (lane + 32 * H); c < cols; c += 128) put(c, a.get(xr, c), gw(c));
+    }
+}
+
+// row_inv and dw[c] += dy * x * row_inv in one pass (up to kNormHold * 128 columns): a warp keeps the sums of its rows for its
+// columns in registers, the block adds its warps in shared memory, one atomic per column and block.  dw is zeroed before.
+template <int H>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy,
+                                                                 float* __restrict__ row_inv, float* __restrict__ dw, size_t rows, Vec4 a, float eps) {
+    __shared__ float4 part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cols = a.cols;
+    float4 acc[H];
+#pragma unroll
+    for (int j = 0; j < H; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (size_t row = (size_t)blockIdx.x * 8 + warp; row < rows; row += (size_t)gridDim.x * 8) {
+        const float* xr = x + row * (size_t)cols;
+        const float* gr = dy + row * (size_t)cols;
+        float4 h[H], gh[H];
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < H; ++j) h[j] = a.get(xr, 4 * (lane + 32 * j));
+#pragma unroll
+        for (int j = 0; j < H; ++j) gh[j] = a.get(gr, 4 * (lane + 32 * j));
+#pragma unroll
+        for (int j = 0; j < H; ++j) ss += dot4(h[j], h[j]);
+        const float inv = rsqrtf(warp_sum(ss) / (float)cols + eps);
+        if (lane == 0) row_inv[row] = inv;
+#pragma unroll
+        for (int j = 0; j < H; ++j) {
+            const float4 g = gh[j];
+            acc[j].x += g.x * h[j].x * inv; acc[j].y += g.y * h[j].y * inv;
+            acc[j].z += g.z * h[j].z * inv; acc[j].w += g.w * h[j].w * inv;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+        if (128 * j >= cols) break;
+        part[warp][lane] = acc[j];
+        __syncthreads();
+        if (threadIdx.x < 128 && 128 * j + (int)threadIdx.x < cols) {
+            float s = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += reinterpret_cast<const float*>(part[k])[threadIdx.x];
+            atomicAdd(dw + 128 * j + threadIdx.x, s);
+        }
+        __syncthreads();
     }
 }
 
@@ -110,90 +205,114 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_w_kernel(const float* __restr
 }
 
 // ---- swiglu ----------------------------------------------------------------------------------
+// W = 4: 128-bit accesses (hidden % 4 == 0, 16-byte aligned tensors); HBM-bound, 4096 x 768: 14 us with scalar accesses.
+__device__ __forceinline__ void swiglu_grads(float gate, float up, float go, float& dg, float& du) {
+    const float sig = 1.0f / (1.0f + expf(-gate));
+    dg = go * up * (sig + gate * sig * (1.0f - sig));
+    du = go * gate * sig;
+}
+template <int W>
 __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ packed, float* __restrict__ out,
                                                      size_t rows, int hidden) {
-    const size_t n = rows * (size_t)hidden;
+    const int hw = hidden / W;
+    const size_t n = rows * (size_t)hw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row = i / hidden;
-        const int col = (int)(i - row * hidden);
-        const float gate = packed[row * 2 * hidden + col];
-        const float up = packed[row * 2 * hidden + hidden + col];
-        const float sig = 1.0f / (1.0f + expf(-gate));
-        out[i] = gate * sig * up;
+        const size_t row = i / hw;
+        const size_t base = row * 2 * hidden + (i - row * hw) * W;
+        if (W == 4) {
+            const float4 g = __ldg(reinterpret_cast<const float4*>(packed + base)), u = __ldg(reinterpret_cast<const float4*>(packed + base + hidden));
+            reinterpret_cast<float4*>(out)[i] = make_float4(g.x * (1.0f / (1.0f + expf(-g.x))) * u.x, g.y * (1.0f / (1.0f + expf(-g.y))) * u.y,
+                                                            g.z * (1.0f / (1.0f + expf(-g.z))) * u.z, g.w * (1.0f / (1.0f + expf(-g.w))) * u.w);
+        } else {
+            const float gate = packed[base], up = packed[base + hidden];
+            const float sig = 1.0f / (1.0f + expf(-gate));
+            out[i] = gate * sig * up;
+        }
     }
 }
+template <int W>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* __restrict__ packed, const float* __restrict__ dy,
                                                          float* __restrict__ dpacked, size_t rows, int hidden) {
-    const size_t n = rows * (size_t)hidden;
+    const int hw = hidden / W;
+    const size_t n = rows * (size_t)hw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row = i / hidden;
-        const int col = (int)(i - row * hidden);
-        const size_t base = row * 2 * hidden;
-        const float gate = packed[base + col];
-        const float up = packed[base + hidden + col];
-        const float go = dy[i];
-        const float sig = 1.0f / (1.0f + expf(-gate));
-        dpacked[base + col] = go * up * (sig + gate * sig * (1.0f - sig));
-        dpacked[base + hidden + col] = go * gate * sig;
+        const size_t row = i / hw;
+        const size_t base = row * 2 * hidden + (i - row * hw) * W;
+        if (W == 4) {
+            const float4 g = __ldg(reinterpret_cast<const float4*>(packed + base)), u = __ldg(reinterpret_cast<const float4*>(packed + base + hidden));
+            const float4 go = __ldg(reinterpret_cast<const float4*>(dy) + i);
+            float4 a, b;
+            swiglu_grads(g.x, u.x, go.x, a.x, b.x); swiglu_grads(g.y, u.y, go.y, a.y, b.y);
+            swiglu_grads(g.z, u.z, go.z, a.z, b.z); swiglu_grads(g.w, u.w, go.w, a.w, b.w);
+            *reinterpret_cast<float4*>(dpacked + base) = a;
+            *reinterpret_cast<float4*>(dpacked + base + hidden) = b;
+        } else {
+            swiglu_grads(packed[base], packed[base + hidden], dy[i], dpacked[base], dpacked[base + hidden]);
+        }
     }
 }
 
 // ---- mean softmax cross-entropy --------------------------------------------------------------
-// A row of logits is read from HBM once: each of the 256 threads keeps its strided share (up to kCeHold values,
-// i.e. rows of up to 32768 classes; longer rows re-read the tail from memory) in registers for the max, sum
-// and gradient passes.
-constexpr int kCeHold = 128;
+// One block of 512 threads per row.  Maximum and sum of exponentials come from ONE pass: a thread keeps a running maximum and
+// the sum relative to it (four values at a time: one rescaling where a value exceeds the maximum), and the block combines the
+// pairs.  Backward reads the row a second time, from L2, and writes it: nothing of the row is kept in registers, so four rows
+// per SM are in flight.  HBM-bound.  4096 x 32000, with the row held in registers (one block of 256 threads per SM): forward
+// 255 us, backward 362 us.
+constexpr int kCeThreads = 512;
 
+__device__ __forceinline__ void online_add(float v, float& m, float& s) {
+    if (v > m) { s = s * expf(m - v) + 1.0f; m = v; }
+    else s += expf(v - m);
+}
 template <bool BACKWARD>
-__global__ void __launch_bounds__(256) ce_kernel(const float* __restrict__ logits, const int* __restrict__ targets,
-                                                 float* __restrict__ partial, const float* __restrict__ grad_out,
-                                                 float* __restrict__ grad_logits, size_t rows, int cols) {
+__global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict__ logits, const int* __restrict__ targets,
+                                                        float* __restrict__ partial, const float* __restrict__ grad_out,
+                                                        float* __restrict__ grad_logits, size_t rows, int cols, int vec) {
     __shared__ float red[32];
     const float gscale = BACKWARD ? grad_out[0] / (float)rows : 0.0f;
+    const int n4 = vec ? cols >> 2 : 0;            // 128-bit part; vec: rows start on 16-byte boundaries
     for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
         const float* l = logits + row * (size_t)cols;
-        float hold[kCeHold];
-        float m = -FLT_MAX;
-#pragma unroll
-        for (int j = 0; j < kCeHold; ++j) {
-            const int c = threadIdx.x + j * 256;
-            hold[j] = c < cols ? l[c] : -FLT_MAX;
-            m = fmaxf(m, hold[j]);
+        const float4* l4 = reinterpret_cast<const float4*>(l);
+        float m = -FLT_MAX, s = 0.0f;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < n4; i += kCeThreads) {
+            const float4 v = BACKWARD ? __ldg(l4 + i) : __ldcs(l4 + i);
+            const float mv = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+            if (mv > m) { s *= expf(m - mv); m = mv; }
+            s += (expf(v.x - m) + expf(v.y - m)) + (expf(v.z - m) + expf(v.w - m));
         }
-        for (int c = threadIdx.x + kCeHold * 256; c < cols; c += 256) m = fmaxf(m, l[c]);
+        for (int c = 4 * n4 + threadIdx.x; c < cols; c += kCeThreads) online_add(l[c], m, s);
+        const float mt = m;
         m = block_max(m, red);
-        float s = 0.0f;
-#pragma unroll
-        for (int j = 0; j < kCeHold; ++j) {
-            const int c = threadIdx.x + j * 256;
-            if (c < cols) {
-                hold[j] = expf(hold[j] - m);
-                s += hold[j];
-            }
-        }
-        for (int c = threadIdx.x + kCeHold * 256; c < cols; c += 256) s += expf(l[c] - m);
-        s = block_sum(s, red);
+        s = block_sum(s * expf(mt - m), red);
         const int t = targets[row];
         if (!BACKWARD) {
             if (threadIdx.x == 0) partial[row] = (t < 0 || t >= cols) ? 0.0f : logf(s) + m - l[t];
         } else {
             const float inv = 1.0f / s;
             float* g = grad_logits + row * (size_t)cols;
-#pragma unroll
-            for (int j = 0; j < kCeHold; ++j) {
-                const int c = threadIdx.x + j * 256;
-                if (c < cols) g[c] = gscale * (hold[j] * inv - (c == t ? 1.0f : 0.0f));
+            float4* g4 = reinterpret_cast<float4*>(g);
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n4; i += kCeThreads) {
+                const float4 v = __ldcs(l4 + i);
+                const int c = 4 * i;
+                __stcs(g4 + i, make_float4(gscale * (expf(v.x - m) * inv - (c == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.y - m) * inv - (c + 1 == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.z - m) * inv - (c + 2 == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.w - m) * inv - (c + 3 == t ? 1.0f : 0.0f))));
             }
-            for (int c = threadIdx.x + kCeHold * 256; c < cols; c += 256)
+            for (int c = 4 * n4 + threadIdx.x; c < cols; c += kCeThreads)
                 g[c] = gscale * (expf(l[c] - m) * inv - (c == t ? 1.0f : 0.0f));
         }
     }
 }
-__global__ void __launch_bounds__(256) mean_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n,
+__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n,
                                                    size_t denom) {
     __shared__ float red[32];
     float s = 0.0f;
-    for (size_t i = threadIdx.x; i < n; i += blockDim.x) s += in[i];
+#pragma unroll 4
+    for (size_t i = threadIdx.x; i < n; i += 1024) s += in[i];
     s = block_sum(s, red);
     if (threadIdx.x == 0) out[0] = denom > 0 ? s / (float)denom : 0.0f;
 }
@@ -212,7 +331,9 @@ __device__ __forceinline__ void key_range(const GqaDims& p, int tq, int& k0, int
     if (k0 > k1) k0 = k1;
 }
 
-// ---- attention as batched fp32 products + a row pass ------------------------------------------
+#include "attention.cuh"
+
+// ---- attention as batched fp32 products + a row pass (head sizes above 64, or few queries over many keys) ------------------------------------------
 // The seven products of attention forward and backward (S = scale*Q K^T, O = P V, dP = dO V^T,
 // dq = scale*dS K, dv = P^T dO, dk = scale*dS^T Q) are one batched, strided, shared-memory-tiled
 // SIMT fp32 product; exact fp32 FMAs, no tensor cores (tf32 would not hold the reference's fp32
@@ -394,42 +515,74 @@ __global__ void __launch_bounds__(256) position_backward_kernel(const float* __r
         grad_position[i] = acc;
     }
 }
-// Rotary embedding on x [batch*tokens, channels] with n_head heads of head_dim at the front of each row; one thread
-// per rotated pair.  split_half pairs (i, i + head_dim/2), otherwise (2i, 2i+1).  inverse negates the angle.
-__global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, float* __restrict__ out, size_t rows, int tokens,
+// Rotary embedding on x [batch*tokens, channels] with n_head heads of head_dim at the front of each row.  split_half pairs
+// (i, i + head_dim/2), otherwise (2i, 2i+1).  inverse negates the angle.  Block = one token position: sines and cosines of its
+// pairs are formed once (powf and sincosf cost 15 us per call when every element formed its own) and serve the rows of
+// that position in all batch elements of the block's share.
+__global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
                                                    int channels, int n_head, int head_dim, int rotary_dim, int token_offset,
-                                                   float theta, int inverse, int split_half) {
-    const size_t n = rows * (size_t)channels;
+                                                   float theta, int inverse, int split_half, int shared_turns) {
+    extern __shared__ float2 rot[];                   // (cos, sin) of pair i
     int rd = rotary_dim <= 0 ? head_dim : rotary_dim;
     rd = rd < head_dim ? rd : head_dim;
     rd -= rd & 1;
-    const int half = head_dim >> 1;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row = i / channels;
-        const int c = (int)(i - row * channels);
-        const int head = c / head_dim, d = c - head * head_dim;
-        if (head >= n_head) continue;                 // the shaders leave such channels unwritten
-        int pair, lo, hi;                             // pair index and the two channels it rotates
-        bool first;
-        if (split_half) {
-            if (half <= 0 || d >= half * 2) { out[i] = x[i]; continue; }
-            pair = d < half ? d : d - half;
-            if (pair >= (rd >> 1)) { out[i] = x[i]; continue; }
-            lo = pair; hi = half + pair; first = d < half;
-        } else {
-            if (d >= rd) { out[i] = x[i]; continue; }
-            pair = d >> 1;
-            lo = d & ~1; hi = lo + 1; first = d == lo;
-        }
-        const int token = (int)(row % tokens);
-        const float exponent = (float)(2 * pair) / (float)head_dim;
+    const int half = head_dim >> 1, token = blockIdx.x;
+    const int per = (batch + (int)gridDim.y - 1) / (int)gridDim.y, b0 = (int)blockIdx.y * per, b1 = min(batch, b0 + per);
+    auto turn = [&](int i) {
+        const float exponent = (float)(2 * i) / (float)head_dim;
         float angle = (float)(token_offset + token) / powf(theta, exponent);
         if (inverse) angle = -angle;
         float sn, cs;
         sincosf(angle, &sn, &cs);
-        const size_t base = row * (size_t)channels + (size_t)head * head_dim;
-        const float a = x[base + lo], b = x[base + hi];
-        out[i] = first ? a * cs - b * sn : (split_half ? b * cs + a * sn : a * sn + b * cs);
+        return make_float2(cs, sn);
+    };
+    const size_t step = (size_t)tokens * channels;    // the same position of the next batch element
+    const float* xp = x + (size_t)token * channels + b0 * step;
+    float* op = out + (size_t)token * channels + b0 * step;
+    bool formed = false;
+    for (int c0 = 0; c0 < channels; c0 += 256) {
+        const int c = c0 + (int)threadIdx.x;
+        const int head = c / head_dim, d = c - head * head_dim;
+        const bool mine = c < channels && head < n_head;      // the shaders leave channels beyond the heads unwritten
+        int pair = -1, other = 0;                     // pair index and the channel this one is rotated with
+        bool first = true;
+        if (split_half) {
+            if (half > 0 && d < half * 2) {
+                pair = d < half ? d : d - half;
+                first = d < half;
+                other = first ? c + half : c - half;
+            }
+        } else if (d < rd) {
+            pair = d >> 1;
+            first = (d & 1) == 0;
+            other = first ? c + 1 : c - 1;
+        }
+        const bool turned = pair >= 0 && pair < (rd >> 1);
+        for (int b = b0; b < b1 || !formed; b += 4) {
+            float me[4], ot[4];                       // four batch elements in flight
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const bool in = mine && b + k < b1;
+                me[k] = in ? xp[(size_t)(b - b0 + k) * step + c] : 0.0f;
+                ot[k] = in && turned ? xp[(size_t)(b - b0 + k) * step + other] : 0.0f;
+            }
+            if (!formed) {
+                if (shared_turns)
+                    for (int i = threadIdx.x; i < rd >> 1; i += 256) rot[i] = turn(i);
+                __syncthreads();
+                formed = true;
+            }
+            if (!mine) continue;
+            if (turned) {
+                const float2 t = shared_turns ? rot[pair] : turn(pair);
+                const float cs = t.x, sn = t.y;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) me[k] = first ? me[k] * cs - ot[k] * sn : (split_half ? me[k] * cs + ot[k] * sn : ot[k] * sn + me[k] * cs);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (b + k < b1) op[(size_t)(b - b0 + k) * step + c] = me[k];
+        }
     }
 }
 __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ param, const float* __restrict__ grad, float* __restrict__ m,
@@ -459,22 +612,44 @@ int row_grid(size_t rows, int sm_count) {
 
 }  // namespace
 
+namespace {
+bool all16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
+    return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+int warp_row_grid(size_t rows, int sm_count) {
+    const size_t b = (rows + 7) / 8, cap = (size_t)sm_count * 8;
+    return (int)(b < cap ? b : cap);
+}
+}  // namespace
+
 cudaError_t launch_rmsnorm(const float* x, const float* w, float* out, size_t rows, int cols, float eps, int sm_count,
                            cudaStream_t stream) {
-    rmsnorm_kernel<<<row_grid(rows, sm_count), 128, 0, stream>>>(x, w, out, nullptr, rows, cols, eps);
+    const Vec4 a = {cols % 4 == 0 && all16(x, w, out), cols};
+    if (cols <= 384) rmsnorm_kernel<3><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, out, nullptr, rows, a, eps);
+    else rmsnorm_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, out, nullptr, rows, a, eps);
     return cudaGetLastError();
 }
 cudaError_t launch_rmsnorm_backward_x(const float* x, const float* w, const float* dy, float* dx, size_t rows, int cols,
                                       float eps, int sm_count, cudaStream_t stream) {
-    rmsnorm_bwd_x_kernel<<<row_grid(rows, sm_count), 128, 0, stream>>>(x, w, dy, dx, rows, cols, eps);
+    const Vec4 a = {cols % 4 == 0 && all16(x, w, dy, dx), cols};
+    if (cols <= 384) rmsnorm_bwd_x_kernel<3><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, dy, dx, rows, a, eps);
+    else rmsnorm_bwd_x_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, dy, dx, rows, a, eps);
     return cudaGetLastError();
 }
 cudaError_t launch_rmsnorm_backward_weight(const float* x, const float* dy, float* row_inv, float* dw, size_t rows,
                                            int cols, float eps, int sm_count, cudaStream_t stream) {
-    rmsnorm_kernel<<<row_grid(rows, sm_count), 128, 0, stream>>>(x, nullptr, nullptr, row_inv, rows, cols, eps);
-    cudaError_t e = cudaGetLastError();
+    const Vec4 a = {cols % 4 == 0 && all16(x, dy), cols};
+    cudaError_t e = cudaMemsetAsync(dw, 0, (size_t)cols * sizeof(float), stream);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(dw, 0, (size_t)cols * sizeof(float), stream);
+    if (cols <= kNormHold * 128) {
+        const size_t b = (rows + 7) / 8, cap = 2 * (size_t)sm_count;      // every block ends in one atomic per column
+        const int grid = (int)(b < cap ? b : cap);
+        if (cols <= 384) rmsnorm_bwd_w_rows_kernel<3><<<grid, 256, 0, stream>>>(x, dy, row_inv, dw, rows, a, eps);
+        else rmsnorm_bwd_w_rows_kernel<kNormHold><<<grid, 256, 0, stream>>>(x, dy, row_inv, dw, rows, a, eps);
+        return cudaGetLastError();
+    }
+    rmsnorm_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, nullptr, nullptr, row_inv, rows, a, eps);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int col_blocks = (cols + 31) / 32;
     size_t splits = ((size_t)sm_count * 4 + col_blocks - 1) / col_blocks;
@@ -487,31 +662,31 @@ cudaError_t launch_rmsnorm_backward_weight(const float* x, const float* dy, floa
 }
 cudaError_t launch_swiglu(const float* packed, float* out, size_t rows, int hidden, int sm_count, cudaStream_t stream) {
     const size_t n = rows * (size_t)hidden;
-    size_t blocks = (n + 255) / 256;
-    if (blocks > (size_t)sm_count * 16) blocks = (size_t)sm_count * 16;
-    swiglu_kernel<<<(int)blocks, 256, 0, stream>>>(packed, out, rows, hidden);
+    if (hidden % 4 == 0 && all16(packed, out)) swiglu_kernel<4><<<flat_grid(n / 4, sm_count), 256, 0, stream>>>(packed, out, rows, hidden);
+    else swiglu_kernel<1><<<flat_grid(n, sm_count), 256, 0, stream>>>(packed, out, rows, hidden);
     return cudaGetLastError();
 }
 cudaError_t launch_swiglu_backward(const float* packed, const float* dy, float* dpacked, size_t rows, int hidden,
                                    int sm_count, cudaStream_t stream) {
     const size_t n = rows * (size_t)hidden;
-    size_t blocks = (n + 255) / 256;
-    if (blocks > (size_t)sm_count * 16) blocks = (size_t)sm_count * 16;
-    swiglu_bwd_kernel<<<(int)blocks, 256, 0, stream>>>(packed, dy, dpacked, rows, hidden);
+    if (hidden % 4 == 0 && all16(packed, dy, dpacked)) swiglu_bwd_kernel<4><<<flat_grid(n / 4, sm_count), 256, 0, stream>>>(packed, dy, dpacked, rows, hidden);
+    else swiglu_bwd_kernel<1><<<flat_grid(n, sm_count), 256, 0, stream>>>(packed, dy, dpacked, rows, hidden);
     return cudaGetLastError();
 }
 cudaError_t launch_softmax_cross_entropy(const float* logits, const int* targets, float* partial, float* out, size_t rows,
                                          int cols, int sm_count, cudaStream_t stream) {
-    ce_kernel<false><<<row_grid(rows, sm_count), 256, 0, stream>>>(logits, targets, partial, nullptr, nullptr, rows, cols);
+    ce_kernel<false><<<row_grid(rows, sm_count), kCeThreads, 0, stream>>>(logits, targets, partial, nullptr, nullptr, rows, cols,
+                                                                          cols % 4 == 0 && all16(logits, nullptr));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    mean_kernel<<<1, 256, 0, stream>>>(partial, out, rows, rows);
+    mean_kernel<<<1, 1024, 0, stream>>>(partial, out, rows, rows);
     return cudaGetLastError();
 }
 cudaError_t launch_softmax_cross_entropy_backward(const float* logits, const int* targets, const float* grad_out,
                                                   float* grad_logits, size_t rows, int cols, int sm_count,
                                                   cudaStream_t stream) {
-    ce_kernel<true><<<row_grid(rows, sm_count), 256, 0, stream>>>(logits, targets, nullptr, grad_out, grad_logits, rows, cols);
+    ce_kernel<true><<<row_grid(rows, sm_count), kCeThreads, 0, stream>>>(logits, targets, nullptr, grad_out, grad_logits, rows, cols,
+                                                                         cols % 4 == 0 && all16(logits, grad_logits));
     return cudaGetLastError();
 }
 
@@ -536,9 +711,13 @@ cudaError_t launch_position_backward(const float* grad_out, float* grad_position
 cudaError_t launch_rope(const float* x, float* out, size_t rows, int tokens, int channels, int n_head, int head_dim,
                         int rotary_dim, int token_offset, float theta, int inverse, int split_half, int sm_count,
                         cudaStream_t stream) {
-    rope_kernel<<<flat_grid(rows * (size_t)channels, sm_count), 256, 0, stream>>>(x, out, rows, tokens, channels, n_head, head_dim,
-                                                                                  rotary_dim, token_offset, theta, inverse,
-                                                                                  split_half);
+    const int batch = (int)(rows / (size_t)tokens);
+    int by = (8 * sm_count + tokens - 1) / tokens;     // blocks per position: eight blocks per SM where the batch allows it
+    if (by > batch) by = batch;
+    if (by > 65535) by = 65535;
+    const int shared_turns = head_dim <= 8192;         // 32 KB of them at most
+    rope_kernel<<<dim3((unsigned)tokens, (unsigned)by), 256, shared_turns ? (size_t)(head_dim / 2 + 1) * sizeof(float2) : 0, stream>>>(
+        x, out, batch, tokens, channels, n_head, head_dim, rotary_dim, token_offset, theta, inverse, split_half, shared_turns);
     return cudaGetLastError();
 }
 cudaError_t launch_adam(float* param, const float* grad, float* m, float* v, size_t n, float lr, float beta1, float beta2,
@@ -547,11 +726,59 @@ cudaError_t launch_adam(float* param, const float* grad, float* m, float* v, siz
     return cudaGetLastError();
 }
 
-// scores_ws: batch*n_head*tq*tk floats of scratch.
+namespace {
+template <typename K>
+cudaError_t with_smem(K kern, size_t bytes) {      // attribute set once per kernel and device
+    return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+// The tiled kernels walk over the keys of a query tile one tile after another: right for any number of keys while there are
+// enough query tiles to fill the device, and up to 1024 keys in any case.
+bool gqa_tiled(int batch, int tq, int tk, int n_head, int hd, int vhd) {
+    return hd <= 64 && vhd == hd && tq <= 65535 * 32 && tk <= 65535 * 64 && (tk <= 1024 || (long long)batch * n_head * ((tq + 63) / 64) >= 148);
+}
+template <int BQ, int NC>
+cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* out, const GqaDims& p, cudaStream_t stream) {
+    constexpr size_t bytes = fwd_floats<BQ, NC>() * 4;
+    cudaError_t e = with_smem(gqa_fwd_kernel<BQ, NC>, bytes);
+    if (e != cudaSuccess) return e;
+    gqa_fwd_kernel<BQ, NC><<<dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), 4 * BQ, bytes, stream>>>(q, k, v, out, p);
+    return cudaGetLastError();
+}
+template <int BQ, int NC>
+cudaError_t run_gqa_bwd(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, float* dk,
+                        float* dv, const GqaDims& p, cudaStream_t stream) {
+    constexpr size_t bq = bwd_q_floats<BQ, NC>() * 4, bk = bwd_k_floats<NC>() * 4;
+    cudaError_t e = with_smem(gqa_bwd_q_kernel<BQ, NC>, bq);
+    if (e == cudaSuccess) e = with_smem(gqa_bwd_k_kernel<NC>, bk);
+    if (e != cudaSuccess) return e;
+    gqa_bwd_q_kernel<BQ, NC><<<dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), 4 * BQ, bq, stream>>>(q, k, v, dout, probs, ds, dq, p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    gqa_bwd_k_kernel<NC><<<dim3(p.batch * p.n_kv, (p.tk + kKT - 1) / kKT), 256, bk, stream>>>(q, dout, probs, ds, dk, dv, p);
+    return cudaGetLastError();
+}
+// query tiles of 64 rows, or of 32 where 64 would leave SMs without a second CTA
+bool wide_q(const GqaDims& p) { return (long long)p.batch * p.n_head * ((p.tq + 63) / 64) >= 2 * 148; }
+}  // namespace
+
+size_t gqa_forward_scratch_floats(int batch, int tq, int tk, int n_head, int hd, int vhd) {
+    return gqa_tiled(batch, tq, tk, n_head, hd, vhd) ? 0 : (size_t)batch * n_head * tq * tk;
+}
+
+// scores_ws: gqa_forward_scratch_floats() floats of scratch.
 cudaError_t launch_gqa_forward(const float* q, const float* k, const float* v, float* out, int batch, int tq, int tk,
                                int key_stride, int n_head, int n_kv, int hd, int vhd, int causal, int q_off, int window,
                                float scale, float* scores_ws, cudaStream_t stream, int* launches) {
     GqaDims p{batch, tq, tk, key_stride, n_head, n_kv, hd, vhd, causal, q_off, window, scale};
+    if (gqa_tiled(batch, tq, tk, n_head, hd, vhd)) {
+        *launches += 1;
+        const bool w = wide_q(p);
+        switch ((hd + 15) / 16) {
+            case 1: return w ? run_gqa_fwd<64, 1>(q, k, v, out, p, stream) : run_gqa_fwd<32, 1>(q, k, v, out, p, stream);
+            case 2: return w ? run_gqa_fwd<64, 2>(q, k, v, out, p, stream) : run_gqa_fwd<32, 2>(q, k, v, out, p, stream);
+            case 3: return w ? run_gqa_fwd<64, 3>(q, k, v, out, p, stream) : run_gqa_fwd<32, 3>(q, k, v, out, p, stream);
+            default: return w ? run_gqa_fwd<64, 4>(q, k, v, out, p, stream) : run_gqa_fwd<32, 4>(q, k, v, out, p, stream);
+        }
+    }
     const int group = n_head / n_kv;
     const long long qc = (long long)n_head * hd, kc = (long long)n_kv * hd, vc = (long long)n_kv * vhd, oc = (long long)n_head * vhd;
     const long long plane = (long long)tq * tk;
@@ -579,6 +806,18 @@ cudaError_t launch_gqa_backward(const float* q, const float* k, const float* v, 
                                 float* dq, float* dk, float* dv, int batch, int tq, int tk, int n_head, int n_kv, int hd,
                                 int causal, int q_off, float scale, cudaStream_t stream, int* launches) {
     GqaDims p{batch, tq, tk, tk, n_head, n_kv, hd, hd, causal, q_off, 0, scale};
+    if (gqa_tiled(batch, tq, tk, n_head, hd, hd)) {
+        *launches += 2;
+        const bool w = wide_q(p);
+#define MCL_GQA_BWD(NC) (w ? run_gqa_bwd<64, NC>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream) : run_gqa_bwd<32, NC>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream))
+        switch ((hd + 15) / 16) {
+            case 1: return MCL_GQA_BWD(1);
+            case 2: return MCL_GQA_BWD(2);
+            case 3: return MCL_GQA_BWD(3);
+            default: return MCL_GQA_BWD(4);
+        }
+#undef MCL_GQA_BWD
+    }
     const int group = n_head / n_kv;
     const long long qc = (long long)n_head * hd, kc = (long long)n_kv * hd;
     const long long plane = (long long)tq * tk;
