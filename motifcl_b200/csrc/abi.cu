@@ -1,5 +1,6 @@
 // C-ABI layer of libmotifcl_cuda.so: contexts, argument checks, dispatch to the kernels.
 // The declarations and the reference interfaces they replace are in include/motifcl_cuda.h.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -242,47 +243,171 @@ bool layer_wanted(const mcl_cuda_ctx* ctx, size_t tokens, size_t I, size_t O) {
 
 #define MCL_CU(ctx, what, call) do { cudaError_t _e = (call); if (_e != cudaSuccess) return fail_cuda(ctx, what, _e); } while (0)
 
-// Tensor-core products on fp16 terms (tc_gemm.cu).  A call carves the terms of its tensors from the workspace, clears one
-// pair of magnitude words per tensor, fills the terms, and runs its products.
+// Tensor-core products on fp16 terms (tc_gemm.cu).  A call carves the terms of its tensors from the workspace, fills them, and
+// runs its products.
 struct TermBuf { size_t planes, scaled, words; size_t rows; int cols, ld; };
-size_t term_bytes(size_t rows, int ld) { return 2 * rows * (size_t)ld * 2 + mcl::kTermPad; }
-TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled, size_t words) {
-    TermBuf t = {0, 0, words, rows, (int)cols, up8(cols)};
-    if (plain) t.planes = cv->reserve(term_bytes(rows, t.ld));
-    if (scaled) t.scaled = cv->reserve(term_bytes(rows, t.ld));
+size_t term_bytes(size_t rows, size_t cols) { return 2 * rows * (size_t)up8(cols) * 2 + mcl::kTermPad; }
+size_t digit_bytes(size_t O, size_t I) { return O * (size_t)up8(I) * 2 + mcl::kTermPad; }
+TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled) {
+    TermBuf t = {0, 0, 0, rows, (int)cols, up8(cols)};
+    t.words = cv->reserve(16);
+    if (plain) t.planes = cv->reserve(term_bytes(rows, cols));
+    if (scaled) t.scaled = cv->reserve(term_bytes(rows, cols));
     return t;
 }
-int fill_terms(mcl_cuda_ctx* ctx, const char* op, char* w, const TermBuf& t, const float* src, const float* col_scale, bool plain) {
-    cudaError_t e = mcl::launch_split_terms(src, (int)t.rows, t.cols, t.ld, col_scale, plain ? w + t.planes : nullptr,
-                                            col_scale ? w + t.scaled : nullptr, reinterpret_cast<uint32_t*>(w + t.words),
-                                            ctx->sm_count, ctx->stream);
-    if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-    ctx->launches += 2;
-    return MCL_CUDA_OK;
+// col_scale != null: the scaled terms are made too
+mcl::SplitDesc split_of(char* w, const TermBuf& t, const float* src, const float* col_scale, bool plain) {
+    mcl::SplitDesc d = {src, (int)t.rows, t.cols, t.ld, col_scale, plain ? w + t.planes : nullptr, col_scale ? w + t.scaled : nullptr,
+                        reinterpret_cast<uint32_t*>(w + t.words)};
+    return d;
 }
 mcl::TcOperand terms_of(char* w, const TermBuf& t, bool scaled, bool mn_major) {
     mcl::TcOperand o = {w + (scaled ? t.scaled : t.planes), (int)t.rows, t.cols, t.ld, 2, mn_major ? 1 : 0,
-                        reinterpret_cast<const uint32_t*>(w + t.words) + (scaled ? 1 : 0)};
+                        reinterpret_cast<const uint32_t*>(w + t.words) + (scaled ? 2 : 0)};
     return o;
 }
 mcl::TcOperand digits_of(const char* T, size_t O, size_t I, bool mn_major) {
     mcl::TcOperand o = {T, (int)O, (int)I, up8(I), 1, mn_major ? 1 : 0, nullptr};
     return o;
 }
-constexpr size_t kWordBytes = 64;      // magnitude words of a call: one pair per tensor, 8 bytes each
+#define MCL_TC(ctx, op, call) do { int _n = 0; cudaError_t _e = (call); (ctx)->launches += _n; if (_e != cudaSuccess) return fail_cuda(ctx, op, _e); } while (0)
 
 // plan of a product with ternary digits (depth unbounded: exact digits) or of two split tensors
 mcl::TcPlan digit_plan(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) { return mcl::tc_plan((int)M, (int)N, (int)K, 2, ctx->sm_count, 0); }
 mcl::TcPlan dense_plan(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
     return mcl::tc_plan((int)M, (int)N, (int)K, 3, ctx->sm_count, mcl::kGradDepthLimit);
 }
-int tc_product(mcl_cuda_ctx* ctx, const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K,
-               const float* col_scale, float* splitk_ws, const mcl::TcPlan& plan) {
-    int launches = 0;
-    cudaError_t e = mcl::launch_tc_gemm(a, b, c, (int)M, (int)N, (int)K, plan, col_scale, splitk_ws, ctx->err_word,
-                                        ctx->max_smem, ctx->sm_count, ctx->stream, &launches);
-    ctx->launches += launches;
-    if (e != cudaSuccess) return fail_cuda(ctx, "tensor-core contraction", e);
+mcl::TcProblem tc_problem(const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K, const mcl::TcPlan& plan,
+                          const float* col_scale, void* splitk_ws) {
+    mcl::TcProblem q = {a, b, c, (int)M, (int)N, (int)K, plan, col_scale, static_cast<float*>(splitk_ws)};
+    return q;
+}
+int tc_product(mcl_cuda_ctx* ctx, const char* op, const mcl::TcProblem& q) {
+    MCL_TC(ctx, op, mcl::launch_tc_products(&q, 1, ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream, &_n));
+    if (q.plan.splits > 1)
+        MCL_LAUNCH(ctx, op, mcl::launch_splitk_reduce(q.splitk_ws, q.c, q.col_scale, q.M, q.N, q.N, q.plan.splits, ctx->stream));
+    return MCL_CUDA_OK;
+}
+int split_tensors(mcl_cuda_ctx* ctx, const char* op, const mcl::SplitDesc* d, int n) {
+    MCL_TC(ctx, op, mcl::launch_split_terms(d, n, ctx->sm_count, ctx->stream, &_n));
+    return MCL_CUDA_OK;
+}
+
+// Y, dX and dW of several layers; the ternary digits come from the packed 6-bit state or, when state == NULL, from the 2-bit
+// words.  y, grad_x, grad_w may be NULL.
+struct ProductLayer {
+    const float* x;
+    const float* grad_out;
+    const uint8_t* state;
+    const uint32_t* packed2;
+    const float* scale;
+    float* y;
+    float* grad_x;
+    float* grad_w;
+    size_t I, O, Nt;
+};
+size_t layer_term_bytes(const ProductLayer& L) {
+    return (L.y || L.grad_w ? term_bytes(L.Nt, L.I) : 0) + (L.grad_w ? term_bytes(L.Nt, L.O) : 0) + (L.grad_x ? term_bytes(L.Nt, L.O) : 0) +
+           (L.y || L.grad_x ? digit_bytes(L.O, L.I) : 0);
+}
+// One chunk of layers.  w == null: returns in *bytes the workspace it needs; else runs it.
+int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, size_t n, size_t C, char* w, size_t* bytes) {
+    std::vector<TermBuf> xb(n), gb(n);
+    std::vector<size_t> t_off(n, 0);
+    std::vector<mcl::TcProblem> pr;
+    std::vector<size_t> k_off;
+    Carver cv;
+    // dW of many layers: a CTA or a pair per tile, whichever takes less in sum
+    int dw_cg = 1;
+    const int min_items = (int)((3 * (size_t)ctx->sm_count + n - 1) / n);
+    if (n > 1) {
+        double cost[2] = {0, 0};
+        for (size_t i = 0; i < n; ++i)
+            for (int cg = 1; cg <= 2 && L[i].grad_w; ++cg)
+                cost[cg - 1] += mcl::tc_plan_shared((int)L[i].O, (int)L[i].I, (int)L[i].Nt, 3, cg, mcl::kGradDepthLimit, min_items).cost;
+        dw_cg = cost[1] < cost[0] ? 2 : 1;
+    }
+    auto row_plan = [&](size_t M, size_t N, size_t K) {
+        return n == 1 ? digit_plan(ctx, M, N, K) : mcl::tc_plan_shared((int)M, (int)N, (int)K, 2, M > 128 ? 2 : 1, 0, 0);
+    };
+    for (size_t i = 0; i < n; ++i) {
+        const ProductLayer& l = L[i];
+        xb[i] = carve_terms(&cv, l.Nt, l.I, l.y || l.grad_w, false);
+        gb[i] = carve_terms(&cv, l.Nt, l.O, l.grad_w != nullptr, l.grad_x != nullptr);
+        if (l.y || l.grad_x) t_off[i] = cv.reserve(digit_bytes(l.O, l.I));
+    }
+    for (size_t i = 0; i < n; ++i) {
+        const ProductLayer& l = L[i];
+        auto add = [&](const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K, const mcl::TcPlan& plan, const float* cs) {
+            k_off.push_back(plan.splits > 1 ? cv.reserve(plan.workspace_bytes) : 0);
+            pr.push_back(tc_problem(a, b, c, M, N, K, plan, cs, w + k_off.back()));
+        };
+        if (l.y) add(terms_of(w, xb[i], false, false), digits_of(w + t_off[i], l.O, l.I, false), l.y, l.Nt, l.O, l.I, row_plan(l.Nt, l.O, l.I), l.scale);
+        if (l.grad_x) add(terms_of(w, gb[i], true, false), digits_of(w + t_off[i], l.O, l.I, true), l.grad_x, l.Nt, l.I, l.O, row_plan(l.Nt, l.I, l.O), nullptr);
+        if (l.grad_w)
+            add(terms_of(w, gb[i], false, true), terms_of(w, xb[i], false, true), l.grad_w, l.O, l.I, l.Nt,
+                n == 1 ? dense_plan(ctx, l.O, l.I, l.Nt)
+                       : mcl::tc_plan_shared((int)l.O, (int)l.I, (int)l.Nt, 3, dw_cg, mcl::kGradDepthLimit, min_items), nullptr);
+    }
+    if (!w) { *bytes = cv.off; return MCL_CUDA_OK; }
+    std::vector<mcl::SplitDesc> sd;
+    std::vector<mcl::ExpandDesc> ed;
+    for (size_t i = 0; i < n; ++i) {
+        const ProductLayer& l = L[i];
+        if (l.y || l.grad_w) sd.push_back(split_of(w, xb[i], l.x, nullptr, true));
+        if (l.grad_x || l.grad_w) sd.push_back(split_of(w, gb[i], l.grad_out, l.grad_x ? l.scale : nullptr, l.grad_w != nullptr));
+        if (l.y || l.grad_x) {
+            const mcl::ExpandDesc d = {l.state, l.packed2, (int)l.O, (int)l.I, up8(l.I), w + t_off[i]};
+            ed.push_back(d);
+        }
+    }
+    MCL_TRY(split_tensors(ctx, op, sd.data(), (int)sd.size()));
+    if (!ed.empty()) MCL_TC(ctx, op, mcl::launch_expand_ternary(ed.data(), (int)ed.size(), (int)C, ctx->sm_count, ctx->stream, &_n));
+    // products of one kind together, the longest items first (they are dealt round-robin)
+    std::stable_sort(pr.begin(), pr.end(), [](const mcl::TcProblem& a, const mcl::TcProblem& b) {
+        const int ta = a.b.planes + 1, tb = b.b.planes + 1;
+        if (ta != tb) return ta > tb;
+        if (a.plan.pair != b.plan.pair) return a.plan.pair > b.plan.pair;
+        return (long long)ta * a.plan.ktiles_per_split * a.plan.bn > (long long)tb * b.plan.ktiles_per_split * b.plan.bn;
+    });
+    MCL_TC(ctx, op, mcl::launch_tc_products(pr.data(), (int)pr.size(), ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream, &_n));
+    std::vector<const float*> part;
+    std::vector<float*> out;
+    std::vector<long long> elems;
+    std::vector<int> splits;
+    for (const mcl::TcProblem& q : pr) {
+        if (q.plan.splits <= 1) continue;
+        if (q.col_scale) {
+            MCL_LAUNCH(ctx, op, mcl::launch_splitk_reduce(q.splitk_ws, q.c, q.col_scale, q.M, q.N, q.N, q.plan.splits, ctx->stream));
+            continue;
+        }
+        part.push_back(q.splitk_ws); out.push_back(q.c); elems.push_back((long long)q.M * q.N); splits.push_back(q.plan.splits);
+    }
+    if (!part.empty())
+        MCL_TC(ctx, op, mcl::launch_splitk_reduce_group(part.data(), out.data(), elems.data(), splits.data(), (int)part.size(), ctx->sm_count, ctx->stream, &_n));
+    return MCL_CUDA_OK;
+}
+// Layers go together while their terms fit kChunkBytes.
+constexpr size_t kChunkBytes = (size_t)6 << 30;
+int products_group(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, size_t n, size_t C) {
+    std::vector<size_t> ends;
+    size_t need = 0;
+    for (size_t i = 0; i < n;) {
+        size_t k = i, sum = 0;
+        while (k < n && (k == i || sum + layer_term_bytes(L[k]) <= kChunkBytes)) sum += layer_term_bytes(L[k++]);
+        size_t b = 0;
+        MCL_TRY(products_chunk(ctx, op, L + i, k - i, C, nullptr, &b));
+        if (b > need) need = b;
+        ends.push_back(k);
+        i = k;
+    }
+    void* wsp = nullptr;
+    MCL_TRY(ws_reserve(ctx, need, &wsp));
+    size_t i = 0;
+    for (size_t e : ends) {
+        MCL_TRY(products_chunk(ctx, op, L + i, e - i, C, static_cast<char*>(wsp), nullptr));
+        i = e;
+    }
     return MCL_CUDA_OK;
 }
 
@@ -528,20 +653,8 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
         return MCL_CUDA_OK;
     }
     if (tc_wanted(ctx, batch, out_features, in_features, y, scale)) {
-        const mcl::TcPlan plan = digit_plan(ctx, batch, out_features, in_features);
-        Carver cv;
-        const size_t o_w = cv.reserve(kWordBytes);
-        const TermBuf xb = carve_terms(&cv, batch, in_features, true, false, o_w);
-        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2 + mcl::kTermPad), o_k = cv.reserve(plan.workspace_bytes);
-        void* wsp = nullptr;
-        MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
-        char* w = static_cast<char*>(wsp);
-        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
-        MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
-                                                       up8(in_features), ctx->sm_count, ctx->stream));
-        return tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, out_features, in_features, false), y, batch,
-                          out_features, in_features, scale, reinterpret_cast<float*>(w + o_k), plan);
+        const ProductLayer l = {x, nullptr, state, nullptr, scale, y, nullptr, nullptr, in_features, out_features, batch};
+        return products_group(ctx, op, &l, 1, C);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_forward(x, state, scale, y, (int)batch, (int)in_features,
                                                          (int)out_features, (int)C, ctx->stream));
@@ -566,20 +679,8 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
         return MCL_CUDA_OK;
     }
     if (tc_wanted(ctx, batch, in_features, out_features, grad_x)) {
-        const mcl::TcPlan plan = digit_plan(ctx, batch, in_features, out_features);
-        Carver cv;
-        const size_t o_w = cv.reserve(kWordBytes);
-        const TermBuf gb = carve_terms(&cv, batch, out_features, false, true, o_w);
-        const size_t o_t = cv.reserve(out_features * (size_t)up8(in_features) * 2 + mcl::kTermPad), o_k = cv.reserve(plan.workspace_bytes);
-        void* wsp = nullptr;
-        MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
-        char* w = static_cast<char*>(wsp);
-        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
-        MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, scale, false));
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, nullptr, (int)C, (int)out_features, (int)in_features, w + o_t,
-                                                       up8(in_features), ctx->sm_count, ctx->stream));
-        return tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, out_features, in_features, true), grad_x, batch,
-                          in_features, out_features, nullptr, reinterpret_cast<float*>(w + o_k), plan);
+        const ProductLayer l = {nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, in_features, out_features, batch};
+        return products_group(ctx, op, &l, 1, C);
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_backward_input(state, scale, grad_out, grad_x, (int)batch,
                                                                 (int)in_features, (int)out_features,
@@ -666,13 +767,12 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     mcl::TcPlan plan = {};
     Carver cv;
     const size_t o_gw = cv.reserve(tile_rows * row_b);
-    size_t o_k = 0, o_w = 0;
+    size_t o_k = 0;
     TermBuf gb, xb;
     if (tc) {
         plan = dense_plan(ctx, tile_rows, in_features, batch);
-        o_w = cv.reserve(kWordBytes);
-        gb = carve_terms(&cv, batch, out_features, true, false, o_w);      // activation-sized, not weight-sized
-        xb = carve_terms(&cv, batch, in_features, true, false, o_w + 8);
+        gb = carve_terms(&cv, batch, out_features, true, false);      // activation-sized, not weight-sized
+        xb = carve_terms(&cv, batch, in_features, true, false);
         o_k = cv.reserve(plan.workspace_bytes);
     }
     void* wsp = nullptr;
@@ -680,9 +780,8 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     char* w = static_cast<char*>(wsp);
     float* gw = reinterpret_cast<float*>(w + o_gw);
     if (tc) {
-        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
-        MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, nullptr, true));
-        MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
+        const mcl::SplitDesc sd[2] = {split_of(w, gb, grad_out, nullptr, true), split_of(w, xb, x, nullptr, true)};
+        MCL_TRY(split_tensors(ctx, op, sd, 2));
     }
     for (size_t r0 = 0; r0 < out_features; r0 += tile_rows) {
         const size_t nr = (out_features - r0 < tile_rows) ? out_features - r0 : tile_rows;
@@ -690,8 +789,7 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
             mcl::TcOperand a = terms_of(w, gb, false, true);
             a.ptr = static_cast<const char*>(a.ptr) + r0 * 2;
             a.cols = (int)nr;
-            MCL_TRY(tc_product(ctx, a, terms_of(w, xb, false, true), gw, nr, in_features, batch, nullptr,
-                               reinterpret_cast<float*>(w + o_k), plan));
+            MCL_TRY(tc_product(ctx, op, tc_problem(a, terms_of(w, xb, false, true), gw, nr, in_features, batch, plan, nullptr, w + o_k)));
         } else {
             MCL_LAUNCH(ctx, "counter update (grad_w tile)",
                        mcl::launch_simt_grad_w(grad_out, x, gw, (int)batch, (int)in_features,
@@ -702,84 +800,6 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
                                                C, in_features, nr, r0, lr, lr_scale, rms_beta, rms_eps, seed);
         if (rc != MCL_CUDA_OK) return rc;
     }
-    return MCL_CUDA_OK;
-}
-
-// Y, dX and dW of one linear; the ternary digits come from the packed 6-bit state or, when
-// state == NULL, from the 2-bit packed weights.
-// Narrow layers take the grouped kernel that splits fp32 operands in shared memory (tc_fused.cu):
-// every column tile of a product converts its A slab again, so the form pays while a layer has few
-// column tiles; wide layers amortise the pre-split planes of tc_gemm.cu better.
-static bool fused_wanted(const mcl_cuda_ctx* ctx, const float* x, const float* grad_out, const void* ternary,
-                         const float* scale, const float* y, const float* grad_x, const float* grad_w, size_t I,
-                         size_t O, size_t Nt) {
-    (void)ternary;
-    if (I % 32 != 0 || O % 32 != 0 || Nt % 4 != 0 || I > 1024 || O > 1024) return false;
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(grad_out) |
-                           reinterpret_cast<uintptr_t>(scale) | reinterpret_cast<uintptr_t>(y) |
-                           reinterpret_cast<uintptr_t>(grad_x) | reinterpret_cast<uintptr_t>(grad_w);
-    if (bits & 15) return false;
-    return 200 * (size_t)1024 <= ctx->max_smem;
-}
-
-static int fused_products(mcl_cuda_ctx* ctx, const char* op, const float* x, const float* grad_out,
-                          const uint8_t* state, const uint32_t* packed2, const float* scale, float* y,
-                          float* grad_x, float* grad_w, size_t C, size_t I, size_t O, size_t Nt) {
-    mcl::FusedProblem pr[3];
-    mcl::FusedOperand oa[3], ob[3];
-    int n = 0, i_dw = -1;
-    size_t k_floats = 0;
-    // the kernel's split-K slices are 32 deep; the depth limit is stated in k-tiles of 64
-    const int depth = mcl::kFusedDwDepth;
-    auto add = [&](int mode, int M, int N, int K) {
-        mcl::FusedProblem& p = pr[n];
-        p = mcl::FusedProblem();
-        p.mode = mode; p.M = M; p.N = N; p.K = K;
-        return &p;
-    };
-    auto operand = [](const float* p, size_t rows, size_t cols, int mn, int box_outer) {
-        mcl::FusedOperand o = {p, (int)rows, (int)cols, (int)cols, mn, box_outer};
-        return o;
-    };
-    if (grad_w) {      // the long work items (K = tokens) first
-        mcl::FusedProblem* p = add(mcl::kFusedDW, (int)O, (int)I, (int)Nt);
-        p->C = grad_w; p->ldc = (int)I;
-        k_floats = mcl::fused_plan(p, ctx->sm_count, depth);
-        oa[n] = operand(grad_out, Nt, O, 1, 4); ob[n] = operand(x, Nt, I, 1, p->BN / 32); i_dw = n++;
-    }
-    if (y) {
-        mcl::FusedProblem* p = add(mcl::kFusedY, (int)Nt, (int)O, (int)I);
-        p->col_scale = scale; p->C = y; p->ldc = (int)O;
-        mcl::fused_plan(p, 0, 0);
-        oa[n] = operand(x, Nt, I, 0, 128); ob[n] = operand(nullptr, O, I, 0, p->BN); ++n;
-    }
-    if (grad_x) {
-        mcl::FusedProblem* p = add(mcl::kFusedDX, (int)Nt, (int)I, (int)O);
-        p->a_kscale = scale; p->C = grad_x; p->ldc = (int)I;
-        mcl::fused_plan(p, 0, 0);
-        oa[n] = operand(grad_out, Nt, O, 0, 128); ob[n] = operand(nullptr, O, I, 1, p->BN / 32); ++n;
-    }
-    Carver cv;
-    const size_t o_t = cv.reserve((y || grad_x) ? O * I * 4 : 0);
-    const size_t o_k = cv.reserve(k_floats * 4);
-    void* wsp = nullptr;
-    MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
-    char* w = static_cast<char*>(wsp);
-    if (y || grad_x) {   // the ternary digits as fp32: the exact operand of Y and dX
-        float* T = reinterpret_cast<float*>(w + o_t);
-        MCL_LAUNCH(ctx, op, mcl::launch_ternary_f32(state, packed2, (int)C, (int)O, (int)I, T, ctx->sm_count, ctx->stream));
-        for (int i = 0; i < n; ++i)
-            if (pr[i].mode != mcl::kFusedDW) ob[i].ptr = T;
-    }
-    if (i_dw >= 0 && pr[i_dw].splits > 1) pr[i_dw].C = reinterpret_cast<float*>(w + o_k);
-    int launches = 0;
-    cudaError_t e = mcl::launch_tc_fused(pr, oa, ob, n, ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream,
-                                         &launches);
-    ctx->launches += launches;
-    if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-    if (i_dw >= 0 && pr[i_dw].splits > 1)
-        MCL_LAUNCH(ctx, op, mcl::launch_splitk_reduce(reinterpret_cast<const float*>(w + o_k), grad_w, nullptr, (int)O, (int)I,
-                                                      (int)I, pr[i_dw].splits, ctx->stream));
     return MCL_CUDA_OK;
 }
 
@@ -799,32 +819,8 @@ static int linear_products(mcl_cuda_ctx* ctx, const char* op, const float* x, co
         if (grad_w) MCL_TRY(mcl_cuda_matmul_f32(ctx, grad_out, x, grad_w, O, Nt, I, 1, 0));
         return MCL_CUDA_OK;
     }
-    if (fused_wanted(ctx, x, grad_out, state ? static_cast<const void*>(state) : packed2, scale, y, grad_x, grad_w, I, O, Nt))
-        return fused_products(ctx, op, x, grad_out, state, packed2, scale, y, grad_x, grad_w, C, I, O, Nt);
-    const mcl::TcPlan p_y = digit_plan(ctx, Nt, O, I), p_x = digit_plan(ctx, Nt, I, O), p_w = dense_plan(ctx, O, I, Nt);
-    size_t k_max = 0;
-    if (y) k_max = p_y.workspace_bytes;
-    if (grad_x && p_x.workspace_bytes > k_max) k_max = p_x.workspace_bytes;
-    if (grad_w && p_w.workspace_bytes > k_max) k_max = p_w.workspace_bytes;
-    Carver cv;
-    const size_t o_w = cv.reserve(kWordBytes);
-    const TermBuf xb = carve_terms(&cv, Nt, I, y || grad_w, false, o_w);
-    const TermBuf gb = carve_terms(&cv, Nt, O, grad_w != nullptr, grad_x != nullptr, o_w + 8);
-    const size_t o_t = cv.reserve(O * (size_t)up8(I) * 2 + mcl::kTermPad);
-    const size_t o_k = cv.reserve(k_max);
-    void* wsp = nullptr;
-    MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
-    char* w = static_cast<char*>(wsp);
-    float* kws = reinterpret_cast<float*>(w + o_k);
-    MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
-    if (y || grad_w) MCL_TRY(fill_terms(ctx, op, w, xb, x, nullptr, true));
-    if (grad_x || grad_w) MCL_TRY(fill_terms(ctx, op, w, gb, grad_out, grad_x ? scale : nullptr, grad_w != nullptr));
-    if (y || grad_x)
-        MCL_LAUNCH(ctx, op, mcl::launch_expand_ternary(state, packed2, (int)C, (int)O, (int)I, w + o_t, up8(I), ctx->sm_count, ctx->stream));
-    if (y) MCL_TRY(tc_product(ctx, terms_of(w, xb, false, false), digits_of(w + o_t, O, I, false), y, Nt, O, I, scale, kws, p_y));
-    if (grad_x) MCL_TRY(tc_product(ctx, terms_of(w, gb, true, false), digits_of(w + o_t, O, I, true), grad_x, Nt, I, O, nullptr, kws, p_x));
-    if (grad_w) MCL_TRY(tc_product(ctx, terms_of(w, gb, false, true), terms_of(w, xb, false, true), grad_w, O, I, Nt, nullptr, kws, p_w));
-    return MCL_CUDA_OK;
+    const ProductLayer l = {x, grad_out, state, packed2, scale, y, grad_x, grad_w, I, O, Nt};
+    return products_group(ctx, op, &l, 1, C);
 }
 
 int mcl_cuda_counter_linear_step(mcl_cuda_ctx* ctx, const float* x, const float* grad_out,
@@ -889,10 +885,8 @@ int mcl_cuda_counter_linear_step_many(mcl_cuda_ctx* ctx, const mcl_cuda_linear_d
         }
         if (L.row_offset + L.update_rows > L.out_features)
             return fail(ctx, MCL_CUDA_EINVAL, "counter linear step (many): update rows exceed out_features");
-        const bool tc = tc_wanted(ctx, L.batch, L.out_features, L.in_features);
-        const void* tern = L.state ? static_cast<const void*>(L.state) : L.packed2_in;
-        if (tc && fused_wanted(ctx, L.x, L.grad_out, tern, L.scale, L.y, L.grad_x, L.grad_w, L.in_features, L.out_features,
-                               L.batch))
+        if (tc_wanted(ctx, L.batch, L.out_features, L.in_features, L.y, L.scale) && tc_wanted(ctx, L.batch, L.in_features, L.out_features, L.grad_x) &&
+            tc_wanted(ctx, L.out_features, L.in_features, L.batch, L.grad_w))
             grouped.push_back(i);
         else
             single.push_back(i);
@@ -910,142 +904,15 @@ int mcl_cuda_counter_linear_step_many(mcl_cuda_ctx* ctx, const mcl_cuda_linear_d
                                              lr_scale, rms_beta, rms_eps, seed));
     }
     if (grouped.empty()) return MCL_CUDA_OK;
-    const int depth = mcl::kFusedDwDepth;
     const size_t ng = grouped.size();
-    // with many layers in flight the K splits of dW only have to respect the accumulation depth
-    const int target_items = (int)((2 * (size_t)ctx->sm_count + ng - 1) / ng);
-    std::vector<mcl::FusedProblem> pr;
-    std::vector<mcl::FusedOperand> oa, ob;
-    std::vector<size_t> t_off(ng), k_off(ng);
-    std::vector<int> dw_splits(ng, 1);
-    Carver cv;
-    auto operand = [](const float* p, size_t rows, size_t cols, int mn, int box_outer) {
-        mcl::FusedOperand o = {p, (int)rows, (int)cols, (int)cols, mn, box_outer};
-        return o;
-    };
-    for (size_t gi = 0; gi < ng; ++gi) {
-        const mcl_cuda_linear_desc& L = layers[grouped[gi]];
-        t_off[gi] = cv.reserve((L.y || L.grad_x) ? L.out_features * L.in_features * 4 : 0);
-        if (!L.grad_w) { k_off[gi] = cv.reserve(0); continue; }
-        mcl::FusedProblem p = mcl::FusedProblem();
-        p.mode = mcl::kFusedDW; p.M = (int)L.out_features; p.N = (int)L.in_features; p.K = (int)L.batch;
-        k_off[gi] = cv.reserve(mcl::fused_plan(&p, target_items, depth) * 4);
-        dw_splits[gi] = p.splits;
+    std::vector<ProductLayer> pl;
+    for (size_t gi : grouped) {
+        const mcl_cuda_linear_desc& L = layers[gi];
+        const ProductLayer l = {L.x, L.grad_out, L.state, L.packed2_in, L.scale, L.y, L.grad_x, L.grad_w, L.in_features, L.out_features, L.batch};
+        pl.push_back(l);
     }
-    void* wsp = nullptr;
-    MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
-    char* w = static_cast<char*>(wsp);
-    // 1. ternary digits of every layer with a row product, as bf16: T [O][I] in the first half of the layer's block,
-    // its transpose after it
-    {
-        std::vector<const uint8_t*> st;
-        std::vector<const uint32_t*> p2;
-        std::vector<void*> T, Tt;
-        std::vector<int> Os, Is;
-        for (size_t gi = 0; gi < ng; ++gi) {
-            const mcl_cuda_linear_desc& L = layers[grouped[gi]];
-            if (!L.y && !L.grad_x) continue;
-            st.push_back(L.state); p2.push_back(L.packed2_in);
-            T.push_back(w + t_off[gi]); Tt.push_back(w + t_off[gi] + L.out_features * L.in_features * 2);
-            Os.push_back((int)L.out_features); Is.push_back((int)L.in_features);
-        }
-        int launches = 0;
-        cudaError_t e = st.empty() ? cudaSuccess
-                                   : mcl::launch_ternary_bf16_group(st.data(), p2.data(), T.data(), Tt.data(), Os.data(), Is.data(), (int)st.size(), (int)C,
-                                                                    ctx->sm_count, ctx->stream, &launches);
-        ctx->launches += launches;
-        if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-    }
-    // 2. all products.  The weight-gradient products (tf32 terms, K = tokens, long work items) and the row products
-    // (bf16 terms against the bf16 digits, 64-deep k-tiles) run in launches of their own: their tiles differ in size,
-    // and a launch sizes its rings for the largest tile of its table.
-    {
-        auto flush = [&]() -> cudaError_t {
-            if (pr.empty()) return cudaSuccess;
-            int launches = 0;
-            cudaError_t e = mcl::launch_tc_fused(pr.data(), oa.data(), ob.data(), (int)pr.size(), ctx->err_word, ctx->max_smem,
-                                                 ctx->sm_count, ctx->stream, &launches);
-            ctx->launches += launches;
-            pr.clear(); oa.clear(); ob.clear();
-            return e;
-        };
-        auto operand_bf16 = [](const void* p, size_t rows, size_t cols, int box_outer) {
-            mcl::FusedOperand o = {static_cast<const float*>(p), (int)rows, (int)cols, (int)cols, 0, box_outer, 1};
-            return o;
-        };
-        for (size_t gi = 0; gi < ng; ++gi) {
-            const mcl_cuda_linear_desc& L = layers[grouped[gi]];
-            const size_t I = L.in_features, O = L.out_features, Nt = L.batch;
-            if (!L.grad_w) continue;
-            mcl::FusedProblem p = mcl::FusedProblem();
-            p.mode = mcl::kFusedDW; p.M = (int)O; p.N = (int)I; p.K = (int)Nt;
-            mcl::fused_plan(&p, target_items, depth);
-            p.C = p.splits > 1 ? reinterpret_cast<float*>(w + k_off[gi]) : L.grad_w; p.ldc = (int)I;
-            pr.push_back(p); oa.push_back(operand(L.grad_out, Nt, O, 1, 4)); ob.push_back(operand(L.x, Nt, I, 1, p.BN / 32));
-            if (pr.size() == (size_t)mcl::kFusedMaxProblems) {
-                cudaError_t e = flush();
-                if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-            }
-        }
-        {
-            cudaError_t e = flush();
-            if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-        }
-        // row products: launches of equal size
-        size_t n_row = 0;
-        for (size_t gi = 0; gi < ng; ++gi) n_row += (layers[grouped[gi]].y ? 1 : 0) + (layers[grouped[gi]].grad_x ? 1 : 0);
-        const size_t n_launch = (n_row + mcl::kFusedMaxProblems - 1) / mcl::kFusedMaxProblems;
-        const size_t per_launch = n_launch ? (n_row + n_launch - 1) / n_launch : 0;
-        for (size_t gi = 0; gi < ng; ++gi) {
-            const mcl_cuda_linear_desc& L = layers[grouped[gi]];
-            const size_t I = L.in_features, O = L.out_features, Nt = L.batch;
-            const char* T = w + t_off[gi];
-            const char* Tt = T + O * I * 2;
-            mcl::FusedProblem p;
-            if (L.y) {
-                p = mcl::FusedProblem();
-                p.mode = mcl::kFusedYB; p.M = (int)Nt; p.N = (int)O; p.K = (int)I;
-                p.col_scale = L.scale; p.C = L.y; p.ldc = (int)O;
-                mcl::fused_plan(&p, 0, 0);
-                pr.push_back(p); oa.push_back(operand(L.x, Nt, I, 0, 128)); ob.push_back(operand_bf16(T, O, I, p.BN));
-            }
-            if (L.grad_x) {
-                p = mcl::FusedProblem();
-                p.mode = mcl::kFusedDXB; p.M = (int)Nt; p.N = (int)I; p.K = (int)O;
-                p.a_kscale = L.scale; p.C = L.grad_x; p.ldc = (int)I;
-                mcl::fused_plan(&p, 0, 0);
-                pr.push_back(p); oa.push_back(operand(L.grad_out, Nt, O, 0, 128)); ob.push_back(operand_bf16(Tt, I, O, p.BN));
-            }
-            if (pr.size() + 2 > per_launch || pr.size() + 2 > (size_t)mcl::kFusedMaxProblems) {
-                cudaError_t e = flush();
-                if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-            }
-        }
-        cudaError_t e = flush();
-        if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-    }
-    // 3. split-K reductions of dW
-    {
-        std::vector<const float*> part;
-        std::vector<float*> out;
-        std::vector<int> elems, splits;
-        for (size_t gi = 0; gi < ng; ++gi) {
-            if (dw_splits[gi] <= 1) continue;
-            const mcl_cuda_linear_desc& L = layers[grouped[gi]];
-            part.push_back(reinterpret_cast<const float*>(w + k_off[gi]));
-            out.push_back(L.grad_w);
-            elems.push_back((int)(L.out_features * L.in_features));
-            splits.push_back(dw_splits[gi]);
-        }
-        if (!part.empty()) {
-            int launches = 0;
-            cudaError_t e = mcl::launch_splitk_reduce_group(part.data(), out.data(), elems.data(), splits.data(), (int)part.size(),
-                                                            ctx->sm_count, ctx->stream, &launches);
-            ctx->launches += launches;
-            if (e != cudaSuccess) return fail_cuda(ctx, op, e);
-        }
-    }
-    // 4. updates
+    MCL_TRY(products_group(ctx, op, pl.data(), ng, C));
+    // the updates of all layers
     {
         std::vector<mcl::UpdateDesc> ud;
         for (size_t gi = 0; gi < ng; ++gi) {
@@ -1152,19 +1019,16 @@ int mcl_cuda_matmul_f32(mcl_cuda_ctx* ctx, const float* a, const float* b, float
     if (tc_wanted(ctx, M, N, K, c)) {
         const mcl::TcPlan plan = dense_plan(ctx, M, N, K);
         Carver cv;
-        const size_t o_w = cv.reserve(kWordBytes);
         // a stored [M,K] or (trans_a) [K,M], b stored [K,N] or (trans_b) [N,K]: split as stored, read in the needed orientation
-        const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false, o_w);
-        const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false, o_w + 8);
+        const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false);
+        const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false);
         const size_t o_k = cv.reserve(plan.workspace_bytes);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
-        MCL_CU(ctx, op, cudaMemsetAsync(w + o_w, 0, kWordBytes, ctx->stream));
-        MCL_TRY(fill_terms(ctx, op, w, ab, a, nullptr, true));
-        MCL_TRY(fill_terms(ctx, op, w, bb, b, nullptr, true));
-        return tc_product(ctx, terms_of(w, ab, false, trans_a != 0), terms_of(w, bb, false, trans_b == 0), c, M, N, K, nullptr,
-                          reinterpret_cast<float*>(w + o_k), plan);
+        const mcl::SplitDesc sd[2] = {split_of(w, ab, a, nullptr, true), split_of(w, bb, b, nullptr, true)};
+        MCL_TRY(split_tensors(ctx, op, sd, 2));
+        return tc_product(ctx, op, tc_problem(terms_of(w, ab, false, trans_a != 0), terms_of(w, bb, false, trans_b == 0), c, M, N, K, plan, nullptr, w + o_k));
     }
     MCL_LAUNCH(ctx, op, mcl::launch_simt_matmul_f32(a, b, c, (int)M, (int)K, (int)N, trans_a, trans_b, ctx->stream));
     return MCL_CUDA_OK;

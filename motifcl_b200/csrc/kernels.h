@@ -63,8 +63,9 @@ cudaError_t launch_simt_grad_w(const float* grad_out, const float* x, float* gra
                                cudaStream_t stream);
 
 // tc_gemm.cu -- tcgen05 / TMEM / TMA contractions on fp16 term planes (see the file header)
-struct TcPlan { int pair, bn, splits, ktiles_per_split; size_t workspace_bytes; };
+struct TcPlan { int pair, bn, splits, ktiles_per_split; size_t workspace_bytes; double cost; };
 TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit);
+TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items);
 // k-tiles of 64 per accumulator for fp32 x fp32 products: 3 x 4 instructions per k-tile add into it, each with a truncation
 // error of about 2.7e-9 relative (K = 4096: 2e-6)
 constexpr int kGradDepthLimit = 64;
@@ -74,75 +75,38 @@ struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major 
     int rows, cols, ld;
     int planes;                // 2: hi and lo terms of an fp32 tensor; 1: ternary digits
     int mn_major;              // the contraction runs over the rows (0: over the columns)
-    const uint32_t* amax;      // bits of the split tensor's largest magnitude (null for digits)
+    const uint32_t* words;     // magnitude words of the split tensor (null for digits)
 };
-// C[M,N] = sum over k of A B (b.planes == 1: two products, b.planes == 2: three)
-cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int M, int N, int K, const TcPlan& plan,
-                           const float* col_scale, float* splitk_ws, int* err_word, size_t max_smem, int sm_count,
-                           cudaStream_t stream, int* launches);
-// fp32 [R,Cc] -> fp16 terms [2][R][ld] of src (planes) and / or of src . col_scale (planes_s); amax: two zeroed words that
-// receive the largest magnitudes of the two.  Two launches.
-cudaError_t launch_split_terms(const float* src, int R, int Cc, int ld, const float* col_scale, void* planes, void* planes_s,
-                               uint32_t* amax, int sm_count, cudaStream_t stream);
-// ternary digits as fp16 [O][ld], from the 6-bit state (state != null) or the 2-bit words (I % 16 == 0, ld == I)
-cudaError_t launch_expand_ternary(const uint8_t* state, const uint32_t* packed2, int C, int O, int I, void* T, int ld,
-                                  int sm_count, cudaStream_t stream);
-
-// tc_fused.cu -- grouped tcgen05 (tf32, two terms) contractions straight from fp32 tensors
-// kFusedYB / kFusedDXB are Y and dX with the activation split into two bf16 terms and the ternary digits given
-// as a K-major bf16 matrix (T [out,in] for Y, its transpose [in,out] for dX): k-tiles of 64, kind::f16
-enum { kFusedY = 0, kFusedDX = 1, kFusedDW = 2, kFusedYB = 3, kFusedDXB = 4 };
-constexpr int kFusedMaxProblems = 63;
-// dW on tf32 terms: 3 products x 4 instructions per 32-deep k-tile add into one accumulator, each with a truncation error of
-// ~2e-8 relative; 16 k-tiles (512 tokens) keep that below 4e-6
-#ifndef MCL_FUSED_FLUSH
-#define MCL_FUSED_FLUSH 16
-#endif
-#ifndef MCL_FUSED_DW_DEPTH
-#define MCL_FUSED_DW_DEPTH 64
-#endif
-constexpr int kFusedFlushKtiles = MCL_FUSED_FLUSH;
-// k-tiles (of 32 tokens) of one dW work item: longer items mean fewer split-K partials to write and add up
-constexpr int kFusedDwDepth = MCL_FUSED_DW_DEPTH;
-struct FusedOperand {          // a row-major tensor read through TMA (host side only)
-    const float* ptr;          // fp32 elements, or bf16 ones when `bf16` is set
+// C[M,N] = sum over k of A B (b.planes == 1: two products, b.planes == 2: three); with plan.splits > 1 into splitk_ws
+// [splits][M][N], which a reduction adds up
+struct TcProblem {
+    TcOperand a, b;
+    float* c;
+    int M, N, K;
+    TcPlan plan;
+    const float* col_scale;    // of the output's columns (plan.splits == 1)
+    float* splitk_ws;
+};
+cudaError_t launch_tc_products(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream,
+                               int* launches);
+struct SplitDesc {             // fp32 [rows, cols] -> fp16 terms [2][rows][ld] of src (planes) and / or of src . col_scale (planes_s)
+    const float* src;
     int rows, cols, ld;
-    int mn_major;              // read as a transposed operand (cols % 32 == 0): 32-byte-atom swizzle, 3-D box
-    int box_outer;             // rows of the box (K-major) or 32-column chunks per box (MN-major)
-    int bf16;                  // K-major bf16 matrix: box of 64 elements x box_outer rows
+    const float* col_scale;
+    void* planes;
+    void* planes_s;
+    uint32_t* words;           // four words: magnitude and exact maximum of the two
 };
-struct FusedProblem {          // C[M,N] = A[M,K] . B[N,K]^T, see the kinds in tc_fused.cu
-    const float* a_kscale;     // DX: A is multiplied by a_kscale[k] (rounded to fp32) before the split
-    const float* col_scale;    // optional scale of output column n (ignored for split-K partials)
-    float* C;                  // [M, ldc], or split-K partials [splits][M][ldc]
-    int M, N, K, ldc;
-    int mode;
-    int BN, tiles_m, tiles_n, splits, ktiles_per_split;   // filled by fused_plan (k-tiles of 32)
-    int nprod;                 // products per k-tile
-    int flush;                 // k-tiles (of 32) one accumulator takes before the epilogue adds it to the output; 0 = the whole item
-    uint32_t prod;             // 4 bits each: A term | B term << 2 (0 = hi, 1 = lo), smallest first
-    int a_map, b_map, item_begin;                         // filled by the launcher
+cudaError_t launch_split_terms(const SplitDesc* d, int n, int sm_count, cudaStream_t stream, int* launches);
+struct ExpandDesc {            // ternary digits as fp16 [O][ld], from the 6-bit state (state != null) or the 2-bit words (I % 16 == 0, ld == I)
+    const uint8_t* state;
+    const uint32_t* packed2;
+    int O, I, ld;
+    void* T;
 };
-// chooses the column tile and the K split of a problem; returns the floats of split-K workspace it needs
-size_t fused_plan(FusedProblem* p, int target_items, int depth_limit);
-// err_word points at two ints: the error word and the work-item counter (zeroed by the launcher)
-cudaError_t launch_tc_fused(const FusedProblem* probs, const FusedOperand* a_ops, const FusedOperand* b_ops, int n,
-                            int* err_word, size_t max_smem, int sm_count, cudaStream_t stream, int* launches);
-// ternary digits of a layer as fp32 [O][I], from the 6-bit state (state != null) or the 2-bit words
-cudaError_t launch_ternary_f32(const uint8_t* state, const uint32_t* packed2, int C, int O, int I, float* T,
-                               int sm_count, cudaStream_t stream);
-// grouped forms: one launch for the layers of a step
-cudaError_t launch_ternary_f32_group(const uint8_t* const* state, const uint32_t* const* packed2, float* const* T, const int* O, const int* I, int n, int C,
-                                     int sm_count, cudaStream_t stream, int* launches);
-cudaError_t launch_splitk_reduce_group(const float* const* partial, float* const* out, const int* elements, const int* splits,
+cudaError_t launch_expand_ternary(const ExpandDesc* d, int n, int C, int sm_count, cudaStream_t stream, int* launches);
+cudaError_t launch_splitk_reduce_group(const float* const* partial, float* const* out, const long long* elements, const int* splits,
                                        int n, int sm_count, cudaStream_t stream, int* launches);
-// ternary digits of the layers as bf16, both orientations: T [O][I] and Tt [I][O]
-cudaError_t launch_ternary_bf16_group(const uint8_t* const* state, const uint32_t* const* packed2, void* const* T, void* const* Tt,
-                                      const int* O, const int* I, int n, int C, int sm_count, cudaStream_t stream, int* launches);
-// tc_gemm.cu: TMA map of a row-major fp32 matrix, 128-byte swizzle, zero fill outside
-bool tc_encode_map_f32(void* map, const float* base, int cols, int rows, int ld, int mn_major, int box_outer);
-// the same for a K-major bf16 matrix: box of 64 elements x box_outer rows
-bool tc_encode_map_bf16(void* map, const void* base, int cols, int rows, int ld, int box_outer);
 cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* col_scale, int M, int N, int ldc,
                                  int splits, cudaStream_t stream);
 

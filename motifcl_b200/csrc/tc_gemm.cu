@@ -35,24 +35,45 @@ constexpr int kMaxStages = 8;
 constexpr int kATileBytes = BM * BK * 2;   // 16 KiB
 constexpr int kLoShift = 12;               // lo terms are stored 2^12 up
 
-struct TcParams {
+// One product of a launch's table.
+struct TcTile {
     const float* col_scale;   // optional, applied when splits == 1
-    const uint32_t* a_amax;   // bits of the largest magnitude of the split tensor (null: operand is unscaled)
-    const uint32_t* b_amax;
+    const uint32_t* a_words;  // magnitude words of the split tensor (null: operand is unscaled)
+    const uint32_t* b_words;
     int M, N, K;
-    int BN, stages, b_bytes;   // b_bytes: one CTA's share of a B tile
+    int BN, stage_bytes;      // tile width; bytes of one ring slot (A tile and this CTA's share of B)
     int a_mn, b_mn;           // operand is stored with M / N contiguous
     int nterms;               // 2: A lo, A hi against one B plane; 3: lo.hi, hi.lo, hi.hi
     int ktiles_per_split, splits;
-    int group_m;
-    int* err;
+    int tiles_m, tiles_n, group_m;
+    int item_begin;           // first work item of the product
 };
+// The table is a kernel argument: 60 products with their tensor maps are 28 KB.
+template <int CAP>
+struct TcTable {
+    int n, n_items, stages, slot_bytes, acc_cols;
+    int* err;
+    TcTile p[CAP];
+    CUtensorMap maps[3 * CAP];      // A, B, C of product i at 3 i
+};
+constexpr int kTcCap = 60;
 
 // exponent of f (see the file header): the largest magnitude lands in [2^14, 2^15)
 __device__ __forceinline__ int term_exp(uint32_t amax_bits) {
     const int e = (int)(amax_bits >> 23);
     const int s = 141 - (e < 1 ? 1 : e);
     return s > 126 ? 126 : s;
+}
+// Exponent that a tensor's terms were made with.  words[0]: magnitude that f was chosen for (the largest of a sample, raised
+// by 2^kSampleRoom, or the exact maximum); words[1]: the exact maximum, found while splitting.  fp16 holds two binades more
+// than words[0] lands in; a tensor whose exact maximum lies beyond them is split again for it.
+__device__ __forceinline__ bool terms_redone(uint32_t w0, uint32_t w1) {
+    const int e0 = (int)(w0 >> 23);
+    return (int)(w1 >> 23) >= (e0 < 1 ? 1 : e0) + 2;
+}
+__device__ __forceinline__ int terms_exp(const uint32_t* words) {
+    const uint32_t w0 = __ldg(words), w1 = __ldg(words + 1);
+    return term_exp(terms_redone(w0, w1) ? w1 : w0);
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
@@ -126,24 +147,28 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 
-// item -> output tile and K slice.  Groups of group_m row tiles run through all column tiles before the next group, so
-// that the CTAs in flight share both operands' tiles in L2.
-struct TcItem { int mt, nt, split; };
-__device__ __forceinline__ TcItem tc_item(int item, int tiles_m, int tiles_n, int group_m) {
+// item -> product, output tile and K slice.  Groups of group_m row tiles run through all column tiles before the next group, so
+// that the CTAs in flight share both operands' tiles in L2.  `pi` only moves forward.
+struct TcItem { int mt, nt, split, kt0, nkt; };
+__device__ __forceinline__ TcItem tc_item(const TcTile* tab, int n, int item, int& pi) {
+    while (pi + 1 < n && item >= tab[pi + 1].item_begin) ++pi;
+    const TcTile& P = tab[pi];
     TcItem t;
-    const int per_split = tiles_m * tiles_n;
-    t.split = item / per_split;
-    int r = item - t.split * per_split;
-    const int per_group = group_m * tiles_n;
+    const int per_split = P.tiles_m * P.tiles_n, local = item - P.item_begin;
+    t.split = local / per_split;
+    int r = local - t.split * per_split;
+    const int per_group = P.group_m * P.tiles_n;
     const int g = r / per_group;
     r -= g * per_group;
-    const int gm = min(group_m, tiles_m - g * group_m);
+    const int gm = min(P.group_m, P.tiles_m - g * P.group_m);
     t.nt = r / gm;
-    t.mt = g * group_m + (r - t.nt * gm);
+    t.mt = g * P.group_m + (r - t.nt * gm);
+    t.kt0 = t.split * P.ktiles_per_split;
+    t.nkt = min(P.ktiles_per_split, (P.K + BK - 1) / BK - t.kt0);
     return t;
 }
 
-// Persistent CTAs of 192 threads; work items (output tile x split-K slice) are dealt round-robin.
+// Persistent CTAs of 192 threads; the work items of all products of the table (output tile x split-K slice) are dealt round-robin.
 //   warp 0        TMA producer (one elected lane): tiles of A and B into a ring of `stages` shared-memory slots
 //   warp 1        MMA issuer (one elected lane): four tcgen05.mma (K = 16 each) per slot; also allocates / frees TMEM
 //   warps 2..5    epilogue: tcgen05.ld of 32 lanes x 64 columns, scale, a swizzled 32 x 32 tile in shared memory, TMA store
@@ -159,41 +184,39 @@ __device__ __forceinline__ TcItem tc_item(int item, int tiles_m, int tiles_n, in
 // Every mbarrier wait is bounded: on time-out the kernel records an error word, skips the rest of its work, frees
 // its TMEM and returns.
 constexpr int kTcThreads = 192;
-constexpr int kSmemSlotTcPair = 16;       // ensure_dynamic_smem: see there
 constexpr int kStageBytes = 8 * 4096;      // epilogue staging: two 32 x 32 float tiles per warp
 
-template <int CG>
-__global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                             const __grid_constant__ CUtensorMap tmB,
-                                                             const __grid_constant__ CUtensorMap tmC,
-                                                             const TcParams p) {
+template <int CG, int CAP>
+__global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ TcTable<CAP> tab) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4];
+    __shared__ TcTile sp[CAP];      // the roles walk the table at every item; the constant bank is too small a cache for it
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int BN = p.BN, S = p.stages;
+    const int S = tab.stages, n_items = tab.n_items;
     const uint32_t rank = CG == 2 ? (blockIdx.x & 1u) : 0u;      // cluster of two consecutive CTAs
     const int unit = (int)blockIdx.x / CG, n_units = (int)gridDim.x / CG;
     const uint32_t staging = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t tiles = staging + kStageBytes;
-    const uint32_t stage_bytes = kATileBytes + (uint32_t)p.b_bytes;
+    const uint32_t slot_bytes = (uint32_t)tab.slot_bytes;
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
     auto acc_full = [&](int a) { return bar0 + 8u * (2 * kMaxStages + a); };
     auto acc_empty = [&](int a) { return bar0 + 8u * (2 * kMaxStages + 2 + a); };
-    uint32_t acc_cols = 32;                       // columns of one accumulator (power of two >= BN)
-    while ((int)acc_cols < BN) acc_cols <<= 1;
-    const uint32_t tmem_cols = 2 * acc_cols;      // <= 512
+    const uint32_t acc_cols = (uint32_t)tab.acc_cols;      // of one accumulator: a power of two >= the widest BN
+    const uint32_t tmem_cols = 2 * acc_cols;               // <= 512
 
-    const int tiles_n = (p.N + BN - 1) / BN, tiles_m = (p.M + CG * BM - 1) / (CG * BM);
-    const int ktiles = (p.K + BK - 1) / BK;
-    const int n_items = tiles_m * tiles_n * p.splits;
-
+    {
+        static_assert(sizeof(TcTile) % 4 == 0, "copied word by word");
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(tab.p);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(sp);
+        for (int i = threadIdx.x; i < tab.n * (int)(sizeof(TcTile) / 4); i += kTcThreads) dst[i] = src[i];
+    }
     if (threadIdx.x == 0) {
-        abort_flag = (*reinterpret_cast<volatile int*>(p.err) != 0);   // an earlier CTA gave up: do not wait at all
+        abort_flag = (*reinterpret_cast<volatile int*>(tab.err) != 0);   // an earlier CTA gave up: do not wait at all
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 4 * CG); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -210,37 +233,40 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         }
     }
     tc_fence_before();
+    __syncthreads();
     if (CG == 2) cluster_sync();
-    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
 
     if (warp == 0) {
         // ---- TMA producer ------------------------------------------------------------------
-        int s = 0;                 // ring slot and its phase, across all items of this CTA
+        int s = 0, pi = 0;         // ring slot and its phase, across all items of this CTA
         uint32_t ph = 1;
         bool ok = true;
         for (int item = unit; item < n_items && ok; item += n_units) {
-            const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
-            const int kt0 = t.split * p.ktiles_per_split;
-            const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
+            const TcItem t = tc_item(sp, tab.n, item, pi);
+            const TcTile& P = sp[pi];
+            const CUtensorMap* tmA = &tab.maps[3 * pi];
+            const CUtensorMap* tmB = &tab.maps[3 * pi + 1];
+            const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn;
+            const uint32_t bytes = (uint32_t)(CG * P.stage_bytes);
             const int m0 = (t.mt * CG + (int)rank) * BM, n0 = t.nt * BN + (int)rank * (BN / CG);
-            for (int term = 0; term < p.nterms && ok; ++term) {
+            for (int term = 0; term < nterms && ok; ++term) {
                 // planes: 0 = hi, 1 = lo; products with a lo term first
-                const int pa = p.nterms == 3 ? (term == 0) : (term + 1 < p.nterms);
-                const int pb = p.nterms == 3 && term == 1;
-                for (int kk = 0; kk < my_kt; ++kk) {
+                const int pa = nterms == 3 ? (term == 0) : (term + 1 < nterms);
+                const int pb = nterms == 3 && term == 1;
+                for (int kk = 0; kk < t.nkt; ++kk) {
                     ok = mbar_wait_all(empty_bar(s), ph, &abort_flag);
-                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 1); break; }
-                    const uint32_t a_dst = tiles + (uint32_t)s * stage_bytes;
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 1); break; }
+                    const uint32_t a_dst = tiles + (uint32_t)s * slot_bytes;
                     const uint32_t bar = CG == 2 ? cluster_addr(full_bar(s), 0) : full_bar(s);
-                    const int k0 = (kt0 + kk) * BK;
+                    const int k0 = (t.kt0 + kk) * BK;
                     if (elect_one()) {
-                        if (rank == 0) mbar_expect_tx(full_bar(s), CG * stage_bytes);
-                        if (p.a_mn) tc_load4<CG>(a_dst, &tmA, bar, m0, k0, 0, pa);
-                        else tc_load<CG>(a_dst, &tmA, bar, k0, m0, pa);
-                        if (p.b_mn) tc_load4<CG>(a_dst + kATileBytes, &tmB, bar, n0, k0, 0, pb);
-                        else tc_load<CG>(a_dst + kATileBytes, &tmB, bar, k0, n0, pb);
+                        if (rank == 0) mbar_expect_tx(full_bar(s), bytes);
+                        if (a_mn) tc_load4<CG>(a_dst, tmA, bar, m0, k0, 0, pa);
+                        else tc_load<CG>(a_dst, tmA, bar, k0, m0, pa);
+                        if (b_mn) tc_load4<CG>(a_dst + kATileBytes, tmB, bar, n0, k0, 0, pb);
+                        else tc_load<CG>(a_dst + kATileBytes, tmB, bar, k0, n0, pb);
                     }
                     __syncwarp();
                     if (++s == S) { s = 0; ph ^= 1u; }
@@ -250,28 +276,29 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     } else if (warp == 1) {
         if (rank == 0) {
             // ---- MMA issuer ----------------------------------------------------------------
-            const uint32_t idesc = idesc_f16(CG * BM, BN, p.a_mn, p.b_mn);
-            const uint32_t a_step = p.a_mn ? 128u : 2u, b_step = p.b_mn ? 128u : 2u;   // 16 k further, in 16-byte units
-            const uint64_t da0 = p.a_mn ? smem_desc_mn_sw128(tiles) : smem_desc_k_sw128(tiles);
-            const uint64_t db0 = p.b_mn ? smem_desc_mn_sw128(tiles + kATileBytes) : smem_desc_k_sw128(tiles + kATileBytes);
-            const uint32_t a_hi = (uint32_t)(da0 >> 32), b_hi = (uint32_t)(db0 >> 32), a0 = (uint32_t)da0, b0 = (uint32_t)db0;
+            const uint64_t dk = smem_desc_k_sw128(tiles), dm = smem_desc_mn_sw128(tiles);
+            const uint32_t k_hi = (uint32_t)(dk >> 32), m_hi = (uint32_t)(dm >> 32), k_lo = (uint32_t)dk, m_lo = (uint32_t)dm;
             uint32_t n_local = 0, ph = 0;
-            int s = 0;
+            int s = 0, pi = 0;
             bool ok = true;
             for (int item = unit; item < n_items && ok; item += n_units, ++n_local) {
-                const int kt0 = (item / (tiles_m * tiles_n)) * p.ktiles_per_split;
-                const int my_kt = min(p.ktiles_per_split, ktiles - kt0);
-                const int total = p.nterms * my_kt, first_hi = total - my_kt;
+                const TcItem t = tc_item(sp, tab.n, item, pi);
+                const TcTile& P = sp[pi];
+                const uint32_t idesc = idesc_f16(CG * BM, P.BN, P.a_mn, P.b_mn);
+                const uint32_t a_step = P.a_mn ? 128u : 2u, b_step = P.b_mn ? 128u : 2u;   // 16 k further, in 16-byte units
+                const uint32_t a_hi = P.a_mn ? m_hi : k_hi, b_hi = P.b_mn ? m_hi : k_hi;
+                const uint32_t a0 = P.a_mn ? m_lo : k_lo, b0 = (P.b_mn ? m_lo : k_lo) + (kATileBytes >> 4);
+                const int total = P.nterms * t.nkt, first_hi = total - t.nkt;
                 const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
                 ok = mbar_wait_all(acc_empty(acc), aph ^ 1u, &abort_flag);
-                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 4); break; }
+                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 4); break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * acc_cols;
                 for (int j = 0; j < total; ++j) {
                     ok = mbar_wait_all(full_bar(s), ph, &abort_flag);
-                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 2); break; }
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 2); break; }
                     tc_fence_after();
-                    const uint32_t off = ((uint32_t)s * stage_bytes) >> 4;
+                    const uint32_t off = ((uint32_t)s * slot_bytes) >> 4;
                     const uint32_t a_lo = a0 + off, b_lo = b0 + off;
                     if (elect_one()) {
                         if (j == first_hi) umma_f16_down12<CG>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc);
@@ -290,20 +317,27 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     } else {
         // ---- epilogue warps: TMEM -> registers -> shared memory -> global ---------------------------
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
-        const bool scale = (p.col_scale != nullptr) && p.splits == 1;
-        const float fa = p.a_amax ? pow2(-term_exp(__ldg(p.a_amax))) : 1.0f;      // undo the powers of two of the split
-        const float fb = p.b_amax ? pow2(-term_exp(__ldg(p.b_amax))) : 1.0f;
         const uint32_t my_stage = staging + (uint32_t)q * 8192u;
         uint32_t n_local = 0, n_store = 0;
+        int pi = 0, at = -1;
+        float fa = 1.0f, fb = 1.0f;
         for (int item = unit; item < n_items; item += n_units, ++n_local) {
-            const TcItem t = tc_item(item, tiles_m, tiles_n, p.group_m);
+            const TcItem t = tc_item(sp, tab.n, item, pi);
+            const TcTile& P = sp[pi];
+            if (pi != at) {                            // undo the powers of two of the split
+                fa = P.a_words ? pow2(-terms_exp(P.a_words)) : 1.0f;
+                fb = P.b_words ? pow2(-terms_exp(P.b_words)) : 1.0f;
+                at = pi;
+            }
+            const CUtensorMap* tmC = &tab.maps[3 * pi + 2];
+            const float* col_scale = P.splits == 1 ? P.col_scale : nullptr;
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
             const bool was = !abort_flag;
             if (!__all_sync(0xffffffffu, was)) break;
-            if (!mbar_wait_warp(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 3); break; }
+            if (!mbar_wait_warp(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 3); break; }
             tc_fence_after();
-            const int n0 = t.nt * BN, row0 = (t.mt * CG + (int)rank) * BM + q * 32;
-            const int ncols = min(BN, p.N - n0);
+            const int n0 = t.nt * P.BN, row0 = (t.mt * CG + (int)rank) * BM + q * 32;
+            const int ncols = min(P.BN, P.N - n0), M = P.M;
             for (int c0 = 0; c0 < ncols; c0 += 64) {
                 uint32_t r[2][32];
                 const uint32_t t_addr = tmem_base + acc * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
@@ -318,7 +352,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                         else asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(acc_empty(acc), 0)) : "memory");
                     }
                 }
-                if (row0 >= p.M) continue;             // rows of the padding: nothing to store
+                if (row0 >= M) continue;               // rows of the padding: nothing to store
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int cc = c0 + 32 * h;
@@ -332,8 +366,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                         float4 o = make_float4(__uint_as_float(r[h][4 * j]), __uint_as_float(r[h][4 * j + 1]),
                                                __uint_as_float(r[h][4 * j + 2]), __uint_as_float(r[h][4 * j + 3]));
                         o.x = o.x * fa * fb; o.y = o.y * fa * fb; o.z = o.z * fa * fb; o.w = o.w * fa * fb;
-                        if (scale && cc + 4 * j < ncols) {            // N % 4 == 0
-                            const float4 sc = __ldg(reinterpret_cast<const float4*>(p.col_scale + n0 + cc + 4 * j));
+                        if (col_scale && cc + 4 * j < ncols) {        // N % 4 == 0
+                            const float4 sc = __ldg(reinterpret_cast<const float4*>(col_scale + n0 + cc + 4 * j));
                             o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
                         }
                         asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
@@ -343,7 +377,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                     __syncwarp();
                     if (lane == 0) {
                         asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-                                     ::"l"(reinterpret_cast<uint64_t>(&tmC)), "r"(buf), "r"(n0 + cc), "r"(row0), "r"(t.split) : "memory");
+                                     ::"l"(reinterpret_cast<uint64_t>(tmC)), "r"(buf), "r"(n0 + cc), "r"(row0), "r"(t.split) : "memory");
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
@@ -385,50 +419,61 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, float* _
     }
 }
 
-// ---- pre-pass 1: largest magnitude of a tensor, and of the tensor times a per-column factor ----------------
-// amax[0] = max |src|, amax[1] = max |src . col_scale| (when col_scale != null), as float bits, by atomicMax into zeroed
-// words.  HBM-bound: one read.
-template <bool VEC>
-__global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ src, size_t R, int Cc,
-                                                   const float* __restrict__ col_scale, uint32_t* __restrict__ amax) {
-    constexpr int W = VEC ? 4 : 1;
-    const int n = Cc / W;                                   // VEC needs Cc % 4 == 0
-    const size_t total = R * (size_t)n, stride = (size_t)gridDim.x * 256;
-    const size_t i0 = (size_t)blockIdx.x * 256 + threadIdx.x;
-    int c = (int)(i0 % (size_t)n);
-    const int step = (int)(stride % (size_t)n);
+// ---- pre-pass 1: the magnitude that a tensor's terms are scaled for ---------------------------------------------
+// Reading a whole tensor for its maximum costs half of what splitting it does (25 us of 67 us for 16384 x 2048), so the choice is
+// made from a sample: the largest of up to 16384 evenly spaced elements, raised by 2^kSampleRoom.  The split itself sees every
+// element and records the exact maximum; a third launch, empty unless some tensor is larger than fp16 holds, splits those
+// again.  Small tensors are sampled whole.  With the room the terms keep all bits of elements down to 2^-20 of the sample's
+// maximum and are off by less than 2^-42 of it below.
+constexpr int kSampleRoom = 8;
+constexpr int kSplitCap = 128;
+struct SplitTensor {
+    const float* src;
+    const float* col_scale;        // of planes_s
+    __half* planes;                // terms [2][R][ld] of src, or null
+    __half* planes_s;              // terms of src . col_scale, or null
+    uint32_t* words;               // {magnitude, exact maximum} of src, then of src . col_scale
+    int R, Cc, ld, vec;            // vec: rows of src and col_scale start on 16-byte boundaries
+};
+struct SplitGroup {
+    int n;
+    long long chunk_begin[kSplitCap + 1];      // chunks of kSplitChunk units of 8 columns
+    SplitTensor t[kSplitCap];
+};
+constexpr int kSplitChunk = 2048;
+
+__global__ void __launch_bounds__(512) sample_magnitude_kernel(const __grid_constant__ SplitGroup g) {
+    const SplitTensor& T = g.t[blockIdx.x];
+    const long long total = (long long)T.R * T.Cc;
+    const long long units = total >> 2, step = units > 4096 ? units / 4096 : 1;       // units of 4 consecutive elements
     float m0 = 0.0f, m1 = 0.0f;
-#pragma unroll 4
-    for (size_t i = i0; i < total; i += stride) {
-        if (VEC) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(src) + i);
-            m0 = fmaxf(fmaxf(m0, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-            if (col_scale) {
-                const float4 s = __ldg(reinterpret_cast<const float4*>(col_scale) + c);
-                m1 = fmaxf(fmaxf(m1, fmaxf(fabsf(v.x * s.x), fabsf(v.y * s.y))), fmaxf(fabsf(v.z * s.z), fabsf(v.w * s.w)));
-            }
-        } else {
-            const float v = __ldg(src + i);
-            m0 = fmaxf(m0, fabsf(v));
-            if (col_scale) m1 = fmaxf(m1, fabsf(v * __ldg(col_scale + c)));
-        }
-        c += step;
-        if (c >= n) c -= n;
+    auto add = [&](long long e) {
+        const float v = __ldg(T.src + e);
+        m0 = fmaxf(m0, fabsf(v));
+        if (T.planes_s) m1 = fmaxf(m1, fabsf(v * __ldg(T.col_scale + (int)(e % T.Cc))));
+    };
+#pragma unroll 2
+    for (long long u = threadIdx.x; u < units && u < 8192; u += 512) {
+        const long long e = u * step * 4;
+        if (e + 3 < total) { add(e); add(e + 1); add(e + 2); add(e + 3); }
     }
-    uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
-    __shared__ uint32_t w0[8], w1[8];
+    for (long long e = (units << 2) + threadIdx.x; e < total; e += 512) add(e);
+    const uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
+    __shared__ uint32_t w0[16], w1[16];
     if ((threadIdx.x & 31) == 0) { w0[threadIdx.x >> 5] = b0; w1[threadIdx.x >> 5] = b1; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) { b0 = max(b0, w0[w]); b1 = max(b1, w1[w]); }
-        if (b0) atomicMax(amax, b0);
-        if (col_scale && b1) atomicMax(amax + 1, b1);
+        uint32_t a = 0, b = 0;
+        for (int w = 0; w < 16; ++w) { a = max(a, w0[w]); b = max(b, w1[w]); }
+        const uint32_t room = step > 1 ? (uint32_t)kSampleRoom << 23 : 0u;
+        T.words[0] = a && a < 0x7b000000u ? a + room : a; T.words[1] = 0u;
+        T.words[2] = b && b < 0x7b000000u ? b + room : b; T.words[3] = 0u;
     }
 }
 
-// ---- pre-pass 2: fp32 [R, Cc] -> fp16 terms [2][R][ld] of src (planes) and of src . col_scale (planes_s) ----------
+// ---- pre-pass 2: fp32 [R, Cc] -> fp16 terms, and the exact maxima ------------------------------------------------
 // Thread = 8 consecutive columns: two 128-bit loads, one 128-bit store per term.  HBM-bound: 4 bytes read, 4 written per
-// element and output.
+// element and output.  All tensors of a step in one launch; FIX: only those whose first choice did not hold.
 __device__ __forceinline__ void split_terms8(const float (&v)[8], float f, uint4* hi, uint4* lo) {
     uint32_t h[4], l[4];
 #pragma unroll
@@ -443,40 +488,102 @@ __device__ __forceinline__ void split_terms8(const float (&v)[8], float f, uint4
     *hi = make_uint4(h[0], h[1], h[2], h[3]);
     *lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
-template <bool VEC>
-__global__ void __launch_bounds__(256) split_terms_kernel(const float* __restrict__ src, int R, int Cc, int ld,
-                                                          const float* __restrict__ col_scale, __half* __restrict__ planes,
-                                                          __half* __restrict__ planes_s, const uint32_t* __restrict__ amax) {
-    const int n8 = (Cc + 7) >> 3;
-    const float f0 = planes ? pow2(term_exp(__ldg(amax))) : 0.0f, f1 = planes_s ? pow2(term_exp(__ldg(amax + 1))) : 0.0f;
-    const size_t total = (size_t)R * n8, stride = (size_t)gridDim.x * 256, ps = (size_t)R * ld;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += stride) {
-        const size_t r = i / (size_t)n8;
-        const int c = (int)(i - r * n8) * 8;
-        const float* s = src + r * Cc + c;
-        float v[8];
-        if (VEC && c + 8 <= Cc) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(s)), b = __ldg(reinterpret_cast<const float4*>(s) + 1);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = c + k < Cc ? __ldg(s + k) : 0.0f;
+template <bool FIX>
+__global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant__ SplitGroup g) {
+    const long long total = g.chunk_begin[g.n];
+    int ti = -1;
+    long long first = 0, last = 0;             // chunks of tensor ti
+    bool do0 = false, do1 = false;
+    float f0 = 0.0f, f1 = 0.0f, m0 = 0.0f, m1 = 0.0f;
+    __shared__ uint32_t red[2];
+    if (threadIdx.x < 2) red[threadIdx.x] = 0u;
+    __syncthreads();
+    auto flush = [&]() {                       // the maxima of this block's share of tensor ti
+        if (FIX || ti < 0) return;
+        const uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
+        if ((threadIdx.x & 31) == 0) { atomicMax(&red[0], b0); atomicMax(&red[1], b1); }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (red[0]) atomicMax(g.t[ti].words + 1, red[0]);
+            if (red[1]) atomicMax(g.t[ti].words + 3, red[1]);
+            red[0] = red[1] = 0u;
         }
-        uint4 hi, lo;
-        const size_t at = r * ld + c;                       // ld % 8 == 0
-        if (planes) {
-            split_terms8(v, f0, &hi, &lo);
-            *reinterpret_cast<uint4*>(planes + at) = hi;
-            *reinterpret_cast<uint4*>(planes + ps + at) = lo;
+        __syncthreads();
+        m0 = m1 = 0.0f;
+    };
+    for (long long ch = blockIdx.x; ch < total; ch += gridDim.x) {
+        if (ch >= last) {
+            flush();
+            int lo = ti < 0 ? 0 : ti, hi = g.n - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (g.chunk_begin[mid] <= ch) lo = mid; else hi = mid - 1;
+            }
+            ti = lo; first = g.chunk_begin[ti]; last = g.chunk_begin[ti + 1];
+            const SplitTensor& T = g.t[ti];
+            do0 = T.planes != nullptr; do1 = T.planes_s != nullptr;
+            if (FIX) {
+                do0 = do0 && terms_redone(__ldg(T.words), __ldg(T.words + 1));
+                do1 = do1 && terms_redone(__ldg(T.words + 2), __ldg(T.words + 3));
+                f0 = do0 ? pow2(term_exp(__ldg(T.words + 1))) : 0.0f;
+                f1 = do1 ? pow2(term_exp(__ldg(T.words + 3))) : 0.0f;
+            } else {
+                f0 = do0 ? pow2(term_exp(__ldg(T.words))) : 0.0f;
+                f1 = do1 ? pow2(term_exp(__ldg(T.words + 2))) : 0.0f;
+            }
         }
-        if (planes_s) {
+        if (FIX && !do0 && !do1) continue;
+        const SplitTensor& T = g.t[ti];
+        const int n8 = (T.Cc + 7) >> 3, Cc = T.Cc, ld = T.ld;
+        const size_t units = (size_t)T.R * n8, ps = (size_t)T.R * ld;
+        size_t u = (size_t)(ch - first) * kSplitChunk + threadIdx.x;
+        size_t r = u / (size_t)n8;
+        int c8 = (int)(u - r * n8);
+#pragma unroll 2
+        for (int k = 0; k < kSplitChunk / 256 && u < units; ++k, u += 256) {
+            const int c = c8 * 8;
+            const float* src = T.src + r * Cc + c;
+            float v[8];
+            if (T.vec && c + 8 <= Cc) {
+                const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(v[k], c + k < Cc ? __ldg(col_scale + c + k) : 0.0f);
-            split_terms8(v, f1, &hi, &lo);
-            *reinterpret_cast<uint4*>(planes_s + at) = hi;
-            *reinterpret_cast<uint4*>(planes_s + ps + at) = lo;
+                for (int q = 0; q < 8; ++q) v[q] = c + q < Cc ? __ldg(src + q) : 0.0f;
+            }
+            uint4 hi, lo;
+            const size_t at = r * ld + c;                       // ld % 8 == 0
+            if (do0) {
+                if (!FIX) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) m0 = fmaxf(m0, fabsf(v[q]));
+                }
+                split_terms8(v, f0, &hi, &lo);
+                *reinterpret_cast<uint4*>(T.planes + at) = hi;
+                *reinterpret_cast<uint4*>(T.planes + ps + at) = lo;
+            }
+            if (do1) {
+                float sc[8];
+                if (T.vec && c + 8 <= Cc) {
+                    const float4 a = __ldg(reinterpret_cast<const float4*>(T.col_scale + c)), b = __ldg(reinterpret_cast<const float4*>(T.col_scale + c) + 1);
+                    sc[0] = a.x; sc[1] = a.y; sc[2] = a.z; sc[3] = a.w; sc[4] = b.x; sc[5] = b.y; sc[6] = b.z; sc[7] = b.w;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) sc[q] = c + q < Cc ? __ldg(T.col_scale + c + q) : 0.0f;
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    v[q] = __fmul_rn(v[q], sc[q]);
+                    if (!FIX) m1 = fmaxf(m1, fabsf(v[q]));
+                }
+                split_terms8(v, f1, &hi, &lo);
+                *reinterpret_cast<uint4*>(T.planes_s + at) = hi;
+                *reinterpret_cast<uint4*>(T.planes_s + ps + at) = lo;
+            }
+            for (c8 += 256; c8 >= n8; c8 -= n8) ++r;            // 256 units further
         }
     }
+    flush();
 }
 
 // ---- pre-pass 3: packed 6-bit state -> fp16 ternary digits T [O][ld] --------------------------------------------
@@ -487,51 +594,78 @@ __device__ __forceinline__ uint32_t digit_pair(uint32_t two_codes, int lv) {
     const __half2 h = __floats2half2_rn((float)((int)(two_codes & 63u) / lv - 1), (float)((int)(two_codes >> 6) / lv - 1));
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+constexpr int kExpandCap = 128;
+struct ExpandGroup {
+    int n, C;
+    long long unit_begin[kExpandCap + 1];      // units of 16 weights (VEC) or of 4
+    const uint8_t* state[kExpandCap];          // 6-bit state of the layer, or null: then
+    const uint32_t* packed2[kExpandCap];       // its 2-bit words (field = t + 1, 16 per word; in_features % 16 == 0)
+    __half* T[kExpandCap];
+    int I[kExpandCap], ld[kExpandCap];
+};
 template <bool VEC>
-__global__ void __launch_bounds__(256) expand_ternary_kernel(const uint8_t* __restrict__ state, int C, int O, int I,
-                                                             __half* __restrict__ T, int ld) {
+__global__ void __launch_bounds__(256) expand_ternary_kernel(const __grid_constant__ ExpandGroup g) {
     __shared__ uint32_t lut[4096];
-    for (int e = threadIdx.x; e < 4096; e += 256) lut[e] = digit_pair((uint32_t)e, 2 * C - 1);
+    for (int e = threadIdx.x; e < 4096; e += 256) lut[e] = digit_pair((uint32_t)e, 2 * g.C - 1);
     __syncthreads();
-    if (VEC) {
-        const size_t total = (size_t)O * (I >> 4);
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(state);
-        for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {   // ld == I here
-            const uint32_t a = __ldg(w + 3 * i), b = __ldg(w + 3 * i + 1), c = __ldg(w + 3 * i + 2);
-            const uint32_t g0 = a & 0xFFFFFFu, g1 = (a >> 24) | (b << 8), g2 = (b >> 16) | (c << 16), g3 = c >> 8;
-            uint4* o = reinterpret_cast<uint4*>(T + 16 * i);
-            o[0] = make_uint4(lut[g0 & 4095u], lut[g0 >> 12], lut[g1 & 4095u], lut[(g1 >> 12) & 4095u]);
-            o[1] = make_uint4(lut[g2 & 4095u], lut[(g2 >> 12) & 4095u], lut[g3 & 4095u], lut[g3 >> 12]);
-        }
-    } else {
-        const int gpr = I >> 2;
-        const size_t total = (size_t)O * gpr;
-        for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t)gridDim.x * 256) {
-            const uint8_t* s = state + i * 3;
-            const uint32_t g = (uint32_t)__ldg(s) | ((uint32_t)__ldg(s + 1) << 8) | ((uint32_t)__ldg(s + 2) << 16);
-            const size_t o = i / (size_t)gpr;
-            *reinterpret_cast<uint2*>(T + o * ld + (i - o * gpr) * 4) = make_uint2(lut[g & 4095u], lut[g >> 12]);
+    const __half2 off = __floats2half2_rn(1025.0f, 1025.0f);
+    const long long total = g.unit_begin[g.n];
+    int li = 0;
+    for (long long u = (long long)blockIdx.x * 256 + threadIdx.x; u < total; u += (long long)gridDim.x * 256) {
+        while (u >= g.unit_begin[li + 1]) ++li;
+        const long long i = u - g.unit_begin[li];
+        if (VEC) {                                              // rows follow one another: ld == I
+            uint4* o = reinterpret_cast<uint4*>(g.T[li] + 16 * i);
+            if (g.state[li]) {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(g.state[li]);
+                const uint32_t a = __ldg(w + 3 * i), b = __ldg(w + 3 * i + 1), c = __ldg(w + 3 * i + 2);
+                const uint32_t g0 = a & 0xFFFFFFu, g1 = (a >> 24) | (b << 8), g2 = (b >> 16) | (c << 16), g3 = c >> 8;
+                o[0] = make_uint4(lut[g0 & 4095u], lut[g0 >> 12], lut[g1 & 4095u], lut[(g1 >> 12) & 4095u]);
+                o[1] = make_uint4(lut[g2 & 4095u], lut[(g2 >> 12) & 4095u], lut[g3 & 4095u], lut[g3 >> 12]);
+            } else {
+                const uint32_t w = __ldg(g.packed2[li] + i);
+                uint32_t h[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {                   // fp16 1024 + field in both halves, minus 1025
+                    const uint32_t two = 0x64006400u | ((w >> (4 * j)) & 3u) | (((w >> (4 * j + 2)) & 3u) << 16);
+                    const __half2 t = __hsub2(*reinterpret_cast<const __half2*>(&two), off);
+                    h[j] = *reinterpret_cast<const uint32_t*>(&t);
+                }
+                o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+                o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            }
+        } else {                                                // byte-wise state access
+            const uint8_t* s = g.state[li] + i * 3;
+            const uint32_t w = (uint32_t)__ldg(s) | ((uint32_t)__ldg(s + 1) << 8) | ((uint32_t)__ldg(s + 2) << 16);
+            const int gpr = g.I[li] >> 2;
+            const long long o = i / gpr;
+            *reinterpret_cast<uint2*>(g.T[li] + o * g.ld[li] + (i - o * gpr) * 4) = make_uint2(lut[w & 4095u], lut[w >> 12]);
         }
     }
 }
 
-// Same expansion from the 2-bit packed weights (field = t + 1, 16 per word): what ranks that do
-// not own a layer's counter state use after the all-gather of packed weights.
-__global__ void __launch_bounds__(256) expand_ternary_p2_kernel(const uint32_t* __restrict__ packed2, size_t words,
-                                                                __half* __restrict__ T) {
-    const __half2 off = __floats2half2_rn(1025.0f, 1025.0f);
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) {
-        const uint32_t w = __ldg(packed2 + i);
-        uint32_t h[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {      // fp16 1024 + field in both halves, minus 1025
-            const uint32_t two = 0x64006400u | ((w >> (4 * j)) & 3u) | (((w >> (4 * j + 2)) & 3u) << 16);
-            const __half2 t = __hsub2(*reinterpret_cast<const __half2*>(&two), off);
-            h[j] = *reinterpret_cast<const uint32_t*>(&t);
+// out[i] = sum over z of partial[z][i], z ascending, for the split-K products of a step
+constexpr int kReduceCap = 128;
+struct ReduceGroup {
+    int n;
+    long long unit_begin[kReduceCap + 1];      // float4s
+    const float* partial[kReduceCap];
+    float* out[kReduceCap];
+    int splits[kReduceCap];
+};
+__global__ void __launch_bounds__(256) splitk_reduce_group_kernel(const __grid_constant__ ReduceGroup g) {
+    const long long total = g.unit_begin[g.n];
+    int li = 0;
+    for (long long u = (long long)blockIdx.x * 256 + threadIdx.x; u < total; u += (long long)gridDim.x * 256) {
+        while (u >= g.unit_begin[li + 1]) ++li;
+        const long long i = u - g.unit_begin[li], n4 = g.unit_begin[li + 1] - g.unit_begin[li];
+        const float4* p = reinterpret_cast<const float4*>(g.partial[li]) + i;
+        float4 acc = __ldg(p);
+        for (int z = 1; z < g.splits[li]; ++z) {
+            const float4 v = __ldg(p + z * n4);
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        uint4* o = reinterpret_cast<uint4*>(T + 16 * i);       // in_features % 16 == 0, so rows follow one another
-        o[0] = make_uint4(h[0], h[1], h[2], h[3]);
-        o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        reinterpret_cast<float4*>(g.out[li])[i] = acc;
     }
 }
 
@@ -620,7 +754,7 @@ TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit) {
                 if (real > 1) cost += ((double)(real + 1) * M * N * 4.0) / 3000.0 + 4000.0;
                 if (cost < best_cost) {
                     best_cost = cost;
-                    best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per;
+                    best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per; best.cost = cost;
                 }
             }
         }
@@ -629,53 +763,87 @@ TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit) {
     return best;
 }
 
-cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int M, int N, int K, const TcPlan& plan,
-                           const float* col_scale, float* splitk_ws, int* err_word, size_t max_smem, int sm_count,
-                           cudaStream_t stream, int* launches) {
-    if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
-    const int bn = plan.bn, cg = plan.pair ? 2 : 1, splits = plan.splits, b_rows = bn / cg;
-    float* out = splits > 1 ? splitk_ws : c;
-    CUtensorMap ma, mb, mc;
-    if (!make_map(&ma, a, BM)) return cudaErrorInvalidValue;
-    if (!make_map(&mb, b, b_rows)) return cudaErrorInvalidValue;
-    if (!make_out_map(&mc, out, M, N, splits)) return cudaErrorInvalidValue;
-    TcParams p;
-    p.col_scale = col_scale;
-    p.M = M; p.N = N; p.K = K;
-    p.BN = bn;
-    p.a_mn = a.mn_major; p.b_mn = b.mn_major;
-    p.a_amax = a.amax; p.b_amax = b.amax;
-    p.b_bytes = (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
-    p.group_m = 12 / cg;          // 12 row tiles x 12 column tiles in flight on 148 SMs
-    p.nterms = b.planes == 2 ? 3 : 2;
-    p.splits = splits;
-    p.ktiles_per_split = plan.ktiles_per_split;
-    p.err = err_word;
-    const size_t stage_bytes = (size_t)kATileBytes + (size_t)p.b_bytes;
-    int stages = (int)((max_smem - 2048 - kStageBytes) / stage_bytes);
+// The same choice for one product among many that share a launch: what counts is the sum of the items' times, so tiles
+// waste least and K is split only where the accumulation depth asks for it, or `min_items` for more items.
+TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items) {
+    TcPlan best = {};
+    double best_cost = 1e300;
+    const int ktiles = (K + BK - 1) / BK, tm = (M + cg * BM - 1) / (cg * BM);
+    for (int bn = 64; bn <= 256; bn += 32) {
+        const int tiles = tm * ((N + bn - 1) / bn);
+        int s = depth_limit > 0 ? (ktiles + depth_limit - 1) / depth_limit : 1;
+        if (depth_limit > 0)
+            while (tiles * s < min_items && ktiles >= 16 * (s + 1)) ++s;
+        const int per = (ktiles + s - 1) / s, real = (ktiles + per - 1) / per;
+        const double cyc = (double)nterms * (2 * bn > 2 * (128 + bn / cg) ? 2 * bn : 2 * (128 + bn / cg));
+        const double cost = cg * ((double)tiles * real * (per * cyc + 500.0));
+        if (cost < best_cost) {
+            best_cost = cost;
+            best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per;
+        }
+    }
+    best.cost = best_cost;
+    best.workspace_bytes = best.splits > 1 ? (size_t)best.splits * M * N * sizeof(float) : 0;
+    return best;
+}
+
+namespace {
+template <int CG, int CAP>
+cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream) {
+    static thread_local TcTable<CAP> tab;      // 28 KB: built in place, copied by the launch
+    tab.n = n;
+    tab.err = err_word;
+    tab.slot_bytes = 0;
+    int items = 0, bn_max = 64, want = 2;
+    for (int i = 0; i < n; ++i) {
+        const TcProblem& q = probs[i];
+        const TcOperand &a = q.a, &b = q.b;
+        if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (q.N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
+        const int bn = q.plan.bn, b_rows = bn / CG;
+        float* out = q.plan.splits > 1 ? q.splitk_ws : q.c;
+        if (!make_map(&tab.maps[3 * i], a, BM) || !make_map(&tab.maps[3 * i + 1], b, b_rows) ||
+            !make_out_map(&tab.maps[3 * i + 2], out, q.M, q.N, q.plan.splits)) return cudaErrorInvalidValue;
+        TcTile& p = tab.p[i];
+        p.col_scale = q.col_scale;
+        p.a_words = a.words; p.b_words = b.words;
+        p.M = q.M; p.N = q.N; p.K = q.K;
+        p.BN = bn;
+        p.stage_bytes = kATileBytes + (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
+        p.a_mn = a.mn_major; p.b_mn = b.mn_major;
+        p.nterms = b.planes == 2 ? 3 : 2;
+        p.ktiles_per_split = q.plan.ktiles_per_split; p.splits = q.plan.splits;
+        p.tiles_m = (q.M + CG * BM - 1) / (CG * BM); p.tiles_n = (q.N + bn - 1) / bn;
+        p.group_m = 12 / CG;                   // 12 row tiles x 12 column tiles in flight on 148 SMs
+        p.item_begin = items;
+        items += p.tiles_m * p.tiles_n * p.splits;
+        if (p.stage_bytes > tab.slot_bytes) tab.slot_bytes = p.stage_bytes;
+        if (bn > bn_max) bn_max = bn;
+        if (p.nterms * p.ktiles_per_split > want) want = p.nterms * p.ktiles_per_split;
+    }
+    tab.n_items = items;
+    tab.acc_cols = 64;
+    while (tab.acc_cols < bn_max) tab.acc_cols *= 2;
+    int stages = (int)((max_smem - 1024 - sizeof(TcTile) * CAP - 2048 - kStageBytes) / (size_t)tab.slot_bytes);
     if (stages > kMaxStages) stages = kMaxStages;
-    const int want = p.nterms * p.ktiles_per_split;   // slots one work item fills
-    const int n_items = ((N + bn - 1) / bn) * ((M + cg * BM - 1) / (cg * BM)) * splits;
-    // Two accumulators of one CTA take 2 * pow2(BN) TMEM columns of the SM's 512.  Narrow tiles
-    // (BN <= 128) with short main loops leave room for a second resident CTA, which doubles the
-    // loads in flight where the loop is latency-bound; then each CTA gets half the shared memory.
+    // Two accumulators of one CTA take 2 * pow2(BN) TMEM columns of the SM's 512.  Narrow tiles (BN <= 128) with short main
+    // loops leave room for a second resident CTA, which doubles the loads in flight where the loop is latency-bound; then
+    // each CTA gets half the shared memory.
     bool two_ctas = false;
-    if (cg == 1 && bn <= 128 && want <= 32 && n_items > sm_count) {
-        const int half = (int)((((max_smem - 4096) / 2) - 1024 - kStageBytes) / stage_bytes);
+    if (CG == 1 && bn_max <= 128 && want <= 32 && items > sm_count) {
+        const int half = (int)((max_smem / 2 - 2048 - sizeof(TcTile) * CAP - 1024 - kStageBytes) / (size_t)tab.slot_bytes);
         if (half >= 3) { two_ctas = true; if (half < stages) stages = half; }
     }
     if (stages > want) stages = want;
-    if (stages < 2) stages = 2;
-    const size_t smem = (size_t)stages * stage_bytes + 1024 + kStageBytes;
-    if (smem > max_smem) return cudaErrorInvalidConfiguration;
-    p.stages = stages;
-    const void* kern = cg == 2 ? reinterpret_cast<const void*>(tc_gemm_kernel<2>) : reinterpret_cast<const void*>(tc_gemm_kernel<1>);
-    cudaError_t e = ensure_dynamic_smem(kern, cg == 2 ? kSmemSlotTcPair : 4, max_smem);
+    if (stages < 2) return cudaErrorInvalidConfiguration;
+    tab.stages = stages;
+    const size_t smem = (size_t)stages * tab.slot_bytes + 1024 + kStageBytes;
+    const auto kern = tc_gemm_kernel<CG, CAP>;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), CG == 2 ? (CAP > 1 ? 24 : 16) : (CAP > 1 ? 25 : 4), max_smem);
     if (e != cudaSuccess) return e;
-    int units = (sm_count / cg) * (two_ctas ? 2 : 1);
-    if (units > n_items) units = n_items;
+    int units = (sm_count / CG) * (two_ctas ? 2 : 1);
+    if (units > items) units = items;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(units * cg));
+    cfg.gridDim = dim3((unsigned)(units * CG));
     cfg.blockDim = dim3(kTcThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -683,55 +851,49 @@ cudaError_t launch_tc_gemm(const TcOperand& a, const TcOperand& b, float* c, int
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = cg == 2 ? 1 : 0;
-    e = cg == 2 ? cudaLaunchKernelEx(&cfg, tc_gemm_kernel<2>, ma, mb, mc, p) : cudaLaunchKernelEx(&cfg, tc_gemm_kernel<1>, ma, mb, mc, p);
-    if (e != cudaSuccess) return e;
-    ++*launches;
-    if (splits > 1) {
-        e = launch_splitk_reduce(splitk_ws, c, col_scale, M, N, N, splits, stream);
+    cfg.numAttrs = CG == 2 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, tab);
+}
+}  // namespace
+
+// Products in launches of up to kTcCap each; all of a launch have the same plan.pair.
+cudaError_t launch_tc_products(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream,
+                               int* launches) {
+    for (int i = 0; i < n;) {
+        int k = 1;
+        while (i + k < n && k < kTcCap && probs[i + k].plan.pair == probs[i].plan.pair) ++k;
+        const cudaError_t e = probs[i].plan.pair
+            ? (k == 1 ? run_tc_table<2, 1>(probs + i, 1, err_word, max_smem, sm_count, stream) : run_tc_table<2, kTcCap>(probs + i, k, err_word, max_smem, sm_count, stream))
+            : (k == 1 ? run_tc_table<1, 1>(probs + i, 1, err_word, max_smem, sm_count, stream) : run_tc_table<1, kTcCap>(probs + i, k, err_word, max_smem, sm_count, stream));
         if (e != cudaSuccess) return e;
         ++*launches;
+        i += k;
     }
     return cudaSuccess;
 }
 
-// K-major use: 2-D {cols, rows}, box {32, box_outer rows}, 128-byte swizzle.  MN-major use (cols % 32 == 0):
-// 3-D {32, rows, cols / 32} with the 32-column chunk as the outermost index, box {32, 32, box_outer chunks},
-// 128-byte swizzle with 32-byte atoms.  Elements outside the tensor read as zero.
-bool tc_encode_map_f32(void* map, const float* base, int cols, int rows, int ld, int mn_major, int box_outer) {
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return false;
-    CUtensorMap* m = static_cast<CUtensorMap*>(map);
-    void* ptr = const_cast<float*>(base);
-    if (!mn_major) {
-        cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-        cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-        cuuint32_t box[2] = {32, (cuuint32_t)box_outer};
-        cuuint32_t estr[2] = {1, 1};
-        return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+cudaError_t launch_splitk_reduce_group(const float* const* partial, float* const* out, const long long* elements, const int* splits,
+                                       int n, int sm_count, cudaStream_t stream, int* launches) {
+    for (int done = 0; done < n;) {
+        ReduceGroup g;
+        const int take = n - done < kReduceCap ? n - done : kReduceCap;
+        long long units = 0;
+        for (int j = 0; j < take; ++j) {
+            g.unit_begin[j] = units;
+            g.partial[j] = partial[done + j]; g.out[j] = out[done + j]; g.splits[j] = splits[done + j];
+            units += elements[done + j] / 4;
+        }
+        g.unit_begin[take] = units;
+        g.n = take;
+        long long blocks = (units + 255) / 256;
+        if (blocks > (long long)sm_count * 8) blocks = (long long)sm_count * 8;
+        splitk_reduce_group_kernel<<<(int)blocks, 256, 0, stream>>>(g);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        ++*launches;
+        done += take;
     }
-    if (cols % 32 != 0) return false;
-    cuuint64_t dims[3] = {32, (cuuint64_t)rows, (cuuint64_t)(cols / 32)};
-    cuuint64_t strides[2] = {(cuuint64_t)ld * 4, 128};
-    cuuint32_t box[3] = {32, 32, (cuuint32_t)box_outer};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-bool tc_encode_map_bf16(void* map, const void* base, int cols, int rows, int ld, int box_outer) {
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    return enc(static_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return cudaSuccess;
 }
 
 cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* col_scale, int M, int N, int ldc,
@@ -743,40 +905,65 @@ cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* co
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_terms(const float* src, int R, int Cc, int ld, const float* col_scale, void* planes, void* planes_s,
-                               uint32_t* amax, int sm_count, cudaStream_t stream) {
-    const bool vec = (Cc & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0 &&
-                     (col_scale == nullptr || (reinterpret_cast<uintptr_t>(col_scale) & 15) == 0);
-    __half* p0 = static_cast<__half*>(planes);
-    __half* p1 = static_cast<__half*>(planes_s);
-    const float* cs = p1 ? col_scale : nullptr;
-    auto blocks = [&](size_t work, int per_sm) {
-        const size_t b = (work + 255) / 256;
-        return (int)(b < (size_t)sm_count * per_sm ? (b ? b : 1) : (size_t)sm_count * per_sm);
-    };
-    const size_t n = (size_t)R * Cc;
-    if (vec) amax_kernel<true><<<blocks(n / 4, 8), 256, 0, stream>>>(src, R, Cc, cs, amax);
-    else amax_kernel<false><<<blocks(n, 8), 256, 0, stream>>>(src, R, Cc, cs, amax);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const int nb = blocks((size_t)R * ((Cc + 7) / 8), 8);
-    if (vec) split_terms_kernel<true><<<nb, 256, 0, stream>>>(src, R, Cc, ld, cs, p0, p1, amax);
-    else split_terms_kernel<false><<<nb, 256, 0, stream>>>(src, R, Cc, ld, cs, p0, p1, amax);
-    return cudaGetLastError();
+cudaError_t launch_split_terms(const SplitDesc* d, int n, int sm_count, cudaStream_t stream, int* launches) {
+    for (int done = 0; done < n;) {
+        SplitGroup g;
+        const int take = n - done < kSplitCap ? n - done : kSplitCap;
+        long long chunks = 0;
+        bool sampled = false;                  // a tensor sampled whole needs no second look
+        for (int j = 0; j < take; ++j) {
+            const SplitDesc& q = d[done + j];
+            SplitTensor& t = g.t[j];
+            t.src = q.src; t.col_scale = q.planes_s ? q.col_scale : nullptr;
+            t.planes = static_cast<__half*>(q.planes); t.planes_s = static_cast<__half*>(q.planes_s);
+            t.words = q.words; t.R = q.rows; t.Cc = q.cols; t.ld = q.ld;
+            t.vec = (q.cols & 3) == 0 && (reinterpret_cast<uintptr_t>(q.src) & 15) == 0 &&
+                    (t.col_scale == nullptr || (reinterpret_cast<uintptr_t>(t.col_scale) & 15) == 0);
+            g.chunk_begin[j] = chunks;
+            chunks += ((long long)q.rows * ((q.cols + 7) / 8) + kSplitChunk - 1) / kSplitChunk;
+            if ((long long)q.rows * q.cols / 4 >= 2 * 4096) sampled = true;
+        }
+        g.chunk_begin[take] = chunks;
+        g.n = take;
+        const int grid = (int)(chunks < (long long)sm_count * 8 ? chunks : (long long)sm_count * 8);
+        sample_magnitude_kernel<<<take, 512, 0, stream>>>(g);
+        split_terms_kernel<false><<<grid, 256, 0, stream>>>(g);
+        if (sampled) split_terms_kernel<true><<<grid < sm_count ? grid : sm_count, 256, 0, stream>>>(g);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        *launches += sampled ? 3 : 2;
+        done += take;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t launch_expand_ternary(const uint8_t* state, const uint32_t* packed2, int C, int O, int I, void* T, int ld,
-                                  int sm_count, cudaStream_t stream) {
-    __half* t = static_cast<__half*>(T);
-    const size_t units = (size_t)O * ((I + 15) / 16);
-    int blocks = (int)((units + 255) / 256 < (size_t)sm_count * 8 ? (units + 255) / 256 : (size_t)sm_count * 8);
-    if (!state)
-        expand_ternary_p2_kernel<<<blocks, 256, 0, stream>>>(packed2, (size_t)O * (I / 16), t);
-    else if (I % 16 == 0 && ld == I && (reinterpret_cast<uintptr_t>(state) & 3) == 0)
-        expand_ternary_kernel<true><<<blocks, 256, 0, stream>>>(state, C, O, I, t, ld);
-    else
-        expand_ternary_kernel<false><<<blocks, 256, 0, stream>>>(state, C, O, I, t, ld);
-    return cudaGetLastError();
+cudaError_t launch_expand_ternary(const ExpandDesc* d, int n, int C, int sm_count, cudaStream_t stream, int* launches) {
+    for (int vec = 0; vec < 2; ++vec) {        // layers with aligned rows of whole words, then the others
+        for (int i = 0; i < n;) {
+            ExpandGroup g;
+            g.n = 0; g.C = C;
+            long long units = 0;
+            for (; i < n && g.n < kExpandCap; ++i) {
+                const bool v = d[i].I % 16 == 0 && d[i].ld == d[i].I && (!d[i].state || (reinterpret_cast<uintptr_t>(d[i].state) & 3) == 0);
+                if (v != (vec == 0)) continue;
+                g.unit_begin[g.n] = units;
+                g.state[g.n] = d[i].state; g.packed2[g.n] = d[i].packed2; g.T[g.n] = static_cast<__half*>(d[i].T);
+                g.I[g.n] = d[i].I; g.ld[g.n] = d[i].ld;
+                units += (long long)d[i].O * (d[i].I / (v ? 16 : 4));
+                ++g.n;
+            }
+            if (g.n == 0) continue;
+            g.unit_begin[g.n] = units;
+            long long blocks = (units + 255) / 256;
+            if (blocks > (long long)sm_count * 8) blocks = (long long)sm_count * 8;
+            if (vec == 0) expand_ternary_kernel<true><<<(int)blocks, 256, 0, stream>>>(g);
+            else expand_ternary_kernel<false><<<(int)blocks, 256, 0, stream>>>(g);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+            ++*launches;
+        }
+    }
+    return cudaSuccess;
 }
 
 }  // namespace mcl
