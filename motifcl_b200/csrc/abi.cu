@@ -37,11 +37,9 @@ struct mcl_cuda_ctx {
     uint64_t lane_mark = 0;      // launches at the last lane_fork (when this context is a lane)
     bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end
     uint64_t recorded_launches = 0;
+    cudaGraphNode_t last_gemv = nullptr;   // node of the last gemv_mma launch of the recording
     int live_batches = 0;        // recorded batches not yet destroyed: they hold addresses inside the workspace
 };
-
-// ticket words of the sliced table look-up GEMV, one per block of 256 output rows
-constexpr int kGemvTicketWords = 4096;
 
 struct mcl_cuda_batch {
     cudaGraph_t graph = nullptr;
@@ -174,9 +172,9 @@ int create_impl(int device, cudaStream_t stream, bool own, mcl_cuda_ctx** out_ct
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         cudaGetLastError();
     }
-    // [0] error word, [1] work-item counter, [16 ...) ticket words of the table look-up GEMV (zero between launches)
-    e = cudaMalloc(reinterpret_cast<void**>(&ctx->err_word), (16 + kGemvTicketWords) * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(ctx->err_word, 0, (16 + kGemvTicketWords) * sizeof(int));
+    // [0] error word, [1] work-item counter
+    e = cudaMalloc(reinterpret_cast<void**>(&ctx->err_word), 16 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(ctx->err_word, 0, 16 * sizeof(int));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
     if (e != cudaSuccess) {
@@ -456,6 +454,7 @@ int mcl_cuda_batch_begin(mcl_cuda_ctx* ctx) {
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail_cuda(ctx, "batch_begin", e);
     ctx->recording = true;
+    ctx->last_gemv = nullptr;
     ctx->recorded_launches = ctx->launches;
     return MCL_CUDA_OK;
 }
@@ -1416,6 +1415,16 @@ int mcl_cuda_peer_allreduce_f32(mcl_cuda_ctx* ctx, const void* const* peer_data,
     return MCL_CUDA_OK;
 }
 
+// The one node that the next launch of a recording will depend on, or null.
+static cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    if (!ctx->recording || cudaStreamGetCaptureInfo_v2(ctx->stream, &st, nullptr, &graph, &deps, &n) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
+}
+
 int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* packed2,
                           const float* scale, float* y, size_t M, size_t in_features,
                           size_t out_features) {
@@ -1430,20 +1439,18 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
     MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
     MCL_TRY(check_ptr(ctx, op, "y", y, 4));
     DeviceGuard guard(ctx->device);
-    if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && M == 1 &&
-        mcl::gemv_lut_supported((int)M, (int)in_features, (int)out_features, packed2, kGemvTicketWords)) {
-        // one activation row: one launch that looks pairs of weights up in a table of activation sums
-        void* wsp = nullptr;
-        const size_t need = mcl::gemv_lut_workspace_bytes((int)in_features, (int)out_features);
-        if (need) MCL_TRY(ws_reserve(ctx, need, &wsp));
-        MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_lut(x, packed2, scale, y, (int)in_features, (int)out_features,
-                                                         static_cast<float*>(wsp),
-                                                         reinterpret_cast<unsigned int*>(ctx->err_word + 16), ctx->sm_count,
-                                                         ctx->max_smem, ctx->stream));
+    if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && mcl::gemv_mma_supported((int)M, (int)in_features, packed2, ctx->max_smem)) {
+        // One launch against three up to M = 8 (20 matrices of an 8B-scale model: 90 us against 194 at M = 2, 181 against 249 at
+        // M = 8; level at 11).  Only in a recording is it known what runs before: two of these in a row overlap, the
+        // second one's weights being no result of the first.
+        const cudaGraphNode_t tail = recorded_tail(ctx);
+        MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features,
+                                                         tail != nullptr && tail == ctx->last_gemv, ctx->sm_count, ctx->max_smem, ctx->stream));
+        ctx->last_gemv = recorded_tail(ctx);
         return MCL_CUDA_OK;
     }
     if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && M == 1) {
-        // a single activation row whose shape the table kernels do not take: streaming the words through the CUDA
+        // a single activation row whose shape the integer MMAs do not take: streaming the words through the CUDA
         // cores in one launch still beats the three launches of the tensor-core route
         MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_stream(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features,
                                                             ctx->sm_count, ctx->stream));

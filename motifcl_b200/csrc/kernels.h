@@ -111,19 +111,17 @@ cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* co
                                  int splits, cudaStream_t stream);
 
 // gemv.cu
-// M <= 2: one CUDA-core launch that streams the 2-bit words (in_features % 16 == 0)
+// M = 1: one CUDA-core launch that streams the 2-bit words (in_features % 16 == 0)
 cudaError_t launch_ternary_gemv_stream(const float* x, const uint32_t* packed2, const float* scale, float* y, int M,
                                        int in_features, int out_features, int sm_count, cudaStream_t stream);
-// table look-up kernels for M = 1 (in_features % 256 == 0, 16-byte aligned words); tickets: zeroed words, one per 256 rows
-bool gemv_lut_supported(int M, int in_features, int out_features, const void* packed2, int ticket_words);
-size_t gemv_lut_workspace_bytes(int in_features, int out_features);
-cudaError_t launch_ternary_gemv_lut(const float* x, const uint32_t* packed2, const float* scale, float* y,
-                                    int in_features, int out_features, float* part, unsigned int* tickets, int sm_count,
-                                    size_t max_smem, cudaStream_t stream);
 cudaError_t launch_ternary_gemv(const float* x, const uint32_t* packed2, const float* scale, float* y,
                                 int M, int in_features, int out_features, int sm_count,
                                 cudaStream_t stream);
 
+// gemv_mma.cu -- M <= 8 in one launch of integer MMAs; follows: the launch before this one on the stream is a launch of the same kernel
+bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem);
+cudaError_t launch_ternary_gemv_mma(const float* x, const uint32_t* packed2, const float* scale, float* y, int M, int in_features,
+                                    int out_features, bool follows, int sm_count, size_t max_smem, cudaStream_t stream);
 
 // peer_reduce.cu -- one-shot sum of a small vector over the GPUs of a node (peer loads, bounded flag wait)
 constexpr int kPeerMaxWorld = 8;
