@@ -319,8 +319,7 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    const int pair = tid >> 6;
-    const int vlane = tid & 63;
+    const int warp = tid >> 5;
     const int lv = 2 * p.C - 1;
     const float Cf = (float)p.C;
     const float neg_lr = -p.lr;
@@ -338,6 +337,7 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
     for (int batch = batch0; batch < nbatches; batch += batch_step) {
         const int row0 = batch * R;
         const int nrows = min(R, p.rows - row0);
+        const float s_old = tid < nrows ? p.scale[row0 + tid] : 0.0f, v_old = tid < nrows ? p.v[row0 + tid] : 0.0f;
 
         // ---- load: the batch's rows are contiguous in global memory ------------------------
         {
@@ -365,12 +365,13 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
         }
         __syncthreads();
 
-        // ---- stats: warp pair `pair` walks rows pair, pair + (NT / 64), ... ---------------------
-        for (int r = pair; r < nrows; r += (NT / 64)) {
-            float a = 0.0f, b = 0.0f;
+        // ---- stats: a warp per row, two of the 64 lanes of the reduction per thread; then the constants of all rows at once ------
+        // (a pair of warps that finished each row before its next one spent 1500 clocks a row on one lane's divisions)
+        for (int r = warp; r < nrows; r += NT / 32) {
+            float a0 = 0.0f, a1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
             const float4* g4 = gw_s + r * gpr;
             const uint32_t* raw = reinterpret_cast<const uint32_t*>(st_s + (size_t)r * L.sb);
-            for (int g = vlane; g < gpr; g += 64) {
+            auto add = [&](const int g, float& a, float& b) {
                 const float4 gw = g4[swz4(g)];
                 a = __fadd_rn(a, __fmul_rn(gw.x, gw.x));
                 a = __fadd_rn(a, __fmul_rn(gw.y, gw.y));
@@ -383,25 +384,23 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
                     b = __fadd_rn(b, __fmul_rn(gw.z, lut->e[(w >> 12) & 63u].x));
                     b = __fadd_rn(b, __fmul_rn(gw.w, lut->e[(w >> 18) & 63u].x));
                 }
+            };
+            for (int g = lane; g < gpr; g += 64) {
+                add(g, a0, b0);
+                if (g + 32 < gpr) add(g + 32, a1, b1);
             }
-            if (vlane >= 32) {
-                part[pair * 64 + lane] = a;
-                part[pair * 64 + 32 + lane] = b;
-            }
-            asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
-            if (vlane < 32) {
-                a = __fadd_rn(a, part[pair * 64 + lane]);
-                b = __fadd_rn(b, part[pair * 64 + 32 + lane]);
+            float a = __fadd_rn(a0, a1), b = __fadd_rn(b0, b1);
 #pragma unroll
-                for (int s = 16; s > 0; s >>= 1) {
-                    a = __fadd_rn(a, __shfl_down_sync(0xffffffffu, a, s));
-                    b = __fadd_rn(b, __shfl_down_sync(0xffffffffu, b, s));
-                }
-                if (lane == 0) rowc[r] = finish_row_stats<WITH_Q>(p, row0 + r, a, b, Cf, p.scale[row0 + r], p.v[row0 + r]);
+            for (int s = 16; s > 0; s >>= 1) {
+                a = __fadd_rn(a, __shfl_down_sync(0xffffffffu, a, s));
+                if (WITH_Q) b = __fadd_rn(b, __shfl_down_sync(0xffffffffu, b, s));
             }
-            asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
-            rowtab[r * 64 + vlane] = row_entry(lut, vlane, rowc[r].k_reb, sa_tick);     // one entry per old code value
+            if (lane == 0) { part[2 * r] = a; part[2 * r + 1] = b; }
         }
+        __syncthreads();
+        if (tid < nrows) rowc[tid] = finish_row_stats<WITH_Q>(p, row0 + tid, part[2 * tid], part[2 * tid + 1], Cf, s_old, v_old);
+        __syncthreads();
+        for (int e = tid; e < nrows * 64; e += NT) rowtab[e] = row_entry(lut, e & 63, rowc[e >> 6].k_reb, sa_tick);     // one entry per old code value
         __syncthreads();
 
         // ---- tick: 16 weights per thread-iteration, units of the whole batch flattened --------

@@ -447,17 +447,31 @@ __global__ void __launch_bounds__(512) sample_magnitude_kernel(const __grid_cons
     const long long total = (long long)T.R * T.Cc;
     const long long units = total >> 2, step = units > 4096 ? units / 4096 : 1;       // units of 4 consecutive elements
     float m0 = 0.0f, m1 = 0.0f;
-    auto add = [&](long long e) {
-        const float v = __ldg(T.src + e);
-        m0 = fmaxf(m0, fabsf(v));
-        if (T.planes_s) m1 = fmaxf(m1, fabsf(v * __ldg(T.col_scale + (int)(e % T.Cc))));
-    };
-#pragma unroll 2
-    for (long long u = threadIdx.x; u < units && u < 8192; u += 512) {
-        const long long e = u * step * 4;
-        if (e + 3 < total) { add(e); add(e + 1); add(e + 2); add(e + 3); }
+    auto add = [&](float v, float s) { m0 = fmaxf(m0, fabsf(v)); m1 = fmaxf(m1, fabsf(__fmul_rn(v, s))); };
+    const long long used = step > 1 ? min(units / step, 8192ll) : units;        // u * step < units; at most 8191 where step is 1
+    // a thread's loads all at once (taken two at a time, and with four divisions per unit, the launch took 19 us for 84 tensors)
+    if (T.vec && used * step * 4 < 0x7fffffffll) {               // a unit lies in one row
+        const int n = (int)used, st4 = (int)step * 4;
+        for (int u0 = threadIdx.x; u0 < n; u0 += 8 * 512) {
+            float4 v[8], s[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int e = min(u0 + k * 512, n - 1) * st4;
+                v[k] = __ldg(reinterpret_cast<const float4*>(T.src + e));
+                s[k] = T.planes_s ? __ldg(reinterpret_cast<const float4*>(T.col_scale + (uint32_t)e % (uint32_t)T.Cc)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { add(v[k].x, s[k].x); add(v[k].y, s[k].y); add(v[k].z, s[k].z); add(v[k].w, s[k].w); }
+        }
+    } else {
+        for (long long u = threadIdx.x; u < used; u += 512)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const long long e = u * step * 4 + k;
+                add(__ldg(T.src + e), T.planes_s ? __ldg(T.col_scale + (int)(e % T.Cc)) : 0.0f);
+            }
     }
-    for (long long e = (units << 2) + threadIdx.x; e < total; e += 512) add(e);
+    for (long long e = (units << 2) + threadIdx.x; e < total; e += 512) add(__ldg(T.src + e), T.planes_s ? __ldg(T.col_scale + (int)(e % T.Cc)) : 0.0f);
     const uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
     __shared__ uint32_t w0[16], w1[16];
     if ((threadIdx.x & 31) == 0) { w0[threadIdx.x >> 5] = b0; w1[threadIdx.x >> 5] = b1; }
@@ -490,6 +504,12 @@ __device__ __forceinline__ void split_terms8(const float (&v)[8], float f, uint4
 }
 template <bool FIX>
 __global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant__ SplitGroup g) {
+    if (FIX) {
+        const int t = threadIdx.x;              // kSplitCap <= 256
+        const bool redo = t < g.n && ((g.t[t].planes && terms_redone(__ldg(g.t[t].words), __ldg(g.t[t].words + 1))) ||
+                                      (g.t[t].planes_s && terms_redone(__ldg(g.t[t].words + 2), __ldg(g.t[t].words + 3))));
+        if (!__syncthreads_or(redo)) return;
+    }
     const long long total = g.chunk_begin[g.n];
     int ti = -1;
     long long first = 0, last = 0;             // chunks of tensor ti
@@ -532,7 +552,10 @@ __global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant_
                 f1 = do1 ? pow2(term_exp(__ldg(T.words + 2))) : 0.0f;
             }
         }
-        if (FIX && !do0 && !do1) continue;
+        if (FIX && !do0 && !do1) {              // on to the first chunk of this block beyond the tensor
+            ch += (last - 1 - ch) / gridDim.x * gridDim.x;
+            continue;
+        }
         const SplitTensor& T = g.t[ti];
         const int n8 = (T.Cc + 7) >> 3, Cc = T.Cc, ld = T.ld;
         const size_t units = (size_t)T.R * n8, ps = (size_t)T.R * ld;
