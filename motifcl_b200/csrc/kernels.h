@@ -63,9 +63,9 @@ cudaError_t launch_simt_grad_w(const float* grad_out, const float* x, float* gra
                                cudaStream_t stream);
 
 // tc_gemm.cu -- tcgen05 / TMEM / TMA contractions on fp16 term planes (see the file header)
-struct TcPlan { int pair, bn, splits, ktiles_per_split; size_t workspace_bytes; double cost; };
+struct TcPlan { int pair, bn, splits, ktiles_per_split, together; size_t workspace_bytes; double cost; };
 TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit);
-TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items);
+TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items, bool together = false);
 // k-tiles of 64 per accumulator for fp32 x fp32 products: 3 x 4 instructions per k-tile add into it, each with a truncation
 // error of about 2.7e-9 relative (K = 4096: 2e-6)
 constexpr int kGradDepthLimit = 64;

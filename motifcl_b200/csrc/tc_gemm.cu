@@ -41,7 +41,8 @@ struct TcTile {
     const uint32_t* a_words;  // magnitude words of the split tensor (null: operand is unscaled)
     const uint32_t* b_words;
     int M, N, K;
-    int BN, stage_bytes;      // tile width; bytes of one ring slot (A tile and this CTA's share of B)
+    int BN, stage_bytes;      // tile width; bytes of one ring slot (A tile and this CTA's share of B, or both terms of them)
+    int b_bytes;              // this CTA's share of a B tile
     int a_mn, b_mn;           // operand is stored with M / N contiguous
     int nterms;               // 2: A lo, A hi against one B plane; 3: lo.hi, hi.lo, hi.hi
     int ktiles_per_split, splits;
@@ -181,12 +182,16 @@ __device__ __forceinline__ TcItem tc_item(const TcTile* tab, int n, int item, in
 // CG = 1 and BN = 256 a k-tile of 64 moves 96 KB through a 128 B/clk pipe (768 cycles) for 512 cycles of MMA; with CG = 2
 // 64 KB (512).  All loads count on the leader's barrier.
 //
+// TOGETHER: a slot holds both terms of A and of B for one k-tile; hi.hi goes into one accumulator, lo.hi and hi.lo into a
+// second one beside it, and the epilogue adds the second scaled down by 2^-12.  Every plane is read once (4 tiles per k-tile
+// instead of 6): dW of 42 layers at 8192 tokens 456 -> 365 us, memory reads 2.2 -> 1.1 GB, 5.5 GB through L2 (15 TB/s: the bound).
+//
 // Every mbarrier wait is bounded: on time-out the kernel records an error word, skips the rest of its work, frees
 // its TMEM and returns.
 constexpr int kTcThreads = 192;
 constexpr int kStageBytes = 8 * 4096;      // epilogue staging: two 32 x 32 float tiles per warp
 
-template <int CG, int CAP>
+template <int CG, int CAP, bool TOGETHER>
 __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ TcTable<CAP> tab) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4];
@@ -206,7 +211,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     auto empty_bar = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
     auto acc_full = [&](int a) { return bar0 + 8u * (2 * kMaxStages + a); };
     auto acc_empty = [&](int a) { return bar0 + 8u * (2 * kMaxStages + 2 + a); };
-    const uint32_t acc_cols = (uint32_t)tab.acc_cols;      // of one accumulator: a power of two >= the widest BN
+    const uint32_t acc_cols = (uint32_t)tab.acc_cols;      // of one accumulator: a power of two >= the widest BN; together: of two
+    const uint32_t lo_cols = acc_cols >> 1;                // together: the lo products' accumulator starts here
     const uint32_t tmem_cols = 2 * acc_cols;               // <= 512
 
     {
@@ -251,7 +257,27 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn;
             const uint32_t bytes = (uint32_t)(CG * P.stage_bytes);
             const int m0 = (t.mt * CG + (int)rank) * BM, n0 = t.nt * BN + (int)rank * (BN / CG);
-            for (int term = 0; term < nterms && ok; ++term) {
+            const uint32_t b_bytes = (uint32_t)P.b_bytes;
+            for (int kk = 0; TOGETHER && kk < t.nkt; ++kk) {
+                ok = mbar_wait_all(empty_bar(s), ph, &abort_flag);
+                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 1); break; }
+                const uint32_t a_dst = tiles + (uint32_t)s * slot_bytes, b_dst = a_dst + 2 * kATileBytes;
+                const uint32_t bar = CG == 2 ? cluster_addr(full_bar(s), 0) : full_bar(s);
+                const int k0 = (t.kt0 + kk) * BK;
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(full_bar(s), bytes);
+                    for (int pl = 0; pl < 2; ++pl) {
+                        if (a_mn) tc_load4<CG>(a_dst + pl * kATileBytes, tmA, bar, m0, k0, 0, pl);
+                        else tc_load<CG>(a_dst + pl * kATileBytes, tmA, bar, k0, m0, pl);
+                        if (pl == 1 && nterms == 2) break;
+                        if (b_mn) tc_load4<CG>(b_dst + pl * b_bytes, tmB, bar, n0, k0, 0, pl);
+                        else tc_load<CG>(b_dst + pl * b_bytes, tmB, bar, k0, n0, pl);
+                    }
+                }
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1u; }
+            }
+            for (int term = 0; !TOGETHER && term < nterms && ok; ++term) {
                 // planes: 0 = hi, 1 = lo; products with a lo term first
                 const int pa = nterms == 3 ? (term == 0) : (term + 1 < nterms);
                 const int pb = nterms == 3 && term == 1;
@@ -294,7 +320,32 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                 if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 4); break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * acc_cols;
-                for (int j = 0; j < total; ++j) {
+                for (int j = 0; TOGETHER && j < t.nkt; ++j) {
+                    ok = mbar_wait_all(full_bar(s), ph, &abort_flag);
+                    if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 2); break; }
+                    tc_fence_after();
+                    const uint32_t off = ((uint32_t)s * slot_bytes) >> 4;
+                    const uint32_t a_lo = a0 + off, b_lo = b0 + off + (kATileBytes >> 4), b_next = (uint32_t)P.b_bytes >> 4;
+                    if (elect_one()) {
+                        const uint32_t more = j != 0 ? 1u : 0u;
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; ++kk)           // hi.hi
+                            umma_f16<CG>(d_tmem, a_lo + a_step * kk, a_hi, b_lo + b_step * kk, b_hi, idesc, kk ? 1u : more);
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; ++kk)           // lo.hi
+                            umma_f16<CG>(d_tmem + lo_cols, a_lo + (kATileBytes >> 4) + a_step * kk, a_hi, b_lo + b_step * kk, b_hi, idesc, kk ? 1u : more);
+                        if (P.nterms == 3) {
+#pragma unroll
+                            for (int kk = 0; kk < BK / 16; ++kk)       // hi.lo
+                                umma_f16<CG>(d_tmem + lo_cols, a_lo + a_step * kk, a_hi, b_lo + b_next + b_step * kk, b_hi, idesc, 1u);
+                        }
+                        tc_commit<CG>(empty_bar(s));
+                        if (j == t.nkt - 1) tc_commit<CG>(acc_full(acc));
+                    }
+                    __syncwarp();
+                    if (++s == S) { s = 0; ph ^= 1u; }
+                }
+                for (int j = 0; !TOGETHER && j < total; ++j) {
                     ok = mbar_wait_all(full_bar(s), ph, &abort_flag);
                     if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 2); break; }
                     tc_fence_after();
@@ -344,6 +395,18 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                 tmem_ld32(t_addr, r[0]);
                 if (c0 + 32 < ncols) tmem_ld32(t_addr + 32, r[1]);
                 tmem_ld_wait();
+                if (TOGETHER) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (c0 + 32 * h >= ncols) break;
+                        uint32_t l[32];
+                        tmem_ld32(t_addr + lo_cols + 32 * h, l);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            r[h][j] = __float_as_uint(fmaf(__uint_as_float(l[j]), 1.0f / (1 << kLoShift), __uint_as_float(r[h][j])));
+                    }
+                }
                 if (c0 + 64 >= ncols) {                // the accumulator is in registers: release it
                     tc_fence_before();
                     __syncwarp();
@@ -788,21 +851,27 @@ TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit) {
 
 // The same choice for one product among many that share a launch: what counts is the sum of the items' times, so tiles
 // waste least and K is split only where the accumulation depth asks for it, or `min_items` for more items.
-TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items) {
+// `together` (three terms): the three of a k-tile from one slot.  A term after the other over the whole of K reads the hi
+// planes twice, and with the slices of 18 layers in flight the second time from memory (dW of 42 layers at 8192 tokens: 2.2 GB
+// from memory and 9.4 GB through L2, which was its bound).  Then the lo products cannot wait for the scale-down of the first
+// hi product and get an accumulator of their own, so BN stops at 128.
+TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items, bool together) {
     TcPlan best = {};
     double best_cost = 1e300;
     const int ktiles = (K + BK - 1) / BK, tm = (M + cg * BM - 1) / (cg * BM);
-    for (int bn = 64; bn <= 256; bn += 32) {
+    for (int bn = 64; bn <= (together ? 128 : 256); bn += 32) {
         const int tiles = tm * ((N + bn - 1) / bn);
         int s = depth_limit > 0 ? (ktiles + depth_limit - 1) / depth_limit : 1;
         if (depth_limit > 0)
             while (tiles * s < min_items && ktiles >= 16 * (s + 1)) ++s;
         const int per = (ktiles + s - 1) / s, real = (ktiles + per - 1) / per;
-        const double cyc = (double)nterms * (2 * bn > 2 * (128 + bn / cg) ? 2 * bn : 2 * (128 + bn / cg));
+        // together: both operands are read MN-major, in whole chunks of 64; an SM takes about 28 bytes per clock out of L2
+        const double cyc = together ? 2.0 * (128 + (bn / cg + 63) / 64 * 64) * 128 / 28
+                                    : (double)nterms * (2 * bn > 2 * (128 + bn / cg) ? 2 * bn : 2 * (128 + bn / cg));
         const double cost = cg * ((double)tiles * real * (per * cyc + 500.0));
         if (cost < best_cost) {
             best_cost = cost;
-            best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per;
+            best.pair = cg == 2; best.bn = bn; best.splits = real; best.ktiles_per_split = per; best.together = together;
         }
     }
     best.cost = best_cost;
@@ -811,7 +880,7 @@ TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, 
 }
 
 namespace {
-template <int CG, int CAP>
+template <int CG, int CAP, bool TOGETHER>
 cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream) {
     static thread_local TcTable<CAP> tab;      // 28 KB: built in place, copied by the launch
     tab.n = n;
@@ -831,7 +900,8 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
         p.a_words = a.words; p.b_words = b.words;
         p.M = q.M; p.N = q.N; p.K = q.K;
         p.BN = bn;
-        p.stage_bytes = kATileBytes + (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
+        p.b_bytes = (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
+        p.stage_bytes = q.plan.together ? 2 * kATileBytes + b.planes * p.b_bytes : kATileBytes + p.b_bytes;
         p.a_mn = a.mn_major; p.b_mn = b.mn_major;
         p.nterms = b.planes == 2 ? 3 : 2;
         p.ktiles_per_split = q.plan.ktiles_per_split; p.splits = q.plan.splits;
@@ -841,18 +911,21 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
         items += p.tiles_m * p.tiles_n * p.splits;
         if (p.stage_bytes > tab.slot_bytes) tab.slot_bytes = p.stage_bytes;
         if (bn > bn_max) bn_max = bn;
-        if (p.nterms * p.ktiles_per_split > want) want = p.nterms * p.ktiles_per_split;
+        const int slots = (q.plan.together ? 1 : p.nterms) * p.ktiles_per_split;
+        if (slots > want) want = slots;
     }
     tab.n_items = items;
     tab.acc_cols = 64;
     while (tab.acc_cols < bn_max) tab.acc_cols *= 2;
+    if (TOGETHER) tab.acc_cols *= 2;
+    if (tab.acc_cols > 256) return cudaErrorInvalidValue;
     int stages = (int)((max_smem - 1024 - sizeof(TcTile) * CAP - 2048 - kStageBytes) / (size_t)tab.slot_bytes);
     if (stages > kMaxStages) stages = kMaxStages;
     // Two accumulators of one CTA take 2 * pow2(BN) TMEM columns of the SM's 512.  Narrow tiles (BN <= 128) with short main
     // loops leave room for a second resident CTA, which doubles the loads in flight where the loop is latency-bound; then
     // each CTA gets half the shared memory.
     bool two_ctas = false;
-    if (CG == 1 && bn_max <= 128 && want <= 32 && items > sm_count) {
+    if (CG == 1 && !TOGETHER && bn_max <= 128 && want <= 32 && items > sm_count) {
         const int half = (int)((max_smem / 2 - 2048 - sizeof(TcTile) * CAP - 1024 - kStageBytes) / (size_t)tab.slot_bytes);
         if (half >= 3) { two_ctas = true; if (half < stages) stages = half; }
     }
@@ -860,8 +933,8 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
     if (stages < 2) return cudaErrorInvalidConfiguration;
     tab.stages = stages;
     const size_t smem = (size_t)stages * tab.slot_bytes + 1024 + kStageBytes;
-    const auto kern = tc_gemm_kernel<CG, CAP>;
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), CG == 2 ? (CAP > 1 ? 24 : 16) : (CAP > 1 ? 25 : 4), max_smem);
+    const auto kern = tc_gemm_kernel<CG, CAP, TOGETHER>;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), TOGETHER ? (CG == 2 ? 30 : 31) : CG == 2 ? (CAP > 1 ? 24 : 16) : (CAP > 1 ? 25 : 4), max_smem);
     if (e != cudaSuccess) return e;
     int units = (sm_count / CG) * (two_ctas ? 2 : 1);
     if (units > items) units = items;
@@ -879,15 +952,23 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
 }
 }  // namespace
 
-// Products in launches of up to kTcCap each; all of a launch have the same plan.pair.
+// Products in launches of up to kTcCap each; all of a launch have the same plan.pair and plan.together.
 cudaError_t launch_tc_products(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream,
                                int* launches) {
     for (int i = 0; i < n;) {
         int k = 1;
-        while (i + k < n && k < kTcCap && probs[i + k].plan.pair == probs[i].plan.pair) ++k;
-        const cudaError_t e = probs[i].plan.pair
-            ? (k == 1 ? run_tc_table<2, 1>(probs + i, 1, err_word, max_smem, sm_count, stream) : run_tc_table<2, kTcCap>(probs + i, k, err_word, max_smem, sm_count, stream))
-            : (k == 1 ? run_tc_table<1, 1>(probs + i, 1, err_word, max_smem, sm_count, stream) : run_tc_table<1, kTcCap>(probs + i, k, err_word, max_smem, sm_count, stream));
+        while (i + k < n && k < kTcCap && probs[i + k].plan.pair == probs[i].plan.pair && probs[i + k].plan.together == probs[i].plan.together) ++k;
+        const bool pair = probs[i].plan.pair;
+        cudaError_t e;
+        if (probs[i].plan.together)
+            e = pair ? run_tc_table<2, kTcCap, true>(probs + i, k, err_word, max_smem, sm_count, stream)
+                     : run_tc_table<1, kTcCap, true>(probs + i, k, err_word, max_smem, sm_count, stream);
+        else if (k == 1)
+            e = pair ? run_tc_table<2, 1, false>(probs + i, 1, err_word, max_smem, sm_count, stream)
+                     : run_tc_table<1, 1, false>(probs + i, 1, err_word, max_smem, sm_count, stream);
+        else
+            e = pair ? run_tc_table<2, kTcCap, false>(probs + i, k, err_word, max_smem, sm_count, stream)
+                     : run_tc_table<1, kTcCap, false>(probs + i, k, err_word, max_smem, sm_count, stream);
         if (e != cudaSuccess) return e;
         ++*launches;
         i += k;

@@ -1,0 +1,29 @@
+"""Weight gradients of layers stepped together whose operands exceed L2: all terms of a k-tile from one slot."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("I,O,tokens,layers", [(288, 288, 32769, 3), (768, 288, 20000, 3), (64, 1000, 24001, 3), (320, 132, 60000, 3)])
+def test_grad_w_of_a_large_group(I, O, tokens, layers):
+    from motifcl_b200 import Context
+    from motifcl_b200.runtime import linear_descs
+    stream = torch.cuda.Stream(device=0)
+    with torch.cuda.stream(stream):
+        ctx = Context.on_torch_stream(0)
+        g = torch.Generator(device=DEV).manual_seed(I + O)
+        ls = []
+        for _ in range(layers):
+            ls.append(dict(x=torch.randn(tokens, I, device=DEV, generator=g), grad_out=torch.randn(tokens, O, device=DEV, generator=g) * 0.02,
+                           state=torch.randint(0, 256, (O * I // 4 * 3,), device=DEV, generator=g, dtype=torch.int32).to(torch.uint8),
+                           scale=torch.full((O,), 0.05, device=DEV), v=torch.zeros(O, device=DEV), y=torch.empty(tokens, O, device=DEV),
+                           grad_x=torch.empty(tokens, I, device=DEV), grad_w=torch.full((O, I), 7.0, device=DEV), packed2_out=None))
+        descs = linear_descs([dict(l, in_features=I, out_features=O, batch=tokens, update_rows=0) for l in ls])
+        ctx.counter_linear_step_many(descs, 11, 3e-3, 0.0, 0.9, 1e-3, 1)
+        for l in ls:
+            want = l["grad_out"].double().T @ l["x"].double()
+            assert float((l["grad_w"].double() - want).norm() / want.norm()) <= 5e-6
+            assert float((l["grad_w"].double() - want).abs().max() / want.square().mean().sqrt()) <= 5e-5
