@@ -65,9 +65,9 @@ def algorithmic(wl):
                 update_bytes=5.75 * W + 16.0 * rows)
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of the contraction kernel for one step of a workload, from the ncu
-# capture summarised in profiles/ (captured on a subset of the layers and scaled by layers where noted there)
-MEASURED_TRAFFIC_BYTES = {"cfg2": 3.412e9}     # 458.8 MB on the first 6 layers (both contraction launches) x (2180.0 / 293.1 MB algorithmic)
+# dram__bytes_read.sum + dram__bytes_write.sum of the contraction kernel's launches for one step of a workload, from the ncu
+# capture summarised in profiles/grouped_step_cfg2.md
+MEASURED_TRAFFIC_BYTES = {"cfg2": 3.248e9}
 
 
 class ClockSampler:
@@ -655,12 +655,12 @@ def time_wide_workload(ctx, wl, dev, steps, warmup, group=None):
     rec = {"workload": wl["desc"], "n_gpus": world, "tokens_per_gpu": wl["tokens"], "linears": len(wl["linears"]),
            "weights": alg["weights"], "steps": steps, "warmup": warmup, "ms_per_step": ms,
            "tokens_per_s": wl["tokens"] * world / (ms * 1e-3), "gpu_launches_per_step": (ctx.launch_count - l1) // steps,
-           "roofline": {"kernel": "whole step per GPU: operand splits, tc_gemm_kernel contractions (bf16 terms, 3 / 3 / 6 "
+           "roofline": {"kernel": "whole step per GPU: operand splits, tc_gemm_kernel contractions (fp16 terms, 2 / 2 / 3 "
                                   "products), fused update" + (", collectives overlapped" if world > 1 else ""),
                         "bound": "tensor", "achieved": tf, "peak": tf_peak, "unit": "TFLOP/s", "frac": tf / tf_peak,
                         "peak_kind": f"{peak_kind} bf16 sustained", "flop_per_step": alg["gemm_flop"],
-                        "pass_adjusted": {"bf16_pass_units_per_3_useful": 12.0, "ceiling": tf_peak / 4.0,
-                                          "frac": tf / (tf_peak / 4.0)}}}
+                        "pass_adjusted": {"bf16_pass_units_per_3_useful": 7.0, "ceiling": tf_peak * 3.0 / 7.0,
+                                          "frac": tf / (tf_peak * 3.0 / 7.0)}}}
     if world > 1:
         rec["collectives_per_step"] = {"reduce_scatter_bytes_in": 4.0 * alg["weights"],
                                        "all_gather_bytes_out": alg["weights"] / 4.0 + 4.0 * alg["rows"]}
@@ -934,13 +934,13 @@ def main():
     gemm_gbs = alg["gemm_bytes"] / (ms_gemm * 1e-3) / 1e9
     upd_gbs = alg["update_bytes"] / world / (ms_upd * 1e-3) / 1e9      # each rank updates its row shard
     # The scope table counts the three products as 6*tokens*weights flop against the dense bf16 rate.  Two more
-    # views explain the number: the pass-adjusted ceiling (fp32 fidelity costs 2 + 2 bf16 products for Y and dX and
-    # 3 tf32 products at half the bf16 rate for dW on narrow layers = 10 bf16-pass units per 3 useful) and the HBM view
+    # views explain the number: the pass-adjusted ceiling (fp32 fidelity costs 2 + 2 passes of fp16 terms for Y and
+    # dX and 3 for dW = 7 per 3 useful) and the HBM view
     # (algorithmic bytes of the products at the copy bandwidth), which is the larger ideal time when layers are narrow.
-    units = 10.0
+    units = 7.0
     traffic = MEASURED_TRAFFIC_BYTES.get(args.workload)
-    roofline = {"kernel": "counter-linear contractions (Y, dX, dW) of all linears: tc_fused_kernel (bf16 / tf32 hi-lo terms, "
-                          "A operands in tensor memory)",
+    roofline = {"kernel": "counter-linear contractions (Y, dX, dW) of all linears: tc_gemm_kernel (two fp16 terms per "
+                          "fp32 operand, CTA pairs)",
                 "bound": "tensor", "achieved": gemm_tf, "peak": tf_peak, "unit": "TFLOP/s", "frac": gemm_tf / tf_peak,
                 "peak_kind": f"{peak_kind} bf16 sustained", "traffic": traffic,
                 "flop_per_step": alg["gemm_flop"], "ms": ms_gemm,

@@ -172,14 +172,13 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
                                   float lr_scale, float rms_beta, float rms_eps, uint32_t seed);
 
 /* ---- how the three contractions are computed (no reference counterpart: the reference has one
- * fp32 path).  mode MCL_CUDA_GEMM_AUTO: tensor cores (tcgen05, bf16 term splitting) for shapes
+ * fp32 path).  mode MCL_CUDA_GEMM_AUTO: tensor cores (tcgen05, fp16 term splitting) for shapes
  * that are large and aligned enough, the exact CUDA-core kernels otherwise;
  * MCL_CUDA_GEMM_EXACT: always the CUDA-core kernels, whose every output equals the reference's
  * k-ascending fp32 sum bit for bit; MCL_CUDA_GEMM_TENSOR: tensor cores whenever the shape
- * allows.  act_terms (2 or 3) = bf16 terms per fp32 activation in Y and dX; grad_terms (3 or 6)
- * = term products in dW = dY^T X.  Defaults: AUTO, 3, 6 (error of every product below 1e-5
- * relative L2 against the fp32 reference sum; 2 / 3 also meet that bound and cost 7/12 of the
- * tensor-core time). ---- */
+ * allows.  act_terms (2 or 3) and grad_terms (3 or 6) are accepted as ever (defaults 3 and 6); every setting runs two fp16
+ * terms per fp32 tensor: two products for Y and dX, three for dW, below 1e-5 relative L2 against the fp32
+ * reference sum. ---- */
 #define MCL_CUDA_GEMM_AUTO 0
 #define MCL_CUDA_GEMM_EXACT 1
 #define MCL_CUDA_GEMM_TENSOR 2
