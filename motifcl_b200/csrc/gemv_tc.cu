@@ -13,6 +13,9 @@
 //   * sum_k x t = sum_k x f - sum_k x, so a per-row digit sum is subtracted at the end.
 // Integer accumulation is exact and order-independent, which makes split-K over atomics
 // deterministic.  A finalize kernel recombines the digits in double precision.
+// A CTA takes half of an SM's shared memory and tensor memory (one accumulator, three expanded tiles): the 2.4 us before its first
+// tile and the waits of its chain pass under another launch's work.  4 blocks of an 8B-scale model, 16 rows: 239 -> 184 us beside
+// other work, 423 -> 382 us alone (two accumulators, four tiles and all of the shared memory before).
 #include <cuda.h>
 
 #include "kernels.h"
@@ -27,7 +30,8 @@ constexpr int GV_RAW = GV_ROWS * (GV_KB / 4);          // 8 KiB staging of packe
 
 constexpr int GV_THREADS = 320;
 constexpr int GV_MAX_STAGES = 12;      // slots of the raw ring (packed weights + activation digits)
-constexpr int GV_EXP = 4;              // expanded tiles in flight in tensor memory, 64 columns each
+constexpr int GV_EXP = 3;              // expanded tiles in flight in tensor memory, 64 columns each
+constexpr int GV_ACOL0 = 64;           // after the accumulator; 256 columns in all, so that an SM holds two such CTAs
 constexpr int GV_ACOLS = 64;           // a [128 rows x 256 int8] tile = 64 32-bit columns
 
 struct GvParams {
@@ -60,11 +64,11 @@ __device__ __forceinline__ uint32_t idesc_i8(int m, int n) {
 __device__ __forceinline__ int gv_kperm(int k) { return (k & ~15) | ((k & 3) << 2) | ((k >> 2) & 3); }
 
 
-__global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_constant__ CUtensorMap tmP,
+__global__ void __launch_bounds__(GV_THREADS, 2) gemv_tc_kernel(const __grid_constant__ CUtensorMap tmP,
                                                              const __grid_constant__ CUtensorMap tmX,
                                                              const GvParams p) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * GV_EXP + 4];
+    __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * GV_EXP + 2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -82,11 +86,10 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_consta
     auto empty_bar = [&](int s) { return bar0 + 8u * (GV_MAX_STAGES + s); };
     auto a_full = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + e); };
     auto a_empty = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + GV_EXP + e); };
-    auto acc_full = [&](int a) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * GV_EXP + a); };
-    auto acc_empty = [&](int a) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * GV_EXP + 2 + a); };
-    // TMEM columns: [0, 2 Nq) two accumulators, [a_col0, a_col0 + GV_EXP * 64) expanded tiles
-    const uint32_t a_col0 = 128;
-    const uint32_t tmem_cols = 512;
+    const uint32_t acc_full = bar0 + 8u * (2 * GV_MAX_STAGES + 2 * GV_EXP), acc_empty = acc_full + 8u;
+    // TMEM columns: [0, Nq) the accumulator, [a_col0, a_col0 + GV_EXP * 64) expanded tiles
+    const uint32_t a_col0 = GV_ACOL0;
+    const uint32_t tmem_cols = 256;
 
     const int row_tiles = (p.O + GV_ROWS - 1) / GV_ROWS;
     const int n_items = row_tiles * p.splits;
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_consta
         abort_flag = (*reinterpret_cast<volatile int*>(p.err) != 0);
         for (int s = 0; s < S; ++s) { mbar_init(raw_full(s), 1); mbar_init(empty_bar(s), 1); }
         for (int e = 0; e < GV_EXP; ++e) { mbar_init(a_full(e), 128); mbar_init(a_empty(e), 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 128); }
+        mbar_init(acc_full, 1); mbar_init(acc_empty, 128);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -138,10 +141,9 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_consta
                 const int split = item / row_tiles;
                 const int kb0 = split * p.kb_per_split;
                 const int nkb = min(p.kb_per_split, p.kblocks - kb0);
-                const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
-                if (!mbar_wait(acc_empty(acc), aph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 14); break; }
+                if (!mbar_wait(acc_empty, (n_local & 1u) ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 14); break; }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * (uint32_t)Nq;
+                const uint32_t d_tmem = tmem_base;
                 for (int j = 0; j < nkb; ++j, ++it) {
                     const int s = (int)(it % (uint32_t)S);
                     const int e = (int)(it % GV_EXP);
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_consta
                     umma_commit(empty_bar(s));
                 }
                 if (abort_flag) break;
-                umma_commit(acc_full(acc));
+                umma_commit(acc_full);
             }
         }
     } else if (warp < 6) {
@@ -215,33 +217,29 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_tc_kernel(const __grid_consta
         uint32_t n_local = 0;
         for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n_local) {
             const int rt = item % row_tiles;
-            const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
             bool ok = !abort_flag;
-            if (ok && !mbar_wait(acc_full(acc), aph, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 15); ok = false; }
+            if (ok && !mbar_wait(acc_full, n_local & 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 15); ok = false; }
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
             const int row = rt * GV_ROWS + q * 32 + lane;
             int* dst = p.acc + row;
-            for (int c0 = 0; c0 < Nq; c0 += 16) {
-                uint32_t v[16];
-                tmem_ld16(tmem_base + acc * (uint32_t)Nq + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
-                tmem_ld_wait();
-                if (row < p.O) {
-                    // columns at and beyond 4 M are padding of the digit matrix (all zero): nothing to add
-                    if (p.splits == 1) {
+            uint32_t v[4][16];                      // all of it, then the next item may have the accumulator
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < p.ncols) dst[(size_t)(c0 + j) * p.O] = (int)v[j];
-                    } else {
+            for (int c = 0; c < 4; ++c)
+                if (c * 16 < Nq) tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), v[c]);
+            tmem_ld_wait();
+            tc_fence_before();
+            mbar_arrive(acc_empty);
+            if (row < p.O) {
+                // columns at and beyond 4 M are padding of the digit matrix (all zero): nothing to add
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < p.ncols) atomicAdd(dst + (size_t)(c0 + j) * p.O, (int)v[j]);
-                    }
+                for (int c = 0; c < 64; ++c) {
+                    if (c >= p.ncols) break;
+                    if (p.splits == 1) dst[(size_t)c * p.O] = (int)v[c >> 4][c & 15];
+                    else atomicAdd(dst + (size_t)c * p.O, (int)v[c >> 4][c & 15]);
                 }
             }
-            tc_fence_before();
-            mbar_arrive(acc_empty(acc));
         }
     }
     __syncwarp();
@@ -391,7 +389,7 @@ cudaError_t launch_ternary_gemv_tc(const float* x, const uint32_t* packed2, cons
     p.splits = splits = (p.kblocks + p.kb_per_split - 1) / p.kb_per_split;
     p.acc = acc; p.err = err_word;
     const size_t stage_bytes = (size_t)GV_RAW + 2 * (size_t)Nq * 128;
-    int stages = (int)((max_smem - 2048) / stage_bytes);
+    int stages = (int)((max_smem / 2 - 3072) / stage_bytes);
     if (stages > GV_MAX_STAGES) stages = GV_MAX_STAGES;
     if (stages < 2) return cudaErrorInvalidConfiguration;
     p.stages = stages;
