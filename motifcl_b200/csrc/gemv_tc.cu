@@ -381,7 +381,7 @@ cudaError_t launch_ternary_gemv_tc(const float* x, const uint32_t* packed2, cons
     const int row_tiles = (O + GV_ROWS - 1) / GV_ROWS;
     int splits = 1;
     if (row_tiles < 2 * sm_count) {
-        splits = (3 * sm_count + row_tiles - 1) / row_tiles;
+        splits = (2 * sm_count + row_tiles - 1) / row_tiles;     // two items per CTA: 184 us with three, 179 with two, 16 rows as above
         if (splits > p.kblocks / 2) splits = p.kblocks / 2;
         if (splits < 1) splits = 1;
     }
