@@ -1027,10 +1027,8 @@ def main():
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
                 "data": "synthetic",
                 "config": base_config(args.workload, wl, world),
-                "arm": {"precision": "fp32 in/out; layers up to 1024 features: Y and dX = tcgen05 bf16 on two bf16 terms of the fp32 "
-                                     "activations against exact bf16 ternary digits (2 products), dW = tcgen05 tf32 on "
-                                     "hi/lo terms of both operands (3 products); wider layers: tcgen05 bf16 on 3 "
-                                     "terms (3 / 6 products); fp32 accumulate in TMEM; relative L2 <= 1e-5 vs the "
+                "arm": {"precision": "fp32 in/out; tcgen05 fp16 on two scaled fp16 terms per fp32 tensor (24 bits): "
+                                     "Y and dX 2 products against exact fp16 ternary digits, dW 3; fp32 accumulate in TMEM; relative L2 <= 1e-5 vs the "
                                      "fp32 reference sums (tested; measured <= 6e-6); counter update bit-exact",
                         "grouped_call": not args.no_group, "lanes": 1 if not args.no_group else args.lanes,
                         "recorded_batch": not args.eager,
