@@ -66,11 +66,12 @@ __device__ __forceinline__ int term_exp(uint32_t amax_bits) {
     return s > 126 ? 126 : s;
 }
 // Exponent that a tensor's terms were made with.  words[0]: magnitude that f was chosen for (the largest of a sample, raised
-// by 2^kSampleRoom, or the exact maximum); words[1]: the exact maximum, found while splitting.  fp16 holds two binades more
-// than words[0] lands in; a tensor whose exact maximum lies beyond them is split again for it.
+// by 2^kSampleRoom, or the exact maximum); words[1]: the exact maximum, found while splitting.  words[0] lands in [2^14, 2^15);
+// of the binade above it fp16 rounds everything from 65520 up to infinity, so a tensor whose exact maximum has any larger
+// exponent than words[0] is split again for it.
 __device__ __forceinline__ bool terms_redone(uint32_t w0, uint32_t w1) {
     const int e0 = (int)(w0 >> 23);
-    return (int)(w1 >> 23) >= (e0 < 1 ? 1 : e0) + 2;
+    return (int)(w1 >> 23) > (e0 < 1 ? 1 : e0);
 }
 __device__ __forceinline__ int terms_exp(const uint32_t* words) {
     const uint32_t w0 = __ldg(words), w1 = __ldg(words + 1);
