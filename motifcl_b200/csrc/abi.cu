@@ -37,7 +37,8 @@ struct mcl_cuda_ctx {
     uint64_t lane_mark = 0;      // launches at the last lane_fork (when this context is a lane)
     bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end
     uint64_t recorded_launches = 0;
-    cudaGraphNode_t last_gemv = nullptr;   // node of the last gemv_mma launch of the recording
+    cudaGraphNode_t last_gemv = nullptr;   // node of the last gemv_mma launch on this stream, and the capture it belongs to: a
+    unsigned long long last_capture = 0;   // handle alone may come back for a node of a later one
     int live_batches = 0;        // recorded batches not yet destroyed: they hold addresses inside the workspace
 };
 
@@ -459,7 +460,6 @@ int mcl_cuda_batch_begin(mcl_cuda_ctx* ctx) {
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail_cuda(ctx, "batch_begin", e);
     ctx->recording = true;
-    ctx->last_gemv = nullptr;
     ctx->recorded_launches = ctx->launches;
     return MCL_CUDA_OK;
 }
@@ -1420,13 +1420,13 @@ int mcl_cuda_peer_allreduce_f32(mcl_cuda_ctx* ctx, const void* const* peer_data,
     return MCL_CUDA_OK;
 }
 
-// The one node that the next launch of a recording will depend on, or null.
-static cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx) {
+// The one node that the next launch of a recording will depend on, or null; *capture: id of the recording.
+static cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx, unsigned long long* capture) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     size_t n = 0;
-    if (!ctx->recording || cudaStreamGetCaptureInfo_v2(ctx->stream, &st, nullptr, &graph, &deps, &n) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (!ctx->recording || cudaStreamGetCaptureInfo_v2(ctx->stream, &st, capture, &graph, &deps, &n) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
 }
 
@@ -1448,10 +1448,12 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
         // One launch against three up to M = 8 (20 matrices of an 8B-scale model: 90 us against 194 at M = 2, 181 against 249 at
         // M = 8; level at 11).  Only in a recording is it known what runs before: two of these in a row overlap, the
         // second one's weights being no result of the first.
-        const cudaGraphNode_t tail = recorded_tail(ctx);
-        MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features,
-                                                         tail != nullptr && tail == ctx->last_gemv, ctx->sm_count, ctx->max_smem, ctx->stream));
-        ctx->last_gemv = recorded_tail(ctx);
+        unsigned long long capture = 0;
+        const cudaGraphNode_t tail = recorded_tail(ctx, &capture);
+        const bool follows = tail != nullptr && tail == ctx->last_gemv && capture == ctx->last_capture;
+        MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features, follows,
+                                                         ctx->sm_count, ctx->max_smem, ctx->stream));
+        ctx->last_gemv = recorded_tail(ctx, &ctx->last_capture);
         return MCL_CUDA_OK;
     }
     if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && M == 1) {

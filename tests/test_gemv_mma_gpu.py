@@ -64,3 +64,41 @@ def test_recorded_chain_reads_the_result_before_it(M):
     for _ in range(6):
         want = (want @ up_d.T * us.cpu().numpy()) @ down_d.T * ds.cpu().numpy()
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+def test_lane_recorded_again_reads_words_made_just_before():
+    """A lane that ended an earlier recording with a GEMV: in the next recording the words are the result of the kernel before it,
+    whatever handles the destroyed recording's nodes leave behind."""
+    rng = np.random.default_rng(5)
+    O, I, M = 8192, 4096, 2
+    old, _, scale = _matrix(rng, O, I)
+    state = torch.from_numpy(rng.integers(0, 256, O * I // 4 * 3, dtype=np.uint8)).to(DEV)
+    x = rng.standard_normal((M, I)).astype(np.float32)
+    stream, ctx = _context()
+    from motifcl_b200 import Context
+    with torch.cuda.stream(stream):
+        lane = Context(0)
+        sc, dx, y = torch.from_numpy(scale).to(DEV), torch.from_numpy(x).to(DEV), torch.empty(M, O, device=DEV)
+        words, w = torch.empty_like(old), torch.empty(O, I, device=DEV)
+        ctx.counter_decode_weight(state, sc, w, I, O, 11)
+        want = dx.double() @ w.double().T
+        ctx.finish()
+        for _ in range(4):
+            ctx.batch_begin()
+            ctx.lane_fork(lane)
+            for _ in range(2):
+                lane.ternary_gemv(dx, old, sc, y, M, I, O)
+            ctx.lane_join(lane)
+            ctx.batch_end().close()
+            ctx.batch_begin()
+            ctx.lane_fork(lane)
+            lane.counter_pack2(state, words, I, O, 11)
+            lane.ternary_gemv(dx, words, sc, y, M, I, O)
+            ctx.lane_join(lane)
+            batch = ctx.batch_end()
+            words.zero_()
+            batch.launch()
+            ctx.finish()
+            batch.close()
+            assert float((y.double() - want).norm() / want.norm()) <= 1e-6
+        lane.close()
