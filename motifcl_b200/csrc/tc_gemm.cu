@@ -24,6 +24,7 @@
 
 #include "counter_codec.cuh"
 #include "kernels.h"
+#include "sample_rule.h"
 #include "tc_ptx.cuh"
 
 namespace mcl {
@@ -485,7 +486,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, float* _
 
 // ---- pre-pass 1: the magnitude that a tensor's terms are scaled for ---------------------------------------------
 // Reading a whole tensor for its maximum costs half of what splitting it does (25 us of 67 us for 16384 x 2048), so the choice is
-// made from a sample: the largest of up to 16384 evenly spaced elements, raised by 2^kSampleRoom.  The split itself sees every
+// made from a sample: the largest of up to 16384 elements spread over rows and columns, raised by 2^kSampleRoom.  The split itself sees every
 // element and records the exact maximum; a third launch, empty unless some tensor is larger than fp16 holds, splits those
 // again.  Small tensors are sampled whole.  With the room the terms keep all bits of elements down to 2^-20 of the sample's
 // maximum and are off by less than 2^-42 of it below.
@@ -509,18 +510,18 @@ constexpr int kSplitChunk = 2048;
 __global__ void __launch_bounds__(512) sample_magnitude_kernel(const __grid_constant__ SplitGroup g) {
     const SplitTensor& T = g.t[blockIdx.x];
     const long long total = (long long)T.R * T.Cc;
-    const long long units = total >> 2, step = units > 4096 ? units / 4096 : 1;       // units of 4 consecutive elements
+    const long long units = total >> 2, step = units > kSampleUnits ? units / kSampleUnits : 1;       // units of 4 consecutive elements
     float m0 = 0.0f, m1 = 0.0f;
     auto add = [&](float v, float s) { m0 = fmaxf(m0, fabsf(v)); m1 = fmaxf(m1, fabsf(__fmul_rn(v, s))); };
-    const long long used = step > 1 ? min(units / step, 8192ll) : units;        // u * step < units; at most 8191 where step is 1
+    const long long used = step > 1 ? min(units / step, 2ll * kSampleUnits) : units;        // (u + 1) * step <= units; at most 8191 where step is 1
     // a thread's loads all at once (taken two at a time, and with four divisions per unit, the launch took 19 us for 84 tensors)
     if (T.vec && used * step * 4 < 0x7fffffffll) {               // a unit lies in one row
-        const int n = (int)used, st4 = (int)step * 4;
+        const int n = (int)used;
         for (int u0 = threadIdx.x; u0 < n; u0 += 8 * 512) {
             float4 v[8], s[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const int e = min(u0 + k * 512, n - 1) * st4;
+                const int e = 4 * (int)sample_unit(min(u0 + k * 512, n - 1), step);
                 v[k] = __ldg(reinterpret_cast<const float4*>(T.src + e));
                 s[k] = T.planes_s ? __ldg(reinterpret_cast<const float4*>(T.col_scale + (uint32_t)e % (uint32_t)T.Cc)) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
@@ -531,7 +532,7 @@ __global__ void __launch_bounds__(512) sample_magnitude_kernel(const __grid_cons
         for (long long u = threadIdx.x; u < used; u += 512)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const long long e = u * step * 4 + k;
+                const long long e = sample_unit(u, step) * 4 + k;
                 add(__ldg(T.src + e), T.planes_s ? __ldg(T.col_scale + (int)(e % T.Cc)) : 0.0f);
             }
     }
@@ -1026,7 +1027,7 @@ cudaError_t launch_split_terms(const SplitDesc* d, int n, int sm_count, cudaStre
                     (t.col_scale == nullptr || (reinterpret_cast<uintptr_t>(t.col_scale) & 15) == 0);
             g.chunk_begin[j] = chunks;
             chunks += ((long long)q.rows * ((q.cols + 7) / 8) + kSplitChunk - 1) / kSplitChunk;
-            if ((long long)q.rows * q.cols / 4 >= 2 * 4096) sampled = true;
+            if ((long long)q.rows * q.cols / 4 >= 2 * kSampleUnits) sampled = true;
         }
         g.chunk_begin[take] = chunks;
         g.n = take;

@@ -70,3 +70,23 @@ def test_synthetic_shapes_and_weight_counts():
     codes = codec.unpack_codes(st, 288)
     assert codes.min() == 0 and codes.max() == 63
     assert synth.seed_for(2, 3, 1) == 20261125 + 2000 + 30 + 1
+
+
+@pytest.mark.parametrize("rows,cols", [(8192, 288), (4096, 32000), (16384, 2048), (777, 1000), (1024, 512), (65536, 256)])
+def test_magnitude_sample_covers_rows_and_columns(tmp_path, rows, cols):
+    """The sampled units of a tensor stay inside it, one to a run, and see its columns evenly, also where a run is whole rows."""
+    import subprocess
+    units = rows * cols // 4
+    step = max(1, units // 4096)
+    src = tmp_path / "s.cpp"
+    src.write_text('#include <cstdio>\n#include "sample_rule.h"\nint main() { for (long long u = 0; u < %d; ++u) '
+                   'std::printf("%%lld\\n", mcl::sample_unit(u, %d)); }\n' % (units // step, step))
+    exe = str(tmp_path / "s")
+    subprocess.check_call(["g++", "-std=c++17", "-I", os.path.join(os.path.dirname(mb._lib.HEADER_PATH), os.pardir, "motifcl_b200", "csrc"), str(src), "-o", exe])
+    at = np.array(subprocess.check_output([exe]).split(), dtype=np.int64)
+    assert at.size >= 4096 and at.max() < units and np.array_equal(at // step, np.arange(at.size))
+    groups = cols // 4
+    seen = np.bincount(at % groups, minlength=groups)
+    assert seen.max() <= 3 * -(-at.size // groups) + 2                          # no column is favoured
+    assert np.count_nonzero(seen) >= 0.35 * min(groups, at.size)                 # chance would give 1 - e^(-samples / groups)
+    assert np.count_nonzero(np.bincount(at // groups, minlength=rows)) >= 0.35 * min(rows, at.size)
