@@ -178,7 +178,17 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
  * k-ascending fp32 sum bit for bit; MCL_CUDA_GEMM_TENSOR: tensor cores whenever the shape
  * allows.  act_terms (2 or 3) and grad_terms (3 or 6) are accepted as ever (defaults 3 and 6); every setting runs two fp16
  * terms per fp32 tensor: two products for Y and dX, three for dW, below 1e-5 relative L2 against the fp32
- * reference sum. ---- */
+ * reference sum.  What the 1e-5 is relative to on the tensor cores:
+ *   Y, dX, and the rows of c that come from rows of a (columns from rows of b): each row (column) by itself.  A row far below the others
+ *     keeps its bits; an infinity, a NaN or a huge value reaches only the rows (columns) that it belongs to.
+ *   dW, and matmul_f32 with trans_a and without trans_b: the sum over the tokens, with elements that are below 2^-42 of the largest
+ *     max|x_t| max|dy_t| of a token t lost.  So a token 2^20 above the others costs nothing, one 2^42 above them hides their
+ *     part of the elements that it does not reach itself, which an fp32 sum would keep.  Infinities and NaN stay in
+ *     their row or column of dW.
+ *   matmul_f32, an operand contracted over its rows alone (b without trans_b and without trans_a, a with both): elements below 2^-42 of
+ *     its largest finite one are lost.
+ * MCL_CUDA_GEMM_EXACT has none of these limits.  The one-launch kernels of narrow layers (forward, backward_input, update_fused)
+ * carry every element with its own exponent. ---- */
 #define MCL_CUDA_GEMM_AUTO 0
 #define MCL_CUDA_GEMM_EXACT 1
 #define MCL_CUDA_GEMM_TENSOR 2

@@ -244,29 +244,36 @@ bool layer_wanted(const mcl_cuda_ctx* ctx, size_t tokens, size_t I, size_t O) {
 
 // Tensor-core products on fp16 terms (tc_gemm.cu).  A call carves the terms of its tensors from the workspace, fills them, and
 // runs its products.
-struct TermBuf { size_t planes, scaled, words; size_t rows; int cols, ld; };
+enum Scaling { kByRow, kByPartner };     // planes: a scale per row, or one that completes those of the partner's rows (kernels.h, SplitDesc)
+struct TermBuf { size_t planes, scaled, words, inv, inv_s; size_t rows; int cols, ld; Scaling how; };
 size_t term_bytes(size_t rows, size_t cols) { return 2 * rows * (size_t)up8(cols) * 2 + mcl::kTermPad; }
 size_t digit_bytes(size_t O, size_t I) { return O * (size_t)up8(I) * 2 + mcl::kTermPad; }
-TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled) {
-    TermBuf t = {0, 0, 0, rows, (int)cols, up8(cols)};
-    t.words = cv->reserve(16);
+TermBuf carve_terms(Carver* cv, size_t rows, size_t cols, bool plain, bool scaled, Scaling how) {
+    TermBuf t = {0, 0, 0, 0, 0, rows, (int)cols, up8(cols), how};
     if (plain) t.planes = cv->reserve(term_bytes(rows, cols));
-    if (scaled) t.scaled = cv->reserve(term_bytes(rows, cols));
+    if (plain && how == kByRow) t.inv = cv->reserve(rows * sizeof(float));
+    if (plain && how == kByPartner) t.words = cv->reserve(2 * sizeof(uint32_t));
+    if (scaled) { t.scaled = cv->reserve(term_bytes(rows, cols)); t.inv_s = cv->reserve(rows * sizeof(float)); }
     return t;
 }
-// col_scale != null: the scaled terms are made too
-mcl::SplitDesc split_of(char* w, const TermBuf& t, const float* src, const float* col_scale, bool plain) {
+// col_scale != null: the scaled terms are made too; partner: whose row scales the plain planes complete (null: none)
+mcl::SplitDesc split_of(char* w, const TermBuf& t, const float* src, const float* col_scale, bool plain, const TermBuf* partner) {
     mcl::SplitDesc d = {src, (int)t.rows, t.cols, t.ld, col_scale, plain ? w + t.planes : nullptr, col_scale ? w + t.scaled : nullptr,
-                        reinterpret_cast<uint32_t*>(w + t.words)};
+                        plain && t.how == kByRow ? reinterpret_cast<float*>(w + t.inv) : nullptr,
+                        col_scale ? reinterpret_cast<float*>(w + t.inv_s) : nullptr,
+                        plain && partner ? reinterpret_cast<const float*>(w + partner->inv) : nullptr,
+                        plain && t.how == kByPartner ? reinterpret_cast<uint32_t*>(w + t.words) : nullptr};
     return d;
 }
 mcl::TcOperand terms_of(char* w, const TermBuf& t, bool scaled, bool mn_major) {
-    mcl::TcOperand o = {w + (scaled ? t.scaled : t.planes), (int)t.rows, t.cols, t.ld, 2, mn_major ? 1 : 0,
-                        reinterpret_cast<const uint32_t*>(w + t.words) + (scaled ? 2 : 0)};
+    mcl::TcOperand o = {w + (scaled ? t.scaled : t.planes), (int)t.rows, t.cols, t.ld, 2, mn_major ? 1 : 0, nullptr, nullptr};
+    if (scaled) o.inv = reinterpret_cast<const float*>(w + t.inv_s);
+    else if (t.how == kByPartner) o.words = reinterpret_cast<const uint32_t*>(w + t.words);
+    else if (!mn_major) o.inv = reinterpret_cast<const float*>(w + t.inv);
     return o;
 }
 mcl::TcOperand digits_of(const char* T, size_t O, size_t I, bool mn_major) {
-    mcl::TcOperand o = {T, (int)O, (int)I, up8(I), 1, mn_major ? 1 : 0, nullptr};
+    mcl::TcOperand o = {T, (int)O, (int)I, up8(I), 1, mn_major ? 1 : 0, nullptr, nullptr};
     return o;
 }
 #define MCL_TC(ctx, op, call) do { int _n = 0; cudaError_t _e = (call); (ctx)->launches += _n; if (_e != cudaSuccess) return fail_cuda(ctx, op, _e); } while (0)
@@ -336,8 +343,8 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     };
     for (size_t i = 0; i < n; ++i) {
         const ProductLayer& l = L[i];
-        xb[i] = carve_terms(&cv, l.Nt, l.I, l.y || l.grad_w, false);
-        gb[i] = carve_terms(&cv, l.Nt, l.O, l.grad_w != nullptr, l.grad_x != nullptr);
+        xb[i] = carve_terms(&cv, l.Nt, l.I, l.y || l.grad_w, false, kByRow);
+        gb[i] = carve_terms(&cv, l.Nt, l.O, l.grad_w != nullptr, l.grad_x != nullptr, kByPartner);
         if (l.y || l.grad_x) t_off[i] = cv.reserve(digit_bytes(l.O, l.I));
     }
     for (size_t i = 0; i < n; ++i) {
@@ -358,8 +365,8 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     std::vector<mcl::ExpandDesc> ed;
     for (size_t i = 0; i < n; ++i) {
         const ProductLayer& l = L[i];
-        if (l.y || l.grad_w) sd.push_back(split_of(w, xb[i], l.x, nullptr, true));
-        if (l.grad_x || l.grad_w) sd.push_back(split_of(w, gb[i], l.grad_out, l.grad_x ? l.scale : nullptr, l.grad_w != nullptr));
+        if (l.y || l.grad_w) sd.push_back(split_of(w, xb[i], l.x, nullptr, true, nullptr));
+        if (l.grad_x || l.grad_w) sd.push_back(split_of(w, gb[i], l.grad_out, l.grad_x ? l.scale : nullptr, l.grad_w != nullptr, &xb[i]));
         if (l.y || l.grad_x) {
             const mcl::ExpandDesc d = {l.state, l.packed2, (int)l.O, (int)l.I, up8(l.I), w + t_off[i]};
             ed.push_back(d);
@@ -775,8 +782,8 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     TermBuf gb, xb;
     if (tc) {
         plan = dense_plan(ctx, tile_rows, in_features, batch);
-        gb = carve_terms(&cv, batch, out_features, true, false);      // activation-sized, not weight-sized
-        xb = carve_terms(&cv, batch, in_features, true, false);
+        gb = carve_terms(&cv, batch, out_features, true, false, kByPartner);      // activation-sized, not weight-sized
+        xb = carve_terms(&cv, batch, in_features, true, false, kByRow);
         o_k = cv.reserve(plan.workspace_bytes);
     }
     void* wsp = nullptr;
@@ -784,7 +791,7 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     char* w = static_cast<char*>(wsp);
     float* gw = reinterpret_cast<float*>(w + o_gw);
     if (tc) {
-        const mcl::SplitDesc sd[2] = {split_of(w, gb, grad_out, nullptr, true), split_of(w, xb, x, nullptr, true)};
+        const mcl::SplitDesc sd[2] = {split_of(w, xb, x, nullptr, true, nullptr), split_of(w, gb, grad_out, nullptr, true, &xb)};
         MCL_TRY(split_tensors(ctx, op, sd, 2));
     }
     for (size_t r0 = 0; r0 < out_features; r0 += tile_rows) {
@@ -1023,14 +1030,17 @@ int mcl_cuda_matmul_f32(mcl_cuda_ctx* ctx, const float* a, const float* b, float
     if (tc_wanted(ctx, M, N, K, c)) {
         const mcl::TcPlan plan = dense_plan(ctx, M, N, K);
         Carver cv;
-        // a stored [M,K] or (trans_a) [K,M], b stored [K,N] or (trans_b) [N,K]: split as stored, read in the needed orientation
-        const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false);
-        const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false);
+        // a stored [M,K] or (trans_a) [K,M], b stored [K,N] or (trans_b) [N,K]: split as stored, read in the needed orientation.  Rows
+        // that are rows or columns of c are scaled by row; of two that are both contracted over, the larger is, and the
+        // smaller completes it.
+        const bool both = trans_a && !trans_b, a_rows = !trans_a || (both && M >= N), b_rows = trans_b || (both && M < N);
+        const TermBuf ab = carve_terms(&cv, trans_a ? K : M, trans_a ? M : K, true, false, a_rows ? kByRow : kByPartner);
+        const TermBuf bb = carve_terms(&cv, trans_b ? N : K, trans_b ? K : N, true, false, b_rows ? kByRow : kByPartner);
         const size_t o_k = cv.reserve(plan.workspace_bytes);
         void* wsp = nullptr;
         MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
         char* w = static_cast<char*>(wsp);
-        const mcl::SplitDesc sd[2] = {split_of(w, ab, a, nullptr, true), split_of(w, bb, b, nullptr, true)};
+        const mcl::SplitDesc sd[2] = {split_of(w, ab, a, nullptr, true, both && !a_rows ? &bb : nullptr), split_of(w, bb, b, nullptr, true, both && !b_rows ? &ab : nullptr)};
         MCL_TRY(split_tensors(ctx, op, sd, 2));
         return tc_product(ctx, op, tc_problem(terms_of(w, ab, false, trans_a != 0), terms_of(w, bb, false, trans_b == 0), c, M, N, K, plan, nullptr, w + o_k));
     }

@@ -75,7 +75,8 @@ struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major 
     int rows, cols, ld;
     int planes;                // 2: hi and lo terms of an fp32 tensor; 1: ternary digits
     int mn_major;              // the contraction runs over the rows (0: over the columns)
-    const uint32_t* words;     // magnitude words of the split tensor (null for digits)
+    const float* inv;          // K-major and scaled by row: 2^-s of every row (else null)
+    const uint32_t* words;     // words of the exponent g, where this operand is the one that carries it (at most one of a product)
 };
 // C[M,N] = sum over k of A B (b.planes == 1: two products, b.planes == 2: three); with plan.splits > 1 into splitk_ws
 // [splits][M][N], which a reduction adds up
@@ -89,13 +90,20 @@ struct TcProblem {
 };
 cudaError_t launch_tc_products(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream,
                                int* launches);
-struct SplitDesc {             // fp32 [rows, cols] -> fp16 terms [2][rows][ld] of src (planes) and / or of src . col_scale (planes_s)
+// fp32 [rows, cols] -> fp16 terms [2][rows][ld] of src (planes) and / or of src . col_scale (planes_s).  planes_s, and planes where
+// row_inv is given, are scaled by a power of two 2^s of each row; row_inv / row_inv_s receive 2^-s.  Planes without row_inv are scaled by
+// 2^(g - s_t), with 2^-s_t from `comp` (row_inv of the tensor on the other side of a contraction over the rows; null: 1), and
+// words receives what g follows from.
+struct SplitDesc {
     const float* src;
     int rows, cols, ld;
     const float* col_scale;
     void* planes;
     void* planes_s;
-    uint32_t* words;           // four words: magnitude and exact maximum of the two
+    float* row_inv;
+    float* row_inv_s;
+    const float* comp;
+    uint32_t* words;           // two words
 };
 cudaError_t launch_split_terms(const SplitDesc* d, int n, int sm_count, cudaStream_t stream, int* launches);
 struct ExpandDesc {            // ternary digits as fp16 [O][ld], from the 6-bit state (state != null) or the 2-bit words (I % 16 == 0, ld == I)

@@ -10,14 +10,21 @@
 // so every tensor is split once, in its own layout, and T is expanded once: a transposed operand is the
 // same shared-memory tile with the MN-major bit of the instruction descriptor.
 //
-// How an fp32 tensor becomes two fp16 terms (split_terms_kernel): with m = the largest magnitude of the tensor and
-// f = 2^(14 - floor(log2 m)), hi = fp16(a f) and lo = fp16((a f - hi) 2^12).  hi keeps 11 bits, the residual is at most
-// half a unit of hi and keeps 11 more below its sign: |a f - hi - lo 2^-12| <= 2^-23 |a f|, the last bit of fp32 (the first
-// bf16 form of this file needed three 8-bit terms for the same bits).  lo is stored 2^12 up so that it stays a normal
-// number wherever hi is: elements down to 2^-28 of the largest keep all their bits, smaller ones are off by less
-// than 2^-50 of it.  The lo products go into the accumulator first; the first hi product scales it down by 2^-12
-// (tcgen05.mma scale-input-d), and the epilogue undoes f.  Ternary digits are exact in fp16.  Cost per product of a
-// step in bf16-rate passes: Y, dX 2 (3 before), dW 3 (hi.hi + hi.lo + lo.hi; 6 before).
+// How an fp32 tensor becomes two fp16 terms (split_terms_kernel): with a power of two f that brings the largest magnitude
+// into [2^14, 2^15), hi = fp16(a f) and lo = fp16((a f - hi) 2^12).  hi keeps 11 bits, the residual is at most half a unit of
+// hi and keeps 11 more below its sign: |a f - hi - lo 2^-12| <= 2^-23 |a f|, the last bit of fp32 (the first bf16 form of this
+// file needed three 8-bit terms for the same bits).  lo is stored 2^12 up so that it stays a normal number wherever hi is:
+// elements down to 2^-28 of the largest keep all their bits, smaller ones are off by less than 2^-50 of it.
+// What f belongs to:
+//   an operand whose rows are rows (or columns) of the product: each row has its own f from its own largest finite element,
+//       and the epilogue undoes it.  A row far below the others keeps its bits; an infinity, a NaN or a huge value stays in
+//       the rows (columns) of the product that it belongs to.
+//   dW and other products along the rows of both: one operand has a scale 2^s_t per row t as above, the other 2^(g - s_t), and
+//       the epilogue undoes 2^g.  g follows from the largest |a_t| max|b_t|, so what is lost is below 2^-42 (sampled, see
+//       there) of the largest product.  Infinities and NaN stay in their column.
+// The lo products go into the accumulator first; the first hi product scales it down by 2^-12 (tcgen05.mma scale-input-d).
+// Ternary digits are exact in fp16.  Cost per product of a step in bf16-rate passes: Y, dX 2 (3 before), dW 3
+// (hi.hi + hi.lo + lo.hi; 6 before).
 // The kernel is bound by the tensor pipe; its time at a stated size stands at tc_gemm_kernel.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -39,8 +46,9 @@ constexpr int kLoShift = 12;               // lo terms are stored 2^12 up
 // One product of a launch's table.
 struct TcTile {
     const float* col_scale;   // optional, applied when splits == 1
-    const uint32_t* a_words;  // magnitude words of the split tensor (null: operand is unscaled)
-    const uint32_t* b_words;
+    const float* a_inv;       // 2^-s of every row of A, of every row of B (column of the product); null: 1
+    const float* b_inv;
+    const uint32_t* words;    // the product's words of g (null: g = 0)
     int M, N, K;
     int BN, stage_bytes;      // tile width; bytes of one ring slot (A tile and this CTA's share of B, or both terms of them)
     int b_bytes;              // this CTA's share of a B tile
@@ -60,24 +68,24 @@ struct TcTable {
 };
 constexpr int kTcCap = 60;
 
-// exponent of f (see the file header): the largest magnitude lands in [2^14, 2^15)
+// s of a row (see the file header): its largest magnitude lands in [2^14, 2^15)
 __device__ __forceinline__ int term_exp(uint32_t amax_bits) {
     const int e = (int)(amax_bits >> 23);
     const int s = 141 - (e < 1 ? 1 : e);
     return s > 126 ? 126 : s;
 }
-// Exponent that a tensor's terms were made with.  words[0]: magnitude that f was chosen for (the largest of a sample, raised
-// by 2^kSampleRoom, or the exact maximum); words[1]: the exact maximum, found while splitting.  words[0] lands in [2^14, 2^15);
-// of the binade above it fp16 rounds everything from 65520 up to infinity, so a tensor whose exact maximum has any larger
-// exponent than words[0] is split again for it.
-__device__ __forceinline__ bool terms_redone(uint32_t w0, uint32_t w1) {
-    const int e0 = (int)(w0 >> 23);
-    return (int)(w1 >> 23) > (e0 < 1 ? 1 : e0);
+// g of a tensor that goes with the row scales of another: words hold biased exponents, of an element that is its own plus that of
+// its row's 2^-s; 0: no finite element but zeros.  words[0]: what g is first chosen for (the largest of a sample and kSampleRoom, or
+// the exact maximum), words[1]: the exact maximum, found while splitting.  words[0] lands in [2^14, 2^15); of the binade above it
+// fp16 rounds everything from 65520 up to infinity, so a tensor with a larger exact maximum is split again for it.
+constexpr uint32_t kWordBias = 512;
+__device__ __forceinline__ int word_g(uint32_t w) { return 141 - (w ? (int)w - (int)kWordBias : 1); }
+__device__ __forceinline__ bool terms_redone(uint32_t w0, uint32_t w1) { return w1 > w0; }
+__device__ __forceinline__ int terms_g(const uint32_t* words) { return word_g(max(__ldg(words), __ldg(words + 1))); }
+__device__ __forceinline__ uint32_t word_of(uint32_t amax_bits, int row_exp) {     // amax_bits: of a finite magnitude
+    return amax_bits ? (uint32_t)((int)max(amax_bits >> 23, 1u) + row_exp + (int)kWordBias) : 0u;
 }
-__device__ __forceinline__ int terms_exp(const uint32_t* words) {
-    const uint32_t w0 = __ldg(words), w1 = __ldg(words + 1);
-    return term_exp(terms_redone(w0, w1) ? w1 : w0);
-}
+__device__ __forceinline__ int exp_of(float pow) { return (int)(__float_as_uint(pow) >> 23) - 127; }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
 // Instruction descriptor, kind::f16: D = f32 (bits 4-5 = 1), A = B = f16 (bits 7-9, 10-12 = 0), A / B MN-major at bits
@@ -372,18 +380,43 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const uint32_t my_stage = staging + (uint32_t)q * 8192u;
         uint32_t n_local = 0, n_store = 0;
-        int pi = 0, at = -1;
-        float fa = 1.0f, fb = 1.0f;
+        int pi = 0, at = -1, g = 0;
+        // The row's 2^-s of an item, and the factors of its first 64 columns, lane = column (2^-s of the rows of B, or col_scale: no
+        // product has both), are fetched one item ahead, further columns 64 ahead: read where they are used, their latency was 15 to 25 %
+        // of products with short main loops.
+        auto row_bits = [&](const TcTile& P, const TcItem& t) {
+            const int row = (t.mt * CG + (int)rank) * BM + q * 32 + lane;
+            return P.a_inv && row < P.M ? __float_as_int(__ldg(P.a_inv + row)) : 0x3F800000;
+        };
+        auto columns = [&](const TcTile& P) { return P.b_inv ? P.b_inv : P.splits == 1 ? P.col_scale : nullptr; };
+        auto column = [&](const float* f, int c, int N) { return f && c < N ? __ldg(f + c) : 1.0f; };
+        TcItem t = {}, t_next = {};
+        int inv_bits = 0, inv_next = 0, pi_next = 0;
+        float col[2], col_next[2] = {1.0f, 1.0f};
+        auto ahead = [&](int item) {
+            if (item >= n_items) return;
+            t_next = tc_item(sp, tab.n, item, pi_next);
+            const TcTile& P = sp[pi_next];
+            const float* f = columns(P);
+            inv_next = row_bits(P, t_next);
+            col_next[0] = column(f, t_next.nt * P.BN + lane, P.N);
+            col_next[1] = column(f, t_next.nt * P.BN + 32 + lane, P.N);
+        };
+        ahead(unit);
         for (int item = unit; item < n_items; item += n_units, ++n_local) {
-            const TcItem t = tc_item(sp, tab.n, item, pi);
+            t = t_next; pi = pi_next; inv_bits = inv_next;
+            col[0] = col_next[0]; col[1] = col_next[1];
+            ahead(item + n_units);
             const TcTile& P = sp[pi];
-            if (pi != at) {                            // undo the powers of two of the split
-                fa = P.a_words ? pow2(-terms_exp(P.a_words)) : 1.0f;
-                fb = P.b_words ? pow2(-terms_exp(P.b_words)) : 1.0f;
+            const float* factors = columns(P);
+            if (pi != at) {
+                g = P.words ? terms_g(P.words) : 0;
                 at = pi;
             }
+            // undo the powers of two of the split: the row's and g in two halves, so that no step leaves fp32 unless the result does
+            const int e = max(-252, (inv_bits >> 23) - 127 - g), e1 = e >> 1;
+            const float r1 = pow2(e1), r2 = pow2(e - e1);
             const CUtensorMap* tmC = &tab.maps[3 * pi + 2];
-            const float* col_scale = P.splits == 1 ? P.col_scale : nullptr;
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
             const bool was = !abort_flag;
             if (!__all_sync(0xffffffffu, was)) break;
@@ -393,6 +426,11 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             const int ncols = min(P.BN, P.N - n0), M = P.M;
             for (int c0 = 0; c0 < ncols; c0 += 64) {
                 uint32_t r[2][32];
+                float col_later[2] = {1.0f, 1.0f};
+                if (c0 + 64 < ncols) {
+                    col_later[0] = column(factors, n0 + c0 + 64 + lane, P.N);
+                    col_later[1] = column(factors, n0 + c0 + 96 + lane, P.N);
+                }
                 const uint32_t t_addr = tmem_base + acc * acc_cols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
                 tmem_ld32(t_addr, r[0]);
                 if (c0 + 32 < ncols) tmem_ld32(t_addr + 32, r[1]);
@@ -427,17 +465,18 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");     // the store before last has read this buffer
                     __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float4 o = make_float4(__uint_as_float(r[h][4 * j]), __uint_as_float(r[h][4 * j + 1]),
-                                               __uint_as_float(r[h][4 * j + 2]), __uint_as_float(r[h][4 * j + 3]));
-                        o.x = o.x * fa * fb; o.y = o.y * fa * fb; o.z = o.z * fa * fb; o.w = o.w * fa * fb;
-                        if (col_scale && cc + 4 * j < ncols) {        // N % 4 == 0
-                            const float4 sc = __ldg(reinterpret_cast<const float4*>(col_scale + n0 + cc + 4 * j));
-                            o.x *= sc.x; o.y *= sc.y; o.z *= sc.z; o.w *= sc.w;
-                        }
-                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(buf + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) << 4)), "f"(o.x), "f"(o.y), "f"(o.z), "f"(o.w) : "memory");
+                    for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) * r1);
+                    if (factors) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) * __shfl_sync(0xffffffffu, col[h], j));
                     }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) * r2);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(buf + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) << 4)), "r"(r[h][4 * j]), "r"(r[h][4 * j + 1]),
+                                       "r"(r[h][4 * j + 2]), "r"(r[h][4 * j + 3]) : "memory");
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
@@ -446,6 +485,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
+                col[0] = col_later[0]; col[1] = col_later[1];
             }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -484,7 +524,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, float* _
     }
 }
 
-// ---- pre-pass 1: the magnitude that a tensor's terms are scaled for ---------------------------------------------
+// ---- pre-pass 1: a magnitude for the tensors that complete another's row scales ---------------------------------
 // Reading a whole tensor for its maximum costs half of what splitting it does (25 us of 67 us for 16384 x 2048), so the choice is
 // made from a sample: the largest of up to 16384 elements spread over rows and columns, raised by 2^kSampleRoom.  The split itself sees every
 // element and records the exact maximum; a third launch, empty unless some tensor is larger than fp16 holds, splits those
@@ -497,178 +537,318 @@ struct SplitTensor {
     const float* col_scale;        // of planes_s
     __half* planes;                // terms [2][R][ld] of src, or null
     __half* planes_s;              // terms of src . col_scale, or null
-    uint32_t* words;               // {magnitude, exact maximum} of src, then of src . col_scale
+    float* row_inv;                // 2^-s of the rows of planes; null: planes are scaled by 2^(g - s_t) of comp and words
+    float* row_inv_s;              // of the rows of planes_s
+    const float* comp;             // 2^-s_t of the partner's rows, or null
+    uint32_t* words;
     int R, Cc, ld, vec;            // vec: rows of src and col_scale start on 16-byte boundaries
+    int rows_per_chunk;            // whole rows, at most SplitShape::kUnits units; 0: a row is larger
+    uint32_t magic;                // ceil(2^32 / units per row); 0: one
 };
 struct SplitGroup {
     int n;
-    long long chunk_begin[kSplitCap + 1];      // chunks of kSplitChunk units of 8 columns
+    int chunk_begin[kSplitCap + 1];
     SplitTensor t[kSplitCap];
 };
-constexpr int kSplitChunk = 2048;
+constexpr int kSplitRows = 256;                     // rows per chunk at most
+// NT threads per block: units of 8 columns per thread and chunk, chunks in shared memory (0: loaded to registers), blocks per SM
+template <int NT> struct SplitShape;
+template <> struct SplitShape<256> { static constexpr int kPer = 2, kUnits = 512, kStages = 2, kBlocks = 5, kSmem = 2 * 512 * 32; };
+template <> struct SplitShape<1024> { static constexpr int kPer = 4, kUnits = 4096, kStages = 0, kBlocks = 1, kSmem = 0; };
+
+__device__ __forceinline__ uint32_t finite_bits(float v) {
+    const uint32_t b = __float_as_uint(v) & 0x7FFFFFFFu;
+    return b < 0x7F800000u ? b : 0u;
+}
 
 __global__ void __launch_bounds__(512) sample_magnitude_kernel(const __grid_constant__ SplitGroup g) {
     const SplitTensor& T = g.t[blockIdx.x];
+    if (!T.words) return;
     const long long total = (long long)T.R * T.Cc;
     const long long units = total >> 2, step = units > kSampleUnits ? units / kSampleUnits : 1;       // units of 4 consecutive elements
-    float m0 = 0.0f, m1 = 0.0f;
-    auto add = [&](float v, float s) { m0 = fmaxf(m0, fabsf(v)); m1 = fmaxf(m1, fabsf(__fmul_rn(v, s))); };
+    uint32_t m = 0;
+    auto row_exp = [&](long long r) { return T.comp ? exp_of(__ldg(T.comp + r)) : 0; };
     const long long used = step > 1 ? min(units / step, 2ll * kSampleUnits) : units;        // (u + 1) * step <= units; at most 8191 where step is 1
     // a thread's loads all at once (taken two at a time, and with four divisions per unit, the launch took 19 us for 84 tensors)
     if (T.vec && used * step * 4 < 0x7fffffffll) {               // a unit lies in one row
         const int n = (int)used;
         for (int u0 = threadIdx.x; u0 < n; u0 += 8 * 512) {
-            float4 v[8], s[8];
+            float4 v[8];
+            int x[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 const int e = 4 * (int)sample_unit(min(u0 + k * 512, n - 1), step);
                 v[k] = __ldg(reinterpret_cast<const float4*>(T.src + e));
-                s[k] = T.planes_s ? __ldg(reinterpret_cast<const float4*>(T.col_scale + (uint32_t)e % (uint32_t)T.Cc)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[k] = row_exp((uint32_t)e / (uint32_t)T.Cc);
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) { add(v[k].x, s[k].x); add(v[k].y, s[k].y); add(v[k].z, s[k].z); add(v[k].w, s[k].w); }
+            for (int k = 0; k < 8; ++k)
+                m = max(m, word_of(max(max(finite_bits(v[k].x), finite_bits(v[k].y)), max(finite_bits(v[k].z), finite_bits(v[k].w))), x[k]));
         }
     } else {
         for (long long u = threadIdx.x; u < used; u += 512)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const long long e = sample_unit(u, step) * 4 + k;
-                add(__ldg(T.src + e), T.planes_s ? __ldg(T.col_scale + (int)(e % T.Cc)) : 0.0f);
+                m = max(m, word_of(finite_bits(__ldg(T.src + e)), row_exp(e / T.Cc)));
             }
     }
-    for (long long e = (units << 2) + threadIdx.x; e < total; e += 512) add(__ldg(T.src + e), T.planes_s ? __ldg(T.col_scale + (int)(e % T.Cc)) : 0.0f);
-    const uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
-    __shared__ uint32_t w0[16], w1[16];
-    if ((threadIdx.x & 31) == 0) { w0[threadIdx.x >> 5] = b0; w1[threadIdx.x >> 5] = b1; }
+    for (long long e = (units << 2) + threadIdx.x; e < total; e += 512) m = max(m, word_of(finite_bits(__ldg(T.src + e)), row_exp(e / T.Cc)));
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ uint32_t w0[16];
+    if ((threadIdx.x & 31) == 0) w0[threadIdx.x >> 5] = m;
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t a = 0, b = 0;
-        for (int w = 0; w < 16; ++w) { a = max(a, w0[w]); b = max(b, w1[w]); }
-        const uint32_t room = step > 1 ? (uint32_t)kSampleRoom << 23 : 0u;
-        T.words[0] = a && a < 0x7b000000u ? a + room : a; T.words[1] = 0u;
-        T.words[2] = b && b < 0x7b000000u ? b + room : b; T.words[3] = 0u;
+        uint32_t a = 0;
+        for (int w = 0; w < 16; ++w) a = max(a, w0[w]);
+        T.words[0] = a && step > 1 ? a + kSampleRoom : a;
+        T.words[1] = 0u;
     }
 }
 
-// ---- pre-pass 2: fp32 [R, Cc] -> fp16 terms, and the exact maxima ------------------------------------------------
-// Thread = 8 consecutive columns: two 128-bit loads, one 128-bit store per term.  HBM-bound: 4 bytes read, 4 written per
-// element and output.  All tensors of a step in one launch; FIX: only those whose first choice did not hold.
-__device__ __forceinline__ void split_terms8(const float (&v)[8], float f, uint4* hi, uint4* lo) {
+// ---- pre-pass 2: fp32 [R, Cc] -> fp16 terms, the rows' scales and the exact maxima -------------------------------
+// HBM-bound: 4 bytes read, 4 written per element and output.  A block takes chunks of whole rows, units of 8 columns (one
+// 128-bit store per term and unit) that stay in registers between the rows' maxima, found through shared memory, and
+// the split.  All tensors of a step in one launch; FIX: only those whose first g did not hold.
+//   256 threads, rows up to 4096 columns: the chunk is one contiguous piece of memory that cp.async brings one chunk ahead, five
+//       blocks per SM.  42 layers at 8192 tokens: X 160 us at 5.8 TB/s, dY and dY . scale 308 at 5.5 (issue slots 70 % busy).  Larger
+//       chunks or three of them in flight with fewer blocks: 1 to 8 % of the step slower; chunks half as large 8 %.
+//   1024 threads, rows up to 32768 columns: a chunk is loaded straight to the registers of a block that fills the SM.  4096 rows of 32000:
+//       163 us at 6.1 TB/s; with the row read twice, the second time from L2, 235 (five blocks per SM: half of it came from
+//       memory again) to 263.
+// Still wider rows are read twice.
+// eight scaled values as terms; lo of an infinity is NaN
+__device__ __forceinline__ void split_terms8(const float (&a)[8], uint4* __restrict__ hi, uint4* __restrict__ lo) {
     uint32_t h[4], l[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float a = v[2 * k] * f, b = v[2 * k + 1] * f;
-        const __half2 hh = __floats2half2_rn(a, b);
+        const __half2 hh = __floats2half2_rn(a[2 * k], a[2 * k + 1]);
         const float2 back = __half22float2(hh);
-        const __half2 ll = __floats2half2_rn((a - back.x) * (float)(1 << kLoShift), (b - back.y) * (float)(1 << kLoShift));
+        const __half2 ll = __floats2half2_rn((a[2 * k] - back.x) * (float)(1 << kLoShift), (a[2 * k + 1] - back.y) * (float)(1 << kLoShift));
         h[k] = *reinterpret_cast<const uint32_t*>(&hh);
         l[k] = *reinterpret_cast<const uint32_t*>(&ll);
     }
     *hi = make_uint4(h[0], h[1], h[2], h[3]);
     *lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
-template <bool FIX>
-__global__ void __launch_bounds__(256) split_terms_kernel(const __grid_constant__ SplitGroup g) {
+__device__ __forceinline__ uint32_t max_bits8(const float (&v)[8]) {       // of the largest finite magnitude
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))),
+                          fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
+    uint32_t b = __float_as_uint(m);           // NaN only where all are
+    if (b >= 0x7F800000u) {
+        b = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) b = max(b, finite_bits(v[q]));
+    }
+    return b;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void load8(const float* src, int left, bool vec, float (&v)[8]) {
+    if (vec && left >= 8) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = q < left ? __ldg(src + q) : 0.0f;
+    }
+}
+__device__ __forceinline__ int tensor_of_chunk(const SplitGroup& g, int from, int ch) {
+    while (ch >= g.chunk_begin[from + 1]) ++from;
+    return from;
+}
+// ROWS: every tensor has planes scaled by row and no others
+template <bool FIX, bool ROWS, int NT>
+__global__ void __launch_bounds__(NT, SplitShape<NT>::kBlocks) split_terms_kernel(const __grid_constant__ SplitGroup g) {
+    constexpr int kPer = SplitShape<NT>::kPer, kUnits = SplitShape<NT>::kUnits, kStages = SplitShape<NT>::kStages;
+    auto redo = [&](int t) { return g.t[t].words && terms_redone(__ldg(g.t[t].words), __ldg(g.t[t].words + 1)); };
     if (FIX) {
         const int t = threadIdx.x;              // kSplitCap <= 256
-        const bool redo = t < g.n && ((g.t[t].planes && terms_redone(__ldg(g.t[t].words), __ldg(g.t[t].words + 1))) ||
-                                      (g.t[t].planes_s && terms_redone(__ldg(g.t[t].words + 2), __ldg(g.t[t].words + 3))));
-        if (!__syncthreads_or(redo)) return;
+        if (!__syncthreads_or(t < g.n && redo(t))) return;
     }
-    const long long total = g.chunk_begin[g.n];
-    int ti = -1;
-    long long first = 0, last = 0;             // chunks of tensor ti
-    bool do0 = false, do1 = false;
-    float f0 = 0.0f, f1 = 0.0f, m0 = 0.0f, m1 = 0.0f;
-    __shared__ uint32_t red[2];
-    if (threadIdx.x < 2) red[threadIdx.x] = 0u;
+    // maxima of a chunk's rows, of src and of src . col_scale.  Three sets in turn: the one of chunk i + 2 is cleared between the
+    // barriers of chunks i and i + 1, when all have read chunk i - 1's and none writes chunk i + 2's.
+    extern __shared__ __align__(16) float ring[];      // [kStages][kUnits * 8]
+    __shared__ uint32_t row_max[3][2][kSplitRows];
+    for (int i = threadIdx.x; i < 3 * 2 * kSplitRows; i += NT) (&row_max[0][0][0])[i] = 0u;
     __syncthreads();
-    auto flush = [&]() {                       // the maxima of this block's share of tensor ti
-        if (FIX || ti < 0) return;
-        const uint32_t b0 = __reduce_max_sync(0xffffffffu, __float_as_uint(m0)), b1 = __reduce_max_sync(0xffffffffu, __float_as_uint(m1));
-        if ((threadIdx.x & 31) == 0) { atomicMax(&red[0], b0); atomicMax(&red[1], b1); }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (red[0]) atomicMax(g.t[ti].words + 1, red[0]);
-            if (red[1]) atomicMax(g.t[ti].words + 3, red[1]);
-            red[0] = red[1] = 0u;
+    const int total = g.chunk_begin[g.n], tid = threadIdx.x, lane = tid & 31;
+    int pch = blockIdx.x, pti = 0, pslot = 0, slot = 0;    // next chunk to fetch, its tensor and slot; slot of the current chunk
+    auto fetch = [&]() {                       // one group per chunk, empty where a chunk is read directly
+        if (pch < total) {
+            pti = tensor_of_chunk(g, pti, pch);
+            const SplitTensor& T = g.t[pti];
+            if (T.vec && T.rows_per_chunk && (!FIX || redo(pti))) {
+                const int r0 = (pch - g.chunk_begin[pti]) * T.rows_per_chunk, n4 = min(T.rows_per_chunk, T.R - r0) * (T.Cc >> 2);
+                const float4* src = reinterpret_cast<const float4*>(T.src + (size_t)r0 * T.Cc) + tid;
+                const uint32_t dst = smem_u32(ring + pslot * (kUnits * 8)) + 16u * tid;
+#pragma unroll
+                for (int k = 0; k < 2 * kPer; ++k)
+                    if (tid + NT * k < n4) cp_async16(dst + 16u * NT * k, src + NT * k);
+            }
+            pch += gridDim.x;
         }
-        __syncthreads();
-        m0 = m1 = 0.0f;
+        pslot = pslot == kStages - 1 ? 0 : pslot + 1;
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    for (long long ch = blockIdx.x; ch < total; ch += gridDim.x) {
+    for (int i = 0; i < kStages - 1; ++i) fetch();
+    int ti = -1, first = 0, last = 0, set = 0;         // chunks of tensor ti
+    bool skip = false;
+    uint32_t chosen = 0, word = 0;             // the word that g was first chosen for; the largest of this thread's share of the tensor
+    int gexp = 0;
+    auto flush = [&]() {                       // only what is above counts
+        if (ROWS || FIX || !__any_sync(0xffffffffu, word > chosen)) return;
+        const uint32_t b = __reduce_max_sync(0xffffffffu, word);
+        if (lane == 0) atomicMax(g.t[ti].words + 1, b);
+    };
+    for (int ch = blockIdx.x; ch < total; ch += gridDim.x) {
         if (ch >= last) {
             flush();
-            int lo = ti < 0 ? 0 : ti, hi = g.n - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (g.chunk_begin[mid] <= ch) lo = mid; else hi = mid - 1;
-            }
-            ti = lo; first = g.chunk_begin[ti]; last = g.chunk_begin[ti + 1];
-            const SplitTensor& T = g.t[ti];
-            do0 = T.planes != nullptr; do1 = T.planes_s != nullptr;
-            if (FIX) {
-                do0 = do0 && terms_redone(__ldg(T.words), __ldg(T.words + 1));
-                do1 = do1 && terms_redone(__ldg(T.words + 2), __ldg(T.words + 3));
-                f0 = do0 ? pow2(term_exp(__ldg(T.words + 1))) : 0.0f;
-                f1 = do1 ? pow2(term_exp(__ldg(T.words + 3))) : 0.0f;
-            } else {
-                f0 = do0 ? pow2(term_exp(__ldg(T.words))) : 0.0f;
-                f1 = do1 ? pow2(term_exp(__ldg(T.words + 2))) : 0.0f;
+            ti = tensor_of_chunk(g, ti < 0 ? 0 : ti, ch);
+            first = g.chunk_begin[ti]; last = g.chunk_begin[ti + 1];
+            skip = FIX && !redo(ti);
+            chosen = word = 0;
+            if (!ROWS && g.t[ti].words) {
+                word = chosen = __ldg(g.t[ti].words + (FIX ? 1 : 0));
+                gexp = word_g(chosen);
             }
         }
-        if (FIX && !do0 && !do1) {              // on to the first chunk of this block beyond the tensor
-            ch += (last - 1 - ch) / gridDim.x * gridDim.x;
-            continue;
+        if (kStages) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kStages ? kStages - 2 : 0) : "memory");
+            __syncthreads();                   // this chunk has landed for all; the slot before it has been read by all
+            fetch();
         }
+        const float* landed = ring + slot * (kUnits * 8);
+        slot = slot == kStages - 1 ? 0 : slot + 1;
+        if (skip) continue;
         const SplitTensor& T = g.t[ti];
-        const int n8 = (T.Cc + 7) >> 3, Cc = T.Cc, ld = T.ld;
-        const size_t units = (size_t)T.R * n8, ps = (size_t)T.R * ld;
-        size_t u = (size_t)(ch - first) * kSplitChunk + threadIdx.x;
-        size_t r = u / (size_t)n8;
-        int c8 = (int)(u - r * n8);
-#pragma unroll 2
-        for (int k = 0; k < kSplitChunk / 256 && u < units; ++k, u += 256) {
-            const int c = c8 * 8;
-            const float* src = T.src + r * Cc + c;
-            float v[8];
-            if (T.vec && c + 8 <= Cc) {
-                const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
-                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-            } else {
+        const int n8 = (T.Cc + 7) >> 3, Cc = T.Cc;
+        const bool plain = ROWS || T.planes != nullptr, by_row = ROWS || T.row_inv != nullptr, scaled = !ROWS && !FIX && T.planes_s != nullptr;
+        const bool maxima = (plain && by_row) || scaled;       // FIX: a tensor that is not scaled by row
+        uint32_t (&rm)[2][kSplitRows] = row_max[set];
+        const int r0 = T.rows_per_chunk ? (ch - first) * T.rows_per_chunk : ch - first;
+        const size_t at0 = (size_t)r0 * n8, ps = (size_t)T.R * n8;       // in units: ld = 8 n8
+        uint4* const p0 = reinterpret_cast<uint4*>(T.planes) + at0;
+        uint4* const p1 = reinterpret_cast<uint4*>(T.planes_s) + at0;
+        auto times_scale = [&](const float (&v)[8], int c, float (&a)[8]) {
+            load8(T.col_scale + c, Cc - c, T.vec, a);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) v[q] = c + q < Cc ? __ldg(src + q) : 0.0f;
-            }
-            uint4 hi, lo;
-            const size_t at = r * ld + c;                       // ld % 8 == 0
-            if (do0) {
-                if (!FIX) {
+            for (int q = 0; q < 8; ++q) a[q] = __fmul_rn(v[q], a[q]);
+        };
+        // scale, split and store unit u of the chunk: columns [c, c + 8) of row r0 + r, whose maxima are m0 and m1
+        auto store = [&](const float (&v)[8], int u, int r, int c, uint32_t m0, uint32_t m1) {
+            float a[8];
+            if (plain) {
+                if (by_row) {
+                    const int s = term_exp(m0);
+                    const float f = pow2(s);
+                    if (c == 0) T.row_inv[r0 + r] = pow2(-s);
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) m0 = fmaxf(m0, fabsf(v[q]));
-                }
-                split_terms8(v, f0, &hi, &lo);
-                *reinterpret_cast<uint4*>(T.planes + at) = hi;
-                *reinterpret_cast<uint4*>(T.planes + ps + at) = lo;
-            }
-            if (do1) {
-                float sc[8];
-                if (T.vec && c + 8 <= Cc) {
-                    const float4 a = __ldg(reinterpret_cast<const float4*>(T.col_scale + c)), b = __ldg(reinterpret_cast<const float4*>(T.col_scale + c) + 1);
-                    sc[0] = a.x; sc[1] = a.y; sc[2] = a.z; sc[3] = a.w; sc[4] = b.x; sc[5] = b.y; sc[6] = b.z; sc[7] = b.w;
+                    for (int q = 0; q < 8; ++q) a[q] = v[q] * f;
                 } else {
+                    const int x = T.comp ? exp_of(__ldg(T.comp + r0 + r)) : 0;
+                    // a row with finite elements other than zeros needs no more than 2^164, and below 2^-252 nothing is left of it
+                    const int e = max(-252, min(252, gexp + x)), e0 = e >> 1;
+                    const float f0 = pow2(e0), f1 = pow2(e - e0);
+                    if (!FIX) word = max(word, word_of(max_bits8(v), x));
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) sc[q] = c + q < Cc ? __ldg(T.col_scale + c + q) : 0.0f;
+                    for (int q = 0; q < 8; ++q) a[q] = v[q] * f0 * f1;
                 }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    v[q] = __fmul_rn(v[q], sc[q]);
-                    if (!FIX) m1 = fmaxf(m1, fabsf(v[q]));
-                }
-                split_terms8(v, f1, &hi, &lo);
-                *reinterpret_cast<uint4*>(T.planes_s + at) = hi;
-                *reinterpret_cast<uint4*>(T.planes_s + ps + at) = lo;
+                split_terms8(a, p0 + u, p0 + ps + u);
             }
-            for (c8 += 256; c8 >= n8; c8 -= n8) ++r;            // 256 units further
+            if (scaled) {
+                const int s = term_exp(m1);
+                const float f = pow2(s);
+                if (c == 0) T.row_inv_s[r0 + r] = pow2(-s);
+                times_scale(v, c, a);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) a[q] *= f;
+                split_terms8(a, p1 + u, p1 + ps + u);
+            }
+        };
+        auto unit_maxima = [&](const float (&v)[8], int c, uint32_t* m0, uint32_t* m1) {
+            *m0 = *m1 = 0u;
+            if (plain && by_row) *m0 = max_bits8(v);
+            if (scaled) { float a[8]; times_scale(v, c, a); *m1 = max_bits8(a); }
+        };
+        if (T.rows_per_chunk) {
+            const int units = min(T.rows_per_chunk, T.R - r0) * n8;
+            float v[kPer][8];
+            int rl[kPer];                 // row in the chunk
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const int u = tid + NT * k, uc = min(u, units - 1);
+                rl[k] = T.magic ? (int)__umulhi((uint32_t)uc, T.magic) : uc;       // uc n8 < 2^32: exact
+                const int c = 8 * (uc - rl[k] * n8);
+                if (kStages && T.vec) {
+                    const float4* p = reinterpret_cast<const float4*>(landed + rl[k] * Cc + c);
+                    const float4 a = p[0], b = c + 8 <= Cc ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f);      // Cc % 4 == 0
+                    v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w; v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+                } else {
+                    load8(T.src + (size_t)(r0 + rl[k]) * Cc + c, Cc - c, !kStages && T.vec, v[k]);
+                }
+            }
+            if (maxima) {
+#pragma unroll
+                for (int k = 0; k < kPer; ++k) {
+                    // the 32 units of a warp follow one another: mostly one row, or the end of one and the start of the next
+                    const int uc = min(tid + NT * k, units - 1);
+                    uint32_t m0, m1;
+                    unit_maxima(v[k], 8 * (uc - rl[k] * n8), &m0, &m1);
+                    const int ra = __shfl_sync(0xffffffffu, rl[k], 0), rb = __shfl_sync(0xffffffffu, rl[k], 31);
+                    if (rb == ra) {
+                        if (plain && by_row) { const uint32_t w = __reduce_max_sync(0xffffffffu, m0); if (lane == 0) atomicMax(&rm[0][ra], w); }
+                        if (scaled) { const uint32_t w = __reduce_max_sync(0xffffffffu, m1); if (lane == 0) atomicMax(&rm[1][ra], w); }
+                    } else if (rb == ra + 1) {
+                        const bool in = rl[k] == ra;
+                        if (plain && by_row) {
+                            const uint32_t w = __reduce_max_sync(0xffffffffu, in ? m0 : 0u), x = __reduce_max_sync(0xffffffffu, in ? 0u : m0);
+                            if (lane < 2) atomicMax(&rm[0][ra + lane], lane ? x : w);
+                        }
+                        if (scaled) {
+                            const uint32_t w = __reduce_max_sync(0xffffffffu, in ? m1 : 0u), x = __reduce_max_sync(0xffffffffu, in ? 0u : m1);
+                            if (lane < 2) atomicMax(&rm[1][ra + lane], lane ? x : w);
+                        }
+                    } else {
+                        if (plain && by_row) atomicMax(&rm[0][rl[k]], m0);
+                        if (scaled) atomicMax(&rm[1][rl[k]], m1);
+                    }
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const int u = tid + NT * k;
+                if (u < units) store(v[k], u, rl[k], 8 * (u - rl[k] * n8), rm[0][rl[k]], rm[1][rl[k]]);
+            }
+        } else {
+            const float* src = T.src + (size_t)r0 * Cc;
+            if (maxima) {
+                uint32_t m0 = 0, m1 = 0;
+#pragma unroll 4
+                for (int u = tid; u < n8; u += NT) {
+                    float v[8];
+                    uint32_t a, b;
+                    load8(src + 8 * u, Cc - 8 * u, T.vec, v);
+                    unit_maxima(v, 8 * u, &a, &b);
+                    m0 = max(m0, a); m1 = max(m1, b);
+                }
+                m0 = __reduce_max_sync(0xffffffffu, m0); m1 = __reduce_max_sync(0xffffffffu, m1);
+                if (lane == 0) { atomicMax(&rm[0][0], m0); atomicMax(&rm[1][0], m1); }
+                __syncthreads();
+            }
+#pragma unroll 2
+            for (int u = tid; u < n8; u += NT) {
+                float v[8];
+                load8(src + 8 * u, Cc - 8 * u, T.vec, v);
+                store(v, u, 0, 8 * u, rm[0][0], rm[1][0]);
+            }
+        }
+        if (maxima) {
+            const int clear = set == 0 ? 2 : set - 1;
+            for (int i = tid; i < 2 * kSplitRows; i += NT) (&row_max[clear][0][0])[i] = 0u;
+            set = set == 2 ? 0 : set + 1;
         }
     }
     flush();
@@ -892,14 +1072,15 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
     for (int i = 0; i < n; ++i) {
         const TcProblem& q = probs[i];
         const TcOperand &a = q.a, &b = q.b;
-        if (a.planes != 2 || b.planes < 1 || b.planes > 2 || (q.N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
+        if (a.planes != 2 || (a.words && b.words) || b.planes < 1 || b.planes > 2 || (q.N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
         const int bn = q.plan.bn, b_rows = bn / CG;
         float* out = q.plan.splits > 1 ? q.splitk_ws : q.c;
         if (!make_map(&tab.maps[3 * i], a, BM) || !make_map(&tab.maps[3 * i + 1], b, b_rows) ||
             !make_out_map(&tab.maps[3 * i + 2], out, q.M, q.N, q.plan.splits)) return cudaErrorInvalidValue;
         TcTile& p = tab.p[i];
         p.col_scale = q.col_scale;
-        p.a_words = a.words; p.b_words = b.words;
+        p.a_inv = a.inv; p.b_inv = b.inv;
+        p.words = a.words ? a.words : b.words;
         p.M = q.M; p.N = q.N; p.K = q.K;
         p.BN = bn;
         p.b_bytes = (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
@@ -1011,34 +1192,59 @@ cudaError_t launch_splitk_reduce(const float* partial, float* c, const float* co
     return cudaGetLastError();
 }
 
+namespace {
+template <int NT>
+cudaError_t run_split(const SplitGroup& g, bool rows_only, bool sampled, int sm_count, cudaStream_t stream) {
+    using S = SplitShape<NT>;
+    const int chunks = g.chunk_begin[g.n], grid = chunks < sm_count * S::kBlocks ? chunks : sm_count * S::kBlocks;
+    if (rows_only) split_terms_kernel<false, true, NT><<<grid, NT, S::kSmem, stream>>>(g);
+    else split_terms_kernel<false, false, NT><<<grid, NT, S::kSmem, stream>>>(g);
+    if (sampled) split_terms_kernel<true, false, NT><<<grid, NT, S::kSmem, stream>>>(g);
+    return cudaGetLastError();
+}
+}  // namespace
+
+// Tensors of their own first, then those that complete the row scales of one of these.
 cudaError_t launch_split_terms(const SplitDesc* d, int n, int sm_count, cudaStream_t stream, int* launches) {
-    for (int done = 0; done < n;) {
-        SplitGroup g;
-        const int take = n - done < kSplitCap ? n - done : kSplitCap;
-        long long chunks = 0;
-        bool sampled = false;                  // a tensor sampled whole needs no second look
-        for (int j = 0; j < take; ++j) {
-            const SplitDesc& q = d[done + j];
-            SplitTensor& t = g.t[j];
-            t.src = q.src; t.col_scale = q.planes_s ? q.col_scale : nullptr;
-            t.planes = static_cast<__half*>(q.planes); t.planes_s = static_cast<__half*>(q.planes_s);
-            t.words = q.words; t.R = q.rows; t.Cc = q.cols; t.ld = q.ld;
-            t.vec = (q.cols & 3) == 0 && (reinterpret_cast<uintptr_t>(q.src) & 15) == 0 &&
-                    (t.col_scale == nullptr || (reinterpret_cast<uintptr_t>(t.col_scale) & 15) == 0);
-            g.chunk_begin[j] = chunks;
-            chunks += ((long long)q.rows * ((q.cols + 7) / 8) + kSplitChunk - 1) / kSplitChunk;
-            if ((long long)q.rows * q.cols / 4 >= 2 * kSampleUnits) sampled = true;
+    for (int dependent = 0; dependent < 2; ++dependent) {
+        for (int i = 0; i < n;) {
+            SplitGroup g;
+            g.n = 0;
+            bool words = false, rows_only = true, sampled = false, wide = false;     // a tensor sampled whole needs no second look
+            for (; i < n && g.n < kSplitCap; ++i) {
+                const SplitDesc& q = d[i];
+                if ((q.comp != nullptr) != (dependent == 1)) continue;
+                SplitTensor& t = g.t[g.n++];
+                t.src = q.src; t.col_scale = q.planes_s ? q.col_scale : nullptr;
+                t.planes = static_cast<__half*>(q.planes); t.planes_s = static_cast<__half*>(q.planes_s);
+                t.row_inv = q.row_inv; t.row_inv_s = q.row_inv_s; t.comp = q.comp;
+                t.words = q.planes && !q.row_inv ? q.words : nullptr;
+                t.R = q.rows; t.Cc = q.cols; t.ld = q.ld;
+                t.vec = (q.cols & 3) == 0 && (reinterpret_cast<uintptr_t>(q.src) & 15) == 0 &&
+                        (t.col_scale == nullptr || (reinterpret_cast<uintptr_t>(t.col_scale) & 15) == 0);
+                if ((q.cols + 7) / 8 > SplitShape<256>::kUnits) wide = true;
+                if (t.words) words = true;
+                if (!t.planes || !t.row_inv || t.planes_s) rows_only = false;
+                if (t.words && (long long)q.rows * q.cols / 4 >= 2 * kSampleUnits) sampled = true;
+            }
+            if (g.n == 0) continue;
+            const int units = wide ? SplitShape<1024>::kUnits : SplitShape<256>::kUnits;
+            long long chunks = 0;
+            for (int j = 0; j < g.n; ++j) {
+                SplitTensor& t = g.t[j];
+                const int n8 = (t.Cc + 7) / 8;
+                t.rows_per_chunk = n8 > units ? 0 : units / n8 < kSplitRows ? units / n8 : kSplitRows;
+                t.magic = n8 == 1 ? 0u : (uint32_t)((0x100000000ull + (uint32_t)n8 - 1) / (uint32_t)n8);
+                g.chunk_begin[j] = (int)chunks;
+                chunks += t.rows_per_chunk ? ((long long)t.R + t.rows_per_chunk - 1) / t.rows_per_chunk : t.R;
+                if (chunks > 0x3fffffff) return cudaErrorInvalidValue;
+            }
+            g.chunk_begin[g.n] = (int)chunks;
+            if (words) sample_magnitude_kernel<<<g.n, 512, 0, stream>>>(g);
+            const cudaError_t e = wide ? run_split<1024>(g, rows_only, sampled, sm_count, stream) : run_split<256>(g, rows_only, sampled, sm_count, stream);
+            if (e != cudaSuccess) return e;
+            *launches += 1 + (words ? 1 : 0) + (sampled ? 1 : 0);
         }
-        g.chunk_begin[take] = chunks;
-        g.n = take;
-        const int grid = (int)(chunks < (long long)sm_count * 8 ? chunks : (long long)sm_count * 8);
-        sample_magnitude_kernel<<<take, 512, 0, stream>>>(g);
-        split_terms_kernel<false><<<grid, 256, 0, stream>>>(g);
-        if (sampled) split_terms_kernel<true><<<grid < sm_count ? grid : sm_count, 256, 0, stream>>>(g);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        *launches += sampled ? 3 : 2;
-        done += take;
     }
     return cudaSuccess;
 }
