@@ -66,8 +66,9 @@ cudaError_t launch_simt_grad_w(const float* grad_out, const float* x, float* gra
 struct TcPlan { int pair, bn, splits, ktiles_per_split, together; size_t workspace_bytes; double cost; };
 TcPlan tc_plan(int M, int N, int K, int nterms, int sm_count, int depth_limit);
 TcPlan tc_plan_shared(int M, int N, int K, int nterms, int cg, int depth_limit, int min_items, bool together = false);
-// k-tiles of 64 per accumulator for fp32 x fp32 products: 3 x 4 instructions per k-tile add into it, each with a truncation
-// error of about 2.7e-9 relative (K = 4096: 2e-6)
+// k-tiles of 64 per accumulator for fp32 x fp32 products.  Each instruction that adds into an accumulator truncates it; the
+// error is about 2.7e-9 for each on terms of either sign (K = 4096: 2e-6) and half a last bit, 6e-8, for each of the leading
+// products where a sum grows in one direction (four per k-tile: 1.5e-5).
 constexpr int kGradDepthLimit = 64;
 constexpr size_t kTermPad = 1024;  // readable bytes after the last plane of a TcOperand
 struct TcOperand {             // fp16 planes [planes][rows][ld] of a row-major tensor with `cols` columns

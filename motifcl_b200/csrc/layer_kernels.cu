@@ -17,6 +17,8 @@
 // Every wait on an mbarrier is bounded; on time-out the error word is set and the results are invalid.
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "counter_codec.cuh"
 #include "counter_update_body.cuh"
 #include "kernels.h"
@@ -299,6 +301,7 @@ struct LayerUpdParams {
     UpdParams u;              // of the whole layer; rows_per_batch = rows of a CTA
 };
 constexpr int kDwK = 32;                      // tokens per k-tile: two MMA steps
+constexpr int kDwDepth = kGradDepthLimit * 64 / kDwK;      // k-tiles that one accumulator takes before it is added up in fp32
 constexpr int kDwChunk = kDwK * 128;          // bytes of 64 columns x 32 tokens
 constexpr int kDwATerm = 2 * kDwChunk;
 
@@ -361,7 +364,8 @@ __device__ __forceinline__ void update_rows_by_group(const UpdParams& p, const i
     }
 }
 
-template <bool WITH_Q, bool U16>
+// DEEP: slices of more than kDwDepth k-tiles.  A form of its own: with the segments in it the loop spills, which cost 2 to 9 %.
+template <bool WITH_Q, bool U16, bool DEEP>
 __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid_constant__ LayerUpdParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[2];
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
     const uint32_t tmem = tmem_slot;
     bool ok = true;
     int it = 0;                                   // k-tiles so far: stage = it & 1
+    const int nseg = DEEP ? (p.slice / kDwK + kDwDepth - 1) / kDwDepth : 1;
     for (int pass = 0; pass < p.np; ++pass) {
         const int n0 = pass * p.pw, nw = min(p.pw, I - n0), nwp = (nw + 15) & ~15, per = nwp >> 2;
         const uint32_t bterm = (uint32_t)((nwp + 63) / 64) * kDwChunk;
@@ -450,93 +455,101 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
             for (int j = 0; j < 4; ++j)
                 r.b[j] = b_tok[j] < left && b_off[j] >= 0 ? __ldg(reinterpret_cast<const float4*>(g + b_off[j])) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
-        Regs r0, r1;
-        if (nkt > 0) load(0, r0);
-        if (nkt > 1) load(1, r1);
-        auto step = [&](int kt, Regs& r) {
-            const uint32_t st = stage0 + (uint32_t)(it & 1) * (uint32_t)p.stage_bytes, sb = st + 3u * kDwATerm;
-            if (it >= 2 && ok) ok = mbar_wait(bar0 + 8u * (it & 1), ((uint32_t)(it >> 1) - 1u) & 1u, &abort_flag);
-            auto put = [&](uint32_t at, uint32_t term, float4 v) {     // four columns of one token, three terms
-                uint32_t u0[3], u1[3];
-                split3(v.x, v.y, u0); split3(v.z, v.w, u1);
+        for (int seg = 0; seg < nseg; ++seg) {
+            const int k0 = DEEP ? seg * kDwDepth : 0, k1 = DEEP ? min(nkt, k0 + kDwDepth) : nkt;
+            Regs r0, r1;
+            if (k0 < k1) load(k0, r0);
+            if (k0 + 1 < k1) load(k0 + 1, r1);
+            auto step = [&](int kt, Regs& r) {
+                const uint32_t st = stage0 + (uint32_t)(it & 1) * (uint32_t)p.stage_bytes, sb = st + 3u * kDwATerm;
+                if (it >= 2 && ok) ok = mbar_wait(bar0 + 8u * (it & 1), ((uint32_t)(it >> 1) - 1u) & 1u, &abort_flag);
+                auto put = [&](uint32_t at, uint32_t term, float4 v) {     // four columns of one token, three terms
+                    uint32_t u0[3], u1[3];
+                    split3(v.x, v.y, u0); split3(v.z, v.w, u1);
 #pragma unroll
-                for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * term, u0[t], u1[t]);
-            };
+                    for (int t = 0; t < 3; ++t) sts64(at + (uint32_t)t * term, u0[t], u1[t]);
+                };
 #pragma unroll
-            for (int j = 0; j < 2; ++j) put(st + a_at + 2048u * j, kDwATerm, r.a[j]);
+                for (int j = 0; j < 2; ++j) put(st + a_at + 2048u * j, kDwATerm, r.a[j]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (b_tok[j] < kDwK) put(sb + b_at[j], bterm, r.b[j]);
-            if (kt + 2 < nkt) load(kt + 2, r);
-            fence_proxy_async();
-            __syncthreads();
-            if (warp == 0) {
-                tc_fence_after();
-                if (elect_one()) {
-                    // terms: 0 = hi .. 2 = lo, smallest products first
-                    const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+                for (int j = 0; j < 4; ++j)
+                    if (b_tok[j] < kDwK) put(sb + b_at[j], bterm, r.b[j]);
+                if (kt + 2 < k1) load(kt + 2, r);
+                fence_proxy_async();
+                __syncthreads();
+                if (warp == 0) {
+                    tc_fence_after();
+                    if (elect_one()) {
+                        // terms: 0 = hi .. 2 = lo, smallest products first
+                        const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) {
-                        const uint64_t da = desc_mn(st + (uint32_t)pa[q] * kDwATerm, kDwChunk), db = desc_mn(sb + (uint32_t)pb[q] * bterm, kDwChunk);
+                        for (int q = 0; q < 6; ++q) {
+                            const uint64_t da = desc_mn(st + (uint32_t)pa[q] * kDwATerm, kDwChunk), db = desc_mn(sb + (uint32_t)pb[q] * bterm, kDwChunk);
 #pragma unroll
-                        for (int kk = 0; kk < kDwK / 16; ++kk)         // 16 tokens = 2048 bytes further
-                            umma_bf16(q == 5 ? tmem : tmem + cols, da + 128u * kk, db + 128u * kk, idesc_bf16(128, nwp, 1, 1),
-                                      (kt | kk) != 0 || (q > 0 && q < 5) ? 1u : 0u);
-                    }
-                    umma_commit(bar0 + 8u * (it & 1));
-                }
-                __syncwarp();
-            }
-            ++it;
-        };
-        for (int kt = 0; kt < nkt; kt += 2) {
-            step(kt, r0);
-            if (kt + 1 < nkt) step(kt + 1, r1);
-        }
-        if (it > 0 && ok) ok = mbar_wait(bar0 + 8u * ((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, &abort_flag);
-        tc_fence_after();
-        // sum over the cluster, 128 columns at a time; the exchange tile lies over the (finished) stages
-        for (int c0 = 0; c0 < nw; c0 += 128) {
-            const int q = warp & 3, cc = (warp >> 2) * 32, row = q * 32 + lane;
-            if (c0 + cc < nw && q * 32 < valid) {
-                uint32_t r[32], r1[32];
-                if (nkt > 0) {
-                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + cc), r);
-                    tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)(c0 + cc), r1);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = 0;
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    sts128u(stage0 + (uint32_t)row * 512u + (uint32_t)(((cc >> 2) + j) ^ (row & 7)) * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-            }
-            tc_fence_before();
-            cluster_sync_all();
-            for (int i = tid; i < my_rows * 32; i += kLThreads) {
-                const int r = i >> 5, c = i & 31, g = ((n0 + c0) >> 2) + c;
-                if (c0 + 4 * c < nw) {
-                    const int mr = my_row0 + r;
-                    const uint32_t at = stage0 + (uint32_t)mr * 512u + (uint32_t)(c ^ (mr & 7)) * 16u;
-                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (uint32_t k = 0; k < cs; k += 4) {             // four remote loads in flight
-                        float4 v[4];
-#pragma unroll
-                        for (uint32_t i4 = 0; i4 < 4; ++i4) v[i4] = ld_peer(at, k + i4);
-#pragma unroll
-                        for (uint32_t i4 = 0; i4 < 4; ++i4) {
-                            sum.x = __fadd_rn(sum.x, v[i4].x); sum.y = __fadd_rn(sum.y, v[i4].y);
-                            sum.z = __fadd_rn(sum.z, v[i4].z); sum.w = __fadd_rn(sum.w, v[i4].w);
+                            for (int kk = 0; kk < kDwK / 16; ++kk)         // 16 tokens = 2048 bytes further
+                                umma_bf16(q == 5 ? tmem : tmem + cols, da + 128u * kk, db + 128u * kk, idesc_bf16(128, nwp, 1, 1),
+                                          ((kt - k0) | kk) != 0 || (q > 0 && q < 5) ? 1u : 0u);
                         }
+                        umma_commit(bar0 + 8u * (it & 1));
                     }
-                    gw_s[r * gpr + (U16 ? swz4(g) : g)] = sum;
+                    __syncwarp();
                 }
+                ++it;
+            };
+            for (int kt = k0; kt < k1; kt += 2) {
+                step(kt, r0);
+                if (kt + 1 < k1) step(kt + 1, r1);
             }
-            cluster_sync_all();
+            if (it > 0 && ok) ok = mbar_wait(bar0 + 8u * ((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, &abort_flag);
             tc_fence_after();
+            // sum over the cluster, 128 columns at a time; the exchange tile lies over the (finished) stages
+            for (int c0 = 0; c0 < nw; c0 += 128) {
+                const int q = warp & 3, cc = (warp >> 2) * 32, row = q * 32 + lane;
+                if (c0 + cc < nw && q * 32 < valid) {
+                    uint32_t r[32], r1[32];
+                    if (k0 < k1) {
+                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + cc), r);
+                        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)(c0 + cc), r1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r1[j]));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = 0;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        sts128u(stage0 + (uint32_t)row * 512u + (uint32_t)(((cc >> 2) + j) ^ (row & 7)) * 16u, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                }
+                tc_fence_before();
+                cluster_sync_all();
+                for (int i = tid; i < my_rows * 32; i += kLThreads) {
+                    const int r = i >> 5, c = i & 31, g = ((n0 + c0) >> 2) + c;
+                    if (c0 + 4 * c < nw) {
+                        const int mr = my_row0 + r;
+                        const uint32_t at = stage0 + (uint32_t)mr * 512u + (uint32_t)(c ^ (mr & 7)) * 16u;
+                        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (uint32_t k = 0; k < cs; k += 4) {             // four remote loads in flight
+                            float4 v[4];
+#pragma unroll
+                            for (uint32_t i4 = 0; i4 < 4; ++i4) v[i4] = ld_peer(at, k + i4);
+#pragma unroll
+                            for (uint32_t i4 = 0; i4 < 4; ++i4) {
+                                sum.x = __fadd_rn(sum.x, v[i4].x); sum.y = __fadd_rn(sum.y, v[i4].y);
+                                sum.z = __fadd_rn(sum.z, v[i4].z); sum.w = __fadd_rn(sum.w, v[i4].w);
+                            }
+                        }
+                        float4& to = gw_s[r * gpr + (U16 ? swz4(g) : g)];
+                        if (DEEP && seg > 0) {
+                            sum.x = __fadd_rn(to.x, sum.x); sum.y = __fadd_rn(to.y, sum.y);
+                            sum.z = __fadd_rn(to.z, sum.z); sum.w = __fadd_rn(to.w, sum.w);
+                        }
+                        to = sum;
+                    }
+                }
+                cluster_sync_all();
+                tc_fence_after();
+            }
         }
     }
     if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
@@ -586,11 +599,6 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
     const int I = d.in_features, O = d.rows;
     const bool with_q = lr_scale != 0.0f;
     const bool u16 = I % 16 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 3) == 0;
-    auto kern = u16 ? (with_q ? layer_update_kernel<true, true> : layer_update_kernel<false, true>)
-                    : (with_q ? layer_update_kernel<true, false> : layer_update_kernel<false, false>);
-    const int slot = 20 + (u16 ? 2 : 0) + (with_q ? 1 : 0);
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), slot, max_smem);
-    if (e != cudaSuccess) return e;
     // Rows per cluster and CTAs per cluster: a CTA contracts its slice of the tokens (all columns, whatever the rows), then
     // moves its rows x columns through the exchange once.  More CTAs shorten the slices, fewer rows per cluster shorten the
     // exchange; all CTAs should be resident at once.  Times in cycles from the stamps of both phases.
@@ -604,6 +612,16 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
                                 ((double)np * kt * (400.0 + 5.0 * (m + pw)) + (double)m * I * 4 / 16.0 + np * ((pw + 127) / 128) * 1500.0 + 4000.0 + (double)(m / c) * I * 0.6);
             if (cost < best) { best = cost; mr = m; cs = c; }
         }
+    const int slice = ((tokens + cs - 1) / cs + kDwK - 1) / kDwK * kDwK;
+    const bool deep = slice > kDwDepth * kDwK;
+    const auto pick = [&](auto d) {
+        constexpr bool D = decltype(d)::value;
+        return u16 ? (with_q ? layer_update_kernel<true, true, D> : layer_update_kernel<false, true, D>)
+                   : (with_q ? layer_update_kernel<true, false, D> : layer_update_kernel<false, false, D>);
+    };
+    const auto kern = deep ? pick(std::true_type()) : pick(std::false_type());
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (deep ? 32 : 20) + (u16 ? 2 : 0) + (with_q ? 1 : 0), max_smem);
+    if (e != cudaSuccess) return e;
     {
         const int tiles = (O + mr - 1) / mr;
         LayerUpdParams p;
@@ -621,7 +639,7 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
         if (p.np > 16) return cudaErrorInvalidConfiguration;
         p.off_stage = (int)base;
         p.dy = dy; p.x = x; p.tokens = tokens; p.O = O;
-        p.slice = ((tokens + cs - 1) / cs + kDwK - 1) / kDwK * kDwK;
+        p.slice = slice;
         p.vec_dy = (O & 3) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
         const uint32_t upr = (uint32_t)(I / 16);
         p.magic = upr <= 1 ? 0u : (uint32_t)((0x100000000ull + upr - 1) / upr);

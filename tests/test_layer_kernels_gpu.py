@@ -64,3 +64,17 @@ def test_update_against_the_exact_path(ctx, N, I, O, lr_scale):
     (st, sc, v), (est, esc, ev) = res
     assert float((st != est).double().mean()) <= 2e-4          # a rounding that falls the other way for a last-bit gradient difference
     assert float((sc - esc).norm() / esc.norm()) < 1e-6 and float((v - ev).norm() / ev.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("N", [32768, 32800, 98304, 300000, 500000])
+def test_update_of_many_tokens(ctx, N):
+    """dW of a long sum that grows all the way: an accumulator truncates less than a last bit for each of the 256 instructions that add
+    leading products into it, and v (with rms_beta = 0 the mean square of a row of dW) shows twice that."""
+    I, O = 64, 40
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, dy = torch.rand(N, I, device="cuda", generator=g) + 0.5, torch.rand(N, O, device="cuda", generator=g) * 0.02 + 0.01
+    st, sc, v = torch.zeros(O * I // 4 * 3, dtype=torch.uint8, device="cuda"), torch.full((O,), 0.05, device="cuda"), torch.zeros(O, device="cuda")
+    ctx.counter_update_fused(st, sc, v, dy, x, None, 11, I, O, N, 3e-3, 0.0, 0.0, 1e-3, 99)
+    ctx.finish()
+    want = (dy.double().T @ x.double()).square().mean(dim=1)
+    assert float(((v.double() - want) / want).abs().max()) <= 2 * 256 * 2.0 ** -23
