@@ -398,6 +398,15 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
         MCL_TC(ctx, op, mcl::launch_splitk_reduce_group(part.data(), out.data(), elems.data(), splits.data(), (int)part.size(), ctx->sm_count, ctx->stream, &_n));
     return MCL_CUDA_OK;
 }
+// One product of a layer that the one-launch kernels can take: by them, unless the terms split once are faster and their workspace
+// can be had (it cannot grow in a recording or under live batches, and these kernels need none)
+bool layer_route(mcl_cuda_ctx* ctx, const char* op, const ProductLayer& l, size_t N, size_t K, size_t C) {
+    if (!layer_wanted(ctx, l.Nt, l.I, l.O)) return false;
+    if (!tc_wanted(ctx, l.Nt, N, K, l.y ? l.y : l.grad_x, l.y ? l.scale : nullptr) || mcl::layer_rows_pay(l.Nt, N, K, ctx->sm_count)) return true;
+    size_t bytes = 0;
+    void* wsp = nullptr;
+    return products_chunk(ctx, op, &l, 1, C, nullptr, &bytes) != MCL_CUDA_OK || ws_reserve(ctx, bytes, &wsp) != MCL_CUDA_OK;
+}
 // Layers go together while their terms fit kChunkBytes.
 constexpr size_t kChunkBytes = (size_t)6 << 30;
 int products_group(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, size_t n, size_t C) {
@@ -658,15 +667,13 @@ int mcl_cuda_counter_forward(mcl_cuda_ctx* ctx, const float* x, const uint8_t* s
     MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
     MCL_TRY(check_ptr(ctx, op, "y", y, 4));
     DeviceGuard guard(ctx->device);
-    if (layer_wanted(ctx, batch, in_features, out_features)) {
+    const ProductLayer l = {x, nullptr, state, nullptr, scale, y, nullptr, nullptr, in_features, out_features, batch};
+    if (layer_route(ctx, op, l, out_features, in_features, C)) {
         MCL_LAUNCH(ctx, op, mcl::launch_layer_rows(0, x, state, scale, y, (int)batch, (int)in_features, (int)out_features, (int)C,
                                                    ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream));
         return MCL_CUDA_OK;
     }
-    if (tc_wanted(ctx, batch, out_features, in_features, y, scale)) {
-        const ProductLayer l = {x, nullptr, state, nullptr, scale, y, nullptr, nullptr, in_features, out_features, batch};
-        return products_group(ctx, op, &l, 1, C);
-    }
+    if (tc_wanted(ctx, batch, out_features, in_features, y, scale)) return products_group(ctx, op, &l, 1, C);
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_forward(x, state, scale, y, (int)batch, (int)in_features,
                                                          (int)out_features, (int)C, ctx->stream));
     return MCL_CUDA_OK;
@@ -684,15 +691,13 @@ int mcl_cuda_counter_backward_input(mcl_cuda_ctx* ctx, const uint8_t* state, con
     MCL_TRY(check_ptr(ctx, op, "grad_out", grad_out, 4));
     MCL_TRY(check_ptr(ctx, op, "grad_x", grad_x, 4));
     DeviceGuard guard(ctx->device);
-    if (layer_wanted(ctx, batch, in_features, out_features)) {
+    const ProductLayer l = {nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, in_features, out_features, batch};
+    if (layer_route(ctx, op, l, in_features, out_features, C)) {
         MCL_LAUNCH(ctx, op, mcl::launch_layer_rows(1, grad_out, state, scale, grad_x, (int)batch, (int)in_features, (int)out_features, (int)C,
                                                    ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream));
         return MCL_CUDA_OK;
     }
-    if (tc_wanted(ctx, batch, in_features, out_features, grad_x)) {
-        const ProductLayer l = {nullptr, grad_out, state, nullptr, scale, nullptr, grad_x, nullptr, in_features, out_features, batch};
-        return products_group(ctx, op, &l, 1, C);
-    }
+    if (tc_wanted(ctx, batch, in_features, out_features, grad_x)) return products_group(ctx, op, &l, 1, C);
     MCL_LAUNCH(ctx, op, mcl::launch_simt_counter_backward_input(state, scale, grad_out, grad_x, (int)batch,
                                                                 (int)in_features, (int)out_features,
                                                                 (int)C, ctx->stream));
@@ -745,18 +750,6 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
     MCL_TRY(check_ptr(ctx, op, "state", state, 1));
     if (packed2_out && in_features % 16 != 0)
         return fail(ctx, MCL_CUDA_EINVAL, "counter update: packed2 output requires in_features % 16 == 0");
-    if (layer_wanted(ctx, batch, in_features, out_features) && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-        MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
-        MCL_TRY(check_ptr(ctx, op, "v", v, 4));
-        if (packed2_out) MCL_TRY(check_ptr(ctx, op, "packed2_out", packed2_out, 4));
-        DeviceGuard guard(ctx->device);
-        mcl::UpdateDesc d;
-        d.state = state; d.scale = scale; d.v = v; d.grad_w = nullptr; d.packed2 = packed2_out;
-        d.in_features = (int)in_features; d.rows = (int)out_features; d.row_offset = 0;
-        MCL_LAUNCH(ctx, op, mcl::launch_layer_update(d, grad_out, x, (int)batch, (int)C, lr, lr_scale, rms_beta, rms_eps, seed, ctx->seed_offset,
-                                                     ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
-        return MCL_CUDA_OK;
-    }
     // Row tile of grad_w: 1/8 of the dense [out,in] gradient, raised to 4 MiB where that is still under 1/5 of the
     // dense gradient (fewer launches for mid-sized layers) and capped at 32 MiB; at least one row; rounded to a multiple
     // of 128 rows when that fits.  The dense gradient is never materialised: the reference's memory-truth gate
@@ -787,6 +780,19 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
         o_k = cv.reserve(plan.workspace_bytes);
     }
     void* wsp = nullptr;
+    if (layer_wanted(ctx, batch, in_features, out_features) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+        (!tc || mcl::layer_update_pays(batch, in_features, out_features, (out_features + tile_rows - 1) / tile_rows, ctx->sm_count) ||
+         ws_reserve(ctx, cv.off, &wsp) != MCL_CUDA_OK)) {
+        MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
+        MCL_TRY(check_ptr(ctx, op, "v", v, 4));
+        if (packed2_out) MCL_TRY(check_ptr(ctx, op, "packed2_out", packed2_out, 4));
+        mcl::UpdateDesc d;
+        d.state = state; d.scale = scale; d.v = v; d.grad_w = nullptr; d.packed2 = packed2_out;
+        d.in_features = (int)in_features; d.rows = (int)out_features; d.row_offset = 0;
+        MCL_LAUNCH(ctx, op, mcl::launch_layer_update(d, grad_out, x, (int)batch, (int)C, lr, lr_scale, rms_beta, rms_eps, seed, ctx->seed_offset,
+                                                     ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
+        return MCL_CUDA_OK;
+    }
     MCL_TRY(ws_reserve(ctx, cv.off, &wsp));
     char* w = static_cast<char*>(wsp);
     float* gw = reinterpret_cast<float*>(w + o_gw);

@@ -34,6 +34,9 @@ cudaError_t launch_pack2(const uint8_t* state, uint32_t* packed2, int C, int in_
 
 // layer_kernels.cu -- one launch per product of a narrow layer, operands converted inside the kernel
 bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features);
+// rather these kernels than the split-once route of tc_gemm.cu: a product [tokens, N] over K; the update, whose other route takes `tiles` row tiles
+bool layer_rows_pay(size_t tokens, size_t N, size_t K, int sm_count);
+bool layer_update_pays(size_t tokens, size_t in_features, size_t out_features, size_t tiles, int sm_count);
 // dx = 0: c[tokens, O] = a (scale T)^T;  dx = 1: c[tokens, I] = (a . scale) T
 cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, const float* scale, float* c, int tokens, int I, int O,
                               int C, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream);

@@ -562,9 +562,62 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
 }  // namespace
 
 bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features) {
-    // A row kernel converts its activations once per column tile and the update converts x once per 128 output rows: beyond
-    // these widths the terms split once by tc_gemm.cu are cheaper.
     return in_features % 4 == 0 && in_features <= 1024 && out_features <= 2048 && tokens <= (1u << 20);
+}
+
+namespace {
+// column tile of the row kernels: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per column)
+double rows_cost(int tokens, int N, int K, int sm_count, int* bn_out) {
+    const int tm = (tokens + 127) / 128, nkt = (K + 63) / 64;
+    double best = 1e30;
+    for (int bn = 32; bn <= 256; bn += 32) {
+        const int tiles = tm * ((N + bn - 1) / bn);
+        const double cost = (double)((tiles + sm_count - 1) / sm_count) * (nkt * (900.0 + 5.0 * bn) + 4000.0 + 6.0 * bn);
+        if (cost < best) { best = cost; *bn_out = bn; }
+    }
+    return best;
+}
+// Rows per cluster and CTAs per cluster of the update: a CTA contracts its slice of the tokens (all columns, whatever the rows),
+// then moves its rows x columns through the exchange once.  More CTAs shorten the slices, fewer rows per cluster shorten the
+// exchange; all CTAs should be resident at once.  Times in cycles from the stamps of both phases.
+struct UpdateShape { int np, pw, mr, cs, ktiles; double exchange; };
+UpdateShape update_shape(int tokens, int I, int O, int sm_count) {
+    UpdateShape u = {(I + 255) / 256, 0, 128, 8, 0, 0.0};
+    u.pw = ((I + u.np - 1) / u.np + 63) / 64 * 64;
+    double best = 1e30;
+    for (int c = 4; c <= 8; c *= 2)            // clusters of 16 need two waves where eights need one: 288 x 288 at 256 rows 55 us, not 40
+        for (int m = 128; m >= 32; m /= 2) {
+            const int ctas = (O + m - 1) / m * c, kt = ((tokens + c - 1) / c + kDwK - 1) / kDwK;
+            const double exchange = (double)m * I * 4 / 16.0 + u.np * ((u.pw + 127) / 128) * 1500.0 + 4000.0 + (double)(m / c) * I * 0.6;
+            const double cost = (double)((ctas + sm_count - 1) / sm_count) * ((double)u.np * kt * (400.0 + 5.0 * (m + u.pw)) + exchange);
+            if (cost < best) { best = cost; u.mr = m; u.cs = c; u.ktiles = kt; u.exchange = exchange; }
+        }
+    return u;
+}
+}  // namespace
+
+// Which route a product of one layer takes, by its shape alone: the one-launch kernels, or terms split once (tc_gemm.cu), which need
+// activation-sized workspace and have to be a fifth faster to be worth that.  Models in us, fitted to 36 shapes of 64 to 2048
+// features at 32 to 262144 tokens (B200), within 10 % for nearly all.  One launch against split: 288 x 288 forward 27 / 30 us at
+// 16384 tokens, 92 / 79 at 65536, 346 / 256 at 262144 (the line: about 100000); 288 x 1536 17 / 22 at 2048, 48 / 38 at 8192 (6000);
+// 1024 x 1024 23 / 26 at 1024, 42 / 36 at 4096, 81 / 53 at 8192 (5000).
+namespace { bool worth_workspace(double layer, double split) { return layer > 1.2 * split + 2.0; } }
+bool layer_rows_pay(size_t tokens, size_t N, size_t K, int sm_count) {
+    int bn = 0;
+    const double layer = 1.8 + 1.864 / 1900.0 * rows_cost((int)tokens, (int)N, (int)K, sm_count, &bn);
+    const double bytes = (double)tokens * (12.0 * K + 4.0 * N), flops = 4.0 * tokens * N * K;
+    // split by the terms' kernels: launches, the pass over the digits, then memory or the tensor pipe
+    const double split = 13.8 + 0.0075 * K + 1.5e-6 * N * K + (bytes / 4.7e6 > flops / 1.1e9 ? bytes / 4.7e6 : flops / 1.1e9);
+    return !worth_workspace(layer, split);
+}
+// The same for the update, whose other route forms grad_w in `tiles` row tiles (288 x 768: 165 / 241 us at 16384 tokens, 610 / 406 at
+// 65536; 512 x 512: 121 / 179 at 4096, 386 / 240 at 16384).  Clusters of 8 fit the GPCs 15 at a time, of 4 about 34.
+bool layer_update_pays(size_t tokens, size_t I, size_t O, size_t tiles, int sm_count) {
+    const UpdateShape u = update_shape((int)tokens, (int)I, (int)O, sm_count);
+    const int clusters = ((int)O + u.mr - 1) / u.mr, fit = u.cs == 8 ? sm_count * 15 / 148 : sm_count * 34 / 148;
+    const double layer = 5.0 + (clusters + fit - 1) / fit * (u.np * u.ktiles * (0.85 + 0.002 * u.pw) + u.exchange / 1900.0);
+    const double split = 60.0 + 18.0 * tiles + (double)tokens * (8.0 * (I + O) + 4.0 * tiles * I + 4.0 * O) / 4.4e6;
+    return !worth_workspace(layer, split);
 }
 
 cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, const float* scale, float* c, int tokens, int I, int O,
@@ -574,14 +627,8 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
     p.M = tokens; p.N = dx ? I : O; p.K = dx ? O : I; p.in_features = I; p.C = C;
     p.vec = (p.K & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
     p.err = err_word;
-    // column tile: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per column)
+    rows_cost(tokens, p.N, p.K, sm_count, &p.BN);
     const int tm = (tokens + 127) / 128;
-    double best = 1e30;
-    for (int bn = 32; bn <= 256; bn += 32) {
-        const int tiles = tm * ((p.N + bn - 1) / bn), nkt = (p.K + 63) / 64;
-        const double cost = (double)((tiles + sm_count - 1) / sm_count) * (nkt * (900.0 + 5.0 * bn) + 4000.0 + 6.0 * bn);
-        if (cost < best) { best = cost; p.BN = bn; }
-    }
     p.stage_bytes = 3 * kRowATerm + (dx ? (p.BN + 63) / 64 * 8192 : p.BN * 128);
     const size_t smem = 2 * (size_t)p.stage_bytes + 1024;
     const void* kern = dx ? reinterpret_cast<const void*>(layer_rows_kernel<true>) : reinterpret_cast<const void*>(layer_rows_kernel<false>);
@@ -599,19 +646,8 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
     const int I = d.in_features, O = d.rows;
     const bool with_q = lr_scale != 0.0f;
     const bool u16 = I % 16 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 3) == 0;
-    // Rows per cluster and CTAs per cluster: a CTA contracts its slice of the tokens (all columns, whatever the rows), then
-    // moves its rows x columns through the exchange once.  More CTAs shorten the slices, fewer rows per cluster shorten the
-    // exchange; all CTAs should be resident at once.  Times in cycles from the stamps of both phases.
-    const int np = (I + 255) / 256, pw = ((I + np - 1) / np + 63) / 64 * 64;
-    int mr = 128, cs = 8;
-    double best = 1e30;
-    for (int c = 4; c <= 8; c *= 2)            // clusters of 16 need two waves where eights need one: 288 x 288 at 256 rows 55 us, not 40
-        for (int m = 128; m >= 32; m /= 2) {
-            const int ctas = (O + m - 1) / m * c, kt = ((tokens + c - 1) / c + kDwK - 1) / kDwK;
-            const double cost = (double)((ctas + sm_count - 1) / sm_count) *
-                                ((double)np * kt * (400.0 + 5.0 * (m + pw)) + (double)m * I * 4 / 16.0 + np * ((pw + 127) / 128) * 1500.0 + 4000.0 + (double)(m / c) * I * 0.6);
-            if (cost < best) { best = cost; mr = m; cs = c; }
-        }
+    const UpdateShape shape = update_shape(tokens, I, O, sm_count);
+    const int mr = shape.mr, cs = shape.cs;
     const int slice = ((tokens + cs - 1) / cs + kDwK - 1) / kDwK * kDwK;
     const bool deep = slice > kDwDepth * kDwK;
     const auto pick = [&](auto d) {
@@ -629,7 +665,7 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
         const int R = mr / cs;
         const size_t base = (u16_layout(I, R, with_q, kLThreads / 64).total + 1023) & ~size_t(1023);
         size_t smem = 0;
-        for (p.np = np; p.np <= 16; ++p.np) {
+        for (p.np = shape.np; p.np <= 16; ++p.np) {
             p.pw = ((I + p.np - 1) / p.np + 63) / 64 * 64;
             p.stage_bytes = 3 * kDwATerm + 3 * (p.pw / 64) * kDwChunk;
             const size_t area = 2 * (size_t)p.stage_bytes > 65536 ? 2 * (size_t)p.stage_bytes : 65536;

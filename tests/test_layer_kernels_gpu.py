@@ -78,3 +78,39 @@ def test_update_of_many_tokens(ctx, N):
     ctx.finish()
     want = (dy.double().T @ x.double()).square().mean(dim=1)
     assert float(((v.double() - want) / want).abs().max()) <= 2 * 256 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("N,I,O", [(40000, 288, 768), (40000, 768, 288), (8200, 1024, 1024), (5001, 1024, 1540), (70000, 288, 288), (33001, 512, 516)])
+def test_both_routes_of_a_layer(N, I, O):
+    """Token counts beyond those that the one-launch kernels take by themselves: split terms, or, where a recording keeps the workspace from
+    growing, the one-launch kernels all the same; both against float64."""
+    from motifcl_b200 import Context
+    st, sc, v, x, dy = _layer(N, I, O, N + I)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        ctx = Context.on_torch_stream(0)
+        w = torch.empty(O, I, device="cuda")
+        ctx.counter_decode_weight(st, torch.ones_like(sc), w, I, O, 11)
+        ctx.finish()
+        wy, wdx = (x.double() @ w.double().T) * sc.double(), (dy * sc).double() @ w.double()
+        wv = (dy.double().T @ x.double()).square().mean(dim=1)
+        for recorded in (True, False):
+            y, dx = torch.full((N, O), 7.0, device="cuda"), torch.full((N, I), 7.0, device="cuda")
+            s2, c2, v2 = st.clone(), sc.clone(), v.clone()
+            torch.cuda.synchronize()
+            if recorded:
+                ctx.batch_begin()
+            ctx.counter_forward(x, st, sc, y, N, I, O, 11)
+            ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+            ctx.counter_update_fused(s2, c2, v2, dy, x, None, 11, I, O, N, 3e-3, 0.0, 0.0, 1e-3, 99)
+            if recorded:
+                batch = ctx.batch_end()
+                batch.launch()
+            ctx.finish()
+            if recorded:
+                assert ctx.workspace_bytes == 0
+                batch.close()
+            assert float((y - wy).norm() / wy.norm()) < 1e-6 and float((dx - wdx).norm() / wdx.norm()) < 1e-6
+            assert float(((v2.double() - wv) / wv).abs().max()) <= 2 * 256 * 2.0 ** -23
+        ctx.close()
