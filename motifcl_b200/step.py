@@ -112,10 +112,11 @@ class CounterStack:
     def step(self, xs, dys, base_seed: int = 12345, recorded: bool = False):
         """xs[i]: [tokens, in_i], dys[i]: [tokens, out_i] device tensors.  One full step.
 
-        recorded=True (single GPU): the first call runs eagerly (sizing the workspace) and
-        records the same calls into one batch; later calls replay it -- one graph launch per
-        step, as the reference submits one command buffer per step.  The per-step seed then
-        comes from a device word that is bumped after every replay."""
+        recorded=True (single GPU): a first step on a set of tensors runs eagerly (and sizes the workspace), a second one in a
+        row on the same tensors is recorded into one batch and replayed, as all later ones are -- one graph launch per
+        step, as the reference submits one command buffer per step.  The per-step seed of a replay comes from a device word
+        that is bumped after it.  A program whose tensors are new at every step pays for no recording (1000 tokens, 42
+        linears, B200: 0.32 to 0.44 ms a step against 0.81 with a recording of each; 0.26 replayed)."""
         if self.world > 1:
             self._step_dp(xs, dys, (base_seed + self.step_index) & 0xFFFFFFFF)
             self.step_index += 1
@@ -128,28 +129,32 @@ class CounterStack:
     # -- single GPU --------------------------------------------------------------------------
     def _step_recorded(self, xs, dys, base_seed):
         key = (tuple(t.data_ptr() for t in xs), tuple(t.data_ptr() for t in dys), base_seed)
-        if self._batch is None or self._batch_key != key:
+        if self._batch_key != key:
             if self._batch is not None:
                 self._batch.close()
                 self._batch = None
+            self._step_eager(xs, dys, (base_seed + self.step_index) & 0xFFFFFFFF)
+            self._batch_key = key
+            self.step_index += 1
+            return
+        if self._batch is None:
             self._step_word.fill_(self.step_index)
             for lane in self.lanes:
                 lane.set_seed_offset(self._step_word)
             try:
-                self._step_eager(xs, dys, base_seed)          # this call's step; also sizes the workspace
-                self._step_word.add_(1)
-                self.step_index += 1
-                self.ctx.finish()
                 self.ctx.batch_begin()
                 try:
                     self._step_eager(xs, dys, base_seed)      # recorded, not run
                 finally:
                     self._batch = self.ctx.batch_end()
+            except Exception:
+                if self._batch is not None:
+                    self._batch.close()                       # of a part of the step
+                self._batch = self._batch_key = None
+                raise
             finally:
                 for lane in self.lanes:
                     lane.set_seed_offset(None)
-            self._batch_key = key
-            return
         self._batch.launch()
         self._step_word.add_(1)
         self.step_index += 1
@@ -165,9 +170,11 @@ class CounterStack:
     def _descs(self, xs, dys, update: bool, part: str = "all"):
         """part: "all" products, "dw" the weight gradients only, "rows" Y and dX only."""
         key = (tuple(t.data_ptr() for t in xs), tuple(t.data_ptr() for t in dys), update, part)
-        cache = self.__dict__.setdefault("_desc_cache", {})
+        cache = self.__dict__.setdefault("_desc_cache", {})       # the last eight: a program may have new tensors at every step
         if key not in cache:
             from .runtime import linear_descs
+            if len(cache) >= 8:
+                del cache[next(iter(cache))]
             cache[key] = linear_descs([
                 dict(x=x, grad_out=dy, state=None if self.world > 1 else l.state, scale=l.scale, v=l.v,
                      y=l.y if part != "dw" else None, grad_x=l.dx if part != "dw" else None,

@@ -561,6 +561,34 @@ def test_recorded_batch_replays_the_step_with_a_per_step_seed(ctx, orc):
     assert np.array_equal(lin.state.cpu().numpy(), o[0])
 
 
+@pytest.mark.parametrize("grouped", [False, True])
+def test_recorded_step_on_new_tensors_records_only_what_comes_again(ctx, grouped, monkeypatch):
+    """Steps on tensors that change: the same results as unrecorded steps, and a recording only for the second step in a row on the same
+    tensors (a recording costs as much as a short step)."""
+    from motifcl_b200 import Context
+    from motifcl_b200.step import CounterLinearState, CounterStack, Hyper
+    c = CASES["cfg1"]
+    N, I, O = c["N"], c["I"], c["O"]
+    sets = [(_t(c["x"]) * k, _t(c["dy"]) * k) for k in (1.0, 0.5, 2.0)]
+    order = [0, 1, 0, 2, 2, 2, 1, 1, 2, 2, 0] + [0] * 3
+    begun = []
+    real = Context.batch_begin
+    monkeypatch.setattr(Context, "batch_begin", lambda self: (begun.append(len(seen)), real(self))[1])
+    results = []
+    for recorded in (False, True):
+        lin = CounterLinearState(synth.LinearShape("l", O, I), c["state"], c["scale"], c["v"], torch.device(DEV))
+        stack = CounterStack(ctx, [lin], Hyper(lr=0.05), N, grouped=grouped)
+        seen = []
+        for k in order:
+            seen.append(k)
+            stack.step([sets[k][0]], [sets[k][1]], base_seed=100, recorded=recorded)
+        ctx.finish()
+        results.append([t.cpu().numpy() for t in (lin.state, lin.scale, lin.v, lin.packed2, lin.y, lin.dx, lin.grad_w)])
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
+    assert begun == [k + 1 for k in range(1, len(order)) if order[k] == order[k - 1] and (k == 1 or order[k - 2] != order[k])]
+
+
 @pytest.mark.parametrize("mode", ["tensor", "exact"])
 def test_products_from_packed2_equal_products_from_state(ctx, orc, mode):
     """What a data-parallel rank runs for layers whose state it does not own: Y, dX, dW from the
