@@ -173,7 +173,7 @@ int create_impl(int device, cudaStream_t stream, bool own, mcl_cuda_ctx** out_ct
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         cudaGetLastError();
     }
-    // [0] error word, [1] work-item counter
+    // [0] error word, [8] work items drawn and [9] CTAs done of the running contraction (tc_gemm.cu leaves both at zero)
     e = cudaMalloc(reinterpret_cast<void**>(&ctx->err_word), 16 * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->err_word, 0, 16 * sizeof(int));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
@@ -204,7 +204,7 @@ int check_device_error(mcl_cuda_ctx* ctx) {
             case 2: case 12: who = "MMA lane (operand tile never arrived)"; break;
             case 13: case 15: who = "epilogue / converter warps (accumulator or tile never completed)"; break;
             case 14: who = "MMA lane (accumulator never drained)"; break;
-            case 16: case 17: who = "work-item queue (scheduler lane and its readers lost step)"; break;
+            case 16: case 17: who = "work items (the drawing warp and its readers lost step)"; break;
             case 21: who = "wide-row counter update (a row slot was never marked ready or released)"; break;
             case 41: who = "single-layer kernel (a k-tile's MMAs never completed)"; break;
             case 31: who = "peer all-reduce (a rank never announced its partial result)"; break;

@@ -179,8 +179,12 @@ __device__ __forceinline__ TcItem tc_item(const TcTile* tab, int n, int item, in
     return t;
 }
 
-// Persistent CTAs of 192 threads; the work items of all products of the table (output tile x split-K slice) are dealt round-robin.
-//   warp 0        TMA producer (one elected lane): tiles of A and B into a ring of `stages` shared-memory slots
+// Persistent CTAs of 192 threads (pairs of them with CG = 2); the work items of all products of the table (output tile x split-K slice)
+// are drawn from a counter.  A CTA whose SM is taken by another kernel, a collective for instance, then costs its share and not a
+// second wave: Y and dX of 21 layers (8192 x 288 -> 768) beside a kernel that holds 16 SMs 786 us, dealt round-robin
+// 1055 (660 alone); of 16384 x 2048 -> 2048 517 and 743 (457).
+//   warp 0        TMA producer (one elected lane): tiles of A and B into a ring of `stages` shared-memory slots; the leader's draws the
+//                 items, one ahead of its copies, and hands them to all other warps through a ring of kDealt words
 //   warp 1        MMA issuer (one elected lane): four tcgen05.mma (K = 16 each) per slot; also allocates / frees TMEM
 //   warps 2..5    epilogue: tcgen05.ld of 32 lanes x 64 columns, scale, a swizzled 32 x 32 tile in shared memory, TMA store
 // Two accumulators live in TMEM (columns [0,BN) and [ACC,ACC+BN)), so the epilogue of one item
@@ -199,12 +203,50 @@ __device__ __forceinline__ TcItem tc_item(const TcTile* tab, int n, int item, in
 // Every mbarrier wait is bounded: on time-out the kernel records an error word, skips the rest of its work, frees
 // its TMEM and returns.
 constexpr int kTcThreads = 192;
+constexpr int kDealt = 4;                  // items between the draw and the epilogue's prefetch: one each in copies, MMAs, epilogue and ahead
+constexpr int kQueueWord = 8;              // of the context's words: items drawn, CTAs (pairs) that are done
 constexpr int kStageBytes = 8 * 4096;      // epilogue staging: two 32 x 32 float tiles per warp
+
+template <int CG>
+__device__ __forceinline__ bool deal_try(uint32_t bar, uint32_t parity) {      // the word may come from the other CTA of a pair
+    if (CG == 1) return mbar_try_wait(bar, parity);
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+template <int CG>
+__device__ __forceinline__ bool deal_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {      // whole warp, bounded
+    if (__all_sync(0xffffffffu, deal_try<CG>(bar, parity))) return true;
+    const unsigned long long t0 = clock64();
+    unsigned spins = 0;
+    while (!__all_sync(0xffffffffu, deal_try<CG>(bar, parity))) {
+        if ((++spins & 0x3FFu) == 0) {
+            const bool stop = *abort_flag || clock64() - t0 > kWaitCycles;
+            if (__any_sync(0xffffffffu, stop)) return false;
+        }
+    }
+    return true;
+}
+// The word has been read (the arrive takes it as an operand) and nothing was written: no release, which would wait for the warp's
+// stores and cost the row products of narrow layers 3 %.
+template <int CG>
+__device__ __forceinline__ void deal_return(uint32_t bar, int word) {
+    if (CG == 1) asm volatile("{\n\t.reg .b32 w;\n\tmov.b32 w, %1;\n\tmbarrier.arrive.relaxed.cta.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(word) : "memory");
+    else asm volatile("{\n\t.reg .b32 w;\n\tmov.b32 w, %1;\n\tmbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n\t}" ::"r"(cluster_addr(bar, 0)), "r"(word) : "memory");
+}
+// the word to the other CTA of the pair, counted by the barrier there
+__device__ __forceinline__ void deal_to_peer(uint32_t word_addr, uint32_t bar, int word) {
+    const uint32_t b = cluster_addr(bar, 1);
+    asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], 4;" ::"r"(b) : "memory");
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr(word_addr, 1)), "r"(word), "r"(b) : "memory");
+}
 
 template <int CG, int CAP, bool TOGETHER>
 __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ TcTable<CAP> tab) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4];
+    __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4 + 2 * kDealt];
+    __shared__ int dealt[kDealt];
     __shared__ TcTile sp[CAP];      // the roles walk the table at every item; the constant bank is too small a cache for it
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
@@ -212,7 +254,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = tab.stages, n_items = tab.n_items;
     const uint32_t rank = CG == 2 ? (blockIdx.x & 1u) : 0u;      // cluster of two consecutive CTAs
-    const int unit = (int)blockIdx.x / CG, n_units = (int)gridDim.x / CG;
+    int* const queue = tab.err + kQueueWord;
+    int drawn = n_items;                   // warp 0 of the leader, lane 0
+    if (rank == 0 && threadIdx.x == 0) drawn = atomicAdd(queue, 1);
     const uint32_t staging = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t tiles = staging + kStageBytes;
     const uint32_t slot_bytes = (uint32_t)tab.slot_bytes;
@@ -221,6 +265,17 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     auto empty_bar = [&](int s) { return bar0 + 8u * (kMaxStages + s); };
     auto acc_full = [&](int a) { return bar0 + 8u * (2 * kMaxStages + a); };
     auto acc_empty = [&](int a) { return bar0 + 8u * (2 * kMaxStages + 2 + a); };
+    auto deal_full = [&](int i) { return bar0 + 8u * (2 * kMaxStages + 4 + i); };
+    auto deal_empty = [&](int i) { return bar0 + 8u * (2 * kMaxStages + 4 + kDealt + i); };
+    // the k-th item of this CTA, or -1 after the last; k is the caller's own count
+    auto take = [&](uint32_t k) -> int {
+        const uint32_t i = k % kDealt;
+        if (!deal_wait<CG>(deal_full(i), (k / kDealt) & 1u, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 16); return -1; }
+        const int item = *reinterpret_cast<volatile int*>(&dealt[i]);
+        __syncwarp();
+        if (lane == 0) deal_return<CG>(deal_empty(i), item);
+        return item;
+    };
     const uint32_t acc_cols = (uint32_t)tab.acc_cols;      // of one accumulator: a power of two >= the widest BN; together: of two
     const uint32_t lo_cols = acc_cols >> 1;                // together: the lo products' accumulator starts here
     const uint32_t tmem_cols = 2 * acc_cols;               // <= 512
@@ -235,6 +290,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         abort_flag = (*reinterpret_cast<volatile int*>(tab.err) != 0);   // an earlier CTA gave up: do not wait at all
         for (int s = 0; s < S; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 4 * CG); }
+        // readers of a dealt word: MMA warp and four epilogue warps, and the other CTA's producer and four epilogue warps
+        for (int i = 0; i < kDealt; ++i) { mbar_init(deal_full(i), 1); mbar_init(deal_empty(i), 5 * CG); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -259,7 +316,25 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         int s = 0, pi = 0;         // ring slot and its phase, across all items of this CTA
         uint32_t ph = 1;
         bool ok = true;
-        for (int item = unit; item < n_items && ok; item += n_units) {
+        for (uint32_t k = 0; ok; ++k) {
+            int item;
+            if (rank == 0) {
+                item = __shfl_sync(0xffffffffu, drawn, 0);
+                if (item >= n_items) item = -1;
+                const uint32_t i = k % kDealt;
+                ok = deal_wait<CG>(deal_empty(i), ((k / kDealt) & 1u) ^ 1u, &abort_flag);
+                if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 17); break; }
+                if (lane == 0) {
+                    *reinterpret_cast<volatile int*>(&dealt[i]) = item;
+                    mbar_arrive(deal_full(i));
+                    if (CG == 2) deal_to_peer(smem_u32(&dealt[i]), deal_full(i), item);
+                }
+                __syncwarp();
+                if (item >= 0 && lane == 0) drawn = atomicAdd(queue, 1);      // arrives under the copies
+            } else {
+                item = take(k);
+            }
+            if (item < 0) break;
             const TcItem t = tc_item(sp, tab.n, item, pi);
             const TcTile& P = sp[pi];
             const CUtensorMap* tmA = &tab.maps[3 * pi];
@@ -317,7 +392,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             uint32_t n_local = 0, ph = 0;
             int s = 0, pi = 0;
             bool ok = true;
-            for (int item = unit; item < n_items && ok; item += n_units, ++n_local) {
+            for (int item = take(0); item >= 0 && ok; item = take(++n_local)) {
                 const TcItem t = tc_item(sp, tab.n, item, pi);
                 const TcTile& P = sp[pi];
                 const uint32_t idesc = idesc_f16(CG * BM, P.BN, P.a_mn, P.b_mn);
@@ -393,8 +468,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         TcItem t = {}, t_next = {};
         int inv_bits = 0, inv_next = 0, pi_next = 0;
         float col[2], col_next[2] = {1.0f, 1.0f};
+        int item = take(0), item_next = -1;
         auto ahead = [&](int item) {
-            if (item >= n_items) return;
+            if (item < 0) return;
             t_next = tc_item(sp, tab.n, item, pi_next);
             const TcTile& P = sp[pi_next];
             const float* f = columns(P);
@@ -402,11 +478,12 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             col_next[0] = column(f, t_next.nt * P.BN + lane, P.N);
             col_next[1] = column(f, t_next.nt * P.BN + 32 + lane, P.N);
         };
-        ahead(unit);
-        for (int item = unit; item < n_items; item += n_units, ++n_local) {
+        ahead(item);
+        for (; item >= 0; item = item_next, ++n_local) {
             t = t_next; pi = pi_next; inv_bits = inv_next;
             col[0] = col_next[0]; col[1] = col_next[1];
-            ahead(item + n_units);
+            item_next = take(n_local + 1);     // drawn when the copies of this item have been issued: before its accumulator is full
+            ahead(item_next);
             const TcTile& P = sp[pi];
             const float* factors = columns(P);
             if (pi != at) {
@@ -502,6 +579,11 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
     if (warp == 1) {
         if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+    // the last one to leave sets the counter back for the next launch: everyone has drawn for the last time
+    if (rank == 0 && threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(queue + 1, 1) == (int)gridDim.x / CG - 1) { queue[0] = 0; queue[1] = 0; }
     }
 }
 

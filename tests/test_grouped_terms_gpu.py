@@ -27,3 +27,40 @@ def test_grad_w_of_a_large_group(I, O, tokens, layers):
             want = l["grad_out"].double().T @ l["x"].double()
             assert float((l["grad_w"].double() - want).norm() / want.norm()) <= 5e-6
             assert float((l["grad_w"].double() - want).abs().max() / want.square().mean().sqrt()) <= 5e-5
+
+
+def test_contractions_side_by_side_and_again():
+    """Two contexts' contractions at once, so that CTAs start late and find their items taken, then again: the counters are back at
+    zero.  An item's result does not depend on who computes it: all runs equal the first, bit for bit."""
+    from motifcl_b200 import Context
+    from motifcl_b200.runtime import linear_descs
+    sides = []
+    for I, O, tokens, layers in ((288, 768, 8192, 6), (2048, 1024, 3000, 2), (512, 512, 777, 9)):
+        stream = torch.cuda.Stream(device=0)
+        with torch.cuda.stream(stream):
+            ctx = Context.on_torch_stream(0)
+            g = torch.Generator(device=DEV).manual_seed(I)
+            ls = [dict(x=torch.randn(tokens, I, device=DEV, generator=g), grad_out=torch.randn(tokens, O, device=DEV, generator=g),
+                       state=torch.randint(0, 256, (O * I // 4 * 3,), device=DEV, generator=g, dtype=torch.int32).to(torch.uint8),
+                       scale=torch.full((O,), 0.05, device=DEV), v=torch.zeros(O, device=DEV), y=torch.empty(tokens, O, device=DEV),
+                       grad_x=torch.empty(tokens, I, device=DEV), grad_w=torch.empty(O, I, device=DEV), packed2_out=None) for _ in range(layers)]
+            descs = linear_descs([dict(l, in_features=I, out_features=O, batch=tokens, update_rows=0) for l in ls])
+            ctx.counter_linear_step_many(descs, 11, 3e-3, 0.0, 0.9, 1e-3, 1)
+            ctx.finish()
+            w = torch.empty(O, I, device=DEV)
+            ctx.counter_decode_weight(ls[-1]["state"], ls[-1]["scale"], w, I, O, 11)
+            ctx.finish()
+            want = ls[-1]["x"].double() @ w.double().T
+            assert float((ls[-1]["y"].double() - want).norm() / want.norm()) <= 1e-6
+            sides.append((ctx, descs, ls, [{n: l[n].clone() for n in ("y", "grad_x", "grad_w")} for l in ls], stream))
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for ctx, descs, ls, first, stream in sides:
+            with torch.cuda.stream(stream):
+                for l in ls:
+                    l["y"].fill_(7.0), l["grad_x"].fill_(7.0), l["grad_w"].fill_(7.0)
+                ctx.counter_linear_step_many(descs, 11, 3e-3, 0.0, 0.9, 1e-3, 1)
+        for ctx, _, ls, first, _ in sides:
+            ctx.finish()
+            for l, f in zip(ls, first):
+                assert all(torch.equal(l[n], f[n]) for n in f)
