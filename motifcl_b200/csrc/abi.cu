@@ -29,8 +29,6 @@ struct mcl_cuda_ctx {
     size_t ws_bytes = 0;
     // how the contractions run (mcl_cuda_set_gemm_mode)
     int gemm_mode = MCL_CUDA_GEMM_AUTO;
-    int act_terms = 3;
-    int grad_terms = 6;
     int* err_word = nullptr;     // device word the tensor-core kernels set when a bounded wait gives up
     const uint32_t* seed_offset = nullptr;   // device word added to every update seed (mcl_cuda_set_seed_offset)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -570,7 +568,7 @@ int mcl_cuda_set_gemm_mode(mcl_cuda_ctx* ctx, int mode, int act_terms, int grad_
         return fail(ctx, MCL_CUDA_EINVAL, "set_gemm_mode: unknown mode");
     if (act_terms != 2 && act_terms != 3) return fail(ctx, MCL_CUDA_EINVAL, "set_gemm_mode: act_terms must be 2 or 3");
     if (grad_terms != 3 && grad_terms != 6) return fail(ctx, MCL_CUDA_EINVAL, "set_gemm_mode: grad_terms must be 3 or 6");
-    ctx->gemm_mode = mode; ctx->act_terms = act_terms; ctx->grad_terms = grad_terms;
+    ctx->gemm_mode = mode;                 // every setting runs the same two fp16 terms
     return MCL_CUDA_OK;
 }
 int mcl_cuda_alloc(mcl_cuda_ctx* ctx, size_t bytes, void** out_dptr) {

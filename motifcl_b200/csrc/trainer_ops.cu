@@ -780,7 +780,7 @@ cudaError_t launch_adam(float* param, const float* grad, float* m, float* v, siz
 
 namespace {
 template <typename K>
-cudaError_t with_smem(K kern, size_t bytes) {      // attribute set once per kernel and device
+cudaError_t with_smem(K kern, size_t bytes) {      // set on every call: it holds per device
     return bytes <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 // The tiled kernels walk over the keys of a query tile one tile after another: right for any number of keys while there are

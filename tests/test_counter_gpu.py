@@ -236,12 +236,10 @@ def test_ternary_gemv_vs_oracle(ctx, orc, M, O, I):
     assert rel_l2(y.cpu().numpy(), orc.forward(x, st, scale, 11, O)) <= 1e-5
 
 
-@pytest.mark.parametrize("O,I", [(203, 1024), (33, 4096), (2380, 2048), (64, 256), (500, 3840), (3000, 1280),   # one table for the whole row
-                                 (5000, 8192), (100, 6144), (257, 14336)])     # sliced tables, ticket reduction
-def test_single_row_gemv_table_kernels_vs_oracle(ctx, orc, O, I):
-    """One activation row on the table look-up kernels: row counts that are no multiple of 16 or 256, every field
-    value (3 included: random words), repeated launches (the ticket words must come back to zero) and a recorded
-    batch replayed several times."""
+@pytest.mark.parametrize("O,I", [(203, 1024), (33, 4096), (2380, 2048), (64, 256), (500, 3840), (3000, 1280), (5000, 8192), (100, 6144), (257, 14336)])
+def test_single_row_gemv_vs_oracle(ctx, orc, O, I):
+    """One activation row: row counts that are no multiple of 16 or 256, rows of one slice per CTA and of several, every field value
+    (3 included: random words), repeated launches and a recorded batch replayed several times."""
     rng = np.random.default_rng(O + I)
     words = rng.integers(0, 2 ** 32, size=(O, I // 16), dtype=np.uint64).astype(np.uint32)
     fields = np.zeros((O, I), np.float64)
@@ -625,10 +623,9 @@ FUSED_SHAPES = [(256, 64, 64), (1000, 96, 32), (2048, 288, 288), (1024, 288, 768
 
 
 @pytest.mark.parametrize("N,I,O", FUSED_SHAPES)
-def test_fused_tf32_products_vs_oracle(ctx, orc, N, I, O):
-    """Layers up to 1024 features whose dimensions are multiples of 32 take the kernel that reads the
-    fp32 tensors through TMA and multiplies tf32 hi/lo terms (transposed operands in place):
-    every product within 1e-5 relative L2 of the fp32 reference sums, ragged token counts included."""
+def test_step_products_of_narrow_layers_vs_oracle(ctx, orc, N, I, O):
+    """All products of one layer of up to 1024 features through the step call (fp16 terms, transposed operands read in place):
+    each within 1e-5 relative L2 of the fp32 reference sums, ragged token counts included."""
     rng = np.random.default_rng(N + 3 * I + 7 * O)
     C = 11
     state = codec.pack_codes(rng.integers(0, 64, size=(O, I)).astype(np.uint8)).reshape(-1)
