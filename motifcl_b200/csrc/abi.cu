@@ -111,7 +111,13 @@ int ws_reserve(mcl_cuda_ctx* ctx, size_t bytes, void** out) {
             return fail(ctx, MCL_CUDA_EINVAL, "workspace would grow (to " + std::to_string(bytes) + " bytes) while " +
                                                   std::to_string(ctx->live_batches) + " recorded batch(es) hold addresses inside it: "
                                                   "run the largest call once before recording, or destroy the batches first");
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        // a capture that the caller runs on the stream would be broken by the wait and the allocation
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(ctx->stream, &st);
+        if (e != cudaSuccess) return fail_cuda(ctx, "workspace capture status", e);
+        if (st != cudaStreamCaptureStatusNone)
+            return fail(ctx, MCL_CUDA_EINVAL, "workspace would grow while the stream is being captured: run the same calls once uncaptured first");
+        e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return fail_cuda(ctx, "workspace sync", e);
         if (ctx->ws) cudaFree(ctx->ws);
         ctx->ws = nullptr;

@@ -114,3 +114,35 @@ def test_both_routes_of_a_layer(N, I, O):
             assert float((y - wy).norm() / wy.norm()) < 1e-6 and float((dx - wdx).norm() / wdx.norm()) < 1e-6
             assert float(((v2.double() - wv) / wv).abs().max()) <= 2 * 256 * 2.0 ** -23
         ctx.close()
+
+
+def test_layer_calls_under_a_capture_of_the_caller():
+    """A graph that the caller captures on the context's stream: layer calls that would rather have workspace run without, and a call that
+    cannot is refused without breaking the capture."""
+    from motifcl_b200 import Context, MotifclCudaError
+    N, I, O = 8200, 1024, 1024
+    st, sc, v, x, dy = _layer(N, I, O, 4)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        ctx = Context.on_torch_stream(0)
+        w, y, dx = torch.empty(O, I, device="cuda"), torch.empty(N, O, device="cuda"), torch.empty(N, I, device="cuda")
+        ctx.counter_decode_weight(st, torch.ones_like(sc), w, I, O, 11)
+        wy, wdx = (x.double() @ w.double().T) * sc.double(), (dy * sc).double() @ w.double()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        try:
+            ctx.counter_forward(x, st, sc, y, N, I, O, 11)
+            ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+            with pytest.raises(MotifclCudaError):
+                ctx.matmul_f32(x, w, y, N, I, O, trans_b=True)
+        finally:
+            graph.capture_end()
+        for _ in range(2):
+            y.zero_(), dx.zero_()
+            graph.replay()
+            ctx.finish()
+            assert float((y - wy).norm() / wy.norm()) < 1e-6 and float((dx - wdx).norm() / wdx.norm()) < 1e-6
+        del graph
+        ctx.close()
