@@ -59,7 +59,9 @@ int mcl_cuda_download(mcl_cuda_ctx* ctx, void* dst_host, const void* src, size_t
 /* Number of kernels this library has launched on the context so far. */
 uint64_t mcl_cuda_launch_count(mcl_cuda_ctx* ctx);
 /* Bytes of device memory the context's internal workspace holds (grow-only scratch of the entry points: the row tile
- * of grad_w of the fused update, operand planes, split-K partial sums).  It is how a caller checks the memory-native
+ * of grad_w of the fused update, operand planes, split-K partial sums).  Operand planes take 4 bytes per element of each split
+ * tensor; a grouped step (mcl_cuda_counter_linear_step_many) holds those of all its layers at once, up to 6 GB (1.7 GB for 42
+ * layers of dim 288 / 768 at 8192 tokens).  It is how a caller checks the memory-native
  * property MotifCL gates on (tests/test_memory_truth_gate.cpp:30-126: the fused update may allocate less than a
  * quarter of a dense fp32 weight). */
 size_t mcl_cuda_workspace_bytes(mcl_cuda_ctx* ctx);

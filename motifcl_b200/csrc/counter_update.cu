@@ -312,8 +312,8 @@ counter_update_dense_kernel(const UpdParams p) {
 //            one unit, writes the new state words over the old ones in the slot, the warp copies its 384 bytes out
 //            with 16-byte stores and stores its 32 words of 2-bit fields; a warp that has passed a row releases its slot.
 // Measured on B200 (8192 x 4096 fp32 gradient, CUDA events): 1.95 TB/s = 0.30 of the copy bandwidth; the kernel issues
-// ~55 instructions per weight (two 32-bit hashes, the quotient, floor / compare / two table look-ups), which at four
-// instructions per clock and SM bounds it near 0.55 whatever the memory system does.
+// 67 instructions per weight (two 32-bit hashes, the quotient, floor / compare / two table look-ups), which at four
+// instructions per clock and SM caps it near 0.47; it reaches two thirds of that, with dependent chains and one busy pipe in between.
 // Every wait is bounded: on time-out the kernel sets *err (when given) and all roles leave.
 constexpr int kWsThreads = 512;
 // Every fourth warp is a stats warp: warps are dealt to the SM's four schedulers by warp number, so the stats warps

@@ -262,7 +262,8 @@ cudaError_t mv_launch(MvParams p, int sm_count, size_t max_smem, int slot, bool 
     const size_t group_bytes = (size_t)S * Mp * MV_ROWS * 8;
     // Clusters of 8 do not tile the GPCs: of sm_count / 8 the last ones share SMs with others, which then hold the whole launch up.
     // Seven eighths of the SMs (16 clusters of 8): 20 matrices of an 8B-scale model 88 -> 81 us for one row, 118 -> 106 for four, 181 -> 166
-    // for eight with other work beside them, 162 and 164 us alone; 12 clusters 84 and 204, 30 (two CTAs on every SM) 109 and 139.
+    // for eight with other work beside them (one row alone 164 -> 162); 12 clusters 84 and 204, 30 (two CTAs on every SM) 109 and 139: one
+    // setting for all rows, which is not the best one for eight.
     int clusters = sm_count * 7 / 8 / S;
     if (clusters < 1) clusters = 1;
     if (clusters > groups) clusters = groups;
