@@ -199,10 +199,10 @@ int mcl_cuda_set_gemm_mode(mcl_cuda_ctx* ctx, int mode, int act_terms, int grad_
 /* ---- the steps of SEVERAL counter linears in one call (the reference records the dispatches of
  * a step into one command buffer, include/motifcl/runtime/vulkan_backend.hpp:138 VulkanDispatchRecording; this is
  * that recording stated as data).  Layer i does exactly what mcl_cuda_counter_linear_step does with
- * the same arguments; layers whose shapes allow it (in and out features multiples of 32 up to 1024,
- * 16-byte aligned tensors) share grouped launches: one expansion of the ternary digits, the
- * products of all layers as one table of tensor-core work items, one split-K reduction, one
- * update.  Layers are independent: no tensor of one may alias a tensor of another. ---- */
+ * the same arguments; layers whose shapes allow it (in and out features multiples of 4, 16-byte
+ * aligned outputs and scale, batch x in x out of 2^22 or more) share grouped launches: the split of
+ * the tensors, one expansion of the ternary digits, the products of all layers as tables of tensor-core
+ * work items, one split-K reduction, one update.  Layers are independent: no tensor of one may alias a tensor of another. ---- */
 typedef struct mcl_cuda_linear_desc {
     const float* x;          /* [batch, in] */
     const float* grad_out;   /* [batch, out] */

@@ -138,19 +138,19 @@ def test_products_at_the_ends_of_fp32(ctx):
             assert float(_row_errors(c, want).max()) <= _bound(K), (up, ta, tb)
 
 
-def test_partner_scales_of_a_weight_gradient(ctx):
+@pytest.mark.parametrize("tokens,I,O", [(4096, 288, 320), (600, 64, 5000), (300, 64, 33000)])       # each block size of the split, and rows read twice
+def test_partner_scales_of_a_weight_gradient(ctx, tokens, I, O):
     """dW whose largest contributions come from rows where x is small and grad_out large: the scale that completes x's row scales is
     not the one of the largest grad_out, and a sample that misses the row is put right."""
-    tokens, I, O = 4096, 288, 320
     state, scale, x, dy = _linear(tokens, I, O, 9)
-    for row, dn, up in ((5, 40, 60), (4000, 60, 40), (777, 0, 30), (778, 100, 100)):
+    for row, dn, up in ((5, 40, 60), (tokens - 96, 60, 40), (177, 0, 30), (178, 100, 100)):
         x2, dy2 = x.clone(), dy.clone()
         x2[row] *= 2.0 ** -dn
         dy2[row, 11] *= 2.0 ** up
         for grouped in (0, 2):
             y, dx, dw, wy, wdx, wdw = _products(ctx, state, scale, x2, dy2, grouped)
             assert float((dw.double() - wdw).norm() / wdw.norm()) <= _bound(tokens)
-            assert float(_row_errors(y, wy).max()) <= 1e-6 and float(_row_errors(dx, wdx).max()) <= 4e-6
+            assert float(_row_errors(y, wy).max()) <= 1e-6 and float(_row_errors(dx, wdx).max()) <= 2.0 ** -22 + 2.0 ** -24 * 4 * (O / 64)
 
 
 @pytest.mark.parametrize("K", [1, 7, 8, 9, 130, 252, 257, 4095, 4096, 4104, 10924, 32764, 32776, 40001])
