@@ -77,6 +77,8 @@ size_t mcl_cuda_workspace_bytes(mcl_cuda_ctx* ctx);
  * a call that would make the workspace grow is refused (MCL_CUDA_ERR_ARG, "workspace would grow")
  * instead of freeing memory the batch still points into; destroy the batches first, or run the
  * larger call once before recording.
+ * Decode GEMVs (mcl_cuda_ternary_gemv) that follow one another in a recording share launches where none of them reads or
+ * overwrites what another one writes; a batch then stands for fewer launches than calls.
  * Recording captures the calling thread's work on the context's stream only.  Do not enqueue
  * work of other libraries that hands off to streams of their own (an NCCL collective through a
  * framework's process group, for one) between begin and end: such work is not part of the batch

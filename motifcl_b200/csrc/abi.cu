@@ -14,6 +14,19 @@
 #include "kernels.h"
 #include "motifcl_cuda.h"
 
+// The GEMV launches that stand at the end of a recording, with nothing else between them.
+struct GemvChain {
+    struct Launch {
+        bool tc;                           // two nodes of gemv_tc.cu, or one of gemv_mma.cu
+        cudaGraphNode_t node[2];
+        int M;
+        std::vector<mcl::GemvItem> items;
+    };
+    std::vector<Launch> launches;
+    cudaGraphNode_t tail = nullptr;        // node of the last one, and the capture it belongs to: a handle alone may come back for a
+    unsigned long long capture = 0;        // node of a later one
+};
+
 struct mcl_cuda_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -35,8 +48,7 @@ struct mcl_cuda_ctx {
     uint64_t lane_mark = 0;      // launches at the last lane_fork (when this context is a lane)
     bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end
     uint64_t recorded_launches = 0;
-    cudaGraphNode_t last_gemv = nullptr;   // node of the last gemv_mma launch on this stream, and the capture it belongs to: a
-    unsigned long long last_capture = 0;   // handle alone may come back for a node of a later one
+    GemvChain gemvs;             // launches at the end of the recording
     int live_batches = 0;        // recorded batches not yet destroyed: they hold addresses inside the workspace
 };
 
@@ -480,6 +492,7 @@ int mcl_cuda_batch_begin(mcl_cuda_ctx* ctx) {
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail_cuda(ctx, "batch_begin", e);
     ctx->recording = true;
+    ctx->gemvs = GemvChain();
     ctx->recorded_launches = ctx->launches;
     return MCL_CUDA_OK;
 }
@@ -1450,6 +1463,54 @@ static cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx, unsigned long long* capt
     return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
 }
 
+// The launch of the chain that `item` can join: the earliest one with room, behind which nothing reads or writes what the item
+// writes, or writes what it reads.  Null: none.
+static GemvChain::Launch* joinable(GemvChain& chain, const mcl::GemvItem& item, int M, bool mma, bool tc) {
+    struct Range { uintptr_t begin, end; };
+    const auto range = [](const void* p, size_t bytes) { const uintptr_t b = reinterpret_cast<uintptr_t>(p); return Range{b, b + bytes}; };
+    const auto meet = [](Range a, Range b) { return a.begin < b.end && b.begin < a.end; };
+    const auto out = [&](const mcl::GemvItem& i, int m) { return range(i.y, (size_t)m * i.out_features * 4); };
+    const auto takes = [&](const mcl::GemvItem& i, int m, Range r) {
+        return meet(range(i.x, (size_t)m * i.in_features * 4), r) || meet(range(i.packed2, (size_t)i.in_features / 4 * i.out_features), r) ||
+               meet(range(i.scale, (size_t)i.out_features * 4), r);
+    };
+    GemvChain::Launch* found = nullptr;
+    for (size_t l = chain.launches.size(); l-- > 0;) {
+        GemvChain::Launch& at = chain.launches[l];
+        for (const mcl::GemvItem& i : at.items)
+            if (meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M))) return found;
+        if (at.M == M && at.items.size() < mcl::kGemvListCap &&
+            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items[0].in_features, item.in_features))) found = &at;
+    }
+    return found;
+}
+
+// The nodes of a recorded launch take its list, which has grown.  The one node of gemv_mma.cu becomes the first of gemv_tc.cu where the
+// list is long enough for it and the second can stand right behind.
+static cudaError_t join_gemv(mcl_cuda_ctx* ctx, GemvChain::Launch& at, int M, bool last) {
+    const mcl::GemvItem* items = at.items.data();
+    const int n = (int)at.items.size();
+    const bool room = mcl::gemv_tc_workspace_bytes(items, n, M, ctx->sm_count) <= ctx->ws_bytes;
+    const auto tc = [&](int parts, const cudaGraphNode_t* nodes) {
+        return mcl::launch_ternary_gemv_tc(items, n, M, ctx->ws, parts, false, nodes, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
+    };
+    if (at.tc) return room ? tc(3, at.node) : cudaErrorMemoryAllocation;
+    bool can = room && last && mcl::gemv_tc_pays(items, n, M, ctx->sm_count);
+    for (const mcl::GemvItem& i : at.items) can = can && mcl::gemv_tc_supported(M, i.in_features, i.packed2);
+    if (!can) return mcl::launch_ternary_gemv_mma(items, n, M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
+    cudaError_t e = tc(1, at.node);
+    if (e != cudaSuccess) return e;
+    e = tc(2, nullptr);
+    if (e != cudaSuccess) {
+        mcl::launch_ternary_gemv_mma(items, n - 1, M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
+        return e;
+    }
+    ++ctx->launches;
+    at.node[1] = ctx->gemvs.tail = recorded_tail(ctx, &ctx->gemvs.capture);
+    at.tc = true;
+    return cudaSuccess;
+}
+
 int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* packed2,
                           const float* scale, float* y, size_t M, size_t in_features,
                           size_t out_features) {
@@ -1464,36 +1525,56 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
     MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
     MCL_TRY(check_ptr(ctx, op, "y", y, 4));
     DeviceGuard guard(ctx->device);
-    if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && mcl::gemv_mma_supported((int)M, (int)in_features, packed2, ctx->max_smem)) {
-        // One launch against three up to M = 8 (20 matrices of an 8B-scale model: 90 us against 194 at M = 2, 181 against 249 at
-        // M = 8; level at 11).  Only in a recording is it known what runs before: two of these in a row overlap, the
-        // second one's weights being no result of the first.
+    const mcl::GemvItem item = {x, packed2, scale, y, (int)in_features, (int)out_features};
+    const bool exact = ctx->gemm_mode == MCL_CUDA_GEMM_EXACT;
+    const bool mma = !exact && mcl::gemv_mma_supported((int)M, (int)in_features, packed2, ctx->max_smem);
+    const bool tc = !exact && mcl::gemv_tc_supported((int)M, (int)in_features, packed2) && (mma || out_features >= 128) && (mma || M > 1);
+    if (mma || tc) {
+        // Only in a recording is it known what runs before and after: a matrix joins a launch there where nothing that was recorded since
+        // has to do with it.
+        GemvChain& chain = ctx->gemvs;
         unsigned long long capture = 0;
         const cudaGraphNode_t tail = recorded_tail(ctx, &capture);
-        const bool follows = tail != nullptr && tail == ctx->last_gemv && capture == ctx->last_capture;
-        MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features, follows,
-                                                         ctx->sm_count, ctx->max_smem, ctx->stream));
-        ctx->last_gemv = recorded_tail(ctx, &ctx->last_capture);
+        const bool follows = tail != nullptr && tail == chain.tail && capture == chain.capture;
+        if (!follows) chain.launches.clear();
+        if (GemvChain::Launch* at = joinable(chain, item, (int)M, mma, tc)) {
+            at->items.push_back(item);
+            if (join_gemv(ctx, *at, (int)M, at == &chain.launches.back()) == cudaSuccess) return MCL_CUDA_OK;
+            at->items.pop_back();
+            cudaGetLastError();
+        }
+        GemvChain::Launch at = {!mma || (tc && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count)), {}, (int)M, {item}};
+        void* wsp = ctx->ws;
+        if (tc) {
+            // Where it can grow, room for the digits of more xs than this one, also for a call that does without: the launches of a recording
+            // may take the call together with others.
+            const size_t need = mcl::gemv_tc_workspace_bytes(&item, 1, (int)M, ctx->sm_count);
+            if (need > ctx->ws_bytes && (at.tc || !ctx->recording)) {
+                const std::string error = ctx->error;
+                const int rc = ws_reserve(ctx, need + (size_t(16) << 20), &wsp);
+                if (rc != MCL_CUDA_OK && !mma) return rc;
+                if (rc != MCL_CUDA_OK) { ctx->error = error; at.tc = false; }
+            }
+        }
+        if (at.tc) {
+            for (int part = 0; part < 2 && at.tc; ++part) {
+                MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_tc(&item, 1, (int)M, wsp, 1 << part, follows, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
+                at.node[part] = recorded_tail(ctx, &chain.capture);
+            }
+        }
+        if (!at.tc) {
+            MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(&item, 1, (int)M, follows, nullptr, ctx->sm_count, ctx->max_smem, ctx->stream));
+            at.node[0] = recorded_tail(ctx, &chain.capture);
+        }
+        chain.tail = at.node[at.tc ? 1 : 0];
+        if (chain.tail) chain.launches.push_back(at);
         return MCL_CUDA_OK;
     }
-    if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && M == 1) {
+    if (!exact && M == 1) {
         // a single activation row whose shape the integer MMAs do not take: streaming the words through the CUDA
-        // cores in one launch still beats the three launches of the tensor-core route
+        // cores in one launch still beats the launches of the tensor-core route
         MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_stream(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features,
                                                             ctx->sm_count, ctx->stream));
-        return MCL_CUDA_OK;
-    }
-    if (ctx->gemm_mode != MCL_CUDA_GEMM_EXACT && out_features >= 128 &&
-        mcl::gemv_tc_supported((int)M, (int)in_features, (int)out_features) &&
-        reinterpret_cast<uintptr_t>(packed2) % 16 == 0) {
-        void* wsp = nullptr;
-        MCL_TRY(ws_reserve(ctx, mcl::gemv_tc_workspace_bytes((int)M, (int)in_features, (int)out_features), &wsp));
-        int launches = 0;
-        cudaError_t e = mcl::launch_ternary_gemv_tc(x, packed2, scale, y, (int)M, (int)in_features, (int)out_features,
-                                                    wsp, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream,
-                                                    &launches);
-        ctx->launches += launches;
-        if (e != cudaSuccess) return fail_cuda(ctx, op, e);
         return MCL_CUDA_OK;
     }
     MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv(x, packed2, scale, y, (int)M, (int)in_features,

@@ -9,14 +9,21 @@
 // each forms the int8 digits of its own slice of x (with its own power-of-two scale, so nothing has to be known of the rest of
 // the row), and the slices of an output meet through distributed shared memory in slice order.  (3) Bytes in flight: a
 // warp's next units are loaded into registers while it works on one, the first ones before the activations are touched at all.
-// Where the launch before this one in a recorded batch is a launch of this kernel, those first loads even pass under its tail
+// Where the launch before this one in a recorded batch is a decode GEMV too, those first loads even pass under its tail
 // (programmatic dependent launch): the words of a matrix are no output of such a launch; x may be, and is read after the wait.
+//
+// A recording puts matrices that do not depend on one another into one launch (a list): set-up, digits and hand-over of a launch are 2 to 4
+// us, as long as the words of a small matrix take.  One row of x, launches apart and as a list: q, k, v of 2048 x 2048 (three
+// launches of 4.0 us) 7.8 us, w1 and w3 of 14336 x 4096 21 us (two of 10.7); 4 blocks of 1280 / 5120, 20 matrices, 60 and 21 us.  Long lists
+// are quicker on gemv_tc.cu (gemv_tc_pays).
 //
 // x is scaled to whole numbers of 30 bits and sign below the slice's largest magnitude and written as four signed digits of
 // base 256; one row alone (M = 1) has columns to spare and gets the 31 bits of the remainder as a second row.  Integer sums are
 // exact; the offset of the fields (f = t + 1) is taken off as a digit sum; slices are put together in double precision.
 // Legacy integer MMAs run at 2025 multiply-adds per clock and SM here (measured): 128 weights per clock for M <= 4 and 63 for
 // M = 8; beyond that the tcgen05 kernel is the faster one.
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace mcl {
@@ -28,18 +35,30 @@ constexpr int MV_CHUNK = 256;          // weights of a row per unit: 64 bytes, 1
 constexpr int MV_ROWS = 32;            // rows of a unit
 constexpr int MV_MAX_S = 8;
 
-struct MvParams {
+// One launch takes a list of matrices; their groups of 32 rows are numbered through.
+struct MvMat {
+    const uint4* words;
     const float* x;
-    const uint32_t* packed2;
     const float* scale;
     float* y;
-    int M, I, O;
+    long long cost;                    // of everything before it, in chunks
+    int I, O;
+    int first;                         // number of its first group
+    int next;                          // the first matrix behind it that has another x
+};
+template <int CAP>         // one matrix, or kGemvListCap
+struct MvTable {
+    long long cost;
+    int n, groups, M;
     int log_s;                         // CTAs of a cluster
-    int groups_q, groups_r;            // row groups of a cluster (the first groups_r clusters take one more)
+    int groups_q, groups_r;            // one matrix: groups of a cluster (the first groups_r clusters take one more)
     int block;                         // groups whose partial sums are held at a time
     int owned;                         // of them, the most that one CTA of the cluster finishes
     int xq_bytes;                      // the digits of the widest slice
+    MvMat m[CAP];
 };
+constexpr int MV_GROUP_COST = 1;       // chunks that the end of a group counts for
+__host__ __device__ inline int mv_chunks(int I) { return (I + MV_CHUNK - 1) / MV_CHUNK; }
 
 __device__ __forceinline__ uint4 mv_load(const uint4* p) {
     uint4 v;
@@ -57,44 +76,111 @@ __device__ __forceinline__ void mv_mma(int (&c)[4], uint32_t a0, uint32_t a1, ui
 }
 __device__ __forceinline__ uint32_t mv_word(const uint4& v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
 
+// LIST: more than one matrix.  A cluster takes a run of groups, cut so that all clusters have the same number of chunks whatever the matrices are.  Matrices with
+// one x are neighbours in the list (a segment): their digits are formed once.  The words are loaded ahead across groups, rounds
+// (a barrier) and segments (new digits) alike.
 // NT: tiles of eight digit columns (two rows of x each); R: units a warp has in registers
-template <int NT, int R>
-__global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams p) {
+template <int NT, int R, bool LIST>
+__global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_constant__ MvTable<LIST ? kGemvListCap : 1> p) {
     extern __shared__ __align__(128) unsigned char mv_smem[];
     __shared__ unsigned int amax[8];
     __shared__ int corr[NT * 8];
-    __shared__ double xscale[MV_MAX_S][8];          // of every slice: the value of one unit of its whole numbers
+    __shared__ double xscale[2][MV_MAX_S][8];       // of every slice: the value of one unit of its whole numbers; two segments
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
     const int lg_s = p.log_s, S = 1 << lg_s, rank = blockIdx.x & (S - 1), cid = blockIdx.x >> lg_s;
-    const int M = p.M, Mp = M == 1 ? 2 : M, I = p.I, O = p.O;
-    const int g_begin = cid * p.groups_q + min(cid, p.groups_r);
-    const int g_end = g_begin + p.groups_q + (cid < p.groups_r ? 1 : 0);
-    const int NC = (I + MV_CHUNK - 1) / MV_CHUNK;
-    const int c0 = (rank * NC) >> lg_s, nc = (((rank + 1) * NC) >> lg_s) - c0;
-    const int row16 = I >> 6;                       // 16-byte pieces of a row
+    const int M = p.M, Mp = M == 1 ? 2 : M;
+    int mat = 0, g_begin, g_end;                    // matrix of the group at hand; this cluster's groups
+    if (LIST) {
+        // the first group at or behind a share of the cost, and its matrix
+        auto cut = [&](int c, int& m) -> int {
+            const long long t = p.cost * c / (gridDim.x >> lg_s);
+            while (m + 1 < p.n && t >= p.m[m + 1].cost) ++m;
+            const int per = mv_chunks(p.m[m].I) + MV_GROUP_COST, end = m + 1 < p.n ? p.m[m + 1].first : p.groups;
+            const int f = p.m[m].first + (int)((t - p.m[m].cost + per - 1) / per);
+            if (f >= end && m + 1 < p.n) ++m;
+            return min(f, end);
+        };
+        int behind = 0;
+        g_begin = cut(cid, mat);
+        g_end = (cid + 1) * S == (int)gridDim.x ? p.groups : cut(cid + 1, behind);
+    } else {
+        g_begin = cid * p.groups_q + min(cid, p.groups_r);
+        g_end = g_begin + p.groups_q + (cid < p.groups_r ? 1 : 0);
+    }
+    auto segment_end = [&](int m) -> int {
+        if (!LIST) return g_end;
+        const int k = p.m[m].next;
+        return min(g_end, k < p.n ? p.m[k].first : p.groups);
+    };
 
     uint4 w[R][4];
-    const uint4* words = reinterpret_cast<const uint4*>(p.packed2);
-    int fg = g_begin + warp, fc = 0;                // load cursor: group, chunk
-    auto load = [&](int end, uint4 (&u)[4]) {
-        if (fg >= end) return;
-        const int piece = (c0 + fc) * 4 + tq;
-        if (piece < row16) {
+    // load cursor: group lf of matrix lm, its chunk lc; the warp takes every MV_WARPS-th group of a segment
+    int lm = mat, lf = g_begin + warp, lc = 0, l_end = g_begin < g_end ? segment_end(mat) : g_begin, l_c0 = 0, l_nc = 1, l_row16 = 0;
+    const uint4* l_words = nullptr;                 // this lane's piece of the group's first row, in the slice's first chunk
+    uint32_t l_off[4];                              // from there to its four rows, in pieces
+    auto seek = [&](bool segment) {                 // lf has moved
+        if constexpr (LIST) {
+            while (lf >= l_end && l_end < g_end) {
+                lm = p.m[lm].next;
+                lf = l_end + warp;
+                l_end = segment_end(lm);
+                segment = true;
+            }
+            if (lf >= l_end) return;
+            while (lm + 1 < p.n && lf >= p.m[lm + 1].first) ++lm;
+            if (segment) {
+                const int NC = mv_chunks(p.m[lm].I);
+                l_c0 = (rank * NC) >> lg_s;
+                l_nc = (((rank + 1) * NC) >> lg_s) - l_c0;
+                l_row16 = p.m[lm].I >> 6;               // 16-byte pieces of a row
+            }
+            const int row = (lf - p.m[lm].first) * MV_ROWS, last = p.m[lm].O - 1 - row;
+            l_words = p.m[lm].words + (size_t)row * l_row16 + l_c0 * 4 + tq;
 #pragma unroll
-            for (int h = 0; h < 4; ++h) u[h] = mv_load(words + (size_t)min(fg * MV_ROWS + h * 8 + g, O - 1) * row16 + piece);
+            for (int h = 0; h < 4; ++h) l_off[h] = (uint32_t)(min(h * 8 + g, last) * l_row16);
+        }
+    };
+    auto load = [&](uint4 (&u)[4]) {
+        if (lf >= l_end) return;
+        const int piece = (l_c0 + lc) * 4 + tq;
+        if (piece < l_row16) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                u[h] = mv_load(LIST ? l_words + lc * 4 + l_off[h] : p.m[0].words + (size_t)min(lf * MV_ROWS + h * 8 + g, p.m[0].O - 1) * l_row16 + piece);
         } else {
 #pragma unroll
             for (int h = 0; h < 4; ++h) u[h] = make_uint4(0, 0, 0, 0);       // beyond the row: the digits there are zero as well
         }
-        if (++fc == nc) { fc = 0; fg += MV_WARPS; }
+        if (++lc == l_nc) { lc = 0; lf += MV_WARPS; seek(false); }
     };
+    if (LIST) {
+        seek(true);
+    } else {
+        const int NC = mv_chunks(p.m[0].I);
+        l_c0 = (rank * NC) >> lg_s;
+        l_nc = (((rank + 1) * NC) >> lg_s) - l_c0;
+        l_row16 = p.m[0].I >> 6;
+    }
 #pragma unroll
-    for (int j = 0; j < R; ++j) load(min(g_begin + p.block, g_end), w[j]);
+    for (int j = 0; j < R; ++j) load(w[j]);
     if (threadIdx.x < 8) amax[threadIdx.x] = 0u;
     if (threadIdx.x < NT * 8) corr[threadIdx.x] = 0;
     if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // only "this CTA runs": nothing to publish
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t part0 = (uint32_t)__cvta_generic_to_shared(mv_smem) + (uint32_t)p.xq_bytes;
+    const uint32_t part_bytes = (uint32_t)(p.owned * Mp) * (MV_ROWS * 8u);      // one slice's sums for the groups a CTA finishes
+    int parity = 0;
+    bool first = true;
+#pragma unroll 1
+    for (int seg = 0, s_begin = g_begin; LIST ? s_begin < g_end : seg == 0; ++seg) {
+    const int s_end = segment_end(mat), I = p.m[mat].I, NC = mv_chunks(I);
+    const float* const x = p.m[mat].x;
+    const int c0 = (rank * NC) >> lg_s, nc = (((rank + 1) * NC) >> lg_s) - c0;
+    if (LIST && seg > 0) {
+        if (threadIdx.x < 8) amax[threadIdx.x] = 0u;
+        if (threadIdx.x < NT * 8) corr[threadIdx.x] = 0;
+    }
     __syncthreads();
 
     // -- the digits of this slice: a warp takes 128 activations of one row at a time, four a lane --------------------
@@ -104,7 +190,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
         const int m = unit / per_row, k = k0 + (unit - m * per_row) * 128 + lane * 4;
         unsigned int top = 0u;
         if (k < I) {
-            const float4 v = mv_load_x(p.x + (size_t)m * I + k);
+            const float4 v = mv_load_x(x + (size_t)m * I + k);
             top = max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
                       max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu));
         }
@@ -120,7 +206,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
         int e = max((int)(top >> 23) - 126, -90);   // 2^e above every magnitude (of the smallest ones: 2^-90)
         if (top >= 0x7F800000u) e = 0;
         const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
-        const float4 t = k < I ? mv_load_x(p.x + (size_t)m * I + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 t = k < I ? mv_load_x(x + (size_t)m * I + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float f[4] = {t.x * inv, t.y * inv, t.z * inv, t.w * inv};
         uint32_t r[4];
 #pragma unroll
@@ -149,7 +235,8 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
         if (lane < 4) atomicAdd(&corr[mp * 4 + d], sum);
     }
     __syncthreads();
-    if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster runs
+    if (S > 1 && first) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster runs
+    first = false;
     if ((int)threadIdx.x < 8 * S && (int)(threadIdx.x & 7) < M) {
         const int m = threadIdx.x & 7;
         const unsigned int top = amax[m];
@@ -158,29 +245,25 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
                                             : __longlong_as_double((long long)(1023 + e - 30) << 52);
         uint32_t to;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to)
-                     : "r"((uint32_t)__cvta_generic_to_shared(&xscale[rank][m])), "r"(threadIdx.x >> 3));
+                     : "r"((uint32_t)__cvta_generic_to_shared(&xscale[seg & 1][rank][m])), "r"(threadIdx.x >> 3));
         asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
     }
 
     // -- the contraction ---------------------------------------------------------------------------------------------
-    const uint32_t part0 = (uint32_t)__cvta_generic_to_shared(mv_smem) + (uint32_t)p.xq_bytes;
-    const uint32_t part_bytes = (uint32_t)(p.owned * Mp) * (MV_ROWS * 8u);      // one slice's sums for the groups a CTA finishes
-    int parity = 0;
-    for (int gb = g_begin; gb < g_end; gb += p.block, parity ^= 1) {
-        const int ge = min(gb + p.block, g_end);
-        if (gb != g_begin) {
-            fg = gb + warp; fc = 0;
-#pragma unroll
-            for (int j = 0; j < R; ++j) load(ge, w[j]);
-        }
+    int grp = s_begin + warp;
+#pragma unroll 1
+    for (int gb = s_begin; gb < s_end; gb += p.block, parity ^= 1) {
+        const int ge = min(gb + p.block, s_end);
         const uint32_t part = (uint32_t)(parity * S) * part_bytes;
         int acc[2][NT][4] = {};
         int cc = 0;
 #pragma unroll 1
-        for (int grp = gb + warp; grp < ge;) {
+        while (grp < ge) {
+            int used = 0;
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 if (grp < ge) {
+                    used = j + 1;
                     const uint4* bx = reinterpret_cast<const uint4*>(mv_smem) + cc * (NT * 128) + lane;
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -200,7 +283,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
                                        (a[2 * h + 1] >> 6) & 0x03030303u, v.z, v.w);
                         }
                     }
-                    load(ge, w[j]);
+                    load(w[j]);
                     if (++cc == nc) {
                         // the slice of this group is complete: its sums, two digits to a word, go to the CTA that finishes the group
                         const int li = grp - gb;
@@ -225,6 +308,19 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
                     }
                 }
             }
+            // a round may end inside the ring of registers: the next unit has to stand in front again
+#pragma unroll 1
+            for (; used < R && ge < g_end; --used) {
+                if (used == 0) break;
+                uint4 t[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    t[h] = w[0][h];
+#pragma unroll
+                    for (int j = 0; j + 1 < R; ++j) w[j][h] = w[j + 1][h];
+                    w[R - 1][h] = t[h];
+                }
+            }
         }
         const int nb = ge - gb, cnt = nb > rank ? (nb - rank + S - 1) >> lg_s : 0, per = M * MV_ROWS;
         if (S > 1) {
@@ -236,9 +332,12 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
         // two buffers: sums of the block after the next land here only after the barrier that follows these reads
         const unsigned char* src = mv_smem + p.xq_bytes + part;
         for (int i = threadIdx.x; i < cnt * per; i += MV_THREADS) {
-            const int slot = i / per, j = i - slot * per, m = j / MV_ROWS, o = (gb + (slot << lg_s) + rank) * MV_ROWS + (j & (MV_ROWS - 1));
+            const int slot = i / per, j = i - slot * per, m = j / MV_ROWS, f = gb + (slot << lg_s) + rank;
+            int k = mat;
+            while (LIST && k + 1 < p.n && f >= p.m[k + 1].first) ++k;
+            const int o = (f - p.m[k].first) * MV_ROWS + (j & (MV_ROWS - 1)), O = p.m[k].O;
             if (o >= O) continue;
-            const float sc = __ldg(p.scale + o);
+            const float sc = __ldg(p.m[k].scale + o);
             const size_t at = (size_t)(slot * Mp * MV_ROWS + j) * 8;
             double sum = 0.0;
 #pragma unroll 4
@@ -249,43 +348,68 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const MvParams 
                     const int2 u = *reinterpret_cast<const int2*>(src + s * part_bytes + at + MV_ROWS * 8);
                     t += ((double)u.x * 65536.0 + (double)u.y) * (1.0 / 1073741824.0);
                 }
-                sum += xscale[s][m] * t;
+                sum += xscale[seg & 1][s][m] * t;
             }
-            p.y[(size_t)m * O + o] = (float)((double)sc * sum);
+            p.m[k].y[(size_t)m * O + o] = (float)((double)sc * sum);
         }
     }
+    if (s_end < g_end) mat = p.m[mat].next;
+    s_begin = s_end;
+    }
+    if (S > 1 && first) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int NT, int R>
-cudaError_t mv_launch(MvParams p, int sm_count, size_t max_smem, int slot, bool follows, cudaStream_t stream) {
-    const int groups = (p.O + MV_ROWS - 1) / MV_ROWS, Mp = p.M == 1 ? 2 : p.M, NC = (p.I + MV_CHUNK - 1) / MV_CHUNK, S = 1 << p.log_s;
+template <int NT, int R, int CAP>
+cudaError_t mv_launch(MvTable<CAP>& p, int segments, int sm_count, size_t max_smem, int slot, bool follows, const cudaGraphNode_t* nodes, cudaStream_t stream) {
+    constexpr bool LIST = CAP > 1;
+    const int Mp = p.M == 1 ? 2 : p.M, S = 1 << p.log_s;
     const size_t group_bytes = (size_t)S * Mp * MV_ROWS * 8;
+    int nc = 1;
+    for (int i = 0; i < p.n; ++i) nc = std::max(nc, (mv_chunks(p.m[i].I) + S - 1) / S);
+    p.xq_bytes = nc * NT * 2048;
     // Clusters of 8 do not tile the GPCs: of sm_count / 8 the last ones share SMs with others, which then hold the whole launch up.
     // Seven eighths of the SMs (16 clusters of 8): 20 matrices of an 8B-scale model 88 -> 81 us for one row, 118 -> 106 for four, 181 -> 166
     // for eight with other work beside them (one row alone 164 -> 162); 12 clusters 84 and 204, 30 (two CTAs on every SM) 109 and 139: one
     // setting for all rows, which is not the best one for eight.
     int clusters = sm_count * 7 / 8 / S;
     if (clusters < 1) clusters = 1;
-    if (clusters > groups) clusters = groups;
-    p.groups_q = groups / clusters; p.groups_r = groups % clusters;
-    p.block = p.groups_q + (p.groups_r ? 1 : 0);
-    p.owned = (p.block + S - 1) / S;
-    p.xq_bytes = ((NC + S - 1) / S) * NT * 2048;
+    if (clusters > p.groups) clusters = p.groups;
+    p.groups_q = p.groups / clusters; p.groups_r = p.groups % clusters;
     const size_t budget = max_smem - 4096;
-    if ((size_t)p.xq_bytes + 2 * group_bytes > budget) return cudaErrorInvalidConfiguration;
+    const size_t room = p.xq_bytes < budget ? budget - p.xq_bytes : 0;
+    // Groups of a cluster at most (one segment: all of them have one length, and a share of the cost, rounded to whole chunks, has the
+    // starts of groups / clusters + 2 of them at most); with several segments there are several rounds.
+    const int most = !LIST ? p.groups_q + (p.groups_r ? 1 : 0) : segments == 1 ? p.groups / clusters + 2 : p.groups;
     int bufs = 1;
-    while (p.xq_bytes + bufs * p.owned * group_bytes > budget) { bufs = 2; p.owned = (p.owned + 1) / 2; p.block = p.owned * S; }
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(gemv_mma_kernel<NT, R>), slot, max_smem);
+    p.owned = (most + S - 1) / S;
+    if (segments > 1 || (size_t)p.owned * group_bytes > room) {
+        bufs = 2;
+        const int fit = (int)std::min((size_t)1 << 20, room / (2 * group_bytes));
+        p.owned = std::min(p.owned, std::max(fit, 1));
+    }
+    p.block = p.owned * S;
+    const size_t smem = p.xq_bytes + bufs * p.owned * group_bytes;
+    if (smem > max_smem - 4096) return cudaErrorInvalidConfiguration;
+    const void* kern = reinterpret_cast<const void*>(gemv_mma_kernel<NT, R, LIST>);
+    cudaError_t e = ensure_dynamic_smem(kern, LIST ? slot + 10 : slot, max_smem);
     if (e != cudaSuccess) return e;
+    if (nodes) {
+        void* args[] = {&p};
+        cudaKernelNodeParams kp = {};
+        kp.func = const_cast<void*>(kern);
+        kp.gridDim = dim3(clusters * S); kp.blockDim = dim3(MV_THREADS); kp.sharedMemBytes = (unsigned)smem;
+        kp.kernelParams = args;
+        return cudaGraphKernelNodeSetParams(nodes[0], &kp);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(clusters * S); cfg.blockDim = dim3(MV_THREADS); cfg.stream = stream;
-    cfg.dynamicSmemBytes = p.xq_bytes + bufs * p.owned * group_bytes;
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[2];
     int n = 0;
     if (S > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = S; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; ++n; }
     if (follows) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; ++n; }
     cfg.attrs = at; cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, gemv_mma_kernel<NT, R>, p);
+    return cudaLaunchKernelEx(&cfg, gemv_mma_kernel<NT, R, LIST>, p);
 }
 
 // The widest portable cluster: the fixed part of a call (digits of a slice, sums of an output) shrinks with the slice (20 matrices
@@ -305,17 +429,53 @@ bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_
     return (size_t)((NC + S - 1) / S) * ((M + 1) / 2) * 2048 + 2 * (size_t)S * (M == 1 ? 2 : M) * MV_ROWS * 8 + 4096 <= max_smem;
 }
 
-cudaError_t launch_ternary_gemv_mma(const float* x, const uint32_t* packed2, const float* scale, float* y, int M, int in_features,
-                                    int out_features, bool follows, int sm_count, size_t max_smem, cudaStream_t stream) {
-    MvParams p = {};
-    p.x = x; p.packed2 = packed2; p.scale = scale; p.y = y; p.M = M; p.I = in_features; p.O = out_features;
-    p.log_s = mv_log_s(in_features);
-    switch ((M + 1) / 2) {
-        case 1: return mv_launch<1, 4>(p, sm_count, max_smem, 26, follows, stream);
-        case 2: return mv_launch<2, 3>(p, sm_count, max_smem, 27, follows, stream);
-        case 3: return mv_launch<3, 2>(p, sm_count, max_smem, 28, follows, stream);
-        default: return mv_launch<4, 2>(p, sm_count, max_smem, 29, follows, stream);
+bool gemv_mma_joins(int first_in_features, int in_features) { return mv_chunks(in_features) >= 1 << mv_log_s(first_in_features); }
+
+namespace {
+template <int CAP>
+cudaError_t mv_list(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count, size_t max_smem,
+                    cudaStream_t stream) {
+    MvTable<CAP> p;
+    p.n = n; p.M = M; p.log_s = mv_log_s(items[0].in_features);
+    // one x after the other
+    bool taken[CAP] = {};
+    int k = 0, segments = 0;
+    long long groups = 0;
+    p.cost = 0;
+    for (int i = 0; i < n; ++i) {
+        if (taken[i]) continue;
+        const int begin = k;
+        for (int j = i; j < n; ++j) {
+            if (taken[j] || items[j].x != items[i].x || items[j].in_features != items[i].in_features) continue;
+            taken[j] = true;
+            const GemvItem& it = items[j];
+            MvMat& m = p.m[k++];
+            m.words = reinterpret_cast<const uint4*>(it.packed2); m.x = it.x; m.scale = it.scale; m.y = it.y;
+            m.I = it.in_features; m.O = it.out_features;
+            m.first = (int)groups; m.cost = p.cost;
+            const long long g = (it.out_features + (long long)MV_ROWS - 1) / MV_ROWS;
+            groups += g;
+            p.cost += g * (mv_chunks(m.I) + MV_GROUP_COST);
+        }
+        for (int j = begin; j < k; ++j) p.m[j].next = k;
+        ++segments;
     }
+    if (groups > 0x3fffffff) return cudaErrorInvalidValue;
+    p.groups = (int)groups;
+    switch ((M + 1) / 2) {
+        case 1: return mv_launch<1, 4, CAP>(p, segments, sm_count, max_smem, 26, follows, nodes, stream);
+        case 2: return mv_launch<2, 3, CAP>(p, segments, sm_count, max_smem, 27, follows, nodes, stream);
+        case 3: return mv_launch<3, 2, CAP>(p, segments, sm_count, max_smem, 28, follows, nodes, stream);
+        default: return mv_launch<4, 2, CAP>(p, segments, sm_count, max_smem, 29, follows, nodes, stream);
+    }
+}
+
+}  // namespace
+
+cudaError_t launch_ternary_gemv_mma(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count,
+                                    size_t max_smem, cudaStream_t stream) {
+    return n == 1 ? mv_list<1>(items, n, M, follows, nodes, sm_count, max_smem, stream)
+                  : mv_list<kGemvListCap>(items, n, M, follows, nodes, sm_count, max_smem, stream);
 }
 
 }  // namespace mcl

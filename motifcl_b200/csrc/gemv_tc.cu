@@ -3,20 +3,27 @@
 //
 // CUDA cores cannot keep up with 4 weights per byte (one multiply-add per weight and
 // activation row), so the contraction runs as integer MMA, exactly:
-//   * each activation row is scaled by a power of two to |x'| < 1 and written as four signed
-//     7-bit digits, x' = (q0 + q1/128 + q2/128^2 + q3/128^3) / 64, truncation error < 4e-9;
-//     digit d of row m is row 4m+d of an int8 matrix Xq [N, in] (N = 16, 32, 48 or 64);
-//   * a CTA streams a [128 rows x 256 weights] tile of packed 2-bit fields (f = t + 1) through
-//     TMA, four warps expand the fields to int8 in the K-major 128-byte-swizzle layout that
-//     tcgen05.mma reads, and one thread issues kind::i8 MMAs  acc[128, N] += F . Xq^T  into
-//     int32 accumulators in TMEM;
-//   * sum_k x t = sum_k x f - sum_k x, so a per-row digit sum is subtracted at the end.
-// Integer accumulation is exact and order-independent, which makes split-K over atomics
-// deterministic.  A finalize kernel recombines the digits in double precision.
-// A CTA takes half of an SM's shared memory and tensor memory (one accumulator, three expanded tiles): the 2.4 us before its first
-// tile and the waits of its chain pass under another launch's work.  4 blocks of an 8B-scale model, 16 rows: 239 -> 184 us beside
-// other work, 423 -> 382 us alone (two accumulators, four tiles and all of the shared memory before).
+//   * each activation row is scaled to whole numbers of 30 bits and sign below its largest magnitude and written as four signed
+//     digits of base 256; digit d of row m is row 4m+d of an int8 matrix Xq [N, in] (N = 16, 32, 48 or 64).  One row alone has
+//     digit rows to spare: its second four hold the 30 bits that the first leave over;
+//   * a CTA streams [RT * 128 rows x 256 weights] tiles of packed 2-bit fields (f = t + 1) through TMA, four warps per 128 rows expand
+//     the fields to int8 in TENSOR MEMORY, and one thread issues kind::i8 MMAs  acc[128, N] += F . Xq^T  with the A operand from there;
+//   * sum_k x t = sum_k x f - sum_k x, so a per-row digit sum is subtracted at the end; digits are put together in whole numbers.
+//
+// One launch takes a list of matrices.  Its k-blocks are numbered through, tile by tile, and every CTA takes the
+// same number of them in a row: nothing is left idle whatever the shapes are.  A tile that lies in one CTA is finished from tensor
+// memory; one that a cut runs through is added up by atomics (whole numbers: any order gives the same sum) in a slot of the
+// workspace, and the last CTA to arrive finishes it.  The launch before it writes the digits of every x once and clears slots and tickets; the
+// first weights are on their way meanwhile (programmatic dependent launch).
+//
+// What bounds it: an SM has to take 90 weights per clock at 6.5 TB/s (the copies alone run at 5.1 to 5.9 TB/s in these boxes).  20 matrices
+// of an 8B-scale model (210 MB) as one list take 60 us for one row of x, 66 for 8 and 80 for 16 (2.6 to 3.5 TB/s; 48, 54 and 68 with
+// other work beside them), where a launch or three per matrix took 157, 333 and 368.  MMAs issued from a single-lane branch cost 93 cycles
+// each whatever their N (62 us of an earlier 78 for one row); 64 digit columns bring 16 KB of digits beside 16 KB of words per
+// k-block, so two accumulators (RT = 2) share them: 16 rows 82 -> 80 us, one row 70 -> 60.
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "tc_ptx.cuh"
@@ -24,22 +31,28 @@
 namespace mcl {
 namespace {
 
-constexpr int GV_ROWS = 128;       // output rows per tile (UMMA M)
+constexpr int GV_ROWS = 128;       // rows of an accumulator (UMMA M)
 constexpr int GV_KB = 256;         // weights per k-block = 64 packed bytes per row
-constexpr int GV_RAW = GV_ROWS * (GV_KB / 4);          // 8 KiB staging of packed bytes
-
-constexpr int GV_THREADS = 320;
-constexpr int GV_MAX_STAGES = 12;      // slots of the raw ring (packed weights + activation digits)
-constexpr int GV_EXP = 3;              // expanded tiles in flight in tensor memory, 64 columns each
-constexpr int GV_ACOL0 = 64;           // after the accumulator; 256 columns in all, so that an SM holds two such CTAs
+constexpr int GV_RAW = GV_ROWS * (GV_KB / 4);          // 8 KiB of packed bytes
+constexpr int GV_MAX_STAGES = 8;       // slots of the raw ring (packed weights + activation digits)
 constexpr int GV_ACOLS = 64;           // a [128 rows x 256 int8] tile = 64 32-bit columns
+constexpr int GV_TMEM = 256;           // columns of a CTA, half of an SM's: accumulators (64 each), then expanded tiles
 
-struct GvParams {
-    int O, I, Nq;
-    int ncols;         // 4 * M: digit columns that carry data
-    int kblocks, kb_per_split, splits, stages;
-    int* acc;          // int32 [Nq][O]: column n of all rows contiguous, so a warp's 32 rows coalesce
+struct GvMat {
+    const float* scale;
+    float* y;
+    const int* corr;
+    const float* xscale;
+    int O, kblocks, x;
+    int first, tile;   // numbers of its first unit (k-block of a tile) and tile
+};
+struct GvTable {
+    int n, units, tiles, M, Nq, stages;
     int* err;
+    int* acc;          // slots of [RT][Nq][128] sums for tiles that a cut runs through, by tile or by the CTA that begins it, whichever are fewer
+    int* tickets;
+    GvMat m[kGemvListCap];
+    CUtensorMap maps[kGemvListCap], xmaps[kGemvXCap];
 };
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -57,20 +70,33 @@ __device__ __forceinline__ uint32_t idesc_i8(int m, int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// Expansion of one packed word (16 fields) into 16 bytes costs seven logic ops when output word i
-// takes the fields 4j + i (j = byte index): (w >> 2i) & 0x03030303.  That permutes k inside every
-// group of 16 (byte 4i + j of the group holds weight 4j + i); a contraction over k does not care as
-// long as the activation digits are stored in the same order, which gemv_quantize_kernel does.
-__device__ __forceinline__ int gv_kperm(int k) { return (k & ~15) | ((k & 3) << 2) | ((k >> 2) & 3); }
+// D += A.B, A in tensor memory, B's descriptor as low and high words
+__device__ __forceinline__ void umma_i8_tsu(uint32_t tmem_c, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accum) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], b, %4, p;\n\t}"
+                 ::"r"(tmem_c), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
+}
 
+// a CTA's units of one tile
+struct GvPart { int m, tile, kb0, nkb; };
+__device__ __forceinline__ GvPart gv_part(const GvTable& p, int u, int end, int m) {
+    while (m + 1 < p.n && u >= p.m[m + 1].first) ++m;
+    const int kbs = p.m[m].kblocks, local = u - p.m[m].first, tile = local / kbs, kb0 = local - tile * kbs;
+    return {m, tile, kb0, min(kbs - kb0, end - u)};
+}
+__device__ __forceinline__ int gv_cut(const GvTable& p, int cta) { return (int)((long long)p.units * cta / gridDim.x); }
+__device__ __forceinline__ int gv_cta_of(const GvTable& p, int u) { return (int)(((long long)(u + 1) * gridDim.x - 1) / p.units); }
 
-__global__ void __launch_bounds__(GV_THREADS, 2) gemv_tc_kernel(const __grid_constant__ CUtensorMap tmP,
-                                                             const __grid_constant__ CUtensorMap tmX,
-                                                             const GvParams p) {
+// RT: accumulators (128 rows each) of a tile, which share the digits that a k-block loads
+template <int RT>
+__global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid_constant__ GvTable p) {
+    constexpr int EXP = (GV_TMEM - 64 * RT) / GV_ACOLS;        // expanded tiles in flight in tensor memory
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * GV_EXP + 2];
+    __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * EXP + 2 * RT];
     __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, last_ticket;
+    __shared__ int4 corr[16];              // of the matrix at hand: digit sums of every row of x, and its scale
+    __shared__ double xscale[16];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = p.stages, Nq = p.Nq;
@@ -80,30 +106,27 @@ __global__ void __launch_bounds__(GV_THREADS, 2) gemv_tc_kernel(const __grid_con
     // expanded int8 weight tile is four times larger than its packed form; it is written to TENSOR MEMORY
     // (tcgen05.st, thread = row = TMEM lane) and the MMA takes its A operand from there, so neither the
     // expansion nor the operand fetch uses shared-memory bandwidth.
-    const uint32_t stage_bytes = GV_RAW + 2 * b_tile;
+    const uint32_t stage_bytes = RT * GV_RAW + 2 * b_tile;
     const uint32_t bar0 = smem_u32(bars);
     auto raw_full = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (GV_MAX_STAGES + s); };
     auto a_full = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + e); };
-    auto a_empty = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + GV_EXP + e); };
-    const uint32_t acc_full = bar0 + 8u * (2 * GV_MAX_STAGES + 2 * GV_EXP), acc_empty = acc_full + 8u;
-    // TMEM columns: [0, Nq) the accumulator, [a_col0, a_col0 + GV_EXP * 64) expanded tiles
-    const uint32_t a_col0 = GV_ACOL0;
-    const uint32_t tmem_cols = 256;
-
-    const int row_tiles = (p.O + GV_ROWS - 1) / GV_ROWS;
-    const int n_items = row_tiles * p.splits;
+    auto a_empty = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + EXP + e); };
+    auto acc_full = [&](int h) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * EXP + h); };
+    auto acc_empty = [&](int h) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * EXP + RT + h); };
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int u_begin = gv_cut(p, blockIdx.x), u_end = gv_cut(p, blockIdx.x + 1);
 
     if (threadIdx.x == 0) {
         abort_flag = (*reinterpret_cast<volatile int*>(p.err) != 0);
         for (int s = 0; s < S; ++s) { mbar_init(raw_full(s), 1); mbar_init(empty_bar(s), 1); }
-        for (int e = 0; e < GV_EXP; ++e) { mbar_init(a_full(e), 128); mbar_init(a_empty(e), 1); }
-        mbar_init(acc_full, 1); mbar_init(acc_empty, 128);
+        for (int e = 0; e < EXP; ++e) { mbar_init(a_full(e), 4); mbar_init(a_empty(e), 1); }
+        for (int h = 0; h < RT; ++h) { mbar_init(acc_full(h), 1); mbar_init(acc_empty(h), 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_slot)), "r"(tmem_cols) : "memory");
+                     ::"r"(smem_u32(&tmem_slot)), "r"(GV_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -113,131 +136,199 @@ __global__ void __launch_bounds__(GV_THREADS, 2) gemv_tc_kernel(const __grid_con
 
     if (warp == 0) {
         if (lane == 0) {
-            // ---- TMA producer: packed weight tile + the two activation-digit tiles of a k-block ----
-            uint32_t it = 0;
-            for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x) {
-                const int rt = item % row_tiles, split = item / row_tiles;
-                const int kb0 = split * p.kb_per_split;
-                const int nkb = min(p.kb_per_split, p.kblocks - kb0);
-                for (int j = 0; j < nkb; ++j, ++it) {
-                    const int s = (int)(it % (uint32_t)S);
-                    const uint32_t ph = (it / (uint32_t)S) & 1u;
-                    if (!mbar_wait(empty_bar(s), ph ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 11); break; }
-                    const uint32_t st = base + (uint32_t)s * stage_bytes;
-                    const int kb = kb0 + j;
-                    mbar_expect_tx(raw_full(s), GV_RAW + 2 * b_tile);
-                    tma_load_2d(st, &tmP, raw_full(s), kb * (GV_KB / 4), rt * GV_ROWS);
-                    tma_load_2d(st + GV_RAW, &tmX, raw_full(s), kb * GV_KB, 0);
-                    tma_load_2d(st + GV_RAW + b_tile, &tmX, raw_full(s), kb * GV_KB + 128, 0);
+            // ---- TMA producer: packed weights and the two digit tiles of a k-block.  The weights of the first slots do not
+            // wait for the kernel before this one, which writes the digits ----
+            bool waited = false;
+            int it = 0, m = 0;
+            int late[GV_MAX_STAGES], late_x[GV_MAX_STAGES];        // k-blocks whose digits are still to be asked for
+            auto digits = [&](int s, int x, int kb) {
+                const uint32_t st = base + (uint32_t)s * stage_bytes + RT * GV_RAW;
+                tma_load_2d(st, &p.xmaps[x], raw_full(s), kb * GV_KB, 0);
+                tma_load_2d(st + b_tile, &p.xmaps[x], raw_full(s), kb * GV_KB + 128, 0);
+            };
+            auto wait_before = [&] {
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+                for (int i = 0; i < it && i < S; ++i) digits(i, late_x[i], late[i]);
+                waited = true;
+            };
+            for (int u = u_begin; u < u_end && !abort_flag;) {
+                const GvPart t = gv_part(p, u, u_end, m);
+                m = t.m;
+                u += t.nkb;
+                const int x = p.m[m].x;
+                for (int j = 0; j < t.nkb; ++j, ++it) {
+                    const int s = it % S, kb = t.kb0 + j;
+                    if (it == S) wait_before();
+                    if (!mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 11); break; }
+                    mbar_expect_tx(raw_full(s), stage_bytes);
+                    tma_load_2d(base + (uint32_t)s * stage_bytes, &p.maps[m], raw_full(s), kb * (GV_KB / 4), t.tile * (RT * GV_ROWS));
+                    if (waited) digits(s, x, kb);
+                    else { late[s] = kb; late_x[s] = x; }
                 }
             }
+            if (!waited) wait_before();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer: 8 x (128 x Nq x 32) int8 MMAs per k-block ------------------------------
-            const uint32_t idesc = idesc_i8(GV_ROWS, Nq);
-            uint32_t it = 0, n_local = 0;
-            for (int item = blockIdx.x; item < n_items && !abort_flag; item += gridDim.x, ++n_local) {
-                const int split = item / row_tiles;
-                const int kb0 = split * p.kb_per_split;
-                const int nkb = min(p.kb_per_split, p.kblocks - kb0);
-                if (!mbar_wait(acc_empty, (n_local & 1u) ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 14); break; }
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base;
-                for (int j = 0; j < nkb; ++j, ++it) {
-                    const int s = (int)(it % (uint32_t)S);
-                    const int e = (int)(it % GV_EXP);
+        // ---- MMA issuer: RT x 8 x (128 x Nq x 32) int8 MMAs per k-block.  The whole warp runs the loop and one lane is elected around
+        // the instructions: descriptors are warp-uniform then (93 cycles an MMA from a single-lane branch, whatever its N) ----
+        const uint32_t idesc = idesc_i8(GV_ROWS, Nq);
+        const uint64_t db0 = smem_desc_k_sw128(base + RT * GV_RAW);
+        const uint32_t db_hi = (uint32_t)(db0 >> 32), db_lo = (uint32_t)db0, db_stage = stage_bytes >> 4, db_half = b_tile >> 4;
+        int it = 0, n_local = 0, m = 0, s = 0, e = 0;
+        uint32_t e_ph = 0;
+        bool ok = true;
+        for (int u = u_begin; u < u_end && ok; ++n_local) {
+            const GvPart t = gv_part(p, u, u_end, m);
+            m = t.m;
+            u += t.nkb;
+            for (int j = 0; j < t.nkb && ok; ++j, ++it) {
+#pragma unroll
+                for (int h = 0; h < RT; ++h) {
+                    if (j == 0 && !mbar_wait_all(acc_empty(h), (n_local & 1) ^ 1, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 14); ok = false; break; }
                     // the expanders arrive after they have seen the raw slot: this wait covers the digit tiles too
-                    if (!mbar_wait(a_full(e), (it / GV_EXP) & 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 12); break; }
+                    if (!mbar_wait_all(a_full(e), e_ph, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 12); ok = false; break; }
                     tc_fence_after();
-                    const uint32_t st = base + (uint32_t)s * stage_bytes;
-                    const uint32_t a_tm = tmem_base + a_col0 + (uint32_t)e * GV_ACOLS;
+                    const uint32_t a_tm = tmem_base + 64 * RT + (uint32_t)e * GV_ACOLS, d_tm = tmem_base + 64 * h, db = db_lo + (uint32_t)s * db_stage;
+                    if (elect_one()) {
+                        const uint32_t more = j != 0 ? 1u : 0u;
 #pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        const uint64_t db = smem_desc_k_sw128(st + GV_RAW + t * b_tile);
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)      // 32 int8 of k = 8 TMEM columns of A, 32 bytes (+2) of B
-                            umma_i8_ts(d_tmem, a_tm + (uint32_t)(t * 32 + kk * 8), db + 2u * kk, idesc, (j | t | kk) != 0 ? 1u : 0u);
+                        for (int i = 0; i < 8; ++i)             // 32 int8 of k = 8 TMEM columns of A, 32 bytes (+2) of B
+                            umma_i8_tsu(d_tm, a_tm + 8 * i, db + (i >> 2) * db_half + 2 * (i & 3), db_hi, idesc, i ? 1u : more);
+                        umma_commit(a_empty(e));
+                        if (h + 1 == RT) umma_commit(empty_bar(s));
+                        if (j + 1 == t.nkb) umma_commit(acc_full(h));
                     }
-                    umma_commit(a_empty(e));
-                    umma_commit(empty_bar(s));
+                    __syncwarp();
+                    if (++e == EXP) { e = 0; e_ph ^= 1u; }
                 }
-                if (abort_flag) break;
-                umma_commit(acc_full);
+                if (++s == S) s = 0;
             }
         }
-    } else if (warp < 6) {
+    } else if (warp < 2 + 4 * RT) {
         // ---- expanders: 2-bit fields -> int8, written to tensor memory; thread = tile row = TMEM lane ----
         // a warp may touch the TMEM lanes of its quarter (warp % 4) only: that quarter is its 32 tile rows
-        const int r = ((warp & 3) << 5) | lane;         // 0..127
+        const int h = (warp - 2) >> 2, r = ((warp & 3) << 5) | lane;         // 0..127
         const uint32_t rsw64 = (uint32_t)((r >> 1) & 3);
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        uint32_t it = 0;
-        bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const int split = item / row_tiles;
-            const int kb0 = split * p.kb_per_split;
-            const int nkb = min(p.kb_per_split, p.kblocks - kb0);
-            for (int j = 0; j < nkb; ++j, ++it) {
-                const int s = (int)(it % (uint32_t)S);
-                const uint32_t ph = (it / (uint32_t)S) & 1u;
-                const int e = (int)(it % GV_EXP);
-                if (abort_flag || !mbar_wait(raw_full(s), ph, &abort_flag) ||
-                    !mbar_wait(a_empty(e), ((it / GV_EXP) & 1u) ^ 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 13); ok = false; break; }
-                tc_fence_after();      // the MMAs that read this TMEM slot have completed (a_empty)
-                unsigned char* st = smem_raw + (base - smem_u32(smem_raw)) + (size_t)s * stage_bytes;
-                const uint4* raw = reinterpret_cast<const uint4*>(st + r * 64);
-                const uint32_t a_tm = tmem_base + lane_base + a_col0 + (uint32_t)e * GV_ACOLS;
+        for (int it = 0; it < u_end - u_begin; ++it) {
+            const int s = it % S, e = (it * RT + h) % EXP;
+            if (!mbar_wait_all(raw_full(s), (it / S) & 1, &abort_flag) ||
+                !mbar_wait_all(a_empty(e), (((it * RT + h) / EXP) & 1) ^ 1, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 13); break; }
+            tc_fence_after();      // the MMAs that read this TMEM slot have completed (a_empty)
+            const unsigned char* st = smem_raw + (base - smem_u32(smem_raw)) + (size_t)s * stage_bytes + h * GV_RAW;
+            const uint4* raw = reinterpret_cast<const uint4*>(st + r * 64);
+            const uint32_t a_tm = tmem_base + lane_base + 64 * RT + (uint32_t)e * GV_ACOLS;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {           // half a row: 32 packed bytes = 128 weights = 32 TMEM columns
-                    uint32_t v[32];
+            for (int half = 0; half < 2; ++half) {           // half a row: 32 packed bytes = 128 weights = 32 TMEM columns
+                uint32_t v[32];
 #pragma unroll
-                    for (int cc = 0; cc < 2; ++cc) {
-                        const int c = 2 * h + cc;
-                        const uint4 pk = raw[c ^ rsw64];    // staging was written with the 64-byte swizzle
-                        const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+                for (int cc = 0; cc < 2; ++cc) {
+                    const uint4 pk = raw[(2 * half + cc) ^ rsw64];    // staging was written with the 64-byte swizzle
+                    const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+                    // One packed word (16 fields) into 16 bytes costs seven logic operations when output word i takes the fields
+                    // 4j + i (j = byte index): (w >> 2i) & 0x03030303.  That permutes k inside every group of 16; the digits are
+                    // stored in the same order.
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {       // one word = 16 weights = four columns of int8
-                            v[cc * 16 + q * 4 + 0] = w[q] & 0x03030303u;
-                            v[cc * 16 + q * 4 + 1] = (w[q] >> 2) & 0x03030303u;
-                            v[cc * 16 + q * 4 + 2] = (w[q] >> 4) & 0x03030303u;
-                            v[cc * 16 + q * 4 + 3] = (w[q] >> 6) & 0x03030303u;
-                        }
+                    for (int q = 0; q < 4; ++q) {
+                        v[cc * 16 + q * 4 + 0] = w[q] & 0x03030303u;
+                        v[cc * 16 + q * 4 + 1] = (w[q] >> 2) & 0x03030303u;
+                        v[cc * 16 + q * 4 + 2] = (w[q] >> 4) & 0x03030303u;
+                        v[cc * 16 + q * 4 + 3] = (w[q] >> 6) & 0x03030303u;
                     }
-                    tmem_st32(a_tm + (uint32_t)(32 * h), v);
                 }
-                tmem_st_wait();
-                tc_fence_before();
-                mbar_arrive(a_full(e));
+                tmem_st32(a_tm + (uint32_t)(32 * half), v);
             }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(a_full(e));
         }
     } else {
-        // ---- epilogue warps: int32 accumulator -> global (atomic when k is split) ---------------
-        const int q = warp & 3;
-        uint32_t n_local = 0;
-        for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n_local) {
-            const int rt = item % row_tiles;
-            bool ok = !abort_flag;
-            if (ok && !mbar_wait(acc_full, n_local & 1u, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 15); ok = false; }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const int row = rt * GV_ROWS + q * 32 + lane;
-            int* dst = p.acc + row;
-            uint32_t v[4][16];                      // all of it, then the next item may have the accumulator
+        // ---- epilogue warps -------------------------------------------------------------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");       // digit sums, scales, cleared slots
+        const int q = warp & 3, M = p.M;
+        int n_local = 0, m = 0, x = 0;
+        bool ok = true;
+        for (int u = u_begin; u < u_end && ok; ++n_local) {
+            const GvPart t = gv_part(p, u, u_end, m);
+            m = t.m;
+            const GvMat& A = p.m[m];
+            u += t.nkb;
+            const bool whole = t.nkb == A.kblocks;
+            if (n_local == 0 || A.x != x) {
+                x = A.x;
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                const int i = threadIdx.x - (64 + 128 * RT);
+                if (i < Nq / 4) corr[i] = reinterpret_cast<const int4*>(A.corr)[i];
+                else if (i >= 32 && i < 32 + M) xscale[i - 32] = (double)A.xscale[i - 32];
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            }
+            // sixteen digit columns of a row: four rows of x
+            auto finish = [&](int row, int c16, const uint32_t* v, double sc) {
+                if (row >= A.O) return;
+                long long n[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (c * 16 < Nq) tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 16), v[c]);
-            tmem_ld_wait();
-            tc_fence_before();
-            mbar_arrive(acc_empty);
-            if (row < p.O) {
-                // columns at and beyond 4 M are padding of the digit matrix (all zero): nothing to add
+                for (int j = 0; j < 4; ++j) {
+                    const int4 c = corr[c16 * 4 + j];
+                    n[j] = ((long long)((int)v[4 * j] - c.x) * 256 + ((int)v[4 * j + 1] - c.y)) * 65536 +
+                           ((long long)((int)v[4 * j + 2] - c.z) * 256 + ((int)v[4 * j + 3] - c.w));
+                }
+                if (M == 1) {
+                    A.y[row] = (float)(sc * (xscale[0] * ((double)n[0] + (double)n[1] * (1.0 / 1073741824.0))));
+                } else {
 #pragma unroll
-                for (int c = 0; c < 64; ++c) {
-                    if (c >= p.ncols) break;
-                    if (p.splits == 1) dst[(size_t)c * p.O] = (int)v[c >> 4][c & 15];
-                    else atomicAdd(dst + (size_t)c * p.O, (int)v[c >> 4][c & 15]);
+                    for (int j = 0; j < 4; ++j)
+                        if (c16 * 4 + j < M) A.y[(size_t)(c16 * 4 + j) * A.O + row] = (float)(sc * (xscale[c16 * 4 + j] * (double)n[j]));
+                }
+            };
+            const int tile_u = A.first + t.tile * A.kblocks;
+            const int from = whole ? 0 : gv_cta_of(p, tile_u);
+            const int slot_i = p.tiles < (int)gridDim.x ? A.tile + t.tile : from;
+            int* slot = p.acc + (size_t)slot_i * (RT * Nq * GV_ROWS);
+#pragma unroll 1
+            for (int h = 0; h < RT && ok; ++h) {
+                ok = !abort_flag;
+                if (ok && !mbar_wait(acc_full(h), n_local & 1, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 15); ok = false; }
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const int lrow = q * 32 + lane, row = (t.tile * RT + h) * GV_ROWS + lrow;
+                const double sc = whole && row < A.O ? (double)A.scale[row] : 0.0;
+#pragma unroll 1
+                for (int c = 0; c < Nq / 16; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + 64 * h + 16 * c, v);
+                    tmem_ld_wait();
+                    if (whole) finish(row, c, v, sc);
+                    else if (row < A.O) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) atomicAdd(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow, (int)v[j]);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(h));
+            }
+            if (!ok || whole) continue;
+            // the last of the CTAs that share the tile finishes it
+            __threadfence();
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (threadIdx.x == 64 + 128 * RT) last_ticket = atomicAdd(p.tickets + slot_i, 1) == gv_cta_of(p, tile_u + A.kblocks - 1) - from;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (last_ticket) {
+                __threadfence();
+#pragma unroll 1
+                for (int h = 0; h < RT; ++h) {
+                    const int lrow = q * 32 + lane, row = (t.tile * RT + h) * GV_ROWS + lrow;
+                    const double sc = row < A.O ? (double)A.scale[row] : 0.0;
+                    int v[32];                     // half of the widest list in flight at once
+#pragma unroll 1
+                    for (int c = 0; c < Nq / 16; c += 2) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = c * 16 + j < Nq ? __ldcg(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow) : 0;
+                        finish(row, c, reinterpret_cast<const uint32_t*>(v), sc);
+                        if (c + 1 < Nq / 16) finish(row, c + 1, reinterpret_cast<const uint32_t*>(v) + 16, sc);
+                    }
                 }
             }
         }
@@ -250,74 +341,101 @@ __global__ void __launch_bounds__(GV_THREADS, 2) gemv_tc_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(GV_TMEM) : "memory");
     }
 }
 
-// ---- activation rows -> four int8 digit rows each, digit sums, power-of-two scale ---------------
-// grid = Nq / 4 blocks (one per activation row slot; slots >= M are written as zeros)
-__global__ void __launch_bounds__(256) gemv_quantize_kernel(const float* __restrict__ x, int M, int I,
-                                                            signed char* __restrict__ xq, int* __restrict__ corr,
-                                                            float* __restrict__ xscale, int4* __restrict__ acc_clear,
-                                                            long long clear_int4) {
-    __shared__ float red[256];
+__device__ __forceinline__ float4 gv_load_x(const float4* p) {       // never before the wait on the grid this one depends on
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+// ---- activation rows -> four int8 digit rows each, digit sums, power-of-two scale; slots and tickets of the contraction cleared ----
+// blocks: Nq / 4 per x (one per group of four digit rows; those without an activation row are written as zeros), then those that clear
+constexpr int GQ_THREADS = 512;
+struct GqTable {
+    int n, M, groups, I[kGemvXCap];
+    const float* x[kGemvXCap];
+    signed char* xq[kGemvXCap];
+    int* corr[kGemvXCap];
+    float* xscale[kGemvXCap];
+    int4* clear;
+    size_t clear_n;
+};
+__global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_constant__ GqTable p) {
+    __shared__ unsigned int top_s;
     __shared__ int isum[4];
-    const int m = blockIdx.x, tid = threadIdx.x;
-    if (blockIdx.y > 0) {
-        // the blocks of the other grid rows only zero the split-K accumulators of the contraction that follows
-        const long long nthr = (long long)gridDim.x * (gridDim.y - 1) * 256;
-        for (long long i = ((long long)(blockIdx.y - 1) * gridDim.x + blockIdx.x) * 256 + tid; i < clear_int4; i += nthr)
-            acc_clear[i] = make_int4(0, 0, 0, 0);
+    const int tid = threadIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int xi = blockIdx.x / p.groups;
+    if (xi >= p.n) {
+        const size_t nthr = (size_t)(gridDim.x - p.n * p.groups) * GQ_THREADS;
+        for (size_t i = (size_t)(blockIdx.x - p.n * p.groups) * GQ_THREADS + tid; i < p.clear_n; i += nthr) p.clear[i] = make_int4(0, 0, 0, 0);
         return;
     }
-    signed char* q0 = xq + (size_t)(4 * m) * I;
-    if (m >= M) {
-        for (int k = tid; k < I; k += 256) { q0[k] = 0; q0[I + k] = 0; q0[2 * (size_t)I + k] = 0; q0[3 * (size_t)I + k] = 0; }
+    const int slot = blockIdx.x - xi * p.groups, M = p.M, I = p.I[xi], row = M == 1 ? 0 : slot;
+    uint4* q = reinterpret_cast<uint4*>(p.xq[xi] + (size_t)(4 * slot) * I);
+    const int pitch = I >> 4;
+    if (slot >= (M == 1 ? 2 : M)) {
+        for (int i = tid; i < 4 * pitch; i += GQ_THREADS) q[i] = make_uint4(0, 0, 0, 0);
+        if (tid < 4) p.corr[xi][4 * slot + tid] = 0;
         return;
     }
-    const float* xr = x + (size_t)m * I;
-    float amax = 0.0f;
-    for (int k = tid; k < I; k += 256) amax = fmaxf(amax, fabsf(__ldg(xr + k)));
-    red[tid] = amax;
+    const float4* x = reinterpret_cast<const float4*>(p.x[xi] + (size_t)row * I);
+    if (tid == 0) top_s = 0u;
     if (tid < 4) isum[tid] = 0;
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (tid < s) red[tid] = fmaxf(red[tid], red[tid + s]);
-        __syncthreads();
+    unsigned int top = 0u;
+    for (int i = tid; i < I / 4; i += GQ_THREADS) {
+        const float4 v = gv_load_x(x + i);
+        top = max(max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), max(__float_as_uint(v.y) & 0x7FFFFFFFu, __float_as_uint(v.z) & 0x7FFFFFFFu)),
+                  __float_as_uint(v.w) & 0x7FFFFFFFu);
     }
-    amax = red[0];
-    int e = 0;
-    if (amax > 0.0f) frexpf(amax, &e);              // amax = f * 2^e, f in [0.5, 1): 2^e > amax
-    const float inv = ldexpf(64.0f, -e);            // x * inv = x' * 64 with |x'| < 1, exact scaling
-    int s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int k = tid; k < I; k += 256) {
-        float v = __ldg(xr + k) * inv;
-        const float d0 = rintf(v); v = (v - d0) * 128.0f;
-        const float d1 = rintf(v); v = (v - d1) * 128.0f;
-        const float d2 = rintf(v); v = (v - d2) * 128.0f;
-        const float d3 = rintf(v);
-        const int kp = gv_kperm(k);          // the order in which the expanded weights lie
-        q0[kp] = (signed char)d0; q0[I + kp] = (signed char)d1;
-        q0[2 * (size_t)I + kp] = (signed char)d2; q0[3 * (size_t)I + kp] = (signed char)d3;
-        s0 += (int)d0; s1 += (int)d1; s2 += (int)d2; s3 += (int)d3;
-    }
-    atomicAdd(&isum[0], s0); atomicAdd(&isum[1], s1); atomicAdd(&isum[2], s2); atomicAdd(&isum[3], s3);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((tid & 31) == 0) atomicMax(&top_s, top);
     __syncthreads();
-    if (tid < 4) corr[4 * m + tid] = isum[tid];
-    if (tid == 0) xscale[m] = ldexpf(1.0f, e) / 64.0f;
-}
-
-// y[m,o] = scale[o] * xscale[m] * sum_d 128^-d * (acc[o][4m+d] - corr[4m+d])
-__global__ void gemv_finalize_kernel(const int* __restrict__ acc, const int* __restrict__ corr,
-                                     const float* __restrict__ xscale, const float* __restrict__ scale,
-                                     float* __restrict__ y, int M, int O, int Nq) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-    if (o >= O) return;
-    const int a0 = __ldg(acc + (size_t)(4 * m + 0) * O + o), a1 = __ldg(acc + (size_t)(4 * m + 1) * O + o);
-    const int a2 = __ldg(acc + (size_t)(4 * m + 2) * O + o), a3 = __ldg(acc + (size_t)(4 * m + 3) * O + o);
-    const double sum = (double)(a0 - corr[4 * m]) + (double)(a1 - corr[4 * m + 1]) * (1.0 / 128.0) +
-                       (double)(a2 - corr[4 * m + 2]) * (1.0 / 16384.0) + (double)(a3 - corr[4 * m + 3]) * (1.0 / 2097152.0);
-    y[(size_t)m * O + o] = (float)((double)__ldg(scale + o) * (double)xscale[m] * sum);
+    top = top_s;
+    int e = max((int)(top >> 23) - 126, -90);       // 2^e above every magnitude (of the smallest ones: 2^-90)
+    if (top >= 0x7F800000u) e = 0;
+    const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
+    int sum[4] = {0, 0, 0, 0};
+    for (int g = tid; g < pitch; g += GQ_THREADS) {
+        uint32_t r[16];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = gv_load_x(x + 4 * g + j);
+            const float f[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                int n = __float2int_rn(f[a]);
+                // what the 30 bits leave over: nothing from 2^23 on, where f is a whole number itself
+                if (M == 1 && slot == 1) n = __float2int_rn((f[a] - (float)n) * 1073741824.0f);
+                r[4 * j + a] = ((uint32_t)n + 0x80808080u) ^ 0x80808080u;        // four signed bytes, base 256
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {                // byte 3 is the leading digit; word i of a digit row takes the elements 4 j + i
+            uint32_t o[4];
+            const uint32_t pick = (uint32_t)(3 - d) | ((uint32_t)(7 - d) << 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                o[i] = __byte_perm(__byte_perm(r[i], r[4 + i], pick), __byte_perm(r[8 + i], r[12 + i], pick), 0x5410);
+                sum[d] = __dp4a((int)o[i], 0x01010101, sum[d]);
+            }
+            q[(size_t)d * pitch + g] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        sum[d] = __reduce_add_sync(0xffffffffu, sum[d]);
+        if ((tid & 31) == 0) atomicAdd(&isum[d], sum[d]);
+    }
+    __syncthreads();
+    if (tid < 4) p.corr[xi][4 * slot + tid] = isum[tid];
+    if (tid == 0 && slot < M)       // an infinity or NaN: so is the row
+        p.xscale[xi][slot] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 + e - 30) << 23);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -348,86 +466,139 @@ bool gv_map_2d(CUtensorMap* map, const void* basep, size_t inner_bytes, size_t r
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+
+int gv_nq(int M) { return (4 * (M == 1 ? 2 : M) + 15) / 16 * 16; }
+size_t round_up(size_t n) { return (n + 1023) & ~size_t(1023); }
+constexpr size_t kGvCorr = 64 * sizeof(int);      // then up to 16 scales
+
 }  // namespace
 
-bool gemv_tc_supported(int M, int in_features, int out_features) {
-    return M >= 1 && M <= 16 && in_features % 64 == 0 && in_features >= 256 && out_features >= 1;
+bool gemv_tc_supported(int M, int in_features, const void* packed2) {
+    return M >= 1 && M <= 16 && in_features % 64 == 0 && in_features >= 256 && in_features <= (1 << 22) && reinterpret_cast<uintptr_t>(packed2) % 16 == 0;      // 32-bit sums of digits times fields
 }
 
-// workspace: Xq [64][in] int8 | corr [64] int | xscale [16] float | acc [Nq][out] int32
-size_t gemv_tc_workspace_bytes(int M, int in_features, int out_features) {
-    const int Nq = 16 * ((M + 3) / 4);
-    size_t o = ((size_t)64 * in_features + 1023) & ~size_t(1023);
-    o += 1024;
-    o += ((size_t)out_features * Nq * sizeof(int) + 1023) & ~size_t(1023);
-    return o;
+// tickets | a slot per CTA (two CTAs on every SM) | per x: Xq [Nq][in] int8, digit sums, scales
+size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count) {
+    size_t bytes = round_up(2 * sm_count * sizeof(int)) + (size_t)2 * sm_count * 2 * gv_nq(M) * GV_ROWS * sizeof(int);
+    int xs = 0;
+    for (int i = 0; i < n; ++i) {
+        bool known = false;
+        for (int j = 0; j < i; ++j) known = known || (items[j].x == items[i].x && items[j].in_features == items[i].in_features);
+        if (known) continue;
+        bytes += round_up((size_t)gv_nq(M) * items[i].in_features) + 1024;
+        ++xs;
+    }
+    return xs <= kGemvXCap ? bytes : ~size_t(0);
 }
 
-cudaError_t launch_ternary_gemv_tc(const float* x, const uint32_t* packed2, const float* scale, float* y, int M,
-                                   int in_features, int out_features, void* workspace, int* err_word, int sm_count,
-                                   size_t max_smem, cudaStream_t stream, int* launches) {
-    const int I = in_features, O = out_features;
-    const int Nq = 16 * ((M + 3) / 4);
+namespace {
+long long gv_blocks(const GemvItem* items, int n) {        // k-blocks of 128 rows
+    long long u = 0;
+    for (int i = 0; i < n; ++i) u += (items[i].out_features + (long long)GV_ROWS - 1) / GV_ROWS * ((items[i].in_features + GV_KB - 1) / GV_KB);
+    return u;
+}
+}  // namespace
+
+// Against gemv_mma.cu (M <= 8), by k-blocks: that one needs no second launch and starts 5 us earlier, this one takes eight rows as fast as one.
+// us as gemv_mma / gemv_tc: M = 1 w1 and w3 of 14336 x 4096 (3584 k-blocks) 21 / 26, all 20 matrices of 4 blocks (25600) 81 / 60; M = 4
+// 3584 k-blocks 26 / 27, 2100 27 / 21; M = 8 4096 x 4096 (512) 9.6 / 12.9, q, k, v (768) 16.1 / 15.8, 14336 x 4096 (1792) 24.6 / 19.8.
+bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count) {
+    return gv_blocks(items, n) >= (long long)sm_count * (M <= 2 ? 28 : M <= 4 ? 14 : 6);
+}
+
+cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
+                                   int* err_word, int sm_count, size_t max_smem, cudaStream_t stream) {
+    const int Nq = gv_nq(M);
+    // Two CTAs on every SM and tiles of 256 rows, or one and 128.  One row: 2100 k-blocks 22.6 and 20.8 us, 5760 26.8 and 35.0, 25600 60 and 118; 16
+    // rows, alone and with other work beside them: 5760 35 / 26.8 and 43 / 19.7, 25600 80 / 68 and 141 / 66.
+    const bool large = gv_blocks(items, n) >= (long long)sm_count * (M <= 8 ? 24 : 64);
+    const int RT = large ? 2 : 1;
     char* w = static_cast<char*>(workspace);
-    signed char* xq = reinterpret_cast<signed char*>(w);
-    size_t o = ((size_t)64 * I + 1023) & ~size_t(1023);
-    int* corr = reinterpret_cast<int*>(w + o);
-    float* xscale = reinterpret_cast<float*>(w + o + 512);
-    int* acc = reinterpret_cast<int*>(w + o + 1024);
-
-    GvParams p;
-    p.O = O; p.I = I; p.Nq = Nq; p.ncols = 4 * M;
-    p.kblocks = (I + GV_KB - 1) / GV_KB;
-    const int row_tiles = (O + GV_ROWS - 1) / GV_ROWS;
-    int splits = 1;
-    if (row_tiles < 2 * sm_count) {
-        splits = (2 * sm_count + row_tiles - 1) / row_tiles;     // two items per CTA: 184 us with three, 179 with two, 16 rows as above
-        if (splits > p.kblocks / 2) splits = p.kblocks / 2;
-        if (splits < 1) splits = 1;
+    GvTable p;
+    GqTable g;
+    p.n = n; p.M = M; p.Nq = Nq; p.err = err_word;
+    p.tickets = reinterpret_cast<int*>(w);
+    w += round_up(2 * sm_count * sizeof(int));
+    p.acc = reinterpret_cast<int*>(w);
+    w += (size_t)2 * sm_count * 2 * Nq * GV_ROWS * sizeof(int);
+    g.n = 0; g.M = M; g.groups = Nq / 4;
+    long long units = 0, tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        const GemvItem& it = items[i];
+        int x = 0;
+        while (x < g.n && (g.x[x] != it.x || g.I[x] != it.in_features)) ++x;
+        if (x == g.n) {
+            if (x == kGemvXCap) return cudaErrorInvalidValue;
+            ++g.n;
+            g.x[x] = it.x; g.I[x] = it.in_features;
+            g.xq[x] = reinterpret_cast<signed char*>(w);
+            w += round_up((size_t)Nq * it.in_features);
+            g.corr[x] = reinterpret_cast<int*>(w);
+            g.xscale[x] = reinterpret_cast<float*>(w + kGvCorr);
+            w += 1024;
+            if (!gv_map_2d(&p.xmaps[x], g.xq[x], it.in_features, Nq, it.in_features, 128, Nq, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
+        }
+        GvMat& m = p.m[i];
+        m.scale = it.scale; m.y = it.y; m.corr = g.corr[x]; m.xscale = g.xscale[x];
+        m.O = it.out_features; m.x = x;
+        m.kblocks = (it.in_features + GV_KB - 1) / GV_KB;
+        m.first = (int)units;
+        m.tile = (int)tiles;
+        const long long of = (it.out_features + (long long)RT * GV_ROWS - 1) / (RT * GV_ROWS);
+        tiles += of;
+        units += of * m.kblocks;
+        if (units > 0x3fffffff) return cudaErrorInvalidValue;
+        if (!gv_map_2d(&p.maps[i], it.packed2, (size_t)it.in_features / 4, it.out_features, (size_t)it.in_features / 4, GV_KB / 4, RT * GV_ROWS,
+                       CU_TENSOR_MAP_SWIZZLE_64B)) return cudaErrorInvalidValue;
     }
-    p.kb_per_split = (p.kblocks + splits - 1) / splits;
-    p.splits = splits = (p.kblocks + p.kb_per_split - 1) / p.kb_per_split;
-    p.acc = acc; p.err = err_word;
-    const size_t stage_bytes = (size_t)GV_RAW + 2 * (size_t)Nq * 128;
-    int stages = (int)((max_smem / 2 - 3072) / stage_bytes);
-    if (stages > GV_MAX_STAGES) stages = GV_MAX_STAGES;
-    if (stages < 2) return cudaErrorInvalidConfiguration;
-    p.stages = stages;
-
-    CUtensorMap mp, mx;
-    if (!gv_map_2d(&mp, packed2, (size_t)I / 4, (size_t)O, (size_t)I / 4, GV_KB / 4, GV_ROWS, CU_TENSOR_MAP_SWIZZLE_64B))
-        return cudaErrorInvalidValue;
-    if (!gv_map_2d(&mx, xq, (size_t)I, 64, (size_t)I, 128, Nq, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
-
-    // one launch quantizes the activations and, when k is split, zeroes the digit columns of the accumulators
-    // that carry data (O * 4 M ints: O is padded to a multiple of 4 by the 1 KiB rounding of the workspace)
-    const long long clear_int4 = splits > 1 ? ((long long)O * 4 * M + 3) / 4 : 0;
-    int clear_rows = 0;
-    if (clear_int4 > 0) {
-        clear_rows = (int)((clear_int4 + (long long)(Nq / 4) * 256 * 8 - 1) / ((long long)(Nq / 4) * 256 * 8));
-        if (clear_rows < 1) clear_rows = 1;
-        if (clear_rows > 64) clear_rows = 64;
+    p.units = (int)units; p.tiles = (int)tiles;
+    const size_t stage_bytes = (size_t)RT * GV_RAW + 2 * (size_t)Nq * 128;
+    p.stages = std::min(GV_MAX_STAGES, (int)((max_smem / 2 - 3072) / stage_bytes));
+    if (p.stages < 2) return cudaErrorInvalidConfiguration;
+    const size_t smem = p.stages * stage_bytes + 1024;
+    // One matrix of few tiles: no CTA has parts of two (4096 x 4096, 16 rows: 16.2 -> 13.1 us), and a tile is cut only where that saves more
+    // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).
+    int per = (large ? 2 : 1) * sm_count;
+    if (n == 1 && tiles <= sm_count) {
+        const int kbs = p.m[0].kblocks, cut = std::max(1, std::min(kbs / 2, (int)(sm_count / tiles)));
+        per = (int)tiles * (kbs - kbs / cut > 6 ? cut : 1);
     }
-    gemv_quantize_kernel<<<dim3(Nq / 4, 1 + clear_rows), 256, 0, stream>>>(x, M, I, xq, corr, xscale,
-                                                                           reinterpret_cast<int4*>(acc), clear_int4);
-    cudaError_t e = cudaGetLastError();
+    const int ctas = (int)std::min<long long>(per, units);
+    // the tickets stand before the slots: one range
+    g.clear = reinterpret_cast<int4*>(p.tickets);
+    g.clear_n = (round_up(2 * sm_count * sizeof(int)) + (size_t)std::min<long long>(ctas, tiles) * RT * Nq * GV_ROWS * sizeof(int)) / 16;
+    // whole clusters of 8: the first launch may stand in a node of gemv_mma.cu
+    const int q_blocks = (g.n * g.groups + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS)) + 7) / 8 * 8;
+
+    const void* kern = RT == 2 ? reinterpret_cast<const void*>(gemv_tc_kernel<2>) : reinterpret_cast<const void*>(gemv_tc_kernel<1>);
+    cudaError_t e = ensure_dynamic_smem(kern, RT == 2 ? 5 : 40, max_smem);
     if (e != cudaSuccess) return e;
-    ++*launches;
-    const size_t smem = (size_t)stages * stage_bytes + 1024;
-    e = ensure_dynamic_smem(reinterpret_cast<const void*>(gemv_tc_kernel), 5, max_smem);
-    if (e != cudaSuccess) return e;
-    int ctas = row_tiles * splits;
-    if (ctas > sm_count) ctas = sm_count;
-    gemv_tc_kernel<<<ctas, GV_THREADS, smem, stream>>>(mp, mx, p);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    ++*launches;
-    gemv_finalize_kernel<<<dim3((O + 255) / 256, M), 256, 0, stream>>>(acc, corr, xscale, scale, y, M, O, Nq);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    ++*launches;
-    return cudaSuccess;
+    cudaKernelNodeParams kp = {};
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    if (parts & 1) {
+        void* args[] = {&g};
+        kp.func = reinterpret_cast<void*>(gemv_quantize_kernel);
+        kp.gridDim = cfg.gridDim = dim3(q_blocks); kp.blockDim = cfg.blockDim = dim3(GQ_THREADS);
+        kp.kernelParams = args;
+        cfg.numAttrs = follows ? 1 : 0;
+        e = nodes ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : cudaLaunchKernelEx(&cfg, gemv_quantize_kernel, g);
+        if (e != cudaSuccess) return e;
+    }
+    if (parts & 2) {
+        void* args[] = {&p};
+        kp.func = const_cast<void*>(kern);
+        kp.gridDim = cfg.gridDim = dim3(ctas); kp.blockDim = cfg.blockDim = dim3(192 + 128 * RT);
+        kp.sharedMemBytes = (unsigned)smem; cfg.dynamicSmemBytes = smem;
+        kp.kernelParams = args;
+        cfg.numAttrs = 1;
+        e = nodes ? cudaGraphKernelNodeSetParams(nodes[1], &kp)
+                  : RT == 2 ? cudaLaunchKernelEx(&cfg, gemv_tc_kernel<2>, p) : cudaLaunchKernelEx(&cfg, gemv_tc_kernel<1>, p);
+    }
+    return e;
 }
-
 
 }  // namespace mcl

@@ -130,10 +130,29 @@ cudaError_t launch_ternary_gemv(const float* x, const uint32_t* packed2, const f
                                 int M, int in_features, int out_features, int sm_count,
                                 cudaStream_t stream);
 
-// gemv_mma.cu -- M <= 8 in one launch of integer MMAs; follows: the launch before this one on the stream is a launch of the same kernel
+// Decode GEMVs.  A launch takes a list of matrices, M rows of x each (the xs may be one or several).  In a recording, the nodes of a launch
+// can take a longer list instead (`nodes`).  follows: the launch before this one on the stream is one of these.
+constexpr int kGemvListCap = 48;       // the list is a kernel argument, in gemv_tc.cu with a tensor map for every matrix
+constexpr int kGemvXCap = 8;           // different xs of a list of gemv_tc.cu
+struct GemvItem {
+    const float* x;
+    const uint32_t* packed2;
+    const float* scale;
+    float* y;
+    int in_features, out_features;
+};
+// gemv_mma.cu -- M <= 8, one launch (one node) of integer mma.sync; clusters sized for the first matrix of the list
 bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem);
-cudaError_t launch_ternary_gemv_mma(const float* x, const uint32_t* packed2, const float* scale, float* y, int M, int in_features,
-                                    int out_features, bool follows, int sm_count, size_t max_smem, cudaStream_t stream);
+bool gemv_mma_joins(int first_in_features, int in_features);
+cudaError_t launch_ternary_gemv_mma(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count,
+                                    size_t max_smem, cudaStream_t stream);
+// gemv_tc.cu -- M <= 16, two launches (two nodes): digits, integer tcgen05.  parts: bit 0 the first launch, bit 1 the second; with `nodes`,
+// the parts whose node takes the list.
+bool gemv_tc_supported(int M, int in_features, const void* packed2);
+bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count);                    // against gemv_mma.cu
+size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count);      // ~0: more xs than a launch takes
+cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
+                                   int* err_word, int sm_count, size_t max_smem, cudaStream_t stream);
 
 // peer_reduce.cu -- one-shot sum of a small vector over the GPUs of a node (peer loads, bounded flag wait)
 constexpr int kPeerMaxWorld = 8;
@@ -147,13 +166,6 @@ struct PeerTable {
     int rank, world;
 };
 cudaError_t launch_peer_allreduce(const PeerTable& tab, size_t n, int parity, float* out, int* err_word, cudaStream_t stream);
-
-// gemv_tc.cu -- the same GEMV as integer tensor-core MMA on digit-split activations
-bool gemv_tc_supported(int M, int in_features, int out_features);
-size_t gemv_tc_workspace_bytes(int M, int in_features, int out_features);
-cudaError_t launch_ternary_gemv_tc(const float* x, const uint32_t* packed2, const float* scale, float* y, int M,
-                                   int in_features, int out_features, void* workspace, int* err_word, int sm_count,
-                                   size_t max_smem, cudaStream_t stream, int* launches);
 
 // eltwise.cu: op 0 add, 1 sub, 2 mul, 3 mul_scalar, 4 add_scalar, 5 zero, 6 a - alpha*b
 cudaError_t launch_eltwise_f32(int op, const float* a, const float* b, float* out, size_t n, float alpha,

@@ -1,4 +1,4 @@
-"""Ternary GEMV of up to eight activation rows: clusters that split a row's chunks, 32-row units, recorded chains."""
+"""Ternary GEMV: clusters that split a row's chunks, 32-row units, tiles cut between CTAs, recorded chains and lists."""
 import numpy as np
 import pytest
 
@@ -22,8 +22,8 @@ def _context():
         return stream, Context.on_torch_stream(0)
 
 
-@pytest.mark.parametrize("M", [1, 2, 3, 5, 6, 7, 8])
-@pytest.mark.parametrize("O,I", [(1, 64), (31, 256), (33, 320), (130, 1984), (257, 2112), (600, 14336), (9000, 512), (20001, 768)])
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 6, 7, 8, 9, 13, 16])
+@pytest.mark.parametrize("O,I", [(1, 64), (31, 256), (33, 320), (130, 1984), (257, 2112), (600, 14336), (9000, 512), (20001, 768), (128, 256), (129, 28672)])
 def test_edges_of_chunks_units_and_clusters(M, O, I):
     rng = np.random.default_rng(O * 31 + I + M)
     w, digits, scale = _matrix(rng, O, I)
@@ -102,3 +102,75 @@ def test_lane_recorded_again_reads_words_made_just_before():
             batch.close()
             assert float((y.double() - want).norm() / want.norm()) <= 1e-6
         lane.close()
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 6, 8, 9, 16])
+@pytest.mark.parametrize("shapes", [
+    [(196, 256), (133, 256), (1025, 256)],                                    # clusters of one
+    [(4096, 2048), (131, 2048), (6000, 14336), (257, 2112), (4096, 2048)],     # several lengths in clusters of eight
+    [(9000, 512), (640, 4096), (177, 512), (640, 4096), (130, 1024)],         # clusters of 2, 4 and 8: three launches
+    [(140, 320)] * 70,                                                        # more than one launch holds
+])
+def test_independent_matrices_of_a_recording_share_launches(M, shapes):
+    """As one launch each, whatever shares a launch: two xs per length, rounds that end inside a matrix and a ring, cut tiles.  The sums
+    are whole numbers; two kernels may round them differently (2^-24 each) and differ in what digits of 30 bits lose (2^-31 of the
+    largest activation)."""
+    rng = np.random.default_rng(M * 100 + len(shapes))
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        xs = {(I, h): torch.from_numpy(rng.standard_normal((M, I)).astype(np.float32)).to(DEV) for _, I in shapes for h in (0, 1)}
+        mats = [_matrix(rng, O, I)[::2] for O, I in shapes]
+        mats = [(w, torch.from_numpy(s).to(DEV)) for w, s in mats]
+        ys, single = [[torch.full((M, O), 5.0, device=DEV) for O, _ in shapes] for _ in range(2)]
+
+        def sweep(out):
+            for i, ((O, I), (w, s)) in enumerate(zip(shapes, mats)):
+                ctx.ternary_gemv(xs[I, i & 1], w, s, out[i], M, I, O)
+        sweep(single)
+        ctx.finish()
+        before = ctx.launch_count
+        ctx.batch_begin()
+        sweep(ys)
+        batch = ctx.batch_end()
+        batch.launch()
+        ctx.finish()
+        assert ctx.launch_count - before < len(shapes)
+        batch.close()
+    for a, b in zip(ys, single):
+        assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2 * 2.0 ** -24 + 2.0 ** -26
+        assert M <= 8 or torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,per", [(2, 1), (12, 2)])
+def test_recorded_matrices_that_depend_on_one_another_keep_their_order(M, per):
+    """Products of one x share a launch; what reads their results, overwrites them or stands behind another kernel does not join it."""
+    rng = np.random.default_rng(3)
+    D, H = 2048, 4096
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        x, a, b, c = [torch.from_numpy(rng.standard_normal((M, n)).astype(np.float32)).to(DEV) for n in (D, H, D, D)]
+        up, down, square = [(lambda w, s: (w, torch.from_numpy(s * 0.02).to(DEV)))(*_matrix(rng, *s)[::2]) for s in ((H, D), (D, H), (D, D))]
+
+        def calls():
+            ctx.ternary_gemv(x, *up, a, M, D, H)
+            ctx.ternary_gemv(x, *square, b, M, D, D)         # beside the first
+            ctx.ternary_gemv(a, *down, c, M, H, D)           # reads the first
+            ctx.ternary_gemv(c, *up, a, M, D, H)             # reads the third and overwrites what it read
+            ctx.ternary_gemv(x, *square, c, M, D, D)         # overwrites what the fourth read
+            ctx.eltwise(0, c, b, c, M * D)                   # c += b
+            ctx.ternary_gemv(c, *square, b, M, D, D)
+            ctx.ternary_gemv(x, *square, c, M, D, D)         # overwrites what the launch before it reads
+        calls()
+        want = [t.clone() for t in (a, b, c)]
+        ctx.finish()
+        before = ctx.launch_count
+        ctx.batch_begin()
+        calls()
+        batch = ctx.batch_end()
+        for _ in range(3):
+            batch.launch()
+        ctx.finish()
+        assert (ctx.launch_count - before) == 3 * (6 * per + 1)
+        for t, w in zip((a, b, c), want):
+            assert torch.equal(t, w)
+        batch.close()
