@@ -50,6 +50,8 @@ constexpr int kTailRow = 2 * kTailK + 1;
 template <bool WITH_Q>
 __global__ void __launch_bounds__(kUpdThreads, 3)
 counter_update_dense_kernel(const UpdParams p) {
+    grid_release();
+    grid_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int I = p.in_features;
     const int gpr = I >> 2;
@@ -374,6 +376,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
 template <bool WITH_Q>
 __global__ void __launch_bounds__(kWsThreads, 1)
 counter_update_ws_kernel(const UpdParams p, const uint32_t pow16, const uint32_t pow17, const int nslots, int* err) {
+    grid_release();
+    grid_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     const int I = p.in_features;
     const int gpr = I >> 2, upr = I >> 4, row_bytes = gpr * 3;
@@ -548,6 +552,8 @@ counter_update_ws_kernel(const UpdParams p, const uint32_t pow16, const uint32_t
 template <bool WITH_Q>
 __global__ void __launch_bounds__(kUpdThreads, kUpdCtasPerSm)
 counter_update_u16_kernel(const UpdParams p, const uint32_t unit_magic, const uint32_t pow16, const uint32_t pow17) {
+    grid_release();
+    grid_wait();
     update_u16_body<WITH_Q>(p, unit_magic, pow16, pow17, blockIdx.x, gridDim.x, true);
 }
 
@@ -562,6 +568,8 @@ struct UpdGroup {
 template <bool WITH_Q>
 __global__ void __launch_bounds__(kUpdThreads, kUpdCtasPerSm)
 counter_update_u16_group_kernel(const __grid_constant__ UpdGroup g, const uint32_t pow16, const uint32_t pow17) {
+    grid_release();
+    grid_wait();
     const int grid = (int)gridDim.x, b = (int)blockIdx.x;
     int built_c = -1;
     for (int j = 0; j < g.n; ++j) {
@@ -670,8 +678,7 @@ cudaError_t launch_counter_update_dense(uint8_t* state, float* scale, float* v, 
             cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), with_q ? 10 : 11, max_smem);
             if (e != cudaSuccess) return e;
             const int grid = rows < sm_count ? rows : sm_count;
-            kern<<<grid, kWsThreads, L.total, stream>>>(p, 1u << 16, 1u << 17, L.nslots, err_word);
-            return cudaGetLastError();
+            return launch_chained(kern, dim3(grid), dim3(kWsThreads), L.total, stream, p, 1u << 16, 1u << 17, L.nslots, err_word);
         }
     }
     if (in_features % 16 == 0 && sp0 % 4 == 0) {
@@ -699,8 +706,7 @@ cudaError_t launch_counter_update_dense(uint8_t* state, float* scale, float* v, 
             auto kern = with_q ? counter_update_u16_kernel<true> : counter_update_u16_kernel<false>;
             cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), with_q ? 2 : 3, max_smem);
             if (e != cudaSuccess) return e;
-            kern<<<grid, kUpdThreads, L.total, stream>>>(p, magic, 1u << 16, 1u << 17);
-            return cudaGetLastError();
+            return launch_chained(kern, dim3(grid), dim3(kUpdThreads), L.total, stream, p, magic, 1u << 16, 1u << 17);
         }
     }
     int R = kMaxRowsPerBatch;
@@ -724,8 +730,7 @@ cudaError_t launch_counter_update_dense(uint8_t* state, float* scale, float* v, 
     auto kern = with_q ? counter_update_dense_kernel<true> : counter_update_dense_kernel<false>;
     cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), with_q ? 0 : 1, max_smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kUpdThreads, smem, stream>>>(p);
-    return cudaGetLastError();
+    return launch_chained(kern, dim3(grid), dim3(kUpdThreads), smem, stream, p);
 }
 
 static cudaError_t launch_update_group_narrow(const UpdateDesc* d, int n, int C, float lr, float lr_scale, float rms_beta,
@@ -811,8 +816,7 @@ static cudaError_t launch_update_group_narrow(const UpdateDesc* d, int n, int C,
             auto kern = with_q ? counter_update_u16_group_kernel<true> : counter_update_u16_group_kernel<false>;
             cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), with_q ? 8 : 9, max_smem);
             if (e != cudaSuccess) return e;
-            kern<<<grid, kUpdThreads, smem, stream>>>(g, 1u << 16, 1u << 17);
-            e = cudaGetLastError();
+            e = launch_chained(kern, dim3(grid), dim3(kUpdThreads), smem, stream, g, 1u << 16, 1u << 17);
             if (e != cudaSuccess) return e;
             ++*launches;
         }

@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
     if (threadIdx.x < 8) amax[threadIdx.x] = 0u;
     if (threadIdx.x < NT * 8) corr[threadIdx.x] = 0;
     if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // only "this CTA runs": nothing to publish
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_release();
+    grid_wait();
     const uint32_t part0 = (uint32_t)__cvta_generic_to_shared(mv_smem) + (uint32_t)p.xq_bytes;
     const uint32_t part_bytes = (uint32_t)(p.owned * Mp) * (MV_ROWS * 8u);      // one slice's sums for the groups a CTA finishes
     int parity = 0;

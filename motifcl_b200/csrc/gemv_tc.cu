@@ -114,7 +114,6 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
     auto a_empty = [&](int e) { return bar0 + 8u * (2 * GV_MAX_STAGES + EXP + e); };
     auto acc_full = [&](int h) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * EXP + h); };
     auto acc_empty = [&](int h) { return bar0 + 8u * (2 * GV_MAX_STAGES + 2 * EXP + RT + h); };
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int u_begin = gv_cut(p, blockIdx.x), u_end = gv_cut(p, blockIdx.x + 1);
 
     if (threadIdx.x == 0) {
@@ -131,6 +130,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
     }
     tc_fence_before();
     __syncthreads();
+    grid_release();
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
 
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 tma_load_2d(st + b_tile, &p.xmaps[x], raw_full(s), kb * GV_KB + 128, 0);
             };
             auto wait_before = [&] {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
+                grid_wait();
                 for (int i = 0; i < it && i < S; ++i) digits(i, late_x[i], late[i]);
                 waited = true;
             };
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         }
     } else {
         // ---- epilogue warps -------------------------------------------------------------------
-        asm volatile("griddepcontrol.wait;" ::: "memory");       // digit sums, scales, cleared slots
+        grid_wait();       // digit sums, scales, cleared slots
         const int q = warp & 3, M = p.M;
         int n_local = 0, m = 0, x = 0;
         bool ok = true;
@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
     __shared__ unsigned int top_s;
     __shared__ int isum[4];
     const int tid = threadIdx.x;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_release();
+    grid_wait();
     const int xi = blockIdx.x / p.groups;
     if (xi >= p.n) {
         const size_t nthr = (size_t)(gridDim.x - p.n * p.groups) * GQ_THREADS;

@@ -185,12 +185,14 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
         }
     };
     Regs r0, r1;
-    load(0, r0);
-    if (nkt > 1) load(1, r1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_release();
     for (int e = tid; e < 4096; e += kLThreads) lut[e] = digit[e & 63] | (digit[e >> 6] << 16);
+    grid_wait();
+    load(0, r0);
+    if (nkt > 1) load(1, r1);
     __syncthreads();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16(128, BN, 0, DX ? 1u : 0u);
@@ -400,18 +402,22 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
         if (u.packed2) u.packed2 += (size_t)row * (I >> 4);
         u.rows = my_rows; u.row_offset = row;
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    grid_release();
     if (U16 && my_rows > 0) {                     // what the update needs beside the gradient is in place before it
         build_decode_lut(reinterpret_cast<DecodeLut*>(smem), u.C, tid, kLThreads);
         build_tick_table(reinterpret_cast<uint32_t*>(smem + L.off_tick), u.C, tid, kLThreads);
+    }
+    grid_wait();
+    if (U16 && my_rows > 0) {
         u16_load_state<kLThreads>(u, L, smem, 0, my_rows);
         if (tid < my_rows) {
             asm volatile("prefetch.global.L2 [%0];" ::"l"(u.scale + tid));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(u.v + tid));
         }
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const uint32_t tmem = tmem_slot;
     bool ok = true;
     int it = 0;                                   // k-tiles so far: stage = it & 1
@@ -635,9 +641,7 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
     cudaError_t e = ensure_dynamic_smem(kern, dx ? 18 : 17, max_smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)tm, (unsigned)((p.N + p.BN - 1) / p.BN));
-    if (dx) layer_rows_kernel<true><<<grid, kLThreads, smem, stream>>>(p);
-    else layer_rows_kernel<false><<<grid, kLThreads, smem, stream>>>(p);
-    return cudaGetLastError();
+    return launch_chained(dx ? layer_rows_kernel<true> : layer_rows_kernel<false>, grid, dim3(kLThreads), smem, stream, p);
 }
 
 cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
@@ -690,11 +694,13 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
         cfg.blockDim = dim3(kLThreads);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // launch_chained, with clusters
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         return cudaLaunchKernelEx(&cfg, kern, p);
     }
 }

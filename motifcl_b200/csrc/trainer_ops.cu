@@ -71,6 +71,8 @@ template <int H>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                       float* __restrict__ out, float* __restrict__ row_inv,
                                                       size_t rows, Vec4 a, float eps) {
+    grid_release();
+    grid_wait();
     const int lane = threadIdx.x & 31, cols = a.cols;
     for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (size_t)gridDim.x * 8) {
         const float* xr = x + row * (size_t)cols;
@@ -105,6 +107,8 @@ template <int H>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                             const float* __restrict__ dy, float* __restrict__ dx,
                                                             size_t rows, Vec4 a, float eps) {
+    grid_release();
+    grid_wait();
     const int lane = threadIdx.x & 31, cols = a.cols;
     for (size_t row = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (size_t)gridDim.x * 8) {
         const float* xr = x + row * (size_t)cols;
@@ -142,6 +146,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* __restr
 template <int H>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                                                                  float* __restrict__ row_inv, float* __restrict__ dw, size_t rows, Vec4 a, float eps) {
+    grid_release();
+    grid_wait();
     __shared__ float4 part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cols = a.cols;
     float4 acc[H];
@@ -186,6 +192,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* __
 __global__ void __launch_bounds__(256) rmsnorm_bwd_w_kernel(const float* __restrict__ x, const float* __restrict__ dy,
                                                             const float* __restrict__ row_inv, float* __restrict__ dw,
                                                             size_t rows, int cols, size_t rows_per_block) {
+    grid_release();
+    grid_wait();
     __shared__ float part[8][33];
     const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + cx;
@@ -214,6 +222,8 @@ __device__ __forceinline__ void swiglu_grads(float gate, float up, float go, flo
 template <int W>
 __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ packed, float* __restrict__ out,
                                                      size_t rows, int hidden) {
+    grid_release();
+    grid_wait();
     const int hw = hidden / W;
     const size_t n = rows * (size_t)hw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -233,6 +243,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ p
 template <int W>
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* __restrict__ packed, const float* __restrict__ dy,
                                                          float* __restrict__ dpacked, size_t rows, int hidden) {
+    grid_release();
+    grid_wait();
     const int hw = hidden / W;
     const size_t n = rows * (size_t)hw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -268,6 +280,8 @@ template <bool BACKWARD>
 __global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict__ logits, const int* __restrict__ targets,
                                                         float* __restrict__ partial, const float* __restrict__ grad_out,
                                                         float* __restrict__ grad_logits, size_t rows, int cols, int vec) {
+    grid_release();
+    grid_wait();
     __shared__ float red[32];
     const float gscale = BACKWARD ? grad_out[0] / (float)rows : 0.0f;
     const int n4 = vec ? cols >> 2 : 0;            // 128-bit part; vec: rows start on 16-byte boundaries
@@ -309,6 +323,8 @@ __global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict_
 }
 __global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n,
                                                    size_t denom) {
+    grid_release();
+    grid_wait();
     __shared__ float red[32];
     float s = 0.0f;
 #pragma unroll 4
@@ -522,6 +538,8 @@ __global__ void __launch_bounds__(256) position_backward_kernel(const float* __r
 __global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
                                                    int channels, int n_head, int head_dim, int rotary_dim, int token_offset,
                                                    float theta, int inverse, int split_half, int shared_turns) {
+    grid_release();
+    grid_wait();
     extern __shared__ float2 rot[];                   // (cos, sin) of pair i
     int rd = rotary_dim <= 0 ? head_dim : rotary_dim;
     rd = rd < head_dim ? rd : head_dim;
@@ -591,6 +609,8 @@ __global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, 
 constexpr int kRopeIn = 4;             // quads of a thread in flight
 __global__ void __launch_bounds__(256) rope_quads_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
                                                          int channels, int head_dim, int rd, int token_offset, float theta, int inverse) {
+    grid_release();
+    grid_wait();
     extern __shared__ float2 rot[];                   // (cos, sin) of pair i
     const int token = blockIdx.x, quads = channels >> 2;
     const int per = (batch + (int)gridDim.y - 1) / (int)gridDim.y, b0 = (int)blockIdx.y * per, n = (min(batch, b0 + per) - b0) * quads;
@@ -664,15 +684,15 @@ int warp_row_grid(size_t rows, int sm_count) {
 cudaError_t launch_rmsnorm(const float* x, const float* w, float* out, size_t rows, int cols, float eps, int sm_count,
                            cudaStream_t stream) {
     const Vec4 a = {cols % 4 == 0 && all16(x, w, out), cols};
-    if (cols <= 384) rmsnorm_kernel<3><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, out, nullptr, rows, a, eps);
-    else rmsnorm_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, out, nullptr, rows, a, eps);
+    if (cols <= 384) launch_chained(rmsnorm_kernel<3>, dim3(warp_row_grid(rows, sm_count)), dim3(256), 0, stream, x, w, out, nullptr, rows, a, eps);
+    else launch_chained(rmsnorm_kernel<kNormHold>, dim3(warp_row_grid(rows, sm_count)), dim3(256), 0, stream, x, w, out, nullptr, rows, a, eps);
     return cudaGetLastError();
 }
 cudaError_t launch_rmsnorm_backward_x(const float* x, const float* w, const float* dy, float* dx, size_t rows, int cols,
                                       float eps, int sm_count, cudaStream_t stream) {
     const Vec4 a = {cols % 4 == 0 && all16(x, w, dy, dx), cols};
-    if (cols <= 384) rmsnorm_bwd_x_kernel<3><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, dy, dx, rows, a, eps);
-    else rmsnorm_bwd_x_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, w, dy, dx, rows, a, eps);
+    if (cols <= 384) launch_chained(rmsnorm_bwd_x_kernel<3>, dim3(warp_row_grid(rows, sm_count)), dim3(256), 0, stream, x, w, dy, dx, rows, a, eps);
+    else launch_chained(rmsnorm_bwd_x_kernel<kNormHold>, dim3(warp_row_grid(rows, sm_count)), dim3(256), 0, stream, x, w, dy, dx, rows, a, eps);
     return cudaGetLastError();
 }
 cudaError_t launch_rmsnorm_backward_weight(const float* x, const float* dy, float* row_inv, float* dw, size_t rows,
@@ -683,11 +703,11 @@ cudaError_t launch_rmsnorm_backward_weight(const float* x, const float* dy, floa
     if (cols <= kNormHold * 128) {
         const size_t b = (rows + 7) / 8, cap = 2 * (size_t)sm_count;      // every block ends in one atomic per column
         const int grid = (int)(b < cap ? b : cap);
-        if (cols <= 384) rmsnorm_bwd_w_rows_kernel<3><<<grid, 256, 0, stream>>>(x, dy, row_inv, dw, rows, a, eps);
-        else rmsnorm_bwd_w_rows_kernel<kNormHold><<<grid, 256, 0, stream>>>(x, dy, row_inv, dw, rows, a, eps);
+        if (cols <= 384) launch_chained(rmsnorm_bwd_w_rows_kernel<3>, dim3((unsigned)grid), dim3(256), 0, stream, x, dy, row_inv, dw, rows, a, eps);
+        else launch_chained(rmsnorm_bwd_w_rows_kernel<kNormHold>, dim3((unsigned)grid), dim3(256), 0, stream, x, dy, row_inv, dw, rows, a, eps);
         return cudaGetLastError();
     }
-    rmsnorm_kernel<kNormHold><<<warp_row_grid(rows, sm_count), 256, 0, stream>>>(x, nullptr, nullptr, row_inv, rows, a, eps);
+    launch_chained(rmsnorm_kernel<kNormHold>, dim3(warp_row_grid(rows, sm_count)), dim3(256), 0, stream, x, nullptr, nullptr, row_inv, rows, a, eps);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int col_blocks = (cols + 31) / 32;
@@ -695,37 +715,34 @@ cudaError_t launch_rmsnorm_backward_weight(const float* x, const float* dy, floa
     if (splits > (rows + 63) / 64) splits = (rows + 63) / 64;
     if (splits < 1) splits = 1;
     const size_t rows_per_block = (rows + splits - 1) / splits;
-    rmsnorm_bwd_w_kernel<<<dim3(col_blocks, (unsigned)splits), 256, 0, stream>>>(x, dy, row_inv, dw, rows, cols,
-                                                                                 rows_per_block);
+    launch_chained(rmsnorm_bwd_w_kernel, dim3(col_blocks, (unsigned)splits), dim3(256), 0, stream, x, dy, row_inv, dw, rows, cols, rows_per_block);
     return cudaGetLastError();
 }
 cudaError_t launch_swiglu(const float* packed, float* out, size_t rows, int hidden, int sm_count, cudaStream_t stream) {
     const size_t n = rows * (size_t)hidden;
-    if (hidden % 4 == 0 && all16(packed, out)) swiglu_kernel<4><<<flat_grid(n / 4, sm_count), 256, 0, stream>>>(packed, out, rows, hidden);
-    else swiglu_kernel<1><<<flat_grid(n, sm_count), 256, 0, stream>>>(packed, out, rows, hidden);
+    if (hidden % 4 == 0 && all16(packed, out)) launch_chained(swiglu_kernel<4>, dim3(flat_grid(n / 4, sm_count)), dim3(256), 0, stream, packed, out, rows, hidden);
+    else launch_chained(swiglu_kernel<1>, dim3(flat_grid(n, sm_count)), dim3(256), 0, stream, packed, out, rows, hidden);
     return cudaGetLastError();
 }
 cudaError_t launch_swiglu_backward(const float* packed, const float* dy, float* dpacked, size_t rows, int hidden,
                                    int sm_count, cudaStream_t stream) {
     const size_t n = rows * (size_t)hidden;
-    if (hidden % 4 == 0 && all16(packed, dy, dpacked)) swiglu_bwd_kernel<4><<<flat_grid(n / 4, sm_count), 256, 0, stream>>>(packed, dy, dpacked, rows, hidden);
-    else swiglu_bwd_kernel<1><<<flat_grid(n, sm_count), 256, 0, stream>>>(packed, dy, dpacked, rows, hidden);
+    if (hidden % 4 == 0 && all16(packed, dy, dpacked)) launch_chained(swiglu_bwd_kernel<4>, dim3(flat_grid(n / 4, sm_count)), dim3(256), 0, stream, packed, dy, dpacked, rows, hidden);
+    else launch_chained(swiglu_bwd_kernel<1>, dim3(flat_grid(n, sm_count)), dim3(256), 0, stream, packed, dy, dpacked, rows, hidden);
     return cudaGetLastError();
 }
 cudaError_t launch_softmax_cross_entropy(const float* logits, const int* targets, float* partial, float* out, size_t rows,
                                          int cols, int sm_count, cudaStream_t stream) {
-    ce_kernel<false><<<row_grid(rows, sm_count), kCeThreads, 0, stream>>>(logits, targets, partial, nullptr, nullptr, rows, cols,
-                                                                          cols % 4 == 0 && all16(logits, nullptr));
+    launch_chained(ce_kernel<false>, dim3(row_grid(rows, sm_count)), dim3(kCeThreads), 0, stream, logits, targets, partial, nullptr, nullptr, rows, cols, cols % 4 == 0 && all16(logits, nullptr));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    mean_kernel<<<1, 1024, 0, stream>>>(partial, out, rows, rows);
+    launch_chained(mean_kernel, dim3(1), dim3(1024), 0, stream, partial, out, rows, rows);
     return cudaGetLastError();
 }
 cudaError_t launch_softmax_cross_entropy_backward(const float* logits, const int* targets, const float* grad_out,
                                                   float* grad_logits, size_t rows, int cols, int sm_count,
                                                   cudaStream_t stream) {
-    ce_kernel<true><<<row_grid(rows, sm_count), kCeThreads, 0, stream>>>(logits, targets, nullptr, grad_out, grad_logits, rows, cols,
-                                                                         cols % 4 == 0 && all16(logits, grad_logits));
+    launch_chained(ce_kernel<true>, dim3(row_grid(rows, sm_count)), dim3(kCeThreads), 0, stream, logits, targets, nullptr, grad_out, grad_logits, rows, cols, cols % 4 == 0 && all16(logits, grad_logits));
     return cudaGetLastError();
 }
 
@@ -763,13 +780,11 @@ cudaError_t launch_rope(const float* x, float* out, size_t rows, int tokens, int
         long long want = (quads + 256 * kRopeIn - 1) / (256 * kRopeIn);
         if (want > by) want = by;
         if (quads < 0x7fffffffll) {
-            rope_quads_kernel<<<dim3((unsigned)tokens, (unsigned)want), 256, (size_t)(head_dim / 2 + 1) * sizeof(float2), stream>>>(
-                x, out, batch, tokens, channels, head_dim, rd, token_offset, theta, inverse);
+            launch_chained(rope_quads_kernel, dim3((unsigned)tokens, (unsigned)want), dim3(256), (size_t)(head_dim / 2 + 1) * sizeof(float2), stream, x, out, batch, tokens, channels, head_dim, rd, token_offset, theta, inverse);
             return cudaGetLastError();
         }
     }
-    rope_kernel<<<dim3((unsigned)tokens, (unsigned)by), 256, shared_turns ? (size_t)(head_dim / 2 + 1) * sizeof(float2) : 0, stream>>>(
-        x, out, batch, tokens, channels, n_head, head_dim, rotary_dim, token_offset, theta, inverse, split_half, shared_turns);
+    launch_chained(rope_kernel, dim3((unsigned)tokens, (unsigned)by), dim3(256), shared_turns ? (size_t)(head_dim / 2 + 1) * sizeof(float2) : 0, stream, x, out, batch, tokens, channels, n_head, head_dim, rotary_dim, token_offset, theta, inverse, split_half, shared_turns);
     return cudaGetLastError();
 }
 cudaError_t launch_adam(float* param, const float* grad, float* m, float* v, size_t n, float lr, float beta1, float beta2,
@@ -793,7 +808,7 @@ cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* o
     constexpr size_t bytes = fwd_floats<BQ, NC>() * 4;
     cudaError_t e = with_smem(gqa_fwd_kernel<BQ, NC>, bytes);
     if (e != cudaSuccess) return e;
-    gqa_fwd_kernel<BQ, NC><<<dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), 4 * BQ, bytes, stream>>>(q, k, v, out, p);
+    launch_chained(gqa_fwd_kernel<BQ, NC>, dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), dim3(4 * BQ), bytes, stream, q, k, v, out, p);
     return cudaGetLastError();
 }
 template <int BQ, int NC>
@@ -803,9 +818,9 @@ cudaError_t run_gqa_bwd(const float* q, const float* k, const float* v, const fl
     cudaError_t e = with_smem(gqa_bwd_q_kernel<BQ, NC>, bq);
     if (e == cudaSuccess) e = with_smem(gqa_bwd_k_kernel<NC>, bk);
     if (e != cudaSuccess) return e;
-    gqa_bwd_q_kernel<BQ, NC><<<dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), 4 * BQ, bq, stream>>>(q, k, v, dout, probs, ds, dq, p);
+    launch_chained(gqa_bwd_q_kernel<BQ, NC>, dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), dim3(4 * BQ), bq, stream, q, k, v, dout, probs, ds, dq, p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    gqa_bwd_k_kernel<NC><<<dim3(p.batch * p.n_kv, (p.tk + kKT - 1) / kKT), 256, bk, stream>>>(q, dout, probs, ds, dk, dv, p);
+    launch_chained(gqa_bwd_k_kernel<NC>, dim3(p.batch * p.n_kv, (p.tk + kKT - 1) / kKT), dim3(256), bk, stream, q, dout, probs, ds, dk, dv, p);
     return cudaGetLastError();
 }
 // query tiles of 64 rows, or of 32 where 64 would leave SMs without a second CTA

@@ -146,3 +146,57 @@ def test_layer_calls_under_a_capture_of_the_caller():
             assert float((y - wy).norm() / wy.norm()) < 1e-6 and float((dx - wdx).norm() / wdx.norm()) < 1e-6
         del graph
         ctx.close()
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_launches_that_overlap_give_the_bits_of_launches_apart(recorded):
+    """Every launch reads what the one before it wrote (a memset and a fork among them), many times over in buffers that are taken again."""
+    from motifcl_b200 import Context
+    stream = torch.cuda.Stream(device=0)
+    with torch.cuda.stream(stream):
+        ctx, lane = Context.on_torch_stream(0), Context(0)
+        g = torch.Generator(device="cuda").manual_seed(5)
+        N, D, F = 192, 288, 320
+        x0 = torch.randn(N, D, device="cuda", generator=g)
+        st0 = torch.randint(0, 256, (F * D // 4 * 3,), device="cuda", generator=g, dtype=torch.int32).to(torch.uint8)
+        packed = torch.randn(N, 2 * F, device="cuda", generator=g)
+
+        def state():
+            s = {"x": x0.clone(), "st": st0.clone(), "scale": torch.full((F,), 0.07, device="cuda"), "v": torch.full((F,), 0.01, device="cuda")}
+            for n, shape in (("h", (N, D)), ("r", (N, D)), ("y", (N, F)), ("dx", (N, D)), ("act", (N, F)), ("inv", (N,)), ("dw", (D,))):
+                s[n] = torch.zeros(shape, device="cuda")
+            return s
+
+        def calls(s, apart):
+            def after():
+                if apart:
+                    ctx.finish()
+            one = s["scale"][:D]
+            for _ in range(3):
+                ctx.rmsnorm(s["x"], one, s["h"], N, D, 1e-5); after()
+                ctx.rope(s["h"], s["r"], 2, N // 2, D, 6, 48); after()
+                ctx.counter_forward(s["r"], s["st"], s["scale"], s["y"], N, D, F, 11); after()
+                ctx.counter_backward_input(s["st"], s["scale"], s["y"], s["dx"], N, D, F, 11); after()
+                ctx.counter_update_fused(s["st"], s["scale"], s["v"], s["y"], s["r"], None, 11, D, F, N, 3e-3, 0.05, 0.9, 1e-3, 77); after()
+                ctx.swiglu(packed, s["act"], N, F); after()
+                ctx.rmsnorm_backward_weight(s["dx"], s["r"], s["inv"], s["dw"], N, D, 1e-5); after()
+                ctx.lane_fork(lane); ctx.lane_join(lane); after()
+                ctx.rmsnorm_backward_x(s["dx"], one, s["r"], s["x"], N, D, 1e-5); after()
+        a, b = state(), state()
+        calls(a, True)
+        ctx.finish()
+        if recorded:
+            ctx.batch_begin()
+            calls(b, False)
+            batch = ctx.batch_end()
+            batch.launch()
+            ctx.finish()
+            batch.close()
+        else:
+            calls(b, False)
+            ctx.finish()
+        lane.close()
+    for n in a:
+        if n != "dw":                    # added up with atomics
+            assert torch.equal(a[n], b[n]), n
+    assert torch.isfinite(a["x"]).all() and not torch.equal(a["st"], st0)
