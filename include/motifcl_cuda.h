@@ -300,7 +300,9 @@ int mcl_cuda_eltwise_f32(mcl_cuda_ctx* ctx, int op, const float* a, const float*
  *   gqa_forward             q [B*Tq, n_head*hd], k [B*key_stride, n_kv*hd], v [B*key_stride, n_kv*vhd],
  *                           out [B*Tq, n_head*vhd]; causal with query_offset, optional sliding window (0 = none);
  *                           f32 keys/values, no mask
- *   gqa_backward            probs_scratch, ds_scratch [B*n_head*Tq*Tk]; grad_q/k/v shaped like q/k/v ---- */
+ *   gqa_backward            probs_scratch, ds_scratch [B*n_head*Tq*Tk]; grad_q/k/v shaped like q/k/v
+ *                           (attention, head_dim <= 64: an infinity or NaN in q, k, v or grad_out may make everything NaN that is
+ *                           computed from a tile of 64 rows it lies in) ---- */
 int mcl_cuda_rmsnorm(mcl_cuda_ctx* ctx, const float* x, const float* weight, float* out, size_t rows, size_t cols,
                      float eps);
 int mcl_cuda_rmsnorm_backward_x(mcl_cuda_ctx* ctx, const float* x, const float* weight, const float* grad_out,

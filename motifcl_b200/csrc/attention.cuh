@@ -1,5 +1,6 @@
-// Grouped-query attention, forward and backward, for head sizes up to 64: exact fp32 FMAs on tiles in shared memory (tf32 would
-// not hold the reference's accuracy), scores never written by the forward pass.  Included by trainer_ops.cu.
+// Grouped-query attention, forward and backward, for head sizes up to 64 and grids that do not fill the GPU (attention_mma.cuh takes
+// those that do): exact fp32 FMAs on tiles in shared memory (tf32 would not hold the reference's accuracy), scores never written by
+// the forward pass.  Included by trainer_ops.cu.
 //
 // A CTA owns BQ queries of one head and walks over tiles of 64 keys with TWO groups of 2 BQ threads that take alternate tiles
 // (a training step has few query tiles: one group left 10 warps on an SM, each issuing every 5.6 cycles) and merge at the end.

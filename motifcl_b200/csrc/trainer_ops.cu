@@ -348,6 +348,7 @@ __device__ __forceinline__ void key_range(const GqaDims& p, int tq, int& k0, int
 }
 
 #include "attention.cuh"
+#include "attention_mma.cuh"
 
 // ---- attention as batched fp32 products + a row pass (head sizes above 64, or few queries over many keys) ------------------------------------------
 // The seven products of attention forward and backward (S = scale*Q K^T, O = P V, dP = dO V^T,
@@ -803,28 +804,36 @@ cudaError_t with_smem(K kern, size_t bytes) {      // set on every call: it hold
 bool gqa_tiled(int batch, int tq, int tk, int n_head, int hd, int vhd) {
     return hd <= 64 && vhd == hd && tq <= 65535 * 32 && tk <= 65535 * 64 && (tk <= 1024 || (long long)batch * n_head * ((tq + 63) / 64) >= 148);
 }
-template <int BQ, int NC>
-cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* out, const GqaDims& p, cudaStream_t stream) {
-    constexpr size_t bytes = fwd_floats<BQ, NC>() * 4;
-    cudaError_t e = with_smem(gqa_fwd_kernel<BQ, NC>, bytes);
+// Attention is not launched early (launch_chained): where the kernel before it holds some of the SMs, all its few long CTAs would be placed on
+// the others (2 sequences of 512, 12 heads of 64: backward 207 us, 257 when launched early).
+template <int NC>
+cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* out, const GqaDims& p, cudaStream_t stream, bool mma) {
+    const size_t bytes = mma ? 2 * (AttTile<NC>::kBytes + AttTile<NC>::kRaw) : fwd_floats<32, NC>() * 4;
+    const auto kern = mma ? gqa_fwd_mma_kernel<NC> : gqa_fwd_kernel<32, NC>;
+    const cudaError_t e = with_smem(kern, bytes);
     if (e != cudaSuccess) return e;
-    launch_chained(gqa_fwd_kernel<BQ, NC>, dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), dim3(4 * BQ), bytes, stream, q, k, v, out, p);
+    const int rows = mma ? 64 : 32;
+    kern<<<dim3(p.batch * p.n_head, (p.tq + rows - 1) / rows), 128, bytes, stream>>>(q, k, v, out, p);
     return cudaGetLastError();
 }
-template <int BQ, int NC>
+template <int NC>
 cudaError_t run_gqa_bwd(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, float* dk,
-                        float* dv, const GqaDims& p, cudaStream_t stream) {
-    constexpr size_t bq = bwd_q_floats<BQ, NC>() * 4, bk = bwd_k_floats<NC>() * 4;
-    cudaError_t e = with_smem(gqa_bwd_q_kernel<BQ, NC>, bq);
-    if (e == cudaSuccess) e = with_smem(gqa_bwd_k_kernel<NC>, bk);
+                        float* dv, const GqaDims& p, cudaStream_t stream, bool mma) {
+    const size_t tiles = 2 * (AttTile<NC>::kBytes + AttTile<NC>::kRaw), bq = mma ? tiles : bwd_q_floats<32, NC>() * 4, bk = mma ? tiles : bwd_k_floats<NC>() * 4;
+    const auto kq = mma ? gqa_bwd_q_mma_kernel<NC> : gqa_bwd_q_kernel<32, NC>;
+    const auto kk = mma ? gqa_bwd_k_mma_kernel<NC> : gqa_bwd_k_kernel<NC>;
+    cudaError_t e = with_smem(kq, bq);
+    if (e == cudaSuccess) e = with_smem(kk, bk);
     if (e != cudaSuccess) return e;
-    launch_chained(gqa_bwd_q_kernel<BQ, NC>, dim3(p.batch * p.n_head, (p.tq + BQ - 1) / BQ), dim3(4 * BQ), bq, stream, q, k, v, dout, probs, ds, dq, p);
+    const int rows = mma ? 64 : 32;
+    kq<<<dim3(p.batch * p.n_head, (p.tq + rows - 1) / rows), 128, bq, stream>>>(q, k, v, dout, probs, ds, dq, p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    launch_chained(gqa_bwd_k_kernel<NC>, dim3(p.batch * p.n_kv, (p.tk + kKT - 1) / kKT), dim3(256), bk, stream, q, dout, probs, ds, dk, dv, p);
+    kk<<<dim3(p.batch * p.n_kv, (p.tk + kKT - 1) / kKT), mma ? 128 : 256, bk, stream>>>(q, dout, probs, ds, dk, dv, p);
     return cudaGetLastError();
 }
-// query tiles of 64 rows, or of 32 where 64 would leave SMs without a second CTA
-bool wide_q(const GqaDims& p) { return (long long)p.batch * p.n_head * ((p.tq + 63) / 64) >= 2 * 148; }
+// Tensor cores where tiles of 64 queries give every SM two CTAs, or where all keys are one tile; else their one warp per 16 queries is a longer chain than the FMA
+// kernels' 32 queries by 128 threads (figures in attention_mma.cuh)
+bool on_tensor_cores(const GqaDims& p) { return p.tk <= kKT || (long long)p.batch * p.n_head * ((p.tq + 63) / 64) >= 2 * 148; }
 }  // namespace
 
 size_t gqa_forward_scratch_floats(int batch, int tq, int tk, int n_head, int hd, int vhd) {
@@ -838,12 +847,12 @@ cudaError_t launch_gqa_forward(const float* q, const float* k, const float* v, f
     GqaDims p{batch, tq, tk, key_stride, n_head, n_kv, hd, vhd, causal, q_off, window, scale};
     if (gqa_tiled(batch, tq, tk, n_head, hd, vhd)) {
         *launches += 1;
-        const bool w = wide_q(p);
+        const bool w = on_tensor_cores(p);
         switch ((hd + 15) / 16) {
-            case 1: return w ? run_gqa_fwd<64, 1>(q, k, v, out, p, stream) : run_gqa_fwd<32, 1>(q, k, v, out, p, stream);
-            case 2: return w ? run_gqa_fwd<64, 2>(q, k, v, out, p, stream) : run_gqa_fwd<32, 2>(q, k, v, out, p, stream);
-            case 3: return w ? run_gqa_fwd<64, 3>(q, k, v, out, p, stream) : run_gqa_fwd<32, 3>(q, k, v, out, p, stream);
-            default: return w ? run_gqa_fwd<64, 4>(q, k, v, out, p, stream) : run_gqa_fwd<32, 4>(q, k, v, out, p, stream);
+            case 1: return run_gqa_fwd<1>(q, k, v, out, p, stream, w);
+            case 2: return run_gqa_fwd<2>(q, k, v, out, p, stream, w);
+            case 3: return run_gqa_fwd<3>(q, k, v, out, p, stream, w);
+            default: return run_gqa_fwd<4>(q, k, v, out, p, stream, w);
         }
     }
     const int group = n_head / n_kv;
@@ -875,15 +884,13 @@ cudaError_t launch_gqa_backward(const float* q, const float* k, const float* v, 
     GqaDims p{batch, tq, tk, tk, n_head, n_kv, hd, hd, causal, q_off, 0, scale};
     if (gqa_tiled(batch, tq, tk, n_head, hd, hd)) {
         *launches += 2;
-        const bool w = wide_q(p);
-#define MCL_GQA_BWD(NC) (w ? run_gqa_bwd<64, NC>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream) : run_gqa_bwd<32, NC>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream))
+        const bool w = on_tensor_cores(p);
         switch ((hd + 15) / 16) {
-            case 1: return MCL_GQA_BWD(1);
-            case 2: return MCL_GQA_BWD(2);
-            case 3: return MCL_GQA_BWD(3);
-            default: return MCL_GQA_BWD(4);
+            case 1: return run_gqa_bwd<1>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream, w);
+            case 2: return run_gqa_bwd<2>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream, w);
+            case 3: return run_gqa_bwd<3>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream, w);
+            default: return run_gqa_bwd<4>(q, k, v, dout, probs, ds, dq, dk, dv, p, stream, w);
         }
-#undef MCL_GQA_BWD
     }
     const int group = n_head / n_kv;
     const long long qc = (long long)n_head * hd, kc = (long long)n_kv * hd;

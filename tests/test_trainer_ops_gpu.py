@@ -355,3 +355,37 @@ def test_mse_loss_and_backward_follow_the_opencl_kernels_order(ctx, n):
     want_g = ((np.float32(0.75) * np.float32(2.0)) * (pred - target).astype(np.float32)).astype(np.float32) / np.float32(n)
     assert np.array_equal(g_d.cpu().numpy().view(np.uint32), want_g.astype(np.float32).view(np.uint32))
 
+
+
+@pytest.mark.parametrize("B,Tq,Tk,H,G,hd,causal,q_off", [
+    (1, 64, 64, 1, 1, 16, True, 0),            # one tile of either kind
+    (2, 65, 63, 3, 3, 33, False, 0),           # a row beyond one, a key short of one, an odd head
+    (1, 129, 129, 4, 2, 48, True, 0),          # odd rows of keys: single stores of the probabilities
+    (3, 31, 190, 4, 1, 64, True, 159),         # one kv head for all, queries at the end of the keys
+    (60, 130, 128, 5, 5, 40, True, 3),         # tiles of 64 queries
+    (1, 1, 257, 2, 2, 50, False, 0),
+    (2, 200, 70, 2, 1, 62, True, 0),           # queries that see every key
+])
+def test_gqa_at_the_edges_of_its_tiles(ctx, B, Tq, Tk, H, G, hd, causal, q_off):
+    """Products of three-term operands: within fp32 rounding of float64, whatever part of a tile exists."""
+    g = torch.Generator().manual_seed(Tq * 7 + Tk + hd)
+    r = lambda n, c: torch.randn(n, c, generator=g, dtype=torch.float64).float().double().requires_grad_()      # fp32 values
+    q, k, v, dout = r(B * Tq, H * hd), r(B * Tk, G * hd), r(B * Tk, G * hd), r(B * Tq, H * hd).detach()
+    scale = 1.0 / math.sqrt(hd)
+    ref, p = _attention_reference(q, k, v, B, Tq, Tk, H, G, hd, hd, causal, q_off, 0, scale)
+    qd, kd, vd = dev(q.detach()), dev(k.detach()), dev(v.detach())
+    out = torch.full((B * Tq, H * hd), 7.0, device="cuda")
+    ctx.gqa_forward(qd, kd, vd, out, B, Tq, Tk, Tk, H, G, hd, hd, causal, q_off, 0, scale)
+    torch.cuda.synchronize()
+    assert rel_l2(out, ref) <= 5e-7
+    ref.backward(dout)
+    probs, ds = torch.full((B * H * Tq * Tk,), 7.0, device="cuda"), torch.full((B * H * Tq * Tk,), 7.0, device="cuda")
+    dq, dk, dv = torch.full_like(qd, 7.0), torch.full_like(kd, 7.0), torch.full_like(vd, 7.0)
+    ctx.gqa_backward(qd, kd, vd, dev(dout), probs, ds, dq, dk, dv, B, Tq, Tk, H, G, hd, causal, q_off, scale)
+    torch.cuda.synchronize()
+    dp = dout.view(B, Tq, H, hd).permute(0, 2, 1, 3) @ v.detach().view(B, Tk, G, hd).permute(0, 2, 1, 3).repeat_interleave(H // G, dim=1).transpose(-1, -2)
+    pd = p.detach()
+    assert rel_l2(probs.view(B, H, Tq, Tk), pd) <= 1e-6
+    assert rel_l2(ds.view(B, H, Tq, Tk), pd * (dp - (pd * dp).sum(-1, keepdim=True))) <= 1e-6
+    for a, b in ((dq, q.grad), (dk, k.grad), (dv, v.grad)):
+        assert rel_l2(a, b) <= 1e-6
