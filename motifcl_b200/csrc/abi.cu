@@ -301,13 +301,17 @@ mcl::TcPlan dense_plan(const mcl_cuda_ctx* ctx, size_t M, size_t N, size_t K) {
 }
 mcl::TcProblem tc_problem(const mcl::TcOperand& a, const mcl::TcOperand& b, float* c, size_t M, size_t N, size_t K, const mcl::TcPlan& plan,
                           const float* col_scale, void* splitk_ws) {
-    mcl::TcProblem q = {a, b, c, (int)M, (int)N, (int)K, plan, col_scale, static_cast<float*>(splitk_ws)};
+    mcl::TcProblem q = {a, b, c, (int)M, (int)N, (int)K, plan, col_scale, static_cast<float*>(splitk_ws), 0};
     return q;
+}
+cudaError_t reduce_of(const mcl::TcProblem& q, cudaStream_t stream) {
+    const int rows = q.turned ? q.N : q.M, cols = q.turned ? q.M : q.N;
+    return mcl::launch_splitk_reduce(q.splitk_ws, q.c, q.col_scale, rows, cols, cols, q.plan.splits, stream);
 }
 int tc_product(mcl_cuda_ctx* ctx, const char* op, const mcl::TcProblem& q) {
     MCL_TC(ctx, op, mcl::launch_tc_products(&q, 1, ctx->err_word, ctx->max_smem, ctx->sm_count, ctx->stream, &_n));
     if (q.plan.splits > 1)
-        MCL_LAUNCH(ctx, op, mcl::launch_splitk_reduce(q.splitk_ws, q.c, q.col_scale, q.M, q.N, q.N, q.plan.splits, ctx->stream));
+        MCL_LAUNCH(ctx, op, reduce_of(q, ctx->stream));
     return MCL_CUDA_OK;
 }
 int split_tensors(mcl_cuda_ctx* ctx, const char* op, const mcl::SplitDesc* d, int n) {
@@ -354,8 +358,15 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
                 cost[cg - 1] += mcl::tc_plan_shared((int)L[i].O, (int)L[i].I, (int)L[i].Nt, 3, cg, mcl::kGradDepthLimit, min_items, together).cost;
         dw_cg = cost[1] < cost[0] ? 2 : 1;
     }
-    auto row_plan = [&](size_t M, size_t N, size_t K) {
-        return n == 1 ? digit_plan(ctx, M, N, K) : mcl::tc_plan_shared((int)M, (int)N, (int)K, 2, M > 128 ? 2 : 1, 0, 0);
+    // A product with digits alone in its launch runs as C^T = T X^T where that wastes less of the last tile of tokens: tokens are then its
+    // columns, in tiles of 64 to 256, not its rows, in tiles of 128 or 256 (777 tokens: 800 columns for 1024 rows).  A forward, us: 777 x 4096 ->
+    // 14336 205 -> 180, 300 x 4096 -> 4096 56.6 -> 50.6, 90 x 1024 -> 1024 22.5 -> 19.3.  Not where an accumulator would take a longer
+    // slice of K: its error grows with it (40 x 4096 -> 14336, 5 slices: 86 us and 1.1e-7, turned in one 89 and 3.1e-7).
+    auto row_plan = [&](size_t M, size_t N, size_t K, bool* turned) {
+        if (n > 1) return mcl::tc_plan_shared((int)M, (int)N, (int)K, 2, M > 128 ? 2 : 1, 0, 0);
+        const mcl::TcPlan straight = digit_plan(ctx, M, N, K), other = digit_plan(ctx, N, M, K);
+        *turned = other.cost < 0.98 * straight.cost && other.ktiles_per_split <= straight.ktiles_per_split;
+        return *turned ? other : straight;
     };
     for (size_t i = 0; i < n; ++i) {
         const ProductLayer& l = L[i];
@@ -369,8 +380,15 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
             k_off.push_back(plan.splits > 1 ? cv.reserve(plan.workspace_bytes) : 0);
             pr.push_back(tc_problem(a, b, c, M, N, K, plan, cs, w + k_off.back()));
         };
-        if (l.y) add(terms_of(w, xb[i], false, false), digits_of(w + t_off[i], l.O, l.I, false), l.y, l.Nt, l.O, l.I, row_plan(l.Nt, l.O, l.I), l.scale);
-        if (l.grad_x) add(terms_of(w, gb[i], true, false), digits_of(w + t_off[i], l.O, l.I, true), l.grad_x, l.Nt, l.I, l.O, row_plan(l.Nt, l.I, l.O), nullptr);
+        auto add_rows = [&](const mcl::TcOperand& terms, const mcl::TcOperand& digits, float* c, size_t N, size_t K, const float* cs) {
+            bool turned = false;
+            const mcl::TcPlan plan = row_plan(l.Nt, N, K, &turned);
+            if (turned) add(digits, terms, c, N, l.Nt, K, plan, cs);
+            else add(terms, digits, c, l.Nt, N, K, plan, cs);
+            pr.back().turned = turned;
+        };
+        if (l.y) add_rows(terms_of(w, xb[i], false, false), digits_of(w + t_off[i], l.O, l.I, false), l.y, l.O, l.I, l.scale);
+        if (l.grad_x) add_rows(terms_of(w, gb[i], true, false), digits_of(w + t_off[i], l.O, l.I, true), l.grad_x, l.I, l.O, nullptr);
         if (l.grad_w)
             add(terms_of(w, gb[i], false, true), terms_of(w, xb[i], false, true), l.grad_w, l.O, l.I, l.Nt,
                 n == 1 ? dense_plan(ctx, l.O, l.I, l.Nt)
@@ -392,7 +410,7 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     if (!ed.empty()) MCL_TC(ctx, op, mcl::launch_expand_ternary(ed.data(), (int)ed.size(), (int)C, ctx->sm_count, ctx->stream, &_n));
     // products of one kind together, the longest items first (they are dealt round-robin)
     std::stable_sort(pr.begin(), pr.end(), [](const mcl::TcProblem& a, const mcl::TcProblem& b) {
-        const int ta = a.b.planes + 1, tb = b.b.planes + 1;
+        const int ta = a.turned ? 2 : a.b.planes + 1, tb = b.turned ? 2 : b.b.planes + 1;
         if (ta != tb) return ta > tb;
         if (a.plan.pair != b.plan.pair) return a.plan.pair > b.plan.pair;
         return (long long)ta * a.plan.ktiles_per_split * a.plan.bn > (long long)tb * b.plan.ktiles_per_split * b.plan.bn;
@@ -405,7 +423,7 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     for (const mcl::TcProblem& q : pr) {
         if (q.plan.splits <= 1) continue;
         if (q.col_scale) {
-            MCL_LAUNCH(ctx, op, mcl::launch_splitk_reduce(q.splitk_ws, q.c, q.col_scale, q.M, q.N, q.N, q.plan.splits, ctx->stream));
+            MCL_LAUNCH(ctx, op, reduce_of(q, ctx->stream));
             continue;
         }
         part.push_back(q.splitk_ws); out.push_back(q.c); elems.push_back((long long)q.M * q.N); splits.push_back(q.plan.splits);

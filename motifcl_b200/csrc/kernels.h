@@ -114,6 +114,7 @@ struct TcProblem {
     TcPlan plan;
     const float* col_scale;    // of the output's columns (plan.splits == 1)
     float* splitk_ws;
+    int turned;                // c is [N][M]: a the digits, b the split tensor (scaled by row); col_scale of the rows of the product
 };
 cudaError_t launch_tc_products(const TcProblem* probs, int n, int* err_word, size_t max_smem, int sm_count, cudaStream_t stream,
                                int* launches);

@@ -7,6 +7,7 @@
 //     Y  [tokens,out] = X  . T^T          A = terms of X    [tokens,in]     B = T [out,in]
 //     dX [tokens,in ] = (dY.s) . T        A = terms of dY.s [tokens,out]    B = T [out,in], read MN-major
 //     dW [out,in]     = dY^T . X          A = terms of dY, B = terms of X   both [tokens, .], read MN-major
+// (Y and dX also turned, as C^T = T . X^T and T^T . (dY.s)^T with tokens as columns, where the plan wastes less of a tile),
 // so every tensor is split once, in its own layout, and T is expanded once: a transposed operand is the
 // same shared-memory tile with the MN-major bit of the instruction descriptor.
 //
@@ -53,7 +54,8 @@ struct TcTile {
     int BN, stage_bytes;      // tile width; bytes of one ring slot (A tile and this CTA's share of B, or both terms of them)
     int b_bytes;              // this CTA's share of a B tile
     int a_mn, b_mn;           // operand is stored with M / N contiguous
-    int nterms;               // 2: A lo, A hi against one B plane; 3: lo.hi, hi.lo, hi.hi
+    int turned;               // C is [N][M]: A are the digits (one plane), B the terms, col_scale belongs to the rows of the product
+    int nterms;               // 2: A lo, A hi against one B plane (turned: B's against A); 3: lo.hi, hi.lo, hi.hi
     int ktiles_per_split, splits;
     int tiles_m, tiles_n, group_m;
     int item_begin;           // first work item of the product
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             const TcTile& P = sp[pi];
             const CUtensorMap* tmA = &tab.maps[3 * pi];
             const CUtensorMap* tmB = &tab.maps[3 * pi + 1];
-            const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn;
+            const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn, turned = P.turned;
             const uint32_t bytes = (uint32_t)(CG * P.stage_bytes);
             const int m0 = (t.mt * CG + (int)rank) * BM, n0 = t.nt * BN + (int)rank * (BN / CG);
             const uint32_t b_bytes = (uint32_t)P.b_bytes;
@@ -364,8 +366,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             }
             for (int term = 0; !TOGETHER && term < nterms && ok; ++term) {
                 // planes: 0 = hi, 1 = lo; products with a lo term first
-                const int pa = nterms == 3 ? (term == 0) : (term + 1 < nterms);
-                const int pb = nterms == 3 && term == 1;
+                const int pa = nterms == 3 ? (term == 0) : !turned && term == 0;
+                const int pb = nterms == 3 ? (term == 1) : turned && term == 0;
                 for (int kk = 0; kk < t.nkt; ++kk) {
                     ok = mbar_wait_all(empty_bar(s), ph, &abort_flag);
                     if (!ok) { abort_flag = 1; if (lane == 0) atomicExch(tab.err, 1); break; }
@@ -461,7 +463,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         // of products with short main loops.
         auto row_bits = [&](const TcTile& P, const TcItem& t) {
             const int row = (t.mt * CG + (int)rank) * BM + q * 32 + lane;
-            return P.a_inv && row < P.M ? __float_as_int(__ldg(P.a_inv + row)) : 0x3F800000;
+            const float* f = !P.turned ? P.a_inv : P.splits == 1 ? P.col_scale : nullptr;
+            return f && row < P.M ? __float_as_int(__ldg(f + row)) : 0x3F800000;
         };
         auto columns = [&](const TcTile& P) { return P.b_inv ? P.b_inv : P.splits == 1 ? P.col_scale : nullptr; };
         auto column = [&](const float* f, int c, int N) { return f && c < N ? __ldg(f + c) : 1.0f; };
@@ -492,7 +495,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             }
             // undo the powers of two of the split: the row's and g in two halves, so that no step leaves fp32 unless the result does
             const int e = max(-252, (inv_bits >> 23) - 127 - g), e1 = e >> 1;
-            const float r1 = pow2(e1), r2 = pow2(e - e1);
+            const bool turned = P.turned;
+            const float r1 = pow2(e1), r2 = turned ? __int_as_float(inv_bits) : pow2(e - e1);      // turned: the row's scale
             const CUtensorMap* tmC = &tab.maps[3 * pi + 2];
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
             const bool was = !abort_flag;
@@ -541,6 +545,17 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                     ++n_store;
                     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");     // the store before last has read this buffer
                     __syncwarp();
+                    if (turned) {
+                        // the power of two of a column (a row of C) in two halves around the scale; a lane's values go down a column of the box
+                        const int ce = (__float_as_int(col[h]) >> 23) - 127, ce1 = ce >> 1;
+                        const float k1 = pow2(ce1), k2 = pow2(ce - ce1);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float v = __uint_as_float(r[h][j]) * __shfl_sync(0xffffffffu, k1, j) * r2 * __shfl_sync(0xffffffffu, k2, j);
+                            asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf + (uint32_t)j * 128u + (uint32_t)(((lane >> 2) ^ (j & 7)) << 4) + (uint32_t)((lane & 3) << 2)),
+                                         "f"(v) : "memory");
+                        }
+                    } else {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) r[h][j] = __float_as_uint(__uint_as_float(r[h][j]) * r1);
                     if (factors) {
@@ -554,11 +569,12 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
                                      ::"r"(buf + (uint32_t)lane * 128u + (uint32_t)((j ^ (lane & 7)) << 4)), "r"(r[h][4 * j]), "r"(r[h][4 * j + 1]),
                                        "r"(r[h][4 * j + 2]), "r"(r[h][4 * j + 3]) : "memory");
+                    }
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
                         asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-                                     ::"l"(reinterpret_cast<uint64_t>(tmC)), "r"(buf), "r"(n0 + cc), "r"(row0), "r"(t.split) : "memory");
+                                     ::"l"(reinterpret_cast<uint64_t>(tmC)), "r"(buf), "r"(turned ? row0 : n0 + cc), "r"(turned ? n0 + cc : row0), "r"(t.split) : "memory");
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
                 }
@@ -1154,11 +1170,13 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
     for (int i = 0; i < n; ++i) {
         const TcProblem& q = probs[i];
         const TcOperand &a = q.a, &b = q.b;
-        if (a.planes != 2 || (a.words && b.words) || b.planes < 1 || b.planes > 2 || (q.N & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
+        const int out_rows = q.turned ? q.N : q.M, out_cols = q.turned ? q.M : q.N;
+        if (q.turned ? a.planes != 1 || b.planes != 2 || !b.inv || q.plan.together : a.planes != 2 || b.planes < 1 || b.planes > 2) return cudaErrorInvalidValue;
+        if ((a.words && b.words) || (out_cols & 3) || (a.ld & 7) || (b.ld & 7)) return cudaErrorInvalidValue;
         const int bn = q.plan.bn, b_rows = bn / CG;
         float* out = q.plan.splits > 1 ? q.splitk_ws : q.c;
         if (!make_map(&tab.maps[3 * i], a, BM) || !make_map(&tab.maps[3 * i + 1], b, b_rows) ||
-            !make_out_map(&tab.maps[3 * i + 2], out, q.M, q.N, q.plan.splits)) return cudaErrorInvalidValue;
+            !make_out_map(&tab.maps[3 * i + 2], out, out_rows, out_cols, q.plan.splits)) return cudaErrorInvalidValue;
         TcTile& p = tab.p[i];
         p.col_scale = q.col_scale;
         p.a_inv = a.inv; p.b_inv = b.inv;
@@ -1168,7 +1186,8 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
         p.b_bytes = (b.mn_major ? (b_rows + 63) / 64 * 64 : b_rows) * BK * 2;
         p.stage_bytes = q.plan.together ? 2 * kATileBytes + b.planes * p.b_bytes : kATileBytes + p.b_bytes;
         p.a_mn = a.mn_major; p.b_mn = b.mn_major;
-        p.nterms = b.planes == 2 ? 3 : 2;
+        p.turned = q.turned;
+        p.nterms = !q.turned && b.planes == 2 ? 3 : 2;
         p.ktiles_per_split = q.plan.ktiles_per_split; p.splits = q.plan.splits;
         p.tiles_m = (q.M + CG * BM - 1) / (CG * BM); p.tiles_n = (q.N + bn - 1) / bn;
         p.group_m = 12 / CG;                   // 12 row tiles x 12 column tiles in flight on 148 SMs

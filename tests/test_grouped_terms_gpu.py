@@ -64,3 +64,30 @@ def test_contractions_side_by_side_and_again():
             ctx.finish()
             for l, f in zip(ls, first):
                 assert all(torch.equal(l[n], f[n]) for n in f)
+
+
+@pytest.mark.parametrize("N,I,O", [(40, 1088, 1156), (70, 4096, 1028), (300, 2048, 1100), (777, 1024, 3076), (161, 1156, 4100), (1030, 1536, 1032)])
+def test_row_products_on_tokens_that_leave_a_tile_ragged(N, I, O):
+    """Tokens as columns of the product (digits times activations) or as its rows, whichever wastes less: rows 2^-80 to 2^80 of one another
+    keep their bits (24 of the row's largest element, by as many as are added up), an infinity stays in its row."""
+    from motifcl_b200 import Context
+    rng = np.random.default_rng(N + I + O)
+    ctx = Context.on_torch_stream(0)
+    ctx.set_gemm_mode("tensor")
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    st, sc = dev(rng.integers(0, 256, O * I // 4 * 3, dtype=np.uint8)), dev(rng.uniform(0.02, 0.2, O).astype(np.float32))
+    w = torch.empty(O, I, device="cuda")
+    ctx.counter_decode_weight(st, torch.ones_like(sc), w, I, O, 11)
+    rows = np.exp2(rng.integers(-80, 81, (N, 1))).astype(np.float32)
+    x, dy = dev(rng.standard_normal((N, I)).astype(np.float32) * rows), dev(rng.standard_normal((N, O)).astype(np.float32) * rows)
+    x[N // 2, 3] = float("inf")
+    y, dx = torch.full((N, O), 7.0, device="cuda"), torch.full((N, I), 7.0, device="cuda")
+    ctx.counter_forward(x, st, sc, y, N, I, O, 11)
+    ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+    ctx.finish()
+    keep = torch.arange(N, device="cuda") != N // 2
+    for got, want in ((y, (x.double() @ w.double().T) * sc.double()), (dx, (dy * sc).double() @ w.double())):
+        err = (got[keep].double() - want[keep]).norm(dim=1) / want[keep].norm(dim=1)
+        assert float(err.max()) < 1e-6
+    assert not torch.isfinite(y[N // 2]).all() and torch.isfinite(y[keep]).all()
+    ctx.close()
