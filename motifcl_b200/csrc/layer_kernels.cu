@@ -93,12 +93,14 @@ struct RowParams {
     float* c;                 // [M, N]
     int M, N, K, in_features, C;
     int BN, stage_bytes;
+    int parts, kt_per;        // CTAs of a cluster along K and k-tiles of each
     int vec;                  // rows of a start on 16-byte boundaries
     int* err;
 };
 constexpr int kRowATerm = 128 * 128;          // bytes of one A term per stage
 
-template <bool DX>
+// CUT: K is cut over the CTAs of a cluster (a form of its own: with both ways out in it the other one lost 1 us a launch)
+template <bool DX, bool CUT>
 __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[2];
@@ -125,7 +127,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
     // A: 4 float4 of a k-tile per thread: rows tid / 16 + 32 j, the same 4 k in each.  Digits: units of 16 weights, up to 2 per
     // thread.  All addresses are formed once and advance by a constant per k-tile.
     struct Regs { float4 a[4], sc4; uint32_t w[2][3]; };
-    const int nkt = (p.K + 63) / 64, nu = 4 * BN;         // units per k-tile: BN rows x 4 (Y) or 64 rows x BN / 16 (dX)
+    const int kt0 = CUT ? (int)blockIdx.z * p.kt_per : 0, nkt = CUT ? min((p.K + 63) / 64 - kt0, p.kt_per) : (p.K + 63) / 64, nu = 4 * BN;         // units per k-tile: BN rows x 4 (Y) or 64 rows x BN / 16 (dX)
     const int rb = I / 4 * 3, ka = (tid & 15) * 4, arow = tid >> 4;
     const float* ap = p.a + (size_t)(m0 + arow) * p.K + ka;
     const size_t astep = (size_t)32 * p.K;
@@ -191,16 +193,16 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
     grid_release();
     for (int e = tid; e < 4096; e += kLThreads) lut[e] = digit[e & 63] | (digit[e >> 6] << 16);
     grid_wait();
-    load(0, r0);
-    if (nkt > 1) load(1, r1);
+    load(kt0, r0);
+    if (nkt > 1) load(kt0 + 1, r1);
     __syncthreads();
     const uint32_t tmem = tmem_slot;
     const uint32_t idesc = idesc_bf16(128, BN, 0, DX ? 1u : 0u);
     bool ok = true;
-    auto step = [&](int kt, Regs& r) {
-        const int s = kt & 1;
+    auto step = [&](int i, Regs& r) {
+        const int s = i & 1, kt = kt0 + i;
         const uint32_t st = stage0 + (uint32_t)s * (uint32_t)p.stage_bytes, sb = st + 3u * kRowATerm;
-        if (kt >= 2 && ok) ok = mbar_wait(bar0 + 8u * s, ((uint32_t)(kt >> 1) - 1u) & 1u, &abort_flag);
+        if (i >= 2 && ok) ok = mbar_wait(bar0 + 8u * s, ((uint32_t)(i >> 1) - 1u) & 1u, &abort_flag);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float4 v = r.a[j];
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
                 sts128u(sb + (u_at[j] ^ 16u), h[4], h[5], h[6], h[7]);
             }
         }
-        if (kt + 2 < nkt) load(kt + 2, r);
+        if (i + 2 < nkt) load(kt + 2, r);
         fence_proxy_async();
         __syncthreads();
         if (warp == 0) {
@@ -243,22 +245,72 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
                         umma_bf16(t == 0 ? tmem : tmem + cols, da + 2u * kk, db + (DX ? 128u : 2u) * kk, idesc,
-                                  (kt | kk) != 0 || t == 1 ? 1u : 0u);
+                                  (i | kk) != 0 || t == 1 ? 1u : 0u);
                 }
                 umma_commit(bar0 + 8u * s);
             }
             __syncwarp();
         }
     };
-    for (int kt = 0; kt < nkt; kt += 2) {
-        step(kt, r0);
-        if (kt + 1 < nkt) step(kt + 1, r1);
+    for (int i = 0; i < nkt; i += 2) {
+        step(i, r0);
+        if (i + 1 < nkt) step(i + 1, r1);
     }
     if (ok) ok = mbar_wait(bar0 + 8u * ((nkt - 1) & 1), (uint32_t)((nkt - 1) >> 1) & 1u, &abort_flag);
     if (!ok && tid == 0) atomicExch(p.err, kErrLayer);
     tc_fence_after();
-    // epilogue: warp = 32 rows x a quarter of the columns; a 32 x 33 tile in shared memory turns lane = row into lane = column
-    {
+    if constexpr (CUT) {
+        // K is cut over the CTAs of a cluster: each publishes both accumulators, then adds its share of the rows over all of them in rank
+        // order, the leading ones with their rounding errors carried along (a plain sum of rounded parts: error 4.3 -> 5.8e-8)
+        const int q = warp & 3, pitch = (BN + 4) * 4;
+        const uint32_t small = stage0 + 128u * (uint32_t)pitch;
+        for (int c0 = (warp >> 2) * 32; c0 < BN; c0 += 128) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t r[32];
+                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (half ? cols : 0u) + (uint32_t)c0, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    sts128u((half ? small : stage0) + (uint32_t)((q * 32 + lane) * pitch + (c0 + 4 * j) * 4), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            }
+        }
+        cluster_sync_all();
+        const int share = 128 / p.parts, quads = BN >> 2, row0 = (int)cluster_rank() * share;
+        const bool wide = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15) == 0;
+        auto add = [](float& s, float& e, float v, float w) {      // s + e += v + w, s rounded, e what that loses
+            const float t = __fadd_rn(s, v), u = __fsub_rn(t, s);
+            e = __fadd_rn(e, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(v, u)), w));
+            s = t;
+        };
+        for (int i = tid; i < share * quads; i += kLThreads) {
+            const int row = row0 + i / quads, c = (i % quads) * 4, m = m0 + row, n = n0 + c;
+            if (m >= p.M || n >= p.N) continue;
+            const uint32_t at = (uint32_t)(row * pitch + c * 4);
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), e = sum;
+            for (int k = 0; k < p.parts; k += 2) {                 // four remote loads in flight
+                const float4 v0 = ld_peer(stage0 + at, (uint32_t)k), w0 = ld_peer(small + at, (uint32_t)k);
+                const float4 v1 = ld_peer(stage0 + at, (uint32_t)k + 1), w1 = ld_peer(small + at, (uint32_t)k + 1);
+                add(sum.x, e.x, v0.x, w0.x); add(sum.y, e.y, v0.y, w0.y); add(sum.z, e.z, v0.z, w0.z); add(sum.w, e.w, v0.w, w0.w);
+                add(sum.x, e.x, v1.x, w1.x); add(sum.y, e.y, v1.y, w1.y); add(sum.z, e.z, v1.z, w1.z); add(sum.w, e.w, v1.w, w1.w);
+            }
+            sum.x += e.x; sum.y += e.y; sum.z += e.z; sum.w += e.w;
+            if (!DX) {
+                const float4 sc = load4(p.scale, n, p.N, false);
+                sum.x *= sc.x; sum.y *= sc.y; sum.z *= sc.z; sum.w *= sc.w;
+            }
+            float* out = p.c + (size_t)m * p.N + n;
+            if (wide) *reinterpret_cast<float4*>(out) = sum;
+            else {
+                out[0] = sum.x;
+                if (n + 1 < p.N) out[1] = sum.y;
+                if (n + 2 < p.N) out[2] = sum.z;
+                if (n + 3 < p.N) out[3] = sum.w;
+            }
+        }
+        cluster_sync_all();                                // before this CTA's shared memory goes
+    } else {
+        // epilogue: warp = 32 rows x a quarter of the columns; a 32 x 33 tile in shared memory turns lane = row into lane = column
         const int q = warp & 3, part = warp >> 2;
         float* tile = reinterpret_cast<float*>(smem) + warp * 32 * 33;
         for (int c0 = part * 32; c0 < BN && n0 + c0 < p.N; c0 += 128) {
@@ -572,15 +624,22 @@ bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features) {
 }
 
 namespace {
-// column tile of the row kernels: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per column)
-double rows_cost(int tokens, int N, int K, int sm_count, int* bn_out) {
+constexpr int kCutColumns = 192;              // both accumulators of a tile, published in shared memory: 200 KB
+// Column tile of the row kernels and CTAs that share its K: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per
+// column), in ns.  K is cut where that fits one wave: a cluster pays two barriers and the exchange of its tile, each CTA leaves out
+// k-tiles of a microsecond.  Forward, backward and update of one layer, us, uncut and cut: 128 -> 1200 at 200 rows 47 and 28, 1024 -> 1024 at 64
+// 78 and 51, 512 -> 128 at 128 42 and 32 (with 5 of each from launches that overlap); cut in four, 288 -> 288 at 256 would lose 2 of 30.
+double rows_cost(int tokens, int N, int K, int sm_count, int* bn_out, int* parts_out) {
     const int tm = (tokens + 127) / 128, nkt = (K + 63) / 64;
     double best = 1e30;
-    for (int bn = 32; bn <= 256; bn += 32) {
-        const int tiles = tm * ((N + bn - 1) / bn);
-        const double cost = (double)((tiles + sm_count - 1) / sm_count) * (nkt * (900.0 + 5.0 * bn) + 4000.0 + 6.0 * bn);
-        if (cost < best) { best = cost; *bn_out = bn; }
-    }
+    for (int bn = 32; bn <= 256; bn += 32)
+        for (int parts = 1; parts <= (bn <= kCutColumns ? 8 : 1); parts *= 2) {
+            const int tiles = tm * ((N + bn - 1) / bn), per = (nkt + parts - 1) / parts;
+            // clusters of 8 fit the GPCs 15 at a time, of 4 about 34
+            if (parts > 1 && ((parts - 1) * per >= nkt || tiles > (parts == 8 ? sm_count * 15 / 148 : parts == 4 ? sm_count * 34 / 148 : sm_count * 70 / 148))) continue;
+            const double cost = (double)((tiles * parts + sm_count - 1) / sm_count) * (per * (900.0 + 5.0 * bn) + 4000.0 + 6.0 * bn) + (parts > 1 ? 1500.0 + 40.0 * bn : 0.0);
+            if (cost < best) { best = cost; *bn_out = bn; *parts_out = parts; }
+        }
     return best;
 }
 // Rows per cluster and CTAs per cluster of the update: a CTA contracts its slice of the tokens (all columns, whatever the rows),
@@ -609,8 +668,8 @@ UpdateShape update_shape(int tokens, int I, int O, int sm_count) {
 // 1024 x 1024 23 / 26 at 1024, 42 / 36 at 4096, 81 / 53 at 8192 (5000).
 namespace { bool worth_workspace(double layer, double split) { return layer > 1.2 * split + 2.0; } }
 bool layer_rows_pay(size_t tokens, size_t N, size_t K, int sm_count) {
-    int bn = 0;
-    const double layer = 1.8 + 1.864 / 1900.0 * rows_cost((int)tokens, (int)N, (int)K, sm_count, &bn);
+    int bn = 0, parts = 0;
+    const double layer = 1.8 + 1.864 / 1900.0 * rows_cost((int)tokens, (int)N, (int)K, sm_count, &bn, &parts);
     const double bytes = (double)tokens * (12.0 * K + 4.0 * N), flops = 4.0 * tokens * N * K;
     // split by the terms' kernels: launches, the pass over the digits, then memory or the tensor pipe
     const double split = 13.8 + 0.0075 * K + 1.5e-6 * N * K + (bytes / 4.7e6 > flops / 1.1e9 ? bytes / 4.7e6 : flops / 1.1e9);
@@ -633,15 +692,28 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
     p.M = tokens; p.N = dx ? I : O; p.K = dx ? O : I; p.in_features = I; p.C = C;
     p.vec = (p.K & 3) == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0;
     p.err = err_word;
-    rows_cost(tokens, p.N, p.K, sm_count, &p.BN);
+    rows_cost(tokens, p.N, p.K, sm_count, &p.BN, &p.parts);
+    p.kt_per = ((p.K + 63) / 64 + p.parts - 1) / p.parts;
     const int tm = (tokens + 127) / 128;
     p.stage_bytes = 3 * kRowATerm + (dx ? (p.BN + 63) / 64 * 8192 : p.BN * 128);
-    const size_t smem = 2 * (size_t)p.stage_bytes + 1024;
-    const void* kern = dx ? reinterpret_cast<const void*>(layer_rows_kernel<true>) : reinterpret_cast<const void*>(layer_rows_kernel<false>);
-    cudaError_t e = ensure_dynamic_smem(kern, dx ? 18 : 17, max_smem);
+    const bool cut = p.parts > 1;
+    const size_t stages = 2 * (size_t)p.stage_bytes, sums = cut ? (size_t)2 * 128 * (p.BN + 4) * 4 : 0, smem = (stages > sums ? stages : sums) + 1024;
+    const auto kern = dx ? (cut ? layer_rows_kernel<true, true> : layer_rows_kernel<true, false>) : (cut ? layer_rows_kernel<false, true> : layer_rows_kernel<false, false>);
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (cut ? 45 : 17) + (dx ? 1 : 0), max_smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)tm, (unsigned)((p.N + p.BN - 1) / p.BN));
-    return launch_chained(dx ? layer_rows_kernel<true> : layer_rows_kernel<false>, grid, dim3(kLThreads), smem, stream, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)tm, (unsigned)((p.N + p.BN - 1) / p.BN), (unsigned)p.parts);
+    cfg.blockDim = dim3(kLThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // launch_chained, with clusters
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = (unsigned)p.parts;
+    cfg.attrs = attr;
+    cfg.numAttrs = cut ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,

@@ -244,7 +244,8 @@ __device__ __forceinline__ void deal_to_peer(uint32_t word_addr, uint32_t bar, i
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr(word_addr, 1)), "r"(word), "r"(b) : "memory");
 }
 
-template <int CG, int CAP, bool TOGETHER>
+// TURNED: products of the table may be (a form of its own: the second way out costs the others 1 %)
+template <int CG, int CAP, bool TOGETHER, bool TURNED>
 __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_constant__ TcTable<CAP> tab) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxStages + 4 + 2 * kDealt];
@@ -341,7 +342,8 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             const TcTile& P = sp[pi];
             const CUtensorMap* tmA = &tab.maps[3 * pi];
             const CUtensorMap* tmB = &tab.maps[3 * pi + 1];
-            const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn, turned = P.turned;
+            const int BN = P.BN, nterms = P.nterms, a_mn = P.a_mn, b_mn = P.b_mn;
+            const bool turned = TURNED && P.turned;
             const uint32_t bytes = (uint32_t)(CG * P.stage_bytes);
             const int m0 = (t.mt * CG + (int)rank) * BM, n0 = t.nt * BN + (int)rank * (BN / CG);
             const uint32_t b_bytes = (uint32_t)P.b_bytes;
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
         // of products with short main loops.
         auto row_bits = [&](const TcTile& P, const TcItem& t) {
             const int row = (t.mt * CG + (int)rank) * BM + q * 32 + lane;
-            const float* f = !P.turned ? P.a_inv : P.splits == 1 ? P.col_scale : nullptr;
+            const float* f = !(TURNED && P.turned) ? P.a_inv : P.splits == 1 ? P.col_scale : nullptr;
             return f && row < P.M ? __float_as_int(__ldg(f + row)) : 0x3F800000;
         };
         auto columns = [&](const TcTile& P) { return P.b_inv ? P.b_inv : P.splits == 1 ? P.col_scale : nullptr; };
@@ -495,7 +497,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
             }
             // undo the powers of two of the split: the row's and g in two halves, so that no step leaves fp32 unless the result does
             const int e = max(-252, (inv_bits >> 23) - 127 - g), e1 = e >> 1;
-            const bool turned = P.turned;
+            const bool turned = TURNED && P.turned;
             const float r1 = pow2(e1), r2 = turned ? __int_as_float(inv_bits) : pow2(e - e1);      // turned: the row's scale
             const CUtensorMap* tmC = &tab.maps[3 * pi + 2];
             const uint32_t acc = n_local & 1u, aph = (n_local >> 1) & 1u;
@@ -1217,8 +1219,10 @@ cudaError_t run_tc_table(const TcProblem* probs, int n, int* err_word, size_t ma
     if (stages < 2) return cudaErrorInvalidConfiguration;
     tab.stages = stages;
     const size_t smem = (size_t)stages * tab.slot_bytes + 1024 + kStageBytes;
-    const auto kern = tc_gemm_kernel<CG, CAP, TOGETHER>;
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), TOGETHER ? (CG == 2 ? 30 : 31) : CG == 2 ? (CAP > 1 ? 24 : 16) : (CAP > 1 ? 25 : 4), max_smem);
+    bool turned = false;
+    for (int i = 0; i < n; ++i) turned = turned || probs[i].turned;
+    const auto kern = turned ? tc_gemm_kernel<CG, CAP, TOGETHER, !TOGETHER> : tc_gemm_kernel<CG, CAP, TOGETHER, false>;
+    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), turned ? 41 + 2 * (CG == 2) + (CAP > 1) : TOGETHER ? (CG == 2 ? 30 : 31) : CG == 2 ? (CAP > 1 ? 24 : 16) : (CAP > 1 ? 25 : 4), max_smem);
     if (e != cudaSuccess) return e;
     int units = (sm_count / CG) * (two_ctas ? 2 : 1);
     if (units > items) units = items;

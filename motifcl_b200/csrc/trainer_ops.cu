@@ -605,35 +605,32 @@ __global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, 
     }
 }
 // The ordinary form: even heads of adjacent pairs, 16-byte aligned rows of whole heads.  Block = one position as above, thread = four
-// channels of a batch element, all of its loads in flight under the forming of the turns (rope_kernel loads every element
+// channels of a batch element, all of its loads in flight at once (rope_kernel loads every element
 // twice, once for its partner: 12 us for 16 x 256 rows of 288 channels, of which 1.5 are traffic).
 constexpr int kRopeIn = 4;             // quads of a thread in flight
 __global__ void __launch_bounds__(256) rope_quads_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
                                                          int channels, int head_dim, int rd, int token_offset, float theta, int inverse) {
     grid_release();
-    grid_wait();
     extern __shared__ float2 rot[];                   // (cos, sin) of pair i
     const int token = blockIdx.x, quads = channels >> 2;
     const int per = (batch + (int)gridDim.y - 1) / (int)gridDim.y, b0 = (int)blockIdx.y * per, n = (min(batch, b0 + per) - b0) * quads;
     const size_t step = (size_t)tokens * channels, start = (size_t)token * channels + b0 * step;
-    bool formed = false;
+    // the turns need nothing of memory: formed under the end of the launch before
+    for (int i = threadIdx.x; i < rd >> 1; i += 256) {
+        float angle = (float)(token_offset + token) / powf(theta, (float)(2 * i) / (float)head_dim);
+        if (inverse) angle = -angle;
+        float sn, cs;
+        sincosf(angle, &sn, &cs);
+        rot[i] = make_float2(cs, sn);
+    }
+    grid_wait();
+    __syncthreads();
     for (int u0 = threadIdx.x; u0 - (int)threadIdx.x < n; u0 += 256 * kRopeIn) {
         float4 v[kRopeIn];
 #pragma unroll
         for (int k = 0; k < kRopeIn; ++k) {
             const int u = u0 + k * 256, b = u / quads;
             if (u < n) v[k] = __ldg(reinterpret_cast<const float4*>(x + start + b * step) + (u - b * quads));
-        }
-        if (!formed) {
-            for (int i = threadIdx.x; i < rd >> 1; i += 256) {
-                float angle = (float)(token_offset + token) / powf(theta, (float)(2 * i) / (float)head_dim);
-                if (inverse) angle = -angle;
-                float sn, cs;
-                sincosf(angle, &sn, &cs);
-                rot[i] = make_float2(cs, sn);
-            }
-            __syncthreads();
-            formed = true;
         }
 #pragma unroll
         for (int k = 0; k < kRopeIn; ++k) {

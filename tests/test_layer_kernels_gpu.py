@@ -27,7 +27,8 @@ def _layer(N, I, O, seed):
             dev((rng.standard_normal((N, O)) * 0.02).astype(np.float32)))
 
 
-@pytest.mark.parametrize("N,I,O", SHAPES)
+# the last four: K cut over clusters of 8, 4 and 2, in parts that are not of one length, beside whole K
+@pytest.mark.parametrize("N,I,O", SHAPES + [(40, 1024, 1025), (130, 100, 2047), (4096, 288, 1536), (600, 640, 301)])
 def test_row_products_against_float64(ctx, N, I, O):
     st, sc, _, x, dy = _layer(N, I, O, N + I + O)
     w = torch.empty(O, I, device="cuda")
