@@ -815,15 +815,23 @@ int mcl_cuda_counter_update_fused(mcl_cuda_ctx* ctx, uint8_t* state, float* scal
         o_k = cv.reserve(plan.workspace_bytes);
     }
     void* wsp = nullptr;
-    if (layer_wanted(ctx, batch, in_features, out_features) && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+    const bool fused = mcl::layer_kernels_fit(batch, in_features, out_features) && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    // few multiply-adds without tensor cores: one launch, the same sums
+    const bool small = fused && !layer_wanted(ctx, batch, in_features, out_features) && (double)batch * (double)in_features * (double)out_features < (double)(1u << 22);
+    if (small || (fused && layer_wanted(ctx, batch, in_features, out_features) &&
         (!tc || mcl::layer_update_pays(batch, in_features, out_features, (out_features + tile_rows - 1) / tile_rows, ctx->sm_count) ||
-         ws_reserve(ctx, cv.off, &wsp) != MCL_CUDA_OK)) {
+         ws_reserve(ctx, cv.off, &wsp) != MCL_CUDA_OK))) {
         MCL_TRY(check_ptr(ctx, op, "scale", scale, 4));
         MCL_TRY(check_ptr(ctx, op, "v", v, 4));
         if (packed2_out) MCL_TRY(check_ptr(ctx, op, "packed2_out", packed2_out, 4));
         mcl::UpdateDesc d;
         d.state = state; d.scale = scale; d.v = v; d.grad_w = nullptr; d.packed2 = packed2_out;
         d.in_features = (int)in_features; d.rows = (int)out_features; d.row_offset = 0;
+        if (small) {
+            MCL_LAUNCH(ctx, op, mcl::launch_exact_update(d, grad_out, x, (int)batch, (int)C, lr, lr_scale, rms_beta, rms_eps, seed, ctx->seed_offset,
+                                                         ctx->sm_count, ctx->max_smem, ctx->stream));
+            return MCL_CUDA_OK;
+        }
         MCL_LAUNCH(ctx, op, mcl::launch_layer_update(d, grad_out, x, (int)batch, (int)C, lr, lr_scale, rms_beta, rms_eps, seed, ctx->seed_offset,
                                                      ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
         return MCL_CUDA_OK;

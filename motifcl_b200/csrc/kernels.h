@@ -67,6 +67,10 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
 cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
                                 float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int sm_count,
                                 size_t max_smem, cudaStream_t stream);
+// the same in the order of the exact kernels (simt_gemm.cu), for layers that fit those kernels and few multiply-adds
+cudaError_t launch_exact_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
+                                float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int sm_count, size_t max_smem,
+                                cudaStream_t stream);
 
 // simt_gemm.cu -- fp32 CUDA-core contractions (any shape; exact fp32 FMA accumulation)
 cudaError_t launch_simt_matmul_f32(const float* a, const float* b, float* c, int M, int K, int N,

@@ -617,6 +617,69 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
     else update_rows_by_group<WITH_Q>(u, my_rows, smem, L);
 }
 
+// ---- memory-native update of a small layer in the order of the exact kernels ----------------------------------------------
+// A CTA owns a few rows: a thread forms four columns of one of them, tokens ascending, multiply and add rounded separately (the sum of
+// simt_gemm.cu, bit for bit), into shared memory, where the update runs on whole rows.  Before, grad_w went through memory in up to eight row
+// tiles of two launches each, 5 to 19 us a launch: 64 x 64 at 32 tokens 66 us, 128 x 200 at 128 132 us.  Bound: the chain of loads and sums.
+// Forward, backward and update, before and now: 64 x 64 at 32 tokens 110 and 22 us, at 1000 907 and 61; 128 -> 200 at 128 195 and 31; 1000 -> 33 at
+// 100 333 and 55.
+template <bool WITH_Q, bool U16>
+__global__ void __launch_bounds__(kLThreads, 1) exact_update_kernel(const __grid_constant__ LayerUpdParams p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x, I = p.u.in_features, gpr = I >> 2, R = p.u.rows_per_batch;
+    const int row0 = (int)blockIdx.x * R, my_rows = min(R, p.O - row0);
+    const U16Layout L = u16_layout(I, R, WITH_Q, kLThreads / 64);
+    float4* gw_s = reinterpret_cast<float4*>(smem + L.off_gw);
+    UpdParams u = p.u;
+    u.state += (size_t)row0 * gpr * 3;
+    u.scale += row0; u.v += row0;
+    if (u.packed2) u.packed2 += (size_t)row0 * (I >> 4);
+    u.rows = my_rows; u.row_offset = row0;
+    grid_release();
+    if (U16) {
+        build_decode_lut(reinterpret_cast<DecodeLut*>(smem), u.C, tid, kLThreads);
+        build_tick_table(reinterpret_cast<uint32_t*>(smem + L.off_tick), u.C, tid, kLThreads);
+    }
+    grid_wait();
+    if (U16) u16_load_state<kLThreads>(u, L, smem, 0, my_rows);
+    constexpr int AHEAD = 8;                  // tokens loaded at a time, one such set ahead of the sums
+    struct Set { float4 x[AHEAD]; float d[AHEAD]; };
+    for (int i = tid; i < my_rows * gpr; i += kLThreads) {
+        const int r = i / gpr, g = i - r * gpr;
+        const float4* xp = reinterpret_cast<const float4*>(p.x) + g;
+        const float* dp = p.dy + row0 + r;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto load = [&](int t0, Set& s) {
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j) {
+                const int t = min(t0 + j, p.tokens - 1);
+                s.x[j] = __ldg(xp + (size_t)t * gpr);
+                s.d[j] = __ldg(dp + (size_t)t * p.O);
+            }
+        };
+        auto sum = [&](int t0, const Set& s) {
+#pragma unroll
+            for (int j = 0; j < AHEAD; ++j) {
+                if (t0 + j >= p.tokens) break;
+                acc.x = __fadd_rn(acc.x, __fmul_rn(s.d[j], s.x[j].x)); acc.y = __fadd_rn(acc.y, __fmul_rn(s.d[j], s.x[j].y));
+                acc.z = __fadd_rn(acc.z, __fmul_rn(s.d[j], s.x[j].z)); acc.w = __fadd_rn(acc.w, __fmul_rn(s.d[j], s.x[j].w));
+            }
+        };
+        Set a, b;
+        load(0, a);
+        for (int t0 = 0; t0 < p.tokens; t0 += 2 * AHEAD) {
+            if (t0 + AHEAD < p.tokens) load(t0 + AHEAD, b);
+            sum(t0, a);
+            if (t0 + 2 * AHEAD < p.tokens) load(t0 + 2 * AHEAD, a);
+            sum(t0 + AHEAD, b);
+        }
+        gw_s[r * gpr + (U16 ? swz4(g) : g)] = acc;
+    }
+    __syncthreads();
+    if (U16) update_u16_body<WITH_Q, true, kLThreads>(u, p.magic, 1u << 16, 1u << 17, 0, 1, false);
+    else update_rows_by_group<WITH_Q>(u, my_rows, smem, L);
+}
+
 }  // namespace
 
 bool layer_kernels_fit(size_t tokens, size_t in_features, size_t out_features) {
@@ -628,7 +691,7 @@ constexpr int kCutColumns = 192;              // both accumulators of a tile, pu
 // Column tile of the row kernels and CTAs that share its K: waves of CTAs times the time of a k-tile (conversion of A, then digits and MMAs per
 // column), in ns.  K is cut where that fits one wave: a cluster pays two barriers and the exchange of its tile, each CTA leaves out
 // k-tiles of a microsecond.  Forward, backward and update of one layer, us, uncut and cut: 128 -> 1200 at 200 rows 47 and 28, 1024 -> 1024 at 64
-// 78 and 51, 512 -> 128 at 128 42 and 32 (with 5 of each from launches that overlap); cut in four, 288 -> 288 at 256 would lose 2 of 30.
+// 78 and 51, 512 -> 128 at 128 42 and 32 (5 to 7 of each from launches that overlap); cut in four, 288 -> 288 at 256 would lose 2 of 30.
 double rows_cost(int tokens, int N, int K, int sm_count, int* bn_out, int* parts_out) {
     const int tm = (tokens + 127) / 128, nkt = (K + 63) / 64;
     double best = 1e30;
@@ -716,6 +779,41 @@ cudaError_t launch_layer_rows(int dx, const float* a, const uint8_t* state, cons
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
+namespace {
+void fill_update(LayerUpdParams& p, const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale, float rms_beta,
+                 float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int rows) {
+    const int I = d.in_features, O = d.rows;
+    p.dy = dy; p.x = x; p.tokens = tokens; p.O = O;
+    p.vec_dy = (O & 3) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
+    const uint32_t upr = (uint32_t)(I / 16);
+    p.magic = upr <= 1 ? 0u : (uint32_t)((0x100000000ull + upr - 1) / upr);
+    p.err = err_word;
+    UpdParams& u = p.u;
+    u.state = d.state; u.scale = d.scale; u.v = d.v; u.grad_w = nullptr; u.packed2 = d.packed2;
+    u.C = C; u.in_features = I; u.rows = O; u.row_offset = 0; u.rows_per_batch = rows;
+    u.state_align = (I % 64 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 15) == 0 && (reinterpret_cast<uintptr_t>(d.packed2) & 15) == 0) ? 16 : 4;
+    u.lr = lr; u.lr_scale = lr_scale; u.rms_beta = rms_beta; u.rms_eps = rms_eps; u.seed = seed; u.seed_offset = seed_offset;
+}
+}  // namespace
+
+cudaError_t launch_exact_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
+                                float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int sm_count, size_t max_smem,
+                                cudaStream_t stream) {
+    const int I = d.in_features, O = d.rows, gpr = I / 4;
+    const bool with_q = lr_scale != 0.0f, u16 = I % 16 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 3) == 0;
+    // rows of a CTA: all SMs first, then as many as its threads take at once
+    int R = (O + sm_count - 1) / sm_count;
+    if (R > kLThreads / gpr) R = kLThreads / gpr;
+    if (R < 1) R = 1;
+    LayerUpdParams p = {};
+    fill_update(p, d, dy, x, tokens, C, lr, lr_scale, rms_beta, rms_eps, seed, seed_offset, nullptr, R);
+    const auto kern = u16 ? (with_q ? exact_update_kernel<true, true> : exact_update_kernel<false, true>)
+                          : (with_q ? exact_update_kernel<true, false> : exact_update_kernel<false, false>);
+    const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), 48 + (u16 ? 2 : 0) + (with_q ? 1 : 0), max_smem);
+    if (e != cudaSuccess) return e;
+    return launch_chained(kern, dim3((unsigned)((O + R - 1) / R)), dim3(kLThreads), u16_layout(I, R, with_q, kLThreads / 64).total, stream, p);
+}
+
 cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const float* x, int tokens, int C, float lr, float lr_scale,
                                 float rms_beta, float rms_eps, uint32_t seed, const uint32_t* seed_offset, int* err_word, int sm_count,
                                 size_t max_smem, cudaStream_t stream) {
@@ -750,17 +848,8 @@ cudaError_t launch_layer_update(const UpdateDesc& d, const float* dy, const floa
         }
         if (p.np > 16) return cudaErrorInvalidConfiguration;
         p.off_stage = (int)base;
-        p.dy = dy; p.x = x; p.tokens = tokens; p.O = O;
+        fill_update(p, d, dy, x, tokens, C, lr, lr_scale, rms_beta, rms_eps, seed, seed_offset, err_word, R);
         p.slice = slice;
-        p.vec_dy = (O & 3) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
-        const uint32_t upr = (uint32_t)(I / 16);
-        p.magic = upr <= 1 ? 0u : (uint32_t)((0x100000000ull + upr - 1) / upr);
-        p.err = err_word;
-        UpdParams& u = p.u;
-        u.state = d.state; u.scale = d.scale; u.v = d.v; u.grad_w = nullptr; u.packed2 = d.packed2;
-        u.C = C; u.in_features = I; u.rows = O; u.row_offset = 0; u.rows_per_batch = R;
-        u.state_align = (I % 64 == 0 && (reinterpret_cast<uintptr_t>(d.state) & 15) == 0 && (reinterpret_cast<uintptr_t>(d.packed2) & 15) == 0) ? 16 : 4;
-        u.lr = lr; u.lr_scale = lr_scale; u.rms_beta = rms_beta; u.rms_eps = rms_eps; u.seed = seed; u.seed_offset = seed_offset;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(tiles * cs));
         cfg.blockDim = dim3(kLThreads);

@@ -201,3 +201,32 @@ def test_launches_that_overlap_give_the_bits_of_launches_apart(recorded):
         if n != "dw":                    # added up with atomics
             assert torch.equal(a[n], b[n]), n
     assert torch.isfinite(a["x"]).all() and not torch.equal(a["st"], st0)
+
+
+@pytest.mark.parametrize("lr_scale", [0.0, 0.05])
+@pytest.mark.parametrize("N,I,O", [(1, 16, 1), (33, 64, 32), (35, 68, 37), (17, 1000, 149), (8, 1024, 300), (129, 128, 200), (1000, 64, 64), (65, 48, 1300), (7, 4, 2)])
+def test_small_products_and_updates_in_the_order_of_the_reference(orc, N, I, O, lr_scale):
+    """Below 2^22 multiply-adds, bit for bit: tokens and features ascending, multiply and add rounded apart, whatever part of a tile of
+    16, a slice of 64 or a set of eight tokens exists; the update in one launch, with and without 2-bit words."""
+    from motifcl_b200 import Context
+    st, sc, v, x, dy = _layer(N, I, O, N + I + O)
+    hy = (3e-3, lr_scale, 0.9, 1e-3, 4242)
+    own = Context.on_torch_stream(0)
+    y, dx = torch.full((N, O), 7.0, device="cuda"), torch.full((N, I), 7.0, device="cuda")
+    p2 = torch.zeros(O, I // 16, dtype=torch.int32, device="cuda") if I % 16 == 0 else None
+    h = lambda a: a.cpu().numpy().copy()
+    hst, hsc, hv, hx, hdy = h(st), h(sc), h(v), h(x), h(dy)
+    own.counter_forward(x, st, sc, y, N, I, O, 11)
+    own.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+    before = own.launch_count
+    own.counter_update_fused(st, sc, v, dy, x, p2, 11, I, O, N, *hy)
+    own.finish()
+    assert own.launch_count - before == 1
+    assert np.array_equal(h(y).view(np.uint32), orc.forward(hx, hst, hsc, 11, O).view(np.uint32))
+    assert np.array_equal(h(dx).view(np.uint32), orc.backward_input(hdy, hst, hsc, 11, I).view(np.uint32))
+    e = orc.update_fused(hst, hsc, hv, hdy, hx, 11, *hy)
+    assert np.array_equal(h(st), e[0])
+    assert np.array_equal(h(sc).view(np.uint32), e[1].view(np.uint32)) and np.array_equal(h(v).view(np.uint32), e[2].view(np.uint32))
+    if p2 is not None:
+        assert np.array_equal(h(p2).view(np.uint32).reshape(-1), np.asarray(e[3]).reshape(-1))
+    own.close()
