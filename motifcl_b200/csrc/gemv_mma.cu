@@ -58,7 +58,20 @@ struct MvTable {
     MvMat m[CAP];
 };
 constexpr int MV_GROUP_COST = 1;       // chunks that the end of a group counts for
+constexpr int MV_X_COST = 64;          // and the digits of another x, in the cluster whose run goes over to it: 1.6 us
 __host__ __device__ inline int mv_chunks(int I) { return (I + MV_CHUNK - 1) / MV_CHUNK; }
+
+// The first group at or behind cluster c's share of the cost, and its matrix (m: one at or before it).
+template <int CAP>
+__host__ __device__ inline int mv_cut(const MvTable<CAP>& p, int c, int clusters, int& m) {
+    if (c == clusters) return p.groups;
+    const long long t = p.cost * c / clusters;
+    while (m + 1 < p.n && t >= p.m[m + 1].cost) ++m;
+    const int per = mv_chunks(p.m[m].I) + MV_GROUP_COST, end = m + 1 < p.n ? p.m[m + 1].first : p.groups;
+    const int f = p.m[m].first + (int)((t - p.m[m].cost + per - 1) / per);
+    if (f >= end && m + 1 < p.n) ++m;
+    return f < end ? f : end;
+}
 
 __device__ __forceinline__ uint4 mv_load(const uint4* p) {
     uint4 v;
@@ -91,18 +104,10 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
     const int M = p.M, Mp = M == 1 ? 2 : M;
     int mat = 0, g_begin, g_end;                    // matrix of the group at hand; this cluster's groups
     if (LIST) {
-        // the first group at or behind a share of the cost, and its matrix
-        auto cut = [&](int c, int& m) -> int {
-            const long long t = p.cost * c / (gridDim.x >> lg_s);
-            while (m + 1 < p.n && t >= p.m[m + 1].cost) ++m;
-            const int per = mv_chunks(p.m[m].I) + MV_GROUP_COST, end = m + 1 < p.n ? p.m[m + 1].first : p.groups;
-            const int f = p.m[m].first + (int)((t - p.m[m].cost + per - 1) / per);
-            if (f >= end && m + 1 < p.n) ++m;
-            return min(f, end);
-        };
+        const int clusters = gridDim.x >> lg_s;
         int behind = 0;
-        g_begin = cut(cid, mat);
-        g_end = (cid + 1) * S == (int)gridDim.x ? p.groups : cut(cid + 1, behind);
+        g_begin = mv_cut(p, cid, clusters, mat);
+        g_end = mv_cut(p, cid + 1, clusters, behind);
     } else {
         g_begin = cid * p.groups_q + min(cid, p.groups_r);
         g_end = g_begin + p.groups_q + (cid < p.groups_r ? 1 : 0);
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
 }
 
 template <int NT, int R, int CAP>
-cudaError_t mv_launch(MvTable<CAP>& p, int segments, int sm_count, size_t max_smem, int slot, bool follows, const cudaGraphNode_t* nodes, cudaStream_t stream) {
+cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, bool follows, const cudaGraphNode_t* nodes, cudaStream_t stream) {
     constexpr bool LIST = CAP > 1;
     const int Mp = p.M == 1 ? 2 : p.M, S = 1 << p.log_s;
     const size_t group_bytes = (size_t)S * Mp * MV_ROWS * 8;
@@ -377,12 +382,24 @@ cudaError_t mv_launch(MvTable<CAP>& p, int segments, int sm_count, size_t max_sm
     p.groups_q = p.groups / clusters; p.groups_r = p.groups % clusters;
     const size_t budget = max_smem - 4096;
     const size_t room = p.xq_bytes < budget ? budget - p.xq_bytes : 0;
-    // Groups of a cluster at most (one segment: all of them have one length, and a share of the cost, rounded to whole chunks, has the
-    // starts of groups / clusters + 2 of them at most); with several segments there are several rounds.
-    const int most = !LIST ? p.groups_q + (p.groups_r ? 1 : 0) : segments == 1 ? p.groups / clusters + 2 : p.groups;
-    int bufs = 1;
+    // The longest run of one cluster with one x.  Two buffers where a cluster takes more than one.  Room for more than that would keep the CTAs of
+    // the launch behind this one off the SMs until it ends: blocks of 14336 x 4096 whose w3 and w2 share a list, one row, 41.6 us with the room for
+    // all groups, 36.0 so, 35.8 with MV_X_COST (38.6 as single launches); of 5632 x 2048 17.4, 16.1, 15.7 (19.5).
+    int most = 1, bufs = 1;
+    if (!LIST) most = p.groups_q + (p.groups_r ? 1 : 0);
+    for (int c = 0; LIST && c < clusters; ++c) {
+        int m = 0, behind = 0;
+        int begin = mv_cut(p, c, clusters, m);
+        const int end = mv_cut(p, c + 1, clusters, behind);
+        for (int k = m; begin < end; k = p.m[k].next) {
+            const int stop = std::min(end, p.m[k].next < p.n ? p.m[p.m[k].next].first : p.groups);
+            most = std::max(most, stop - begin);
+            if (stop < end) bufs = 2;
+            begin = stop;
+        }
+    }
     p.owned = (most + S - 1) / S;
-    if (segments > 1 || (size_t)p.owned * group_bytes > room) {
+    if ((size_t)p.owned * bufs * group_bytes > room) {
         bufs = 2;
         const int fit = (int)std::min((size_t)1 << 20, room / (2 * group_bytes));
         p.owned = std::min(p.owned, std::max(fit, 1));
@@ -439,12 +456,13 @@ cudaError_t mv_list(const GemvItem* items, int n, int M, bool follows, const cud
     p.n = n; p.M = M; p.log_s = mv_log_s(items[0].in_features);
     // one x after the other
     bool taken[CAP] = {};
-    int k = 0, segments = 0;
+    int k = 0;
     long long groups = 0;
     p.cost = 0;
     for (int i = 0; i < n; ++i) {
         if (taken[i]) continue;
         const int begin = k;
+        if (k > 0) p.cost += MV_X_COST;
         for (int j = i; j < n; ++j) {
             if (taken[j] || items[j].x != items[i].x || items[j].in_features != items[i].in_features) continue;
             taken[j] = true;
@@ -458,15 +476,14 @@ cudaError_t mv_list(const GemvItem* items, int n, int M, bool follows, const cud
             p.cost += g * (mv_chunks(m.I) + MV_GROUP_COST);
         }
         for (int j = begin; j < k; ++j) p.m[j].next = k;
-        ++segments;
     }
     if (groups > 0x3fffffff) return cudaErrorInvalidValue;
     p.groups = (int)groups;
     switch ((M + 1) / 2) {
-        case 1: return mv_launch<1, 4, CAP>(p, segments, sm_count, max_smem, 26, follows, nodes, stream);
-        case 2: return mv_launch<2, 3, CAP>(p, segments, sm_count, max_smem, 27, follows, nodes, stream);
-        case 3: return mv_launch<3, 2, CAP>(p, segments, sm_count, max_smem, 28, follows, nodes, stream);
-        default: return mv_launch<4, 2, CAP>(p, segments, sm_count, max_smem, 29, follows, nodes, stream);
+        case 1: return mv_launch<1, 4, CAP>(p, sm_count, max_smem, 26, follows, nodes, stream);
+        case 2: return mv_launch<2, 3, CAP>(p, sm_count, max_smem, 27, follows, nodes, stream);
+        case 3: return mv_launch<3, 2, CAP>(p, sm_count, max_smem, 28, follows, nodes, stream);
+        default: return mv_launch<4, 2, CAP>(p, sm_count, max_smem, 29, follows, nodes, stream);
     }
 }
 

@@ -499,11 +499,16 @@ long long gv_blocks(const GemvItem* items, int n) {        // k-blocks of 128 ro
 }
 }  // namespace
 
-// Against gemv_mma.cu (M <= 8), by k-blocks: that one needs no second launch and starts 5 us earlier, this one takes eight rows as fast as one.
-// us as gemv_mma / gemv_tc: M = 1 w1 and w3 of 14336 x 4096 (3584 k-blocks) 21 / 26, all 20 matrices of 4 blocks (25600) 81 / 60; M = 4
-// 3584 k-blocks 26 / 27, 2100 27 / 21; M = 8 4096 x 4096 (512) 9.6 / 12.9, q, k, v (768) 16.1 / 15.8, 14336 x 4096 (1792) 24.6 / 19.8.
+// Against gemv_mma.cu (M <= 8), by k-blocks: that one needs no second launch and starts 5 us earlier, this one takes eight rows as fast as one and
+// many xs as fast as few, which there are a round and new digits each.  us as gemv_mma / gemv_tc, alone.  Three xs and more: M = 1 2624 k-blocks
+// 18.9 / 22.7, 2800 21.4 / 25.0, 3936 37 / 23; M = 4 1400 18.6 / 18.6, 2624 31 / 23 (17.3 / 11.6 with other work beside it).  One or two: M = 1 w1
+// and w3 of 14336 x 4096 (3584) 21 / 26; M = 4 these 26.0 / 24.5, two of 14336 and 4096 x 4096 between single launches (2304) 16.1 / 18.4.  M = 8,
+// however many: 4096 x 4096 (512) 9.6 / 12.9, 720 18.6 / 18.8, 14336 x 4096 (1792) 24.6 / 19.8.
 bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count) {
-    return gv_blocks(items, n) >= (long long)sm_count * (M <= 2 ? 28 : M <= 4 ? 14 : 6);
+    int xs = 1;
+    for (int i = 1; i < n; ++i) xs += items[i].x != items[i - 1].x;
+    const int per = M > 4 ? 6 : xs > 2 ? (M > 2 ? 14 : 22) : (M > 2 ? 20 : 28);
+    return gv_blocks(items, n) >= (long long)sm_count * per;
 }
 
 cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
