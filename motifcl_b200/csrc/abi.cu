@@ -14,17 +14,19 @@
 #include "kernels.h"
 #include "motifcl_cuda.h"
 
-// The GEMV launches that stand at the end of a recording, with nothing else between them.
-struct GemvChain {
-    struct Launch {
-        bool tc;                           // two nodes of gemv_tc.cu, or one of gemv_mma.cu
-        cudaGraphNode_t node[2];
-        int M;
-        std::vector<mcl::GemvItem> items;
-    };
-    std::vector<Launch> launches;
-    cudaGraphNode_t tail = nullptr;        // node of the last one, and the capture it belongs to: a handle alone may come back for a
+// Decode GEMVs of a recording: launches that take a list of matrices each.
+struct GemvList {
+    bool tc;                               // two nodes of gemv_tc.cu, or one of gemv_mma.cu
+    cudaGraphNode_t node[2];               // what is recorded behind the launch depends on the last of them
+    int M;
+    std::vector<mcl::GemvItem> items;
+};
+struct GemvRecord {
+    std::vector<GemvList> lists;
+    size_t open = 0;                       // from here on: with nothing else between and behind them, open to further matrices
+    cudaGraphNode_t tail = nullptr;        // last node of the last one, and the capture it belongs to: a handle alone may come back for a
     unsigned long long capture = 0;        // node of a later one
+    void close() { open = lists.size(); tail = nullptr; }
 };
 
 struct mcl_cuda_ctx {
@@ -48,7 +50,7 @@ struct mcl_cuda_ctx {
     uint64_t lane_mark = 0;      // launches at the last lane_fork (when this context is a lane)
     bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end
     uint64_t recorded_launches = 0;
-    GemvChain gemvs;             // launches at the end of the recording
+    GemvRecord gemvs;            // of the recording
     int live_batches = 0;        // recorded batches not yet destroyed: they hold addresses inside the workspace
 };
 
@@ -465,6 +467,65 @@ int products_group(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     return MCL_CUDA_OK;
 }
 
+// The one node that the next launch of a recording will depend on, or null; *capture: id of the recording.
+cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx, unsigned long long* capture) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    if (!ctx->recording || cudaStreamGetCaptureInfo_v2(ctx->stream, &st, capture, &graph, &deps, &n) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
+}
+
+// The open list that `item` can join: the earliest one with room, behind which nothing reads or writes what the item writes, or writes
+// what it reads.  Null: none.
+GemvList* joinable(GemvRecord& rec, const mcl::GemvItem& item, int M, bool mma, bool tc) {
+    struct Range { uintptr_t begin, end; };
+    const auto range = [](const void* p, size_t bytes) { const uintptr_t b = reinterpret_cast<uintptr_t>(p); return Range{b, b + bytes}; };
+    const auto meet = [](Range a, Range b) { return a.begin < b.end && b.begin < a.end; };
+    const auto out = [&](const mcl::GemvItem& i, int m) { return range(i.y, (size_t)m * i.out_features * 4); };
+    const auto takes = [&](const mcl::GemvItem& i, int m, Range r) {
+        return meet(range(i.x, (size_t)m * i.in_features * 4), r) || meet(range(i.packed2, (size_t)i.in_features / 4 * i.out_features), r) ||
+               meet(range(i.scale, (size_t)i.out_features * 4), r);
+    };
+    GemvList* found = nullptr;
+    for (size_t l = rec.lists.size(); l-- > rec.open;) {
+        GemvList& at = rec.lists[l];
+        for (const mcl::GemvItem& i : at.items)
+            if (meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M))) return found;
+        if (at.M == M && at.items.size() < mcl::kGemvListCap &&
+            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items[0].in_features, item.in_features))) found = &at;
+    }
+    return found;
+}
+
+// The nodes of a recorded launch take its list, which has grown.
+cudaError_t join_gemv(mcl_cuda_ctx* ctx, GemvList& at) {
+    const mcl::GemvItem* items = at.items.data();
+    const int n = (int)at.items.size();
+    if (!at.tc) return mcl::launch_ternary_gemv_mma(items, n, at.M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
+    if (mcl::gemv_tc_workspace_bytes(items, n, at.M, ctx->sm_count) > ctx->ws_bytes) return cudaErrorMemoryAllocation;
+    return mcl::launch_ternary_gemv_tc(items, n, at.M, ctx->ws, 3, false, at.node, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
+}
+
+// The recording is complete: a list of gemv_mma.cu that has become long enough for gemv_tc.cu goes there.  Its node, on which whatever
+// was recorded behind it depends, becomes the contraction; the digits get a node in front of it.
+cudaError_t lay_out_gemvs(mcl_cuda_ctx* ctx, cudaGraph_t graph) {
+    for (GemvList& at : ctx->gemvs.lists) {
+        const mcl::GemvItem* items = at.items.data();
+        const int n = (int)at.items.size();
+        bool go = !at.tc && n > 1 && mcl::gemv_tc_workspace_bytes(items, n, at.M, ctx->sm_count) <= ctx->ws_bytes && mcl::gemv_tc_pays(items, n, at.M, ctx->sm_count);
+        for (const mcl::GemvItem& i : at.items) go = go && mcl::gemv_tc_supported(at.M, i.in_features, i.packed2);
+        if (!go) continue;
+        const cudaGraphNode_t nodes[2] = {nullptr, at.node[0]};
+        const cudaError_t e = mcl::launch_ternary_gemv_tc(items, n, at.M, ctx->ws, 3, false, nodes, graph, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
+        if (e != cudaSuccess) return e;
+        ++ctx->launches;
+    }
+    ctx->gemvs = GemvRecord();
+    return cudaSuccess;
+}
+
 }  // namespace
 
 extern "C" {
@@ -510,7 +571,7 @@ int mcl_cuda_batch_begin(mcl_cuda_ctx* ctx) {
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return fail_cuda(ctx, "batch_begin", e);
     ctx->recording = true;
-    ctx->gemvs = GemvChain();
+    ctx->gemvs = GemvRecord();
     ctx->recorded_launches = ctx->launches;
     return MCL_CUDA_OK;
 }
@@ -524,6 +585,8 @@ int mcl_cuda_batch_end(mcl_cuda_ctx* ctx, mcl_cuda_batch** out_batch) {
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess || graph == nullptr) { cudaGetLastError(); return fail_cuda(ctx, "batch_end", e); }
+    e = lay_out_gemvs(ctx, graph);
+    if (e != cudaSuccess) { cudaGraphDestroy(graph); return fail_cuda(ctx, "batch_end (decode lists)", e); }
     mcl_cuda_batch* b = new (std::nothrow) mcl_cuda_batch();
     if (!b) { cudaGraphDestroy(graph); return fail(ctx, MCL_CUDA_ENOMEM, "out of host memory"); }
     b->graph = graph;
@@ -565,6 +628,8 @@ int mcl_cuda_lane_fork(mcl_cuda_ctx* ctx, mcl_cuda_ctx* lane) {
     cudaError_t e = cudaEventRecord(lane->ev_fork, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(lane->stream, lane->ev_fork, 0);
     if (e != cudaSuccess) return fail_cuda(ctx, "lane_fork", e);
+    ctx->gemvs.close();                        // what the lane does from here on stands behind what was recorded
+    lane->gemvs = GemvRecord();
     lane->recording = ctx->recording;
     lane->lane_mark = lane->launches;
     return MCL_CUDA_OK;
@@ -576,6 +641,8 @@ int mcl_cuda_lane_join(mcl_cuda_ctx* ctx, mcl_cuda_ctx* lane) {
     cudaError_t e = cudaEventRecord(lane->ev_join, lane->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, lane->ev_join, 0);
     if (e != cudaSuccess) return fail_cuda(ctx, "lane_join", e);
+    ctx->gemvs.close();
+    lane->gemvs = GemvRecord();
     lane->recording = false;
     ctx->launches += lane->launches - lane->lane_mark;    // account the lane's kernels to the owner
     lane->launches = lane->lane_mark;
@@ -1479,64 +1546,6 @@ int mcl_cuda_peer_allreduce_f32(mcl_cuda_ctx* ctx, const void* const* peer_data,
     return MCL_CUDA_OK;
 }
 
-// The one node that the next launch of a recording will depend on, or null; *capture: id of the recording.
-static cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx, unsigned long long* capture) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    cudaGraph_t graph = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t n = 0;
-    if (!ctx->recording || cudaStreamGetCaptureInfo_v2(ctx->stream, &st, capture, &graph, &deps, &n) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
-}
-
-// The launch of the chain that `item` can join: the earliest one with room, behind which nothing reads or writes what the item
-// writes, or writes what it reads.  Null: none.
-static GemvChain::Launch* joinable(GemvChain& chain, const mcl::GemvItem& item, int M, bool mma, bool tc) {
-    struct Range { uintptr_t begin, end; };
-    const auto range = [](const void* p, size_t bytes) { const uintptr_t b = reinterpret_cast<uintptr_t>(p); return Range{b, b + bytes}; };
-    const auto meet = [](Range a, Range b) { return a.begin < b.end && b.begin < a.end; };
-    const auto out = [&](const mcl::GemvItem& i, int m) { return range(i.y, (size_t)m * i.out_features * 4); };
-    const auto takes = [&](const mcl::GemvItem& i, int m, Range r) {
-        return meet(range(i.x, (size_t)m * i.in_features * 4), r) || meet(range(i.packed2, (size_t)i.in_features / 4 * i.out_features), r) ||
-               meet(range(i.scale, (size_t)i.out_features * 4), r);
-    };
-    GemvChain::Launch* found = nullptr;
-    for (size_t l = chain.launches.size(); l-- > 0;) {
-        GemvChain::Launch& at = chain.launches[l];
-        for (const mcl::GemvItem& i : at.items)
-            if (meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M))) return found;
-        if (at.M == M && at.items.size() < mcl::kGemvListCap &&
-            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items[0].in_features, item.in_features))) found = &at;
-    }
-    return found;
-}
-
-// The nodes of a recorded launch take its list, which has grown.  The one node of gemv_mma.cu becomes the first of gemv_tc.cu where the
-// list is long enough for it and the second can stand right behind.
-static cudaError_t join_gemv(mcl_cuda_ctx* ctx, GemvChain::Launch& at, int M, bool last) {
-    const mcl::GemvItem* items = at.items.data();
-    const int n = (int)at.items.size();
-    const bool room = mcl::gemv_tc_workspace_bytes(items, n, M, ctx->sm_count) <= ctx->ws_bytes;
-    const auto tc = [&](int parts, const cudaGraphNode_t* nodes) {
-        return mcl::launch_ternary_gemv_tc(items, n, M, ctx->ws, parts, false, nodes, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
-    };
-    if (at.tc) return room ? tc(3, at.node) : cudaErrorMemoryAllocation;
-    bool can = room && last && mcl::gemv_tc_pays(items, n, M, ctx->sm_count);
-    for (const mcl::GemvItem& i : at.items) can = can && mcl::gemv_tc_supported(M, i.in_features, i.packed2);
-    if (!can) return mcl::launch_ternary_gemv_mma(items, n, M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
-    cudaError_t e = tc(1, at.node);
-    if (e != cudaSuccess) return e;
-    e = tc(2, nullptr);
-    if (e != cudaSuccess) {
-        mcl::launch_ternary_gemv_mma(items, n - 1, M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
-        return e;
-    }
-    ++ctx->launches;
-    at.node[1] = ctx->gemvs.tail = recorded_tail(ctx, &ctx->gemvs.capture);
-    at.tc = true;
-    return cudaSuccess;
-}
-
 int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* packed2,
                           const float* scale, float* y, size_t M, size_t in_features,
                           size_t out_features) {
@@ -1558,18 +1567,18 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
     if (mma || tc) {
         // Only in a recording is it known what runs before and after: a matrix joins a launch there where nothing that was recorded since
         // has to do with it.
-        GemvChain& chain = ctx->gemvs;
+        GemvRecord& rec = ctx->gemvs;
         unsigned long long capture = 0;
         const cudaGraphNode_t tail = recorded_tail(ctx, &capture);
-        const bool follows = tail != nullptr && tail == chain.tail && capture == chain.capture;
-        if (!follows) chain.launches.clear();
-        if (GemvChain::Launch* at = joinable(chain, item, (int)M, mma, tc)) {
+        const bool follows = tail != nullptr && tail == rec.tail && capture == rec.capture;
+        if (!follows) rec.close();
+        if (GemvList* at = joinable(rec, item, (int)M, mma, tc)) {
             at->items.push_back(item);
-            if (join_gemv(ctx, *at, (int)M, at == &chain.launches.back()) == cudaSuccess) return MCL_CUDA_OK;
+            if (join_gemv(ctx, *at) == cudaSuccess) return MCL_CUDA_OK;
             at->items.pop_back();
             cudaGetLastError();
         }
-        GemvChain::Launch at = {!mma || (tc && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count)), {}, (int)M, {item}};
+        GemvList at = {!mma || (tc && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count)), {}, (int)M, {item}};
         void* wsp = ctx->ws;
         if (tc) {
             // Where it can grow, room for the digits of more xs than this one, also for a call that does without: the launches of a recording
@@ -1583,17 +1592,16 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
             }
         }
         if (at.tc) {
-            for (int part = 0; part < 2 && at.tc; ++part) {
-                MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_tc(&item, 1, (int)M, wsp, 1 << part, follows, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
-                at.node[part] = recorded_tail(ctx, &chain.capture);
+            for (int part = 0; part < 2; ++part) {
+                MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_tc(&item, 1, (int)M, wsp, 1 << part, follows, nullptr, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream));
+                at.node[part] = recorded_tail(ctx, &rec.capture);
             }
-        }
-        if (!at.tc) {
+        } else {
             MCL_LAUNCH(ctx, op, mcl::launch_ternary_gemv_mma(&item, 1, (int)M, follows, nullptr, ctx->sm_count, ctx->max_smem, ctx->stream));
-            at.node[0] = recorded_tail(ctx, &chain.capture);
+            at.node[0] = recorded_tail(ctx, &rec.capture);
         }
-        chain.tail = at.node[at.tc ? 1 : 0];
-        if (chain.tail) chain.launches.push_back(at);
+        rec.tail = at.node[at.tc ? 1 : 0];
+        if (rec.tail) rec.lists.push_back(at);
         return MCL_CUDA_OK;
     }
     if (!exact && M == 1) {

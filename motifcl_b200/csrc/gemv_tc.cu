@@ -24,6 +24,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "kernels.h"
 #include "tc_ptx.cuh"
@@ -470,6 +471,11 @@ bool gv_map_2d(CUtensorMap* map, const void* basep, size_t inner_bytes, size_t r
 int gv_nq(int M) { return (4 * (M == 1 ? 2 : M) + 15) / 16 * 16; }
 size_t round_up(size_t n) { return (n + 1023) & ~size_t(1023); }
 constexpr size_t kGvCorr = 64 * sizeof(int);      // then up to 16 scales
+long long gv_blocks(const GemvItem* items, int n) {        // k-blocks of 128 rows
+    long long u = 0;
+    for (int i = 0; i < n; ++i) u += (items[i].out_features + (long long)GV_ROWS - 1) / GV_ROWS * ((items[i].in_features + GV_KB - 1) / GV_KB);
+    return u;
+}
 
 }  // namespace
 
@@ -488,16 +494,8 @@ size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count
         bytes += round_up((size_t)gv_nq(M) * items[i].in_features) + 1024;
         ++xs;
     }
-    return xs <= kGemvXCap ? bytes : ~size_t(0);
+    return xs <= kGemvXCap && gv_blocks(items, n) <= 0x3fffffff ? bytes : ~size_t(0);
 }
-
-namespace {
-long long gv_blocks(const GemvItem* items, int n) {        // k-blocks of 128 rows
-    long long u = 0;
-    for (int i = 0; i < n; ++i) u += (items[i].out_features + (long long)GV_ROWS - 1) / GV_ROWS * ((items[i].in_features + GV_KB - 1) / GV_KB);
-    return u;
-}
-}  // namespace
 
 // Against gemv_mma.cu (M <= 8), by k-blocks: that one needs no second launch and starts 5 us earlier, this one takes eight rows as fast as one and
 // many xs as fast as few, which there are a round and new digits each.  us as gemv_mma / gemv_tc, alone.  Three xs and more: M = 1 2624 k-blocks
@@ -511,8 +509,38 @@ bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count) {
     return gv_blocks(items, n) >= (long long)sm_count * per;
 }
 
+namespace {
+// A kernel node between `node` and what it depended on: `node` comes right behind it, overlapping at the seam.  It is a single kernel
+// afterwards (no clusters).
+cudaError_t put_before(cudaGraph_t graph, cudaGraphNode_t node, const cudaKernelNodeParams& kp) {
+    size_t n = 0;
+    cudaError_t e = cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &n);
+    if (e != cudaSuccess) return e;
+    std::vector<cudaGraphNode_t> from(n), to(n, node);
+    std::vector<cudaGraphEdgeData> edges(n);
+    if (n > 0) e = cudaGraphNodeGetDependencies_v2(node, from.data(), edges.data(), &n);
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeKernel;
+    np.kernel.func = kp.func; np.kernel.gridDim = kp.gridDim; np.kernel.blockDim = kp.blockDim;
+    np.kernel.sharedMemBytes = kp.sharedMemBytes; np.kernel.kernelParams = kp.kernelParams;
+    cudaGraphNode_t made = nullptr;
+    e = cudaGraphAddNode_v2(&made, graph, from.data(), edges.data(), n, &np);
+    if (e == cudaSuccess && n > 0) e = cudaGraphRemoveDependencies_v2(graph, from.data(), to.data(), edges.data(), n);
+    if (e != cudaSuccess) return e;
+    cudaGraphEdgeData seam = {};
+    seam.from_port = cudaGraphKernelNodePortProgrammatic;
+    seam.type = cudaGraphDependencyTypeProgrammatic;
+    e = cudaGraphAddDependencies_v2(graph, &made, &node, &seam, 1);
+    if (e != cudaSuccess) return e;
+    cudaKernelNodeAttrValue at = {};
+    at.clusterDim.x = at.clusterDim.y = at.clusterDim.z = 1;
+    return cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeClusterDimension, &at);
+}
+}  // namespace
+
 cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
-                                   int* err_word, int sm_count, size_t max_smem, cudaStream_t stream) {
+                                   cudaGraph_t graph, int* err_word, int sm_count, size_t max_smem, cudaStream_t stream) {
     const int Nq = gv_nq(M);
     // Two CTAs on every SM and tiles of 256 rows, or one and 128.  One row: 2100 k-blocks 22.6 and 20.8 us, 5760 26.8 and 35.0, 25600 60 and 118; 16
     // rows, alone and with other work beside them: 5760 35 / 26.8 and 43 / 19.7, 25600 80 / 68 and 141 / 66.
@@ -572,8 +600,7 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     // the tickets stand before the slots: one range
     g.clear = reinterpret_cast<int4*>(p.tickets);
     g.clear_n = (round_up(2 * sm_count * sizeof(int)) + (size_t)std::min<long long>(ctas, tiles) * RT * Nq * GV_ROWS * sizeof(int)) / 16;
-    // whole clusters of 8: the first launch may stand in a node of gemv_mma.cu
-    const int q_blocks = (g.n * g.groups + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS)) + 7) / 8 * 8;
+    const int q_blocks = g.n * g.groups + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS));
 
     const void* kern = RT == 2 ? reinterpret_cast<const void*>(gemv_tc_kernel<2>) : reinterpret_cast<const void*>(gemv_tc_kernel<1>);
     cudaError_t e = ensure_dynamic_smem(kern, RT == 2 ? 5 : 40, max_smem);
@@ -590,7 +617,7 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
         kp.gridDim = cfg.gridDim = dim3(q_blocks); kp.blockDim = cfg.blockDim = dim3(GQ_THREADS);
         kp.kernelParams = args;
         cfg.numAttrs = follows ? 1 : 0;
-        e = nodes ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : cudaLaunchKernelEx(&cfg, gemv_quantize_kernel, g);
+        e = !nodes ? cudaLaunchKernelEx(&cfg, gemv_quantize_kernel, g) : nodes[0] ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : put_before(graph, nodes[1], kp);
         if (e != cudaSuccess) return e;
     }
     if (parts & 2) {

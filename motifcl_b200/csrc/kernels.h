@@ -175,12 +175,12 @@ bool gemv_mma_joins(int first_in_features, int in_features);
 cudaError_t launch_ternary_gemv_mma(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count,
                                     size_t max_smem, cudaStream_t stream);
 // gemv_tc.cu -- M <= 16, two launches (two nodes): digits, integer tcgen05.  parts: bit 0 the first launch, bit 1 the second; with `nodes`,
-// the parts whose node takes the list.
+// the parts whose node takes the list.  nodes[0] null: the first gets a node of `graph` right before nodes[1].
 bool gemv_tc_supported(int M, int in_features, const void* packed2);
 bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count);                    // against gemv_mma.cu
-size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count);      // ~0: more xs than a launch takes
+size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count);      // ~0: more xs or k-blocks than a launch takes
 cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
-                                   int* err_word, int sm_count, size_t max_smem, cudaStream_t stream);
+                                   cudaGraph_t graph, int* err_word, int sm_count, size_t max_smem, cudaStream_t stream);
 
 // peer_reduce.cu -- one-shot sum of a small vector over the GPUs of a node (peer loads, bounded flag wait)
 constexpr int kPeerMaxWorld = 8;

@@ -174,3 +174,54 @@ def test_recorded_matrices_that_depend_on_one_another_keep_their_order(M, per):
         for t, w in zip((a, b, c), want):
             assert torch.equal(t, w)
         batch.close()
+
+
+@pytest.mark.parametrize("M,shapes", [(4, [(14336, 4096), (14336, 4096)]), (8, [(4096, 4096)] * 2), (3, [(9000, 512)] * 60), (12, [(4096, 4096)] * 2)])
+@pytest.mark.parametrize("by", ["lane", "event"])
+def test_work_beside_a_recorded_list_waits_for_its_matrices(M, shapes, by):
+    """A lane, or another stream by an event, reads and overwrites the first result while further matrices are recorded that the first
+    one's launch could take; the list then grows long enough for the other kernel."""
+    from motifcl_b200 import Context
+    rng = np.random.default_rng(M)
+    stream, ctx = _context()
+    side = torch.cuda.Stream(device=0)
+    with torch.cuda.stream(stream):
+        lane = Context(0) if by == "lane" else Context(0, side.cuda_stream)
+        x = {I: torch.from_numpy(rng.standard_normal((M, I)).astype(np.float32)).to(DEV) for _, I in shapes}
+        mats = [(lambda w, s: (w, torch.from_numpy(s).to(DEV)))(*_matrix(rng, O, I)[::2]) for O, I in shapes]
+        ys, want = [[torch.full((M, O), 5.0, device=DEV) for O, _ in shapes] for _ in range(2)]
+        seen = torch.zeros_like(ys[0])
+
+        def call(out, i):
+            O, I = shapes[i]
+            ctx.ternary_gemv(x[I], *mats[i], out[i], M, I, O)
+        for i in range(len(shapes)):
+            call(want, i)
+        ctx.finish()
+        lane.finish()
+        ctx.batch_begin()
+        call(ys, 0)
+        if by == "lane":
+            ctx.lane_fork(lane)
+        else:
+            side.wait_event(stream.record_event())
+        lane.eltwise(4, ys[0], None, seen, seen.numel(), 1.0)          # seen = y + 1
+        lane.eltwise(3, ys[0], None, ys[0], seen.numel(), 2.0)         # y = 2 y
+        for i in range(1, len(shapes)):
+            call(ys, i)
+        if by == "lane":
+            ctx.lane_join(lane)
+        else:
+            stream.wait_event(side.record_event())
+        batch = ctx.batch_end()
+        for _ in range(3):
+            for y in ys:
+                y.fill_(7.0)
+            batch.launch()
+            ctx.finish()
+            assert torch.allclose(seen, want[0] + 1.0, rtol=1e-6, atol=1e-5)
+            assert torch.allclose(ys[0], 2.0 * want[0], rtol=1e-6, atol=1e-5)
+            for y, w in zip(ys[1:], want[1:]):
+                assert torch.allclose(y, w, rtol=1e-6, atol=1e-5)
+        batch.close()
+        lane.close()
