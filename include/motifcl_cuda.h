@@ -76,9 +76,12 @@ size_t mcl_cuda_workspace_bytes(mcl_cuda_ctx* ctx);
  * A batch holds addresses inside the context's workspace: while any batch of a context is alive,
  * a call that would make the workspace grow is refused (MCL_CUDA_ERR_ARG, "workspace would grow")
  * instead of freeing memory the batch still points into; destroy the batches first, or run the
- * larger call once before recording.
+ * larger call once before recording.  Where a graph that the context does not count may hold such addresses (a
+ * capture of the caller, a batch in which the context was a lane), growth keeps the old memory until the context is
+ * destroyed.
  * Decode GEMVs (mcl_cuda_ternary_gemv) that follow one another in a recording share launches where none of them reads or
- * overwrites what another one writes; a batch then stands for fewer launches than calls.
+ * overwrites what another one writes; a batch then stands for fewer launches than calls.  Long lists of up to 8 rows take
+ * workspace, which batch_end makes where the context has none; where it cannot, they run without.
  * Recording captures the calling thread's work on the context's stream only.  Do not enqueue
  * work of other libraries that hands off to streams of their own (an NCCL collective through a
  * framework's process group, for one) between begin and end: such work is not part of the batch

@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <new>
 #include <set>
@@ -16,6 +17,7 @@
 
 // Decode GEMVs of a recording: launches that take a list of matrices each.
 struct GemvList {
+    mcl_cuda_ctx* ctx;                     // the recording context or a lane of it
     bool tc;                               // two nodes of gemv_tc.cu, or one of gemv_mma.cu
     cudaGraphNode_t node[2];               // what is recorded behind the launch depends on the last of them
     int M;
@@ -42,13 +44,18 @@ struct mcl_cuda_ctx {
     // grow-only workspace used by entry points that need scratch (row tiles of grad_w, ...)
     void* ws = nullptr;
     size_t ws_bytes = 0;
+    bool ws_recorded = false;    // the recording holds addresses inside it
+    bool ws_held = false;        // and so may a graph that live_batches does not count: a capture of the caller, a batch this context was a lane of
+    std::vector<void*> ws_kept;  // earlier ones that a graph may hold
+    size_t ws_kept_bytes = 0;
     // how the contractions run (mcl_cuda_set_gemm_mode)
     int gemm_mode = MCL_CUDA_GEMM_AUTO;
     int* err_word = nullptr;     // device word the tensor-core kernels set when a bounded wait gives up
     const uint32_t* seed_offset = nullptr;   // device word added to every update seed (mcl_cuda_set_seed_offset)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint64_t lane_mark = 0;      // launches at the last lane_fork (when this context is a lane)
-    bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end
+    bool recording = false;      // between mcl_cuda_batch_begin and mcl_cuda_batch_end, on a lane between fork and join
+    bool is_lane = false;        // of the recording
     uint64_t recorded_launches = 0;
     GemvRecord gemvs;            // of the recording
     int live_batches = 0;        // recorded batches not yet destroyed: they hold addresses inside the workspace
@@ -117,7 +124,40 @@ int check_hypers(mcl_cuda_ctx* ctx, const char* op, float lr, float lr_scale, fl
     return MCL_CUDA_OK;
 }
 
+// A larger workspace.  The old one is freed, or kept as long as the context where a graph may hold addresses inside it; the new one is then
+// half as large again at least where it can be, so that all kept ones together stay below twice the one in use.
+int ws_grow(mcl_cuda_ctx* ctx, size_t bytes) {
+    const bool keep = ctx->ws && (ctx->ws_held || ctx->ws_recorded || ctx->live_batches > 0);
+    if (!keep) {
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return fail_cuda(ctx, "workspace sync", e);
+        if (ctx->ws) cudaFree(ctx->ws);
+        ctx->ws = nullptr;
+        ctx->ws_bytes = 0;
+    }
+    void* fresh = nullptr;
+    size_t take = keep ? std::max(bytes, ctx->ws_bytes / 2 * 3) : bytes;
+    cudaError_t e = cudaMalloc(&fresh, take);
+    if (e != cudaSuccess && take > bytes) { cudaGetLastError(); e = cudaMalloc(&fresh, take = bytes); }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(ctx, MCL_CUDA_ENOMEM, "workspace allocation of " + std::to_string(bytes) + " bytes failed");
+    }
+    if (keep) { ctx->ws_kept.push_back(ctx->ws); ctx->ws_kept_bytes += ctx->ws_bytes; }
+    ctx->ws = fresh;
+    ctx->ws_bytes = take;
+    ctx->ws_held = ctx->ws_recorded = false;
+    return MCL_CUDA_OK;
+}
+// whether the caller captures the context's stream
+bool foreign_capture(const mcl_cuda_ctx* ctx) {
+    if (ctx->recording) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
 int ws_reserve(mcl_cuda_ctx* ctx, size_t bytes, void** out) {
+    const bool foreign = foreign_capture(ctx);
     if (bytes > ctx->ws_bytes) {
         if (ctx->recording)
             return fail(ctx, MCL_CUDA_EINVAL, "workspace would grow while recording a batch: run the same calls once unrecorded first");
@@ -126,23 +166,13 @@ int ws_reserve(mcl_cuda_ctx* ctx, size_t bytes, void** out) {
                                                   std::to_string(ctx->live_batches) + " recorded batch(es) hold addresses inside it: "
                                                   "run the largest call once before recording, or destroy the batches first");
         // a capture that the caller runs on the stream would be broken by the wait and the allocation
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        cudaError_t e = cudaStreamIsCapturing(ctx->stream, &st);
-        if (e != cudaSuccess) return fail_cuda(ctx, "workspace capture status", e);
-        if (st != cudaStreamCaptureStatusNone)
+        if (foreign)
             return fail(ctx, MCL_CUDA_EINVAL, "workspace would grow while the stream is being captured: run the same calls once uncaptured first");
-        e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return fail_cuda(ctx, "workspace sync", e);
-        if (ctx->ws) cudaFree(ctx->ws);
-        ctx->ws = nullptr;
-        ctx->ws_bytes = 0;
-        e = cudaMalloc(&ctx->ws, bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return fail(ctx, MCL_CUDA_ENOMEM, "workspace allocation of " + std::to_string(bytes) + " bytes failed");
-        }
-        ctx->ws_bytes = bytes;
+        const int rc = ws_grow(ctx, bytes);
+        if (rc != MCL_CUDA_OK) return rc;
     }
+    if (foreign || ctx->is_lane) ctx->ws_held = true;
+    else if (ctx->recording) ctx->ws_recorded = true;
     *out = ctx->ws;
     return MCL_CUDA_OK;
 }
@@ -508,21 +538,44 @@ cudaError_t join_gemv(mcl_cuda_ctx* ctx, GemvList& at) {
     return mcl::launch_ternary_gemv_tc(items, n, at.M, ctx->ws, 3, false, at.node, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
 }
 
-// The recording is complete: a list of gemv_mma.cu that has become long enough for gemv_tc.cu goes there.  Its node, on which whatever
-// was recorded behind it depends, becomes the contraction; the digits get a node in front of it.
+// The recording is complete: a list of gemv_mma.cu that has become long enough for gemv_tc.cu goes there, where its context's workspace
+// is large enough or can grow (the capture has ended; what the graph already holds of the old one is kept).  Its node, on which whatever was
+// recorded behind it depends, becomes the contraction; the digits get a node in front of it.
 cudaError_t lay_out_gemvs(mcl_cuda_ctx* ctx, cudaGraph_t graph) {
-    for (GemvList& at : ctx->gemvs.lists) {
+    std::vector<GemvList> lists;
+    lists.swap(ctx->gemvs.lists);
+    ctx->gemvs = GemvRecord();
+    std::vector<size_t> need(lists.size(), 0);         // 0: stays where it is
+    std::map<mcl_cuda_ctx*, size_t> most;
+    for (size_t l = 0; l < lists.size(); ++l) {
+        const GemvList& at = lists[l];
         const mcl::GemvItem* items = at.items.data();
         const int n = (int)at.items.size();
-        bool go = !at.tc && n > 1 && mcl::gemv_tc_workspace_bytes(items, n, at.M, ctx->sm_count) <= ctx->ws_bytes && mcl::gemv_tc_pays(items, n, at.M, ctx->sm_count);
+        if (at.ctx != ctx) {
+            std::lock_guard<std::mutex> lock(g_ctx_mutex);
+            if (!g_live_ctx.count(at.ctx)) continue;
+        }
+        bool go = !at.tc && mcl::gemv_tc_pays(items, n, at.M, ctx->sm_count);
         for (const mcl::GemvItem& i : at.items) go = go && mcl::gemv_tc_supported(at.M, i.in_features, i.packed2);
-        if (!go) continue;
+        const size_t bytes = go ? mcl::gemv_tc_workspace_bytes(items, n, at.M, ctx->sm_count) : ~size_t(0);
+        if (bytes == ~size_t(0)) continue;
+        need[l] = bytes;
+        most[at.ctx] = std::max(most[at.ctx], bytes);
+    }
+    for (const auto& m : most) {
+        const std::string error = m.first->error;
+        if (m.second > m.first->ws_bytes && ws_grow(m.first, m.second) != MCL_CUDA_OK) m.first->error = error;
+        if (m.first != ctx) m.first->ws_held = true;
+    }
+    for (size_t l = 0; l < lists.size(); ++l) {
+        const GemvList& at = lists[l];
+        if (need[l] == 0 || need[l] > at.ctx->ws_bytes) continue;
         const cudaGraphNode_t nodes[2] = {nullptr, at.node[0]};
-        const cudaError_t e = mcl::launch_ternary_gemv_tc(items, n, at.M, ctx->ws, 3, false, nodes, graph, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
+        const cudaError_t e = mcl::launch_ternary_gemv_tc(at.items.data(), (int)at.items.size(), at.M, at.ctx->ws, 3, false, nodes, graph, ctx->err_word,
+                                                          ctx->sm_count, ctx->max_smem, ctx->stream);
         if (e != cudaSuccess) return e;
         ++ctx->launches;
     }
-    ctx->gemvs = GemvRecord();
     return cudaSuccess;
 }
 
@@ -548,6 +601,7 @@ void mcl_cuda_destroy(mcl_cuda_ctx* ctx) {
     DeviceGuard guard(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     if (ctx->ws) cudaFree(ctx->ws);
+    for (void* w : ctx->ws_kept) cudaFree(w);
     if (ctx->err_word) cudaFree(ctx->err_word);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
@@ -559,7 +613,7 @@ const char* mcl_cuda_device_name(mcl_cuda_ctx* ctx) { return ctx ? ctx->name.c_s
 int mcl_cuda_sm_count(mcl_cuda_ctx* ctx) { return ctx ? ctx->sm_count : 0; }
 size_t mcl_cuda_device_memory_bytes(mcl_cuda_ctx* ctx) { return ctx ? ctx->device_mem : 0; }
 uint64_t mcl_cuda_launch_count(mcl_cuda_ctx* ctx) { return ctx ? ctx->launches : 0; }
-size_t mcl_cuda_workspace_bytes(mcl_cuda_ctx* ctx) { return ctx ? ctx->ws_bytes : 0; }
+size_t mcl_cuda_workspace_bytes(mcl_cuda_ctx* ctx) { return ctx ? ctx->ws_bytes + ctx->ws_kept_bytes : 0; }
 
 int mcl_cuda_batch_begin(mcl_cuda_ctx* ctx) {
     MCL_NEED_CTX(ctx);
@@ -584,8 +638,9 @@ int mcl_cuda_batch_end(mcl_cuda_ctx* ctx, mcl_cuda_batch** out_batch) {
     ctx->recording = false;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
-    if (e != cudaSuccess || graph == nullptr) { cudaGetLastError(); return fail_cuda(ctx, "batch_end", e); }
+    if (e != cudaSuccess || graph == nullptr) { cudaGetLastError(); ctx->ws_recorded = false; return fail_cuda(ctx, "batch_end", e); }
     e = lay_out_gemvs(ctx, graph);
+    ctx->ws_recorded = false;                   // from here on the batch counts
     if (e != cudaSuccess) { cudaGraphDestroy(graph); return fail_cuda(ctx, "batch_end (decode lists)", e); }
     mcl_cuda_batch* b = new (std::nothrow) mcl_cuda_batch();
     if (!b) { cudaGraphDestroy(graph); return fail(ctx, MCL_CUDA_ENOMEM, "out of host memory"); }
@@ -630,7 +685,7 @@ int mcl_cuda_lane_fork(mcl_cuda_ctx* ctx, mcl_cuda_ctx* lane) {
     if (e != cudaSuccess) return fail_cuda(ctx, "lane_fork", e);
     ctx->gemvs.close();                        // what the lane does from here on stands behind what was recorded
     lane->gemvs = GemvRecord();
-    lane->recording = ctx->recording;
+    lane->recording = lane->is_lane = ctx->recording;
     lane->lane_mark = lane->launches;
     return MCL_CUDA_OK;
 }
@@ -641,9 +696,10 @@ int mcl_cuda_lane_join(mcl_cuda_ctx* ctx, mcl_cuda_ctx* lane) {
     cudaError_t e = cudaEventRecord(lane->ev_join, lane->stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, lane->ev_join, 0);
     if (e != cudaSuccess) return fail_cuda(ctx, "lane_join", e);
+    ctx->gemvs.lists.insert(ctx->gemvs.lists.end(), lane->gemvs.lists.begin(), lane->gemvs.lists.end());
     ctx->gemvs.close();
     lane->gemvs = GemvRecord();
-    lane->recording = false;
+    lane->recording = lane->is_lane = false;
     ctx->launches += lane->launches - lane->lane_mark;    // account the lane's kernels to the owner
     lane->launches = lane->lane_mark;
     return MCL_CUDA_OK;
@@ -1578,18 +1634,16 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
             at->items.pop_back();
             cudaGetLastError();
         }
-        GemvList at = {!mma || (tc && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count)), {}, (int)M, {item}};
-        void* wsp = ctx->ws;
-        if (tc) {
-            // Where it can grow, room for the digits of more xs than this one, also for a call that does without: the launches of a recording
-            // may take the call together with others.
+        // up to 8 rows the workspace is taken outside captures only: what a recording makes of its lists is settled when it is complete
+        GemvList at = {ctx, !mma || (tc && !ctx->recording && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count) && !foreign_capture(ctx)), {}, (int)M, {item}};
+        void* wsp = nullptr;
+        if (at.tc) {
+            // more rows than gemv_mma.cu takes: with room for the digits of further xs, which the launches of a recording may take together
             const size_t need = mcl::gemv_tc_workspace_bytes(&item, 1, (int)M, ctx->sm_count);
-            if (need > ctx->ws_bytes && (at.tc || !ctx->recording)) {
-                const std::string error = ctx->error;
-                const int rc = ws_reserve(ctx, need + (size_t(16) << 20), &wsp);
-                if (rc != MCL_CUDA_OK && !mma) return rc;
-                if (rc != MCL_CUDA_OK) { ctx->error = error; at.tc = false; }
-            }
+            const std::string error = ctx->error;
+            const int rc = ws_reserve(ctx, mma || need <= ctx->ws_bytes ? need : need + (size_t(16) << 20), &wsp);
+            if (rc != MCL_CUDA_OK && !mma) return rc;
+            if (rc != MCL_CUDA_OK) { ctx->error = error; at.tc = false; }
         }
         if (at.tc) {
             for (int part = 0; part < 2; ++part) {
