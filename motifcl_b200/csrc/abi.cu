@@ -128,17 +128,21 @@ int check_hypers(mcl_cuda_ctx* ctx, const char* op, float lr, float lr_scale, fl
 // half as large again at least where it can be, so that all kept ones together stay below twice the one in use.
 int ws_grow(mcl_cuda_ctx* ctx, size_t bytes) {
     const bool keep = ctx->ws && (ctx->ws_held || ctx->ws_recorded || ctx->live_batches > 0);
-    if (!keep) {
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) return fail_cuda(ctx, "workspace sync", e);
-        if (ctx->ws) cudaFree(ctx->ws);
-        ctx->ws = nullptr;
-        ctx->ws_bytes = 0;
-    }
     void* fresh = nullptr;
     size_t take = keep ? std::max(bytes, ctx->ws_bytes / 2 * 3) : bytes;
     cudaError_t e = cudaMalloc(&fresh, take);
     if (e != cudaSuccess && take > bytes) { cudaGetLastError(); e = cudaMalloc(&fresh, take = bytes); }
+    if (!keep && ctx->ws) {
+        const cudaError_t busy = cudaStreamSynchronize(ctx->stream);
+        if (busy != cudaSuccess) { if (e == cudaSuccess) cudaFree(fresh); return fail_cuda(ctx, "workspace sync", busy); }
+        cudaFree(ctx->ws);
+        ctx->ws = nullptr;
+        if (e != cudaSuccess) {            // both do not fit side by side
+            cudaGetLastError();
+            e = cudaMalloc(&fresh, bytes);
+            if (e != cudaSuccess && cudaMalloc(&ctx->ws, ctx->ws_bytes) != cudaSuccess) { ctx->ws = nullptr; ctx->ws_bytes = 0; }
+        }
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(ctx, MCL_CUDA_ENOMEM, "workspace allocation of " + std::to_string(bytes) + " bytes failed");

@@ -167,3 +167,19 @@ def test_lists_of_a_recording_get_workspace_beside_a_batch_that_holds_some(on):
         if who is not ctx:
             who.close()
         ctx.close()
+
+
+def test_growth_that_fails_leaves_the_workspace():
+    """A call whose terms no device can hold (its sizes are refused before anything is read)."""
+    from motifcl_b200 import MotifclCudaError
+    stream, ctx = _context()
+    f = _Forward(4)
+    with torch.cuda.stream(stream):
+        want = f.eager(ctx)
+        before = ctx.workspace_bytes
+        with pytest.raises(MotifclCudaError, match="workspace allocation"):
+            ctx.counter_forward(f.x, f.state, f.scale, f.y, 1 << 29, I, O, 11)
+        assert ctx.workspace_bytes == before
+        f.y.fill_(5.0)
+        assert torch.equal(f.eager(ctx), want)
+        ctx.close()
