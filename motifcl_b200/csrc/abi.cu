@@ -528,7 +528,7 @@ GemvList* joinable(GemvRecord& rec, const mcl::GemvItem& item, int M, bool mma, 
         for (const mcl::GemvItem& i : at.items)
             if (meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M))) return found;
         if (at.M == M && at.items.size() < mcl::kGemvListCap &&
-            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items[0].in_features, item.in_features))) found = &at;
+            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items.data(), (int)at.items.size(), item.in_features))) found = &at;
     }
     return found;
 }

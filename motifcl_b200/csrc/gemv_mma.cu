@@ -45,12 +45,13 @@ struct MvMat {
     int I, O;
     int first;                         // number of its first group
     int next;                          // the first matrix behind it that has another x
+    int log_k;                         // slices of K that a CTA takes (one, or two in a cluster of half as many CTAs as slices)
 };
 template <int CAP>         // one matrix, or kGemvListCap
 struct MvTable {
     long long cost;
     int n, groups, M;
-    int log_s;                         // CTAs of a cluster
+    int log_s, log_p;                  // CTAs of a cluster; slices of the matrix that has most
     int groups_q, groups_r;            // one matrix: groups of a cluster (the first groups_r clusters take one more)
     int block;                         // groups whose partial sums are held at a time
     int owned;                         // of them, the most that one CTA of the cluster finishes
@@ -96,8 +97,9 @@ __device__ __forceinline__ uint32_t mv_word(const uint4& v, int q) { return q ==
 template <int NT, int R, bool LIST>
 __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_constant__ MvTable<LIST ? kGemvListCap : 1> p) {
     extern __shared__ __align__(128) unsigned char mv_smem[];
-    __shared__ unsigned int amax[8];
-    __shared__ int corr[NT * 8];
+    constexpr int KS = LIST ? 2 : 1;                // slices of a CTA
+    __shared__ unsigned int amax[KS][8];
+    __shared__ int corr[KS][NT * 8];
     __shared__ double xscale[2][MV_MAX_S][8];       // of every slice: the value of one unit of its whole numbers; two segments
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tq = lane & 3;
     const int lg_s = p.log_s, S = 1 << lg_s, rank = blockIdx.x & (S - 1), cid = blockIdx.x >> lg_s;
@@ -168,8 +170,8 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
     }
 #pragma unroll
     for (int j = 0; j < R; ++j) load(w[j]);
-    if (threadIdx.x < 8) amax[threadIdx.x] = 0u;
-    if (threadIdx.x < NT * 8) corr[threadIdx.x] = 0;
+    if (threadIdx.x < KS * 8) amax[0][threadIdx.x] = 0u;
+    if (threadIdx.x < KS * NT * 8) corr[0][threadIdx.x] = 0;
     if (S > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // only "this CTA runs": nothing to publish
     grid_release();
     grid_wait();
@@ -182,9 +184,11 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
     const int s_end = segment_end(mat), I = p.m[mat].I, NC = mv_chunks(I);
     const float* const x = p.m[mat].x;
     const int c0 = (rank * NC) >> lg_s, nc = (((rank + 1) * NC) >> lg_s) - c0;
+    const int lg_k = LIST ? p.m[mat].log_k : 0, slice0 = rank << lg_k;
+    const int mid = lg_k ? (((slice0 + 1) * NC) >> (lg_s + 1)) - c0 : nc;       // chunks of the first of two slices
     if (LIST && seg > 0) {
-        if (threadIdx.x < 8) amax[threadIdx.x] = 0u;
-        if (threadIdx.x < NT * 8) corr[threadIdx.x] = 0;
+        if (threadIdx.x < KS * 8) amax[0][threadIdx.x] = 0u;
+        if (threadIdx.x < KS * NT * 8) corr[0][threadIdx.x] = 0;
     }
     __syncthreads();
 
@@ -200,14 +204,15 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
                       max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu));
         }
         top = __reduce_max_sync(0xffffffffu, top);
-        if (lane == 0) atomicMax(&amax[m], top);
+        if (lane == 0) atomicMax(&amax[LIST && (unit - m * per_row) >> 1 >= mid][m], top);
     }
     __syncthreads();
 #pragma unroll 2
     for (int unit = warp; unit < Mp * per_row; unit += MV_WARPS) {
         const int mp = unit / per_row, quad = (unit - mp * per_row) * 32 + lane, k = k0 + quad * 4;
         const int m = M == 1 ? 0 : mp;
-        const unsigned int top = amax[m];
+        const int sl = LIST && (unit - mp * per_row) >> 1 >= mid;
+        const unsigned int top = amax[sl][m];
         int e = max((int)(top >> 23) - 126, -90);   // 2^e above every magnitude (of the smallest ones: 2^-90)
         if (top >= 0x7F800000u) e = 0;
         const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
@@ -237,21 +242,23 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
                                   ((grp16 >> 2) & 3) * 16) = make_uint4(r[0], r[1], r[2], r[3]);
 #pragma unroll
         for (int s = 4; s < 32; s <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
-        if (lane < 4) atomicAdd(&corr[mp * 4 + d], sum);
+        if (lane < 4) atomicAdd(&corr[sl][mp * 4 + d], sum);
     }
     __syncthreads();
     if (S > 1 && first) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // every CTA of the cluster runs
     first = false;
     if ((int)threadIdx.x < 8 * S && (int)(threadIdx.x & 7) < M) {
         const int m = threadIdx.x & 7;
-        const unsigned int top = amax[m];
-        const int e = max((int)(top >> 23) - 126, -90);
-        const double v = top >= 0x7F800000u ? __longlong_as_double(0x7FF8000000000000ll)       // an infinity or NaN: so is the row
-                                            : __longlong_as_double((long long)(1023 + e - 30) << 52);
-        uint32_t to;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to)
-                     : "r"((uint32_t)__cvta_generic_to_shared(&xscale[seg & 1][rank][m])), "r"(threadIdx.x >> 3));
-        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
+        for (int sl = 0; sl < 1 << lg_k; ++sl) {
+            const unsigned int top = amax[sl][m];
+            const int e = max((int)(top >> 23) - 126, -90);
+            const double v = top >= 0x7F800000u ? __longlong_as_double(0x7FF8000000000000ll)       // an infinity or NaN: so is the row
+                                                : __longlong_as_double((long long)(1023 + e - 30) << 52);
+            uint32_t to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to)
+                         : "r"((uint32_t)__cvta_generic_to_shared(&xscale[seg & 1][slice0 + sl][m])), "r"(threadIdx.x >> 3));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
+        }
     }
 
     // -- the contraction ---------------------------------------------------------------------------------------------
@@ -259,7 +266,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
 #pragma unroll 1
     for (int gb = s_begin; gb < s_end; gb += p.block, parity ^= 1) {
         const int ge = min(gb + p.block, s_end);
-        const uint32_t part = (uint32_t)(parity * S) * part_bytes;
+        const uint32_t part = (uint32_t)(parity << p.log_p) * part_bytes;
         int acc[2][NT][4] = {};
         int cc = 0;
 #pragma unroll 1
@@ -289,15 +296,16 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
                         }
                     }
                     load(w[j]);
-                    if (++cc == nc) {
-                        // the slice of this group is complete: its sums, two digits to a word, go to the CTA that finishes the group
-                        const int li = grp - gb;
+                    ++cc;
+                    if (cc == nc || (LIST && cc == mid)) {
+                        // a slice of this group is complete: its sums, two digits to a word, go to the CTA that finishes the group
+                        const int li = grp - gb, sl = LIST && cc > mid;
                         uint32_t dst;
                         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
-                                     : "r"(part0 + part + rank * part_bytes + (uint32_t)((li >> lg_s) * Mp) * (MV_ROWS * 8u)), "r"(li & (S - 1)));
+                                     : "r"(part0 + part + (slice0 + sl) * part_bytes + (uint32_t)((li >> lg_s) * Mp) * (MV_ROWS * 8u)), "r"(li & (S - 1)));
 #pragma unroll
                         for (int t = 0; t < NT; ++t) {
-                            const int s0 = corr[t * 8 + 2 * tq], s1 = corr[t * 8 + 2 * tq + 1], m = 2 * t + (tq >> 1);
+                            const int s0 = corr[sl][t * 8 + 2 * tq], s1 = corr[sl][t * 8 + 2 * tq + 1], m = 2 * t + (tq >> 1);
 #pragma unroll
                             for (int h = 0; h < 4; ++h) {
                                 const int a0 = acc[h >> 1][t][2 * (h & 1)] - s0, a1 = acc[h >> 1][t][2 * (h & 1) + 1] - s1;
@@ -308,8 +316,10 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
 #pragma unroll
                             for (int i = 0; i < 4; ++i) acc[0][t][i] = acc[1][t][i] = 0;
                         }
-                        cc = 0;
-                        grp += MV_WARPS;
+                        if (cc == nc) {
+                            cc = 0;
+                            grp += MV_WARPS;
+                        }
                     }
                 }
             }
@@ -344,17 +354,17 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
             if (o >= O) continue;
             const float sc = __ldg(p.m[k].scale + o);
             const size_t at = (size_t)(slot * Mp * MV_ROWS + j) * 8;
-            double sum = 0.0;
+            double sum = 0.0, rest = 0.0;
 #pragma unroll 4
-            for (int s = 0; s < S; ++s) {
+            for (int s = 0; s < S << lg_k; ++s) {
                 const int2 v = *reinterpret_cast<const int2*>(src + s * part_bytes + at);
-                double t = (double)v.x * 65536.0 + (double)v.y;
+                sum += xscale[seg & 1][s][m] * ((double)v.x * 65536.0 + (double)v.y);
                 if (M == 1) {
                     const int2 u = *reinterpret_cast<const int2*>(src + s * part_bytes + at + MV_ROWS * 8);
-                    t += ((double)u.x * 65536.0 + (double)u.y) * (1.0 / 1073741824.0);
+                    rest += xscale[seg & 1][s][m] * ((double)u.x * 65536.0 + (double)u.y);
                 }
-                sum += xscale[seg & 1][s][m] * t;
             }
+            if (M == 1) sum += rest * (1.0 / 1073741824.0);
             p.m[k].y[(size_t)m * O + o] = (float)((double)sc * sum);
         }
     }
@@ -368,7 +378,7 @@ template <int NT, int R, int CAP>
 cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, bool follows, const cudaGraphNode_t* nodes, cudaStream_t stream) {
     constexpr bool LIST = CAP > 1;
     const int Mp = p.M == 1 ? 2 : p.M, S = 1 << p.log_s;
-    const size_t group_bytes = (size_t)S * Mp * MV_ROWS * 8;
+    const size_t group_bytes = ((size_t)Mp << p.log_p) * MV_ROWS * 8;
     int nc = 1;
     for (int i = 0; i < p.n; ++i) nc = std::max(nc, (mv_chunks(p.m[i].I) + S - 1) / S);
     p.xq_bytes = nc * NT * 2048;
@@ -399,6 +409,7 @@ cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, 
         }
     }
     p.owned = (most + S - 1) / S;
+    if (p.log_p > p.log_s) { p.owned = (p.owned + 1) / 2; bufs = 2; }           // twice the slices in the same room
     if ((size_t)p.owned * bufs * group_bytes > room) {
         bufs = 2;
         const int fit = (int)std::min((size_t)1 << 20, room / (2 * group_bytes));
@@ -416,7 +427,10 @@ cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, 
         kp.func = const_cast<void*>(kern);
         kp.gridDim = dim3(clusters * S); kp.blockDim = dim3(MV_THREADS); kp.sharedMemBytes = (unsigned)smem;
         kp.kernelParams = args;
-        return cudaGraphKernelNodeSetParams(nodes[0], &kp);
+        cudaKernelNodeAttrValue cluster = {};
+        cluster.clusterDim.x = S; cluster.clusterDim.y = cluster.clusterDim.z = 1;
+        e = cudaGraphKernelNodeSetAttribute(nodes[0], cudaLaunchAttributeClusterDimension, &cluster);      // first: a list's clusters only shrink
+        return e == cudaSuccess ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : e;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(clusters * S); cfg.blockDim = dim3(MV_THREADS); cfg.stream = stream;
@@ -429,31 +443,37 @@ cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, 
     return cudaLaunchKernelEx(&cfg, gemv_mma_kernel<NT, R, LIST>, p);
 }
 
+}  // namespace
+
 // The widest portable cluster: the fixed part of a call (digits of a slice, sums of an output) shrinks with the slice (20 matrices
 // of an 8B-scale model, four rows of x: 379 / 262 / 206 us with 2 / 4 / 8).  A slice has one chunk at least.
-int mv_log_s(int in_features) {
+int gemv_log_slices(int in_features) {
     const int NC = (in_features + MV_CHUNK - 1) / MV_CHUNK;
     int s = 3;
     while ((1 << s) > NC) --s;
     return s;
 }
-
-}  // namespace
-
 bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem) {
     if (M < 1 || M > 8 || in_features % 64 != 0 || in_features < 64 || reinterpret_cast<uintptr_t>(packed2) % 16 != 0) return false;
-    const int S = 1 << mv_log_s(in_features), NC = (in_features + MV_CHUNK - 1) / MV_CHUNK;
+    const int S = 1 << gemv_log_slices(in_features), NC = (in_features + MV_CHUNK - 1) / MV_CHUNK;
     return (size_t)((NC + S - 1) / S) * ((M + 1) / 2) * 2048 + 2 * (size_t)S * (M == 1 ? 2 : M) * MV_ROWS * 8 + 4096 <= max_smem;
 }
 
-bool gemv_mma_joins(int first_in_features, int in_features) { return mv_chunks(in_features) >= 1 << mv_log_s(first_in_features); }
+// A list's clusters are those of its shortest rows, a CTA then takes two slices of longer ones (15 matrices of 1280 and 5120, one row: 18.6 us; in clusters of
+// eight, of which short rows leave three CTAs idle, 23).
+bool gemv_mma_joins(const GemvItem* items, int n, int in_features) {
+    int low = gemv_log_slices(in_features), high = low;
+    for (int i = 0; i < n; ++i) { low = std::min(low, gemv_log_slices(items[i].in_features)); high = std::max(high, gemv_log_slices(items[i].in_features)); }
+    return high - low <= 1;
+}
 
 namespace {
 template <int CAP>
 cudaError_t mv_list(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count, size_t max_smem,
                     cudaStream_t stream) {
     MvTable<CAP> p;
-    p.n = n; p.M = M; p.log_s = mv_log_s(items[0].in_features);
+    p.n = n; p.M = M; p.log_s = 3; p.log_p = 0;
+    for (int i = 0; i < n; ++i) { p.log_s = std::min(p.log_s, gemv_log_slices(items[i].in_features)); p.log_p = std::max(p.log_p, gemv_log_slices(items[i].in_features)); }
     // one x after the other
     bool taken[CAP] = {};
     int k = 0;
@@ -470,6 +490,7 @@ cudaError_t mv_list(const GemvItem* items, int n, int M, bool follows, const cud
             MvMat& m = p.m[k++];
             m.words = reinterpret_cast<const uint4*>(it.packed2); m.x = it.x; m.scale = it.scale; m.y = it.y;
             m.I = it.in_features; m.O = it.out_features;
+            m.log_k = gemv_log_slices(it.in_features) - p.log_s;
             m.first = (int)groups; m.cost = p.cost;
             const long long g = (it.out_features + (long long)MV_ROWS - 1) / MV_ROWS;
             groups += g;

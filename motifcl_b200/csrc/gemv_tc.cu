@@ -3,9 +3,13 @@
 //
 // CUDA cores cannot keep up with 4 weights per byte (one multiply-add per weight and
 // activation row), so the contraction runs as integer MMA, exactly:
-//   * each activation row is scaled to whole numbers of 30 bits and sign below its largest magnitude and written as four signed
-//     digits of base 256; digit d of row m is row 4m+d of an int8 matrix Xq [N, in] (N = 16, 32, 48 or 64).  One row alone has
-//     digit rows to spare: its second four hold the 30 bits that the first leave over;
+//   * each activation row is written as whole numbers of 30 bits and sign below its largest magnitude, four signed
+//     digits of base 256; digit d of row m is row 4m+d of an int8 matrix Xq [N, in] (N = 16, 32, 48 or 64).  One row alone is two: the second
+//     holds the 30 bits that the first leaves over;
+//   * up to 8 rows have 30 bits below the largest magnitude of each slice of K (gemv_mma.cu's slices and, bit for bit, its results).  As long as those
+//     magnitudes lie within 2^8 of one another, all slices are written in the unit of the finest, which takes a fifth digit, and the whole of K
+//     is one exact sum (which a double holds, so that gemv_mma.cu's sum of slices is exact as well).  For an x where they do not, every
+//     slice keeps its unit and is taken from the accumulator by itself;
 //   * a CTA streams [RT * 128 rows x 256 weights] tiles of packed 2-bit fields (f = t + 1) through TMA, four warps per 128 rows expand
 //     the fields to int8 in TENSOR MEMORY, and one thread issues kind::i8 MMAs  acc[128, N] += F . Xq^T  with the A operand from there;
 //   * sum_k x t = sum_k x f - sum_k x, so a per-row digit sum is subtracted at the end; digits are put together in whole numbers.
@@ -17,10 +21,11 @@
 // first weights are on their way meanwhile (programmatic dependent launch).
 //
 // What bounds it: an SM has to take 90 weights per clock at 6.5 TB/s (the copies alone run at 5.1 to 5.9 TB/s in these boxes).  20 matrices
-// of an 8B-scale model (210 MB) as one list take 60 us for one row of x, 66 for 8 and 80 for 16 (2.6 to 3.5 TB/s; 48, 54 and 68 with
-// other work beside them), where a launch or three per matrix took 157, 333 and 368.  MMAs issued from a single-lane branch cost 93 cycles
-// each whatever their N (62 us of an earlier 78 for one row); 64 digit columns bring 16 KB of digits beside 16 KB of words per
-// k-block, so two accumulators (RT = 2) share them: 16 rows 82 -> 80 us, one row 70 -> 60.
+// of an 8B-scale model (210 MB) as one list take 62 us for one row of x, 65 for 4, 74 for 8 and 81 for 16 (2.6 to 3.4 TB/s; 50, 52, 63 and 69 with
+// other work beside them), where a launch or three per matrix took 157, 333 and 368.  The fifth digit costs 4 rows 5 % and 8 rows 14 % (16 and 32 more
+// digit columns; without it, in the unit of the largest slice, the others would lose bits); an x in slices takes 94 us for one row, 188 for 8.
+// MMAs issued from a single-lane branch cost 93 cycles each whatever their N (62 us of an earlier 78 for one row); 64 digit columns bring 16 KB of
+// digits beside 16 KB of words per k-block, so two accumulators (RT = 2) share them: 16 rows 82 -> 80 us, one row 70 -> 60.
 #include <cuda.h>
 
 #include <algorithm>
@@ -42,16 +47,20 @@ constexpr int GV_TMEM = 256;           // columns of a CTA, half of an SM's: acc
 struct GvMat {
     const float* scale;
     float* y;
-    const int* corr;
-    const float* xscale;
-    int O, kblocks, x;
+    const long long* sums;     // of x: [slice][16 rows] its whole numbers added up
+    const double* units;       // and the value of one
+    int O, kblocks, x, log_s;
     int first, tile;   // numbers of its first unit (k-block of a tile) and tile
 };
 struct GvTable {
-    int n, units, tiles, M, Nq, stages;
+    int n, xs, tiles, M, Nq, stages;
+    int extra;         // first row of fifth digits
+    int cut_q, cut_r;  // units / CTAs, and what is over
     int* err;
     int* acc;          // slots of [RT][Nq][128] sums for tiles that a cut runs through, by tile or by the CTA that begins it, whichever are fewer
+    double* part;      // an x in slices: [CTA][not begun or begun][slice][row][RT * 128] sums of the tile at hand
     int* tickets;
+    const int* wide;   // [x][8]: whether a row of it has to be taken in slices
     GvMat m[kGemvListCap];
     CUtensorMap maps[kGemvListCap], xmaps[kGemvXCap];
 };
@@ -78,26 +87,78 @@ __device__ __forceinline__ void umma_i8_tsu(uint32_t tmem_c, uint32_t tmem_a, ui
                  ::"r"(tmem_c), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accum) : "memory");
 }
 
-// a CTA's units of one tile
-struct GvPart { int m, tile, kb0, nkb; };
-__device__ __forceinline__ GvPart gv_part(const GvTable& p, int u, int end, int m) {
-    while (m + 1 < p.n && u >= p.m[m + 1].first) ++m;
-    const int kbs = p.m[m].kblocks, local = u - p.m[m].first, tile = local / kbs, kb0 = local - tile * kbs;
-    return {m, tile, kb0, min(kbs - kb0, end - u)};
+__device__ __forceinline__ int gv_slice_at(int s, int kblocks, int log_s) { return (int)(((long long)s * kblocks) >> log_s); }
+// A CTA's units as parts: of one tile, or (SLICED, for the xs in `wide`) of one slice of K of a tile.  One division at the start.
+template <bool SLICED>
+struct GvParts {
+    const GvTable& p;
+    const uint32_t wide;
+    int u, end;                            // the next unit, and the one behind the last
+    int m = 0, kbs, log_s;                 // matrix of the part
+    int tile, kb0, nkb = 0, slice = 0, slice_end;
+    __device__ __forceinline__ GvParts(const GvTable& p, int begin, int end, uint32_t wide = 0) : p(p), wide(wide), u(begin), end(end) {
+        while (m + 1 < p.n && u >= p.m[m + 1].first) ++m;
+        open();
+        const int local = u - p.m[m].first;
+        tile = local / kbs;
+        kb0 = local - tile * kbs;
+        if (SLICED) skip();
+    }
+    __device__ __forceinline__ void open() {
+        kbs = p.m[m].kblocks;
+        log_s = SLICED && (wide >> p.m[m].x & 1) ? p.m[m].log_s : 0;
+        slice_end = SLICED ? gv_slice_at(1, kbs, log_s) : kbs;
+    }
+    __device__ __forceinline__ void skip() { while (slice_end <= kb0) slice_end = gv_slice_at(++slice + 1, kbs, log_s); }      // to the slice of kb0
+    __device__ __forceinline__ bool next() {           // false: no more
+        if (u >= end) return false;
+        if (nkb > 0) {
+            kb0 += nkb;
+            if (kb0 == kbs) {
+                kb0 = 0;
+                slice = 0;
+                ++tile;
+                if (m + 1 < p.n && u >= p.m[m + 1].first) { ++m; tile = 0; }
+                open();
+            }
+            if (SLICED) skip();
+        }
+        nkb = min(slice_end - kb0, end - u);
+        u += nkb;
+        return true;
+    }
+};
+// the first unit of a CTA: units * cta / CTAs
+__device__ __forceinline__ int gv_cut(const GvTable& p, int cta) { return p.cut_q * cta + (int)((uint32_t)(p.cut_r * cta) / gridDim.x); }
+// the CTAs that share the units from `begin` to `end`, one of which is `cta`
+__device__ __forceinline__ int gv_first_cta(const GvTable& p, int cta, int begin) { while (gv_cut(p, cta) > begin) --cta; return cta; }
+__device__ __forceinline__ int gv_last_cta(const GvTable& p, int cta, int end) { while (gv_cut(p, cta + 1) < end) ++cta; return cta; }
+
+__host__ __device__ inline int gv_rows(int M) { return M == 1 ? 2 : M; }        // rows of whole numbers
+// the xs to be taken in slices; a whole warp, after the wait for the launch before
+__device__ __forceinline__ uint32_t gv_wide(const GvTable& p) {
+    const int lane = threadIdx.x & 31, row = lane & 7;
+    uint32_t mask = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int x = 4 * i + (lane >> 3);
+        const uint32_t b = __ballot_sync(0xffffffffu, x < p.xs && row < p.M && *reinterpret_cast<const volatile int*>(p.wide + 8 * x + row) != 0);
+        for (int k = 0; k < 4; ++k) mask |= (b >> (8 * k) & 255u) ? 1u << (4 * i + k) : 0u;
+    }
+    return mask;
 }
-__device__ __forceinline__ int gv_cut(const GvTable& p, int cta) { return (int)((long long)p.units * cta / gridDim.x); }
-__device__ __forceinline__ int gv_cta_of(const GvTable& p, int u) { return (int)(((long long)(u + 1) * gridDim.x - 1) / p.units); }
 
 // RT: accumulators (128 rows each) of a tile, which share the digits that a k-block loads
-template <int RT>
+// ROWS: 4 or 8, for up to so many rows of x; 0 for more, which have one unit for the whole of K and four digits
+template <int RT, int ROWS>
 __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid_constant__ GvTable p) {
     constexpr int EXP = (GV_TMEM - 64 * RT) / GV_ACOLS;        // expanded tiles in flight in tensor memory
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * EXP + 2 * RT];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag, last_ticket;
-    __shared__ int4 corr[16];              // of the matrix at hand: digit sums of every row of x, and its scale
-    __shared__ double xscale[16];
+    __shared__ long long x_sums[8 * 16];   // of the x at hand: of a slice, or of the whole of K
+    __shared__ double x_units[8 * 16];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = p.stages, Nq = p.Nq;
@@ -140,7 +201,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
             // ---- TMA producer: packed weights and the two digit tiles of a k-block.  The weights of the first slots do not
             // wait for the kernel before this one, which writes the digits ----
             bool waited = false;
-            int it = 0, m = 0;
+            int it = 0;
             int late[GV_MAX_STAGES], late_x[GV_MAX_STAGES];        // k-blocks whose digits are still to be asked for
             auto digits = [&](int s, int x, int kb) {
                 const uint32_t st = base + (uint32_t)s * stage_bytes + RT * GV_RAW;
@@ -152,11 +213,8 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 for (int i = 0; i < it && i < S; ++i) digits(i, late_x[i], late[i]);
                 waited = true;
             };
-            for (int u = u_begin; u < u_end && !abort_flag;) {
-                const GvPart t = gv_part(p, u, u_end, m);
-                m = t.m;
-                u += t.nkb;
-                const int x = p.m[m].x;
+            for (GvParts<false> t(p, u_begin, u_end); !abort_flag && t.next();) {
+                const int m = t.m, x = p.m[m].x;
                 for (int j = 0; j < t.nkb; ++j, ++it) {
                     const int s = it % S, kb = t.kb0 + j;
                     if (it == S) wait_before();
@@ -175,14 +233,12 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         const uint32_t idesc = idesc_i8(GV_ROWS, Nq);
         const uint64_t db0 = smem_desc_k_sw128(base + RT * GV_RAW);
         const uint32_t db_hi = (uint32_t)(db0 >> 32), db_lo = (uint32_t)db0, db_stage = stage_bytes >> 4, db_half = b_tile >> 4;
-        int it = 0, n_local = 0, m = 0, s = 0, e = 0;
+        int n_local = 0, s = 0, e = 0;
         uint32_t e_ph = 0;
         bool ok = true;
-        for (int u = u_begin; u < u_end && ok; ++n_local) {
-            const GvPart t = gv_part(p, u, u_end, m);
-            m = t.m;
-            u += t.nkb;
-            for (int j = 0; j < t.nkb && ok; ++j, ++it) {
+        if (ROWS) grid_wait();
+        for (GvParts<ROWS != 0> t(p, u_begin, u_end, ROWS ? gv_wide(p) : 0u); ok && t.next(); ++n_local) {
+            for (int j = 0; j < t.nkb && ok; ++j) {
 #pragma unroll
                 for (int h = 0; h < RT; ++h) {
                     if (j == 0 && !mbar_wait_all(acc_empty(h), (n_local & 1) ^ 1, &abort_flag)) { abort_flag = 1; if (lane == 0) atomicExch(p.err, 14); ok = false; break; }
@@ -246,44 +302,55 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         }
     } else {
         // ---- epilogue warps -------------------------------------------------------------------
-        grid_wait();       // digit sums, scales, cleared slots
-        const int q = warp & 3, M = p.M;
-        int n_local = 0, m = 0, x = 0;
-        bool ok = true;
-        for (int u = u_begin; u < u_end && ok; ++n_local) {
-            const GvPart t = gv_part(p, u, u_end, m);
-            m = t.m;
-            const GvMat& A = p.m[m];
-            u += t.nkb;
-            const bool whole = t.nkb == A.kblocks;
-            if (n_local == 0 || A.x != x) {
+        grid_wait();       // sums and units of the xs, cleared slots
+        const int q = warp & 3, lrow = q * 32 + lane, M = p.M, rows = gv_rows(M);
+        const uint32_t wide = ROWS ? gv_wide(p) : 0u, tmem = tmem_base + ((uint32_t)(q * 32) << 16);
+        const int chunks = ROWS ? ROWS / 4 : Nq / 16;        // of sixteen digit columns: four rows of x
+        const size_t pitch = RT * GV_ROWS;
+        auto slice_sums = [&](int cta, bool begun, int slice) { return p.part + (size_t)(((cta * 2 + begun) * 8 + slice) * rows) * pitch; };
+        auto number = [](int a, int b, int c, int d) { return ((long long)a * 256 + b) * 65536 + ((long long)c * 256 + d); };
+        // four rows of x, from row 4 c on, of an output row
+        auto write = [&](const GvMat& A, int row, int c, const double (&v)[4]) {
+            if (row >= A.O) return;
+            const double sc = (double)A.scale[row];
+            if (M == 1) {
+                A.y[row] = (float)(sc * (v[0] + v[1] * (1.0 / 1073741824.0)));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (4 * c + j < M) A.y[(size_t)(4 * c + j) * A.O + row] = (float)(sc * v[j]);
+            }
+        };
+        auto finish = [&](const GvMat& A, int row, int c, const uint32_t* v, const int* fifth) {
+            double n[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int r = 4 * c + j < rows ? 4 * c + j : 0;
+                n[j] = x_units[r] * (double)(number((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]) +
+                                             (ROWS ? (long long)fifth[j] * 4294967296ll : 0ll) - x_sums[r]);
+            }
+            write(A, row, c, n);
+        };
+        int n_local = 0, x = -1;
+        bool ok = true, begun = false;
+        for (GvParts<ROWS != 0> t(p, u_begin, u_end, wide); ok && t.next(); ++n_local) {
+            const GvMat& A = p.m[t.m];
+            const bool sliced = ROWS && (wide >> A.x & 1);
+            if (t.kb0 == 0 || n_local == 0) begun = t.kb0 == 0;
+            if (A.x != x) {
                 x = A.x;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 const int i = threadIdx.x - (64 + 128 * RT);
-                if (i < Nq / 4) corr[i] = reinterpret_cast<const int4*>(A.corr)[i];
-                else if (i >= 32 && i < 32 + M) xscale[i - 32] = (double)A.xscale[i - 32];
+                const bool in = (i & 15) < rows && i >> 4 < 1 << A.log_s;
+                long long sum = in ? A.sums[i] : 0ll;
+                if (in && !sliced && i < 16)
+                    for (int k = 1; k < 1 << A.log_s; ++k) sum += A.sums[16 * k + i];
+                x_sums[i] = sum;
+                x_units[i] = in ? A.units[i] : 0.0;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
-            // sixteen digit columns of a row: four rows of x
-            auto finish = [&](int row, int c16, const uint32_t* v, double sc) {
-                if (row >= A.O) return;
-                long long n[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int4 c = corr[c16 * 4 + j];
-                    n[j] = ((long long)((int)v[4 * j] - c.x) * 256 + ((int)v[4 * j + 1] - c.y)) * 65536 +
-                           ((long long)((int)v[4 * j + 2] - c.z) * 256 + ((int)v[4 * j + 3] - c.w));
-                }
-                if (M == 1) {
-                    A.y[row] = (float)(sc * (xscale[0] * ((double)n[0] + (double)n[1] * (1.0 / 1073741824.0))));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (c16 * 4 + j < M) A.y[(size_t)(c16 * 4 + j) * A.O + row] = (float)(sc * (xscale[c16 * 4 + j] * (double)n[j]));
-                }
-            };
-            const int tile_u = A.first + t.tile * A.kblocks;
-            const int from = whole ? 0 : gv_cta_of(p, tile_u);
+            const bool whole = begun && t.kb0 + t.nkb == t.kbs;          // with this part all of the tile has been here
+            const int tile_u = A.first + t.tile * t.kbs, from = whole ? blockIdx.x : gv_first_cta(p, blockIdx.x, tile_u);
             const int slot_i = p.tiles < (int)gridDim.x ? A.tile + t.tile : from;
             int* slot = p.acc + (size_t)slot_i * (RT * Nq * GV_ROWS);
 #pragma unroll 1
@@ -293,43 +360,89 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const int lrow = q * 32 + lane, row = (t.tile * RT + h) * GV_ROWS + lrow;
-                const double sc = whole && row < A.O ? (double)A.scale[row] : 0.0;
-#pragma unroll 1
-                for (int c = 0; c < Nq / 16; ++c) {
-                    uint32_t v[16];
-                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + 64 * h + 16 * c, v);
-                    tmem_ld_wait();
-                    if (whole) finish(row, c, v, sc);
-                    else if (row < A.O) {
+                const int row = (t.tile * RT + h) * GV_ROWS + lrow;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) atomicAdd(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow, (int)v[j]);
+                for (int c = 0; c < (ROWS ? ROWS / 4 : 4); ++c) {
+                    if (!ROWS && c == chunks) break;
+                    uint32_t v[16];
+                    int fifth[4] = {};
+                    if (ROWS && !sliced) {
+                        tmem_ld16(tmem + 64 * h + (p.extra & ~15), v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            fifth[j] = (int)((p.extra & 15) ? v[16 - ROWS + 4 * c + j] : v[4 * c + j]);
+                            if (!whole && row < A.O && 4 * c + j < rows) atomicAdd(slot + (h * Nq + p.extra + 4 * c + j) * GV_ROWS + lrow, fifth[j]);
+                        }
+                    }
+                    tmem_ld16(tmem + 64 * h + 16 * c, v);
+                    tmem_ld_wait();
+                    if (sliced) {
+                        const bool first = t.kb0 == gv_slice_at(t.slice, t.kbs, t.log_s);
+                        double* to = slice_sums(blockIdx.x, begun, t.slice) + h * GV_ROWS + lrow;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (4 * c + j < rows)
+                                to[(4 * c + j) * pitch] = (double)(number((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]) -
+                                                                   (first ? x_sums[16 * t.slice + 4 * c + j] : 0ll));
+                    } else if (whole) {
+                        finish(A, row, c, v, fifth);
+                    } else if (row < A.O) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (16 * c + j < 4 * rows) atomicAdd(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow, (int)v[j]);
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty(h));
             }
-            if (!ok || whole) continue;
-            // the last of the CTAs that share the tile finishes it
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (threadIdx.x == 64 + 128 * RT) last_ticket = atomicAdd(p.tickets + slot_i, 1) == gv_cta_of(p, tile_u + A.kblocks - 1) - from;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (last_ticket) {
+            if (!ok || (whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
+            if (!whole) {                 // the last of the CTAs that share the tile finishes it
                 __threadfence();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (threadIdx.x == 64 + 128 * RT) last_ticket = atomicAdd(p.tickets + slot_i, 1) == gv_last_cta(p, blockIdx.x, tile_u + t.kbs) - from;
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!last_ticket) continue;
+                __threadfence();
+            }
 #pragma unroll 1
-                for (int h = 0; h < RT; ++h) {
-                    const int lrow = q * 32 + lane, row = (t.tile * RT + h) * GV_ROWS + lrow;
-                    const double sc = row < A.O ? (double)A.scale[row] : 0.0;
-                    int v[32];                     // half of the widest list in flight at once
+            for (int h = 0; h < RT; ++h) {
+                const int row = (t.tile * RT + h) * GV_ROWS + lrow;
+                if (sliced) {
 #pragma unroll 1
-                    for (int c = 0; c < Nq / 16; c += 2) {
+                    for (int c = 0; c < chunks; ++c) {
+                        double total[4] = {};
+                        for (int slice = 0, cta = from; slice < 1 << t.log_s; ++slice) {
+                            const int k0 = gv_slice_at(slice, t.kbs, t.log_s), k1 = gv_slice_at(slice + 1, t.kbs, t.log_s);
+                            while (gv_cut(p, cta + 1) - tile_u <= k0) ++cta;
+                            double n[4] = {};
+                            for (int i = cta; ; ++i) {
+                                const double* src = slice_sums(i, i == from, slice) + h * GV_ROWS + lrow;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = c * 16 + j < Nq ? __ldcg(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow) : 0;
-                        finish(row, c, reinterpret_cast<const uint32_t*>(v), sc);
-                        if (c + 1 < Nq / 16) finish(row, c + 1, reinterpret_cast<const uint32_t*>(v) + 16, sc);
+                                for (int j = 0; j < 4; ++j)
+                                    if (4 * c + j < rows) n[j] += __ldcg(src + (4 * c + j) * pitch);
+                                if (gv_cut(p, i + 1) - tile_u >= k1) break;
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) total[j] += x_units[16 * slice + (4 * c + j < rows ? 4 * c + j : 0)] * n[j];
+                        }
+                        write(A, row, c, total);
                     }
+                    continue;
+                }
+                constexpr int AT_ONCE = ROWS ? 1 : 2;                   // of the widest list, half in flight
+#pragma unroll
+                for (int c = 0; c < (ROWS ? ROWS / 4 : 4); c += AT_ONCE) {
+                    if (!ROWS && c >= chunks) break;
+                    uint32_t v[16 * AT_ONCE];
+                    int fifth[4] = {};
+#pragma unroll
+                    for (int j = 0; j < 4 && ROWS; ++j) fifth[j] = 4 * c + j < rows ? __ldcg(slot + (h * Nq + p.extra + 4 * c + j) * GV_ROWS + lrow) : 0;
+#pragma unroll
+                    for (int j = 0; j < 16 * AT_ONCE; ++j) v[j] = 16 * c + j < 4 * rows ? (uint32_t)__ldcg(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow) : 0u;
+                    finish(A, row, c, v, fifth);
+                    if (AT_ONCE == 2 && c + 1 < chunks) finish(A, row, c + 1, v + 16 * (AT_ONCE - 1), fifth);
                 }
             }
         }
@@ -352,38 +465,136 @@ __device__ __forceinline__ float4 gv_load_x(const float4* p) {       // never be
     return v;
 }
 
-// ---- activation rows -> four int8 digit rows each, digit sums, power-of-two scale; slots and tickets of the contraction cleared ----
-// blocks: Nq / 4 per x (one per group of four digit rows; those without an activation row are written as zeros), then those that clear
+// ---- activation rows -> int8 digit rows, their sums, power-of-two units; slots and tickets of the contraction cleared ----
+// blocks: one per row of an x (up to 8 rows: per slice and row), then those that clear
 constexpr int GQ_THREADS = 512;
 struct GqTable {
-    int n, M, groups, I[kGemvXCap];
+    int n, M, rows, extra;
+    int I[kGemvXCap], log_s[kGemvXCap], spread[kGemvXCap];      // spread: how far apart the units of slices may be for one of all
+    int first[kGemvXCap + 1];              // number of an x's first block
     const float* x[kGemvXCap];
     signed char* xq[kGemvXCap];
-    int* corr[kGemvXCap];
-    float* xscale[kGemvXCap];
+    long long* sums[kGemvXCap];            // [slice][16]
+    double* units[kGemvXCap];
+    int* wide;                             // [x][8]
     int4* clear;
     size_t clear_n;
 };
+__device__ __forceinline__ bool gq_clear(const GqTable& p) {
+    if (blockIdx.x < p.first[p.n]) return false;
+    const size_t nthr = (size_t)(gridDim.x - p.first[p.n]) * GQ_THREADS;
+    for (size_t i = (size_t)(blockIdx.x - p.first[p.n]) * GQ_THREADS + threadIdx.x; i < p.clear_n; i += nthr) p.clear[i] = make_int4(0, 0, 0, 0);
+    return true;
+}
+// up to 8 rows
+__global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_slices_kernel(const __grid_constant__ GqTable p) {
+    __shared__ unsigned int top[8];
+    __shared__ unsigned long long total;
+    const int tid = threadIdx.x;
+    grid_release();
+    grid_wait();
+    if (gq_clear(p)) return;
+    int xi = 0;
+    while (blockIdx.x >= p.first[xi + 1]) ++xi;
+    const int at = blockIdx.x - p.first[xi], slice = at / p.rows, slot = at - slice * p.rows;
+    const int M = p.M, I = p.I[xi], lg = p.log_s[xi], chunks = (I + GV_KB - 1) / GV_KB;
+    const int k0 = (int)(((long long)slice * chunks) >> lg) * GV_KB, k1 = min((int)(((long long)(slice + 1) * chunks) >> lg) * GV_KB, I);
+    const float* x = p.x[xi] + (size_t)(M == 1 ? 0 : slot) * I;
+    const int warp = tid >> 5, lane = tid & 31;
+    auto quad = [&](int k) { return k < k1 ? gv_load_x(reinterpret_cast<const float4*>(x + k)) : make_float4(0.f, 0.f, 0.f, 0.f); };
+    float4 v = quad(k0 + 4 * tid);            // the slice's own, under the search for the largest magnitudes
+    if (tid < 8) top[tid] = 0u;
+    if (tid == 0) total = 0ull;
+    __syncthreads();
+    // the largest magnitude of every slice, half a chunk of K per warp; eight loads in flight
+    constexpr int WARPS = GQ_THREADS / 32, FLIGHT = 8;
+    for (int u0 = warp; u0 * 128 < I; u0 += FLIGHT * WARPS) {
+        unsigned int t[FLIGHT];
+#pragma unroll
+        for (int i = 0; i < FLIGHT; ++i) {
+            const int k = (u0 + i * WARPS) * 128 + lane * 4;
+            const float4 f = k < I ? gv_load_x(reinterpret_cast<const float4*>(x + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            t[i] = max(max(__float_as_uint(f.x) & 0x7FFFFFFFu, __float_as_uint(f.y) & 0x7FFFFFFFu), max(__float_as_uint(f.z) & 0x7FFFFFFFu, __float_as_uint(f.w) & 0x7FFFFFFFu));
+        }
+#pragma unroll
+        for (int i = 0; i < FLIGHT; ++i) {
+            const int u = u0 + i * WARPS;
+            if (u * 128 >= I) break;
+            t[i] = __reduce_max_sync(0xffffffffu, t[i]);
+            if (lane == 0) atomicMax(&top[((((u >> 1) + 1) << lg) - 1) / chunks], t[i]);
+        }
+    }
+    __syncthreads();
+    auto exponent = [](unsigned int t) { return max((int)(t >> 23) - 126, -90); };       // 2^e above every magnitude (of the smallest ones: 2^-90)
+    int low = 1 << 20, high = -(1 << 20);
+    bool finite = true;
+    for (int k = 0; k < 1 << lg; ++k) {
+        const unsigned int t = top[k];
+        finite = finite && t < 0x7F800000u;
+        if (t == 0u || t >= 0x7F800000u) continue;
+        low = min(low, exponent(t));
+        high = max(high, exponent(t));
+    }
+    const unsigned int mine = top[slice];
+    const int e = mine >= 0x7F800000u || low > high ? 0 : exponent(mine);
+    const bool wide = high - low > p.spread[xi];
+    const int shift = wide || mine == 0u || mine >= 0x7F800000u ? 0 : e - low;
+    const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
+    signed char* const q = p.xq[xi] + (size_t)(4 * slot) * I + k0;
+    signed char* const q5 = p.xq[xi] + (size_t)(p.extra + slot) * I + k0;
+    // Four lanes hold a group of 16 activations, element 4 j + a in register a of lane j; word i of a digit row takes the elements i, 4 + i,
+    // 8 + i, 12 + i.  Two exchanges of bytes leave lane j with byte j of the four.
+    auto turn = [&](uint32_t w) {
+        const uint32_t o1 = __shfl_xor_sync(0xffffffffu, w, 1);
+        const uint32_t h = (lane & 1) ? __byte_perm(w, o1, 0x3715) : __byte_perm(w, o1, 0x6240);
+        const uint32_t o2 = __shfl_xor_sync(0xffffffffu, h, 2);
+        return (lane & 2) ? __byte_perm(o2, h, 0x7632) : __byte_perm(h, o2, 0x5410);
+    };
+    long long sum = 0;
+    for (int g0 = 32 * warp; k0 + 4 * g0 < k1; g0 += GQ_THREADS) {
+        const int g = g0 + lane;
+        if (g0 >= GQ_THREADS) v = quad(k0 + 4 * g);
+        const float f[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+        uint32_t r[4], r5 = 0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            int n = __float2int_rn(f[a]);
+            // what the 30 bits leave over: nothing from 2^23 on, where f is a whole number itself
+            if (M == 1 && slot == 1) n = __float2int_rn((f[a] - (float)n) * 1073741824.0f);
+            sum += n;
+            const long long b = ((long long)n << shift) + 0x80808080ll;          // signed bytes, base 256
+            r[a] = turn((uint32_t)b ^ 0x80808080u);
+            r5 |= ((uint32_t)(b >> 32) & 255u) << (8 * a);
+        }
+        r5 = turn(r5);
+        if (k0 + 4 * g < k1) {
+            const size_t to = (size_t)(g >> 2) * 16;
+            *reinterpret_cast<uint4*>(q + (size_t)(3 - (lane & 3)) * I + to) = make_uint4(r[0], r[1], r[2], r[3]);        // byte 3 is the leading one of four
+            *reinterpret_cast<uint32_t*>(q5 + to + 4 * (lane & 3)) = r5;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) atomicAdd(&total, (unsigned long long)sum);
+    __syncthreads();
+    if (tid == 0) {
+        const int unit = (wide || low > high ? e : low) - 30;
+        p.sums[xi][16 * slice + slot] = (long long)total << shift;
+        p.units[xi][16 * slice + slot] = __longlong_as_double(finite ? (long long)(1023 + unit) << 52 : 0x7FF8000000000000ll);       // an infinity or NaN: so is the row
+        if (slice == 0 && slot < M) p.wide[8 * xi + slot] = wide;
+    }
+}
+
+// more than 8 rows: one unit for the whole of K
 __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_constant__ GqTable p) {
     __shared__ unsigned int top_s;
     __shared__ int isum[4];
     const int tid = threadIdx.x;
     grid_release();
     grid_wait();
-    const int xi = blockIdx.x / p.groups;
-    if (xi >= p.n) {
-        const size_t nthr = (size_t)(gridDim.x - p.n * p.groups) * GQ_THREADS;
-        for (size_t i = (size_t)(blockIdx.x - p.n * p.groups) * GQ_THREADS + tid; i < p.clear_n; i += nthr) p.clear[i] = make_int4(0, 0, 0, 0);
-        return;
-    }
-    const int slot = blockIdx.x - xi * p.groups, M = p.M, I = p.I[xi], row = M == 1 ? 0 : slot;
-    uint4* q = reinterpret_cast<uint4*>(p.xq[xi] + (size_t)(4 * slot) * I);
-    const int pitch = I >> 4;
-    if (slot >= (M == 1 ? 2 : M)) {
-        for (int i = tid; i < 4 * pitch; i += GQ_THREADS) q[i] = make_uint4(0, 0, 0, 0);
-        if (tid < 4) p.corr[xi][4 * slot + tid] = 0;
-        return;
-    }
+    if (gq_clear(p)) return;
+    const int xi = blockIdx.x / p.rows, row = blockIdx.x - xi * p.rows, I = p.I[xi], pitch = I >> 4;
+    uint4* q = reinterpret_cast<uint4*>(p.xq[xi] + (size_t)(4 * row) * I);
     const float4* x = reinterpret_cast<const float4*>(p.x[xi] + (size_t)row * I);
     if (tid == 0) top_s = 0u;
     if (tid < 4) isum[tid] = 0;
@@ -410,10 +621,7 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
             const float f[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                int n = __float2int_rn(f[a]);
-                // what the 30 bits leave over: nothing from 2^23 on, where f is a whole number itself
-                if (M == 1 && slot == 1) n = __float2int_rn((f[a] - (float)n) * 1073741824.0f);
-                r[4 * j + a] = ((uint32_t)n + 0x80808080u) ^ 0x80808080u;        // four signed bytes, base 256
+                r[4 * j + a] = ((uint32_t)__float2int_rn(f[a]) + 0x80808080u) ^ 0x80808080u;        // four signed bytes, base 256
             }
         }
 #pragma unroll
@@ -434,9 +642,10 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
         if ((tid & 31) == 0) atomicAdd(&isum[d], sum[d]);
     }
     __syncthreads();
-    if (tid < 4) p.corr[xi][4 * slot + tid] = isum[tid];
-    if (tid == 0 && slot < M)       // an infinity or NaN: so is the row
-        p.xscale[xi][slot] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : __uint_as_float((uint32_t)(127 + e - 30) << 23);
+    if (tid == 0) {       // an infinity or NaN: so is the row
+        p.sums[xi][row] = ((long long)isum[0] * 256 + isum[1]) * 65536 + ((long long)isum[2] * 256 + isum[3]);
+        p.units[xi][row] = __longlong_as_double(top >= 0x7F800000u ? 0x7FF8000000000000ll : (long long)(1023 + e - 30) << 52);
+    }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -468,9 +677,11 @@ bool gv_map_2d(CUtensorMap* map, const void* basep, size_t inner_bytes, size_t r
 }
 
 
-int gv_nq(int M) { return (4 * (M == 1 ? 2 : M) + 15) / 16 * 16; }
+// digit rows of a launch, and where the fifth digits begin: each of up to 8 rows' stand in sixteen columns of their own or the last of a group's
+int gv_extra(int M) { return M <= 3 ? 12 : M == 4 ? 16 : M <= 6 ? 24 : M <= 8 ? 32 : 0; }
+int gv_nq(int M) { return M <= 3 ? 16 : M <= 6 ? 32 : M <= 8 ? 48 : (4 * M + 15) / 16 * 16; }
 size_t round_up(size_t n) { return (n + 1023) & ~size_t(1023); }
-constexpr size_t kGvCorr = 64 * sizeof(int);      // then up to 16 scales
+constexpr size_t kGvUnits = 1024, kGvXBytes = 2048;      // of an x: 128 sums, 128 units
 long long gv_blocks(const GemvItem* items, int n) {        // k-blocks of 128 rows
     long long u = 0;
     for (int i = 0; i < n; ++i) u += (items[i].out_features + (long long)GV_ROWS - 1) / GV_ROWS * ((items[i].in_features + GV_KB - 1) / GV_KB);
@@ -483,15 +694,46 @@ bool gemv_tc_supported(int M, int in_features, const void* packed2) {
     return M >= 1 && M <= 16 && in_features % 64 == 0 && in_features >= 256 && in_features <= (1 << 22) && reinterpret_cast<uintptr_t>(packed2) % 16 == 0;      // 32-bit sums of digits times fields
 }
 
-// tickets | a slot per CTA (two CTAs on every SM) | per x: Xq [Nq][in] int8, digit sums, scales
+namespace {
+struct GvPlan { int RT, ctas; long long units, tiles; size_t slots, slices; };      // bytes for tiles that a cut runs through
+GvPlan gv_plan(const GemvItem* items, int n, int M, int sm_count) {
+    GvPlan g;
+    // Two CTAs on every SM and tiles of 256 rows, or one and 128.  One row: 2100 k-blocks 22.6 and 20.8 us, 5760 26.8 and 35.0, 25600 60 and 118; 16
+    // rows, alone and with other work beside them: 5760 35 / 26.8 and 43 / 19.7, 25600 80 / 68 and 141 / 66.
+    const bool large = gv_blocks(items, n) >= (long long)sm_count * (M <= 8 ? 24 : 64);
+    g.RT = large ? 2 : 1;
+    g.units = g.tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        const long long of = (items[i].out_features + (long long)g.RT * GV_ROWS - 1) / (g.RT * GV_ROWS);
+        g.tiles += of;
+        g.units += of * ((items[i].in_features + GV_KB - 1) / GV_KB);
+    }
+    // One matrix of few tiles: no CTA has parts of two (4096 x 4096, 16 rows: 16.2 -> 13.1 us), and a tile is cut only where that saves more
+    // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).
+    int per = g.RT * sm_count;
+    if (n == 1 && g.tiles <= sm_count) {
+        const int kbs = (items[0].in_features + GV_KB - 1) / GV_KB, cut = std::max(1, std::min(kbs / 2, (int)(sm_count / g.tiles)));
+        per = (int)g.tiles * (kbs - kbs / cut > 6 ? cut : 1);
+    }
+    g.ctas = (int)std::min<long long>(per, g.units);
+    g.slots = (size_t)std::min<long long>(g.ctas, g.tiles) * g.RT * gv_nq(M) * GV_ROWS * sizeof(int);
+    g.slices = M <= 8 ? (size_t)g.ctas * 16 * gv_rows(M) * g.RT * GV_ROWS * sizeof(double) : 0;
+    return g;
+}
+// more than 8 rows: room for the longest list, which a single matrix may become the first of
+size_t gv_slot_room(const GvPlan& g, int M, int sm_count) { return round_up(M <= 8 ? g.slots : (size_t)2 * sm_count * 2 * gv_nq(M) * GV_ROWS * sizeof(int)); }
+}  // namespace
+
+// tickets | flags of the xs | slots | sums of slices | per x: Xq [Nq][in] int8, sums, units
 size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count) {
-    size_t bytes = round_up(2 * sm_count * sizeof(int)) + (size_t)2 * sm_count * 2 * gv_nq(M) * GV_ROWS * sizeof(int);
+    const GvPlan g = gv_plan(items, n, M, sm_count);
+    size_t bytes = round_up(2 * sm_count * sizeof(int)) + 1024 + gv_slot_room(g, M, sm_count) + round_up(g.slices);
     int xs = 0;
     for (int i = 0; i < n; ++i) {
         bool known = false;
         for (int j = 0; j < i; ++j) known = known || (items[j].x == items[i].x && items[j].in_features == items[i].in_features);
         if (known) continue;
-        bytes += round_up((size_t)gv_nq(M) * items[i].in_features) + 1024;
+        bytes += round_up((size_t)gv_nq(M) * items[i].in_features) + kGvXBytes;
         ++xs;
     }
     return xs <= kGemvXCap && gv_blocks(items, n) <= 0x3fffffff ? bytes : ~size_t(0);
@@ -542,19 +784,25 @@ cudaError_t put_before(cudaGraph_t graph, cudaGraphNode_t node, const cudaKernel
 cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* workspace, int parts, bool follows, const cudaGraphNode_t* nodes,
                                    cudaGraph_t graph, int* err_word, int sm_count, size_t max_smem, cudaStream_t stream) {
     const int Nq = gv_nq(M);
-    // Two CTAs on every SM and tiles of 256 rows, or one and 128.  One row: 2100 k-blocks 22.6 and 20.8 us, 5760 26.8 and 35.0, 25600 60 and 118; 16
-    // rows, alone and with other work beside them: 5760 35 / 26.8 and 43 / 19.7, 25600 80 / 68 and 141 / 66.
-    const bool large = gv_blocks(items, n) >= (long long)sm_count * (M <= 8 ? 24 : 64);
-    const int RT = large ? 2 : 1;
+    const GvPlan plan = gv_plan(items, n, M, sm_count);
+    const int RT = plan.RT, ctas = plan.ctas;
+    if (plan.units > 0x3fffffff) return cudaErrorInvalidValue;
     char* w = static_cast<char*>(workspace);
     GvTable p;
     GqTable g;
-    p.n = n; p.M = M; p.Nq = Nq; p.err = err_word;
+    p.n = n; p.M = M; p.Nq = Nq; p.err = err_word; p.extra = gv_extra(M);
+    p.cut_q = (int)(plan.units / ctas); p.cut_r = (int)(plan.units % ctas);
+    p.tiles = (int)plan.tiles;
+    g.wide = reinterpret_cast<int*>(w);
+    p.wide = g.wide;
+    w += 1024;
     p.tickets = reinterpret_cast<int*>(w);
     w += round_up(2 * sm_count * sizeof(int));
     p.acc = reinterpret_cast<int*>(w);
-    w += (size_t)2 * sm_count * 2 * Nq * GV_ROWS * sizeof(int);
-    g.n = 0; g.M = M; g.groups = Nq / 4;
+    w += gv_slot_room(plan, M, sm_count);
+    p.part = reinterpret_cast<double*>(w);
+    w += round_up(plan.slices);
+    g.n = 0; g.M = M; g.rows = gv_rows(M); g.extra = p.extra; g.first[0] = 0;
     long long units = 0, tiles = 0;
     for (int i = 0; i < n; ++i) {
         const GemvItem& it = items[i];
@@ -566,44 +814,45 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
             g.x[x] = it.x; g.I[x] = it.in_features;
             g.xq[x] = reinterpret_cast<signed char*>(w);
             w += round_up((size_t)Nq * it.in_features);
-            g.corr[x] = reinterpret_cast<int*>(w);
-            g.xscale[x] = reinterpret_cast<float*>(w + kGvCorr);
-            w += 1024;
+            g.sums[x] = reinterpret_cast<long long*>(w);
+            g.units[x] = reinterpret_cast<double*>(w + kGvUnits);
+            w += kGvXBytes;
+            g.log_s[x] = M <= 8 ? gemv_log_slices(it.in_features) : 0;
+            // 30 bits, the spread and the carry of a sum of in_features fit the 53 bits of a double
+            g.spread[x] = 8;
+            while (g.spread[x] > 0 && (1ll << (23 - g.spread[x])) < it.in_features) --g.spread[x];
+            g.first[g.n] = g.first[x] + (g.rows << g.log_s[x]);
             if (!gv_map_2d(&p.xmaps[x], g.xq[x], it.in_features, Nq, it.in_features, 128, Nq, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
         }
         GvMat& m = p.m[i];
-        m.scale = it.scale; m.y = it.y; m.corr = g.corr[x]; m.xscale = g.xscale[x];
-        m.O = it.out_features; m.x = x;
+        m.scale = it.scale; m.y = it.y; m.sums = g.sums[x]; m.units = g.units[x];
+        m.O = it.out_features; m.x = x; m.log_s = g.log_s[x];
         m.kblocks = (it.in_features + GV_KB - 1) / GV_KB;
         m.first = (int)units;
         m.tile = (int)tiles;
         const long long of = (it.out_features + (long long)RT * GV_ROWS - 1) / (RT * GV_ROWS);
         tiles += of;
         units += of * m.kblocks;
-        if (units > 0x3fffffff) return cudaErrorInvalidValue;
         if (!gv_map_2d(&p.maps[i], it.packed2, (size_t)it.in_features / 4, it.out_features, (size_t)it.in_features / 4, GV_KB / 4, RT * GV_ROWS,
                        CU_TENSOR_MAP_SWIZZLE_64B)) return cudaErrorInvalidValue;
     }
-    p.units = (int)units; p.tiles = (int)tiles;
+    p.xs = g.n;
     const size_t stage_bytes = (size_t)RT * GV_RAW + 2 * (size_t)Nq * 128;
-    p.stages = std::min(GV_MAX_STAGES, (int)((max_smem / 2 - 3072) / stage_bytes));
+    p.stages = std::min(GV_MAX_STAGES, (int)((max_smem / 2 - 4608) / stage_bytes));
     if (p.stages < 2) return cudaErrorInvalidConfiguration;
     const size_t smem = p.stages * stage_bytes + 1024;
-    // One matrix of few tiles: no CTA has parts of two (4096 x 4096, 16 rows: 16.2 -> 13.1 us), and a tile is cut only where that saves more
-    // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).
-    int per = (large ? 2 : 1) * sm_count;
-    if (n == 1 && tiles <= sm_count) {
-        const int kbs = p.m[0].kblocks, cut = std::max(1, std::min(kbs / 2, (int)(sm_count / tiles)));
-        per = (int)tiles * (kbs - kbs / cut > 6 ? cut : 1);
-    }
-    const int ctas = (int)std::min<long long>(per, units);
     // the tickets stand before the slots: one range
     g.clear = reinterpret_cast<int4*>(p.tickets);
-    g.clear_n = (round_up(2 * sm_count * sizeof(int)) + (size_t)std::min<long long>(ctas, tiles) * RT * Nq * GV_ROWS * sizeof(int)) / 16;
-    const int q_blocks = g.n * g.groups + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS));
+    g.clear_n = (round_up(2 * sm_count * sizeof(int)) + plan.slots) / 16;
+    const int q_blocks = g.first[g.n] + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS));
 
-    const void* kern = RT == 2 ? reinterpret_cast<const void*>(gemv_tc_kernel<2>) : reinterpret_cast<const void*>(gemv_tc_kernel<1>);
-    cudaError_t e = ensure_dynamic_smem(kern, RT == 2 ? 5 : 40, max_smem);
+    // by rows (up to 4, up to 8, more) and RT
+    static void (*const kernels[3][2])(GvTable) = {{gemv_tc_kernel<1, 4>, gemv_tc_kernel<2, 4>}, {gemv_tc_kernel<1, 8>, gemv_tc_kernel<2, 8>},
+                                                   {gemv_tc_kernel<1, 0>, gemv_tc_kernel<2, 0>}};
+    const int rows = M <= 4 ? 0 : M <= 8 ? 1 : 2;
+    void (*const kernel)(GvTable) = kernels[rows][RT - 1];
+    const void* kern = reinterpret_cast<const void*>(kernel);
+    cudaError_t e = ensure_dynamic_smem(kern, 52 + 2 * rows + RT - 1, max_smem);
     if (e != cudaSuccess) return e;
     cudaKernelNodeParams kp = {};
     cudaLaunchConfig_t cfg = {};
@@ -613,11 +862,12 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     cfg.attrs = &at;
     if (parts & 1) {
         void* args[] = {&g};
-        kp.func = reinterpret_cast<void*>(gemv_quantize_kernel);
+        void (*const digits)(GqTable) = M <= 8 ? gemv_quantize_slices_kernel : gemv_quantize_kernel;
+        kp.func = reinterpret_cast<void*>(digits);
         kp.gridDim = cfg.gridDim = dim3(q_blocks); kp.blockDim = cfg.blockDim = dim3(GQ_THREADS);
         kp.kernelParams = args;
         cfg.numAttrs = follows ? 1 : 0;
-        e = !nodes ? cudaLaunchKernelEx(&cfg, gemv_quantize_kernel, g) : nodes[0] ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : put_before(graph, nodes[1], kp);
+        e = !nodes ? cudaLaunchKernelEx(&cfg, digits, g) : nodes[0] ? cudaGraphKernelNodeSetParams(nodes[0], &kp) : put_before(graph, nodes[1], kp);
         if (e != cudaSuccess) return e;
     }
     if (parts & 2) {
@@ -628,7 +878,7 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
         kp.kernelParams = args;
         cfg.numAttrs = 1;
         e = nodes ? cudaGraphKernelNodeSetParams(nodes[1], &kp)
-                  : RT == 2 ? cudaLaunchKernelEx(&cfg, gemv_tc_kernel<2>, p) : cudaLaunchKernelEx(&cfg, gemv_tc_kernel<1>, p);
+                  : cudaLaunchKernelEx(&cfg, kernel, p);
     }
     return e;
 }

@@ -169,9 +169,12 @@ struct GemvItem {
     float* y;
     int in_features, out_features;
 };
-// gemv_mma.cu -- M <= 8, one launch (one node) of integer mma.sync; clusters sized for the first matrix of the list
+// Slices of K (2^n of them) that up to 8 rows of x have a unit of their own in.  They follow from the length alone, so that a result does
+// not depend on the launch that a matrix is part of, nor on the kernel.
+int gemv_log_slices(int in_features);
+// gemv_mma.cu -- M <= 8, one launch (one node) of integer mma.sync; clusters sized for the shortest rows of a list
 bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem);
-bool gemv_mma_joins(int first_in_features, int in_features);
+bool gemv_mma_joins(const GemvItem* items, int n, int in_features);       // a matrix, such a list
 cudaError_t launch_ternary_gemv_mma(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count,
                                     size_t max_smem, cudaStream_t stream);
 // gemv_tc.cu -- M <= 16, two launches (two nodes): digits, integer tcgen05.  parts: bit 0 the first launch, bit 1 the second; with `nodes`,

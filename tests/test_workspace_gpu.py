@@ -113,7 +113,7 @@ def test_decode_of_up_to_eight_rows_does_without(M):
             del graph
             ctx.ternary_gemv(x, w, scale, y, M, cols, rows)
             ctx.finish()
-            assert float((got.double() - y.double()).norm() / y.double().norm()) <= 2.0 ** -23
+            assert torch.equal(got, y)
             if eager:
                 assert ctx.workspace_bytes == 0
         ctx.close()
@@ -161,7 +161,7 @@ def test_lists_of_a_recording_get_workspace_beside_a_batch_that_holds_some(on):
         ctx.finish()
         assert torch.equal(f.y[:256], want)
         for a, b in zip(ys, single):
-            assert float((a.double() - b.double()).norm() / b.double().norm()) <= 2.0 ** -23
+            assert torch.equal(a, b)
         first.close()
         second.close()
         if who is not ctx:
