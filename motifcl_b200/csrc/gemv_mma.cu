@@ -213,11 +213,9 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
         const int m = M == 1 ? 0 : mp;
         const int sl = LIST && (unit - mp * per_row) >> 1 >= mid;
         const unsigned int top = amax[sl][m];
-        int e = max((int)(top >> 23) - 126, -90);   // 2^e above every magnitude (of the smallest ones: 2^-90)
-        if (top >= 0x7F800000u) e = 0;
-        const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
+        const GemvUnit inv = gemv_unit(top >= 0x7F800000u ? 0 : gemv_exponent(top));
         const float4 t = k < I ? mv_load_x(x + (size_t)m * I + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float f[4] = {t.x * inv, t.y * inv, t.z * inv, t.w * inv};
+        const float f[4] = {t.x * inv.a * inv.b, t.y * inv.a * inv.b, t.z * inv.a * inv.b, t.w * inv.a * inv.b};
         uint32_t r[4];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -251,7 +249,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
         const int m = threadIdx.x & 7;
         for (int sl = 0; sl < 1 << lg_k; ++sl) {
             const unsigned int top = amax[sl][m];
-            const int e = max((int)(top >> 23) - 126, -90);
+            const int e = gemv_exponent(top);
             const double v = top >= 0x7F800000u ? __longlong_as_double(0x7FF8000000000000ll)       // an infinity or NaN: so is the row
                                                 : __longlong_as_double((long long)(1023 + e - 30) << 52);
             uint32_t to;

@@ -525,21 +525,20 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_slices_kernel(const 
         }
     }
     __syncthreads();
-    auto exponent = [](unsigned int t) { return max((int)(t >> 23) - 126, -90); };       // 2^e above every magnitude (of the smallest ones: 2^-90)
     int low = 1 << 20, high = -(1 << 20);
     bool finite = true;
     for (int k = 0; k < 1 << lg; ++k) {
         const unsigned int t = top[k];
         finite = finite && t < 0x7F800000u;
         if (t == 0u || t >= 0x7F800000u) continue;
-        low = min(low, exponent(t));
-        high = max(high, exponent(t));
+        low = min(low, gemv_exponent(t));
+        high = max(high, gemv_exponent(t));
     }
     const unsigned int mine = top[slice];
-    const int e = mine >= 0x7F800000u || low > high ? 0 : exponent(mine);
+    const int e = mine >= 0x7F800000u || low > high ? 0 : gemv_exponent(mine);
     const bool wide = high - low > p.spread[xi];
     const int shift = wide || mine == 0u || mine >= 0x7F800000u ? 0 : e - low;
-    const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
+    const GemvUnit inv = gemv_unit(e);
     signed char* const q = p.xq[xi] + (size_t)(4 * slot) * I + k0;
     signed char* const q5 = p.xq[xi] + (size_t)(p.extra + slot) * I + k0;
     // Four lanes hold a group of 16 activations, element 4 j + a in register a of lane j; word i of a digit row takes the elements i, 4 + i,
@@ -554,7 +553,7 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_slices_kernel(const 
     for (int g0 = 32 * warp; k0 + 4 * g0 < k1; g0 += GQ_THREADS) {
         const int g = g0 + lane;
         if (g0 >= GQ_THREADS) v = quad(k0 + 4 * g);
-        const float f[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+        const float f[4] = {v.x * inv.a * inv.b, v.y * inv.a * inv.b, v.z * inv.a * inv.b, v.w * inv.a * inv.b};
         uint32_t r[4], r5 = 0;
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -609,16 +608,15 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
     if ((tid & 31) == 0) atomicMax(&top_s, top);
     __syncthreads();
     top = top_s;
-    int e = max((int)(top >> 23) - 126, -90);       // 2^e above every magnitude (of the smallest ones: 2^-90)
-    if (top >= 0x7F800000u) e = 0;
-    const float inv = __uint_as_float((uint32_t)(127 + 30 - e) << 23);
+    const int e = top >= 0x7F800000u ? 0 : gemv_exponent(top);
+    const GemvUnit inv = gemv_unit(e);
     int sum[4] = {0, 0, 0, 0};
     for (int g = tid; g < pitch; g += GQ_THREADS) {
         uint32_t r[16];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float4 v = gv_load_x(x + 4 * g + j);
-            const float f[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+            const float f[4] = {v.x * inv.a * inv.b, v.y * inv.a * inv.b, v.z * inv.a * inv.b, v.w * inv.a * inv.b};
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 r[4 * j + a] = ((uint32_t)__float2int_rn(f[a]) + 0x80808080u) ^ 0x80808080u;        // four signed bytes, base 256

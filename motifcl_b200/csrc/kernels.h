@@ -172,6 +172,16 @@ struct GemvItem {
 // Slices of K (2^n of them) that up to 8 rows of x have a unit of their own in.  They follow from the length alone, so that a result does
 // not depend on the launch that a matrix is part of, nor on the kernel.
 int gemv_log_slices(int in_features);
+#ifdef __CUDACC__
+// Whole numbers of 30 bits and sign below a largest magnitude (given as bits of a float without sign): 2^e above it, and the factor
+// 2^(30 - e) in two steps, since it leaves fp32 for magnitudes below 2^-97.
+__device__ __forceinline__ int gemv_exponent(unsigned int top) { return (int)(top >> 23) - 126; }
+struct GemvUnit { float a, b; };
+__device__ __forceinline__ GemvUnit gemv_unit(int e) {
+    const int a = min(30 - e, 127);
+    return {__uint_as_float((uint32_t)(127 + a) << 23), __uint_as_float((uint32_t)(127 + 30 - e - a) << 23)};
+}
+#endif
 // gemv_mma.cu -- M <= 8, one launch (one node) of integer mma.sync; clusters sized for the shortest rows of a list
 bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem);
 bool gemv_mma_joins(const GemvItem* items, int n, int in_features);       // a matrix, such a list

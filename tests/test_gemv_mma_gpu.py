@@ -39,6 +39,33 @@ def test_edges_of_chunks_units_and_clusters(M, O, I):
         assert np.linalg.norm(got[m] - want[m]) <= 1e-6 * np.linalg.norm(size[m])
 
 
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("O,I,n", [(300, 1088, 1), (4096, 4096, 8)])
+def test_the_smallest_magnitudes_have_their_bits(M, O, I, n):
+    """Rows of 2^-90 down to 2^-125 and, beside them, subnormal activations; scales that bring the results back."""
+    rng = np.random.default_rng(M)
+    w, digits, scale = _matrix(rng, O, I)
+    x = (rng.uniform(-1, 1, (M, I)) * 2.0 ** np.linspace(-90, -125, M)[:, None]).astype(np.float32)
+    x[:, ::7] *= np.float32(2.0 ** -6)
+    scale *= np.float32(2.0 ** 100)
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        dx, s = torch.from_numpy(x).to(DEV), torch.from_numpy(scale).to(DEV)
+        ys = [torch.full((M, O), 5.0, device=DEV) for _ in range(n)]
+        ctx.ternary_gemv(dx, w, s, ys[0], M, I, O)
+        ctx.finish()
+        ctx.batch_begin()
+        for y in ys:
+            ctx.ternary_gemv(dx, w, s, y, M, I, O)
+        batch = ctx.batch_end()
+        batch.launch()
+        ctx.finish()
+        batch.close()
+        want = x.astype(np.float64) @ digits.T * scale.astype(np.float64)
+        for m in range(M):
+            assert np.linalg.norm(ys[-1].cpu().numpy()[m] - want[m]) <= 1e-6 * np.linalg.norm(want[m])
+
+
 @pytest.mark.parametrize("M", [1, 4, 8])
 def test_recorded_chain_reads_the_result_before_it(M):
     """Recorded launches overlap: x of every second matrix is the result of the first, whose buffers the next pair takes again."""
