@@ -187,7 +187,6 @@ template <int BQ, int NC>
 __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                          const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr int HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
@@ -307,7 +306,6 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_bwd_q_kernel(const float
                                                            const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
                                                            float* __restrict__ dq, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr int HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
@@ -486,7 +484,6 @@ template <int NC>
 __global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
                                                         const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) float sm[];
     constexpr int HDP = 16 * NC, HS = HDP + 4, KS = kKT + 4;
     const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;

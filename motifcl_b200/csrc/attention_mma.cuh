@@ -149,7 +149,6 @@ template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                                        const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
     constexpr int NT = 128, BQ = 64;
@@ -249,7 +248,6 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
                                                            const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
                                                            float* __restrict__ dq, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
     constexpr int NT = 128, BQ = 64;
@@ -413,7 +411,6 @@ template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_bwd_k_mma_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
                                                         const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
     grid_release();
-    grid_wait();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;

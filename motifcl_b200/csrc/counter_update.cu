@@ -79,7 +79,7 @@ counter_update_dense_kernel(const UpdParams p) {
     const float Cf = (float)p.C;
     const float neg_lr = -p.lr;
     const bool check_t = 4 * lv < 64;      // some code values decode to a ternary digit the tail table lacks
-    const uint32_t seed = p.seed + (p.seed_offset ? __ldg(p.seed_offset) : 0u);
+    const uint32_t seed = p.seed + (p.seed_offset ? load_behind(p.seed_offset) : 0u);
     const bool aligned16 = p.state_align >= 16;   // state rows start and end on 16-byte boundaries
     const bool aligned4 = p.state_align >= 4;     // ... on 4-byte boundaries
 
@@ -112,13 +112,13 @@ counter_update_dense_kernel(const UpdParams p) {
             if (aligned16) {
                 const uint4* s4 = reinterpret_cast<const uint4*>(src);
                 uint4* d4 = reinterpret_cast<uint4*>(dst);
-                for (int i = tid; i < row_bytes / 16; i += kUpdThreads) d4[i] = __ldg(s4 + i);
+                for (int i = tid; i < row_bytes / 16; i += kUpdThreads) d4[i] = load_behind(s4 + i);
             } else if (aligned4) {
                 const uint32_t* s1 = reinterpret_cast<const uint32_t*>(src);
                 uint32_t* d1 = reinterpret_cast<uint32_t*>(dst);
-                for (int i = tid; i < row_bytes / 4; i += kUpdThreads) d1[i] = __ldg(s1 + i);
+                for (int i = tid; i < row_bytes / 4; i += kUpdThreads) d1[i] = load_behind(s1 + i);
             } else {
-                for (int i = tid; i < row_bytes; i += kUpdThreads) dst[i] = __ldg(src + i);
+                for (int i = tid; i < row_bytes; i += kUpdThreads) dst[i] = load_behind(src + i);
             }
         }
         if (WITH_Q) __syncthreads();
@@ -127,7 +127,7 @@ counter_update_dense_kernel(const UpdParams p) {
             float4* dst = reinterpret_cast<float4*>(gw_s + (size_t)r * I);
             const uint32_t* raw = reinterpret_cast<const uint32_t*>(st_s + (size_t)r * sb);
             for (int g = tid; g < gpr; g += kUpdThreads) {
-                const float4 gw = __ldg(src + g);
+                const float4 gw = load_behind(src + g);
                 dst[g] = gw;
                 if (WITH_Q) {
                     const uint32_t w = load_group24(raw, (uint32_t)g * 3u);
@@ -396,7 +396,7 @@ counter_update_ws_kernel(const UpdParams p, const uint32_t pow16, const uint32_t
     const int lv = 2 * p.C - 1;
     const float Cf = (float)p.C;
     const float neg_lr = -p.lr;
-    const uint32_t seed = p.seed + (p.seed_offset ? __ldg(p.seed_offset) : 0u);
+    const uint32_t seed = p.seed + (p.seed_offset ? load_behind(p.seed_offset) : 0u);
     const int D = nslots;
 
     // this CTA's rows: a contiguous block

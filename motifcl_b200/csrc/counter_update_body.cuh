@@ -276,13 +276,13 @@ __device__ __forceinline__ void u16_load_state(const UpdParams& p, const U16Layo
     if (p.state_align >= 16) {        // row_bytes % 16 == 0: one flat copy, smem row stride == row_bytes
         const uint4* s4 = reinterpret_cast<const uint4*>(src);
         uint4* d4 = reinterpret_cast<uint4*>(st_s);
-        for (int i = tid; i < nrows * (row_bytes >> 4); i += NT) d4[i] = __ldg(s4 + i);
+        for (int i = tid; i < nrows * (row_bytes >> 4); i += NT) d4[i] = load_behind(s4 + i);
     } else {                          // rows are 4-byte aligned; smem rows padded to L.sb
         const uint32_t* s1 = reinterpret_cast<const uint32_t*>(src);
         const int wpr = row_bytes >> 2;
         for (int i = tid; i < nrows * wpr; i += NT) {
             const int r = i / wpr, w = i - r * wpr;
-            reinterpret_cast<uint32_t*>(st_s + (size_t)r * L.sb)[w] = __ldg(s1 + i);
+            reinterpret_cast<uint32_t*>(st_s + (size_t)r * L.sb)[w] = load_behind(s1 + i);
         }
     }
 }
@@ -323,7 +323,7 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
     const int lv = 2 * p.C - 1;
     const float Cf = (float)p.C;
     const float neg_lr = -p.lr;
-    const uint32_t seed = p.seed + (p.seed_offset ? __ldg(p.seed_offset) : 0u);
+    const uint32_t seed = p.seed + (p.seed_offset ? load_behind(p.seed_offset) : 0u);
     const bool aligned16 = p.state_align >= 16;
 
     if (build_tables) {
@@ -348,17 +348,17 @@ __device__ __forceinline__ void update_u16_body(const UpdParams& p, const uint32
             if ((gpr & 31) == 0) {  // rows start on a period of the swizzle: the flat float4 index can be swizzled as it is
                 int i = tid;
                 for (; i + 3 * NT < n4; i += 4 * NT) {       // four loads in flight per thread
-                    const float4 v0 = __ldg(gsrc + i), v1 = __ldg(gsrc + i + NT), v2 = __ldg(gsrc + i + 2 * NT),
-                                 v3 = __ldg(gsrc + i + 3 * NT);
+                    const float4 v0 = load_behind(gsrc + i), v1 = load_behind(gsrc + i + NT), v2 = load_behind(gsrc + i + 2 * NT),
+                                 v3 = load_behind(gsrc + i + 3 * NT);
                     gw_s[swz4(i)] = v0; gw_s[swz4(i + NT)] = v1;
                     gw_s[swz4(i + 2 * NT)] = v2; gw_s[swz4(i + 3 * NT)] = v3;
                 }
-                for (; i < n4; i += NT) gw_s[swz4(i)] = __ldg(gsrc + i);
+                for (; i < n4; i += NT) gw_s[swz4(i)] = load_behind(gsrc + i);
             } else {                // flat over the batch; row = i / gpr by multiply-high (gpr = 4 * units per row)
                 for (int i = tid; i < n4; i += NT) {
                     const int r = unit_magic ? (int)__umulhi((uint32_t)i >> 2, unit_magic) : (i >> 2);
                     const int g = i - r * gpr;
-                    gw_s[r * gpr + swz4(g)] = __ldg(gsrc + i);
+                    gw_s[r * gpr + swz4(g)] = load_behind(gsrc + i);
                 }
             }
             }

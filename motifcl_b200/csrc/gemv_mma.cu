@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
             while (LIST && k + 1 < p.n && f >= p.m[k + 1].first) ++k;
             const int o = (f - p.m[k].first) * MV_ROWS + (j & (MV_ROWS - 1)), O = p.m[k].O;
             if (o >= O) continue;
-            const float sc = __ldg(p.m[k].scale + o);
+            const float sc = load_behind(p.m[k].scale + o);
             const size_t at = (size_t)(slot * Mp * MV_ROWS + j) * 8;
             double sum = 0.0, rest = 0.0;
 #pragma unroll 4

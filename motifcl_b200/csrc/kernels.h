@@ -10,8 +10,8 @@ namespace mcl {
 
 // Launches that follow one another on a stream overlap at their seams (programmatic dependent launch): a kernel launched with
 // launch_chained may start when all CTAs of the one before it run, sets itself up, and in grid_wait() waits until that one has completed
-// and its results can be read.  Rules: nothing of global memory that another launch may write is touched before grid_wait(), every CTA
-// gets there, and grid_release() comes after a CTA has its tensor memory, so that no CTA waits for memory that a later launch holds.
+// and its results can be read.  Rules: nothing of global memory that another launch may write is touched before grid_wait() nor, behind it, read
+// otherwise than by ordinary loads (load_behind), every CTA gets there, and grid_release() comes after a CTA has its tensor memory, so that no CTA waits for memory that a later launch holds.
 // What it saves is a few microseconds a launch: one layer of 288 x 288 at 256 rows (three launches) 38 -> 30 us, of 288 x 1536 at 4096 123 ->
 // 115, the fp32 ops of a block (13 launches) 219 -> 206, the update of 8192 x 4096 98 -> 95.  Not for the launches of tc_gemm.cu: long
 // kernels that fill the GPU gain nothing, and split_terms_kernel's waiting CTAs keep other streams' work off (a stack of 42 layers beside two
@@ -29,6 +29,24 @@ cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t sme
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What an earlier launch may have written, behind grid_wait(): an ordinary load that keeps its place.  The read-only path (__ldg, const
+// __restrict__) is for data that nobody writes while the kernel runs, and a kernel that overlaps runs while the one before it writes.
+template <class T>
+__device__ __forceinline__ T load_behind(const T* p) {
+    static_assert(sizeof(T) == 1 || sizeof(T) == 4 || sizeof(T) == 16, "8, 32 or 128 bits");
+    union { T v; uint32_t w[sizeof(T) == 16 ? 4 : 1]; } u;
+    if constexpr (sizeof(T) == 16) {
+        asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.w[0]), "=r"(u.w[1]), "=r"(u.w[2]), "=r"(u.w[3]) : "l"(p));
+        return u.v;
+    } else if constexpr (sizeof(T) == 4) {
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(u.w[0]) : "l"(p));
+        return u.v;
+    } else {
+        uint32_t w;
+        asm volatile("ld.global.u8 %0, [%1];" : "=r"(w) : "l"(p));
+        return static_cast<T>(w);
+    }
+}
 #endif
 
 // counter_update.cu

@@ -66,15 +66,15 @@ __device__ __forceinline__ float4 ld_peer(uint32_t addr, uint32_t rank) {      /
     return v;
 }
 // four consecutive floats of a row of n, zero beyond its end
-__device__ __forceinline__ float4 load4(const float* __restrict__ row, int c, int n, bool vec) {
+__device__ __forceinline__ float4 load4(const float* row, int c, int n, bool vec) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (vec) {
-        if (c < n) v = __ldg(reinterpret_cast<const float4*>(row + c));
+        if (c < n) v = load_behind(reinterpret_cast<const float4*>(row + c));
     } else {
-        if (c < n) v.x = __ldg(row + c);
-        if (c + 1 < n) v.y = __ldg(row + c + 1);
-        if (c + 2 < n) v.z = __ldg(row + c + 2);
-        if (c + 3 < n) v.w = __ldg(row + c + 3);
+        if (c < n) v.x = load_behind(row + c);
+        if (c + 1 < n) v.y = load_behind(row + c + 1);
+        if (c + 2 < n) v.z = load_behind(row + c + 2);
+        if (c + 3 < n) v.w = load_behind(row + c + 3);
     }
     return v;
 }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
         if (p.vec) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                r.a[j] = ((arows >> j) & 1u) && k < p.K ? __ldg(reinterpret_cast<const float4*>(q + j * astep)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r.a[j] = ((arows >> j) & 1u) && k < p.K ? load_behind(reinterpret_cast<const float4*>(q + j * astep)) : make_float4(0.f, 0.f, 0.f, 0.f);
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j) r.a[j] = load4(q + j * astep - k, k, (arows >> j) & 1u ? p.K : 0, false);
@@ -176,12 +176,12 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
             if (in) {
                 if (words) {
                     const uint32_t* s = reinterpret_cast<const uint32_t*>(g + u_off[j]);
-                    r.w[j][0] = __ldg(s); r.w[j][1] = __ldg(s + 1); r.w[j][2] = __ldg(s + 2);
+                    r.w[j][0] = load_behind(s); r.w[j][1] = load_behind(s + 1); r.w[j][2] = load_behind(s + 2);
                 } else {
                     const int nb = 3 * min(4, u_left[j] - (DX ? 0 : 16 * kt));
 #pragma unroll
                     for (int b = 0; b < 12; ++b)
-                        if (b < nb) r.w[j][b >> 2] |= (uint32_t)__ldg(g + u_off[j] + b) << (8 * (b & 3));
+                        if (b < nb) r.w[j][b >> 2] |= (uint32_t)load_behind(g + u_off[j] + b) << (8 * (b & 3));
                 }
             }
         }
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
             tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + cols + (uint32_t)c0, r1);
             tmem_ld_wait();
             const int col = n0 + c0 + lane;
-            const float sc = !DX && col < p.N ? __ldg(p.scale + col) : 1.0f;
+            const float sc = !DX && col < p.N ? load_behind(p.scale + col) : 1.0f;
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = __uint_as_float(r[j]) + __uint_as_float(r1[j]);
@@ -368,7 +368,7 @@ __device__ __forceinline__ void update_rows_by_group(const UpdParams& p, const i
     const float4* gw_s = reinterpret_cast<const float4*>(smem + L.off_gw);
     const int tid = threadIdx.x, lane = tid & 31, pair = tid >> 6, vlane = tid & 63;
     const int I = p.in_features, gpr = I >> 2, lv = 2 * p.C - 1;
-    const uint32_t seed = p.seed + (p.seed_offset ? __ldg(p.seed_offset) : 0u);
+    const uint32_t seed = p.seed + (p.seed_offset ? load_behind(p.seed_offset) : 0u);
     auto group = [&](int r, int g) -> uint32_t {
         const uint8_t* s = p.state + ((size_t)r * gpr + g) * 3;
         return (uint32_t)s[0] | ((uint32_t)s[1] << 8) | ((uint32_t)s[2] << 16);
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
             if (p.vec_dy) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    r.a[j] = warp + 16 * j < left && a_in ? __ldg(reinterpret_cast<const float4*>(q + (size_t)(16 * j) * p.O)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    r.a[j] = warp + 16 * j < left && a_in ? load_behind(reinterpret_cast<const float4*>(q + (size_t)(16 * j) * p.O)) : make_float4(0.f, 0.f, 0.f, 0.f);
             } else {
 #pragma unroll
                 for (int j = 0; j < 2; ++j) r.a[j] = load4(q + (size_t)(16 * j) * p.O - ac, ac, warp + 16 * j < left && a_in ? p.O : 0, false);
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_update_kernel(const __grid
             const float* g = bp + (size_t)kt * kDwK * I;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                r.b[j] = b_tok[j] < left && b_off[j] >= 0 ? __ldg(reinterpret_cast<const float4*>(g + b_off[j])) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r.b[j] = b_tok[j] < left && b_off[j] >= 0 ? load_behind(reinterpret_cast<const float4*>(g + b_off[j])) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
         for (int seg = 0; seg < nseg; ++seg) {
             const int k0 = DEEP ? seg * kDwDepth : 0, k1 = DEEP ? min(nkt, k0 + kDwDepth) : nkt;
@@ -653,8 +653,8 @@ __global__ void __launch_bounds__(kLThreads, 1) exact_update_kernel(const __grid
 #pragma unroll
             for (int j = 0; j < AHEAD; ++j) {
                 const int t = min(t0 + j, p.tokens - 1);
-                s.x[j] = __ldg(xp + (size_t)t * gpr);
-                s.d[j] = __ldg(dp + (size_t)t * p.O);
+                s.x[j] = load_behind(xp + (size_t)t * gpr);
+                s.d[j] = load_behind(dp + (size_t)t * p.O);
             }
         };
         auto sum = [&](int t0, const Set& s) {

@@ -52,10 +52,10 @@ constexpr int kNormHold = 8;          // H of the kernels: 3 for rows of up to 3
 struct Vec4 {                     // 128-bit accesses where rows start on 16-byte boundaries, else scalar ones
     bool vec;
     int cols;
-    __device__ __forceinline__ float4 get(const float* __restrict__ r, int c) const {
-        if (vec) return c < cols ? __ldg(reinterpret_cast<const float4*>(r + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        return make_float4(c < cols ? __ldg(r + c) : 0.f, c + 1 < cols ? __ldg(r + c + 1) : 0.f, c + 2 < cols ? __ldg(r + c + 2) : 0.f,
-                           c + 3 < cols ? __ldg(r + c + 3) : 0.f);
+    __device__ __forceinline__ float4 get(const float* r, int c) const {
+        if (vec) return c < cols ? load_behind(reinterpret_cast<const float4*>(r + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return make_float4(c < cols ? load_behind(r + c) : 0.f, c + 1 < cols ? load_behind(r + c + 1) : 0.f, c + 2 < cols ? load_behind(r + c + 2) : 0.f,
+                           c + 3 < cols ? load_behind(r + c + 3) : 0.f);
     }
     __device__ __forceinline__ void put(float* r, int c, float4 v) const {
         if (vec) { if (c < cols) *reinterpret_cast<float4*>(r + c) = v; return; }
@@ -68,8 +68,8 @@ struct Vec4 {                     // 128-bit accesses where rows start on 16-byt
 __device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
 
 template <int H>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                      float* __restrict__ out, float* __restrict__ row_inv,
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const float* x, const float* w,
+                                                      float* out, float* row_inv,
                                                       size_t rows, Vec4 a, float eps) {
     grid_release();
     grid_wait();
@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float* __restrict__ 
 }
 
 template <int H>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                            const float* __restrict__ dy, float* __restrict__ dx,
+__global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* x, const float* w,
+                                                            const float* dy, float* dx,
                                                             size_t rows, Vec4 a, float eps) {
     grid_release();
     grid_wait();
@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_x_kernel(const float* __restr
 // row_inv and dw[c] += dy * x * row_inv in one pass (up to kNormHold * 128 columns): a warp keeps the sums of its rows for its
 // columns in registers, the block adds its warps in shared memory, one atomic per column and block.  dw is zeroed before.
 template <int H>
-__global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                                                                 float* __restrict__ row_inv, float* __restrict__ dw, size_t rows, Vec4 a, float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* x, const float* dy,
+                                                                 float* row_inv, float* dw, size_t rows, Vec4 a, float eps) {
     grid_release();
     grid_wait();
     __shared__ float4 part[8][32];
@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_w_rows_kernel(const float* __
 }
 
 // dw[c] += sum over this block's rows of dy*x*row_inv; dw is zeroed before the launch.
-__global__ void __launch_bounds__(256) rmsnorm_bwd_w_kernel(const float* __restrict__ x, const float* __restrict__ dy,
-                                                            const float* __restrict__ row_inv, float* __restrict__ dw,
+__global__ void __launch_bounds__(256) rmsnorm_bwd_w_kernel(const float* x, const float* dy,
+                                                            const float* row_inv, float* dw,
                                                             size_t rows, int cols, size_t rows_per_block) {
     grid_release();
     grid_wait();
@@ -220,7 +220,7 @@ __device__ __forceinline__ void swiglu_grads(float gate, float up, float go, flo
     du = go * gate * sig;
 }
 template <int W>
-__global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ packed, float* __restrict__ out,
+__global__ void __launch_bounds__(256) swiglu_kernel(const float* packed, float* out,
                                                      size_t rows, int hidden) {
     grid_release();
     grid_wait();
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ p
         const size_t row = i / hw;
         const size_t base = row * 2 * hidden + (i - row * hw) * W;
         if (W == 4) {
-            const float4 g = __ldg(reinterpret_cast<const float4*>(packed + base)), u = __ldg(reinterpret_cast<const float4*>(packed + base + hidden));
+            const float4 g = load_behind(reinterpret_cast<const float4*>(packed + base)), u = load_behind(reinterpret_cast<const float4*>(packed + base + hidden));
             reinterpret_cast<float4*>(out)[i] = make_float4(g.x * (1.0f / (1.0f + expf(-g.x))) * u.x, g.y * (1.0f / (1.0f + expf(-g.y))) * u.y,
                                                             g.z * (1.0f / (1.0f + expf(-g.z))) * u.z, g.w * (1.0f / (1.0f + expf(-g.w))) * u.w);
         } else {
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ p
     }
 }
 template <int W>
-__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* __restrict__ packed, const float* __restrict__ dy,
-                                                         float* __restrict__ dpacked, size_t rows, int hidden) {
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* packed, const float* dy,
+                                                         float* dpacked, size_t rows, int hidden) {
     grid_release();
     grid_wait();
     const int hw = hidden / W;
@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* __restrict
         const size_t row = i / hw;
         const size_t base = row * 2 * hidden + (i - row * hw) * W;
         if (W == 4) {
-            const float4 g = __ldg(reinterpret_cast<const float4*>(packed + base)), u = __ldg(reinterpret_cast<const float4*>(packed + base + hidden));
-            const float4 go = __ldg(reinterpret_cast<const float4*>(dy) + i);
+            const float4 g = load_behind(reinterpret_cast<const float4*>(packed + base)), u = load_behind(reinterpret_cast<const float4*>(packed + base + hidden));
+            const float4 go = load_behind(reinterpret_cast<const float4*>(dy) + i);
             float4 a, b;
             swiglu_grads(g.x, u.x, go.x, a.x, b.x); swiglu_grads(g.y, u.y, go.y, a.y, b.y);
             swiglu_grads(g.z, u.z, go.z, a.z, b.z); swiglu_grads(g.w, u.w, go.w, a.w, b.w);
@@ -277,9 +277,9 @@ __device__ __forceinline__ void online_add(float v, float& m, float& s) {
     else s += expf(v - m);
 }
 template <bool BACKWARD>
-__global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict__ logits, const int* __restrict__ targets,
-                                                        float* __restrict__ partial, const float* __restrict__ grad_out,
-                                                        float* __restrict__ grad_logits, size_t rows, int cols, int vec) {
+__global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* logits, const int* targets,
+                                                        float* partial, const float* grad_out,
+                                                        float* grad_logits, size_t rows, int cols, int vec) {
     grid_release();
     grid_wait();
     __shared__ float red[32];
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict_
         float m = -FLT_MAX, s = 0.0f;
 #pragma unroll 4
         for (int i = threadIdx.x; i < n4; i += kCeThreads) {
-            const float4 v = BACKWARD ? __ldg(l4 + i) : __ldcs(l4 + i);
+            const float4 v = BACKWARD ? load_behind(l4 + i) : __ldcs(l4 + i);
             const float mv = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
             if (mv > m) { s *= expf(m - mv); m = mv; }
             s += (expf(v.x - m) + expf(v.y - m)) + (expf(v.z - m) + expf(v.w - m));
@@ -307,21 +307,27 @@ __global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* __restrict_
             const float inv = 1.0f / s;
             float* g = grad_logits + row * (size_t)cols;
             float4* g4 = reinterpret_cast<float4*>(g);
-#pragma unroll 4
-            for (int i = threadIdx.x; i < n4; i += kCeThreads) {
-                const float4 v = __ldcs(l4 + i);
-                const int c = 4 * i;
-                __stcs(g4 + i, make_float4(gscale * (expf(v.x - m) * inv - (c == t ? 1.0f : 0.0f)),
-                                           gscale * (expf(v.y - m) * inv - (c + 1 == t ? 1.0f : 0.0f)),
-                                           gscale * (expf(v.z - m) * inv - (c + 2 == t ? 1.0f : 0.0f)),
-                                           gscale * (expf(v.w - m) * inv - (c + 3 == t ? 1.0f : 0.0f))));
+            for (int i0 = threadIdx.x; i0 < n4; i0 += 4 * kCeThreads) {
+                float4 v[4];                       // four loads in flight before the stores
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i0 + k * kCeThreads < n4) v[k] = __ldcs(l4 + i0 + k * kCeThreads);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = i0 + k * kCeThreads, c = 4 * i;
+                    if (i < n4)
+                        __stcs(g4 + i, make_float4(gscale * (expf(v[k].x - m) * inv - (c == t ? 1.0f : 0.0f)),
+                                                   gscale * (expf(v[k].y - m) * inv - (c + 1 == t ? 1.0f : 0.0f)),
+                                                   gscale * (expf(v[k].z - m) * inv - (c + 2 == t ? 1.0f : 0.0f)),
+                                                   gscale * (expf(v[k].w - m) * inv - (c + 3 == t ? 1.0f : 0.0f))));
+                }
             }
             for (int c = 4 * n4 + threadIdx.x; c < cols; c += kCeThreads)
                 g[c] = gscale * (expf(l[c] - m) * inv - (c == t ? 1.0f : 0.0f));
         }
     }
 }
-__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ in, float* __restrict__ out, size_t n,
+__global__ void __launch_bounds__(1024) mean_kernel(const float* in, float* out, size_t n,
                                                    size_t denom) {
     grid_release();
     grid_wait();
@@ -536,7 +542,7 @@ __global__ void __launch_bounds__(256) position_backward_kernel(const float* __r
 // (i, i + head_dim/2), otherwise (2i, 2i+1).  inverse negates the angle.  Block = one token position: sines and cosines of its
 // pairs are formed once (powf and sincosf cost 15 us per call when every element formed its own) and serve the rows of
 // that position in all batch elements of the block's share.
-__global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
+__global__ void __launch_bounds__(256) rope_kernel(const float* x, float* out, int batch, int tokens,
                                                    int channels, int n_head, int head_dim, int rotary_dim, int token_offset,
                                                    float theta, int inverse, int split_half, int shared_turns) {
     grid_release();
@@ -608,7 +614,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const float* __restrict__ x, 
 // channels of a batch element, all of its loads in flight at once (rope_kernel loads every element
 // twice, once for its partner: 12 us for 16 x 256 rows of 288 channels, of which 1.5 are traffic).
 constexpr int kRopeIn = 4;             // quads of a thread in flight
-__global__ void __launch_bounds__(256) rope_quads_kernel(const float* __restrict__ x, float* __restrict__ out, int batch, int tokens,
+__global__ void __launch_bounds__(256) rope_quads_kernel(const float* x, float* out, int batch, int tokens,
                                                          int channels, int head_dim, int rd, int token_offset, float theta, int inverse) {
     grid_release();
     extern __shared__ float2 rot[];                   // (cos, sin) of pair i
@@ -630,7 +636,7 @@ __global__ void __launch_bounds__(256) rope_quads_kernel(const float* __restrict
 #pragma unroll
         for (int k = 0; k < kRopeIn; ++k) {
             const int u = u0 + k * 256, b = u / quads;
-            if (u < n) v[k] = __ldg(reinterpret_cast<const float4*>(x + start + b * step) + (u - b * quads));
+            if (u < n) v[k] = load_behind(reinterpret_cast<const float4*>(x + start + b * step) + (u - b * quads));
         }
 #pragma unroll
         for (int k = 0; k < kRopeIn; ++k) {

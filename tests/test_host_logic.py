@@ -90,3 +90,24 @@ def test_magnitude_sample_covers_rows_and_columns(tmp_path, rows, cols):
     assert seen.max() <= 3 * -(-at.size // groups) + 2                          # no column is favoured
     assert np.count_nonzero(seen) >= 0.35 * min(groups, at.size)                 # chance would give 1 - e^(-samples / groups)
     assert np.count_nonzero(np.bincount(at // groups, minlength=rows)) >= 0.35 * min(rows, at.size)
+
+
+def test_overlapping_kernels_read_by_ordinary_loads():
+    """A kernel that starts before the one in front of it has ended (grid_wait) must not read through the read-only path: __ldg,
+    ld.global.nc or const __restrict__.  The 2-bit words of a decode GEMV, which no such launch writes, are the exception."""
+    csrc = os.path.join(os.path.dirname(mb._lib.HEADER_PATH), os.pardir, "motifcl_b200", "csrc")
+    kernels = 0
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        text = re.sub(r"uint4 mv_load\(.*?\n}", "", text, flags=re.S)
+        head, *parts = re.split(r"(?=__global__)", text)
+        waiting = [p for p in parts if "grid_wait();" in p]
+        kernels += len(waiting)
+        if name == "counter_update_body.cuh" or waiting:           # and the helpers in front of the kernels
+            waiting.append(head)
+        for p in waiting:
+            assert not re.search(r"__ldg\s*\(|ld\.global\.nc", p), (name, p[:120])
+            assert "__restrict__" not in p[:p.find("{")] or p is head, (name, p[:120])
+    assert kernels >= 15
