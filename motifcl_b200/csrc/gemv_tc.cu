@@ -333,7 +333,8 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         };
         int n_local = 0, x = -1;
         bool ok = true, begun = false;
-        for (GvParts<ROWS != 0> t(p, u_begin, u_end, wide); ok && t.next(); ++n_local) {
+        // A warp that gives up (ok) goes on through the parts and passes every barrier of the four: the others may not have seen it yet
+        for (GvParts<ROWS != 0> t(p, u_begin, u_end, wide); t.next(); ++n_local) {
             const GvMat& A = p.m[t.m];
             const bool sliced = ROWS && (wide >> A.x & 1);
             if (t.kb0 == 0 || n_local == 0) begun = t.kb0 == 0;
@@ -397,17 +398,17 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty(h));
             }
-            if (!ok || (whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
+            if ((whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
             if (!whole) {                 // the last of the CTAs that share the tile finishes it
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (threadIdx.x == 64 + 128 * RT) last_ticket = atomicAdd(p.tickets + slot_i, 1) == gv_last_cta(p, blockIdx.x, tile_u + t.kbs) - from;
+                if (threadIdx.x == 64 + 128 * RT) last_ticket = ok && atomicAdd(p.tickets + slot_i, 1) == gv_last_cta(p, blockIdx.x, tile_u + t.kbs) - from;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (!last_ticket) continue;
                 __threadfence();
             }
 #pragma unroll 1
-            for (int h = 0; h < RT; ++h) {
+            for (int h = 0; h < RT && ok; ++h) {
                 const int row = (t.tile * RT + h) * GV_ROWS + lrow;
                 if (sliced) {
 #pragma unroll 1

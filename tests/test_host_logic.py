@@ -111,3 +111,30 @@ def test_overlapping_kernels_read_by_ordinary_loads():
             assert not re.search(r"__ldg\s*\(|ld\.global\.nc", p), (name, p[:120])
             assert "__restrict__" not in p[:p.find("{")] or p is head, (name, p[:120])
     assert kernels >= 15
+
+
+def test_decode_epilogue_passes_its_barriers_whatever_a_warp_has_seen():
+    """A wait that runs out is seen by the four epilogue warps of the decode kernel at different times: what leads to their common
+    barriers may depend on the parts of the list alone, not on the warp's own state (`ok`)."""
+    csrc = os.path.join(os.path.dirname(mb._lib.HEADER_PATH), os.pardir, "motifcl_b200", "csrc")
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, "gemv_tc.cu")).read())
+    at = text.index("for (GvParts", text.index("int n_local = 0, x = -1;"))
+    end = depth = 0
+    for i in range(at, len(text)):                               # the loop over the parts
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0 and text[i] == "}":
+            end = i
+            break
+    loop = text[at:end]
+    assert loop.count("bar.sync 1, 128") == 4
+    code = loop[:loop.rindex("bar.sync 1, 128")]
+    inner = code.index("for (int h = 0; h < RT && ok; ++h) {")   # leaves by itself; no barrier inside
+    depth = 0
+    for i in range(inner, len(code)):
+        depth += {"{": 1, "}": -1}.get(code[i], 0)
+        if depth == 0 and code[i] == "}":
+            break
+    assert "bar.sync" not in code[inner:i]
+    for line in (code[:inner] + code[i:]).splitlines():
+        if re.search(r"\bok\b|\babort_flag\b", line):
+            assert not re.search(r"\bif \((?!threadIdx)|\bfor\b|\bwhile\b|\bcontinue\b|\bbreak\b|\breturn\b", line), line
