@@ -17,6 +17,7 @@
 // Every wait on an mbarrier is bounded; on time-out the error word is set and the results are invalid.
 #include <cuda_bf16.h>
 
+#include <cfloat>
 #include <type_traits>
 
 #include "counter_codec.cuh"
@@ -279,8 +280,8 @@ __global__ void __launch_bounds__(kLThreads, 1) layer_rows_kernel(const RowParam
         const int share = 128 / p.parts, quads = BN >> 2, row0 = (int)cluster_rank() * share;
         const bool wide = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 15) == 0;
         auto add = [](float& s, float& e, float v, float w) {      // s + e += v + w, s rounded, e what that loses
-            const float t = __fadd_rn(s, v), u = __fsub_rn(t, s);
-            e = __fadd_rn(e, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(v, u)), w));
+            const float t = __fadd_rn(s, v), u = __fsub_rn(t, s), lost = __fadd_rn(__fsub_rn(s, __fsub_rn(t, u)), __fsub_rn(v, u));
+            e = __fadd_rn(e, __fadd_rn(fabsf(t) <= FLT_MAX ? lost : 0.0f, w));      // a sum that left fp32 is an infinity and loses nothing
             s = t;
         };
         for (int i = tid; i < share * quads; i += kLThreads) {

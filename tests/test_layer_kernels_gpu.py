@@ -43,6 +43,27 @@ def test_row_products_against_float64(ctx, N, I, O):
     assert float((dx - rdx).norm() / rdx.norm()) < 1e-6
 
 
+# cut over clusters of 8, 8 and 4 in one product at least, and whole K
+@pytest.mark.parametrize("N,I,O", [(40, 1024, 1025), (130, 100, 2047), (600, 640, 301), (127, 288, 288)])
+def test_row_sums_that_leave_fp32_are_infinities(ctx, N, I, O):
+    """Row m of x has the signs of the digits of output m, row m of dy those of input m: every term of one sum is positive."""
+    st, sc, _, x, dy = _layer(N, I, O, N + I + O)
+    w = torch.empty(O, I, device="cuda")
+    ctx.counter_decode_weight(st, torch.ones_like(sc), w, I, O, 11)
+    ctx.finish()
+    n, k = min(N, O), min(N, I)
+    x[:n], dy[:k] = 2e38 * w[:n], 2e38 * w[:, :k].T
+    y, dx = torch.full((N, O), 7.0, device="cuda"), torch.full((N, I), 7.0, device="cuda")
+    torch.cuda.synchronize()
+    ctx.counter_forward(x, st, sc, y, N, I, O, 11)
+    ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
+    ctx.finish()
+    many = w.abs().sum(dim=1)[:n] >= 4                                   # 2e38 each: beyond 3.4e38
+    assert bool(many.any()) and bool((y.diagonal()[:n][many] == float("inf")).all())
+    far = (sc.double() @ w.abs().double())[:k] * 2e38 > 1e39
+    assert bool(far.any()) and bool((dx.diagonal()[:k][far] == float("inf")).all())
+
+
 @pytest.mark.parametrize("lr_scale", [0.0, 1e-3])
 @pytest.mark.parametrize("N,I,O", SHAPES)
 def test_update_against_the_exact_path(ctx, N, I, O, lr_scale):
