@@ -304,8 +304,8 @@ int mcl_cuda_eltwise_f32(mcl_cuda_ctx* ctx, int op, const float* a, const float*
  *                           out [B*Tq, n_head*vhd]; causal with query_offset, optional sliding window (0 = none);
  *                           f32 keys/values, no mask
  *   gqa_backward            probs_scratch, ds_scratch [B*n_head*Tq*Tk]; grad_q/k/v shaped like q/k/v
- *                           (attention, head_dim <= 64: an infinity or NaN in q, k, v or grad_out may make everything NaN that is
- *                           computed from a tile of 64 rows it lies in) ---- */
+ *                           (attention, head_dim <= 64: keys that a query does not attend to count as 0 times their value where
+ *                           they share a tile of 64 with ones that it does, so an infinity or NaN there makes its result NaN) ---- */
 int mcl_cuda_rmsnorm(mcl_cuda_ctx* ctx, const float* x, const float* weight, float* out, size_t rows, size_t cols,
                      float eps);
 int mcl_cuda_rmsnorm_backward_x(mcl_cuda_ctx* ctx, const float* x, const float* weight, const float* grad_out,

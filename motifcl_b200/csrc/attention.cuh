@@ -2,7 +2,7 @@
 // those that do): exact fp32 FMAs on tiles in shared memory (tf32 would not hold the reference's accuracy), scores never written by
 // the forward pass.  Included by trainer_ops.cu.
 //
-// A CTA owns BQ queries of one head and walks over tiles of 64 keys with TWO groups of 2 BQ threads that take alternate tiles
+// A CTA owns 32 queries of one head and walks over tiles of 64 keys with TWO groups of 64 threads that take alternate tiles
 // (a training step has few query tiles: one group left 10 warps on an SM, each issuing every 5.6 cycles) and merge at the end.
 // Thread (ty, tx) of a group holds 8 queries x 4 keys (keys tx + 16 j) of a score tile and 8 queries x NC columns (tx + 16 j) of
 // the output.  Products run on the two-lane FMA (fma.rn.f32x2, the rounding of two FMAs in one issue slot) over pairs of queries:
@@ -20,6 +20,7 @@
 #pragma once
 
 constexpr int kKT = 64;               // keys per tile
+constexpr int kBQ = 32;               // queries per tile
 
 __device__ __forceinline__ float half_sum(float v) {
 #pragma unroll
@@ -101,8 +102,8 @@ __device__ __forceinline__ float2 halves(unsigned long long v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
     return f;
 }
-// s[i][j] = sum over d of a[d][8 ty + i] b[tx + 16 j][d]; a: BQ + 4 floats per d, b: HDP + 4 per row
-template <int BQ, int HDP>
+// s[i][j] = sum over d of a[d][8 ty + i] b[tx + 16 j][d]; a: kBQ + 4 floats per d, b: HDP + 4 per row
+template <int HDP>
 __device__ __forceinline__ void scores(float (&s)[8][4], const float* a, const float* b, int ty, int tx) {
     const float* pa = a + 8 * ty;
     const float* pb = b + tx * (HDP + 4);
@@ -118,7 +119,7 @@ __device__ __forceinline__ void scores(float (&s)[8][4], const float* a, const f
         for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(bv[j]) = *reinterpret_cast<const float4*>(pb + 16 * j * (HDP + 4) + d);
 #pragma unroll
         for (int dd = 0; dd < 4; ++dd) {
-            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(pa + (d + dd) * (BQ + 4)), a1 = *reinterpret_cast<const ulonglong2*>(pa + (d + dd) * (BQ + 4) + 4);
+            const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(pa + (d + dd) * (kBQ + 4)), a1 = *reinterpret_cast<const ulonglong2*>(pa + (d + dd) * (kBQ + 4) + 4);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 unsigned long long bb;
@@ -153,17 +154,17 @@ __device__ __forceinline__ void outer(unsigned long long (&acc)[4][NC], const fl
 }
 __device__ __forceinline__ void group_sync(int group, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(threads) : "memory"); }
 
-// floats of shared memory: rows of HDP + 4 for tiles, of BQ + 4 for transposed probability tiles
-template <int BQ, int NC>
-__host__ __device__ constexpr size_t fwd_group_floats() { return (size_t)2 * kKT * (16 * NC + 4) + kKT * (BQ + 4); }
-template <int BQ, int NC>
-__host__ __device__ constexpr size_t fwd_floats() { return (size_t)16 * NC * (BQ + 4) + 2 * fwd_group_floats<BQ, NC>(); }
-template <int BQ, int NC>
+// floats of shared memory: rows of HDP + 4 for tiles, of kBQ + 4 for transposed probability tiles
+template <int NC>
+__host__ __device__ constexpr size_t fwd_group_floats() { return (size_t)2 * kKT * (16 * NC + 4) + kKT * (kBQ + 4); }
+template <int NC>
+__host__ __device__ constexpr size_t fwd_floats() { return (size_t)16 * NC * (kBQ + 4) + 2 * fwd_group_floats<NC>(); }
+template <int NC>
 __host__ __device__ constexpr size_t bwd_q_group_floats() {      // k and v tiles, or k and dS tiles
-    return (size_t)kKT * (16 * NC + 4) + ((size_t)kKT * (16 * NC + 4) > (size_t)kKT * (BQ + 4) ? (size_t)kKT * (16 * NC + 4) : (size_t)kKT * (BQ + 4));
+    return (size_t)kKT * (16 * NC + 4) + ((size_t)kKT * (16 * NC + 4) > (size_t)kKT * (kBQ + 4) ? (size_t)kKT * (16 * NC + 4) : (size_t)kKT * (kBQ + 4));
 }
-template <int BQ, int NC>
-__host__ __device__ constexpr size_t bwd_q_floats() { return (size_t)2 * 16 * NC * (BQ + 4) + 2 * bwd_q_group_floats<BQ, NC>() + 6 * BQ; }
+template <int NC>
+__host__ __device__ constexpr size_t bwd_q_floats() { return (size_t)2 * 16 * NC * (kBQ + 4) + 2 * bwd_q_group_floats<NC>() + 6 * kBQ; }
 template <int NC>
 __host__ __device__ constexpr size_t bwd_k_group_floats() { return (size_t)2 * 32 * (kKT + 4) + 2 * (size_t)32 * (16 * NC + 4); }
 template <int NC>
@@ -183,18 +184,17 @@ __device__ __forceinline__ void tile_range(const GqaDims& p, int q0, int& kb, in
     ke = b1;
 }
 
-template <int BQ, int NC>
-__global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                         const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
-    grid_release();
+// queries q0 .. q0 + 31 of the head blockIdx.x, by 128 threads
+template <int NC>
+__device__ __forceinline__ void fwd_rows(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, float* __restrict__ out,
+                                         const GqaDims& p, int q0) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
+    constexpr int BQ = kBQ, HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
     float* qs = sm;                                                        // [HDP][QS]
-    float* ks = qs + HDP * QS + grp * fwd_group_floats<BQ, NC>();           // this group's k [64][HS], v [64][HS], P^T [64][QS]
+    float* ks = qs + HDP * QS + grp * fwd_group_floats<NC>();           // this group's k [64][HS], v [64][HS], P^T [64][QS]
     float* vs = ks + kKT * HS;
     float* pt = vs + kKT * HS;
-    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, g = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.key_stride * kld + g * p.hd;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_fwd_kernel(const float* 
         copies_wait<1>();
         group_sync(grp, NT);
         float s[8][4];
-        scores<BQ, HDP>(s, qs, ks, ty, tx);
+        scores<HDP>(s, qs, ks, ty, tx);
         group_sync(grp, NT);
         copy_rows<kKT, NT, HDP, HS>(ks, kb_, kld, k0 + 2 * kKT, p.tk, p.hd, vec, t);
         float alpha[8];
@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_fwd_kernel(const float* 
 #pragma unroll
     for (int i = 0; i < 8; ++i) l[i] = half_sum(l[i]);
     // merge the groups: the second leaves maximum, sum and accumulator in its tiles
-    float* mg = qs + HDP * QS + fwd_group_floats<BQ, NC>();      // [8 + 8 + 8 NC][NT] floats
-    static_assert(fwd_group_floats<BQ, NC>() >= (size_t)(16 + 8 * NC) * NT, "merge area");
+    float* mg = qs + HDP * QS + fwd_group_floats<NC>();      // [8 + 8 + 8 NC][NT] floats
+    static_assert(fwd_group_floats<NC>() >= (size_t)(16 + 8 * NC) * NT, "merge area");
     __syncthreads();
     if (grp == 1) {
 #pragma unroll
@@ -300,21 +300,27 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_fwd_kernel(const float* 
     }
 }
 
-// probs, ds [B, n_head, tq, tk]; dq
-template <int BQ, int NC>
-__global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                                           const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
-                                                           float* __restrict__ dq, GqaDims p) {
+// the tiles with the longest rows first
+__device__ __forceinline__ int tile_begin(const GqaDims& p, int rows) { return ((p.tq + rows - 1) / rows - 1 - (int)blockIdx.y) * rows; }
+template <int NC>
+__global__ void __launch_bounds__(128, 4) gqa_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                         float* __restrict__ out, GqaDims p) {
     grid_release();
+    fwd_rows<NC>(q, k, v, out, p, tile_begin(p, kBQ));
+}
+
+// probs, ds [B, n_head, tq, tk]; dq
+template <int NC>
+__device__ __forceinline__ void bwd_q_rows(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ dout,
+                                           float* __restrict__ probs, float* __restrict__ ds, float* __restrict__ dq, const GqaDims& p, int q0) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
+    constexpr int BQ = kBQ, HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
     float* qs = sm;                       // [HDP][QS]
     float* gs = qs + HDP * QS;            // dO
-    float* ks = gs + HDP * QS + grp * bwd_q_group_floats<BQ, NC>();      // this group's k [64][HS]
+    float* ks = gs + HDP * QS + grp * bwd_q_group_floats<NC>();      // this group's k [64][HS]
     float* vs = ks + kKT * HS;            // pass 1: v [64][HS]; pass 2: dS^T [64][QS]
-    float* st = gs + HDP * QS + 2 * bwd_q_group_floats<BQ, NC>();        // [2][3][BQ]: maximum, sum, sum of P dP of each group
-    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
+    float* st = gs + HDP * QS + 2 * bwd_q_group_floats<NC>();        // [2][3][BQ]: maximum, sum, sum of P dP of each group
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, g = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.tk * kld + g * p.hd;
@@ -340,12 +346,12 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_bwd_q_kernel(const float
         float s[8][4], d[8][4];
         copies_wait<1>();
         group_sync(grp, NT);
-        scores<BQ, HDP>(s, qs, ks, ty, tx);
+        scores<HDP>(s, qs, ks, ty, tx);
         group_sync(grp, NT);
         copy_rows<kKT, NT, HDP, HS>(ks, kb_, kld, k0 + 2 * kKT, p.tk, p.hd, vec, t);
         copies_wait<1>();
         group_sync(grp, NT);
-        scores<BQ, HDP>(d, gs, vs, ty, tx);
+        scores<HDP>(d, gs, vs, ty, tx);
         group_sync(grp, NT);
         copy_rows<kKT, NT, HDP, HS>(vs, vb, kld, k0 + 2 * kKT, p.tk, p.hd, vec, t);
 #pragma unroll
@@ -452,8 +458,8 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_bwd_q_kernel(const float
         copy_rows<kKT, NT, HDP, HS>(ks, kb_, kld, k0 + 2 * kKT, p.tk, p.hd, vec, t);
     }
     copies_wait<0>();
-    float* mg = gs + HDP * QS + bwd_q_group_floats<BQ, NC>();      // the second group's tiles
-    static_assert(bwd_q_group_floats<BQ, NC>() >= (size_t)8 * NC * NT, "merge area");
+    float* mg = gs + HDP * QS + bwd_q_group_floats<NC>();      // the second group's tiles
+    static_assert(bwd_q_group_floats<NC>() >= (size_t)8 * NC * NT, "merge area");
     __syncthreads();
     if (grp == 1) {
 #pragma unroll
@@ -478,12 +484,19 @@ __global__ void __launch_bounds__(4 * BQ, 128 / BQ) gqa_bwd_q_kernel(const float
         }
 }
 
-constexpr int kQT = 32;               // queries per tile of the key kernel
-// CTA = 64 keys of one kv head, two groups of 128 threads that take alternate tiles of 32 queries
 template <int NC>
-__global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
-                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
+__global__ void __launch_bounds__(128, 4) gqa_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                           const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
+                                                           float* __restrict__ dq, GqaDims p) {
     grid_release();
+    bwd_q_rows<NC>(q, k, v, dout, probs, ds, dq, p, tile_begin(p, kBQ));
+}
+
+constexpr int kQT = 32;               // queries per tile of the key kernel
+// 64 keys of one kv head by G groups of 128 threads, which take the tiles of 32 queries in turn
+template <int NC, int G>
+__device__ __forceinline__ void bwd_k_keys(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
+                                           const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, const GqaDims& p) {
     extern __shared__ __align__(16) float sm[];
     constexpr int HDP = 16 * NC, HS = HDP + 4, KS = kKT + 4;
     const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;
@@ -514,22 +527,22 @@ __global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restri
     };
     first(grp);
     second(grp);
-    for (int n = grp; n < count; n += 2) {
+    for (int n = grp; n < count; n += G) {
         copies_wait<2>();
         group_sync(grp, 128);
         outer<NC>(av, ps, KS, gs, HS, kQT, ty, tx);
         group_sync(grp, 128);
-        first(n + 2);
+        first(n + G);
         copies_wait<2>();
         group_sync(grp, 128);
         outer<NC>(ak, ss, KS, qs, HS, kQT, ty, tx);
         group_sync(grp, 128);
-        second(n + 2);
+        second(n + G);
     }
     copies_wait<0>();
     float* mg = sm + bwd_k_group_floats<NC>();
     static_assert(bwd_k_group_floats<NC>() >= (size_t)16 * NC * 128, "merge area");
-    __syncthreads();
+    if (G > 1) __syncthreads();
     if (grp == 1) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -540,7 +553,7 @@ __global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restri
                 mg[((4 * i + 2) * NC + j) * 128 + t] = e.x; mg[((4 * i + 3) * NC + j) * 128 + t] = e.y;
             }
     }
-    __syncthreads();
+    if (G > 1) __syncthreads();
     if (grp == 1) return;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -551,8 +564,14 @@ __global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restri
                 const float2 f = halves(av[i >> 1][j]), e = halves(ak[i >> 1][j]);
                 const long long at = ((long long)b * p.tk + key) * kld + g * p.hd + tx + 16 * j;
                 const int r = 4 * (i >> 1) + (i & 1);
-                dv[at] = (i & 1 ? f.y : f.x) + mg[(r * NC + j) * 128 + t];
-                dk[at] = ((i & 1 ? e.y : e.x) + mg[((r + 2) * NC + j) * 128 + t]) * p.scale;
+                dv[at] = (i & 1 ? f.y : f.x) + (G > 1 ? mg[(r * NC + j) * 128 + t] : 0.0f);
+                dk[at] = ((i & 1 ? e.y : e.x) + (G > 1 ? mg[((r + 2) * NC + j) * 128 + t] : 0.0f)) * p.scale;
             }
     }
+}
+template <int NC>
+__global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
+                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
+    grid_release();
+    bwd_k_keys<NC, 2>(q, dout, probs, ds, dk, dv, p);
 }

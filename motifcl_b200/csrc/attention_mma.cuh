@@ -30,6 +30,7 @@ template <int NC>
 struct AttTile {                                     // 64 rows of HDP columns, three planes of bf16 terms; the pitch keeps ldmatrix free of conflicts
     static constexpr int HDP = 16 * NC, kPitch = HDP + 8, kPlane = 64 * kPitch * 2, kBytes = 3 * kPlane;
     static constexpr int kRaw = 64 * HDP * 4;        // the fp32 rows as they come
+    static constexpr size_t kShared = 2 * (kBytes + kRaw);
 };
 __device__ __forceinline__ uint32_t sm_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // staging rows -> terms; thread t of NT
@@ -145,6 +146,30 @@ __device__ __forceinline__ void load_rows(uint32_t (&a)[NC][3][4], const float* 
 __device__ __forceinline__ float quad_max(float v) { v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1)); return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2)); }
 __device__ __forceinline__ float quad_sum(float v) { v += __shfl_xor_sync(0xffffffffu, v, 1); return v + __shfl_xor_sync(0xffffffffu, v, 2); }
 
+// Terms of an infinity are an infinity and NaNs.  A CTA whose results are not all finite does its part again with the fp32 FMAs of
+// attention.cuh, where an infinity stays one: NaN or infinity in an operand that a result takes shows in the result.
+template <int N>
+__device__ __forceinline__ bool beyond_fp32(const float (&c)[N][4]) {
+    bool b = false;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) b = b || !(fabsf(c[n][i]) <= FLT_MAX);
+    return b;
+}
+template <int NC>
+__device__ __noinline__ void fwd_again(const float* q, const float* k, const float* v, float* out, const GqaDims& p, int q0) {
+    fwd_rows<NC>(q, k, v, out, p, q0);
+}
+template <int NC>
+__device__ __noinline__ void bwd_q_again(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, const GqaDims& p, int q0) {
+    bwd_q_rows<NC>(q, k, v, dout, probs, ds, dq, p, q0);
+}
+template <int NC>
+__device__ __noinline__ void bwd_k_again(const float* q, const float* dout, const float* probs, const float* ds, float* dk, float* dv, const GqaDims& p) {
+    bwd_k_keys<NC, 1>(q, dout, probs, ds, dk, dv, p);
+}
+
 template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                                        const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
@@ -155,7 +180,7 @@ __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __rest
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
     unsigned char *ks = smb, *vs = smb + T::kBytes;
     float *kr = reinterpret_cast<float*>(smb + 2 * T::kBytes), *vr = kr + T::kRaw / 4;
-    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
+    const int q0 = tile_begin(p, BQ);
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, gr = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.key_stride * kld + gr * p.hd;
@@ -228,6 +253,10 @@ __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __rest
         }
     }
     copies_wait<0>();
+    if (__syncthreads_or(beyond_fp32(o))) {
+        for (int r = q0; r < min(q0 + BQ, p.tq); r += kBQ, __syncthreads()) fwd_again<NC>(q, k, v, out, p, r);
+        return;
+    }
     float* ob = out + (long long)b * p.tq * qld + h * p.hd;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -254,7 +283,7 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
     unsigned char *ks = smb, *vs = smb + T::kBytes;
     float *kr = reinterpret_cast<float*>(smb + 2 * T::kBytes), *vr = kr + T::kRaw / 4;
-    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
+    const int q0 = tile_begin(p, BQ);
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, gr = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd, at = (long long)b * p.tq * qld + h * p.hd;
     const float* kb_ = k + (long long)b * p.tk * kld + gr * p.hd;
@@ -388,6 +417,10 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
         }
     }
     copies_wait<0>();
+    if (__syncthreads_or(beyond_fp32(acc))) {
+        for (int r = q0; r < min(q0 + BQ, p.tq); r += kBQ, __syncthreads()) bwd_q_again<NC>(q, k, v, dout, probs, ds, dq, p, r);
+        return;
+    }
     // beyond every query of the tile: zeros
     {
         const float zero[2][4] = {};
@@ -490,6 +523,10 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_k_mma_kernel(const float* __re
         add(ak, qs);
     }
     copies_wait<0>();
+    if (__syncthreads_or(beyond_fp32(av) || beyond_fp32(ak))) {
+        bwd_k_again<NC>(q, dout, probs, ds, dk, dv, p);
+        return;
+    }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         if (key + 8 * r >= p.tk) continue;

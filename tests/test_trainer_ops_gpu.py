@@ -389,3 +389,40 @@ def test_gqa_at_the_edges_of_its_tiles(ctx, B, Tq, Tk, H, G, hd, causal, q_off):
     assert rel_l2(ds.view(B, H, Tq, Tk), pd * (dp - (pd * dp).sum(-1, keepdim=True))) <= 1e-6
     for a, b in ((dq, q.grad), (dk, k.grad), (dv, v.grad)):
         assert rel_l2(a, b) <= 1e-6
+
+
+@pytest.mark.parametrize("where,value", [("v", math.inf), ("v", -math.inf), ("k", math.inf), ("q", math.inf), ("dout", -math.inf), ("dout", math.nan)])
+@pytest.mark.parametrize("B,Tq,Tk,H,G,hd", [(2, 100, 50, 4, 2, 48), (25, 130, 130, 6, 3, 33), (1, 70, 64, 2, 2, 64)])      # on tensor cores
+def test_gqa_infinities_are_those_of_fp32(ctx, B, Tq, Tk, H, G, hd, where, value):
+    """One infinity (of a key: with queries that make its scores minus infinity): results are infinite, NaN or finite where sums in
+    fp32 are, and the finite ones as close as ever."""
+    g = torch.Generator().manual_seed(Tq + hd)
+    t = {n: torch.randn(rows, c, generator=g).double() for n, rows, c in (("q", B * Tq, H * hd), ("k", B * Tk, G * hd), ("v", B * Tk, G * hd), ("dout", B * Tq, H * hd))}
+    row, col = (B * Tk) * 2 // 3, hd + 5
+    t[where][row, col] = value
+    if where == "k":
+        t["q"].view(-1, H, hd)[:, :, 5] = -t["q"].view(-1, H, hd)[:, :, 5].abs() - 0.1
+    heads = lambda x, n, h: x.view(B, n, h, hd).permute(0, 2, 1, 3)
+    rep = lambda x: x.repeat_interleave(H // G, dim=1)
+    qh, kh, vh, gh = heads(t["q"], Tq, H), rep(heads(t["k"], Tk, G)), rep(heads(t["v"], Tk, G)), heads(t["dout"], Tq, H)
+    scale = 1.0 / math.sqrt(hd)
+    p = torch.softmax(qh @ kh.transpose(-1, -2) * scale, dim=-1)
+    dp = gh @ vh.transpose(-1, -2)
+    s = p * (dp - (p * dp).sum(-1, keepdim=True))
+    back = lambda x, n: x.permute(0, 2, 1, 3).reshape(B * n, -1)
+    group = lambda x: x.view(B, G, H // G, Tk, hd).sum(2)
+    want = {"out": back(p @ vh, Tq), "probs": p.reshape(-1), "ds": s.reshape(-1), "dq": back(s @ kh * scale, Tq),
+            "dk": back(group(s.transpose(-1, -2) @ qh * scale), Tk), "dv": back(group(p.transpose(-1, -2) @ gh), Tk)}
+    got = {n: torch.full(w.shape, 7.0, device="cuda") for n, w in want.items()}
+    if where == "q":                     # a score of plus infinity: the row of the output is NaN; its probabilities are not defined
+        want = {"out": want["out"]}
+    q, k, v, dout = (dev(t[n]) for n in ("q", "k", "v", "dout"))
+    ctx.gqa_forward(q, k, v, got["out"], B, Tq, Tk, Tk, H, G, hd, hd, False, 0, 0, scale)
+    ctx.gqa_backward(q, k, v, dout, got["probs"], got["ds"], got["dq"], got["dk"], got["dv"], B, Tq, Tk, H, G, hd, False, 0, scale)
+    torch.cuda.synchronize()
+    for n, w in want.items():
+        x = got[n].cpu().double()
+        finite = torch.isfinite(w)
+        assert torch.equal(torch.isnan(x), torch.isnan(w)) and torch.equal(x == math.inf, w == math.inf) and torch.equal(x == -math.inf, w == -math.inf), n
+        assert rel_l2(x[finite], w[finite]) <= 1e-6, n
+    assert all(not torch.isfinite(want[n]).all() for n in {"v": ("out", "dq"), "k": ("dq",), "q": ("out",), "dout": ("dv",)}[where])
