@@ -22,6 +22,8 @@ struct GemvList {
     cudaGraphNode_t node[2];               // what is recorded behind the launch depends on the last of them
     int M;
     std::vector<mcl::GemvItem> items;
+    void* ws;                              // tc: of the digits and sums
+    size_t ws_bytes;
 };
 struct GemvRecord {
     std::vector<GemvList> lists;
@@ -511,9 +513,10 @@ cudaGraphNode_t recorded_tail(mcl_cuda_ctx* ctx, unsigned long long* capture) {
     return st == cudaStreamCaptureStatusActive && n == 1 ? deps[0] : nullptr;
 }
 
-// The open list that `item` can join: the earliest one with room, behind which nothing reads or writes what the item writes, or writes
-// what it reads.  Null: none.
-GemvList* joinable(GemvRecord& rec, const mcl::GemvItem& item, int M, bool mma, bool tc) {
+// Puts `item` into the earliest open list with room, behind which nothing reads or writes what the item writes, or writes what it reads.
+// False: there is none.  The list's nodes take it when the recording is complete.
+bool join_gemvs(mcl_cuda_ctx* ctx, const mcl::GemvItem& item, int M, bool mma, bool tc) {
+    GemvRecord& rec = ctx->gemvs;
     struct Range { uintptr_t begin, end; };
     const auto range = [](const void* p, size_t bytes) { const uintptr_t b = reinterpret_cast<uintptr_t>(p); return Range{b, b + bytes}; };
     const auto meet = [](Range a, Range b) { return a.begin < b.end && b.begin < a.end; };
@@ -522,29 +525,30 @@ GemvList* joinable(GemvRecord& rec, const mcl::GemvItem& item, int M, bool mma, 
         return meet(range(i.x, (size_t)m * i.in_features * 4), r) || meet(range(i.packed2, (size_t)i.in_features / 4 * i.out_features), r) ||
                meet(range(i.scale, (size_t)i.out_features * 4), r);
     };
+    const auto room = [&](GemvList& at) {
+        if (at.M != M || at.items.size() >= mcl::kGemvListCap || !(at.tc ? tc : mma)) return false;
+        at.items.push_back(item);
+        const int n = (int)at.items.size();
+        const bool fits = at.tc ? mcl::gemv_tc_workspace_bytes(at.items.data(), n, M, ctx->sm_count) <= at.ws_bytes
+                                : mcl::gemv_mma_takes(at.items.data(), n, M, ctx->max_smem);
+        at.items.pop_back();
+        return fits;
+    };
     GemvList* found = nullptr;
-    for (size_t l = rec.lists.size(); l-- > rec.open;) {
+    size_t l = rec.lists.size();
+    for (bool met = false; l-- > rec.open && !met;) {
         GemvList& at = rec.lists[l];
         for (const mcl::GemvItem& i : at.items)
-            if (meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M))) return found;
-        if (at.M == M && at.items.size() < mcl::kGemvListCap &&
-            (at.tc ? tc : mma && mcl::gemv_mma_joins(at.items.data(), (int)at.items.size(), item.in_features))) found = &at;
+            met = met || meet(out(i, at.M), out(item, M)) || takes(i, at.M, out(item, M)) || takes(item, M, out(i, at.M));
+        if (!met && room(at)) found = &at;
     }
-    return found;
+    if (found) found->items.push_back(item);
+    return found != nullptr;
 }
 
-// The nodes of a recorded launch take its list, which has grown.
-cudaError_t join_gemv(mcl_cuda_ctx* ctx, GemvList& at) {
-    const mcl::GemvItem* items = at.items.data();
-    const int n = (int)at.items.size();
-    if (!at.tc) return mcl::launch_ternary_gemv_mma(items, n, at.M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
-    if (mcl::gemv_tc_workspace_bytes(items, n, at.M, ctx->sm_count) > ctx->ws_bytes) return cudaErrorMemoryAllocation;
-    return mcl::launch_ternary_gemv_tc(items, n, at.M, ctx->ws, 3, false, at.node, nullptr, ctx->err_word, ctx->sm_count, ctx->max_smem, ctx->stream);
-}
-
-// The recording is complete: a list of gemv_mma.cu that has become long enough for gemv_tc.cu goes there, where its context's workspace
-// is large enough or can grow (the capture has ended; what the graph already holds of the old one is kept).  Its node, on which whatever was
-// recorded behind it depends, becomes the contraction; the digits get a node in front of it.
+// The recording is complete: the nodes take their lists.  A list of gemv_mma.cu that has become long enough for gemv_tc.cu goes there,
+// where its context's workspace is large enough or can grow (the capture has ended; what the graph already holds of the old one is
+// kept).  Its node, on which whatever was recorded behind it depends, becomes the contraction; the digits get a node in front of it.
 cudaError_t lay_out_gemvs(mcl_cuda_ctx* ctx, cudaGraph_t graph) {
     std::vector<GemvList> lists;
     lists.swap(ctx->gemvs.lists);
@@ -573,12 +577,16 @@ cudaError_t lay_out_gemvs(mcl_cuda_ctx* ctx, cudaGraph_t graph) {
     }
     for (size_t l = 0; l < lists.size(); ++l) {
         const GemvList& at = lists[l];
-        if (need[l] == 0 || need[l] > at.ctx->ws_bytes) continue;
-        const cudaGraphNode_t nodes[2] = {nullptr, at.node[0]};
-        const cudaError_t e = mcl::launch_ternary_gemv_tc(at.items.data(), (int)at.items.size(), at.M, at.ctx->ws, 3, false, nodes, graph, ctx->err_word,
-                                                          ctx->sm_count, ctx->max_smem, ctx->stream);
+        const mcl::GemvItem* items = at.items.data();
+        const int n = (int)at.items.size();
+        const bool go = need[l] > 0 && need[l] <= at.ctx->ws_bytes;
+        if (!go && n == 1) continue;
+        const cudaGraphNode_t front[2] = {nullptr, at.node[0]};
+        const cudaError_t e = go || at.tc ? mcl::launch_ternary_gemv_tc(items, n, at.M, go ? at.ctx->ws : at.ws, 3, false, go ? front : at.node, graph, ctx->err_word,
+                                                                        ctx->sm_count, ctx->max_smem, ctx->stream)
+                                          : mcl::launch_ternary_gemv_mma(items, n, at.M, false, at.node, ctx->sm_count, ctx->max_smem, ctx->stream);
         if (e != cudaSuccess) return e;
-        ++ctx->launches;
+        if (go) ++ctx->launches;
     }
     return cudaSuccess;
 }
@@ -1632,14 +1640,9 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
         const cudaGraphNode_t tail = recorded_tail(ctx, &capture);
         const bool follows = tail != nullptr && tail == rec.tail && capture == rec.capture;
         if (!follows) rec.close();
-        if (GemvList* at = joinable(rec, item, (int)M, mma, tc)) {
-            at->items.push_back(item);
-            if (join_gemv(ctx, *at) == cudaSuccess) return MCL_CUDA_OK;
-            at->items.pop_back();
-            cudaGetLastError();
-        }
+        if (join_gemvs(ctx, item, (int)M, mma, tc)) return MCL_CUDA_OK;
         // up to 8 rows the workspace is taken outside captures only: what a recording makes of its lists is settled when it is complete
-        GemvList at = {ctx, !mma || (tc && !ctx->recording && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count) && !foreign_capture(ctx)), {}, (int)M, {item}};
+        GemvList at = {ctx, !mma || (tc && !ctx->recording && mcl::gemv_tc_pays(&item, 1, (int)M, ctx->sm_count) && !foreign_capture(ctx)), {}, (int)M, {item}, nullptr, 0};
         void* wsp = nullptr;
         if (at.tc) {
             // more rows than gemv_mma.cu takes: with room for the digits of further xs, which the launches of a recording may take together
@@ -1648,6 +1651,8 @@ int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* pac
             const int rc = ws_reserve(ctx, mma || need <= ctx->ws_bytes ? need : need + (size_t(16) << 20), &wsp);
             if (rc != MCL_CUDA_OK && !mma) return rc;
             if (rc != MCL_CUDA_OK) { ctx->error = error; at.tc = false; }
+            at.ws = ctx->ws;
+            at.ws_bytes = ctx->ws_bytes;
         }
         if (at.tc) {
             for (int part = 0; part < 2; ++part) {

@@ -459,10 +459,17 @@ bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_
 
 // A list's clusters are those of its shortest rows, a CTA then takes two slices of longer ones (15 matrices of 1280 and 5120, one row: 18.6 us; in clusters of
 // eight, of which short rows leave three CTAs idle, 23).
-bool gemv_mma_joins(const GemvItem* items, int n, int in_features) {
-    int low = gemv_log_slices(in_features), high = low;
-    for (int i = 0; i < n; ++i) { low = std::min(low, gemv_log_slices(items[i].in_features)); high = std::max(high, gemv_log_slices(items[i].in_features)); }
-    return high - low <= 1;
+bool gemv_mma_takes(const GemvItem* items, int n, int M, size_t max_smem) {
+    int low = 3, high = 0, chunks = 1;
+    long long groups = 0;
+    for (int i = 0; i < n; ++i) {
+        low = std::min(low, gemv_log_slices(items[i].in_features));
+        high = std::max(high, gemv_log_slices(items[i].in_features));
+        chunks = std::max(chunks, mv_chunks(items[i].in_features));
+        groups += (items[i].out_features + (long long)MV_ROWS - 1) / MV_ROWS;
+    }
+    const size_t digits = (size_t)((chunks + (1 << low) - 1) >> low) * ((M + 1) / 2) * 2048, sums = 2 * ((size_t)(M == 1 ? 2 : M) << high) * MV_ROWS * 8;
+    return high - low <= 1 && groups <= 0x3fffffff && digits + sums + 4096 <= max_smem;
 }
 
 namespace {

@@ -202,7 +202,7 @@ __device__ __forceinline__ GemvUnit gemv_unit(int e) {
 #endif
 // gemv_mma.cu -- M <= 8, one launch (one node) of integer mma.sync; clusters sized for the shortest rows of a list
 bool gemv_mma_supported(int M, int in_features, const void* packed2, size_t max_smem);
-bool gemv_mma_joins(const GemvItem* items, int n, int in_features);       // a matrix, such a list
+bool gemv_mma_takes(const GemvItem* items, int n, int M, size_t max_smem);      // as one list, each of them supported
 cudaError_t launch_ternary_gemv_mma(const GemvItem* items, int n, int M, bool follows, const cudaGraphNode_t* nodes, int sm_count,
                                     size_t max_smem, cudaStream_t stream);
 // gemv_tc.cu -- M <= 16, two launches (two nodes): digits, integer tcgen05.  parts: bit 0 the first launch, bit 1 the second; with `nodes`,
