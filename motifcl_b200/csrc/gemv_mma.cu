@@ -90,14 +90,15 @@ __device__ __forceinline__ void mv_mma(int (&c)[4], uint32_t a0, uint32_t a1, ui
 }
 __device__ __forceinline__ uint32_t mv_word(const uint4& v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
 
-// LIST: more than one matrix.  A cluster takes a run of groups, cut so that all clusters have the same number of chunks whatever the matrices are.  Matrices with
+// FORM: 1 for more than one matrix, 2 where a CTA has two slices of some.  A cluster takes a run of groups, cut so that all clusters have the same number of chunks whatever the matrices are.  Matrices with
 // one x are neighbours in the list (a segment): their digits are formed once.  The words are loaded ahead across groups, rounds
 // (a barrier) and segments (new digits) alike.
 // NT: tiles of eight digit columns (two rows of x each); R: units a warp has in registers
-template <int NT, int R, bool LIST>
-__global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_constant__ MvTable<LIST ? kGemvListCap : 1> p) {
+template <int NT, int R, int FORM>
+__global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_constant__ MvTable<FORM ? kGemvListCap : 1> p) {
+    constexpr bool LIST = FORM > 0;
     extern __shared__ __align__(128) unsigned char mv_smem[];
-    constexpr int KS = LIST ? 2 : 1;                // slices of a CTA
+    constexpr int KS = FORM == 2 ? 2 : 1;           // slices of a CTA, at most
     __shared__ unsigned int amax[KS][8];
     __shared__ int corr[KS][NT * 8];
     __shared__ double xscale[2][MV_MAX_S][8];       // of every slice: the value of one unit of its whole numbers; two segments
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
     const int s_end = segment_end(mat), I = p.m[mat].I, NC = mv_chunks(I);
     const float* const x = p.m[mat].x;
     const int c0 = (rank * NC) >> lg_s, nc = (((rank + 1) * NC) >> lg_s) - c0;
-    const int lg_k = LIST ? p.m[mat].log_k : 0, slice0 = rank << lg_k;
+    const int lg_k = KS > 1 ? p.m[mat].log_k : 0, slice0 = rank << lg_k;
     const int mid = lg_k ? (((slice0 + 1) * NC) >> (lg_s + 1)) - c0 : nc;       // chunks of the first of two slices
     if (LIST && seg > 0) {
         if (threadIdx.x < KS * 8) amax[0][threadIdx.x] = 0u;
@@ -204,14 +205,14 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
                       max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu));
         }
         top = __reduce_max_sync(0xffffffffu, top);
-        if (lane == 0) atomicMax(&amax[LIST && (unit - m * per_row) >> 1 >= mid][m], top);
+        if (lane == 0) atomicMax(&amax[KS > 1 && (unit - m * per_row) >> 1 >= mid][m], top);
     }
     __syncthreads();
 #pragma unroll 2
     for (int unit = warp; unit < Mp * per_row; unit += MV_WARPS) {
         const int mp = unit / per_row, quad = (unit - mp * per_row) * 32 + lane, k = k0 + quad * 4;
         const int m = M == 1 ? 0 : mp;
-        const int sl = LIST && (unit - mp * per_row) >> 1 >= mid;
+        const int sl = KS > 1 && (unit - mp * per_row) >> 1 >= mid;
         const unsigned int top = amax[sl][m];
         const GemvUnit inv = gemv_unit(top >= 0x7F800000u ? 0 : gemv_exponent(top));
         const float4 t = k < I ? mv_load_x(x + (size_t)m * I + k) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -295,9 +296,9 @@ __global__ void __launch_bounds__(MV_THREADS, 2) gemv_mma_kernel(const __grid_co
                     }
                     load(w[j]);
                     ++cc;
-                    if (cc == nc || (LIST && cc == mid)) {
+                    if (cc == nc || (KS > 1 && cc == mid)) {
                         // a slice of this group is complete: its sums, two digits to a word, go to the CTA that finishes the group
-                        const int li = grp - gb, sl = LIST && cc > mid;
+                        const int li = grp - gb, sl = KS > 1 && cc > mid;
                         uint32_t dst;
                         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
                                      : "r"(part0 + part + (slice0 + sl) * part_bytes + (uint32_t)((li >> lg_s) * Mp) * (MV_ROWS * 8u)), "r"(li & (S - 1)));
@@ -416,8 +417,10 @@ cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, 
     p.block = p.owned * S;
     const size_t smem = p.xq_bytes + bufs * p.owned * group_bytes;
     if (smem > max_smem - 4096) return cudaErrorInvalidConfiguration;
-    const void* kern = reinterpret_cast<const void*>(gemv_mma_kernel<NT, R, LIST>);
-    cudaError_t e = ensure_dynamic_smem(kern, LIST ? slot + 10 : slot, max_smem);
+    const bool two = LIST && p.log_p > p.log_s;
+    void (*const kernel)(MvTable<CAP>) = two ? gemv_mma_kernel<NT, R, 2 * LIST> : gemv_mma_kernel<NT, R, LIST>;
+    const void* kern = reinterpret_cast<const void*>(kernel);
+    cudaError_t e = ensure_dynamic_smem(kern, two ? slot + 32 : LIST ? slot + 10 : slot, max_smem);
     if (e != cudaSuccess) return e;
     if (nodes) {
         void* args[] = {&p};
@@ -438,7 +441,7 @@ cudaError_t mv_launch(MvTable<CAP>& p, int sm_count, size_t max_smem, int slot, 
     if (S > 1) { at[n].id = cudaLaunchAttributeClusterDimension; at[n].val.clusterDim.x = S; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1; ++n; }
     if (follows) { at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[n].val.programmaticStreamSerializationAllowed = 1; ++n; }
     cfg.attrs = at; cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, gemv_mma_kernel<NT, R, LIST>, p);
+    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
 }  // namespace
