@@ -56,6 +56,7 @@ struct GvTable {
     int n, xs, tiles, M, Nq, stages;
     int extra;         // first row of fifth digits
     int cut_q, cut_r;  // units / CTAs, and what is over
+    int share;         // more than 1: one matrix of more than 8 rows, whose tiles a cluster of so many CTAs has each, and one RT
     int* err;
     int* acc;          // slots of [RT][Nq][128] sums for tiles that a cut runs through, by tile or by the CTA that begins it, whichever are fewer
     double* part;      // an x in slices: [CTA][not begun or begun][slice][row][RT * 128] sums of the tile at hand
@@ -134,6 +135,11 @@ __device__ __forceinline__ int gv_cut(const GvTable& p, int cta) { return p.cut_
 __device__ __forceinline__ int gv_first_cta(const GvTable& p, int cta, int begin) { while (gv_cut(p, cta) > begin) --cta; return cta; }
 __device__ __forceinline__ int gv_last_cta(const GvTable& p, int cta, int end) { while (gv_cut(p, cta + 1) < end) ++cta; return cta; }
 
+// all threads of a cluster; what was written to shared memory before can be read behind it
+__device__ __forceinline__ void gv_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __host__ __device__ inline int gv_rows(int M) { return M == 1 ? 2 : M; }        // rows of whole numbers
 // the xs to be taken in slices; a whole warp, after the wait for the launch before
 __device__ __forceinline__ uint32_t gv_wide(const GvTable& p) {
@@ -153,6 +159,7 @@ __device__ __forceinline__ uint32_t gv_wide(const GvTable& p) {
 template <int RT, int ROWS>
 __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid_constant__ GvTable p) {
     constexpr int EXP = (GV_TMEM - 64 * RT) / GV_ACOLS;        // expanded tiles in flight in tensor memory
+    const bool shared = RT == 1 && ROWS == 0 && p.share > 1;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * EXP + 2 * RT];
     __shared__ uint32_t tmem_slot;
@@ -388,6 +395,11 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                                                                    (first ? x_sums[16 * t.slice + 4 * c + j] : 0ll));
                     } else if (whole) {
                         finish(A, row, c, v, fifth);
+                    } else if (shared) {                     // the CTA's one part: the slots of the ring are free
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)(((4 * c + j) * GV_ROWS + lrow) * 16)),
+                                         "r"(v[4 * j]), "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3]) : "memory");
                     } else if (row < A.O) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -398,7 +410,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty(h));
             }
-            if ((whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
+            if (shared || (whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
             if (!whole) {                 // the last of the CTAs that share the tile finishes it
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -447,8 +459,31 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 }
             }
         }
+        if (shared) {
+            // every CTA finishes some rows of x: it adds up their digits' sums over the cluster
+            gv_cluster_sync();
+            const int rank = (int)(blockIdx.x % p.share), row = (int)(blockIdx.x / p.share) * GV_ROWS + lrow;
+            if (ok && row < p.m[0].O) {
+                const double sc = (double)p.m[0].scale[row];
+                for (int m = rank; m < M; m += p.share) {
+                    int d[4] = {};
+#pragma unroll 4
+                    for (int k = 0; k < p.share; ++k) {
+                        uint32_t from;
+                        int v[4];
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(base + (uint32_t)((m * GV_ROWS + lrow) * 16)), "r"(k));
+                        asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(from) : "memory");
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) d[i] += v[i];
+                    }
+                    p.m[0].y[(size_t)m * p.m[0].O + row] = (float)(sc * (x_units[m] * (double)(number(d[0], d[1], d[2], d[3]) - x_sums[m])));
+                }
+            }
+            gv_cluster_sync();             // before this CTA's shared memory goes
+        }
     }
     __syncwarp();
+    if (shared && warp < 2 + 4 * RT) { gv_cluster_sync(); gv_cluster_sync(); }
     if (abort_flag) {
         const unsigned long long t0 = clock64();
         while (clock64() - t0 < 2000000ull) {}
@@ -600,10 +635,15 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
     if (tid < 4) isum[tid] = 0;
     __syncthreads();
     unsigned int top = 0u;
-    for (int i = tid; i < I / 4; i += GQ_THREADS) {
-        const float4 v = gv_load_x(x + i);
-        top = max(max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), max(__float_as_uint(v.y) & 0x7FFFFFFFu, __float_as_uint(v.z) & 0x7FFFFFFFu)),
-                  __float_as_uint(v.w) & 0x7FFFFFFFu);
+    float4 own[4];                 // this thread's first group of 16, all there are up to 8192
+    for (int g = tid; g < pitch; g += GQ_THREADS) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = gv_load_x(x + 4 * g + j);
+            if (g == tid) own[j] = v;
+            top = max(max(max(top, __float_as_uint(v.x) & 0x7FFFFFFFu), max(__float_as_uint(v.y) & 0x7FFFFFFFu, __float_as_uint(v.z) & 0x7FFFFFFFu)),
+                      __float_as_uint(v.w) & 0x7FFFFFFFu);
+        }
     }
     top = __reduce_max_sync(0xffffffffu, top);
     if ((tid & 31) == 0) atomicMax(&top_s, top);
@@ -616,7 +656,7 @@ __global__ void __launch_bounds__(GQ_THREADS) gemv_quantize_kernel(const __grid_
         uint32_t r[16];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float4 v = gv_load_x(x + 4 * g + j);
+            const float4 v = g == tid ? own[j] : gv_load_x(x + 4 * g + j);
             const float f[4] = {v.x * inv.a * inv.b, v.y * inv.a * inv.b, v.z * inv.a * inv.b, v.w * inv.a * inv.b};
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
@@ -694,7 +734,7 @@ bool gemv_tc_supported(int M, int in_features, const void* packed2) {
 }
 
 namespace {
-struct GvPlan { int RT, ctas; long long units, tiles; size_t slots, slices; };      // bytes for tiles that a cut runs through
+struct GvPlan { int RT, ctas, share; long long units, tiles; size_t slots, slices; };      // bytes for tiles that a cut runs through
 GvPlan gv_plan(const GemvItem* items, int n, int M, int sm_count) {
     GvPlan g;
     // Two CTAs on every SM and tiles of 256 rows, or one and 128.  One row: 2100 k-blocks 22.6 and 20.8 us, 5760 26.8 and 35.0, 25600 60 and 118; 16
@@ -708,11 +748,15 @@ GvPlan gv_plan(const GemvItem* items, int n, int M, int sm_count) {
         g.units += of * ((items[i].in_features + GV_KB - 1) / GV_KB);
     }
     // One matrix of few tiles: no CTA has parts of two (4096 x 4096, 16 rows: 16.2 -> 13.1 us), and a tile is cut only where that saves more
-    // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).
+    // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).  Up to 8 CTAs are a cluster
+    // then and read one another's sums (more than 8 rows; fewer seldom come here): atomics, a fence and a ticket cost 2 us more (4096 x 4096
+    // in a chain, 9 rows: 12.0 -> 10.9 us, 16: 13.6 -> 11.8).
     int per = g.RT * sm_count;
+    g.share = 1;
     if (n == 1 && g.tiles <= sm_count) {
         const int kbs = (items[0].in_features + GV_KB - 1) / GV_KB, cut = std::max(1, std::min(kbs / 2, (int)(sm_count / g.tiles)));
         per = (int)g.tiles * (kbs - kbs / cut > 6 ? cut : 1);
+        if (M > 8 && g.RT == 1 && per <= 8 * g.tiles) g.share = per / (int)g.tiles;
     }
     g.ctas = (int)std::min<long long>(per, g.units);
     g.slots = (size_t)std::min<long long>(g.ctas, g.tiles) * g.RT * gv_nq(M) * GV_ROWS * sizeof(int);
@@ -751,8 +795,7 @@ bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count) {
 }
 
 namespace {
-// A kernel node between `node` and what it depended on: `node` comes right behind it, overlapping at the seam.  It is a single kernel
-// afterwards (no clusters).
+// A kernel node between `node` and what it depended on: `node` comes right behind it, overlapping at the seam.
 cudaError_t put_before(cudaGraph_t graph, cudaGraphNode_t node, const cudaKernelNodeParams& kp) {
     size_t n = 0;
     cudaError_t e = cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &n);
@@ -772,11 +815,7 @@ cudaError_t put_before(cudaGraph_t graph, cudaGraphNode_t node, const cudaKernel
     cudaGraphEdgeData seam = {};
     seam.from_port = cudaGraphKernelNodePortProgrammatic;
     seam.type = cudaGraphDependencyTypeProgrammatic;
-    e = cudaGraphAddDependencies_v2(graph, &made, &node, &seam, 1);
-    if (e != cudaSuccess) return e;
-    cudaKernelNodeAttrValue at = {};
-    at.clusterDim.x = at.clusterDim.y = at.clusterDim.z = 1;
-    return cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeClusterDimension, &at);
+    return cudaGraphAddDependencies_v2(graph, &made, &node, &seam, 1);
 }
 }  // namespace
 
@@ -792,6 +831,7 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     p.n = n; p.M = M; p.Nq = Nq; p.err = err_word; p.extra = gv_extra(M);
     p.cut_q = (int)(plan.units / ctas); p.cut_r = (int)(plan.units % ctas);
     p.tiles = (int)plan.tiles;
+    p.share = plan.share;
     g.wide = reinterpret_cast<int*>(w);
     p.wide = g.wide;
     w += 1024;
@@ -842,7 +882,7 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     const size_t smem = p.stages * stage_bytes + 1024;
     // the tickets stand before the slots: one range
     g.clear = reinterpret_cast<int4*>(p.tickets);
-    g.clear_n = (round_up(2 * sm_count * sizeof(int)) + plan.slots) / 16;
+    g.clear_n = plan.share > 1 ? 0 : (round_up(2 * sm_count * sizeof(int)) + plan.slots) / 16;
     const int q_blocks = g.first[g.n] + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS));
 
     // by rows (up to 4, up to 8, more) and RT
@@ -856,9 +896,11 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     cudaKernelNodeParams kp = {};
     cudaLaunchConfig_t cfg = {};
     cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization; at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = plan.share; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
     if (parts & 1) {
         void* args[] = {&g};
         void (*const digits)(GqTable) = M <= 8 ? gemv_quantize_slices_kernel : gemv_quantize_kernel;
@@ -875,9 +917,15 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
         kp.gridDim = cfg.gridDim = dim3(ctas); kp.blockDim = cfg.blockDim = dim3(192 + 128 * RT);
         kp.sharedMemBytes = (unsigned)smem; cfg.dynamicSmemBytes = smem;
         kp.kernelParams = args;
-        cfg.numAttrs = 1;
-        e = nodes ? cudaGraphKernelNodeSetParams(nodes[1], &kp)
-                  : cudaLaunchKernelEx(&cfg, kernel, p);
+        cfg.numAttrs = plan.share > 1 ? 2 : 1;
+        if (nodes) {
+            cudaKernelNodeAttrValue cluster = {};
+            cluster.clusterDim = at[1].val.clusterDim;
+            e = cudaGraphKernelNodeSetAttribute(nodes[1], cudaLaunchAttributeClusterDimension, &cluster);      // a list that has grown has none
+            if (e == cudaSuccess) e = cudaGraphKernelNodeSetParams(nodes[1], &kp);
+        } else {
+            e = cudaLaunchKernelEx(&cfg, kernel, p);
+        }
     }
     return e;
 }

@@ -290,3 +290,75 @@ def test_a_large_activation_that_no_weight_takes_leaves_the_other_slices(M, O, I
         for (_, digits, scale), (_, _, y) in zip(mats, args):
             want = x.astype(np.float64) @ digits.T * scale.astype(np.float64)
             assert np.linalg.norm(y.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("M", [1, 2, 8, 12, 16])
+def test_lists_that_fill_the_gpu_with_tiles_of_two_accumulators(M):
+    """10752 k-blocks: tiles of 256 rows, two CTAs on every SM, whatever the number of rows; ragged matrices, two xs, one of them (up to 8
+    rows) in slices.  Two launches, against float64 and, bit for bit, against single calls, which up to 2 rows run on the other kernel."""
+    rng = np.random.default_rng(M)
+    shapes = [(14300, 4096), (4096, 14336), (13999, 4096), (4001, 14336), (14336, 4096), (14081, 4096)]
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        g = torch.Generator(device=DEV).manual_seed(M)
+        xs = {I: torch.randn(M, I, device=DEV, generator=g) for I in (4096, 14336)}
+        xs[14336] *= 2.0 ** -(torch.arange(14336, device=DEV) * 3 // 14336 * 6).float()
+        mats = [(torch.randint(-2 ** 31, 2 ** 31 - 1, (O, I // 16), dtype=torch.int32, device=DEV, generator=g),
+                 torch.rand(O, device=DEV, generator=g) + 0.1) for O, I in shapes]
+        ys, single = [[torch.full((M, O), 5.0, device=DEV) for O, _ in shapes] for _ in range(2)]
+
+        def sweep(out):
+            for (O, I), (w, s), y in zip(shapes, mats, out):
+                ctx.ternary_gemv(xs[I], w, s, y, M, I, O)
+        sweep(single)
+        ctx.finish()
+        before = ctx.launch_count
+        ctx.batch_begin()
+        sweep(ys)
+        batch = ctx.batch_end()
+        batch.launch()
+        ctx.finish()
+        assert ctx.launch_count - before == 2
+        batch.close()
+        for (O, I), (w, s), y, one in zip(shapes, mats, ys, single):
+            assert torch.equal(y, one)
+            digits = torch.stack([((w >> (2 * k)) & 3).double() - 1.0 for k in range(16)], dim=2).view(O, I)
+            want = (xs[I].double() @ digits.T) * s.double()
+            for m in range(M):
+                assert float((y[m] - want[m]).norm() / want[m].norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("M", [9, 13, 16])
+@pytest.mark.parametrize("O,I", [(4096, 4096), (4001, 14336), (130, 4160), (2000, 6144), (1024, 14336), (257, 2048), (14336, 4096)])
+def test_one_matrix_whose_tiles_are_cut(M, O, I):
+    """More than 8 rows: sums of a tile over a cluster of 2 to 8 CTAs or, where more share it, over the workspace; alone, as a chain of recorded
+    launches, and as the first of a list that has grown."""
+    rng = np.random.default_rng(O + I + M)
+    w, digits, scale = _matrix(rng, O, I)
+    x = rng.standard_normal((M, I)).astype(np.float32)
+    want = x.astype(np.float64) @ digits.T * scale.astype(np.float64)
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        dx, s = torch.from_numpy(x).to(DEV), torch.from_numpy(scale).to(DEV)
+        one, chain, first, second = [torch.full((M, O), 5.0, device=DEV) for _ in range(4)]
+        ctx.ternary_gemv(dx, w, s, one, M, I, O)
+        ctx.finish()
+        before = ctx.launch_count
+        ctx.batch_begin()
+        for _ in range(3):
+            ctx.ternary_gemv(dx, w, s, chain, M, I, O)           # overwrites its own result: launches of their own
+        batch = ctx.batch_end()
+        ctx.batch_begin()
+        ctx.ternary_gemv(dx, w, s, first, M, I, O)
+        ctx.ternary_gemv(dx, w, s, second, M, I, O)
+        pair = ctx.batch_end()
+        for _ in range(2):
+            batch.launch()
+            pair.launch()
+        ctx.finish()
+        assert ctx.launch_count - before == 2 * (6 + 2)
+        batch.close()
+        pair.close()
+        assert np.linalg.norm(one.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
+        for y in (chain, first, second):
+            assert torch.equal(y, one)
