@@ -58,7 +58,7 @@ def test_row_sums_that_leave_fp32_are_infinities(ctx, N, I, O):
     ctx.counter_forward(x, st, sc, y, N, I, O, 11)
     ctx.counter_backward_input(st, sc, dy, dx, N, I, O, 11)
     ctx.finish()
-    many = w.double().square().sum(dim=1)[:n] * 1e37 > 1e39
+    many = w.double().square().sum(dim=1)[:n] * 1e37 > 5e38
     assert bool(many.any()) and bool((y.diagonal()[:n][many] == float("inf")).all())
     far = (sc.double() @ w.double().square())[:k] * 1e38 > 1e39
     assert bool(far.any()) and bool((dx.diagonal()[:k][far] == float("inf")).all())
