@@ -56,7 +56,7 @@ struct GvTable {
     int n, xs, tiles, M, Nq, stages;
     int extra;         // first row of fifth digits
     int cut_q, cut_r;  // units / CTAs, and what is over
-    int share;         // more than 1: one matrix of more than 8 rows, whose tiles a cluster of so many CTAs has each, and one RT
+    int share;         // CTAs of a cluster
     int* err;
     int* acc;          // slots of [RT][Nq][128] sums for tiles that a cut runs through, by tile or by the CTA that begins it, whichever are fewer
     double* part;      // an x in slices: [CTA][not begun or begun][slice][row][RT * 128] sums of the tile at hand
@@ -156,16 +156,15 @@ __device__ __forceinline__ uint32_t gv_wide(const GvTable& p) {
 
 // RT: accumulators (128 rows each) of a tile, which share the digits that a k-block loads
 // ROWS: 4 or 8, for up to so many rows of x; 0 for more, which have one unit for the whole of K and four digits
-template <int RT, int ROWS>
+// SHARED: one matrix whose tiles a cluster of p.share CTAs has each (RT = 1)
+template <int RT, int ROWS, bool SHARED>
 __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid_constant__ GvTable p) {
     constexpr int EXP = (GV_TMEM - 64 * RT) / GV_ACOLS;        // expanded tiles in flight in tensor memory
-    const bool shared = RT == 1 && ROWS == 0 && p.share > 1;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * GV_MAX_STAGES + 2 * EXP + 2 * RT];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag, last_ticket;
-    __shared__ long long x_sums[8 * 16];   // of the x at hand: of a slice, or of the whole of K
-    __shared__ double x_units[8 * 16];
+    __shared__ struct alignas(16) { long long sum; double unit; } x_of[8 * 16];       // of the x at hand: of a slice, or of the whole of K
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = p.stages, Nq = p.Nq;
@@ -316,10 +315,13 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         const size_t pitch = RT * GV_ROWS;
         auto slice_sums = [&](int cta, bool begun, int slice) { return p.part + (size_t)(((cta * 2 + begun) * 8 + slice) * rows) * pitch; };
         auto number = [](int a, int b, int c, int d) { return ((long long)a * 256 + b) * 65536 + ((long long)c * 256 + d); };
+        // of an output row, loaded under the wait for its sums; late where that would spill (8 rows of x, two accumulators)
+        constexpr bool EARLY = ROWS < 8 || RT == 1;
+        auto scale_of = [&](const GvMat& A, int row) { return row < A.O ? (double)load_behind(A.scale + row) : 0.0; };
         // four rows of x, from row 4 c on, of an output row
-        auto write = [&](const GvMat& A, int row, int c, const double (&v)[4]) {
+        auto write = [&](const GvMat& A, int row, int c, double sc, const double (&v)[4]) {
             if (row >= A.O) return;
-            const double sc = (double)A.scale[row];
+            if (!EARLY) sc = scale_of(A, row);
             if (M == 1) {
                 A.y[row] = (float)(sc * (v[0] + v[1] * (1.0 / 1073741824.0)));
             } else {
@@ -328,15 +330,15 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                     if (4 * c + j < M) A.y[(size_t)(4 * c + j) * A.O + row] = (float)(sc * v[j]);
             }
         };
-        auto finish = [&](const GvMat& A, int row, int c, const uint32_t* v, const int* fifth) {
+        auto finish = [&](const GvMat& A, int row, int c, double sc, const uint32_t* v, const int* fifth) {
             double n[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int r = 4 * c + j < rows ? 4 * c + j : 0;
-                n[j] = x_units[r] * (double)(number((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]) +
-                                             (ROWS ? (long long)fifth[j] * 4294967296ll : 0ll) - x_sums[r]);
+                const auto x = x_of[4 * c + j];                    // beyond the rows there are: zeros
+                n[j] = x.unit * (double)(number((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]) +
+                                         (ROWS ? (long long)fifth[j] * 4294967296ll : 0ll) - x.sum);
             }
-            write(A, row, c, n);
+            write(A, row, c, sc, n);
         };
         int n_local = 0, x = -1;
         bool ok = true, begun = false;
@@ -353,8 +355,8 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 long long sum = in ? A.sums[i] : 0ll;
                 if (in && !sliced && i < 16)
                     for (int k = 1; k < 1 << A.log_s; ++k) sum += A.sums[16 * k + i];
-                x_sums[i] = sum;
-                x_units[i] = in ? A.units[i] : 0.0;
+                x_of[i].sum = sum;
+                x_of[i].unit = in ? A.units[i] : 0.0;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
             const bool whole = begun && t.kb0 + t.nkb == t.kbs;          // with this part all of the tile has been here
@@ -363,12 +365,13 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
             int* slot = p.acc + (size_t)slot_i * (RT * Nq * GV_ROWS);
 #pragma unroll 1
             for (int h = 0; h < RT && ok; ++h) {
+                const int row = (t.tile * RT + h) * GV_ROWS + lrow;
+                const double sc = EARLY && whole ? scale_of(A, row) : 0.0;
                 ok = !abort_flag;
                 if (ok && !mbar_wait(acc_full(h), n_local & 1, &abort_flag)) { abort_flag = 1; atomicExch(p.err, 15); ok = false; }
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                const int row = (t.tile * RT + h) * GV_ROWS + lrow;
 #pragma unroll
                 for (int c = 0; c < (ROWS ? ROWS / 4 : 4); ++c) {
                     if (!ROWS && c == chunks) break;
@@ -380,7 +383,11 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             fifth[j] = (int)((p.extra & 15) ? v[16 - ROWS + 4 * c + j] : v[4 * c + j]);
-                            if (!whole && row < A.O && 4 * c + j < rows) atomicAdd(slot + (h * Nq + p.extra + 4 * c + j) * GV_ROWS + lrow, fifth[j]);
+                            if (SHARED) {
+                                if (4 * c + j < rows) asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + (uint32_t)((rows * 16 + (4 * c + j) * 4) * GV_ROWS + lrow * 4)), "r"(fifth[j]) : "memory");
+                            } else if (!whole && row < A.O && 4 * c + j < rows) {
+                                atomicAdd(slot + (h * Nq + p.extra + 4 * c + j) * GV_ROWS + lrow, fifth[j]);
+                            }
                         }
                     }
                     tmem_ld16(tmem + 64 * h + 16 * c, v);
@@ -392,13 +399,13 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                         for (int j = 0; j < 4; ++j)
                             if (4 * c + j < rows)
                                 to[(4 * c + j) * pitch] = (double)(number((int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]) -
-                                                                   (first ? x_sums[16 * t.slice + 4 * c + j] : 0ll));
+                                                                   (first ? x_of[16 * t.slice + 4 * c + j].sum : 0ll));
                     } else if (whole) {
-                        finish(A, row, c, v, fifth);
-                    } else if (shared) {                     // the CTA's one part: the slots of the ring are free
+                        finish(A, row, c, sc, v, fifth);
+                    } else if (SHARED) {                     // the CTA's one part: the slots of the ring are free
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)(((4 * c + j) * GV_ROWS + lrow) * 16)),
+                            if (4 * c + j < rows) asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(base + (uint32_t)(((4 * c + j) * GV_ROWS + lrow) * 16)),
                                          "r"(v[4 * j]), "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3]) : "memory");
                     } else if (row < A.O) {
 #pragma unroll
@@ -410,7 +417,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty(h));
             }
-            if (shared || (whole && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
+            if (((SHARED || whole) && !sliced) || (t.kb0 + t.nkb != t.kbs && t.u != u_end)) continue;
             if (!whole) {                 // the last of the CTAs that share the tile finishes it
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -422,6 +429,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
 #pragma unroll 1
             for (int h = 0; h < RT && ok; ++h) {
                 const int row = (t.tile * RT + h) * GV_ROWS + lrow;
+                const double sc = EARLY ? scale_of(A, row) : 0.0;
                 if (sliced) {
 #pragma unroll 1
                     for (int c = 0; c < chunks; ++c) {
@@ -438,13 +446,13 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                                 if (gv_cut(p, i + 1) - tile_u >= k1) break;
                             }
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) total[j] += x_units[16 * slice + (4 * c + j < rows ? 4 * c + j : 0)] * n[j];
+                            for (int j = 0; j < 4; ++j) total[j] += x_of[16 * slice + 4 * c + j].unit * n[j];
                         }
-                        write(A, row, c, total);
+                        write(A, row, c, sc, total);
                     }
                     continue;
                 }
-                constexpr int AT_ONCE = ROWS ? 1 : 2;                   // of the widest list, half in flight
+                constexpr int AT_ONCE = ROWS || RT == 2 ? 1 : 2;         // of the widest list, half in flight where registers allow
 #pragma unroll
                 for (int c = 0; c < (ROWS ? ROWS / 4 : 4); c += AT_ONCE) {
                     if (!ROWS && c >= chunks) break;
@@ -454,36 +462,46 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
                     for (int j = 0; j < 4 && ROWS; ++j) fifth[j] = 4 * c + j < rows ? __ldcg(slot + (h * Nq + p.extra + 4 * c + j) * GV_ROWS + lrow) : 0;
 #pragma unroll
                     for (int j = 0; j < 16 * AT_ONCE; ++j) v[j] = 16 * c + j < 4 * rows ? (uint32_t)__ldcg(slot + (h * Nq + c * 16 + j) * GV_ROWS + lrow) : 0u;
-                    finish(A, row, c, v, fifth);
-                    if (AT_ONCE == 2 && c + 1 < chunks) finish(A, row, c + 1, v + 16 * (AT_ONCE - 1), fifth);
+                    finish(A, row, c, sc, v, fifth);
+                    if (AT_ONCE == 2 && c + 1 < chunks) finish(A, row, c + 1, sc, v + 16 * (AT_ONCE - 1), fifth);
                 }
             }
         }
-        if (shared) {
+        if (SHARED) {
             // every CTA finishes some rows of x: it adds up their digits' sums over the cluster
-            gv_cluster_sync();
+            const GvMat& A = p.m[0];
             const int rank = (int)(blockIdx.x % p.share), row = (int)(blockIdx.x / p.share) * GV_ROWS + lrow;
-            if (ok && row < p.m[0].O) {
-                const double sc = (double)p.m[0].scale[row];
-                for (int m = rank; m < M; m += p.share) {
-                    int d[4] = {};
+            const bool in = ok && row < A.O && !(wide & 1u);
+            const double sc = in ? scale_of(A, row) : 0.0;
+            auto sum = [&](int m) {
+                int d[5] = {};
 #pragma unroll 4
-                    for (int k = 0; k < p.share; ++k) {
-                        uint32_t from;
-                        int v[4];
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(base + (uint32_t)((m * GV_ROWS + lrow) * 16)), "r"(k));
-                        asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(from) : "memory");
+                for (int k = 0; k < p.share; ++k) {
+                    uint32_t from;
+                    int v[4];
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(base), "r"(k));
+                    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                                 : "r"(from + (uint32_t)((m * GV_ROWS + lrow) * 16)) : "memory");
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) d[i] += v[i];
+                    for (int i = 0; i < 4; ++i) d[i] += v[i];
+                    if (ROWS) {
+                        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v[0]) : "r"(from + (uint32_t)((rows * 16 + m * 4) * GV_ROWS + lrow * 4)) : "memory");
+                        d[4] += v[0];
                     }
-                    p.m[0].y[(size_t)m * p.m[0].O + row] = (float)(sc * (x_units[m] * (double)(number(d[0], d[1], d[2], d[3]) - x_sums[m])));
                 }
+                return x_of[m].unit * (double)(number(d[0], d[1], d[2], d[3]) + (ROWS ? (long long)d[4] * 4294967296ll : 0ll) - x_of[m].sum);
+            };
+            gv_cluster_sync();
+            if (in && M == 1) {
+                if (rank == 0) A.y[row] = (float)(sc * (sum(0) + sum(1) * (1.0 / 1073741824.0)));
+            } else if (in) {
+                for (int m = rank; m < M; m += p.share) A.y[(size_t)m * A.O + row] = (float)(sc * sum(m));
             }
             gv_cluster_sync();             // before this CTA's shared memory goes
         }
     }
     __syncwarp();
-    if (shared && warp < 2 + 4 * RT) { gv_cluster_sync(); gv_cluster_sync(); }
+    if (SHARED && warp < 2 + 4 * RT) { gv_cluster_sync(); gv_cluster_sync(); }
     if (abort_flag) {
         const unsigned long long t0 = clock64();
         while (clock64() - t0 < 2000000ull) {}
@@ -749,14 +767,14 @@ GvPlan gv_plan(const GemvItem* items, int n, int M, int sm_count) {
     }
     // One matrix of few tiles: no CTA has parts of two (4096 x 4096, 16 rows: 16.2 -> 13.1 us), and a tile is cut only where that saves more
     // than adding up its parts costs (six k-blocks, about 4 us; 1024 -> 4096 and back: 11.2 -> 10.1 us a matrix).  Up to 8 CTAs are a cluster
-    // then and read one another's sums (more than 8 rows; fewer seldom come here): atomics, a fence and a ticket cost 2 us more (4096 x 4096
+    // then and read one another's sums: atomics, a fence and a ticket cost 2 us more (4096 x 4096
     // in a chain, 9 rows: 12.0 -> 10.9 us, 16: 13.6 -> 11.8).
     int per = g.RT * sm_count;
     g.share = 1;
     if (n == 1 && g.tiles <= sm_count) {
         const int kbs = (items[0].in_features + GV_KB - 1) / GV_KB, cut = std::max(1, std::min(kbs / 2, (int)(sm_count / g.tiles)));
         per = (int)g.tiles * (kbs - kbs / cut > 6 ? cut : 1);
-        if (M > 8 && g.RT == 1 && per <= 8 * g.tiles) g.share = per / (int)g.tiles;
+        if (g.RT == 1 && per <= 8 * g.tiles) g.share = per / (int)g.tiles;
     }
     g.ctas = (int)std::min<long long>(per, g.units);
     g.slots = (size_t)std::min<long long>(g.ctas, g.tiles) * g.RT * gv_nq(M) * GV_ROWS * sizeof(int);
@@ -882,16 +900,17 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
     const size_t smem = p.stages * stage_bytes + 1024;
     // the tickets stand before the slots: one range
     g.clear = reinterpret_cast<int4*>(p.tickets);
-    g.clear_n = plan.share > 1 ? 0 : (round_up(2 * sm_count * sizeof(int)) + plan.slots) / 16;
+    g.clear_n = (round_up(2 * sm_count * sizeof(int)) + (plan.share > 1 ? 0 : plan.slots)) / 16;
     const int q_blocks = g.first[g.n] + (int)std::min<size_t>(sm_count, (g.clear_n + 4 * GQ_THREADS - 1) / (4 * GQ_THREADS));
 
-    // by rows (up to 4, up to 8, more) and RT
-    static void (*const kernels[3][2])(GvTable) = {{gemv_tc_kernel<1, 4>, gemv_tc_kernel<2, 4>}, {gemv_tc_kernel<1, 8>, gemv_tc_kernel<2, 8>},
-                                                   {gemv_tc_kernel<1, 0>, gemv_tc_kernel<2, 0>}};
-    const int rows = M <= 4 ? 0 : M <= 8 ? 1 : 2;
-    void (*const kernel)(GvTable) = kernels[rows][RT - 1];
+    // by rows (up to 4, up to 8, more); one accumulator, the same with clusters, two accumulators
+    static void (*const kernels[3][3])(GvTable) = {{gemv_tc_kernel<1, 4, false>, gemv_tc_kernel<1, 4, true>, gemv_tc_kernel<2, 4, false>},
+                                                   {gemv_tc_kernel<1, 8, false>, gemv_tc_kernel<1, 8, true>, gemv_tc_kernel<2, 8, false>},
+                                                   {gemv_tc_kernel<1, 0, false>, gemv_tc_kernel<1, 0, true>, gemv_tc_kernel<2, 0, false>}};
+    const int rows = M <= 4 ? 0 : M <= 8 ? 1 : 2, form = RT == 2 ? 2 : plan.share > 1 ? 1 : 0;
+    void (*const kernel)(GvTable) = kernels[rows][form];
     const void* kern = reinterpret_cast<const void*>(kernel);
-    cudaError_t e = ensure_dynamic_smem(kern, 52 + 2 * rows + RT - 1, max_smem);
+    cudaError_t e = ensure_dynamic_smem(kern, (form == 1 ? 62 : 52 + form / 2) + (form == 1 ? rows : 2 * rows), max_smem);
     if (e != cudaSuccess) return e;
     cudaKernelNodeParams kp = {};
     cudaLaunchConfig_t cfg = {};
@@ -920,9 +939,11 @@ cudaError_t launch_ternary_gemv_tc(const GemvItem* items, int n, int M, void* wo
         cfg.numAttrs = plan.share > 1 ? 2 : 1;
         if (nodes) {
             cudaKernelNodeAttrValue cluster = {};
-            cluster.clusterDim = at[1].val.clusterDim;
-            e = cudaGraphKernelNodeSetAttribute(nodes[1], cudaLaunchAttributeClusterDimension, &cluster);      // a list that has grown has none
+            cluster.clusterDim.x = cluster.clusterDim.y = cluster.clusterDim.z = 1;        // the clusters of what the node was go first
+            e = cudaGraphKernelNodeSetAttribute(nodes[1], cudaLaunchAttributeClusterDimension, &cluster);
             if (e == cudaSuccess) e = cudaGraphKernelNodeSetParams(nodes[1], &kp);
+            cluster.clusterDim.x = plan.share;
+            if (e == cudaSuccess && plan.share > 1) e = cudaGraphKernelNodeSetAttribute(nodes[1], cudaLaunchAttributeClusterDimension, &cluster);
         } else {
             e = cudaLaunchKernelEx(&cfg, kernel, p);
         }
