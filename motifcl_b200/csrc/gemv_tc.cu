@@ -800,16 +800,19 @@ size_t gemv_tc_workspace_bytes(const GemvItem* items, int n, int M, int sm_count
     return xs <= kGemvXCap && gv_blocks(items, n) <= 0x3fffffff ? bytes : ~size_t(0);
 }
 
-// Against gemv_mma.cu (M <= 8), by k-blocks: that one needs no second launch and starts 5 us earlier, this one takes eight rows as fast as one and
-// many xs as fast as few, which there are a round and new digits each.  us as gemv_mma / gemv_tc, alone.  Three xs and more: M = 1 2624 k-blocks
-// 18.9 / 22.7, 2800 21.4 / 25.0, 3936 37 / 23; M = 4 1400 18.6 / 18.6, 2624 31 / 23 (17.3 / 11.6 with other work beside it).  One or two: M = 1 w1
-// and w3 of 14336 x 4096 (3584) 21 / 26; M = 4 these 26.0 / 24.5, two of 14336 and 4096 x 4096 between single launches (2304) 16.1 / 18.4.  M = 8,
-// however many: 4096 x 4096 (512) 9.6 / 12.9, 720 18.6 / 18.8, 14336 x 4096 (1792) 24.6 / 19.8.
+// Against gemv_mma.cu (M <= 8), by k-blocks an SM has: that one needs no second launch and starts 5 us earlier, this one takes eight rows almost as
+// fast as one and many xs as fast as few, which there are a round and new digits each.  Lists as launches of a dependent chain, us as gemv_mma /
+// gemv_tc (A: 4096 x 4096, 512 blocks; B: 14336 x 4096, C: 4096 x 14336, 1792 each).  One x:
+//   1 or 2 rows  10 A 25.5 / 26.6, 2 B 18.5 / 22.2      3 or 4  6 A 20.2 / 23.5, 2 B 23.0 / 23.5, 8 A 25.8 / 24.2
+//   5 or 6       B 16.7 / 16.9, 4 A 18.7 / 24, 6 A 26.0 / 25.8, 2 B 31 / 28     7 or 8  3 A 18.7 / 22.2, B 20.1 / 17.5, C 25.2 / 20.4, 4 A 23.6 / 24.0
+// Several xs:
+//   1 or 2 rows  8 A of 4 21.3 / 24.5, B C 21.3 / 23.3, B B C 36 / 28          3 or 4  5 A of 5 20.1 / 23.5, 6 A of 6 26 / 25, B C 35 / 24.2
+//   5 or 6       4 A of 4 19.5 / 24, 5 A of 5 31 / 25                            7 or 8  2 A of 2 15.0 / 18.4, 3 A of 3 25.4 / 22.5
 bool gemv_tc_pays(const GemvItem* items, int n, int M, int sm_count) {
-    int xs = 1;
-    for (int i = 1; i < n; ++i) xs += items[i].x != items[i - 1].x;
-    const int per = M > 4 ? 6 : xs > 2 ? (M > 2 ? 14 : 22) : (M > 2 ? 20 : 28);
-    return gv_blocks(items, n) >= (long long)sm_count * per;
+    static const int blocks[4][2] = {{37, 32}, {25, 20}, {20, 16}, {12, 10}};       // by pairs of rows; one x or several
+    bool several = false;
+    for (int i = 1; i < n; ++i) several = several || items[i].x != items[0].x || items[i].in_features != items[0].in_features;
+    return M <= 8 && gv_blocks(items, n) >= (long long)sm_count * blocks[(M - 1) / 2][several];
 }
 
 namespace {

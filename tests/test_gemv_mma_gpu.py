@@ -362,3 +362,36 @@ def test_one_matrix_whose_tiles_are_cut(M, O, I):
         assert np.linalg.norm(one.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
         for y in (chain, first, second):
             assert torch.equal(y, one)
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("M,O,I", [(1, 4001, 44032), (2, 4001, 44032), (4, 4001, 44032), (6, 4001, 44032), (7, 4001, 14336), (8, 4001, 14336), (8, 2000, 28672)])
+def test_one_matrix_of_up_to_eight_rows_whose_tiles_are_cut(M, O, I, wide):
+    """Long enough for the tcgen05 kernel by itself: sums of a tile over a cluster, or over the workspace where x has to be taken in slices;
+    alone and as a chain of recorded launches."""
+    stream, ctx = _context()
+    with torch.cuda.stream(stream):
+        g = torch.Generator(device=DEV).manual_seed(M + I)
+        x = torch.randn(M, I, device=DEV, generator=g)
+        if wide:
+            x *= 2.0 ** -(torch.arange(I, device=DEV) * 3 // I * 6).float()
+        w = torch.randint(-2 ** 31, 2 ** 31 - 1, (O, I // 16), dtype=torch.int32, device=DEV, generator=g)
+        s = torch.rand(O, device=DEV, generator=g) + 0.1
+        one, chain = torch.full((M, O), 5.0, device=DEV), torch.full((M, O), 5.0, device=DEV)
+        before = ctx.launch_count
+        ctx.ternary_gemv(x, w, s, one, M, I, O)
+        ctx.finish()
+        ctx.batch_begin()
+        for _ in range(2):
+            ctx.ternary_gemv(x, w, s, chain, M, I, O)
+        batch = ctx.batch_end()
+        for _ in range(2):
+            batch.launch()
+        ctx.finish()
+        assert ctx.launch_count - before == 2 * (1 + 4)
+        batch.close()
+        digits = torch.stack([((w >> (2 * k)) & 3).double() - 1.0 for k in range(16)], dim=2).view(O, I)
+        want = (x.double() @ digits.T) * s.double()
+        assert torch.equal(one, chain)
+        for m in range(M):
+            assert float((one[m] - want[m]).norm() / want[m].norm()) <= 1e-6
