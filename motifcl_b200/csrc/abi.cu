@@ -446,7 +446,7 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
     }
     MCL_TRY(split_tensors(ctx, op, sd.data(), (int)sd.size()));
     if (!ed.empty()) MCL_TC(ctx, op, mcl::launch_expand_ternary(ed.data(), (int)ed.size(), (int)C, ctx->sm_count, ctx->stream, &_n));
-    // products of one kind together, the longest items first (they are dealt round-robin)
+    // products of one kind together, the longest items first (they are drawn in this order)
     std::stable_sort(pr.begin(), pr.end(), [](const mcl::TcProblem& a, const mcl::TcProblem& b) {
         const int ta = a.turned ? 2 : a.b.planes + 1, tb = b.turned ? 2 : b.b.planes + 1;
         if (ta != tb) return ta > tb;
