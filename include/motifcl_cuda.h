@@ -305,7 +305,7 @@ int mcl_cuda_eltwise_f32(mcl_cuda_ctx* ctx, int op, const float* a, const float*
  *                           f32 keys/values, no mask
  *   gqa_backward            probs_scratch, ds_scratch [B*n_head*Tq*Tk]; grad_q/k/v shaped like q/k/v
  *                           (attention, head_dim <= 64: keys that a query does not attend to count as 0 times their value where
- *                           they share a tile of 64 with ones that it does, so an infinity or NaN there makes its result NaN) ---- */
+ *                           they share a tile of 64 with ones that it does, so an infinity or NaN there can make its result NaN) ---- */
 int mcl_cuda_rmsnorm(mcl_cuda_ctx* ctx, const float* x, const float* weight, float* out, size_t rows, size_t cols,
                      float eps);
 int mcl_cuda_rmsnorm_backward_x(mcl_cuda_ctx* ctx, const float* x, const float* weight, const float* grad_out,
@@ -365,7 +365,10 @@ int mcl_cuda_adam_update(mcl_cuda_ctx* ctx, float* param, const float* grad, flo
                          float beta1, float beta2, float eps, float weight_decay, float c1, float c2);
 
 /* ---- ternary decode GEMV, M <= 16 (no reference kernel; semantics of the forward above
- * applied to 2-bit weights).  y[M,out] = x[M,in] * (scale . t)^T.  Requires in % 16 == 0. ---- */
+ * applied to 2-bit weights).  y[M,out] = x[M,in] * (scale . t)^T.  Requires in % 16 == 0.
+ * x enters with 30 bits below the largest magnitude of each of up to eight slices of K (M <= 8) or of its row (M > 8); a row with
+ * an infinity or NaN gives NaN.  A result is the same bits alone, recorded and whatever shares its launch.  An unrecorded call of more
+ * than 8 rows, or of a matrix of tens of millions of weights, may make the workspace grow. ---- */
 int mcl_cuda_ternary_gemv(mcl_cuda_ctx* ctx, const float* x, const uint32_t* packed2,
                           const float* scale, float* y, size_t M, size_t in_features,
                           size_t out_features);

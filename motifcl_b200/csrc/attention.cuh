@@ -184,10 +184,10 @@ __device__ __forceinline__ void tile_range(const GqaDims& p, int q0, int& kb, in
     ke = b1;
 }
 
-// queries q0 .. q0 + 31 of the head blockIdx.x, by 128 threads
 template <int NC>
-__device__ __forceinline__ void fwd_rows(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, float* __restrict__ out,
-                                         const GqaDims& p, int q0) {
+__global__ void __launch_bounds__(4 * kBQ, 128 / kBQ) gqa_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                         const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
+    grid_release();
     extern __shared__ __align__(16) float sm[];
     constexpr int BQ = kBQ, HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
@@ -195,6 +195,7 @@ __device__ __forceinline__ void fwd_rows(const float* __restrict__ q, const floa
     float* ks = qs + HDP * QS + grp * fwd_group_floats<NC>();           // this group's k [64][HS], v [64][HS], P^T [64][QS]
     float* vs = ks + kKT * HS;
     float* pt = vs + kKT * HS;
+    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, g = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.key_stride * kld + g * p.hd;
@@ -300,19 +301,12 @@ __device__ __forceinline__ void fwd_rows(const float* __restrict__ q, const floa
     }
 }
 
-// the tiles with the longest rows first
-__device__ __forceinline__ int tile_begin(const GqaDims& p, int rows) { return ((p.tq + rows - 1) / rows - 1 - (int)blockIdx.y) * rows; }
-template <int NC>
-__global__ void __launch_bounds__(128, 4) gqa_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                                         float* __restrict__ out, GqaDims p) {
-    grid_release();
-    fwd_rows<NC>(q, k, v, out, p, tile_begin(p, kBQ));
-}
-
 // probs, ds [B, n_head, tq, tk]; dq
 template <int NC>
-__device__ __forceinline__ void bwd_q_rows(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v, const float* __restrict__ dout,
-                                           float* __restrict__ probs, float* __restrict__ ds, float* __restrict__ dq, const GqaDims& p, int q0) {
+__global__ void __launch_bounds__(4 * kBQ, 128 / kBQ) gqa_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                           const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
+                                                           float* __restrict__ dq, GqaDims p) {
+    grid_release();
     extern __shared__ __align__(16) float sm[];
     constexpr int BQ = kBQ, HDP = 16 * NC, HS = HDP + 4, QS = BQ + 4, NT = 2 * BQ;
     const int grp = threadIdx.x / NT, t = threadIdx.x % NT, tx = t & 15, ty = t >> 4;
@@ -321,6 +315,7 @@ __device__ __forceinline__ void bwd_q_rows(const float* __restrict__ q, const fl
     float* ks = gs + HDP * QS + grp * bwd_q_group_floats<NC>();      // this group's k [64][HS]
     float* vs = ks + kKT * HS;            // pass 1: v [64][HS]; pass 2: dS^T [64][QS]
     float* st = gs + HDP * QS + 2 * bwd_q_group_floats<NC>();        // [2][3][BQ]: maximum, sum, sum of P dP of each group
+    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, g = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.tk * kld + g * p.hd;
@@ -484,19 +479,12 @@ __device__ __forceinline__ void bwd_q_rows(const float* __restrict__ q, const fl
         }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(128, 4) gqa_bwd_q_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                                           const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
-                                                           float* __restrict__ dq, GqaDims p) {
-    grid_release();
-    bwd_q_rows<NC>(q, k, v, dout, probs, ds, dq, p, tile_begin(p, kBQ));
-}
-
 constexpr int kQT = 32;               // queries per tile of the key kernel
-// 64 keys of one kv head by G groups of 128 threads, which take the tiles of 32 queries in turn
-template <int NC, int G>
-__device__ __forceinline__ void bwd_k_keys(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
-                                           const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, const GqaDims& p) {
+// CTA = 64 keys of one kv head, two groups of 128 threads that take alternate tiles of 32 queries
+template <int NC>
+__global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
+                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
+    grid_release();
     extern __shared__ __align__(16) float sm[];
     constexpr int HDP = 16 * NC, HS = HDP + 4, KS = kKT + 4;
     const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, tx = t & 15, ty = t >> 4;
@@ -527,22 +515,22 @@ __device__ __forceinline__ void bwd_k_keys(const float* __restrict__ q, const fl
     };
     first(grp);
     second(grp);
-    for (int n = grp; n < count; n += G) {
+    for (int n = grp; n < count; n += 2) {
         copies_wait<2>();
         group_sync(grp, 128);
         outer<NC>(av, ps, KS, gs, HS, kQT, ty, tx);
         group_sync(grp, 128);
-        first(n + G);
+        first(n + 2);
         copies_wait<2>();
         group_sync(grp, 128);
         outer<NC>(ak, ss, KS, qs, HS, kQT, ty, tx);
         group_sync(grp, 128);
-        second(n + G);
+        second(n + 2);
     }
     copies_wait<0>();
     float* mg = sm + bwd_k_group_floats<NC>();
     static_assert(bwd_k_group_floats<NC>() >= (size_t)16 * NC * 128, "merge area");
-    if (G > 1) __syncthreads();
+    __syncthreads();
     if (grp == 1) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -553,7 +541,7 @@ __device__ __forceinline__ void bwd_k_keys(const float* __restrict__ q, const fl
                 mg[((4 * i + 2) * NC + j) * 128 + t] = e.x; mg[((4 * i + 3) * NC + j) * 128 + t] = e.y;
             }
     }
-    if (G > 1) __syncthreads();
+    __syncthreads();
     if (grp == 1) return;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -564,14 +552,8 @@ __device__ __forceinline__ void bwd_k_keys(const float* __restrict__ q, const fl
                 const float2 f = halves(av[i >> 1][j]), e = halves(ak[i >> 1][j]);
                 const long long at = ((long long)b * p.tk + key) * kld + g * p.hd + tx + 16 * j;
                 const int r = 4 * (i >> 1) + (i & 1);
-                dv[at] = (i & 1 ? f.y : f.x) + (G > 1 ? mg[(r * NC + j) * 128 + t] : 0.0f);
-                dk[at] = ((i & 1 ? e.y : e.x) + (G > 1 ? mg[((r + 2) * NC + j) * 128 + t] : 0.0f)) * p.scale;
+                dv[at] = (i & 1 ? f.y : f.x) + mg[(r * NC + j) * 128 + t];
+                dk[at] = ((i & 1 ? e.y : e.x) + mg[((r + 2) * NC + j) * 128 + t]) * p.scale;
             }
     }
-}
-template <int NC>
-__global__ void __launch_bounds__(256, 2) gqa_bwd_k_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
-                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
-    grid_release();
-    bwd_k_keys<NC, 2>(q, dout, probs, ds, dk, dv, p);
 }

@@ -11,8 +11,8 @@
 //             (written, as the reference leaves them) and dq += dS K.
 //             kernel 2 (keys): dv = P^T dO, dk = dS^T Q, summed over the query heads of the kv head; P and dS are read in
 //             operand order, 32 bytes of a row by eight lanes.
-// What bounds it: an m16n8k16 takes 16 cycles of a quarter SM here (512 multiply-adds per clock and SM, a sixth of that for fp32; the FMAs of
-// attention.cuh could do 256 but wait for shared memory).  Causal, us with FMAs and here: 16 sequences of 256 tokens, 6 heads of
+// What bounds it: a warp's chain of loads, products and exponentials; the tensor pipe is busy for a quarter to a third of the time (m16n8k16 takes 8
+// cycles of a quarter SM here: 1016 multiply-adds per clock and SM, a sixth of that for fp32; the FMAs of attention.cuh could do 256).  Causal, us with FMAs and here: 16 sequences of 256 tokens, 6 heads of
 // 48: forward 37 and 28, backward 111 and 80; 16 of 512, 12 heads of 64: 316 and 184, 798 and 557; one of 33 tokens, 8 heads of 48: 14 and 8, 40
 // and 24; a grid of 192 CTAs with eight key tiles each (2 of 512, 12 of 64) 50 and 68, 206 and 268.  Error against float64 1.5 to 2.5e-7 (2.1 to 5.1e-7).
 #pragma once
@@ -30,7 +30,6 @@ template <int NC>
 struct AttTile {                                     // 64 rows of HDP columns, three planes of bf16 terms; the pitch keeps ldmatrix free of conflicts
     static constexpr int HDP = 16 * NC, kPitch = HDP + 8, kPlane = 64 * kPitch * 2, kBytes = 3 * kPlane;
     static constexpr int kRaw = 64 * HDP * 4;        // the fp32 rows as they come
-    static constexpr size_t kShared = 2 * (kBytes + kRaw);
 };
 __device__ __forceinline__ uint32_t sm_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // staging rows -> terms; thread t of NT
@@ -146,8 +145,8 @@ __device__ __forceinline__ void load_rows(uint32_t (&a)[NC][3][4], const float* 
 __device__ __forceinline__ float quad_max(float v) { v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1)); return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2)); }
 __device__ __forceinline__ float quad_sum(float v) { v += __shfl_xor_sync(0xffffffffu, v, 1); return v + __shfl_xor_sync(0xffffffffu, v, 2); }
 
-// Terms of an infinity are an infinity and NaNs.  A CTA whose results are not all finite does its part again with the fp32 FMAs of
-// attention.cuh, where an infinity stays one: NaN or infinity in an operand that a result takes shows in the result.
+// Terms of an infinity are an infinity and NaNs.  A warp whose results are not all finite does its rows again as plain fp32 sums over the
+// keys that they attend to: an infinity or NaN in an operand shows in the result.
 template <int N>
 __device__ __forceinline__ bool beyond_fp32(const float (&c)[N][4]) {
     bool b = false;
@@ -155,24 +154,98 @@ __device__ __forceinline__ bool beyond_fp32(const float (&c)[N][4]) {
     for (int n = 0; n < N; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) b = b || !(fabsf(c[n][i]) <= FLT_MAX);
-    return b;
+    return __any_sync(0xffffffffu, b);
 }
-template <int NC>
-__device__ __noinline__ void fwd_again(const float* q, const float* k, const float* v, float* out, const GqaDims& p, int q0) {
-    fwd_rows<NC>(q, k, v, out, p, q0);
+__device__ __forceinline__ float row_dot(const float* a, const float* b, int n) {
+    float s = 0.0f;
+    for (int d = 0; d < n; ++d) s = fmaf(a[d], b[d], s);
+    return s;
 }
-template <int NC>
-__device__ __noinline__ void bwd_q_again(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, const GqaDims& p, int q0) {
-    bwd_q_rows<NC>(q, k, v, dout, probs, ds, dq, p, q0);
+// c (columns lane and lane + 32) += sum over 32 lanes of w times that lane's row; rows: the first of them, ld apart
+__device__ __forceinline__ void add_rows(float (&c)[2], float w, const float* rows, long long ld, int count, int n, int lane) {
+    for (int j = 0; j < count; ++j) {
+        const float f = __shfl_sync(0xffffffffu, w, j);
+        for (int i = 0; i < 2; ++i)
+            if (lane + 32 * i < n) c[i] = fmaf(f, rows[j * ld + lane + 32 * i], c[i]);
+    }
 }
-template <int NC>
-__device__ __noinline__ void bwd_k_again(const float* q, const float* dout, const float* probs, const float* ds, float* dk, float* dv, const GqaDims& p) {
-    bwd_k_keys<NC, 1>(q, dout, probs, ds, dk, dv, p);
+// rows r0 .. r0 + 15: q and out at row 0 of the head
+__device__ __noinline__ void fwd_again(const float* q, const float* k, const float* v, float* out, const GqaDims& p, int r0) {
+    const int lane = threadIdx.x & 31;
+    const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
+    for (int r = r0; r < min(r0 + 16, p.tq); ++r) {
+        const int lo = row_lo(p, r), hi = row_hi(p, r);
+        float m = -FLT_MAX, l = 0.0f, c[2] = {};
+        for (int k0 = lo; k0 < hi; k0 += 32)
+            if (k0 + lane < hi) m = fmaxf(m, row_dot(q + r * qld, k + (k0 + lane) * kld, p.hd) * p.scale);
+        m = warp_max(m);
+        for (int k0 = lo; k0 < hi; k0 += 32) {
+            const float e = k0 + lane < hi ? expf(row_dot(q + r * qld, k + (k0 + lane) * kld, p.hd) * p.scale - m) : 0.0f;
+            l += e;
+            add_rows(c, e, v + k0 * kld, kld, min(32, hi - k0), p.hd, lane);
+        }
+        l = warp_sum(l);
+        for (int i = 0; i < 2; ++i)
+            if (lane + 32 * i < p.hd) out[r * qld + lane + 32 * i] = c[i] * (l > 0.0f ? 1.0f / l : 0.0f);
+    }
+}
+// rows r0 .. r0 + 15 of probs, ds (of this head) and dq
+__device__ __noinline__ void bwd_q_again(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, const GqaDims& p, int r0) {
+    const int lane = threadIdx.x & 31;
+    const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
+    __syncwarp();                                          // other lanes wrote to these rows
+    for (int r = r0; r < min(r0 + 16, p.tq); ++r) {
+        const int hi = row_hi(p, r);
+        float* pr = probs + (long long)r * p.tk;
+        float* dr = ds + (long long)r * p.tk;
+        float m = -FLT_MAX, l = 0.0f, dot = 0.0f, c[2] = {};
+        for (int j = lane; j < hi; j += 32) {              // this lane reads them back
+            pr[j] = row_dot(q + r * qld, k + j * kld, p.hd) * p.scale;
+            dr[j] = row_dot(dout + r * qld, v + j * kld, p.hd);
+            m = fmaxf(m, pr[j]);
+        }
+        m = warp_max(m);
+        for (int j = lane; j < hi; j += 32) {
+            const float e = expf(pr[j] - m);
+            l += e;
+            dot = fmaf(e, dr[j], dot);
+        }
+        l = warp_sum(l);
+        l = l > 0.0f ? 1.0f / l : 0.0f;
+        dot = warp_sum(dot) * l;
+        for (int k0 = 0; k0 < p.tk; k0 += 32) {
+            const int j = k0 + lane;
+            const float e = j < hi ? expf(pr[j] - m) * l : 0.0f, w = j < hi ? e * (dr[j] - dot) : 0.0f;
+            if (j < p.tk) { pr[j] = e; dr[j] = w; }
+            if (k0 < hi) add_rows(c, w, k + k0 * kld, kld, min(32, hi - k0), p.hd, lane);
+        }
+        for (int i = 0; i < 2; ++i)
+            if (lane + 32 * i < p.hd) dq[r * qld + lane + 32 * i] = c[i] * p.scale;
+    }
+}
+// keys k0 .. k0 + 15 of a kv head: q, dout, probs and ds at the first query head of its group
+__device__ __noinline__ void bwd_k_again(const float* q, const float* dout, const float* probs, const float* ds, float* dk, float* dv, const GqaDims& p, int k0) {
+    const int lane = threadIdx.x & 31;
+    const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
+    for (int key = k0; key < min(k0 + 16, p.tk); ++key) {
+        float cv[2] = {}, ck[2] = {};
+        for (int h = 0; h < p.n_head / p.n_kv; ++h)
+            for (int r = p.causal ? max(key - p.q_off, 0) : 0; r < p.tq; ++r) {
+                const long long at = ((long long)h * p.tq + r) * p.tk + key;
+                for (int i = 0; i < 2; ++i)
+                    if (lane + 32 * i < p.hd) {
+                        cv[i] = fmaf(probs[at], dout[r * qld + h * p.hd + lane + 32 * i], cv[i]);
+                        ck[i] = fmaf(ds[at], q[r * qld + h * p.hd + lane + 32 * i], ck[i]);
+                    }
+            }
+        for (int i = 0; i < 2; ++i)
+            if (lane + 32 * i < p.hd) { dv[key * kld + lane + 32 * i] = cv[i]; dk[key * kld + lane + 32 * i] = ck[i] * p.scale; }
+    }
 }
 
 template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                                       const float* __restrict__ v, float* __restrict__ out, GqaDims p) {
+                                                                       const float* __restrict__ v, float* __restrict__ out, const __grid_constant__ GqaDims p) {
     grid_release();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
@@ -180,7 +253,7 @@ __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __rest
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
     unsigned char *ks = smb, *vs = smb + T::kBytes;
     float *kr = reinterpret_cast<float*>(smb + 2 * T::kBytes), *vr = kr + T::kRaw / 4;
-    const int q0 = tile_begin(p, BQ);
+    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, gr = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd;
     const float* kb_ = k + (long long)b * p.key_stride * kld + gr * p.hd;
@@ -253,8 +326,8 @@ __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __rest
         }
     }
     copies_wait<0>();
-    if (__syncthreads_or(beyond_fp32(o))) {
-        for (int r = q0; r < min(q0 + BQ, p.tq); r += kBQ, __syncthreads()) fwd_again<NC>(q, k, v, out, p, r);
+    if (beyond_fp32(o)) {
+        fwd_again(q + (long long)b * p.tq * qld + h * p.hd, kb_, vb, out + (long long)b * p.tq * qld + h * p.hd, p, r0);
         return;
     }
     float* ob = out + (long long)b * p.tq * qld + h * p.hd;
@@ -275,7 +348,7 @@ __global__ void __launch_bounds__(128, 2) gqa_fwd_mma_kernel(const float* __rest
 template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                                            const float* __restrict__ dout, float* __restrict__ probs, float* __restrict__ ds,
-                                                           float* __restrict__ dq, GqaDims p) {
+                                                           float* __restrict__ dq, const __grid_constant__ GqaDims p) {
     grid_release();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
@@ -283,7 +356,7 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
     unsigned char *ks = smb, *vs = smb + T::kBytes;
     float *kr = reinterpret_cast<float*>(smb + 2 * T::kBytes), *vr = kr + T::kRaw / 4;
-    const int q0 = tile_begin(p, BQ);
+    const int tiles = (p.tq + BQ - 1) / BQ, q0 = (tiles - 1 - (int)blockIdx.y) * BQ;
     const int b = blockIdx.x / p.n_head, h = blockIdx.x % p.n_head, gr = h / (p.n_head / p.n_kv);
     const long long qld = (long long)p.n_head * p.hd, kld = (long long)p.n_kv * p.hd, at = (long long)b * p.tq * qld + h * p.hd;
     const float* kb_ = k + (long long)b * p.tk * kld + gr * p.hd;
@@ -417,8 +490,9 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
         }
     }
     copies_wait<0>();
-    if (__syncthreads_or(beyond_fp32(acc))) {
-        for (int r = q0; r < min(q0 + BQ, p.tq); r += kBQ, __syncthreads()) bwd_q_again<NC>(q, k, v, dout, probs, ds, dq, p, r);
+    if (beyond_fp32(acc)) {
+        const long long head = (long long)blockIdx.x * p.tq * p.tk;
+        bwd_q_again(q + at, kb_, vb, dout + at, probs + head, ds + head, dq + at, p, r0);
         return;
     }
     // beyond every query of the tile: zeros
@@ -442,7 +516,7 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_q_mma_kernel(const float* __re
 // CTA = 64 keys of one kv head, a warp 16 of them
 template <int NC>
 __global__ void __launch_bounds__(128, 2) gqa_bwd_k_mma_kernel(const float* __restrict__ q, const float* __restrict__ dout, const float* __restrict__ probs,
-                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, GqaDims p) {
+                                                        const float* __restrict__ ds, float* __restrict__ dk, float* __restrict__ dv, const __grid_constant__ GqaDims p) {
     grid_release();
     extern __shared__ __align__(16) unsigned char smb[];
     using T = AttTile<NC>;
@@ -523,8 +597,9 @@ __global__ void __launch_bounds__(128, 2) gqa_bwd_k_mma_kernel(const float* __re
         add(ak, qs);
     }
     copies_wait<0>();
-    if (__syncthreads_or(beyond_fp32(av) || beyond_fp32(ak))) {
-        bwd_k_again<NC>(q, dout, probs, ds, dk, dv, p);
+    if (beyond_fp32(av) || beyond_fp32(ak)) {
+        const long long first = (long long)b * p.tq * qld + gr * group * p.hd, head = ((long long)b * p.n_head + gr * group) * p.tq * p.tk, to = (long long)b * p.tk * kld + gr * p.hd;
+        bwd_k_again(q + first, dout + first, probs + head, ds + head, dk + to, dv + to, p, k0 + 16 * warp);
         return;
     }
 #pragma unroll

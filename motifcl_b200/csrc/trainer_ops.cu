@@ -10,7 +10,6 @@
 // tiled fp32 products around a softmax row pass instead of the shaders' one workgroup per query.
 #include "kernels.h"
 
-#include <algorithm>
 #include <cfloat>
 
 namespace mcl {
@@ -812,7 +811,7 @@ bool gqa_tiled(int batch, int tq, int tk, int n_head, int hd, int vhd) {
 // the others (2 sequences of 512, 12 heads of 64: backward 207 us, 257 when launched early).
 template <int NC>
 cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* out, const GqaDims& p, cudaStream_t stream, bool mma) {
-    const size_t fma = fwd_floats<NC>() * 4, bytes = mma ? std::max(AttTile<NC>::kShared, fma) : fma;      // either may run on tensor cores
+    const size_t bytes = mma ? 2 * (AttTile<NC>::kBytes + AttTile<NC>::kRaw) : fwd_floats<NC>() * 4;
     const auto kern = mma ? gqa_fwd_mma_kernel<NC> : gqa_fwd_kernel<NC>;
     const cudaError_t e = with_smem(kern, bytes);
     if (e != cudaSuccess) return e;
@@ -823,8 +822,7 @@ cudaError_t run_gqa_fwd(const float* q, const float* k, const float* v, float* o
 template <int NC>
 cudaError_t run_gqa_bwd(const float* q, const float* k, const float* v, const float* dout, float* probs, float* ds, float* dq, float* dk,
                         float* dv, const GqaDims& p, cudaStream_t stream, bool mma) {
-    const size_t fma = bwd_q_floats<NC>() * 4, bq = mma ? std::max(AttTile<NC>::kShared, fma) : fma;
-    const size_t bk = mma ? std::max(AttTile<NC>::kShared, bwd_k_group_floats<NC>() * 4) : bwd_k_floats<NC>() * 4;
+    const size_t tiles = 2 * (AttTile<NC>::kBytes + AttTile<NC>::kRaw), bq = mma ? tiles : bwd_q_floats<NC>() * 4, bk = mma ? tiles : bwd_k_floats<NC>() * 4;
     const auto kq = mma ? gqa_bwd_q_mma_kernel<NC> : gqa_bwd_q_kernel<NC>;
     const auto kk = mma ? gqa_bwd_k_mma_kernel<NC> : gqa_bwd_k_kernel<NC>;
     cudaError_t e = with_smem(kq, bq);

@@ -426,3 +426,34 @@ def test_gqa_infinities_are_those_of_fp32(ctx, B, Tq, Tk, H, G, hd, where, value
         assert torch.equal(torch.isnan(x), torch.isnan(w)) and torch.equal(x == math.inf, w == math.inf) and torch.equal(x == -math.inf, w == -math.inf), n
         assert rel_l2(x[finite], w[finite]) <= 1e-6, n
     assert all(not torch.isfinite(want[n]).all() for n in {"v": ("out", "dq"), "k": ("dq",), "q": ("out",), "dout": ("dv",)}[where])
+
+
+@pytest.mark.parametrize("B,T,H,G,hd", [(2, 60, 4, 2, 48), (25, 130, 6, 3, 33)])            # on tensor cores
+def test_gqa_infinities_stay_out_of_rows_that_do_not_see_them(ctx, B, T, H, G, hd):
+    """Causal: an infinite value reaches its column of the queries from its key on, an infinite gradient that of the keys up to its query, also
+    inside a tile; all else is as with a zero there."""
+    g = torch.Generator().manual_seed(T)
+    q, k, v, dout = (torch.randn(B * T, c * hd, generator=g).double() for c in (H, G, G, H))
+    at, head, col, scale = 37, 1, 5, 1.0 / math.sqrt(hd)
+    v[at, head * hd + col] = dout[at, head * (H // G) * hd + col] = 0.0
+    q.requires_grad_(), k.requires_grad_(), v.requires_grad_()
+    want, _ = _attention_reference(q, k, v, B, T, T, H, G, hd, hd, True, 0, 0, scale)
+    want.backward(dout)
+    vi, gi = v.detach().clone(), dout.clone()
+    vi[at, head * hd + col] = math.inf
+    gi[at, head * (H // G) * hd + col] = math.inf
+    out, probs, ds = torch.full((B * T, H * hd), 7.0, device="cuda"), *(torch.full((B * H * T * T,), 7.0, device="cuda") for _ in range(2))
+    dq, dk, dv = torch.full_like(out, 7.0), *(torch.full((B * T, G * hd), 7.0, device="cuda") for _ in range(2))
+    ctx.gqa_forward(dev(q.detach()), dev(k.detach()), dev(vi), out, B, T, T, T, H, G, hd, hd, True, 0, 0, scale)
+    ctx.gqa_backward(dev(q.detach()), dev(k.detach()), dev(v.detach()), dev(gi), probs, ds, dq, dk, dv, B, T, T, H, G, hd, True, 0, scale)
+    torch.cuda.synchronize()
+    touched = torch.zeros(B * T, H * hd, dtype=torch.bool)
+    for h in range(head * (H // G), (head + 1) * (H // G)):
+        touched[at:T, h * hd + col] = True
+    assert torch.equal(out.cpu() == math.inf, touched) and rel_l2(out.cpu()[~touched], want[~touched]) <= 1e-6
+    touched = torch.zeros(B * T, G * hd, dtype=torch.bool)
+    touched[:at + 1, head * hd + col] = True
+    assert torch.equal(dv.cpu() == math.inf, touched) and rel_l2(dv.cpu()[~touched], v.grad[~touched]) <= 1e-6
+    rows = torch.ones(B * T, H * hd, dtype=torch.bool)
+    rows[at, head * (H // G) * hd:(head * (H // G) + 1) * hd] = False
+    assert rel_l2(dq.cpu()[rows], q.grad[rows]) <= 1e-6
