@@ -307,20 +307,14 @@ __global__ void __launch_bounds__(kCeThreads) ce_kernel(const float* logits, con
             const float inv = 1.0f / s;
             float* g = grad_logits + row * (size_t)cols;
             float4* g4 = reinterpret_cast<float4*>(g);
-            for (int i0 = threadIdx.x; i0 < n4; i0 += 4 * kCeThreads) {
-                float4 v[4];                       // four loads in flight before the stores
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (i0 + k * kCeThreads < n4) v[k] = __ldcs(l4 + i0 + k * kCeThreads);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int i = i0 + k * kCeThreads, c = 4 * i;
-                    if (i < n4)
-                        __stcs(g4 + i, make_float4(gscale * (expf(v[k].x - m) * inv - (c == t ? 1.0f : 0.0f)),
-                                                   gscale * (expf(v[k].y - m) * inv - (c + 1 == t ? 1.0f : 0.0f)),
-                                                   gscale * (expf(v[k].z - m) * inv - (c + 2 == t ? 1.0f : 0.0f)),
-                                                   gscale * (expf(v[k].w - m) * inv - (c + 3 == t ? 1.0f : 0.0f))));
-                }
+#pragma unroll 4
+            for (int i = threadIdx.x; i < n4; i += kCeThreads) {
+                const float4 v = __ldcs(l4 + i);
+                const int c = 4 * i;
+                __stcs(g4 + i, make_float4(gscale * (expf(v.x - m) * inv - (c == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.y - m) * inv - (c + 1 == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.z - m) * inv - (c + 2 == t ? 1.0f : 0.0f)),
+                                           gscale * (expf(v.w - m) * inv - (c + 3 == t ? 1.0f : 0.0f))));
             }
             for (int c = 4 * n4 + threadIdx.x; c < cols; c += kCeThreads)
                 g[c] = gscale * (expf(l[c] - m) * inv - (c == t ? 1.0f : 0.0f));
