@@ -397,8 +397,8 @@ int products_chunk(mcl_cuda_ctx* ctx, const char* op, const ProductLayer* L, siz
         dw_cg = cost[1] < cost[0] ? 2 : 1;
     }
     // A product with digits alone in its launch runs as C^T = T X^T where that wastes less of the last tile of tokens: tokens are then its
-    // columns, in tiles of 64 to 256, not its rows, in tiles of 128 or 256 (777 tokens: 800 columns for 1024 rows).  A forward, us: 777 x 4096 ->
-    // 14336 205 -> 180, 300 x 4096 -> 4096 56.6 -> 50.6, 90 x 1024 -> 1024 22.5 -> 19.3.  Not where an accumulator would take a longer
+    // columns, in tiles of 64 to 256, not its rows, in tiles of 128 or 256 (777 tokens: 800 columns for 1024 rows).  Forwards one after the other on a
+    // stream, us: 777 x 4096 -> 14336 205 -> 180, 300 x 4096 -> 4096 62 -> 53.  Not where an accumulator would take a longer
     // slice of K: its error grows with it (40 x 4096 -> 14336, 5 slices: 86 us and 1.1e-7, turned in one 89 and 3.1e-7).
     auto row_plan = [&](size_t M, size_t N, size_t K, bool* turned) {
         if (n > 1) return mcl::tc_plan_shared((int)M, (int)N, (int)K, 2, M > 128 ? 2 : 1, 0, 0);

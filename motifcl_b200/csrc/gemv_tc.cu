@@ -21,11 +21,12 @@
 // first weights are on their way meanwhile (programmatic dependent launch).
 //
 // What bounds it: an SM has to take 90 weights per clock at 6.5 TB/s (the copies alone run at 5.1 to 5.9 TB/s in these boxes).  20 matrices
-// of an 8B-scale model (210 MB) as one list take 62 us for one row of x, 65 for 4, 74 for 8 and 81 for 16 (2.6 to 3.4 TB/s; 50, 52, 63 and 69 with
-// other work beside them), where a launch or three per matrix took 157, 333 and 368.  The fifth digit costs 4 rows 5 % and 8 rows 14 % (16 and 32 more
-// digit columns; without it, in the unit of the largest slice, the others would lose bits); an x in slices takes 94 us for one row, 188 for 8.
-// MMAs issued from a single-lane branch cost 93 cycles each whatever their N (62 us of an earlier 78 for one row); 64 digit columns bring 16 KB of
-// digits beside 16 KB of words per k-block, so two accumulators (RT = 2) share them: 16 rows 82 -> 80 us, one row 70 -> 60.
+// of an 8B-scale model (210 MB) as one list take 65 us for one row of x, 68 for 4, 77 for 8 and 83 for 16 (2.5 to 3.2 TB/s; 50, 52, 62 and 69 with
+// other work beside them), where a launch or three per matrix took 157, 333 and 368.  The fifth digit costs 4 rows 4 % and 8 rows 13 % (16
+// more digit columns; without it, in the unit of the largest slice, the others would lose bits); an x in slices takes 100 us for one row, 167 for 8.
+// MMAs issued from a single-lane branch took most of the time, whatever their N; 64 digit columns bring 16 KB of digits beside 16 KB of words
+// per k-block, so two accumulators (RT = 2) share them: 16 rows 82 -> 80 us, one row 70 -> 60.  The epilogue of a tile is not overlapped
+// within a CTA: what it loads (scales, sums of x) is loaded under the wait for the accumulator (16 rows 82.9 -> 79.5).
 #include <cuda.h>
 
 #include <algorithm>
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(192 + 128 * RT, 2) gemv_tc_kernel(const __grid
         }
     } else if (warp == 1) {
         // ---- MMA issuer: RT x 8 x (128 x Nq x 32) int8 MMAs per k-block.  The whole warp runs the loop and one lane is elected around
-        // the instructions: descriptors are warp-uniform then (93 cycles an MMA from a single-lane branch, whatever its N) ----
+        // the instructions: descriptors are warp-uniform then ----
         const uint32_t idesc = idesc_i8(GV_ROWS, Nq);
         const uint64_t db0 = smem_desc_k_sw128(base + RT * GV_RAW);
         const uint32_t db_hi = (uint32_t)(db0 >> 32), db_lo = (uint32_t)db0, db_stage = stage_bytes >> 4, db_half = b_tile >> 4;
